@@ -44,6 +44,15 @@ def test_gemm_staged_epilogue_blocks(dtype, M, N):
     t = pre.double().requires_grad_(True)
     torch.nn.functional.gelu(t).sum().backward()
     _near(gemm(x, w, dgelu=True, aux_in=pre), z * t.grad, dtype, 1)
+    # what must not be hidden from an overflow check, and signed zeros
+    odd = torch.zeros(M, K, device="cuda", dtype=dtype)
+    one = torch.zeros(N, K, device="cuda", dtype=dtype)
+    edge = torch.tensor([float("inf"), float("nan"), 0.0, -0.0, 6e4, -6e4], device="cuda").to(dtype)
+    b6 = torch.zeros(N, device="cuda", dtype=dtype)
+    b6[:6] = edge
+    got = gemm(odd, one, bias=b6, gelu=True)[0, :6].float()
+    assert torch.isinf(got[0]) and got[0] > 0 and torch.isnan(got[1]) and (got[2:4] == 0).all()
+    assert got[4] == edge[4].float() and got[5] == 0
     acc = torch.full((M + 1, N + 4), 3.0, device="cuda")
     gemm(x, w, out=acc[:M, :N], accumulate=True, alpha=0.5)
     _near(acc[:M, :N], 0.5 * z + 3.0, dtype, 0)
@@ -52,3 +61,32 @@ def test_gemm_staged_epilogue_blocks(dtype, M, N):
     _near(f32, z, dtype, 0)
     torch.cuda.synchronize()
     assert _lib.read_error() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows", [1, 3, 9, 1187, 5000])
+@pytest.mark.parametrize("H", [256, 512, 768, 1024, 1536, 2048, 3072, 4096])
+def test_layernorm_ring_of_rows(dtype, rows, H):
+    """Every width's split of a row over warps; fewer rows than the ring is deep, and several turns of it."""
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(2)
+    x, res, dy = (torch.randn(rows, H, device="cuda").to(dtype) for _ in range(3))
+    g = (torch.randn(H, device="cuda") * 0.1 + 1).to(dtype)
+    b = (torch.randn(H, device="cuda") * 0.1).to(dtype)
+    for r, p in ((res, 0.0), (None, 0.0), (res, 0.25)):
+        y, z, mean, rstd = K.ln_fwd(x, r, g, b, 1e-5, p=p, seed=7, offset=3)
+        kept = K.dropout(x, p, 7, 3) != 0 if p else None
+        xd = x.double() if kept is None else torch.where(kept, x.double() / (1 - p), 0.0 * x.double())
+        _near(z, xd + (0 if r is None else r.double()), dtype, 1)
+        zz = z.double().requires_grad_(True)
+        gg, bb = g.double().requires_grad_(True), b.double().requires_grad_(True)
+        want = torch.nn.functional.layer_norm(zz, (H,), gg, bb, 1e-5)
+        _near(y, want, dtype, 1)
+        want.backward(dy.double())
+        dz, dx, dg, db = K.ln_bwd(dy, z, g, mean, rstd, p=p, seed=7, offset=3)
+        _near(dz, zz.grad, dtype, 1)
+        if kept is not None:
+            _near(dx, torch.where(kept, zz.grad / (1 - p), 0.0 * zz.grad), dtype, 1)
+        _near(dg, gg.grad, dtype, 0)
+        _near(db, bb.grad, dtype, 0)
