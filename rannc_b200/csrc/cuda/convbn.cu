@@ -116,6 +116,54 @@ __global__ void col2im_kernel(const T* __restrict__ dcols, T* __restrict__ dx, i
 }
 
 // ---------------------------------------------------------------------------------------------------
+// Operands of the implicit-GEMM convolution
+// ---------------------------------------------------------------------------------------------------
+// out [N, H + pad, W + pad, C] = x [N, H, W, C] with zero columns behind every row and zero rows behind every image;
+// one block per padded image row.  Bound by memory: one pass that reads x once and writes every output vector once (a
+// generic pad clears the output and then copies the interior with a strided kernel: 32 x 28 x 28 x 1024 took 80 us
+// that way; this takes 17 us).
+__global__ void __launch_bounds__(256)
+    pad_nhwc_kernel(const uint4* __restrict__ x, uint4* __restrict__ out, int H, int W, int cv, int pad) {
+    const int Wp = W + pad, Hp = H + pad;
+    const int n = blockIdx.x / Hp, y = blockIdx.x - n * Hp;
+    uint4* o = out + static_cast<long long>(blockIdx.x) * Wp * cv;
+    const uint4* row = x + (static_cast<long long>(n) * H + y) * W * cv;
+    const int live = y < H ? W * cv : 0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < Wp * cv; i += 256) o[i] = i < live ? row[i] : make_uint4(0, 0, 0, 0);
+}
+
+// The weight gradient comes out of its GEMM as src [Co, taps, Ci] fp32 and belongs into a [Co, Ci, taps] tensor:
+// added to an fp32 gradient buffer (ADD) or rounded to a 16-bit gradient.  A block takes 128 channels of one
+// filter through shared memory so that both sides are touched in whole lines; the row stride (4 banks) keeps the
+// transposed reads of a 3 x 3 filter nearly conflict-free.
+constexpr int FOLD_C = 128, FOLD_LD = FOLD_C + 4;
+template <typename OutT, bool ADD>
+__global__ void __launch_bounds__(256)
+    wgrad_fold_kernel(const float* __restrict__ src, OutT* __restrict__ dst, int Ci, int taps) {
+    extern __shared__ float tile[];  // [taps][FOLD_LD]
+    const int c0 = blockIdx.x * FOLD_C, nc = min(FOLD_C, Ci - c0);
+    const long long co = blockIdx.y;
+    src += co * taps * Ci + c0;
+    dst += (co * Ci + c0) * taps;
+#pragma unroll 5
+    for (int i = threadIdx.x; i < taps * FOLD_C; i += 256) {
+        const int t = i / FOLD_C, c = i - t * FOLD_C;
+        if (c < nc) tile[t * FOLD_LD + c] = src[static_cast<long long>(t) * Ci + c];
+    }
+    __syncthreads();
+#pragma unroll 5
+    for (int i = threadIdx.x; i < taps * nc; i += 256) {
+        const int c = i / taps, t = i - c * taps;
+        const float v = tile[t * FOLD_LD + c];
+        if constexpr (ADD)
+            dst[i] += v;
+        else
+            dst[i] = from_f32<OutT>(v);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------
 // batch norm
 // ---------------------------------------------------------------------------------------------------
 // part[0][c] += sum_r a(r, c), part[1][c] += sum_r a(r, c) * b(r, c); a thread owns 8 adjacent channels,
@@ -316,6 +364,32 @@ extern "C" int rb_col2im(const void* dcols, void* dx, int N, int H, int W, int C
     else
         col2im_kernel<__half><<<ew_grid(total), 256, 0, st>>>(static_cast<const __half*>(dcols),
                                                              static_cast<__half*>(dx), N, H, W, C, Ho, Wo, k, s, pad);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// x [N, H, W, C] -> out [N, H + pad, W + pad, C], 16-bit elements, zeros behind every row and image
+extern "C" int rb_pad_nhwc(const void* x, void* out, int N, int H, int W, int C, int pad, void* stream) {
+    if (C % 8 || pad < 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15)) return -2;
+    if (N <= 0 || H <= 0 || W <= 0) return 0;
+    rb::pad_nhwc_kernel<<<static_cast<unsigned>(N) * (H + pad), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const uint4*>(x), static_cast<uint4*>(out), H, W, C / 8, pad);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// src fp32 [Co, taps, Ci] into dst [Co, Ci, taps]; dtype 2: added to fp32, 1 / 0: written as bf16 / fp16
+extern "C" int rb_wgrad_fold(const float* src, void* dst, int Co, int Ci, int taps, int dtype, void* stream) {
+    using namespace rb;
+    if (Co <= 0 || Ci <= 0 || taps <= 0) return 0;
+    const int smem = taps * FOLD_LD * static_cast<int>(sizeof(float));
+    if (smem > 48 * 1024 || Co > 65535) return -2;
+    const dim3 grid((Ci + FOLD_C - 1) / FOLD_C, Co);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (dtype == 2)
+        wgrad_fold_kernel<float, true><<<grid, 256, smem, st>>>(src, static_cast<float*>(dst), Ci, taps);
+    else if (dtype == 1)
+        wgrad_fold_kernel<__nv_bfloat16, false><<<grid, 256, smem, st>>>(src, static_cast<__nv_bfloat16*>(dst), Ci, taps);
+    else
+        wgrad_fold_kernel<__half, false><<<grid, 256, smem, st>>>(src, static_cast<__half*>(dst), Ci, taps);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -84,6 +84,7 @@ struct GemmKernelParams {
     int* err;
     // implicit-GEMM convolution: see RbGemmArgs
     int conv_kb_per_tap, conv_b_tap_cols, b_row_shift;
+    int wgrad_taps, wgrad_cols;
     int map_hp, map_wp, map_h, map_w, map_pad;
     int conv_shift[49];
     // 1: the epilogue goes through shared memory and the copy engine (tensor maps of D and of the auxiliary
@@ -295,6 +296,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                             bk = ax;
                         }
                     }
+                    // 64 columns of B (MN-major) from column n on, the rows of this k step
+                    auto b_chunk = [&](int n, int& cx, int& cy) {
+                        cx = n + bx;
+                        cy = bk;
+                        if (p.wgrad_taps > 0) {
+                            // column block -> filter tap: the tap's rows are shifted; past the last tap the
+                            // column lies outside the matrix and reads as zero
+                            const int tap = min(n / p.wgrad_cols, p.wgrad_taps - 1);
+                            cx = n - tap * p.wgrad_cols;
+                            cy = k0 + p.conv_shift[tap];
+                        }
+                    };
                     if constexpr (PAIR) {
                         // both CTAs' bytes are counted on the first CTA's barrier
                         if (crank == 0) mbar_arrive_expect_tx(&full[stage], 2 * STAGE_BYTES);
@@ -310,8 +323,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                             tma_load_3d_pair(b_dst, &tmB, fb, k0, n0, b);
                         } else {
 #pragma unroll
-                            for (int c = 0; c < Cfg<PAIR>::B_ROWS / 64; ++c)
-                                tma_load_3d_pair(b_dst + c * (BK * 128), &tmB, fb, n0 + bx + c * 64, bk, b);
+                            for (int c = 0; c < Cfg<PAIR>::B_ROWS / 64; ++c) {
+                                int cx, cy;
+                                b_chunk(n0 + c * 64, cx, cy);
+                                tma_load_3d_pair(b_dst + c * (BK * 128), &tmB, fb, cx, cy, b);
+                            }
                         }
                     } else {
                         mbar_arrive_expect_tx(&full[stage], STAGE_BYTES);
@@ -327,9 +343,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                             tma_load_3d(b_dst, &tmB, &full[stage], k0, n0, b);
                         } else {
 #pragma unroll
-                            for (int c = 0; c < BN / 64; ++c)
-                                tma_load_3d(b_dst + c * (BK * 128), &tmB, &full[stage], n0 + bx + c * 64,
-                                            bk, b);
+                            for (int c = 0; c < BN / 64; ++c) {
+                                int cx, cy;
+                                b_chunk(n0 + c * 64, cx, cy);
+                                tma_load_3d(b_dst + c * (BK * 128), &tmB, &full[stage], cx, cy, b);
+                            }
                         }
                     }
                     if (++stage == STAGES) {
@@ -1023,6 +1041,18 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
         p.conv_b_tap_cols = a->conv_b_tap_cols;
         for (int t = 0; t < a->conv_taps; ++t) p.conv_shift[t] = a->conv_shift[t];
     }
+    p.wgrad_taps = 0;
+    p.wgrad_cols = 1;
+    if (a->wgrad_taps > 0) {
+        // a 64-column block of B must lie within one tap
+        if (a->wgrad_taps > 49 || a->conv_taps > 0 || a->b_major != 1 || a->conv_c % 64 || a->conv_c <= 0 ||
+            a->N != static_cast<int64_t>(a->wgrad_taps) * a->conv_c || a->batch != 1 || a->b_row_shift ||
+            a->ag_nranks > 1 || a->rs_nranks > 1)
+            return -7;
+        p.wgrad_taps = a->wgrad_taps;
+        p.wgrad_cols = a->conv_c;
+        for (int t = 0; t < a->wgrad_taps; ++t) p.conv_shift[t] = a->conv_shift[t];
+    }
     if (a->map_hp > 0 && (a->batch != 1 || a->rs_nranks > 1 || a->map_wp <= 0)) return -7;
 
     CUtensorMap tmA, tmB;
@@ -1044,7 +1074,8 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
         rc = make_tmap_3d(&tmB, a->B, a->in_dtype, static_cast<uint64_t>(a->conv_taps) * a->conv_b_tap_cols,
                           a->conv_c, 1, a->ldb * 2, static_cast<uint64_t>(a->conv_c) * a->ldb * 2, 64, BK, 1);
     else
-        rc = make_tmap_3d(&tmB, a->B, a->in_dtype, a->N, a->K, a->batch, a->ldb * 2, sB, 64, BK, 1);
+        rc = make_tmap_3d(&tmB, a->B, a->in_dtype, a->wgrad_taps > 0 ? a->conv_c : a->N, a->K, a->batch, a->ldb * 2, sB,
+                          64, BK, 1);
     if (rc) return rc;
 
     // The staged epilogue wants outputs the copy engine can address: plain rows in this GPU's memory, 16-byte

@@ -55,6 +55,11 @@ typedef struct RbGemmArgs {
     // output rows are positions of the padded grid: only the interior (map_pad <= y < map_pad + map_h, same for
     // x) is stored, at row (n * map_h + y - map_pad) * map_w + (x - map_pad) of D.  map_hp = 0: rows are rows.
     int32_t map_hp, map_wp, map_h, map_w, map_pad;
+    // weight gradient of such a convolution (wgrad_taps > 0): B is the padded activation [rows, conv_c] (b_major
+    // = 1, N = wgrad_taps * conv_c); output columns [t * conv_c, (t + 1) * conv_c) are the product with the rows
+    // shifted by conv_shift[t].  One launch for all taps: the gradient operand A is read once per column of
+    // tiles instead of once per tap.
+    int32_t wgrad_taps;
 } RbGemmArgs;
 
 // returns 0 on success, <0 on a host-side error (-2: operand not 16 B aligned)

@@ -28,7 +28,7 @@ class _Args(ctypes.Structure):
         ("conv_taps", ctypes.c_int32), ("conv_c", ctypes.c_int32), ("conv_b_tap_cols", ctypes.c_int32),
         ("b_row_shift", ctypes.c_int32), ("conv_shift", ctypes.c_int32 * 49),
         ("map_hp", ctypes.c_int32), ("map_wp", ctypes.c_int32), ("map_h", ctypes.c_int32),
-        ("map_w", ctypes.c_int32), ("map_pad", ctypes.c_int32),
+        ("map_w", ctypes.c_int32), ("map_pad", ctypes.c_int32), ("wgrad_taps", ctypes.c_int32),
     ]
 
 
@@ -72,7 +72,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
          dgelu: bool = False, out: torch.Tensor | None = None, accumulate: bool = False,
          out_dtype: torch.dtype | None = None, alpha: float = 1.0, max_ctas: int = 0,
          rs_peers=None, rs_ld: int = 0, gather=None, conv=None, b_row_shift: int = 0,
-         row_map=None) -> torch.Tensor:
+         row_map=None, wgrad_shifts=None) -> torch.Tensor:
     """``out = epilogue(alpha * op(a) @ op(b))``.
 
     ``a`` is stored ``[M, K]`` (``trans_a=False``) or ``[K, M]`` (``trans_a=True``).
@@ -84,6 +84,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
     rows shifted by ``shifts[tap]`` (rows outside ``a`` read as zero).  ``b`` is ``[N, T*C]`` (``trans_b=True``) or
     ``[C, T*b_tap_cols]`` with tap t's ``[C, N]`` block at column ``t * b_tap_cols`` (``trans_b=False``).
     ``b_row_shift`` (``trans_b=False`` only): the rows of ``b`` a k-block reads are shifted by this many.
+    ``wgrad_shifts`` (``trans_b=False`` only): ``b`` is the padded activation ``[rows, C]`` and the result has one
+    block of C columns per shift, ``a``'s product with the rows of ``b`` shifted by it (weight gradient of a
+    convolution, all taps in one launch).
     ``row_map = (Hp, Wp, H, W, pad)``: the M rows are positions of a padded image grid; only the interior is
     stored, at the un-padded row index (``out`` has N_img * H * W rows).
     """
@@ -103,6 +106,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
             if br != ac or bc < (T - 1) * int(conv["b_tap_cols"]) + N:
                 raise ValueError("gemm: weight matrix does not hold the taps' blocks")
         K = Kb = T * ac
+    if wgrad_shifts is not None:
+        if trans_b or b.dim() != 2 or a.dim() != 2 or conv is not None or b_row_shift or bc % 64:
+            raise ValueError("gemm: wgrad_shifts needs a 2-D b stored [rows, C], C a multiple of 64")
+        N = bc * len(wgrad_shifts)
     if K != Kb:
         raise ValueError(f"gemm: inner dimensions differ ({K} vs {Kb})")
     batch = max(ba, bb)
@@ -158,6 +165,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         args.conv_c = ac
         args.conv_b_tap_cols = int(conv.get("b_tap_cols", 0))
         for i, sh in enumerate(conv["shifts"]):
+            args.conv_shift[i] = int(sh)
+    if wgrad_shifts is not None:
+        args.wgrad_taps = len(wgrad_shifts)
+        args.conv_c = bc
+        for i, sh in enumerate(wgrad_shifts):
             args.conv_shift[i] = int(sh)
     if b_row_shift:
         if trans_b:

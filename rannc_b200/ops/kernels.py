@@ -280,6 +280,23 @@ def col2im(dcols, N: int, H: int, W: int, C: int, k: int, s: int, pad: int):
     return dx
 
 
+def pad_nhwc(x_nhwc, pad: int):
+    """[N, H, W, C] (contiguous) with ``pad`` zero columns behind every row and ``pad`` zero rows behind every image."""
+    N, H, W, C = x_nhwc.shape
+    out = torch.empty(N, H + pad, W + pad, C, dtype=x_nhwc.dtype, device=x_nhwc.device)
+    _lib.check(_lib.lib().rb_pad_nhwc(_lib.vp(x_nhwc), _lib.vp(out), c_int(N), c_int(H), c_int(W), c_int(C), c_int(pad),
+                                      _lib.stream_ptr()), "rb_pad_nhwc")
+    return out
+
+
+def wgrad_fold(dw2d, dst, taps: int):
+    """fp32 [Co, taps * Ci] into the contiguous [Co, Ci, k, k] tensor ``dst``: added when it is fp32, written
+    (rounded) when it is 16-bit."""
+    Co, Ci = dst.shape[0], dst.shape[1]
+    _lib.check(_lib.lib().rb_wgrad_fold(_lib.vp(dw2d), _lib.vp(dst), c_int(Co), c_int(Ci), c_int(taps),
+                                        c_int(dt_code(dst)), _lib.stream_ptr()), "rb_wgrad_fold")
+
+
 def bn_fwd(x2d, residual2d, gamma32, beta32, run_mean32, run_var32, eps: float, momentum: float, relu: bool):
     """Training-mode batch norm over the rows of [R, C] (+ residual, + ReLU).  Returns (y, mean, rstd);
     the running statistics (fp32, may be None) are updated in place."""

@@ -90,3 +90,38 @@ def test_layernorm_ring_of_rows(dtype, rows, H):
             _near(dx, torch.where(kept, zz.grad / (1 - p), 0.0 * zz.grad), dtype, 1)
         _near(dg, gg.grad, dtype, 0)
         _near(db, bb.grad, dtype, 0)
+
+
+@pytest.mark.parametrize("flat", [False, True])
+@pytest.mark.parametrize("N,C,Co,H,W,k", [(2, 64, 64, 28, 26, 3), (3, 192, 72, 24, 31, 3), (1, 320, 136, 25, 24, 5),
+                                          (2, 1024, 2112, 24, 24, 3), (2, 40, 264, 9, 7, 3)])
+def test_convolution_weight_gradient(flat, N, C, Co, H, W, k):
+    """All taps in one GEMM (column blocks that straddle taps, split and unsplit K), padded operands, and the fold
+    into the [Co, Ci, k, k] layout for both kinds of gradient; a gathered-matrix case last."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops import functional as RF
+
+    torch.manual_seed(3)
+    cl = torch.channels_last
+    x = torch.randn(N, C, H, W, device="cuda").bfloat16().to(memory_format=cl).requires_grad_(True)
+    w = (torch.randn(Co, C, k, k, device="cuda") * (C * k * k) ** -0.5).bfloat16().requires_grad_(True)
+    if flat:
+        w.main_grad = torch.full((Co, C, k, k), 2.0, device="cuda")
+    y = RF.conv2d(x, w, None, 1, k // 2)
+    dy = torch.randn(N, Co, H, W, device="cuda").bfloat16().to(memory_format=cl)
+    y.backward(dy)
+    xr, wr = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    ref = torch.nn.functional.conv2d(xr, wr, None, 1, k // 2)
+    ref.backward(dy.double())
+    torch.cuda.synchronize()
+    assert _lib.read_error() == 0
+    steps = lambda terms: terms / 16 * 2.0 ** -23  # noqa: E731
+    _near(y, ref.detach(), torch.bfloat16, 1, steps(C * k * k))
+    if flat:
+        _near(w.main_grad - 2.0, wr.grad, torch.bfloat16, 0, steps(N * H * W) + 1e-5)
+    else:
+        assert w.grad.shape == w.shape
+        _near(w.grad, wr.grad, torch.bfloat16, 1, steps(N * H * W))
+    # the gathered path rounds every tap's contribution before it sums them
+    terms = 1 if RF._Conv2d._implicit(k, 1, k // 2, C, Co, H, W) else k * k
+    _near(x.grad, xr.grad, torch.bfloat16, terms, steps(Co * k * k) + (4e-3 if terms > 1 else 0.0))
