@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "debug_check.cuh"
 #include "philox.cuh"
 #include "tc_common.cuh"
@@ -202,6 +204,66 @@ __global__ void embed_bwd_kernel(const long long* __restrict__ ids, const T* __r
     for (int i = lane; i < H; i += 32) atomicAdd(dst + i, to_f32<T>(src[i]));
 }
 
+// Vector variant of embed_bwd_kernel: a thread owns 4 adjacent columns (8 bytes per row) of STRIP consecutive rows and
+// keeps their sum in registers for as long as the id stays the same.  Not memory but the atomic units bound this:
+// a segment table has two rows, so in the scalar kernel every token of a batch adds to one of two addresses per
+// column; equal neighbours (segments, padding) cost one reduction per strip here.  Ids that differ cost the same
+// 32-byte sectors as before in a quarter of the instructions.  (8 columns per thread, as two 16-byte reductions 32
+// bytes apart from lane to lane, touches every sector twice and was slower than the scalar kernel on such ids.)
+template <typename T, int STRIP>
+__global__ void __launch_bounds__(256)
+    embed_bwd_vec_kernel(const long long* __restrict__ ids, const T* __restrict__ dout,
+                         float* __restrict__ dtable, int rows, int nv, long long vocab,
+                         long long padding_idx) {
+    constexpr int FLIGHT = STRIP < 8 ? STRIP : 8;   // rows on their way at a time
+    const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    const long long strip = t / nv;
+    const int vec = static_cast<int>(t - strip * nv);
+    const long long r0 = strip * STRIP;
+    if (r0 >= rows) return;
+    const int n = static_cast<int>(min(static_cast<long long>(STRIP), rows - r0));
+    const long long ld = static_cast<long long>(nv) * 4;
+    const T* src = dout + r0 * ld + vec * 4;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    long long cur = -1;   // the id whose sum `acc` holds; -1: none
+    auto flush = [&]() {
+        if (cur < 0) return;
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dtable + cur * ld + vec * 4), "f"(acc[0]),
+                     "f"(acc[1]), "f"(acc[2]), "f"(acc[3])
+                     : "memory");
+    };
+#pragma unroll
+    for (int k0 = 0; k0 < STRIP; k0 += FLIGHT) {
+        if (k0 >= n) break;
+        long long id[FLIGHT];
+        uint2 q[FLIGHT];
+#pragma unroll
+        for (int u = 0; u < FLIGHT; ++u) {
+            id[u] = -1;
+            if (k0 + u < n) {
+                id[u] = ids[r0 + k0 + u];
+                if (id[u] < 0 || id[u] >= vocab || id[u] == padding_idx) id[u] = -1;
+                q[u] = *reinterpret_cast<const uint2*>(src + (k0 + u) * ld);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < FLIGHT; ++u) {
+            if (id[u] < 0) continue;
+            const T* e = reinterpret_cast<const T*>(&q[u]);
+            if (id[u] != cur) {
+                flush();
+                cur = id[u];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[j] = to_f32<T>(e[j]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[j] += to_f32<T>(e[j]);
+            }
+        }
+    }
+    flush();
+}
+
 // Row copy between two row-major buffers with different row offsets; used to
 // pack micro-batch slices and pipeline send buffers.  bytes_per_row % 16 == 0.
 __global__ void rowcopy_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst,
@@ -338,6 +400,27 @@ extern "C" int rb_embed_bwd(const long long* ids, const void* dout, float* dtabl
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (rows <= 0) return 0;
     RB_DEBUG_RANGE(ids, rows, 0, vocab, padding_idx, st);
+    if (H % 4 == 0 && ((reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dtable)) & 15) == 0) {
+        const int nv = H / 4;
+        // long strips save reductions where ids repeat, short ones keep the GPU busy on small batches: below
+        // a million 4-element groups strips of 16 rows leave less than four warps per scheduler
+        const bool longer = static_cast<long long>(rows) * nv >= (1LL << 20);
+        const int strip = longer ? 16 : 4;
+        const long long threads = (static_cast<long long>(rows) + strip - 1) / strip * nv;
+        const unsigned blocks = static_cast<unsigned>((threads + 255) / 256);
+        auto go = [&](auto* d) {
+            using T = std::remove_const_t<std::remove_pointer_t<decltype(d)>>;
+            if (longer)
+                embed_bwd_vec_kernel<T, 16><<<blocks, 256, 0, st>>>(ids, d, dtable, rows, nv, vocab, padding_idx);
+            else
+                embed_bwd_vec_kernel<T, 4><<<blocks, 256, 0, st>>>(ids, d, dtable, rows, nv, vocab, padding_idx);
+        };
+        if (dtype == 1)
+            go(static_cast<const __nv_bfloat16*>(dout));
+        else
+            go(static_cast<const __half*>(dout));
+        return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    }
     const int g = (rows * 32 + 255) / 256;
     if (dtype == 1)
         embed_bwd_kernel<__nv_bfloat16><<<g, 256, 0, st>>>(

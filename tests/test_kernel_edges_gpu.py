@@ -125,3 +125,26 @@ def test_convolution_weight_gradient(flat, N, C, Co, H, W, k):
     # the gathered path rounds every tap's contribution before it sums them
     terms = 1 if RF._Conv2d._implicit(k, 1, k // 2, C, Co, H, W) else k * k
     _near(x.grad, xr.grad, torch.bfloat16, terms, steps(Co * k * k) + (4e-3 if terms > 1 else 0.0))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,H", [(1, 8), (3, 264), (17, 1024), (4099, 256), (16400, 1024)])
+def test_embedding_backward_strips(dtype, rows, H):
+    """Strips of rows whose ids repeat, differ, are the padding id or lie outside the table."""
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(1)
+    V = 37
+    ids = torch.randint(-2, V + 2, (rows,), device="cuda")
+    ids[rows // 3:rows // 2] = 5
+    dout = torch.randn(rows, H, device="cuda").to(dtype)
+    table = torch.ones(V, H, device="cuda")
+    K.embed_bwd(ids, dout, table, padding_idx=9)
+    keep = (ids >= 0) & (ids < V) & (ids != 9)
+    want = torch.ones(V, H, device="cuda", dtype=torch.float64)
+    want.index_add_(0, ids[keep], dout[keep].double())
+    # fp32 sums of up to `rows` terms of size one in any order: error grows like the square root of their number
+    assert (table.double() - want).abs().max().item() <= 2.0 ** -23 * 8 * max(1.0, rows ** 0.5) * 4
+    shifted = torch.ones(V * H + 1, device="cuda")[1:].view(V, H)     # 4-byte aligned only: the scalar kernel
+    K.embed_bwd(ids, dout, shifted, padding_idx=9)
+    assert (shifted.double() - want).abs().max().item() <= 2.0 ** -23 * 8 * max(1.0, rows ** 0.5) * 4
