@@ -166,16 +166,36 @@ __global__ void __launch_bounds__(256)
 // ---------------------------------------------------------------------------------------------------
 // batch norm
 // ---------------------------------------------------------------------------------------------------
-// part[0][c] += sum_r a(r, c), part[1][c] += sum_r a(r, c) * b(r, c); a thread owns 8 adjacent channels,
-// a block of (32, 8) covers 256 channels, rows are strided over threadIdx.y and blockIdx.y.
+__device__ __forceinline__ void ldf8(const float* p, float (&v)[8]) {
+    const float4 a = *reinterpret_cast<const float4*>(p);
+    const float4 b = *reinterpret_cast<const float4*>(p + 4);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+// parameters may be views of a flat buffer that start at any element
+__device__ __forceinline__ void ldf8_any(const float* p, float (&v)[8]) {
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+        ldf8(p, v);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = p[j];
+    }
+}
+
+// A thread owns 8 adjacent channels (16 bytes a row) in every kernel here; a block of (BX, 256 / BX) threads covers
+// BX * 8 channels, rows are strided over threadIdx.y and blockIdx.y.  BX follows the channel count, so that a layer of
+// 64 channels does not leave three quarters of its threads without one.
+//
+// part[0][c] += sum_r a(r, c), part[1][c] += sum_r a(r, c) * b(r, c)
 //   MODE 0 (statistics):  a = x,                 b = x
 //   MODE 1 (backward):    a = dy masked by relu, b = xhat = (x - mean) * rstd
-template <typename T, int MODE>
-__global__ void bn_reduce_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ y,
-                                 const float* __restrict__ mean, const float* __restrict__ rstd,
-                                 float* __restrict__ part, long long R, int C, int relu) {
-    __shared__ float red[2][8][256 + 8];
-    const int col = blockIdx.x * 256 + threadIdx.x * 8;
+template <typename T, int MODE, int BX>
+__global__ void __launch_bounds__(256)
+    bn_reduce_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ y,
+                     const float* __restrict__ mean, const float* __restrict__ rstd,
+                     float* __restrict__ part, long long R, int C, int relu) {
+    constexpr int TY = 256 / BX;
+    __shared__ float red[2][TY][BX * 8 + 8];
+    const int col = (blockIdx.x * BX + threadIdx.x) * 8;
     float s0[8], s1[8], mu[8], rs[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) s0[j] = s1[j] = 0.f, mu[j] = 0.f, rs[j] = 1.f;
@@ -184,7 +204,7 @@ __global__ void bn_reduce_kernel(const T* __restrict__ x, const T* __restrict__ 
 #pragma unroll
             for (int j = 0; j < 8; ++j) mu[j] = mean[col + j], rs[j] = rstd[col + j];
         }
-        for (long long r = blockIdx.y * 8 + threadIdx.y; r < R; r += static_cast<long long>(gridDim.y) * 8) {
+        for (long long r = blockIdx.y * TY + threadIdx.y; r < R; r += static_cast<long long>(gridDim.y) * TY) {
             float a[8];
             ld8(x + r * C + col, a);
             if (MODE == 0) {
@@ -210,80 +230,66 @@ __global__ void bn_reduce_kernel(const T* __restrict__ x, const T* __restrict__ 
         red[1][threadIdx.y][threadIdx.x * 8 + j] = s1[j];
     }
     __syncthreads();
-    const int t = threadIdx.y * 32 + threadIdx.x;
+    const int t = threadIdx.y * BX + threadIdx.x;
+    if (t >= BX * 8) return;
     float a0 = 0.f, a1 = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) a0 += red[0][w][t], a1 += red[1][w][t];
-    const int c = blockIdx.x * 256 + t;
+    for (int w = 0; w < TY; ++w) a0 += red[0][w][t], a1 += red[1][w][t];
+    const int c = blockIdx.x * BX * 8 + t;
     if (c < C) {
         atomicAdd(part + c, a0);
         atomicAdd(part + C + c, a1);
     }
 }
 
-// mean / rstd from the sums, running statistics (momentum, unbiased variance); the per-channel scale and shift
-// of the element-wise pass replace the sums in `part`: y = x * part[0][c] + part[1][c]
-__global__ void bn_finalize_kernel(float* __restrict__ part, float* __restrict__ mean, float* __restrict__ rstd,
-                                   const float* __restrict__ gamma, const float* __restrict__ beta,
-                                   float* __restrict__ run_mean, float* __restrict__ run_var, long long R, int C,
-                                   float eps, float momentum) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
+// y = act(x * scale + shift (+ residual)) with scale = rstd gamma and shift = beta - mean scale.  Every thread derives
+// its 8 channels' scale and shift from the two sums itself (a kernel of C threads in between cost 3 us and a launch for
+// a few hundred cycles of arithmetic); the first row of blocks also writes mean, rstd and the running statistics
+// (momentum, unbiased variance).
+template <typename T, int BX>
+__global__ void __launch_bounds__(256)
+    bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, const float* __restrict__ part,
+                    const float* __restrict__ gamma, const float* __restrict__ beta, float* __restrict__ mean,
+                    float* __restrict__ rstd, float* __restrict__ run_mean, float* __restrict__ run_var,
+                    T* __restrict__ y, long long R, int C, float eps, float momentum, int relu) {
+    constexpr int TY = 256 / BX;
+    const int col = (blockIdx.x * BX + threadIdx.x) * 8;
+    if (col >= C) return;
+    float sc[8], sh[8], p0[8], p1[8];
+    ldf8(part + col, p0);
+    ldf8(part + C + col, p1);
+    ldf8_any(gamma + col, sc);
+    ldf8_any(beta + col, sh);
     const float inv = 1.f / static_cast<float>(R);
-    const float m = part[c] * inv;
-    const float var = fmaxf(part[C + c] * inv - m * m, 0.f);
-    const float rs = rsqrtf(var + eps);
-    mean[c] = m;
-    rstd[c] = rs;
-    const float sc = rs * gamma[c];
-    part[c] = sc;
-    part[C + c] = beta[c] - m * sc;
-    if (run_mean) {
-        const float unbiased = R > 1 ? var * static_cast<float>(R) / static_cast<float>(R - 1) : var;
-        run_mean[c] = (1.f - momentum) * run_mean[c] + momentum * m;
-        run_var[c] = (1.f - momentum) * run_var[c] + momentum * unbiased;
+    const bool writer = blockIdx.y == 0 && threadIdx.y == 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int c = col + j;
+        const float m = p0[j] * inv;
+        const float var = fmaxf(p1[j] * inv - m * m, 0.f);
+        const float rs = rsqrtf(var + eps);
+        sc[j] = rs * sc[j];
+        sh[j] = sh[j] - m * sc[j];
+        if (writer) {
+            mean[c] = m;
+            rstd[c] = rs;
+            if (run_mean) {
+                const float unbiased = R > 1 ? var * static_cast<float>(R) / static_cast<float>(R - 1) : var;
+                run_mean[c] = (1.f - momentum) * run_mean[c] + momentum * m;
+                run_var[c] = (1.f - momentum) * run_var[c] + momentum * unbiased;
+            }
+        }
     }
-}
-
-// backward coefficients: dx = A g + B x + Cc with A = gamma rstd, B = -gamma rstd^2 sum(g xhat) / R,
-// Cc = -A sum(g) / R - B mean; written behind the two sums: part[2..4][C]
-__global__ void bn_bwd_coef_kernel(float* __restrict__ part, const float* __restrict__ mean,
-                                   const float* __restrict__ rstd, const float* __restrict__ gamma, long long R,
-                                   int C) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
-    const float inv = 1.f / static_cast<float>(R);
-    const float A = gamma[c] * rstd[c];
-    const float B = -A * rstd[c] * part[C + c] * inv;
-    part[2 * C + c] = A;
-    part[3 * C + c] = B;
-    part[4 * C + c] = -A * part[c] * inv - B * mean[c];
-}
-
-__device__ __forceinline__ void ldf8(const float* p, float (&v)[8]) {
-    const float4 a = *reinterpret_cast<const float4*>(p);
-    const float4 b = *reinterpret_cast<const float4*>(p + 4);
-    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
-}
-
-// y = act(x * scale + shift (+ residual)); scale / shift per channel, 8 channels = two 16-byte loads each
-template <typename T>
-__global__ void bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, const float* __restrict__ scale,
-                                const float* __restrict__ shift, T* __restrict__ y, long long R, int C, int relu) {
-    const int cv = C / 8;
-    const long long total = R * cv;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int c = static_cast<int>(i % cv) * 8;
-        float v[8], o[8], sc[8], sh[8];
-        ld8(x + i * 8, v);
-        ldf8(scale + c, sc);
-        ldf8(shift + c, sh);
+    const long long step = static_cast<long long>(gridDim.y) * TY;
+#pragma unroll 2
+    for (long long r = blockIdx.y * TY + threadIdx.y; r < R; r += step) {
+        float v[8], o[8];
+        ld8(x + r * C + col, v);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = fmaf(v[j], sc[j], sh[j]);
         if (res) {
             float rr[8];
-            ld8(res + i * 8, rr);
+            ld8(res + r * C + col, rr);
 #pragma unroll
             for (int j = 0; j < 8; ++j) o[j] += rr[j];
         }
@@ -291,37 +297,94 @@ __global__ void bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ r
 #pragma unroll
             for (int j = 0; j < 8; ++j) o[j] = fmaxf(o[j], 0.f);
         }
-        st8(y + i * 8, o);
+        st8(y + r * C + col, o);
     }
 }
 
-// dx = A g + B x + Cc, g = dy masked by relu; dres = g (optional).  coef = [A, B, Cc][C]
-template <typename T>
-__global__ void bn_bwd_apply_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ y,
-                                    const float* __restrict__ coef, T* __restrict__ dx, T* __restrict__ dres,
-                                    long long R, int C, int relu) {
-    const int cv = C / 8;
-    const long long total = R * cv;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int c = static_cast<int>(i % cv) * 8;
-        float v[8], g[8], o[8], A[8], B[8], Cc[8];
-        ld8(x + i * 8, v);
-        ld8(dy + i * 8, g);
+// dx = A g + B x + Cc, g = dy masked by relu, with A = gamma rstd, B = -A rstd sum(g xhat) / R and
+// Cc = -A sum(g) / R - B mean derived per thread from the two sums; dres = g (optional).  The first row of blocks adds
+// the sums to the fp32 gradients of beta and gamma when it is given their buffers.
+template <typename T, int BX>
+__global__ void __launch_bounds__(256)
+    bn_bwd_apply_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ y,
+                        const float* __restrict__ part, const float* __restrict__ mean, const float* __restrict__ rstd,
+                        const float* __restrict__ gamma, float* __restrict__ dgamma, float* __restrict__ dbeta,
+                        T* __restrict__ dx, T* __restrict__ dres, long long R, int C, int relu) {
+    constexpr int TY = 256 / BX;
+    const int col = (blockIdx.x * BX + threadIdx.x) * 8;
+    if (col >= C) return;
+    float A[8], B[8], Cc[8], p0[8], p1[8], rs[8], mu[8];
+    ldf8(part + col, p0);
+    ldf8(part + C + col, p1);
+    ldf8_any(gamma + col, A);
+    ldf8(rstd + col, rs);
+    ldf8(mean + col, mu);
+    const float inv = 1.f / static_cast<float>(R);
+    const bool writer = blockIdx.y == 0 && threadIdx.y == 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int c = col + j;
+        A[j] = A[j] * rs[j];
+        B[j] = -A[j] * rs[j] * p1[j] * inv;
+        Cc[j] = -A[j] * p0[j] * inv - B[j] * mu[j];
+        if (writer && dgamma) dgamma[c] += p1[j];
+        if (writer && dbeta) dbeta[c] += p0[j];
+    }
+    const long long step = static_cast<long long>(gridDim.y) * TY;
+#pragma unroll 2
+    for (long long r = blockIdx.y * TY + threadIdx.y; r < R; r += step) {
+        float v[8], g[8], o[8];
+        ld8(x + r * C + col, v);
+        ld8(dy + r * C + col, g);
         if (relu) {
             float yy[8];
-            ld8(y + i * 8, yy);
+            ld8(y + r * C + col, yy);
 #pragma unroll
             for (int j = 0; j < 8; ++j) g[j] = yy[j] > 0.f ? g[j] : 0.f;
         }
-        ldf8(coef + c, A);
-        ldf8(coef + C + c, B);
-        ldf8(coef + 2 * C + c, Cc);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] = fmaf(A[j], g[j], fmaf(B[j], v[j], Cc[j]));
-        st8(dx + i * 8, o);
-        if (dres) st8(dres + i * 8, g);
+        st8(dx + r * C + col, o);
+        if (dres) st8(dres + r * C + col, g);
     }
+}
+
+// Grid of the batch-norm kernels: blocks of BX * 8 channels, and as many row groups as give the whole grid about
+// `per_sm` blocks per SM, each with four rows or more per thread.
+template <int BX>
+static dim3 bn_grid(long long R, int C, int per_sm) {
+    const int cols = (C + BX * 8 - 1) / (BX * 8);
+    long long split = (R + 4 * (256 / BX) - 1) / (4 * (256 / BX));
+    const long long want = (148LL * per_sm + cols - 1) / cols;
+    if (split > want) split = want;
+    return dim3(cols, static_cast<unsigned>(split < 1 ? 1 : split));
+}
+
+template <typename T, int BX>
+static int bn_fwd_launch(const void* x, const void* res, const float* gamma, const float* beta, void* y, float* part,
+                         float* mean, float* rstd, float* run_mean, float* run_var, long long R, int C, float eps,
+                         float momentum, int relu, cudaStream_t st) {
+    const dim3 block(BX, 256 / BX);
+    const T* xt = static_cast<const T*>(x);
+    cudaMemsetAsync(part, 0, 2 * sizeof(float) * C, st);
+    bn_reduce_kernel<T, 0, BX><<<bn_grid<BX>(R, C, 4), block, 0, st>>>(xt, nullptr, nullptr, nullptr, nullptr, part, R, C, 0);
+    bn_apply_kernel<T, BX><<<bn_grid<BX>(R, C, 4), block, 0, st>>>(xt, static_cast<const T*>(res), part, gamma, beta, mean,
+                                                                   rstd, run_mean, run_var, static_cast<T*>(y), R, C, eps,
+                                                                   momentum, relu);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+template <typename T, int BX>
+static int bn_bwd_launch(const void* x, const void* dy, const void* y, const float* mean, const float* rstd,
+                         const float* gamma, float* part, float* dgamma, float* dbeta, void* dx, void* dres, long long R,
+                         int C, int relu, cudaStream_t st) {
+    const dim3 block(BX, 256 / BX);
+    const T *xt = static_cast<const T*>(x), *dt = static_cast<const T*>(dy), *yt = static_cast<const T*>(y);
+    cudaMemsetAsync(part, 0, 2 * sizeof(float) * C, st);
+    bn_reduce_kernel<T, 1, BX><<<bn_grid<BX>(R, C, 4), block, 0, st>>>(xt, dt, yt, mean, rstd, part, R, C, relu);
+    bn_bwd_apply_kernel<T, BX><<<bn_grid<BX>(R, C, 4), block, 0, st>>>(xt, dt, yt, part, mean, rstd, gamma, dgamma, dbeta,
+                                                                       static_cast<T*>(dx), static_cast<T*>(dres), R, C,
+                                                                       relu);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 static inline int ew_grid(long long n) {
@@ -393,6 +456,11 @@ extern "C" int rb_wgrad_fold(const float* src, void* dst, int Co, int Ci, int ta
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
+#define RB_BN_DISPATCH(FN, ...)                                                                       \
+    (C >= 256 ? (dtype == 1 ? FN<__nv_bfloat16, 32>(__VA_ARGS__) : FN<__half, 32>(__VA_ARGS__))       \
+     : C > 64 ? (dtype == 1 ? FN<__nv_bfloat16, 16>(__VA_ARGS__) : FN<__half, 16>(__VA_ARGS__))       \
+              : (dtype == 1 ? FN<__nv_bfloat16, 8>(__VA_ARGS__) : FN<__half, 8>(__VA_ARGS__)))
+
 // Forward statistics + normalisation.  part: fp32 [2, C] scratch (zeroed here); mean / rstd: fp32 [C] outputs;
 // run_mean / run_var may be null (evaluation of a frozen layer is not handled here: pass training only).
 extern "C" int rb_bn_fwd(const void* x, const void* res, const float* gamma, const float* beta, void* y, float* part,
@@ -401,65 +469,17 @@ extern "C" int rb_bn_fwd(const void* x, const void* res, const float* gamma, con
     using namespace rb;
     if (C % 8 || R <= 0) return -2;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    cudaMemsetAsync(part, 0, 2 * sizeof(float) * C, st);
-    int split = static_cast<int>((R + 63) / 64);
-    const int colblocks = (C + 255) / 256;
-    const int want = (148 * 4 + colblocks - 1) / colblocks;
-    if (split > want) split = want;
-    if (split < 1) split = 1;
-    dim3 grid(colblocks, split), block(32, 8);
-    if (dtype == 1)
-        bn_reduce_kernel<__nv_bfloat16, 0><<<grid, block, 0, st>>>(static_cast<const __nv_bfloat16*>(x), nullptr, nullptr,
-                                                                  nullptr, nullptr, part, R, C, 0);
-    else
-        bn_reduce_kernel<__half, 0><<<grid, block, 0, st>>>(static_cast<const __half*>(x), nullptr, nullptr, nullptr,
-                                                           nullptr, part, R, C, 0);
-    bn_finalize_kernel<<<(C + 255) / 256, 256, 0, st>>>(part, mean, rstd, gamma, beta, run_mean, run_var, R, C, eps,
-                                                        momentum);
-    const long long total = R * (C / 8);
-    if (dtype == 1)
-        bn_apply_kernel<__nv_bfloat16><<<ew_grid(total), 256, 0, st>>>(
-            static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(res), part, part + C,
-            static_cast<__nv_bfloat16*>(y), R, C, relu);
-    else
-        bn_apply_kernel<__half><<<ew_grid(total), 256, 0, st>>>(static_cast<const __half*>(x),
-                                                               static_cast<const __half*>(res), part, part + C,
-                                                               static_cast<__half*>(y), R, C, relu);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return RB_BN_DISPATCH(bn_fwd_launch, x, res, gamma, beta, y, part, mean, rstd, run_mean, run_var, R, C, eps, momentum,
+                          relu, st);
 }
 
-// Backward.  part: fp32 [5, C] scratch; on return part[0] = d beta, part[1] = d gamma (part[2..4]: coefficients).
+// Backward.  part: fp32 [2, C] scratch; on return part[0] = d beta, part[1] = d gamma, which are also added to
+// dbeta_acc / dgamma_acc when those are given.
 extern "C" int rb_bn_bwd(const void* x, const void* dy, const void* y, const float* mean, const float* rstd,
-                         const float* gamma, float* part, void* dx, void* dres, long long R, int C, int relu, int dtype,
-                         void* stream) {
+                         const float* gamma, float* part, float* dgamma_acc, float* dbeta_acc, void* dx, void* dres,
+                         long long R, int C, int relu, int dtype, void* stream) {
     using namespace rb;
     if (C % 8 || R <= 0) return -2;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    cudaMemsetAsync(part, 0, 2 * sizeof(float) * C, st);
-    int split = static_cast<int>((R + 63) / 64);
-    const int colblocks = (C + 255) / 256;
-    const int want = (148 * 4 + colblocks - 1) / colblocks;
-    if (split > want) split = want;
-    if (split < 1) split = 1;
-    dim3 grid(colblocks, split), block(32, 8);
-    const long long total = R * (C / 8);
-    if (dtype == 1) {
-        bn_reduce_kernel<__nv_bfloat16, 1><<<grid, block, 0, st>>>(
-            static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy),
-            static_cast<const __nv_bfloat16*>(y), mean, rstd, part, R, C, relu);
-        bn_bwd_coef_kernel<<<(C + 255) / 256, 256, 0, st>>>(part, mean, rstd, gamma, R, C);
-        bn_bwd_apply_kernel<__nv_bfloat16><<<ew_grid(total), 256, 0, st>>>(
-            static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dy),
-            static_cast<const __nv_bfloat16*>(y), part + 2 * C, static_cast<__nv_bfloat16*>(dx),
-            static_cast<__nv_bfloat16*>(dres), R, C, relu);
-    } else {
-        bn_reduce_kernel<__half, 1><<<grid, block, 0, st>>>(static_cast<const __half*>(x),
-                                                           static_cast<const __half*>(dy),
-                                                           static_cast<const __half*>(y), mean, rstd, part, R, C, relu);
-        bn_bwd_coef_kernel<<<(C + 255) / 256, 256, 0, st>>>(part, mean, rstd, gamma, R, C);
-        bn_bwd_apply_kernel<__half><<<ew_grid(total), 256, 0, st>>>(
-            static_cast<const __half*>(x), static_cast<const __half*>(dy), static_cast<const __half*>(y),
-            part + 2 * C, static_cast<__half*>(dx), static_cast<__half*>(dres), R, C, relu);
-    }
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return RB_BN_DISPATCH(bn_bwd_launch, x, dy, y, mean, rstd, gamma, part, dgamma_acc, dbeta_acc, dx, dres, R, C, relu, st);
 }

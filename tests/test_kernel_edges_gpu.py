@@ -148,3 +148,36 @@ def test_embedding_backward_strips(dtype, rows, H):
     shifted = torch.ones(V * H + 1, device="cuda")[1:].view(V, H)     # 4-byte aligned only: the scalar kernel
     K.embed_bwd(ids, dout, shifted, padding_idx=9)
     assert (shifted.double() - want).abs().max().item() <= 2.0 ** -23 * 8 * max(1.0, rows ** 0.5) * 4
+
+
+@pytest.mark.parametrize("C", [8, 64, 72, 128, 264, 2048])
+@pytest.mark.parametrize("N,H,W", [(1, 1, 2), (3, 5, 7), (8, 28, 28)])
+@pytest.mark.parametrize("flat", [False, True])
+def test_batch_norm_channel_blocks(C, N, H, W, flat):
+    from rannc_b200.ops import functional as RF
+
+    torch.manual_seed(6)
+    dt, cl = torch.bfloat16, torch.channels_last
+    mk = lambda: torch.randn(N, C, H, W, device="cuda").to(dt).to(memory_format=cl)  # noqa: E731
+    x, r, dy = (mk() * 2).requires_grad_(True), mk().requires_grad_(True), mk()
+    g = (torch.rand(C, device="cuda") + 0.5).requires_grad_(True)
+    b = torch.randn(C, device="cuda").requires_grad_(True)
+    if flat:
+        g.main_grad, b.main_grad = torch.full((C,), 3.0, device="cuda"), torch.full((C,), -1.0, device="cuda")
+    rm, rv = torch.zeros(C, device="cuda"), torch.ones(C, device="cuda")
+    y = RF.batch_norm_act(x, g, b, rm, rv, True, 0.1, 1e-5, True, r)
+    y.backward(dy)
+    xr, rr, gr, br = (t.detach().double().requires_grad_(True) for t in (x, r, g, b))
+    rmr, rvr = torch.zeros(C, device="cuda", dtype=torch.float64), torch.ones(C, device="cuda", dtype=torch.float64)
+    pre = torch.nn.functional.batch_norm(xr, rmr, rvr, gr, br, True, 0.1, 1e-5) + rr
+    _near(y, torch.relu(pre).detach(), dt, 1, 1e-5)
+    _near(rm, rmr, dt, 0)
+    _near(rv, rvr, dt, 0, 1e-5)
+    # the mask comes from the rounded output: compare with that mask
+    pre.backward(dy.double() * (y > 0))
+    # two samples: x - mean cancels, and rstd amplifies the 16-bit inputs' exact difference; no extra error
+    _near(x.grad, xr.grad, dt, 1, 1e-4)
+    _near(r.grad, rr.grad, dt, 1)
+    gg, bg = (g.main_grad - 3.0, b.main_grad + 1.0) if flat else (g.grad, b.grad)
+    _near(gg, gr.grad, dt, 0, 1e-5)
+    _near(bg, br.grad, dt, 0, 1e-5)
