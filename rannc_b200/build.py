@@ -1,13 +1,15 @@
-"""In-tree build of the two native libraries.
+"""In-tree build of the three native libraries.
 
 * ``_kernels.so`` : every CUDA kernel (``csrc/cuda/*.cu``), compiled by nvcc for
   sm_100a only and exported through a plain C ABI (called with ctypes).
 * ``_core.so``    : the host-side native core (``csrc/core/*.cpp``: IR, msgpack
   codec, value classifier, partitioner, stage search, cost model, routes,
   batch arithmetic, event recorder, watchdog) as a pybind11 module.
+* ``_host.so``    : the fused operators' host side (``csrc/host/*.cpp``: autograd
+  nodes, output allocation, launches) against PyTorch's C++ API.
 
-Both are written next to this file so that they travel with the source tree.
-``python -m rannc_b200.build`` builds both; nothing is rebuilt when the
+They are written next to this file so that they travel with the source tree.
+``python -m rannc_b200.build`` builds them; nothing is rebuilt when the
 outputs are newer than every source.
 """
 from __future__ import annotations
@@ -22,6 +24,7 @@ from pathlib import Path
 HERE = Path(__file__).resolve().parent
 CUDA_SRC = HERE / "csrc" / "cuda"
 CORE_SRC = HERE / "csrc" / "core"
+HOST_SRC = HERE / "csrc" / "host"
 BUILD_DIR = HERE / "csrc" / "build"
 
 NVCC_FLAGS = [
@@ -110,6 +113,30 @@ def build_core(verbose: bool = False) -> Path:
     return out
 
 
+def build_host(verbose: bool = False) -> Path:
+    """The fused operators' host side (``csrc/host/*.cpp``: autograd nodes and launches) against PyTorch's C++ API.
+    It calls the kernels through addresses it is given at run time, so it links to no CUDA code."""
+    import torch
+    from torch.utils.cpp_extension import include_paths
+
+    ext = sysconfig.get_config_var("EXT_SUFFIX") or ".so"
+    out = HERE / ("_host" + ext)
+    srcs = sorted(HOST_SRC.glob("*.cpp"))
+    hdrs = [CUDA_SRC / "attn.h", CUDA_SRC / "gemm_tcgen05.h"]
+    if _newer(out, srcs + hdrs):
+        return out
+    inc = [d for p in include_paths() + [sysconfig.get_paths()["include"]] for d in ("-isystem", p)]
+    cuda = Path(_nvcc()).parent.parent / "include"
+    lib = Path(torch.__file__).resolve().parent / "lib"
+    log = _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall", "-pthread",
+                "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                *inc, "-isystem", str(cuda), *map(str, srcs), "-o", str(out), "-L", str(lib), f"-Wl,-rpath,{lib}",
+                "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"])
+    if verbose:
+        print(log)
+    return out
+
+
 def build_selftest(sanitize: str = "address,undefined") -> Path:
     """The native core (everything but the Python bindings) linked into a stand-alone self-test program
     (``csrc/core/selftest.cpp``) with the host sanitizers switched on: ``address,undefined`` (default) or
@@ -130,7 +157,7 @@ def build_selftest(sanitize: str = "address,undefined") -> Path:
 
 
 def build_all(verbose: bool = False):
-    return build_core(verbose), build_kernels(verbose)
+    return build_core(verbose), build_kernels(verbose), build_host(verbose)
 
 
 if __name__ == "__main__":
@@ -140,6 +167,5 @@ if __name__ == "__main__":
         print("built", build_selftest("address,undefined"))
         print("built", build_selftest("thread"))
     else:
-        c, k = build_all(verbose="-v" in sys.argv)
-        print("built", c)
-        print("built", k)
+        for path in build_all(verbose="-v" in sys.argv):
+            print("built", path)

@@ -1,0 +1,917 @@
+// The fused operators' host side: argument checks, output allocation, kernel launches and autograd nodes.
+//
+// An operator of a small batch is bound by the host: as Python autograd functions over ctypes, the forward and
+// backward of a linear layer of 32 rows took 155 us for 40 us of device time -- filling a ctypes structure and
+// re-reading strides per GEMM, two trips through the Python autograd machinery, and a hand-over of the interpreter
+// lock to the backward thread.  The nodes here are plain autograd nodes: backward runs without the interpreter
+// unless a gradient listener is installed.
+//
+// Kernels are called through the C ABI of _kernels.so; their addresses are handed over once by ops/_lib.py, so that
+// the regular and the checked build of the library serve the same code.
+// Reference counterpart: the interpreter loop of src/torch/TorchDriver.cpp:566.
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/forward_grad.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/extension.h>
+
+#include <atomic>
+#include <optional>
+#include <unordered_map>
+
+#include "../cuda/attn.h"
+#include "../cuda/gemm_tcgen05.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+using OptTensor = std::optional<Tensor>;
+
+// ------------------------------------------------------------------------------------------------ C ABI
+struct Api {
+    int (*gemm)(const RbGemmArgs*, void*);
+    int (*gelu)(const void*, const void*, void*, long long, int, int, void*);
+    int (*colsum)(const void*, float*, int, int, long long, int, void*);
+    int (*ln_fwd)(const void*, const void*, const void*, const void*, void*, void*, float*, float*, int, int, float,
+                  float, uint64_t, uint64_t, int, void*);
+    int (*ln_bwd)(const void*, const void*, const void*, const float*, const float*, void*, void*, float*, float*,
+                  float*, int, int, float, uint64_t, uint64_t, int, int, void*);
+    int (*ln_bwd_grid)(int);
+    int (*embed_fwd)(const long long*, const void*, void*, int, int, long long, int, void*);
+    int (*embed_bwd)(const long long*, const void*, float*, int, int, long long, long long, int, void*);
+    int (*xent_fwd)(const void*, const long long*, float*, float*, float*, int, int, long long, long long, float, int,
+                    void*);
+    int (*xent_bwd)(const void*, const long long*, const float*, const float*, const float*, void*, int, int, long long,
+                    long long, float, int, void*);
+    int (*attn_fwd)(const RbAttnArgs*, void*);
+    int (*attn_bwd)(const RbAttnArgs*, void*);
+    int (*bn_fwd)(const void*, const void*, const float*, const float*, void*, float*, float*, float*, float*, float*,
+                  long long, int, float, float, int, int, void*);
+    int (*bn_bwd)(const void*, const void*, const void*, const float*, const float*, const float*, float*, float*, float*,
+                  void*, void*, long long, int, int, int, void*);
+} api;
+std::atomic<long long> launches{0};
+PyObject* error_class = nullptr;   // ops._lib.KernelLibraryError
+PyObject* listener = nullptr;      // called with the parameters whose gradients were just written (under the GIL)
+std::atomic<bool> has_listener{false};
+
+void check(int rc, const char* what, int kernels = 1) {
+    if (rc == 0) {
+        launches.fetch_add(kernels, std::memory_order_relaxed);
+        return;
+    }
+    py::gil_scoped_acquire gil;
+    PyErr_Format(error_class ? error_class : PyExc_RuntimeError, "%s failed with code %d", what, rc);
+    python_error e;
+    e.persist();
+    throw e;
+}
+
+void* cur_stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+
+int dt_code(const Tensor& t) {
+    if (t.scalar_type() == at::kBFloat16) return 1;
+    if (t.scalar_type() == at::kHalf) return 0;
+    TORCH_CHECK_TYPE(false, "unsupported dtype ", t.scalar_type());
+}
+const void* cptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+template <typename T = void>
+T* mptr(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr; }
+Tensor opt(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
+Tensor f32(at::IntArrayRef sizes, const Tensor& like) { return at::empty(sizes, like.options().dtype(at::kFloat)); }
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// ------------------------------------------------------------------------------------------------ GEMM
+// A matrix as the copy engine wants it: 16-byte aligned base, unit column stride, row stride a multiple of 8.  One
+// that does not qualify is copied into rows padded to 8 elements; the padding is never read as data.
+struct Mat {
+    Tensor keep;
+    const void* p = nullptr;
+    int64_t rows = 0, cols = 0, ld = 0;
+};
+Mat mat(const Tensor& t) {
+    Mat m;
+    m.rows = t.size(0);
+    m.cols = t.size(1);
+    if (aligned16(t.data_ptr()) && t.stride(1) == 1 && t.stride(0) % 8 == 0) {
+        m.keep = t;
+    } else {
+        m.keep = at::zeros({m.rows, (m.cols + 7) / 8 * 8}, t.options()).narrow(1, 0, m.cols);
+        m.keep.copy_(t);
+    }
+    m.p = m.keep.data_ptr();
+    m.ld = m.keep.stride(0);
+    return m;
+}
+// the [rows, last dimension] matrix of a contiguous tensor, whatever its other dimensions
+Mat rows_of(const Tensor& t) {
+    const int64_t c = t.size(-1);
+    if (aligned16(t.data_ptr()) && c % 8 == 0) {
+        Mat m;
+        m.keep = t;
+        m.p = t.data_ptr();
+        m.cols = m.ld = c;
+        m.rows = c ? t.numel() / c : 0;
+        return m;
+    }
+    return mat(t.reshape({-1, c}));
+}
+Mat columns(const Mat& m, int64_t first, int64_t n) {   // n columns of m (first a multiple of 8)
+    Mat r = m;
+    r.p = static_cast<const char*>(m.p) + first * 2;
+    r.cols = n;
+    return r;
+}
+struct Epi {
+    const void* bias = nullptr;
+    const void* aux_in = nullptr;
+    void* aux_out = nullptr;
+    bool gelu = false, dgelu = false, accumulate = false;
+};
+// out [M, N] = epilogue(op(a) op(b)), rows ldd apart (0: N)
+void gemm(const Mat& a, const Mat& b, bool trans_a, bool trans_b, void* out, bool out_fp32, int dtype, const Epi& e,
+          int64_t ldd = 0) {
+    RbGemmArgs g;
+    memset(&g, 0, sizeof(g));
+    g.A = a.p;
+    g.B = b.p;
+    g.D = out;
+    g.bias = e.bias;
+    g.aux_in = e.aux_in;
+    g.aux_out = e.aux_out;
+    g.M = trans_a ? a.cols : a.rows;
+    g.K = trans_a ? a.rows : a.cols;
+    g.N = trans_b ? b.rows : b.cols;
+    const int64_t kb = trans_b ? b.cols : b.rows;
+    TORCH_CHECK_VALUE(kb == g.K, "gemm: inner dimensions differ (", g.K, " vs ", kb, ")");
+    g.batch = 1;
+    g.lda = a.ld;
+    g.ldb = b.ld;
+    g.ldd = ldd ? ldd : g.N;
+    g.a_major = trans_a ? 1 : 0;
+    g.b_major = trans_b ? 0 : 1;
+    g.in_dtype = dtype;
+    g.out_dtype = out_fp32 ? 1 : 0;
+    g.flags = (e.bias ? RB_GEMM_BIAS : 0) | (e.gelu ? RB_GEMM_GELU : 0) | (e.dgelu ? RB_GEMM_DGELU : 0) |
+              (e.accumulate ? RB_GEMM_ACCUM : 0) | (e.aux_out ? RB_GEMM_AUX_OUT : 0);
+    g.alpha = 1.f;
+    check(api.gemm(&g, cur_stream()), "rb_gemm");
+}
+// dW = dy^T x: added to the fp32 gradient buffer when there is one, returned otherwise
+Tensor weight_grad(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& mg, int dtype) {
+    Epi e;
+    if (mg.defined()) {
+        e.accumulate = true;
+        gemm(dy, x, true, false, mg.data_ptr(), true, dtype, e, mg.stride(0));
+        return Tensor();
+    }
+    Tensor dw = at::empty({dy.cols, x.cols}, w.options());
+    gemm(dy, x, true, false, dw.data_ptr(), false, dtype, e);
+    return dw;
+}
+Tensor bias_grad(const Mat& dy, const Tensor& bias, const Tensor& mg, int dtype) {
+    if (!bias.defined()) return Tensor();
+    Tensor out = mg.defined() ? mg : at::zeros({dy.cols}, bias.options().dtype(at::kFloat));
+    check(api.colsum(dy.p, mptr<float>(out), static_cast<int>(dy.rows), static_cast<int>(dy.cols), dy.ld, dtype, cur_stream()),
+          "rb_colsum");
+    return mg.defined() ? Tensor() : out.to(bias.scalar_type());
+}
+
+// ------------------------------------------------------------------------------------------------ autograd plumbing
+bool wants_grad(std::initializer_list<const Tensor*> ts) {
+    bool any = false;
+    for (const Tensor* t : ts) {
+        if (!t->defined()) continue;
+        TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined(*t),
+                                    "the fused operators have no forward-mode derivative");
+        any = any || t->requires_grad();
+    }
+    return any && at::GradMode::is_enabled();
+}
+template <typename N>
+std::shared_ptr<N> new_node() { return std::shared_ptr<N>(new N(), torch::autograd::deleteNode); }
+
+// Tells the listener, when there is one, which parameters' gradients are in their buffers now.
+void notify(std::initializer_list<std::pair<const Tensor*, const Tensor*>> param_and_buffer) {
+    if (!has_listener.load(std::memory_order_acquire)) return;
+    py::gil_scoped_acquire gil;
+    if (!listener) return;
+    py::list ps;
+    for (auto& pb : param_and_buffer)
+        if (pb.first->defined() && pb.second->defined()) ps.append(py::cast(*pb.first));
+    PyObject* r = PyObject_CallOneArg(listener, ps.ptr());
+    if (!r) {
+        python_error e;
+        e.persist();
+        throw e;
+    }
+    Py_DECREF(r);
+}
+Tensor dense(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
+
+#define RB_NODE(NAME)                                       \
+    std::string name() const override { return NAME; }      \
+    variable_list apply(variable_list&& grads) override {   \
+        std::lock_guard<std::mutex> lock(mutex_);            \
+        if (!grads[0].defined()) return variable_list(num_outputs()); \
+        return run(std::move(grads));                        \
+    }
+
+// ------------------------------------------------------------------------------------------------ linear
+struct LinearNode : Node {
+    SavedVariable x, w, pre;
+    Tensor w_ref, bias, w_mg, b_mg;
+    RB_NODE("RbLinearBackward")
+    void release_variables() override {
+        x.reset_data();
+        w.reset_data();
+        pre.reset_data();
+    }
+    variable_list run(variable_list&& grads) {
+        const Tensor X = x.unpack(), W = w.unpack(), P = pre.unpack();
+        Tensor dy = dense(grads[0]);
+        const int dt = dt_code(X);
+        if (P.defined()) {
+            Tensor d = at::empty(dy.sizes(), dy.options());
+            check(api.gelu(P.data_ptr(), dy.data_ptr(), d.data_ptr(), d.numel(), 1, dt, cur_stream()), "rb_gelu");
+            dy = d;
+        }
+        const Mat d = rows_of(dy);
+        Tensor dx, dw, db;
+        if (task_should_compute_output(0)) {
+            dx = at::empty(X.sizes(), X.options());
+            gemm(d, mat(W), false, false, dx.data_ptr(), false, dt, Epi());
+        }
+        if (task_should_compute_output(1)) dw = weight_grad(d, rows_of(X), W, w_mg, dt);
+        if (bias.defined() && task_should_compute_output(2)) db = bias_grad(d, bias, b_mg, dt);
+        notify({{&w_ref, &w_mg}, {&bias, &b_mg}});
+        return {dx, dw, db};
+    }
+};
+
+// `owner`: the parameter whose gradient is reported when w is a view of one
+Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& bias_, bool gelu, const OptTensor& w_mg,
+              const OptTensor& b_mg, const OptTensor& owner) {
+    const Tensor bias = opt(bias_);
+    const bool req = wants_grad({&x, &w, &bias});
+    Tensor y, pre, xc;
+    {
+        at::NoGradGuard off;
+        xc = dense(x);
+        auto sizes = x.sizes().vec();
+        sizes.back() = w.size(0);
+        y = at::empty(sizes, x.options());
+        Epi e;
+        e.bias = cptr(bias);
+        if (gelu) {
+            e.gelu = true;
+            pre = at::empty(sizes, x.options());
+            e.aux_out = pre.data_ptr();
+        }
+        gemm(rows_of(xc), mat(w), false, true, y.data_ptr(), false, dt_code(x), e);
+    }
+    if (req) {
+        auto n = new_node<LinearNode>();
+        n->set_next_edges(torch::autograd::collect_next_edges(x, w, bias));
+        n->x = SavedVariable(xc, false);
+        n->w = SavedVariable(w, false);
+        n->pre = SavedVariable(pre, false);
+        n->w_ref = owner.has_value() ? *owner : w;
+        n->bias = bias;
+        n->w_mg = opt(w_mg);
+        n->b_mg = opt(b_mg);
+        torch::autograd::set_history(y, n);
+    }
+    return y;
+}
+
+// ------------------------------------------------------------------------------------------------ mlp
+// y = gelu(x W1^T + b1) W2^T + b2; the GELU derivative rides in the epilogue of the dgrad GEMM
+struct MlpNode : Node {
+    SavedVariable x, w1, w2, pre, h;
+    Tensor w1_ref, w2_ref, b1, b2, w1_mg, b1_mg, w2_mg, b2_mg;
+    RB_NODE("RbMlpBackward")
+    void release_variables() override {
+        for (SavedVariable* s : {&x, &w1, &w2, &pre, &h}) s->reset_data();
+    }
+    variable_list run(variable_list&& grads) {
+        const Tensor X = x.unpack(), W1 = w1.unpack(), W2 = w2.unpack(), P = pre.unpack(), Hh = h.unpack();
+        const Tensor dy = dense(grads[0]);
+        const int dt = dt_code(X);
+        const Mat d = rows_of(dy), hm = rows_of(Hh);
+        Tensor dw2 = weight_grad(d, hm, W2, w2_mg, dt);
+        Tensor db2 = bias_grad(d, b2, b2_mg, dt);
+        Tensor dpre = at::empty(P.sizes(), P.options());
+        Epi e;
+        e.dgelu = true;
+        e.aux_in = P.data_ptr();
+        gemm(d, mat(W2), false, false, dpre.data_ptr(), false, dt, e);
+        const Mat dp = rows_of(dpre);
+        Tensor dw1 = weight_grad(dp, rows_of(X), W1, w1_mg, dt);
+        Tensor db1 = bias_grad(dp, b1, b1_mg, dt);
+        Tensor dx;
+        if (task_should_compute_output(0)) {
+            dx = at::empty(X.sizes(), X.options());
+            gemm(dp, mat(W1), false, false, dx.data_ptr(), false, dt, Epi());
+        }
+        notify({{&w1_ref, &w1_mg}, {&b1, &b1_mg}, {&w2_ref, &w2_mg}, {&b2, &b2_mg}});
+        return {dx, dw1, db1, dw2, db2};
+    }
+};
+
+Tensor mlp(const Tensor& x, const Tensor& w1, const OptTensor& b1_, const Tensor& w2, const OptTensor& b2_,
+           const OptTensor& w1_mg, const OptTensor& b1_mg, const OptTensor& w2_mg, const OptTensor& b2_mg) {
+    const Tensor b1 = opt(b1_), b2 = opt(b2_);
+    const bool req = wants_grad({&x, &w1, &b1, &w2, &b2});
+    Tensor xc, pre, h, y;
+    {
+        at::NoGradGuard off;
+        xc = dense(x);
+        auto sizes = x.sizes().vec();
+        sizes.back() = w1.size(0);
+        pre = at::empty(sizes, x.options());
+        h = at::empty(sizes, x.options());
+        sizes.back() = w2.size(0);
+        y = at::empty(sizes, x.options());
+        const int dt = dt_code(x);
+        Epi e;
+        e.bias = cptr(b1);
+        e.gelu = true;
+        e.aux_out = pre.data_ptr();
+        gemm(rows_of(xc), mat(w1), false, true, h.data_ptr(), false, dt, e);
+        Epi e2;
+        e2.bias = cptr(b2);
+        gemm(rows_of(h), mat(w2), false, true, y.data_ptr(), false, dt, e2);
+    }
+    if (req) {
+        auto n = new_node<MlpNode>();
+        n->set_next_edges(torch::autograd::collect_next_edges(x, w1, b1, w2, b2));
+        n->x = SavedVariable(xc, false);
+        n->w1 = SavedVariable(w1, false);
+        n->w2 = SavedVariable(w2, false);
+        n->pre = SavedVariable(pre, false);
+        n->h = SavedVariable(h, false);
+        n->w1_ref = w1;
+        n->w2_ref = w2;
+        n->b1 = b1;
+        n->b2 = b2;
+        n->w1_mg = opt(w1_mg);
+        n->b1_mg = opt(b1_mg);
+        n->w2_mg = opt(w2_mg);
+        n->b2_mg = opt(b2_mg);
+        torch::autograd::set_history(y, n);
+    }
+    return y;
+}
+
+// ------------------------------------------------------------------------------------------------ layer norm
+struct LnNode : Node {
+    SavedVariable z, gamma, mean, rstd;
+    Tensor g_ref, b_ref, g_mg, b_mg;
+    double p = 0;
+    uint64_t seed = 0, offset = 0;
+    RB_NODE("RbLayerNormBackward")
+    void release_variables() override {
+        for (SavedVariable* s : {&z, &gamma, &mean, &rstd}) s->reset_data();
+    }
+    variable_list run(variable_list&& grads) {
+        const Tensor Z = z.unpack(), G = gamma.unpack(), M = mean.unpack(), R = rstd.unpack();
+        const Tensor dy = dense(grads[0]);
+        const int H = static_cast<int>(Z.size(-1)), rows = static_cast<int>(Z.numel() / H);
+        const bool flat = g_mg.defined() && b_mg.defined();
+        Tensor dz = at::empty(Z.sizes(), Z.options()), dx = dz, dg = g_mg, db = b_mg;
+        if (p > 0) dx = at::empty(Z.sizes(), Z.options());
+        if (!flat) {
+            dg = f32({H}, Z);
+            db = f32({H}, Z);
+        }
+        Tensor partial = f32({static_cast<int64_t>(api.ln_bwd_grid(rows)) * 2 * H}, Z);
+        check(api.ln_bwd(dy.data_ptr(), Z.data_ptr(), G.data_ptr(), mptr<float>(M), mptr<float>(R), dz.data_ptr(),
+                         p > 0 ? dx.data_ptr() : nullptr, mptr<float>(dg), mptr<float>(db), mptr<float>(partial), rows, H,
+                         static_cast<float>(p), seed, offset, flat ? 1 : 0, dt_code(Z), cur_stream()),
+              "rb_ln_bwd", 2);
+        if (flat) {
+            notify({{&g_ref, &g_mg}, {&b_ref, &b_mg}});
+            return {dx, dz, Tensor(), Tensor()};
+        }
+        return {dx, dz, dg.to(G.scalar_type()), db.to(G.scalar_type())};
+    }
+};
+
+Tensor layer_norm(const Tensor& x, const OptTensor& res_, const Tensor& gamma, const Tensor& beta, double p, double eps,
+                  uint64_t seed, uint64_t offset, const OptTensor& g_mg, const OptTensor& b_mg) {
+    const Tensor res = opt(res_);
+    const bool req = wants_grad({&x, &res, &gamma, &beta});
+    Tensor y, z, mean, rstd;
+    {
+        at::NoGradGuard off;
+        const Tensor xc = dense(x), rc = res.defined() ? dense(res) : Tensor();
+        const int H = static_cast<int>(x.size(-1)), rows = static_cast<int>(x.numel() / H);
+        y = at::empty(xc.sizes(), xc.options());
+        if (res.defined() || p > 0) z = at::empty(xc.sizes(), xc.options());
+        mean = f32({rows}, x);
+        rstd = f32({rows}, x);
+        check(api.ln_fwd(xc.data_ptr(), cptr(rc), gamma.data_ptr(), beta.data_ptr(), y.data_ptr(), mptr(z),
+                         mptr<float>(mean), mptr<float>(rstd), rows, H, static_cast<float>(eps), static_cast<float>(p), seed,
+                         offset, dt_code(x), cur_stream()),
+              "rb_ln_fwd");
+        if (!z.defined()) z = xc;
+    }
+    if (req) {
+        auto n = new_node<LnNode>();
+        n->set_next_edges(torch::autograd::collect_next_edges(x, res, gamma, beta));
+        n->z = SavedVariable(z, false);
+        n->gamma = SavedVariable(gamma, false);
+        n->mean = SavedVariable(mean, false);
+        n->rstd = SavedVariable(rstd, false);
+        n->g_ref = gamma;
+        n->b_ref = beta;
+        n->g_mg = opt(g_mg);
+        n->b_mg = opt(b_mg);
+        n->p = p;
+        n->seed = seed;
+        n->offset = offset;
+        torch::autograd::set_history(y, n);
+    }
+    return y;
+}
+
+// ------------------------------------------------------------------------------------------------ embedding
+struct EmbeddingNode : Node {
+    SavedVariable ids;
+    Tensor weight, w_mg;
+    int64_t padding = -1;
+    RB_NODE("RbEmbeddingBackward")
+    void release_variables() override { ids.reset_data(); }
+    variable_list run(variable_list&& grads) {
+        const Tensor I = ids.unpack();
+        const Tensor dy = dense(grads[0]);
+        Tensor acc = w_mg.defined() ? w_mg : at::zeros(weight.sizes(), weight.options().dtype(at::kFloat).requires_grad(false));
+        check(api.embed_bwd(static_cast<const long long*>(I.data_ptr()), dy.data_ptr(), mptr<float>(acc),
+                            static_cast<int>(I.numel()), static_cast<int>(dy.size(-1)), weight.size(0), padding, dt_code(dy),
+                            cur_stream()),
+              "rb_embed_bwd");
+        if (w_mg.defined()) {
+            notify({{&weight, &w_mg}});
+            return {Tensor()};
+        }
+        return {acc.to(weight.scalar_type())};
+    }
+};
+
+Tensor embedding(const Tensor& w, const Tensor& ids, int64_t padding, const OptTensor& w_mg) {
+    const bool req = wants_grad({&w});
+    Tensor out, idc;
+    {
+        at::NoGradGuard off;
+        idc = dense(ids);
+        auto sizes = ids.sizes().vec();
+        sizes.push_back(w.size(1));
+        out = at::empty(sizes, w.options().requires_grad(false));
+        check(api.embed_fwd(static_cast<const long long*>(idc.data_ptr()), w.data_ptr(), out.data_ptr(),
+                            static_cast<int>(ids.numel()), static_cast<int>(w.size(1)), w.size(0), dt_code(w), cur_stream()),
+              "rb_embed_fwd");
+    }
+    if (req) {
+        auto n = new_node<EmbeddingNode>();
+        n->set_next_edges(torch::autograd::collect_next_edges(w));
+        n->ids = SavedVariable(idc, false);
+        n->weight = w;
+        n->w_mg = opt(w_mg);
+        n->padding = padding;
+        torch::autograd::set_history(out, n);
+    }
+    return out;
+}
+
+// ------------------------------------------------------------------------------------------------ cross entropy
+struct XentNode : Node {
+    SavedVariable logits, labels, lse, acc;
+    int64_t V = 0, ignore = 0;
+    double weight = 1;
+    RB_NODE("RbCrossEntropyBackward")
+    void release_variables() override {
+        for (SavedVariable* s : {&logits, &labels, &lse, &acc}) s->reset_data();
+    }
+    variable_list run(variable_list&& grads) {
+        const Tensor L = logits.unpack(), lab = labels.unpack(), ls = lse.unpack(), ac = acc.unpack();
+        const Tensor g = grads[0].to(at::kFloat).contiguous();
+        // the logits are dead after the loss: their buffer receives the gradient
+        Tensor d = L.detach();
+        check(api.xent_bwd(L.data_ptr(), static_cast<const long long*>(lab.data_ptr()), mptr<float>(ls), mptr<float>(ac),
+                           mptr<float>(g), d.data_ptr(), static_cast<int>(L.size(0)), static_cast<int>(V), L.stride(0),
+                           ignore, static_cast<float>(weight), dt_code(L), cur_stream()),
+              "rb_xent_bwd");
+        return {d};
+    }
+};
+
+Tensor cross_entropy(const Tensor& logits, const Tensor& labels, int64_t V, int64_t ignore, double weight) {
+    const bool req = wants_grad({&logits});
+    Tensor lse, acc, loss;
+    {
+        at::NoGradGuard off;
+        lse = f32({logits.size(0)}, logits);
+        acc = at::zeros({2}, lse.options());
+        loss = at::empty({}, lse.options());
+        check(api.xent_fwd(logits.data_ptr(), static_cast<const long long*>(labels.data_ptr()), mptr<float>(lse),
+                           mptr<float>(acc), mptr<float>(loss), static_cast<int>(logits.size(0)), static_cast<int>(V),
+                           logits.stride(0), ignore, static_cast<float>(weight), dt_code(logits), cur_stream()),
+              "rb_xent_fwd", 2);
+    }
+    if (req) {
+        auto n = new_node<XentNode>();
+        n->set_next_edges(torch::autograd::collect_next_edges(logits));
+        n->logits = SavedVariable(logits, false);
+        n->labels = SavedVariable(labels, false);
+        n->lse = SavedVariable(lse, false);
+        n->acc = SavedVariable(acc, false);
+        n->V = V;
+        n->ignore = ignore;
+        n->weight = weight;
+        torch::autograd::set_history(loss, n);
+    }
+    return loss;
+}
+
+// ------------------------------------------------------------------------------------------------ QKV + attention
+// Three tensors that lie back to back in one storage, in this order, seen as one (what the parameter storage does
+// with the projections of a block): the address they start at, or null.
+const void* adjacent(const Tensor* t) {
+    const char* p = static_cast<const char*>(t[0].data_ptr());
+    const char* next = p;
+    for (int i = 0; i < 3; ++i) {
+        if (!t[i].defined() || !t[i].is_contiguous() || t[i].scalar_type() != t[0].scalar_type() ||
+            t[i].sizes().slice(1) != t[0].sizes().slice(1) || !t[i].storage().is_alias_of(t[0].storage()) ||
+            static_cast<const char*>(t[i].data_ptr()) != next)
+            return nullptr;
+        next += t[i].nbytes();
+    }
+    return p;
+}
+Mat stacked(const Tensor* w, const Tensor& cat) {   // the three projection weights as one [3 Ho, hid] matrix
+    if (const void* p = adjacent(w)) {
+        if (aligned16(p) && w[0].size(1) % 8 == 0) {
+            Mat m;
+            m.keep = w[0];
+            m.p = p;
+            m.rows = 3 * w[0].size(0);
+            m.cols = m.ld = w[0].size(1);
+            return m;
+        }
+    }
+    return mat(cat.defined() ? cat : at::cat({w[0].detach(), w[1].detach(), w[2].detach()}, 0));
+}
+void attn_args(RbAttnArgs& a, const Tensor& qkv, const Tensor& o, const Tensor& lse, const Tensor& bias, int64_t B, int64_t S,
+               int64_t H, double scale, double p, uint64_t seed, uint64_t offset) {
+    memset(&a, 0, sizeof(a));
+    const char* base = static_cast<const char*>(qkv.data_ptr());
+    const int64_t Ho = H * 64;
+    a.Q = base;
+    a.K = base + Ho * 2;
+    a.V = base + 2 * Ho * 2;
+    a.q_sb = a.k_sb = a.v_sb = S * 3 * Ho;
+    a.q_ss = a.k_ss = a.v_ss = 3 * Ho;
+    a.q_sh = a.k_sh = a.v_sh = 64;
+    a.O = o.data_ptr();
+    a.o_sb = S * Ho;
+    a.o_ss = Ho;
+    a.o_sh = 64;
+    a.lse = mptr<float>(lse);
+    a.key_bias = mptr<float>(bias);
+    a.B = static_cast<int32_t>(B);
+    a.S = static_cast<int32_t>(S);
+    a.H = static_cast<int32_t>(H);
+    a.D = 64;
+    a.dtype = dt_code(qkv);
+    a.scale = static_cast<float>(scale);
+    a.p_drop = static_cast<float>(p);
+    a.seed = seed;
+    a.offset = offset;
+}
+struct QkvNode : Node {
+    SavedVariable x, qkv, o, lse, bias;
+    Tensor w[3], b[3], w_mg[3], b_mg[3], cat;
+    int64_t B = 0, S = 0, H = 0;
+    double p = 0, scale = 1;
+    uint64_t seed = 0, offset = 0;
+    RB_NODE("RbQkvAttentionBackward")
+    void release_variables() override {
+        for (SavedVariable* s : {&x, &qkv, &o, &lse, &bias}) s->reset_data();
+    }
+    variable_list run(variable_list&& grads) {
+        const Tensor X = x.unpack(), Q = qkv.unpack(), O = o.unpack(shared_from_this()), L = lse.unpack(), kb = bias.unpack();
+        const Tensor dO = dense(grads[0]);
+        const int dt = dt_code(X);
+        const int64_t Ho = H * 64;
+        Tensor dqkv = at::empty(Q.sizes(), Q.options());
+        Tensor delta = f32({B, H, S}, Q), dq_acc = f32({B, S, H, 64}, Q);
+        RbAttnArgs a;
+        attn_args(a, Q, O, L, kb, B, S, H, scale, p, seed, offset);
+        Tensor dOa = aligned16(dO.data_ptr()) ? dO : dO.clone();
+        a.dO = dOa.data_ptr();
+        a.do_sb = S * Ho;
+        a.do_ss = Ho;
+        a.do_sh = 64;
+        char* d = static_cast<char*>(dqkv.data_ptr());
+        a.dQ = d;
+        a.dK = d + Ho * 2;
+        a.dV = d + 2 * Ho * 2;
+        a.dq_sb = a.dk_sb = a.dv_sb = S * 3 * Ho;
+        a.dq_ss = a.dk_ss = a.dv_ss = 3 * Ho;
+        a.dq_sh = a.dk_sh = a.dv_sh = 64;
+        a.delta = mptr<float>(delta);
+        a.dq_accum = mptr<float>(dq_acc);
+        check(api.attn_bwd(&a, cur_stream()), "rb_attn_bwd", 3);
+        Mat dm;
+        dm.keep = dqkv;
+        dm.p = d;
+        dm.rows = B * S;
+        dm.cols = dm.ld = 3 * Ho;
+        const Mat xm = rows_of(X);
+        Tensor dx, dw[3], db[3];
+        if (task_should_compute_output(0)) {
+            dx = at::empty(X.sizes(), X.options());
+            gemm(dm, stacked(w, cat), false, false, dx.data_ptr(), false, dt, Epi());
+        }
+        // adjacent fp32 gradient buffers: one weight-gradient GEMM and one column sum serve all three projections
+        const bool all_w = w_mg[0].defined() && w_mg[1].defined() && w_mg[2].defined();
+        const void* wm = all_w ? adjacent(w_mg) : nullptr;
+        if (wm) {
+            Epi e;
+            e.accumulate = true;
+            gemm(dm, xm, true, false, const_cast<void*>(wm), true, dt, e);
+        } else {
+            for (int i = 0; i < 3; ++i) dw[i] = weight_grad(columns(dm, i * Ho, Ho), xm, w[i], w_mg[i], dt);
+        }
+        if (b[0].defined()) {
+            const bool all_b = b_mg[0].defined() && b_mg[1].defined() && b_mg[2].defined();
+            const void* bm = all_b ? adjacent(b_mg) : nullptr;
+            if (bm) {
+                check(api.colsum(dm.p, static_cast<float*>(const_cast<void*>(bm)), static_cast<int>(dm.rows),
+                                 static_cast<int>(dm.cols), dm.ld, dt, cur_stream()),
+                      "rb_colsum");
+            } else {
+                for (int i = 0; i < 3; ++i) db[i] = bias_grad(columns(dm, i * Ho, Ho), b[i], b_mg[i], dt);
+            }
+        }
+        notify({{&w[0], &w_mg[0]}, {&w[1], &w_mg[1]}, {&w[2], &w_mg[2]},
+                {&b[0], &b_mg[0]}, {&b[1], &b_mg[1]}, {&b[2], &b_mg[2]}});
+        return {dx, dw[0], db[0], dw[1], db[1], dw[2], db[2]};
+    }
+};
+
+// cat_w / cat_b: the stacked projections when they are not adjacent in memory and the caller keeps such a stack (of
+// parameters that come and go it keeps none: they are stacked anew for every use)
+Tensor qkv_attention(const Tensor& x, const std::vector<Tensor>& ws, const std::vector<OptTensor>& bs, const OptTensor& key_bias,
+                     double p, double scale, int64_t H, uint64_t seed, uint64_t offset, const std::vector<OptTensor>& w_mgs,
+                     const std::vector<OptTensor>& b_mgs, const OptTensor& cat_w, const OptTensor& cat_b) {
+    const Tensor w[3] = {ws[0], ws[1], ws[2]}, b[3] = {opt(bs[0]), opt(bs[1]), opt(bs[2])};
+    const bool req = wants_grad({&x, &w[0], &b[0], &w[1], &b[1], &w[2], &b[2]});
+    const int64_t B = x.size(0), S = x.size(1), Ho = w[0].size(0);
+    Tensor xc, qkv, o, lse, bias_cat, kb = opt(key_bias), cat = opt(cat_w);
+    {
+        at::NoGradGuard off;
+        xc = dense(x);
+        qkv = at::empty({B, S, 3 * Ho}, x.options());
+        o = at::empty({B, S, Ho}, x.options());
+        lse = f32({B, H, S}, x);
+        Epi e;
+        if (b[0].defined()) {
+            e.bias = adjacent(b);
+            if (!e.bias) {
+                bias_cat = cat_b.has_value() ? *cat_b : at::cat({b[0].detach(), b[1].detach(), b[2].detach()}, 0);
+                e.bias = bias_cat.data_ptr();
+            }
+        }
+        gemm(rows_of(xc), stacked(w, cat), false, true, qkv.data_ptr(), false, dt_code(x), e);
+        RbAttnArgs a;
+        attn_args(a, qkv, o, lse, kb, B, S, H, scale, p, seed, offset);
+        check(api.attn_fwd(&a, cur_stream()), "rb_attn_fwd");
+    }
+    if (req) {
+        auto n = new_node<QkvNode>();
+        n->set_next_edges(torch::autograd::collect_next_edges(x, w[0], b[0], w[1], b[1], w[2], b[2]));
+        torch::autograd::set_history(o, n);
+        n->x = SavedVariable(xc, false);
+        n->qkv = SavedVariable(qkv, false);
+        n->o = SavedVariable(o, true);
+        n->lse = SavedVariable(lse, false);
+        n->bias = SavedVariable(kb, false);
+        for (int i = 0; i < 3; ++i) {
+            n->w[i] = w[i];
+            n->b[i] = b[i];
+            n->w_mg[i] = opt(w_mgs[i]);
+            n->b_mg[i] = opt(b_mgs[i]);
+        }
+        n->cat = cat;
+        n->B = B;
+        n->S = S;
+        n->H = H;
+        n->p = p;
+        n->scale = scale;
+        n->seed = seed;
+        n->offset = offset;
+    }
+    return o;
+}
+// whether the three lie back to back in one storage
+bool are_adjacent(const std::vector<Tensor>& t) { return t.size() == 3 && adjacent(t.data()) != nullptr; }
+
+// ------------------------------------------------------------------------------------------------ batch norm
+Tensor nhwc(const Tensor& t) { return t.contiguous(at::MemoryFormat::ChannelsLast); }
+struct BnNode : Node {
+    SavedVariable x, y, mean, rstd, g32;
+    Tensor gamma, beta, g_mg, b_mg;
+    bool relu = false, has_res = false;
+    RB_NODE("RbBatchNormBackward")
+    void release_variables() override {
+        for (SavedVariable* s : {&x, &y, &mean, &rstd, &g32}) s->reset_data();
+    }
+    variable_list run(variable_list&& grads) {
+        const Tensor X = x.unpack(), Y = y.unpack(shared_from_this()), M = mean.unpack(), R = rstd.unpack(), G = g32.unpack();
+        const Tensor dy = nhwc(grads[0]);
+        const int64_t C = X.size(1);
+        Tensor dx = at::empty_like(X), dres = has_res ? at::empty_like(X) : Tensor();
+        Tensor part = f32({2, C}, X);
+        // fp32 gradient buffers take the sums inside the kernel
+        auto acc = [](const Tensor& mg) {
+            return mg.defined() && mg.scalar_type() == at::kFloat && mg.is_contiguous() ? mptr<float>(mg) : nullptr;
+        };
+        float *ga = acc(g_mg), *ba = acc(b_mg);
+        check(api.bn_bwd(X.data_ptr(), dy.data_ptr(), Y.data_ptr(), mptr<float>(M), mptr<float>(R), mptr<float>(G),
+                         mptr<float>(part), ga, ba, dx.data_ptr(), mptr(dres), X.numel() / C, static_cast<int>(C), relu ? 1 : 0,
+                         dt_code(X), cur_stream()),
+              "rb_bn_bwd", 2);
+        Tensor dg, db;
+        if (g_mg.defined()) {
+            if (!ga) g_mg.add_(part[1]);
+        } else {
+            dg = part[1].to(gamma.scalar_type());
+        }
+        if (b_mg.defined()) {
+            if (!ba) b_mg.add_(part[0]);
+        } else {
+            db = part[0].to(beta.scalar_type());
+        }
+        notify({{&gamma, &g_mg}, {&beta, &b_mg}});
+        return {dx, dres, dg, db};
+    }
+};
+
+Tensor batch_norm_act(const Tensor& x, const OptTensor& res_, const Tensor& gamma, const Tensor& beta,
+                      const OptTensor& run_mean_, const OptTensor& run_var_, double momentum, double eps, bool relu,
+                      const OptTensor& g_mg, const OptTensor& b_mg) {
+    const Tensor res = opt(res_), run_mean = opt(run_mean_), run_var = opt(run_var_);
+    const bool req = wants_grad({&x, &res, &gamma, &beta});
+    Tensor xc, y, mean, rstd, g32;
+    {
+        at::NoGradGuard off;
+        const int64_t C = x.size(1), R = x.numel() / C;
+        xc = nhwc(x);
+        const Tensor rc = res.defined() ? nhwc(res) : Tensor();
+        g32 = gamma.detach().to(at::kFloat);
+        const Tensor b32 = beta.detach().to(at::kFloat);
+        const bool in_kernel = run_mean.defined() && run_mean.scalar_type() == at::kFloat;
+        y = at::empty_like(xc);
+        Tensor part = f32({2, C}, x);
+        mean = f32({C}, x);
+        rstd = f32({C}, x);
+        check(api.bn_fwd(xc.data_ptr(), cptr(rc), mptr<float>(g32), mptr<float>(b32), y.data_ptr(), mptr<float>(part),
+                         mptr<float>(mean), mptr<float>(rstd), in_kernel ? mptr<float>(run_mean) : nullptr,
+                         in_kernel ? mptr<float>(run_var) : nullptr, R, static_cast<int>(C), static_cast<float>(eps),
+                         static_cast<float>(momentum), relu ? 1 : 0, dt_code(x), cur_stream()),
+              "rb_bn_fwd", 2);
+        if (run_mean.defined() && !in_kernel) {
+            // statistics kept in a 16-bit buffer: update them with a few tiny element-wise operations
+            const Tensor var = (1.0 / (rstd * rstd) - eps) * (static_cast<double>(R) / std::max<int64_t>(R - 1, 1));
+            run_mean.mul_(1 - momentum).add_((momentum * mean).to(run_mean.scalar_type()));
+            run_var.mul_(1 - momentum).add_((momentum * var).to(run_var.scalar_type()));
+        }
+    }
+    if (req) {
+        auto n = new_node<BnNode>();
+        n->set_next_edges(torch::autograd::collect_next_edges(x, res, gamma, beta));
+        torch::autograd::set_history(y, n);
+        n->x = SavedVariable(xc, false);
+        n->y = SavedVariable(y, true);
+        n->mean = SavedVariable(mean, false);
+        n->rstd = SavedVariable(rstd, false);
+        n->g32 = SavedVariable(g32, false);
+        n->gamma = gamma;
+        n->beta = beta;
+        n->g_mg = opt(g_mg);
+        n->b_mg = opt(b_mg);
+        n->relu = relu;
+        n->has_res = res.defined();
+    }
+    return y;
+}
+
+// ------------------------------------------------------------------------------------------------ plain products
+// out = epilogue(alpha op(a) op(b)) for 2-D operands
+Tensor product(const Tensor& a, const Tensor& b, bool trans_a, bool trans_b, const OptTensor& bias, const OptTensor& residual,
+               const OptTensor& aux_in, const OptTensor& aux_out, bool gelu, bool dgelu, const OptTensor& out_, bool accumulate,
+               bool fp32_out, double alpha, int64_t max_ctas) {
+    at::NoGradGuard off;
+    const Mat A = mat(a), B = mat(b);
+    RbGemmArgs g;
+    memset(&g, 0, sizeof(g));
+    g.M = trans_a ? A.cols : A.rows;
+    g.K = trans_a ? A.rows : A.cols;
+    g.N = trans_b ? B.rows : B.cols;
+    const int64_t kb = trans_b ? B.cols : B.rows;
+    TORCH_CHECK_VALUE(kb == g.K, "gemm: inner dimensions differ (", g.K, " vs ", kb, ")");
+    Tensor out = out_.has_value() ? *out_ : at::empty({g.M, g.N}, fp32_out ? a.options().dtype(at::kFloat) : a.options());
+    g.A = A.p;
+    g.B = B.p;
+    g.D = out.data_ptr();
+    g.bias = cptr(opt(bias));
+    g.residual = cptr(opt(residual));
+    g.aux_in = cptr(opt(aux_in));
+    g.aux_out = mptr(opt(aux_out));
+    g.batch = 1;
+    g.lda = A.ld;
+    g.ldb = B.ld;
+    g.ldd = out.stride(-2);
+    g.a_major = trans_a ? 1 : 0;
+    g.b_major = trans_b ? 0 : 1;
+    g.in_dtype = dt_code(a);
+    g.out_dtype = fp32_out ? 1 : 0;
+    g.flags = (g.bias ? RB_GEMM_BIAS : 0) | (gelu ? RB_GEMM_GELU : 0) | (dgelu ? RB_GEMM_DGELU : 0) |
+              (g.residual ? RB_GEMM_RESIDUAL : 0) | (accumulate ? RB_GEMM_ACCUM : 0) | (g.aux_out ? RB_GEMM_AUX_OUT : 0);
+    g.alpha = static_cast<float>(alpha);
+    g.max_ctas = static_cast<int32_t>(max_ctas);
+    check(api.gemm(&g, cur_stream()), "rb_gemm");
+    return out;
+}
+
+// ------------------------------------------------------------------------------------------------ bindings
+void init(const std::unordered_map<std::string, uintptr_t>& fns, py::object error) {
+    auto set = [&](auto& slot, const char* name) {
+        slot = reinterpret_cast<std::remove_reference_t<decltype(slot)>>(fns.at(name));
+    };
+    set(api.gemm, "rb_gemm");
+    set(api.gelu, "rb_gelu");
+    set(api.colsum, "rb_colsum");
+    set(api.ln_fwd, "rb_ln_fwd");
+    set(api.ln_bwd, "rb_ln_bwd");
+    set(api.ln_bwd_grid, "rb_ln_bwd_grid");
+    set(api.embed_fwd, "rb_embed_fwd");
+    set(api.embed_bwd, "rb_embed_bwd");
+    set(api.xent_fwd, "rb_xent_fwd");
+    set(api.xent_bwd, "rb_xent_bwd");
+    set(api.attn_fwd, "rb_attn_fwd");
+    set(api.attn_bwd, "rb_attn_bwd");
+    set(api.bn_fwd, "rb_bn_fwd");
+    set(api.bn_bwd, "rb_bn_bwd");
+    error_class = error.release().ptr();
+}
+void set_listener(py::object fn) {
+    Py_XDECREF(listener);
+    listener = fn.is_none() ? nullptr : fn.release().ptr();
+    has_listener.store(listener != nullptr, std::memory_order_release);
+}
+
+// Errors cross the boundary as the exceptions they are (the library's own error class, ValueError, TypeError, ...).
+template <typename F>
+struct Guarded;
+template <typename R, typename... A>
+struct Guarded<R (*)(A...)> {
+    template <R (*F)(A...)>
+    static R call(A... a) {
+        R result{};
+        auto body = [&]() -> bool {
+            HANDLE_TH_ERRORS
+            result = F(std::forward<A>(a)...);
+            return true;
+            END_HANDLE_TH_ERRORS_RET(false)
+        };
+        if (!body()) throw py::error_already_set();
+        return result;
+    }
+};
+#define RB_DEF(NAME) m.def(#NAME, &Guarded<decltype(&NAME)>::call<&NAME>)
+
+}  // namespace
+
+PYBIND11_MODULE(_host, m) {
+    m.doc() = "Host side of the fused operators";
+    m.def("init", &init);
+    m.def("set_listener", &set_listener);
+    m.def("launch_count", [] { return launches.load(std::memory_order_relaxed); });
+    RB_DEF(product);
+    RB_DEF(linear);
+    RB_DEF(mlp);
+    RB_DEF(layer_norm);
+    RB_DEF(embedding);
+    RB_DEF(cross_entropy);
+    RB_DEF(qkv_attention);
+    RB_DEF(are_adjacent);
+    RB_DEF(batch_norm_act);
+}

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import threading
+from ctypes import c_void_p
 from pathlib import Path
 
 import torch
@@ -48,7 +49,7 @@ class _Counting:
 
 def launch_count() -> int:
     """Kernels of this library launched so far in this process."""
-    return _launches
+    return _launches + (_host.launch_count() if _host is not None else 0)
 
 
 class KernelLibraryError(RuntimeError):
@@ -80,6 +81,42 @@ def lib() -> ctypes.CDLL:
         _lib.rb_read_error.restype = ctypes.c_int
         _lib = _Counting(_lib)
         return _lib
+
+
+_host = None
+_HOST_ENTRIES = ("rb_gemm", "rb_gelu", "rb_colsum", "rb_ln_fwd", "rb_ln_bwd", "rb_ln_bwd_grid", "rb_embed_fwd",
+                 "rb_embed_bwd", "rb_xent_fwd", "rb_xent_bwd", "rb_attn_fwd", "rb_attn_bwd", "rb_bn_fwd", "rb_bn_bwd")
+
+
+def host_loaded() -> bool:
+    return _host is not None
+
+
+def host():
+    """The operators' native host side (``_host.so``), given the entry points of the kernel library in use.  Built
+    on first use like the kernels; an error, not a fallback, when that is impossible."""
+    global _host
+    if _host is not None:
+        return _host
+    kernels = lib()
+    with _lock:
+        if _host is not None:
+            return _host
+        import importlib
+
+        try:
+            mod = importlib.import_module("rannc_b200._host")
+        except ImportError:
+            from .. import build
+
+            try:
+                build.build_host()
+                mod = importlib.import_module("rannc_b200._host")
+            except Exception as e:  # noqa: BLE001
+                raise KernelLibraryError(f"cannot build the operators' host side: {e}") from e
+        mod.init({n: ctypes.cast(getattr(kernels, n).raw, c_void_p).value for n in _HOST_ENTRIES}, KernelLibraryError)
+        _host = mod
+        return _host
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)

@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import torch
 
+from . import _lib
 from . import kernels as K
 from ..utils.config import conf
 from .gemm import gemm
@@ -53,7 +54,7 @@ def manual_seed(seed: int) -> None:
 
 
 def _main_grad(p):
-    return getattr(p, "main_grad", None)
+    return None if p is None else getattr(p, "main_grad", None)
 
 
 # ----------------------------------------------------------------------------- gradient reports
@@ -68,15 +69,13 @@ _grad_listener = None
 def set_grad_listener(fn) -> None:
     global _grad_listener
     _grad_listener = fn
+    if fn is not None or _lib.host_loaded():
+        _lib.host().set_listener(fn)
 
 
 def notify_grads(*params) -> None:
     if _grad_listener is not None:
         _grad_listener([p for p in params if p is not None])
-
-
-def _2d(x):
-    return x.reshape(-1, x.shape[-1])
 
 
 def _kernel_ok(x) -> bool:
@@ -85,14 +84,6 @@ def _kernel_ok(x) -> bool:
 
 def _aligned(t) -> bool:
     return t.data_ptr() % 16 == 0 and t.shape[-1] % 8 == 0
-
-
-def _wgrad(dy2, x2, weight, mg):
-    """dW = dy2^T @ x2, into the fp32 main-grad buffer when there is one."""
-    if mg is not None:
-        gemm(dy2, x2, trans_a=True, trans_b=False, out=mg, accumulate=True)
-        return None
-    return gemm(dy2, x2, trans_a=True, trans_b=False)
 
 
 def _bgrad(dy2, bias, mg):
@@ -104,127 +95,30 @@ def _bgrad(dy2, bias, mg):
     return K.colsum(dy2).to(bias.dtype)
 
 
+def _host():
+    """The native operators; like any autograd function without a batching rule they refuse functorch transforms."""
+    if torch._C._are_functorch_transforms_active():
+        raise RuntimeError("the fused operators do not support functorch transforms (vmap, grad, jvp, ...)")
+    return _lib.host()
+
+
 # ----------------------------------------------------------------------------- linear
-class _Linear(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, bias, act):
-        x2 = _2d(x)
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
-        pre = None
-        if act == "gelu":
-            pre = torch.empty(x2.shape[0], weight.shape[0], dtype=x.dtype, device=x.device)
-            y = gemm(x2, weight, bias=bias, gelu=True, aux_out=pre)
-        else:
-            y = gemm(x2, weight, bias=bias)
-        ctx.save_for_backward(x2, weight, pre)
-        ctx.has_bias = bias is not None
-        ctx.bias_ref = bias
-        ctx.w_mg = _main_grad(weight)
-        ctx.b_mg = _main_grad(bias) if bias is not None else None
-        ctx.x_shape = x.shape
-        ctx.act = act
-        return y.view(*x.shape[:-1], weight.shape[0])
-
-    @staticmethod
-    def backward(ctx, dy):
-        x2, weight, pre = ctx.saved_tensors
-        dy2 = _2d(dy)
-        if not dy2.is_contiguous():
-            dy2 = dy2.contiguous()
-        if ctx.act == "gelu":
-            dy2 = K.gelu_bwd(pre, dy2)
-        dx = None
-        if ctx.needs_input_grad[0]:
-            dx = gemm(dy2, weight, trans_b=False).view(ctx.x_shape)
-        dw = _wgrad(dy2, x2, weight, ctx.w_mg) if ctx.needs_input_grad[1] else None
-        db = _bgrad(dy2, ctx.bias_ref, ctx.b_mg) if (ctx.has_bias and ctx.needs_input_grad[2]) else None
-        notify_grads(weight if ctx.w_mg is not None else None, ctx.bias_ref if ctx.b_mg is not None else None)
-        return dx, dw, db, None
-
-
 def linear(x, weight, bias=None, act=None):
     """``act(x @ weight.T + bias)`` with ``act`` in (None, "gelu")."""
     if not (_kernel_ok(x) and weight.dtype == x.dtype and _aligned(x) and _aligned(weight)):
         y = torch.nn.functional.linear(x, weight, bias)
         return torch.nn.functional.gelu(y) if act == "gelu" else y
-    return _Linear.apply(x, weight, bias, act)
-
-
-class _Mlp(torch.autograd.Function):
-    """y = gelu(x W1^T + b1) W2^T + b2; the GELU derivative rides in the dgrad GEMM epilogue."""
-
-    @staticmethod
-    def forward(ctx, x, w1, b1, w2, b2):
-        x2 = _2d(x)
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
-        pre = torch.empty(x2.shape[0], w1.shape[0], dtype=x.dtype, device=x.device)
-        h = gemm(x2, w1, bias=b1, gelu=True, aux_out=pre)
-        y = gemm(h, w2, bias=b2)
-        ctx.save_for_backward(x2, w1, w2, pre, h)
-        ctx.refs = (b1, b2)
-        ctx.mgs = (_main_grad(w1), _main_grad(b1) if b1 is not None else None, _main_grad(w2),
-                   _main_grad(b2) if b2 is not None else None)
-        ctx.x_shape = x.shape
-        return y.view(*x.shape[:-1], w2.shape[0])
-
-    @staticmethod
-    def backward(ctx, dy):
-        x2, w1, w2, pre, h = ctx.saved_tensors
-        b1, b2 = ctx.refs
-        w1_mg, b1_mg, w2_mg, b2_mg = ctx.mgs
-        dy2 = _2d(dy)
-        if not dy2.is_contiguous():
-            dy2 = dy2.contiguous()
-        dw2 = _wgrad(dy2, h, w2, w2_mg)
-        db2 = _bgrad(dy2, b2, b2_mg)
-        dpre = gemm(dy2, w2, trans_b=False, dgelu=True, aux_in=pre)
-        dw1 = _wgrad(dpre, x2, w1, w1_mg)
-        db1 = _bgrad(dpre, b1, b1_mg)
-        dx = gemm(dpre, w1, trans_b=False).view(ctx.x_shape) if ctx.needs_input_grad[0] else None
-        notify_grads(w1 if w1_mg is not None else None, b1 if b1_mg is not None else None,
-                     w2 if w2_mg is not None else None, b2 if b2_mg is not None else None)
-        return dx, dw1, db1, dw2, db2
+    return _host().linear(x, weight, bias, act == "gelu", _main_grad(weight), _main_grad(bias), None)
 
 
 def mlp(x, w1, b1, w2, b2):
+    """y = gelu(x W1^T + b1) W2^T + b2; the GELU derivative rides in the epilogue of a backward GEMM."""
     if not (_kernel_ok(x) and _aligned(x) and _aligned(w1) and _aligned(w2)):
         return torch.nn.functional.linear(torch.nn.functional.gelu(torch.nn.functional.linear(x, w1, b1)), w2, b2)
-    return _Mlp.apply(x, w1, b1, w2, b2)
+    return _host().mlp(x, w1, b1, w2, b2, _main_grad(w1), _main_grad(b1), _main_grad(w2), _main_grad(b2))
 
 
 # ----------------------------------------------------------------------------- layer norm
-class _DropoutAddLayerNorm(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, residual, gamma, beta, p, eps):
-        seed, offset = rng.next() if p > 0.0 else (0, 0)
-        xc = x if x.is_contiguous() else x.contiguous()
-        rc = None if residual is None else (residual if residual.is_contiguous() else residual.contiguous())
-        y, z, mean, rstd = K.ln_fwd(xc, rc, gamma, beta, eps, p, seed, offset)
-        ctx.save_for_backward(z, gamma, mean, rstd)
-        ctx.p, ctx.seed, ctx.offset = p, seed, offset
-        ctx.has_res = residual is not None
-        ctx.g_ref, ctx.b_ref = gamma, beta
-        ctx.g_mg, ctx.b_mg = _main_grad(gamma), _main_grad(beta)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        z, gamma, mean, rstd = ctx.saved_tensors
-        dyc = dy if dy.is_contiguous() else dy.contiguous()
-        use_mg = ctx.g_mg is not None and ctx.b_mg is not None
-        dz, dx, dg, db = K.ln_bwd(dyc, z, gamma, mean, rstd, ctx.p, ctx.seed, ctx.offset,
-                                  dgamma=ctx.g_mg if use_mg else None, dbeta=ctx.b_mg if use_mg else None,
-                                  accumulate=use_mg)
-        if use_mg:
-            dg = db = None
-            notify_grads(ctx.g_ref, ctx.b_ref)
-        else:
-            dg, db = dg.to(gamma.dtype), db.to(gamma.dtype)
-        return dx, (dz if ctx.has_res else None), dg, db, None, None
-
-
 def dropout_add_layer_norm(x, residual, gamma, beta, p: float = 0.0, eps: float = 1e-5, training: bool = True):
     """``LayerNorm(dropout(x, p) + residual)`` over the last dimension."""
     p = p if training else 0.0
@@ -233,7 +127,10 @@ def dropout_add_layer_norm(x, residual, gamma, beta, p: float = 0.0, eps: float 
         if residual is not None:
             h = h + residual
         return torch.nn.functional.layer_norm(h, (x.shape[-1],), gamma, beta, eps)
-    return _DropoutAddLayerNorm.apply(x, residual, gamma, beta, float(p), float(eps))
+    h = _host()
+    seed, offset = rng.next() if p > 0.0 else (0, 0)
+    return h.layer_norm(x, residual, gamma, beta, float(p), float(eps), seed, offset, _main_grad(gamma),
+                        _main_grad(beta))
 
 
 # ----------------------------------------------------------------------------- element-wise
@@ -276,33 +173,10 @@ def gelu(x):
     return _Gelu.apply(x)
 
 
-class _Embedding(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, weight, ids, padding_idx):
-        idc = ids if ids.is_contiguous() else ids.contiguous()
-        ctx.save_for_backward(idc)
-        ctx.w_ref = weight
-        ctx.w_mg = _main_grad(weight)
-        ctx.padding_idx = padding_idx
-        return K.embed_fwd(idc, weight)
-
-    @staticmethod
-    def backward(ctx, dy):
-        (ids,) = ctx.saved_tensors
-        dyc = dy if dy.is_contiguous() else dy.contiguous()
-        if ctx.w_mg is not None:
-            K.embed_bwd(ids, dyc, ctx.w_mg, ctx.padding_idx)
-            notify_grads(ctx.w_ref)
-            return None, None, None
-        acc = torch.zeros(ctx.w_ref.shape, dtype=torch.float32, device=dy.device)
-        K.embed_bwd(ids, dyc, acc, ctx.padding_idx)
-        return acc.to(ctx.w_ref.dtype), None, None
-
-
 def embedding(weight, ids, padding_idx: int = -1):
     if not (_kernel_ok(weight) and weight.shape[1] % 8 == 0 and ids.dtype == torch.int64):
         return torch.nn.functional.embedding(ids, weight, None if padding_idx < 0 else padding_idx)
-    return _Embedding.apply(weight, ids, padding_idx)
+    return _host().embedding(weight, ids, padding_idx, _main_grad(weight))
 
 
 # ----------------------------------------------------------------------------- attention
@@ -358,23 +232,6 @@ def sdpa(q, k, v, attn_mask=None, dropout_p: float = 0.0, is_causal: bool = Fals
 
 
 # ----------------------------------------------------------------------------- loss
-class _SoftmaxXent(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, logits2d, labels, V, ignore_index, weight):
-        loss, lse, acc = K.xent_fwd(logits2d, labels, V, ignore_index, weight)
-        ctx.save_for_backward(logits2d, labels, lse, acc)
-        ctx.V, ctx.ignore_index, ctx.weight = V, ignore_index, weight
-        return loss
-
-    @staticmethod
-    def backward(ctx, gout):
-        logits2d, labels, lse, acc = ctx.saved_tensors
-        g = gout.float().contiguous()
-        # the logits are dead after the loss: their buffer receives the gradient
-        d = K.xent_bwd(logits2d, labels, lse, acc, g, ctx.V, ctx.ignore_index, ctx.weight, inplace=True)
-        return d, None, None, None, None
-
-
 def cross_entropy(logits, labels, num_classes=None, ignore_index: int = -100, weight: float = 1.0):
     """Mean cross entropy over rows whose label is not ``ignore_index``.
 
@@ -385,7 +242,8 @@ def cross_entropy(logits, labels, num_classes=None, ignore_index: int = -100, we
     l2 = logits.reshape(-1, ld)
     if not (_kernel_ok(l2) and l2.stride(1) == 1):
         return torch.nn.functional.cross_entropy(l2[:, :V].float(), labels.reshape(-1), ignore_index=ignore_index) * weight
-    return _SoftmaxXent.apply(l2, labels.reshape(-1).contiguous(), V, ignore_index, float(weight))
+    # the logits are dead after the loss: backward writes the gradient over them
+    return _host().cross_entropy(l2, labels.reshape(-1).contiguous(), V, ignore_index, float(weight))
 
 
 # ----------------------------------------------------------------------------- fused QKV projection + attention
@@ -412,117 +270,6 @@ def _cat_params(tensors):
     return cat
 
 
-_adj_cache = {}
-
-
-def _adjacent_view(tensors):
-    """One [sum of rows, ...] view over tensors that lie back to back in ONE storage (the parameter storage
-    lays the three projection weights of a QKV block out that way), or None when they do not.  Tensors that
-    merely have consecutive addresses in different allocations do not qualify: the view must stay inside the
-    first tensor's storage."""
-    t0 = tensors[0]
-    # windows of streamed parameters / gradients come and go: their views are made afresh and never cached
-    volatile = any(getattr(t, "_rannc_host", None) is not None or getattr(t, "_rannc_window", False)
-                   for t in tensors)
-    key = tuple(t.data_ptr() for t in tensors)
-    if not volatile:
-        hit = _adj_cache.get(key)
-        if hit is not None:
-            return hit[0]
-    es = t0.element_size()
-    ok = all(t.is_contiguous() and t.dtype == t0.dtype and t.shape[1:] == t0.shape[1:] for t in tensors)
-    ptr = t0.data_ptr()
-    total = 0
-    for t in tensors:
-        ok = ok and t.data_ptr() == ptr
-        ptr += t.numel() * es
-        total += t.numel()
-    view = None
-    if ok:
-        try:
-            st = t0.detach().untyped_storage()
-            inside = st.nbytes() >= (t0.storage_offset() + total) * es and \
-                all(t.untyped_storage().data_ptr() == st.data_ptr() for t in tensors)
-            if inside:
-                rows = sum(t.shape[0] for t in tensors)
-                shape = (rows,) + tuple(t0.shape[1:])
-                view = torch.empty(0, dtype=t0.dtype, device=t0.device).set_(st, t0.storage_offset(), shape,
-                                                                             t0.stride())
-        except Exception:  # noqa: BLE001
-            view = None
-    if volatile:
-        return view
-    if len(_adj_cache) > 4096:
-        _adj_cache.clear()
-    _adj_cache[key] = (view, tensors)   # the tensors stay referenced so their addresses are not reused
-    return view
-
-
-class _QkvAttention(torch.autograd.Function):
-    """softmax((x Wq^T)(x Wk^T)^T) (x Wv^T) with ONE projection GEMM over the concatenated weights; the
-    attention kernels read q / k / v as strided views of its [B, S, 3, H, D] output and write dq / dk / dv
-    into one buffer that the single dgrad GEMM consumes."""
-
-    @staticmethod
-    def forward(ctx, x, wq, bq, wk, bk, wv, bv, key_bias, p, scale, H):
-        B, S, hid = x.shape
-        x2 = x.reshape(B * S, hid)
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
-        wcat = _adjacent_view((wq, wk, wv))
-        if wcat is None:
-            wcat = _cat_params((wq, wk, wv))
-        bcat = None
-        if bq is not None:
-            bcat = _adjacent_view((bq, bk, bv))
-            if bcat is None:
-                bcat = _cat_params((bq, bk, bv))
-        Ho = wq.shape[0]
-        D = Ho // H
-        qkv = gemm(x2, wcat, bias=bcat).view(B, S, 3, H, D)
-        seed, offset = rng.next() if p > 0.0 else (0, 0)
-        o, lse = K.attn_fwd(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], key_bias, scale, p, seed, offset)
-        ctx.save_for_backward(x2, qkv, o, lse, key_bias)
-        ctx.ws = (wq, wk, wv)
-        ctx.bs = (bq, bk, bv)
-        ctx.mgs = tuple(_main_grad(t) if t is not None else None for t in (wq, wk, wv, bq, bk, bv))
-        ctx.p, ctx.seed, ctx.offset, ctx.scale = p, seed, offset, scale
-        ctx.dims = (B, S, hid, H, D)
-        return o.view(B, S, Ho)
-
-    @staticmethod
-    def backward(ctx, do):
-        x2, qkv, o, lse, key_bias = ctx.saved_tensors
-        B, S, hid, H, D = ctx.dims
-        Ho = H * D
-        do4 = do.reshape(B, S, H, D)
-        dqkv = torch.empty(B, S, 3, H, D, dtype=qkv.dtype, device=qkv.device)
-        K.attn_bwd(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], o, lse, do4, key_bias, ctx.scale, ctx.p, ctx.seed,
-                   ctx.offset, dq=dqkv[:, :, 0], dk=dqkv[:, :, 1], dv=dqkv[:, :, 2])
-        d2 = dqkv.view(B * S, 3 * Ho)
-        wcat = _adjacent_view(ctx.ws)
-        if wcat is None:
-            wcat = _cat_params(ctx.ws)
-        dx = gemm(d2, wcat, trans_b=False).view(B, S, hid) if ctx.needs_input_grad[0] else None
-        grads_w, grads_b = [None] * 3, [None] * 3
-        # adjacent fp32 gradient buffers: one wgrad GEMM and one column sum serve all three projections
-        wmg = _adjacent_view(ctx.mgs[:3]) if all(m is not None for m in ctx.mgs[:3]) else None
-        if wmg is not None:
-            gemm(d2, x2, trans_a=True, trans_b=False, out=wmg, accumulate=True)
-        else:
-            for i in range(3):
-                grads_w[i] = _wgrad(d2[:, i * Ho:(i + 1) * Ho], x2, ctx.ws[i], ctx.mgs[i])
-        if ctx.bs[0] is not None:
-            bmg = _adjacent_view(ctx.mgs[3:]) if all(m is not None for m in ctx.mgs[3:]) else None
-            if bmg is not None:
-                K.colsum(d2, out=bmg)
-            else:
-                for i in range(3):
-                    grads_b[i] = _bgrad(d2[:, i * Ho:(i + 1) * Ho], ctx.bs[i], ctx.mgs[3 + i])
-        notify_grads(*[t for t, m in zip(ctx.ws + ctx.bs, ctx.mgs) if t is not None and m is not None])
-        return (dx, grads_w[0], grads_b[0], grads_w[1], grads_b[1], grads_w[2], grads_b[2], None, None, None, None)
-
-
 def qkv_attention(x, wq, bq, wk, bk, wv, bv, attn_mask=None, dropout_p: float = 0.0, is_causal: bool = False,
                   scale=None, num_heads: int = 1):
     """Self-attention block input side: the three projections of ``x`` [B, S, hid] and the attention itself.
@@ -541,7 +288,17 @@ def qkv_attention(x, wq, bq, wk, bk, wv, bv, attn_mask=None, dropout_p: float = 
             ok = False
     if ok:
         sc = float(scale) if scale is not None else D ** -0.5
-        return _QkvAttention.apply(x, wq, bq, wk, bk, wv, bv, key_bias, float(dropout_p), sc, num_heads)
+        # ONE projection GEMM over the stacked weights; the attention kernels read q / k / v as strided views of its
+        # [B, S, 3, H, D] output and write dq / dk / dv into one buffer that the single dgrad GEMM consumes
+        h = _host()
+        ws, bs = [wq, wk, wv], [bq, bk, bv]
+        # parameters that are streamed in and out are stacked anew by every use, without a copy that outlives it
+        volatile = any(getattr(t, "_rannc_host", None) is not None or getattr(t, "_rannc_window", False) for t in ws)
+        cat_w = None if volatile or h.are_adjacent(ws) else _cat_params(ws)
+        cat_b = None if volatile or bq is None or h.are_adjacent(bs) else _cat_params(bs)
+        seed, offset = rng.next() if dropout_p > 0.0 else (0, 0)
+        return h.qkv_attention(x, ws, bs, key_bias, float(dropout_p), sc, num_heads, seed, offset,
+                               [_main_grad(t) for t in ws], [_main_grad(t) for t in bs], cat_w, cat_b)
     q = linear(x, wq, bq).view(B, S, num_heads, D).transpose(1, 2)
     k = linear(x, wk, bk).view(B, S, num_heads, D).transpose(1, 2)
     v = linear(x, wv, bv).view(B, S, num_heads, D).transpose(1, 2)
@@ -741,49 +498,13 @@ def conv2d(x, weight, bias=None, stride=1, padding=0, dilation=1, groups=1):
           p[0] == p[1] and Ci % 8 == 0 and Co % 8 == 0 and x.dim() == 4 and isinstance(p[0], int))
     if not ok:
         return torch.nn.functional.conv2d(x, weight, bias, stride, padding, dilation, groups)
+    if kh == 1 and s[0] == 1 and p[0] == 0:
+        # a 1x1 convolution is the linear layer over the pixels of the channels-last activation
+        mg = _main_grad(weight)
+        y = _host().linear(_nhwc(x), weight.reshape(Co, Ci), bias, False, None if mg is None else mg.view(Co, Ci),
+                           _main_grad(bias), weight)
+        return y.permute(0, 3, 1, 2)
     return _Conv2d.apply(x, weight, bias, s[0], p[0])
-
-
-class _BatchNormAct(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, residual, gamma, beta, run_mean, run_var, momentum, eps, relu):
-        N, C, H, W = x.shape
-        x2 = _nhwc(x).reshape(-1, C)
-        r2 = _nhwc(residual).reshape(-1, C) if residual is not None else None
-        g32, b32 = gamma.detach().float(), beta.detach().float()
-        rm = run_mean if (run_mean is not None and run_mean.dtype == torch.float32) else None
-        rv = run_var if rm is not None else None
-        y2, mean, rstd = K.bn_fwd(x2, r2, g32, b32, rm, rv, eps, momentum, relu)
-        if run_mean is not None and rm is None:
-            # statistics kept in a 16-bit buffer: update them with a few tiny element-wise operations
-            with torch.no_grad():
-                R = x2.shape[0]
-                var = (1.0 / (rstd * rstd) - eps) * (R / max(R - 1, 1))
-                run_mean.mul_(1 - momentum).add_((momentum * mean).to(run_mean.dtype))
-                run_var.mul_(1 - momentum).add_((momentum * var).to(run_var.dtype))
-        ctx.save_for_backward(x2, y2, mean, rstd, g32)
-        ctx.meta = (relu, residual is not None, (N, C, H, W), gamma, beta, _main_grad(gamma), _main_grad(beta))
-        return y2.view(N, H, W, C).permute(0, 3, 1, 2)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x2, y2, mean, rstd, g32 = ctx.saved_tensors
-        relu, has_res, (N, C, H, W), gamma, beta, g_mg, b_mg = ctx.meta
-        dy2 = _nhwc(dy).reshape(-1, C)
-        dx2, dres2, dgamma, dbeta = K.bn_bwd(x2, dy2, y2, mean, rstd, g32, relu, has_res)
-        dx = dx2.view(N, H, W, C).permute(0, 3, 1, 2)
-        dres = dres2.view(N, H, W, C).permute(0, 3, 1, 2) if has_res else None
-        dg = db = None
-        if g_mg is not None:
-            g_mg.add_(dgamma)
-        else:
-            dg = dgamma.to(gamma.dtype)
-        if b_mg is not None:
-            b_mg.add_(dbeta)
-        else:
-            db = dbeta.to(beta.dtype)
-        notify_grads(gamma if g_mg is not None else None, beta if b_mg is not None else None)
-        return dx, dres, dg, db, None, None, None, None, None
 
 
 def batch_norm_act(x, gamma, beta, running_mean, running_var, training: bool = True, momentum: float = 0.1,
@@ -797,5 +518,5 @@ def batch_norm_act(x, gamma, beta, running_mean, running_var, training: bool = T
         if residual is not None:
             y = y + residual
         return torch.relu(y) if relu else y
-    return _BatchNormAct.apply(x, residual, gamma, beta, running_mean, running_var, float(momentum), float(eps),
-                               bool(relu))
+    return _host().batch_norm_act(x, residual, gamma, beta, running_mean, running_var, float(momentum), float(eps),
+                                  bool(relu), _main_grad(gamma), _main_grad(beta))

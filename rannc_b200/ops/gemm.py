@@ -90,6 +90,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
     ``row_map = (Hp, Wp, H, W, pad)``: the M rows are positions of a padded image grid; only the interior is
     stored, at the un-padded row index (``out`` has N_img * H * W rows).
     """
+    if a.dim() == 2 and b.dim() == 2 and (out is None or out.dim() == 2) and rs_peers is None and gather is None and \
+            conv is None and row_map is None and wgrad_shifts is None and not b_row_shift:
+        odt = out_dtype or (out.dtype if out is not None else a.dtype)
+        return _lib.host().product(a, b, trans_a, trans_b, bias, residual, aux_in, aux_out, gelu, dgelu, out, accumulate,
+                                   odt != a.dtype, alpha, max_ctas)
     a, ar, ac, lda, ba, sa = _mat(a)
     b, br, bc, ldb, bb, sb = _mat(b)
     M, K = (ac, ar) if trans_a else (ar, ac)

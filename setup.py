@@ -1,9 +1,9 @@
 """Packaging entry: ``python setup.py build_ext --inplace`` (or ``pip install --no-build-isolation -e .``) compiles
-the two native libraries in-tree with ``rannc_b200.build`` -- nvcc for sm_100a only, g++ for the pybind11 core --
-and installs ``rannc_b200`` together with the ``pyrannc`` alias package and the ``bin/rl`` launcher shim.
+the three native libraries in-tree with ``rannc_b200.build`` -- nvcc for sm_100a only, g++ for the pybind11 core and
+for the operators' host side -- and installs ``rannc_b200`` together with the ``pyrannc`` alias package and the ``bin/rl`` launcher shim.
 
 The reference builds its extension through CMake from setup.py (setup.py, CMakeLists.txt); here the build is a
-short Python module because there are only two link targets and no third-party sources."""
+short Python module because there are only three link targets and no third-party sources."""
 import importlib.util
 import os
 
@@ -20,10 +20,11 @@ def _build_native():
     spec.loader.exec_module(mod)
     mod.build_core()
     mod.build_kernels()
+    mod.build_host()
 
 
 class BuildNative(Command):
-    description = "compile _core (pybind11) and _kernels (CUDA, sm_100a) next to the Python sources"
+    description = "compile _core (pybind11), _kernels (CUDA, sm_100a) and _host (PyTorch C++) next to the Python sources"
     user_options = [("inplace", "i", "accepted for compatibility; the build is always in-tree")]
     boolean_options = ["inplace"]
 
@@ -48,7 +49,7 @@ setup(
     version="0.1.0",
     description="Automatic model partitioning and training middleware for PyTorch on NVIDIA B200 (sm_100a)",
     packages=find_packages(include=["rannc_b200", "rannc_b200.*", "pyrannc"]),
-    package_data={"rannc_b200": ["*.so", "csrc/core/*", "csrc/cuda/*"]},
+    package_data={"rannc_b200": ["*.so", "csrc/core/*", "csrc/cuda/*", "csrc/host/*"]},
     scripts=["bin/rl"],
     python_requires=">=3.10",
     install_requires=["torch>=2.6"],
