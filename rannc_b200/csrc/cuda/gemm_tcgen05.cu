@@ -37,28 +37,30 @@
 namespace rb {
 
 constexpr int BM = 128;
-constexpr int BN = 256;
 constexpr int BK = 64;
 constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int EPI_WARPS = 8;                         // two per TMEM lane quarter: each drains 128 of the 256 columns
 constexpr int EPI_THREADS = 32 * EPI_WARPS;
 constexpr int GEMM_THREADS = 64 + EPI_THREADS;
-constexpr int TMEM_COLS = 512;
 constexpr int GROUP_M = 8;
 // Output staging: every epilogue warp owns 4 KiB of shared memory in which it lays out a 32 x 32 block of the
 // tile (16-bit: two blocks of 64-byte rows; fp32: one of 128-byte rows, both swizzled as the tensor map of D
 // says) that the copy engine then writes, or adds, to global memory.
 constexpr int EPI_STAGE_BYTES = 4096;
 
-template <bool PAIR>
+// TN: columns of the output tile.  A wide tile moves the fewest bytes per multiplication; a problem with too few
+// 256-wide tiles to give every SM one takes 128 or 64 columns instead (single-CTA kernel only).
+template <bool PAIR, int TN>
 struct Cfg {
-    static constexpr int STAGES = PAIR ? 6 : 4;
-    static constexpr int B_ROWS = PAIR ? BN / 2 : BN;       // extent of the B tile one CTA loads
-    static constexpr int B_STAGE_BYTES = B_ROWS * BK * 2;   // 16 / 32 KiB
+    static_assert(TN == 256 || (!PAIR && (TN == 128 || TN == 64)), "unsupported tile");
+    static constexpr int B_ROWS = PAIR ? TN / 2 : TN;       // extent of the B tile one CTA loads
+    static constexpr int B_STAGE_BYTES = B_ROWS * BK * 2;   // 8 / 16 / 32 KiB
     static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
+    static constexpr int STAGES = 192 * 1024 / STAGE_BYTES;  // 6 (pair) / 4 / 6 / 8
     static constexpr int SMEM_BYTES =
         STAGES * STAGE_BYTES + EPI_WARPS * EPI_STAGE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
     static constexpr int TILE_M = PAIR ? 2 * BM : BM;       // rows of the output tile of a CTA (pair)
+    static constexpr int TMEM_COLS = 2 * TN;                // two accumulators
 };
 
 struct GemmKernelParams {
@@ -165,16 +167,17 @@ __device__ __forceinline__ void store32(T* ptr, bool vec_ok, int valid, const fl
     }
 }
 
-template <typename InT, typename OutT, bool PAIR>
+template <typename InT, typename OutT, bool PAIR, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
                         const __grid_constant__ CUtensorMap tmB,
                         const __grid_constant__ CUtensorMap tmD,
                         const __grid_constant__ CUtensorMap tmAux, const GemmKernelParams p) {
-    constexpr int STAGES = Cfg<PAIR>::STAGES;
-    constexpr int B_STAGE_BYTES = Cfg<PAIR>::B_STAGE_BYTES;
-    constexpr int STAGE_BYTES = Cfg<PAIR>::STAGE_BYTES;
-    constexpr int TILE_M = Cfg<PAIR>::TILE_M;
+    constexpr int STAGES = Cfg<PAIR, BN>::STAGES;
+    constexpr int B_STAGE_BYTES = Cfg<PAIR, BN>::B_STAGE_BYTES;
+    constexpr int STAGE_BYTES = Cfg<PAIR, BN>::STAGE_BYTES;
+    constexpr int TILE_M = Cfg<PAIR, BN>::TILE_M;
+    constexpr int TMEM_COLS = Cfg<PAIR, BN>::TMEM_COLS;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
@@ -323,7 +326,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                             tma_load_3d_pair(b_dst, &tmB, fb, k0, n0, b);
                         } else {
 #pragma unroll
-                            for (int c = 0; c < Cfg<PAIR>::B_ROWS / 64; ++c) {
+                            for (int c = 0; c < Cfg<PAIR, BN>::B_ROWS / 64; ++c) {
                                 int cx, cy;
                                 b_chunk(n0 + c * 64, cx, cy);
                                 tma_load_3d_pair(b_dst + c * (BK * 128), &tmB, fb, cx, cy, b);
@@ -871,11 +874,11 @@ int num_sms() {
     return n[dev];
 }
 
-template <typename InT, typename OutT, bool PAIR>
+template <typename InT, typename OutT, bool PAIR, int TN>
 static int launch(const RbGemmArgs& a, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmD,
                   const CUtensorMap& tmAux, const GemmKernelParams& p, cudaStream_t stream) {
-    auto kern = gemm_tcgen05_kernel<InT, OutT, PAIR>;
-    constexpr int smem = Cfg<PAIR>::SMEM_BYTES;
+    auto kern = gemm_tcgen05_kernel<InT, OutT, PAIR, TN>;
+    constexpr int smem = Cfg<PAIR, TN>::SMEM_BYTES;
     static bool attr_set[64] = {false};
     static int max_clusters[64] = {0};
     int dev = 0;
@@ -915,6 +918,19 @@ static int launch(const RbGemmArgs& a, const CUtensorMap& tmA, const CUtensorMap
     cfg.gridDim = dim3(2 * clusters, 1, 1);
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmD, tmAux, p);
     return e == cudaSuccess ? 0 : -static_cast<int>(e);
+}
+
+template <typename InT>
+static int dispatch(const RbGemmArgs& a, bool pair, int tn, const CUtensorMap& tmA, const CUtensorMap& tmB,
+                    const CUtensorMap& tmD, const CUtensorMap& tmAux, const GemmKernelParams& p, cudaStream_t st) {
+#define RB_GEMM_LAUNCH(PAIR, TN)                                                             \
+    return a.out_dtype == 0 ? launch<InT, InT, PAIR, TN>(a, tmA, tmB, tmD, tmAux, p, st) \
+                            : launch<InT, float, PAIR, TN>(a, tmA, tmB, tmD, tmAux, p, st)
+    if (pair) RB_GEMM_LAUNCH(true, 256);
+    if (tn == 64) RB_GEMM_LAUNCH(false, 64);
+    if (tn == 128) RB_GEMM_LAUNCH(false, 128);
+    RB_GEMM_LAUNCH(false, 256);
+#undef RB_GEMM_LAUNCH
 }
 
 // RB_GEMM_PAIR_GATHER=1 also puts the gather -> GEMM variant on the pair kernel (same prologue code).  Measured
@@ -963,14 +979,56 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     const bool accum32 = a->out_dtype == 1 && a->flags == RB_GEMM_ACCUM;
     bool pair = pair_enabled() && (a->ag_nranks <= 1 || pair_gather_enabled());
     if (pair) {
-        const long long pt = ((a->M + 2 * BM - 1) / (2 * BM)) * ((a->N + BN - 1) / BN) * a->batch;
+        const long long pt = ((a->M + 2 * BM - 1) / (2 * BM)) * ((a->N + 255) / 256) * a->batch;
         const long long kbs = (a->K + BK - 1) / BK;
         if (pt < num_sms() / 2 && !(accum32 && a->M > BM && pt * (kbs / 4) >= num_sms() / 2)) pair = false;
     }
     p.num_m_blocks = pair ? (p.M + 2 * BM - 1) / (2 * BM) : (p.M + BM - 1) / BM;
-    p.num_n_blocks = (p.N + BN - 1) / BN;
-    p.base_tiles = p.num_m_blocks * p.num_n_blocks * p.batch;
     p.num_kb = (p.K + BK - 1) / BK;
+    const int units = pair ? num_sms() / 2 : num_sms();   // CTAs (or CTA pairs) that run at once
+    // Few output tiles and a long K (weight gradients): split K over CTAs and accumulate with
+    // reductions.  Only for fp32 outputs that accumulate and have no other epilogue work.
+    auto split_for = [&](int tiles) {
+        int split = 1;
+        if (accum32 && tiles < units && p.num_kb >= 8) {
+            double best = 0.0;
+            for (int s = 1; s <= 32 && s * 4 <= p.num_kb; ++s) {
+                const int work = tiles * s;
+                const int waves = (work + units - 1) / units;
+                const double eff = static_cast<double>(work) / (waves * units) - 0.005 * s;
+                if (eff > best + 1e-9) {
+                    best = eff;
+                    split = s;
+                }
+            }
+        }
+        return split;
+    };
+    int tn = 256;
+    if (!pair && a->ag_nranks <= 1 && a->rs_nranks <= 1) {
+        if (a->tile_n == 64 || a->tile_n == 128 || a->tile_n == 256) {
+            tn = a->tile_n;
+        } else {
+            // Narrow tiles move more bytes per product but keep more SMs busy.  Estimated cycles: k steps one CTA
+            // does, each bound by its loads (48 / 32 / 24 KiB), plus the last tile's epilogue.  Measured with 256 /
+            // 128 / 64 columns (us): 32 x 1024 x 1024 10.1 / 9.0 / 8.5; 351 x 3072 x 768 9.5 / 8.7 / 8.0;
+            // 1182 x 768 x 2304 22.0 / 17.1 / 15.4; 2000 x 1024 x 1024 11.0 / 10.1 / 14.4;
+            // 1182 x 2304 x 768 9.9 / 13.0 / 16.2.  The rule took the best or one within 2 % in 21 of 22 shapes.
+            double best = 1e30;
+            for (int t : {256, 128, 64}) {
+                const int tiles = p.num_m_blocks * ((p.N + t - 1) / t) * p.batch;
+                const int s = split_for(tiles);
+                const double steps = static_cast<double>((tiles * s + units - 1) / units) * ((p.num_kb + s - 1) / s);
+                const double cost = steps * (t == 256 ? 768 : (t == 128 ? 512 : 384)) + 12.0 * t;
+                if (cost < 0.98 * best) {
+                    best = cost;
+                    tn = t;
+                }
+            }
+        }
+    }
+    p.num_n_blocks = (p.N + tn - 1) / tn;
+    p.base_tiles = p.num_m_blocks * p.num_n_blocks * p.batch;
     p.ag_nranks = a->ag_nranks > 1 ? a->ag_nranks : 0;
     p.ag_my_idx = a->ag_my_idx;
     p.ag_rows = a->ag_rows;
@@ -993,21 +1051,7 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     if (p.rs_nranks > 1 && (a->out_dtype != 1 || a->flags != RB_GEMM_ACCUM || a->N % a->rs_nranks || p.rs_cols % 32 ||
                             a->rs_nranks > 8 || a->batch != 1))
         return -5;
-    // Few output tiles and a long K (weight gradients): split K over CTAs and accumulate with
-    // reductions.  Only for fp32 outputs that accumulate and have no other epilogue work.
-    const int units = pair ? num_sms() / 2 : num_sms();   // CTAs (or CTA pairs) that run at once
-    if (accum32 && p.base_tiles < units && p.num_kb >= 8) {
-        double best = 0.0;
-        for (int s = 1; s <= 32 && s * 4 <= p.num_kb; ++s) {
-            const int work = p.base_tiles * s;
-            const int waves = (work + units - 1) / units;
-            const double eff = static_cast<double>(work) / (waves * units) - 0.005 * s;
-            if (eff > best + 1e-9) {
-                best = eff;
-                p.split_k = s;
-            }
-        }
-    }
+    p.split_k = split_for(p.base_tiles);
     p.kb_per_split = (p.num_kb + p.split_k - 1) / p.split_k;
     p.split_k = (p.num_kb + p.kb_per_split - 1) / p.kb_per_split;
     p.num_tiles = p.base_tiles * p.split_k;
@@ -1067,7 +1111,7 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
         rc = make_tmap_3d(&tmA, a->A, a->in_dtype, a->M, a->K, a->batch, a->lda * 2, sA, 64, BK, 1);
     if (rc) return rc;
     if (a->b_major == 0)
-        rc = make_tmap_3d(&tmB, a->B, a->in_dtype, a->K, a->N, a->batch, a->ldb * 2, sB, BK, pair ? BN / 2 : BN, 1);
+        rc = make_tmap_3d(&tmB, a->B, a->in_dtype, a->K, a->N, a->batch, a->ldb * 2, sB, BK, pair ? 128 : tn, 1);
     else if (a->conv_taps > 0)
         // the stored matrix is [conv_c rows, conv_taps * conv_b_tap_cols columns]: tap t's [conv_c, N] block
         // starts at column t * conv_b_tap_cols
@@ -1101,19 +1145,8 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
         if (rc) p.staged = 0;
     }
 
-    if (a->in_dtype == 1) {
-        if (a->out_dtype == 0)
-            return pair ? launch<__nv_bfloat16, __nv_bfloat16, true>(*a, tmA, tmB, tmD, tmAux, p, stream)
-                        : launch<__nv_bfloat16, __nv_bfloat16, false>(*a, tmA, tmB, tmD, tmAux, p, stream);
-        return pair ? launch<__nv_bfloat16, float, true>(*a, tmA, tmB, tmD, tmAux, p, stream)
-                    : launch<__nv_bfloat16, float, false>(*a, tmA, tmB, tmD, tmAux, p, stream);
-    } else {
-        if (a->out_dtype == 0)
-            return pair ? launch<__half, __half, true>(*a, tmA, tmB, tmD, tmAux, p, stream)
-                        : launch<__half, __half, false>(*a, tmA, tmB, tmD, tmAux, p, stream);
-        return pair ? launch<__half, float, true>(*a, tmA, tmB, tmD, tmAux, p, stream)
-                    : launch<__half, float, false>(*a, tmA, tmB, tmD, tmAux, p, stream);
-    }
+    return a->in_dtype == 1 ? dispatch<__nv_bfloat16>(*a, pair, tn, tmA, tmB, tmD, tmAux, p, stream)
+                            : dispatch<__half>(*a, pair, tn, tmA, tmB, tmD, tmAux, p, stream);
 }
 
 // Copies the device error word into `host_dst` (pinned host memory) on `stream` without waiting: the caller

@@ -60,6 +60,7 @@ typedef struct RbGemmArgs {
     // shifted by conv_shift[t].  One launch for all taps: the gradient operand A is read once per column of
     // tiles instead of once per tap.
     int32_t wgrad_taps;
+    int32_t tile_n;   // columns of the single-CTA kernel's tile: 0 (chosen by size), 64, 128 or 256
 } RbGemmArgs;
 
 // returns 0 on success, <0 on a host-side error (-2: operand not 16 B aligned)

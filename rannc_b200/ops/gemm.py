@@ -29,6 +29,7 @@ class _Args(ctypes.Structure):
         ("b_row_shift", ctypes.c_int32), ("conv_shift", ctypes.c_int32 * 49),
         ("map_hp", ctypes.c_int32), ("map_wp", ctypes.c_int32), ("map_h", ctypes.c_int32),
         ("map_w", ctypes.c_int32), ("map_pad", ctypes.c_int32), ("wgrad_taps", ctypes.c_int32),
+        ("tile_n", ctypes.c_int32),
     ]
 
 
@@ -72,7 +73,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
          dgelu: bool = False, out: torch.Tensor | None = None, accumulate: bool = False,
          out_dtype: torch.dtype | None = None, alpha: float = 1.0, max_ctas: int = 0,
          rs_peers=None, rs_ld: int = 0, gather=None, conv=None, b_row_shift: int = 0,
-         row_map=None, wgrad_shifts=None) -> torch.Tensor:
+         row_map=None, wgrad_shifts=None, tile_n: int = 0) -> torch.Tensor:
     """``out = epilogue(alpha * op(a) @ op(b))``.
 
     ``a`` is stored ``[M, K]`` (``trans_a=False``) or ``[K, M]`` (``trans_a=True``).
@@ -91,7 +92,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
     stored, at the un-padded row index (``out`` has N_img * H * W rows).
     """
     if a.dim() == 2 and b.dim() == 2 and (out is None or out.dim() == 2) and rs_peers is None and gather is None and \
-            conv is None and row_map is None and wgrad_shifts is None and not b_row_shift:
+            conv is None and row_map is None and wgrad_shifts is None and not b_row_shift and not tile_n:
         odt = out_dtype or (out.dtype if out is not None else a.dtype)
         return _lib.host().product(a, b, trans_a, trans_b, bias, residual, aux_in, aux_out, gelu, dgelu, out, accumulate,
                                    odt != a.dtype, alpha, max_ctas)
@@ -171,6 +172,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         args.conv_b_tap_cols = int(conv.get("b_tap_cols", 0))
         for i, sh in enumerate(conv["shifts"]):
             args.conv_shift[i] = int(sh)
+    args.tile_n = int(tile_n)
     if wgrad_shifts is not None:
         args.wgrad_taps = len(wgrad_shifts)
         args.conv_c = bc

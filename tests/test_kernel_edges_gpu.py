@@ -181,3 +181,29 @@ def test_batch_norm_channel_blocks(C, N, H, W, flat):
     gg, bg = (g.main_grad - 3.0, b.main_grad + 1.0) if flat else (g.grad, b.grad)
     _near(gg, gr.grad, dt, 0, 1e-5)
     _near(bg, br.grad, dt, 0, 1e-5)
+
+
+@pytest.mark.parametrize("tile_n", [64, 128, 256])
+@pytest.mark.parametrize("M,N,K", [(1, 64, 64), (130, 72, 200), (257, 520, 1032), (640, 1160, 72)])
+@pytest.mark.parametrize("trans_a,trans_b", [(False, True), (False, False), (True, False), (True, True)])
+def test_gemm_tile_widths(tile_n, M, N, K, trans_a, trans_b):
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops.gemm import gemm
+
+    torch.manual_seed(5)
+    dt = torch.bfloat16
+    lead = lambda n: (n + 7) // 8 * 8  # noqa: E731
+    a = torch.randn((K, lead(M)) if trans_a else (M, K), device="cuda").to(dt)
+    a = a[:, :M] if trans_a else a
+    b = torch.randn((N, K) if trans_b else (K, N), device="cuda").to(dt)
+    ref = (a.double().t() if trans_a else a.double()) @ (b.double().t() if trans_b else b.double())
+    _near(gemm(a, b, trans_a=trans_a, trans_b=trans_b, tile_n=tile_n), ref, dt, 1)
+    acc = torch.ones(M, N, device="cuda")
+    gemm(a, b, trans_a=trans_a, trans_b=trans_b, out=acc, accumulate=True, tile_n=tile_n)
+    _near(acc, ref + 1.0, dt, 0)
+    # many tiles per CTA: every stage and both accumulators wrap
+    few = torch.empty(M, N, device="cuda", dtype=dt)
+    gemm(a, b, trans_a=trans_a, trans_b=trans_b, out=few, tile_n=tile_n, max_ctas=2)
+    _near(few, ref, dt, 1)
+    torch.cuda.synchronize()
+    assert _lib.read_error() == 0
