@@ -401,38 +401,49 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
     }
 }
 
-// delta[b,h,q] = sum_d dO[b,q,h,d] * O[b,q,h,d], D = 64.  Rows are taken in memory order ((b, q, h): h is
-// the fastest index of a [B, S, H, D] tensor), 8 lanes x 16 bytes per row, so a warp reads 512 contiguous
-// bytes of each tensor per step.
+// delta[b,h,q] = sum_d dO[b,q,h,d] * O[b,q,h,d], D = 64, and the dQ scratch is cleared on the way (a memset of its
+// own cost as much as the rest of this pass).  Rows are taken in memory order ((b, q, h): h is the fastest index of
+// a [B, S, H, D] tensor), 8 lanes x 16 bytes per row, two rows of a thread in flight: bound by memory.
 template <typename T>
-__global__ void attn_delta_kernel(const T* __restrict__ O, const T* __restrict__ dO,
-                                  float* __restrict__ delta, int B, int H, int S, long long o_sb,
-                                  long long o_ss, long long o_sh, long long d_sb, long long d_ss,
-                                  long long d_sh) {
-    const long long rows = static_cast<long long>(B) * S * H;
+__global__ void __launch_bounds__(256)
+    attn_delta_kernel(const T* __restrict__ O, const T* __restrict__ dO,
+                      float* __restrict__ delta, float* __restrict__ dq_accum, int B, int H, int S,
+                      long long o_sb, long long o_ss, long long o_sh, long long d_sb, long long d_ss,
+                      long long d_sh) {
+    const unsigned rows = static_cast<unsigned>(B) * S * H;   // < 2^31: checked by the caller
     const int sub = threadIdx.x & 7;
-    const long long step = (static_cast<long long>(gridDim.x) * blockDim.x) >> 3;
-    // warp-uniform trip count: every lane takes part in the shuffles
-    long long row = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 3;
-    const long long first = (blockIdx.x * static_cast<long long>(blockDim.x) + (threadIdx.x & ~31)) >> 3;
-    for (long long base = first; base < rows; base += step, row += step) {
-        float s = 0.f;
-        int h = 0, q = 0, b = 0;
-        if (row < rows) {
-            h = static_cast<int>(row % H);
-            q = static_cast<int>((row / H) % S);
-            b = static_cast<int>(row / (static_cast<long long>(H) * S));
-            const uint4 ov = *reinterpret_cast<const uint4*>(O + b * o_sb + q * o_ss + h * o_sh + sub * 8);
-            const uint4 dv = *reinterpret_cast<const uint4*>(dO + b * d_sb + q * d_ss + h * d_sh + sub * 8);
-            const T* oe = reinterpret_cast<const T*>(&ov);
-            const T* de = reinterpret_cast<const T*>(&dv);
+    // a block takes 64 consecutive rows: 32 and the 32 behind them
+    const unsigned row0 = blockIdx.x * 64u + (threadIdx.x >> 3);
+    uint4 ov[2], dv[2];
+    long long at[2];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) s = fmaf(to_f32<T>(oe[j]), to_f32<T>(de[j]), s);
+    for (int u = 0; u < 2; ++u) {
+        const unsigned row = row0 + u * 32u;
+        ov[u] = dv[u] = make_uint4(0, 0, 0, 0);
+        at[u] = -1;
+        if (row < rows) {
+            const unsigned bq = row / H, h = row - bq * H, b = bq / S, q = bq - b * S;
+            ov[u] = *reinterpret_cast<const uint4*>(O + b * o_sb + q * o_ss + h * o_sh + sub * 8);
+            dv[u] = *reinterpret_cast<const uint4*>(dO + b * d_sb + q * d_ss + h * d_sh + sub * 8);
+            at[u] = (static_cast<long long>(b) * H + h) * S + q;
         }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        if (at[u] >= 0) {
+            float4* z = reinterpret_cast<float4*>(dq_accum + static_cast<size_t>(row0 + u * 32u) * 64 + sub * 4);
+            z[0] = make_float4(0.f, 0.f, 0.f, 0.f);   // 8 lanes cover the row in two runs of 128 bytes
+            z[8] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        const T* oe = reinterpret_cast<const T*>(&ov[u]);
+        const T* de = reinterpret_cast<const T*>(&dv[u]);
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s = fmaf(to_f32<T>(oe[j]), to_f32<T>(de[j]), s);
         s += __shfl_xor_sync(0xffffffffu, s, 4);
         s += __shfl_xor_sync(0xffffffffu, s, 2);
         s += __shfl_xor_sync(0xffffffffu, s, 1);
-        if (sub == 0 && row < rows) delta[(static_cast<long long>(b) * H + h) * S + q] = s;
+        if (sub == 0 && at[u] >= 0) delta[at[u]] = s;
     }
 }
 
@@ -467,19 +478,10 @@ static int launch_bwd(const RbAttnArgs& a, cudaStream_t st) {
     if ((rc = make_tmap_4d(&tv, a.V, a.dtype, D, S, H, B, a.v_ss * 2, a.v_sh * 2, a.v_sb * 2, 64, 128))) return rc;
     if ((rc = make_tmap_4d(&tdo, a.dO, a.dtype, D, S, H, B, a.do_ss * 2, a.do_sh * 2, a.do_sb * 2, 64, 128))) return rc;
     const long long rows = static_cast<long long>(a.B) * a.H * a.S;
-    unsigned rb_delta_grid = 1;
-    {
-        // 8 lanes per row; the grid is sized so that every thread handles a few rows
-        long long blocks = (rows * 8 + 255) / 256;
-        const long long cap = 148LL * 32;
-        if (blocks > cap) blocks = cap;
-        if (blocks < 1) blocks = 1;
-        rb_delta_grid = static_cast<unsigned>(blocks);
-    }
-    attn_delta_kernel<T><<<rb_delta_grid, 256, 0, st>>>(
-        static_cast<const T*>(a.O), static_cast<const T*>(a.dO), a.delta, a.B, a.H, a.S, a.o_sb,
+    if (rows >= (1LL << 31) - 64) return -2;
+    attn_delta_kernel<T><<<static_cast<unsigned>((rows + 63) / 64), 256, 0, st>>>(
+        static_cast<const T*>(a.O), static_cast<const T*>(a.dO), a.delta, a.dq_accum, a.B, a.H, a.S, a.o_sb,
         a.o_ss, a.o_sh, a.do_sb, a.do_ss, a.do_sh);
-    cudaMemsetAsync(a.dq_accum, 0, static_cast<size_t>(rows) * 64 * sizeof(float), st);
     AttnBwdParams p;
     p.B = a.B; p.H = a.H; p.S = a.S;
     p.scale = a.scale;

@@ -207,3 +207,45 @@ def test_gemm_tile_widths(tile_n, M, N, K, trans_a, trans_b):
     _near(few, ref, dt, 1)
     torch.cuda.synchronize()
     assert _lib.read_error() == 0
+
+
+@pytest.mark.parametrize("B,S,H", [(1, 1, 1), (2, 127, 3), (5, 129, 7), (9, 200, 20), (7, 384, 16), (4, 513, 12)])
+@pytest.mark.parametrize("p", [0.0, 0.25])
+def test_attention_backward_blocks(B, S, H, p):
+    """One, two and more query and key blocks, ragged last blocks, key bias, dropout."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(4)
+    dt = torch.bfloat16
+    qkv = torch.randn(B, S, 3, H, 64, device="cuda").to(dt)
+    q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
+    bias = torch.zeros(B, S, device="cuda")
+    bias[:, S - S // 5:] = -10000.0
+    drop = dict(p_drop=p, seed=5, offset=9)
+    mask = torch.ones(B, H, S, S, device="cuda", dtype=torch.float64)
+    if p:
+        # uniform attention over one-hot values reads the mask out, 64 keys at a time
+        z = torch.zeros(B, S, H, 64, device="cuda", dtype=dt)
+        for w in range(0, S, 64):
+            n = min(64, S - w)
+            one = z.clone()
+            one[:, w:w + n, :, :n] = torch.eye(n, device="cuda", dtype=dt)[None, :, None]
+            mask[:, :, :, w:w + n] = (K.attn_fwd(z, z, one, **drop)[0][..., :n] > 0).permute(0, 2, 1, 3).double()
+        mask /= 1 - p
+    o, lse = K.attn_fwd(q, k, v, key_bias=bias, **drop)
+    qr, kr, vr = (t.double().detach().requires_grad_(True) for t in (q, k, v))
+    sc = torch.einsum("bqhd,bkhd->bhqk", qr, kr) / 8 + bias.double()[:, None, None]
+    ref = torch.einsum("bhqk,bkhd->bqhd", sc.softmax(-1) * mask, vr)
+    do = torch.randn(B, S, H, 64, device="cuda").to(dt)
+    ref.backward(do.double())
+    dq, dk, dv = K.attn_bwd(q, k, v, o, lse, do, key_bias=bias, **drop)
+    torch.cuda.synchronize()
+    assert _lib.read_error() == 0
+    # probabilities and their gradients are rounded to 16 bits before the products, O before delta: a few roundings of
+    # terms as large as the largest result.  dP - delta cancels (down to nothing for a single key), so what is rounded
+    # has the scale of dP, which dV's terms show and dQ itself need not.
+    scale = max(t.grad.abs().max().item() for t in (qr, kr, vr)) + 1e-3
+    for got, want in ((dq, qr.grad), (dk, kr.grad), (dv, vr.grad)):
+        err = (got.double() - want).abs().max().item() / scale
+        assert err < 6 * U[dt], err
