@@ -41,7 +41,8 @@ constexpr int BK = 64;
 constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int EPI_WARPS = 8;                         // two per TMEM lane quarter: each drains 128 of the 256 columns
 constexpr int EPI_THREADS = 32 * EPI_WARPS;
-constexpr int GEMM_THREADS = 64 + EPI_THREADS;
+constexpr int SUM_WARPS = 2;                         // column sums of A: one per 64-column chunk of its tile
+constexpr int GEMM_THREADS = 64 + EPI_THREADS + 32 * SUM_WARPS;
 constexpr int GROUP_M = 8;
 // Output staging: every epilogue warp owns 4 KiB of shared memory in which it lays out a 32 x 32 block of the
 // tile (16-bit: two blocks of 64-byte rows; fp32: one of 128-byte rows, both swizzled as the tensor map of D
@@ -58,7 +59,7 @@ struct Cfg {
     static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
     static constexpr int STAGES = 192 * 1024 / STAGE_BYTES;  // 6 (pair) / 4 / 6 / 8
     static constexpr int SMEM_BYTES =
-        STAGES * STAGE_BYTES + EPI_WARPS * EPI_STAGE_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
+        STAGES * STAGE_BYTES + EPI_WARPS * EPI_STAGE_BYTES + 1024 /*align slack*/ + 384 /*barriers*/;
     static constexpr int TILE_M = PAIR ? 2 * BM : BM;       // rows of the output tile of a CTA (pair)
     static constexpr int TMEM_COLS = 2 * TN;                // two accumulators
 };
@@ -92,6 +93,7 @@ struct GemmKernelParams {
     // 1: the epilogue goes through shared memory and the copy engine (tensor maps of D and of the auxiliary
     // matrix); 0: every thread stores its own row (mapped rows, peers' memory, unaligned outputs)
     int staged;
+    float* a_colsum;   // not null: column sums of the stored A (MN-major) are added here
 };
 
 __device__ __forceinline__ void tile_coords(const GemmKernelParams& p, int tile, int& mb, int& nb,
@@ -190,7 +192,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     uint64_t* tfull = bars + 2 * STAGES;    // [2]
     uint64_t* tempty = bars + 2 * STAGES + 2;  // [2]
     uint64_t* aux_full = bars + 2 * STAGES + 4;  // [EPI_WARPS] a warp's block of the auxiliary matrix has arrived
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4 + EPI_WARPS);
+    uint64_t* used = aux_full + EPI_WARPS;       // [STAGES] a_colsum: the MMAs have read the stage, the sums may
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(used + STAGES);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
@@ -203,7 +206,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1);
+            mbar_init(&empty[s], p.a_colsum ? SUM_WARPS : 1);
+            mbar_init(&used[s], 1);
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(&tfull[a], 1);
@@ -402,10 +406,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         else
                             umma_f16(d_tmem, da, db, idesc, (kb > kb_begin || k > 0) ? 1u : 0u);
                     }
+                    // frees the stage (PAIR: in both CTAs), or hands it on to the warps that sum its columns
+                    uint64_t* done = p.a_colsum ? &used[stage] : &empty[stage];
                     if constexpr (PAIR)
-                        umma_commit_pair(&empty[stage], 3);   // frees the stage in both CTAs
+                        umma_commit_pair(done, 3);
                     else
-                        umma_commit(&empty[stage]);
+                        umma_commit(done);
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
@@ -419,8 +425,62 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                 }
             }
         }
+    } else if (warp >= 2 + EPI_WARPS) {
+        if (p.a_colsum) {
+            // ---------------- column sums of A (bias gradient beside a weight gradient) ----------------
+            // A = dy is stored [K, M] and passes through shared memory anyway: a separate kernel reads it once more
+            // from memory (98 us for 8192 x 30528).  The n-blocks of a tile row share the work: block nb sums the k
+            // steps congruent to nb, so every row is added exactly once and a summed step (16 KiB of shared-memory
+            // reads) comes once per num_n_blocks steps.
+            const int c = warp - (2 + EPI_WARPS);   // 64-column chunk of the tile
+            const int piece = lane & 7, kr = lane >> 3;
+            int stage = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int tile = tile0; tile < p.num_tiles && ok; tile += tile_step) {
+                int mb, nb, b, kb_begin, kb_end;
+                tile_coords(p, tile, mb, nb, b, kb_begin, kb_end);
+                float s[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) s[j] = 0.f;
+                bool any = false;
+                for (int kb = kb_begin; kb < kb_end; ++kb) {
+                    if (!(PAIR ? mbar_wait_cluster(&used[stage], phase, abort_flag)
+                               : mbar_wait(&used[stage], phase, abort_flag))) {
+                        ok = false;
+                        break;
+                    }
+                    if (kb % p.num_n_blocks == nb) {
+                        any = true;
+                        const uint8_t* rows = sA + stage * A_STAGE_BYTES + c * (BK * 128);
+#pragma unroll 8
+                        for (int r = kr; r < BK; r += 4) {
+                            const uint4 q4 = *reinterpret_cast<const uint4*>(rows + r * 128 + ((piece ^ (r & 7)) << 4));
+                            const InT* e = reinterpret_cast<const InT*>(&q4);
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) s[j] += to_f32<InT>(e[j]);
+                        }
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&empty[stage]);
+                    if (++stage == STAGES) {
+                        stage = 0;
+                        phase ^= 1;
+                    }
+                }
+                if (any && ok) {
+                    const int m0 = mb * TILE_M + static_cast<int>(crank) * BM + c * 64 + piece * 8;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        s[j] += __shfl_xor_sync(0xffffffffu, s[j], 8);
+                        s[j] += __shfl_xor_sync(0xffffffffu, s[j], 16);
+                        if (kr == 0 && m0 + j < p.M) atomicAdd(p.a_colsum + m0 + j, s[j]);
+                    }
+                }
+            }
+        }
     } else {
-        // ---------------- epilogue (warps 2..5) ----------------
+        // ---------------- epilogue (warps 2..9) ----------------
         if (p.ag_nranks > 1) {
             // all-gather prologue: the epilogue threads of every CTA copy their share of each peer's
             // shard into the local B buffer (plain 16-byte peer loads), in the order the k loop consumes
@@ -1085,6 +1145,8 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
         p.conv_b_tap_cols = a->conv_b_tap_cols;
         for (int t = 0; t < a->conv_taps; ++t) p.conv_shift[t] = a->conv_shift[t];
     }
+    p.a_colsum = a->a_colsum;
+    if (a->a_colsum && (a->a_major != 1 || a->batch != 1 || a->ag_nranks > 1)) return -8;
     p.wgrad_taps = 0;
     p.wgrad_cols = 1;
     if (a->wgrad_taps > 0) {

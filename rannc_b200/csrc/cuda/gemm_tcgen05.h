@@ -60,6 +60,8 @@ typedef struct RbGemmArgs {
     // shifted by conv_shift[t].  One launch for all taps: the gradient operand A is read once per column of
     // tiles instead of once per tap.
     int32_t wgrad_taps;
+    int32_t reserved_;
+    float* a_colsum;  // a_major = 1 only: the column sums of the stored A ([K, M]) are added to these M floats
     int32_t tile_n;   // columns of the single-CTA kernel's tile: 0 (chosen by size), 64, 128 or 256
 } RbGemmArgs;
 

@@ -132,6 +132,7 @@ struct Epi {
     const void* aux_in = nullptr;
     void* aux_out = nullptr;
     bool gelu = false, dgelu = false, accumulate = false;
+    float* a_colsum = nullptr;   // the column sums of a stored [K, M] are added here
 };
 // out [M, N] = epilogue(op(a) op(b)), rows ldd apart (0: N)
 void gemm(const Mat& a, const Mat& b, bool trans_a, bool trans_b, void* out, bool out_fp32, int dtype, const Epi& e,
@@ -160,26 +161,36 @@ void gemm(const Mat& a, const Mat& b, bool trans_a, bool trans_b, void* out, boo
     g.flags = (e.bias ? RB_GEMM_BIAS : 0) | (e.gelu ? RB_GEMM_GELU : 0) | (e.dgelu ? RB_GEMM_DGELU : 0) |
               (e.accumulate ? RB_GEMM_ACCUM : 0) | (e.aux_out ? RB_GEMM_AUX_OUT : 0);
     g.alpha = 1.f;
+    g.a_colsum = e.a_colsum;
     check(api.gemm(&g, cur_stream()), "rb_gemm");
 }
-// dW = dy^T x: added to the fp32 gradient buffer when there is one, returned otherwise
-Tensor weight_grad(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& mg, int dtype) {
-    Epi e;
-    if (mg.defined()) {
-        e.accumulate = true;
-        gemm(dy, x, true, false, mg.data_ptr(), true, dtype, e, mg.stride(0));
-        return Tensor();
+// Gradients of one weight and its bias: dW = dy^T x and, from the same pass over dy, db = its column sums.  Each is added
+// to the fp32 buffer the parameter has, or returned in the parameter's own type.
+struct Grads {
+    Tensor w, b;
+};
+Grads param_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& w_mg, bool want_w, const Tensor& bias,
+                  const Tensor& b_mg, bool want_b, int dtype) {
+    Grads out;
+    Tensor db;
+    if (bias.defined() && want_b) db = b_mg.defined() ? b_mg : at::zeros({dy.cols}, bias.options().dtype(at::kFloat));
+    if (want_w) {
+        Epi e;
+        e.a_colsum = mptr<float>(db);
+        if (w_mg.defined()) {
+            e.accumulate = true;
+            gemm(dy, x, true, false, w_mg.data_ptr(), true, dtype, e, w_mg.stride(0));
+        } else {
+            out.w = at::empty({dy.cols, x.cols}, w.options());
+            gemm(dy, x, true, false, out.w.data_ptr(), false, dtype, e);
+        }
+    } else if (db.defined()) {
+        check(api.colsum(dy.p, mptr<float>(db), static_cast<int>(dy.rows), static_cast<int>(dy.cols), dy.ld, dtype,
+                         cur_stream()),
+              "rb_colsum");
     }
-    Tensor dw = at::empty({dy.cols, x.cols}, w.options());
-    gemm(dy, x, true, false, dw.data_ptr(), false, dtype, e);
-    return dw;
-}
-Tensor bias_grad(const Mat& dy, const Tensor& bias, const Tensor& mg, int dtype) {
-    if (!bias.defined()) return Tensor();
-    Tensor out = mg.defined() ? mg : at::zeros({dy.cols}, bias.options().dtype(at::kFloat));
-    check(api.colsum(dy.p, mptr<float>(out), static_cast<int>(dy.rows), static_cast<int>(dy.cols), dy.ld, dtype, cur_stream()),
-          "rb_colsum");
-    return mg.defined() ? Tensor() : out.to(bias.scalar_type());
+    if (db.defined() && !b_mg.defined()) out.b = db.to(bias.scalar_type());
+    return out;
 }
 
 // ------------------------------------------------------------------------------------------------ autograd plumbing
@@ -242,15 +253,15 @@ struct LinearNode : Node {
             dy = d;
         }
         const Mat d = rows_of(dy);
-        Tensor dx, dw, db;
+        Tensor dx;
         if (task_should_compute_output(0)) {
             dx = at::empty(X.sizes(), X.options());
             gemm(d, mat(W), false, false, dx.data_ptr(), false, dt, Epi());
         }
-        if (task_should_compute_output(1)) dw = weight_grad(d, rows_of(X), W, w_mg, dt);
-        if (bias.defined() && task_should_compute_output(2)) db = bias_grad(d, bias, b_mg, dt);
+        const Grads gr = param_grads(d, rows_of(X), W, w_mg, task_should_compute_output(1), bias, b_mg,
+                                     bias.defined() && task_should_compute_output(2), dt);
         notify({{&w_ref, &w_mg}, {&bias, &b_mg}});
-        return {dx, dw, db};
+        return {dx, gr.w, gr.b};
     }
 };
 
@@ -304,23 +315,21 @@ struct MlpNode : Node {
         const Tensor dy = dense(grads[0]);
         const int dt = dt_code(X);
         const Mat d = rows_of(dy), hm = rows_of(Hh);
-        Tensor dw2 = weight_grad(d, hm, W2, w2_mg, dt);
-        Tensor db2 = bias_grad(d, b2, b2_mg, dt);
+        const Grads g2 = param_grads(d, hm, W2, w2_mg, true, b2, b2_mg, true, dt);
         Tensor dpre = at::empty(P.sizes(), P.options());
         Epi e;
         e.dgelu = true;
         e.aux_in = P.data_ptr();
         gemm(d, mat(W2), false, false, dpre.data_ptr(), false, dt, e);
         const Mat dp = rows_of(dpre);
-        Tensor dw1 = weight_grad(dp, rows_of(X), W1, w1_mg, dt);
-        Tensor db1 = bias_grad(dp, b1, b1_mg, dt);
+        const Grads g1 = param_grads(dp, rows_of(X), W1, w1_mg, true, b1, b1_mg, true, dt);
         Tensor dx;
         if (task_should_compute_output(0)) {
             dx = at::empty(X.sizes(), X.options());
             gemm(dp, mat(W1), false, false, dx.data_ptr(), false, dt, Epi());
         }
         notify({{&w1_ref, &w1_mg}, {&b1, &b1_mg}, {&w2_ref, &w2_mg}, {&b2, &b2_mg}});
-        return {dx, dw1, db1, dw2, db2};
+        return {dx, g1.w, g1.b, g2.w, g2.b};
     }
 };
 
@@ -639,25 +648,21 @@ struct QkvNode : Node {
             dx = at::empty(X.sizes(), X.options());
             gemm(dm, stacked(w, cat), false, false, dx.data_ptr(), false, dt, Epi());
         }
-        // adjacent fp32 gradient buffers: one weight-gradient GEMM and one column sum serve all three projections
-        const bool all_w = w_mg[0].defined() && w_mg[1].defined() && w_mg[2].defined();
-        const void* wm = all_w ? adjacent(w_mg) : nullptr;
-        if (wm) {
+        // adjacent fp32 gradient buffers: one weight-gradient GEMM (with the column sums of the biases) serves all three
+        // projections
+        auto all = [](const Tensor* t) { return t[0].defined() && t[1].defined() && t[2].defined(); };
+        const void* wm = all(w_mg) ? adjacent(w_mg) : nullptr;
+        const void* bm = b[0].defined() && all(b_mg) ? adjacent(b_mg) : nullptr;
+        if (wm && (bm || !b[0].defined())) {
             Epi e;
             e.accumulate = true;
+            e.a_colsum = static_cast<float*>(const_cast<void*>(bm));
             gemm(dm, xm, true, false, const_cast<void*>(wm), true, dt, e);
         } else {
-            for (int i = 0; i < 3; ++i) dw[i] = weight_grad(columns(dm, i * Ho, Ho), xm, w[i], w_mg[i], dt);
-        }
-        if (b[0].defined()) {
-            const bool all_b = b_mg[0].defined() && b_mg[1].defined() && b_mg[2].defined();
-            const void* bm = all_b ? adjacent(b_mg) : nullptr;
-            if (bm) {
-                check(api.colsum(dm.p, static_cast<float*>(const_cast<void*>(bm)), static_cast<int>(dm.rows),
-                                 static_cast<int>(dm.cols), dm.ld, dt, cur_stream()),
-                      "rb_colsum");
-            } else {
-                for (int i = 0; i < 3; ++i) db[i] = bias_grad(columns(dm, i * Ho, Ho), b[i], b_mg[i], dt);
+            for (int i = 0; i < 3; ++i) {
+                const Grads gr = param_grads(columns(dm, i * Ho, Ho), xm, w[i], w_mg[i], true, b[i], b_mg[i], true, dt);
+                dw[i] = gr.w;
+                db[i] = gr.b;
             }
         }
         notify({{&w[0], &w_mg[0]}, {&w[1], &w_mg[1]}, {&w[2], &w_mg[2]},

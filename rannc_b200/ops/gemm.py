@@ -29,7 +29,7 @@ class _Args(ctypes.Structure):
         ("b_row_shift", ctypes.c_int32), ("conv_shift", ctypes.c_int32 * 49),
         ("map_hp", ctypes.c_int32), ("map_wp", ctypes.c_int32), ("map_h", ctypes.c_int32),
         ("map_w", ctypes.c_int32), ("map_pad", ctypes.c_int32), ("wgrad_taps", ctypes.c_int32),
-        ("tile_n", ctypes.c_int32),
+        ("reserved_", ctypes.c_int32), ("a_colsum", ctypes.c_void_p), ("tile_n", ctypes.c_int32),
     ]
 
 
@@ -73,7 +73,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
          dgelu: bool = False, out: torch.Tensor | None = None, accumulate: bool = False,
          out_dtype: torch.dtype | None = None, alpha: float = 1.0, max_ctas: int = 0,
          rs_peers=None, rs_ld: int = 0, gather=None, conv=None, b_row_shift: int = 0,
-         row_map=None, wgrad_shifts=None, tile_n: int = 0) -> torch.Tensor:
+         row_map=None, wgrad_shifts=None, tile_n: int = 0,
+         a_colsum=None) -> torch.Tensor:
     """``out = epilogue(alpha * op(a) @ op(b))``.
 
     ``a`` is stored ``[M, K]`` (``trans_a=False``) or ``[K, M]`` (``trans_a=True``).
@@ -88,11 +89,14 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
     ``wgrad_shifts`` (``trans_b=False`` only): ``b`` is the padded activation ``[rows, C]`` and the result has one
     block of C columns per shift, ``a``'s product with the rows of ``b`` shifted by it (weight gradient of a
     convolution, all taps in one launch).
+    ``a_colsum`` (``trans_a=True`` only): fp32 vector to which the column sums of the stored ``a`` are added (the bias
+    gradient beside a weight gradient).
     ``row_map = (Hp, Wp, H, W, pad)``: the M rows are positions of a padded image grid; only the interior is
     stored, at the un-padded row index (``out`` has N_img * H * W rows).
     """
     if a.dim() == 2 and b.dim() == 2 and (out is None or out.dim() == 2) and rs_peers is None and gather is None and \
-            conv is None and row_map is None and wgrad_shifts is None and not b_row_shift and not tile_n:
+            conv is None and row_map is None and wgrad_shifts is None and not b_row_shift and not tile_n and \
+            a_colsum is None:
         odt = out_dtype or (out.dtype if out is not None else a.dtype)
         return _lib.host().product(a, b, trans_a, trans_b, bias, residual, aux_in, aux_out, gelu, dgelu, out, accumulate,
                                    odt != a.dtype, alpha, max_ctas)
@@ -173,6 +177,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         for i, sh in enumerate(conv["shifts"]):
             args.conv_shift[i] = int(sh)
     args.tile_n = int(tile_n)
+    args.a_colsum = _lib.ptr(a_colsum)
     if wgrad_shifts is not None:
         args.wgrad_taps = len(wgrad_shifts)
         args.conv_c = bc

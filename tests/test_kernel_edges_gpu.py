@@ -249,3 +249,27 @@ def test_attention_backward_blocks(B, S, H, p):
     for got, want in ((dq, qr.grad), (dk, kr.grad), (dv, vr.grad)):
         err = (got.double() - want).abs().max().item() / scale
         assert err < 6 * U[dt], err
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tile_n", [0, 64, 128])
+@pytest.mark.parametrize("M,N,K", [(2, 40, 1), (72, 8, 63), (130, 520, 200), (1160, 264, 1032), (4104, 1032, 2056),
+                                   (1024, 1024, 16384)])
+def test_gemm_column_sums_beside_weight_gradient(dtype, tile_n, M, N, K):
+    """Every row of dy is added exactly once, whichever tile, split and kernel variant does it."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops.gemm import gemm
+
+    torch.manual_seed(7)
+    dy = torch.zeros(K, (M + 7) // 8 * 8, device="cuda", dtype=dtype)[:, :M]
+    dy.copy_(torch.randn(K, M, device="cuda"))
+    x = torch.randn(K, N, device="cuda").to(dtype)
+    want, ref = dy.double().sum(0), dy.double().t() @ x.double()
+    for kw in (dict(out=torch.ones(M, N, device="cuda"), accumulate=True), dict()):
+        db = torch.full((M,), 2.0, device="cuda")
+        out = gemm(dy, x, trans_a=True, trans_b=False, tile_n=tile_n, a_colsum=db, **kw)
+        torch.cuda.synchronize()
+        assert _lib.read_error() == 0
+        steps = K / 16 * 2.0 ** -23
+        _near(db - 2.0, want, dtype, 0, steps)
+        _near(out, ref + (1.0 if kw else 0.0), dtype, 0 if kw else 1, steps)
