@@ -583,13 +583,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     const int valid = min(32, p.N - col);
                     const bool full_chunk = valid == 32;
                     float v[32];
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
+                    const uint64_t alpha2 = f2_pack(p.alpha, p.alpha);
                     if (has_bias) {
                         float t[32];
                         load32(reinterpret_cast<const InT*>(p.bias) + col, full_chunk, valid, t);
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] += t[j];
+                        for (int j = 0; j < 32; j += 2)
+                            f2_unpack(f2_fma(f2_pack_bits(r[j], r[j + 1]), alpha2, f2_pack(t[j], t[j + 1])), v[j], v[j + 1]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; j += 2)
+                            f2_unpack(f2_mul(f2_pack_bits(r[j], r[j + 1]), alpha2), v[j], v[j + 1]);
                     }
                     uint4 pre[4];   // the value before the activation, in storage precision
                     if (aux_out) {
@@ -601,7 +605,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     }
                     if (act_gelu) {
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
+                        for (int j = 0; j < 32; j += 2) gelu_erf2(v[j], v[j + 1]);
                     }
                     if (act_dgelu) {
                         if (!mbar_wait(abar, aux_phase, abort_flag)) {
@@ -619,7 +623,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         for (int g = 0; g < 4; ++g) {
                             const InT* e = reinterpret_cast<const InT*>(&x[g]);
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) v[g * 8 + j] *= gelu_erf_grad(to_f32<InT>(e[j]));
+                            for (int j = 0; j < 8; j += 2)
+                                gelu_erf_grad2(to_f32<InT>(e[j]), to_f32<InT>(e[j + 1]), v[g * 8 + j], v[g * 8 + j + 1]);
                         }
                     }
                     if (has_res && row_ok) {
@@ -676,7 +681,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     }
                 }
             }
-            if (lane == 0) tma_store_wait<0>();
+            // the staging memory must outlive the copies that read it; their writes are complete when the kernel is
+            if (lane == 0) tma_store_wait_read<0>();
         }
         for (int tile = p.staged ? p.num_tiles : tile0; tile < p.num_tiles; tile += tile_step, ++it) {
             int mb, nb, b, kb_begin, kb_end;
