@@ -309,9 +309,10 @@ __global__ void __launch_bounds__(LN_THREADS, 2)
 
 // dgamma[h] (+)= sum_blocks partial[b][0][h]; dbeta likewise.  grid = 2H/32 blocks of (32, 32): bound by the
 // latency of its loads, so a thread has ten of them at most, four in flight (296 x 2048 floats: 5.2 -> 3.7 us).
+template <typename OutT>
 __global__ void __launch_bounds__(1024)
-    ln_bwd_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dgamma,
-                         float* __restrict__ dbeta, int nblocks, int H, int accumulate) {
+    ln_bwd_reduce_kernel(const float* __restrict__ partial, OutT* __restrict__ dgamma,
+                         OutT* __restrict__ dbeta, int nblocks, int H, int accumulate) {
     __shared__ float red[32][33];
     const int col2 = blockIdx.x * 32 + threadIdx.x;  // in [0, 2H)
     float s = 0.f;
@@ -322,8 +323,8 @@ __global__ void __launch_bounds__(1024)
     if (threadIdx.y == 0) {
 #pragma unroll
         for (int w = 1; w < 32; ++w) s += red[w][threadIdx.x];
-        float* dst = col2 < H ? dgamma + col2 : dbeta + (col2 - H);
-        *dst = accumulate ? *dst + s : s;
+        OutT* dst = col2 < H ? dgamma + col2 : dbeta + (col2 - H);
+        *dst = from_f32<OutT>(accumulate ? to_f32<OutT>(*dst) + s : s);
     }
 }
 
@@ -419,6 +420,24 @@ extern "C" int rb_ln_fwd(const void* x, const void* residual, const void* gamma,
     }
 }
 
+namespace rb {
+static int ln_bwd_rows(const void* dy, const void* z, const void* gamma, const float* mean, const float* rstd, void* dz,
+                       void* dx, float* partial, int grid, int rows, int H, float p, uint64_t seed, uint64_t offset,
+                       int dtype, cudaStream_t st) {
+    if (dtype == 1) {
+        RB_LN_DISPATCH(__nv_bfloat16, launch_bwd, dy, z, gamma, mean, rstd, dz, dx, partial, grid, rows, p, seed, offset, st)
+    } else {
+        RB_LN_DISPATCH(__half, launch_bwd, dy, z, gamma, mean, rstd, dz, dx, partial, grid, rows, p, seed, offset, st)
+    }
+}
+template <typename OutT>
+static int ln_bwd_sums(const float* partial, void* dgamma, void* dbeta, int grid, int H, int accumulate, cudaStream_t st) {
+    ln_bwd_reduce_kernel<OutT><<<2 * H / 32, dim3(32, 32), 0, st>>>(partial, static_cast<OutT*>(dgamma),
+                                                                    static_cast<OutT*>(dbeta), grid, H, accumulate);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+}  // namespace rb
+
 // `partial` is scratch of rb_ln_bwd_grid(rows) * 2 * H floats.  dgamma / dbeta are
 // fp32 [H]; accumulate != 0 adds to them.
 extern "C" int rb_ln_bwd(const void* dy, const void* z, const void* gamma, const float* mean,
@@ -428,21 +447,21 @@ extern "C" int rb_ln_bwd(const void* dy, const void* z, const void* gamma, const
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (rows <= 0) return 0;
     const int grid = rb_ln_bwd_grid(rows);
-    int rc;
-    auto run = [&]() -> int {
-        if (dtype == 1) {
-            RB_LN_DISPATCH(__nv_bfloat16, launch_bwd, dy, z, gamma, mean, rstd, dz, dx, partial,
-                           grid, rows, p, seed, offset, st)
-        } else {
-            RB_LN_DISPATCH(__half, launch_bwd, dy, z, gamma, mean, rstd, dz, dx, partial, grid,
-                           rows, p, seed, offset, st)
-        }
-    };
-    rc = run();
+    const int rc = rb::ln_bwd_rows(dy, z, gamma, mean, rstd, dz, dx, partial, grid, rows, H, p, seed, offset, dtype, st);
+    return rc ? rc : rb::ln_bwd_sums<float>(partial, dgamma, dbeta, grid, H, accumulate, st);
+}
+
+// the same with dgamma / dbeta written in the 16-bit type of the operands (rounded from the fp32 sums)
+extern "C" int rb_ln_bwd16(const void* dy, const void* z, const void* gamma, const float* mean, const float* rstd,
+                           void* dz, void* dx, void* dgamma, void* dbeta, float* partial, int rows, int H, float p,
+                           uint64_t seed, uint64_t offset, int dtype, void* stream) {
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (rows <= 0) return 0;
+    const int grid = rb_ln_bwd_grid(rows);
+    const int rc = rb::ln_bwd_rows(dy, z, gamma, mean, rstd, dz, dx, partial, grid, rows, H, p, seed, offset, dtype, st);
     if (rc) return rc;
-    rb::ln_bwd_reduce_kernel<<<2 * H / 32, dim3(32, 32), 0, st>>>(partial, dgamma, dbeta, grid, H,
-                                                                 accumulate);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return dtype == 1 ? rb::ln_bwd_sums<__nv_bfloat16>(partial, dgamma, dbeta, grid, H, 0, st)
+                      : rb::ln_bwd_sums<__half>(partial, dgamma, dbeta, grid, H, 0, st);
 }
 
 // ---------------------------------------------------------------------------

@@ -41,6 +41,8 @@ struct Api {
                   float, uint64_t, uint64_t, int, void*);
     int (*ln_bwd)(const void*, const void*, const void*, const float*, const float*, void*, void*, float*, float*,
                   float*, int, int, float, uint64_t, uint64_t, int, int, void*);
+    int (*ln_bwd16)(const void*, const void*, const void*, const float*, const float*, void*, void*, void*, void*, float*,
+                    int, int, float, uint64_t, uint64_t, int, void*);
     int (*ln_bwd_grid)(int);
     int (*embed_fwd)(const long long*, const void*, void*, int, int, long long, int, void*);
     int (*embed_bwd)(const long long*, const void*, float*, int, int, long long, long long, int, void*);
@@ -392,23 +394,28 @@ struct LnNode : Node {
         const Tensor Z = z.unpack(), G = gamma.unpack(), M = mean.unpack(), R = rstd.unpack();
         const Tensor dy = dense(grads[0]);
         const int H = static_cast<int>(Z.size(-1)), rows = static_cast<int>(Z.numel() / H);
-        const bool flat = g_mg.defined() && b_mg.defined();
-        Tensor dz = at::empty(Z.sizes(), Z.options()), dx = dz, dg = g_mg, db = b_mg;
+        const bool flat = g_mg.defined() && b_mg.defined(), same = G.scalar_type() == Z.scalar_type();
+        Tensor dz = at::empty(Z.sizes(), Z.options()), dx = dz;
         if (p > 0) dx = at::empty(Z.sizes(), Z.options());
-        if (!flat) {
-            dg = f32({H}, Z);
-            db = f32({H}, Z);
-        }
         Tensor partial = f32({static_cast<int64_t>(api.ln_bwd_grid(rows)) * 2 * H}, Z);
-        check(api.ln_bwd(dy.data_ptr(), Z.data_ptr(), G.data_ptr(), mptr<float>(M), mptr<float>(R), dz.data_ptr(),
-                         p > 0 ? dx.data_ptr() : nullptr, mptr<float>(dg), mptr<float>(db), mptr<float>(partial), rows, H,
-                         static_cast<float>(p), seed, offset, flat ? 1 : 0, dt_code(Z), cur_stream()),
-              "rb_ln_bwd", 2);
-        if (flat) {
+        void* dx_drop = p > 0 ? dx.data_ptr() : nullptr;
+        if (flat || !same) {
+            Tensor dg = flat ? g_mg : f32({H}, Z), db = flat ? b_mg : f32({H}, Z);
+            check(api.ln_bwd(dy.data_ptr(), Z.data_ptr(), G.data_ptr(), mptr<float>(M), mptr<float>(R), dz.data_ptr(), dx_drop,
+                             mptr<float>(dg), mptr<float>(db), mptr<float>(partial), rows, H, static_cast<float>(p), seed,
+                             offset, flat ? 1 : 0, dt_code(Z), cur_stream()),
+                  "rb_ln_bwd", 2);
+            if (!flat) return {dx, dz, dg.to(G.scalar_type()), db.to(G.scalar_type())};
             notify({{&g_ref, &g_mg}, {&b_ref, &b_mg}});
             return {dx, dz, Tensor(), Tensor()};
         }
-        return {dx, dz, dg.to(G.scalar_type()), db.to(G.scalar_type())};
+        // gradients in the parameters' own type, rounded once from the fp32 sums by the reducing kernel
+        Tensor dg = at::empty({H}, G.options()), db = at::empty({H}, G.options());
+        check(api.ln_bwd16(dy.data_ptr(), Z.data_ptr(), G.data_ptr(), mptr<float>(M), mptr<float>(R), dz.data_ptr(), dx_drop,
+                           dg.data_ptr(), db.data_ptr(), mptr<float>(partial), rows, H, static_cast<float>(p), seed, offset,
+                           dt_code(Z), cur_stream()),
+              "rb_ln_bwd16", 2);
+        return {dx, dz, dg, db};
     }
 };
 
@@ -658,6 +665,14 @@ struct QkvNode : Node {
             e.accumulate = true;
             e.a_colsum = static_cast<float*>(const_cast<void*>(bm));
             gemm(dm, xm, true, false, const_cast<void*>(wm), true, dt, e);
+        } else if (!w_mg[0].defined() && !w_mg[1].defined() && !w_mg[2].defined() && !b_mg[0].defined() &&
+                   !b_mg[1].defined() && !b_mg[2].defined()) {
+            // no gradient buffers: still one product, whose row blocks are the three gradients
+            const Grads gr = param_grads(dm, xm, w[0], Tensor(), true, b[0], Tensor(), true, dt);
+            for (int i = 0; i < 3; ++i) {
+                dw[i] = gr.w.narrow(0, i * Ho, Ho);
+                if (gr.b.defined()) db[i] = gr.b.narrow(0, i * Ho, Ho);
+            }
         } else {
             for (int i = 0; i < 3; ++i) {
                 const Grads gr = param_grads(columns(dm, i * Ho, Ho), xm, w[i], w_mg[i], true, b[i], b_mg[i], true, dt);
@@ -866,6 +881,7 @@ void init(const std::unordered_map<std::string, uintptr_t>& fns, py::object erro
     set(api.colsum, "rb_colsum");
     set(api.ln_fwd, "rb_ln_fwd");
     set(api.ln_bwd, "rb_ln_bwd");
+    set(api.ln_bwd16, "rb_ln_bwd16");
     set(api.ln_bwd_grid, "rb_ln_bwd_grid");
     set(api.embed_fwd, "rb_embed_fwd");
     set(api.embed_bwd, "rb_embed_bwd");
