@@ -244,8 +244,9 @@ __global__ void __launch_bounds__(256)
 
 // y = act(x * scale + shift (+ residual)) with scale = rstd gamma and shift = beta - mean scale.  Every thread derives
 // its 8 channels' scale and shift from the two sums itself (a kernel of C threads in between cost 3 us and a launch for
-// a few hundred cycles of arithmetic); the first row of blocks also writes mean, rstd and the running statistics
-// (momentum, unbiased variance).
+// a few hundred cycles of arithmetic: 32 x 14 x 14 x 2048 with residual 13.6 + 3.1 -> 12.6 us, its backward below 18.6 +
+// 2.2 -> 17.3 us); the first row of blocks also writes mean, rstd and the running statistics (momentum, unbiased
+// variance).  One wave of blocks, four per SM: twice as many left a thread five rows to pay for its coefficients with.
 template <typename T, int BX>
 __global__ void __launch_bounds__(256)
     bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, const float* __restrict__ part,

