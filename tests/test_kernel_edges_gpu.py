@@ -273,3 +273,23 @@ def test_gemm_column_sums_beside_weight_gradient(dtype, tile_n, M, N, K):
         steps = K / 16 * 2.0 ** -23
         _near(db - 2.0, want, dtype, 0, steps)
         _near(out, ref + (1.0 if kw else 0.0), dtype, 0 if kw else 1, steps)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,K,N", [(2047, 264, 136), (2048, 264, 136), (4500, 1032, 520), (2304, 768, 768)])
+def test_linear_weight_gradient_both_sides_of_the_split(dtype, rows, K, N):
+    """Weight gradients of the parameter's own type, as one product and as split sums rounded at the end."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops import functional as RF
+
+    torch.manual_seed(8)
+    x = torch.randn(rows, K, device="cuda").to(dtype)
+    w = (torch.randn(N, K, device="cuda") * K ** -0.5).to(dtype).requires_grad_(True)
+    b = torch.randn(N, device="cuda").to(dtype).requires_grad_(True)
+    dy = torch.randn(rows, N, device="cuda").to(dtype)
+    RF.linear(x, w, b).backward(dy)
+    torch.cuda.synchronize()
+    assert _lib.read_error() == 0
+    steps = rows / 16 * 2.0 ** -23
+    _near(w.grad, dy.double().t() @ x.double(), dtype, 1, steps)
+    _near(b.grad, dy.double().sum(0), dtype, 1, steps)
