@@ -6,17 +6,6 @@
 
 namespace rb {
 
-__device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m, uint64_t* bar,
-                                            int c0, int c1, int c2, int c3) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5, %6}], [%2];"
-        :
-        : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)),
-          "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-        : "memory");
-}
-
 // Adds a [32 x 128] fp32 tile of this CTA's shared memory (128-byte swizzled rows) into global memory
 // through the tensor map: one bulk reduction instead of per-thread atomics; rows past the tensor's
 // extent are dropped by the copy engine.  Completion is tracked by the bulk async-group.

@@ -93,6 +93,8 @@ struct GemmKernelParams {
     // 1: the epilogue goes through shared memory and the copy engine (tensor maps of D and of the auxiliary
     // matrix); 0: every thread stores its own row (mapped rows, peers' memory, unaligned outputs)
     int staged;
+    // MN-major operands: 1: all 64-column chunks of a stage in one copy (tensor map [chunk][row][64]); 0: one copy each
+    int a_merged, b_merged;
     float* a_colsum;   // not null: column sums of the stored A (MN-major) are added here
 };
 
@@ -321,6 +323,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         const uint32_t fb = mapa_shared(smem_u32(&full[stage]), 0);
                         if (p.a_major == 0) {
                             tma_load_3d_pair(a_dst, &tmA, fb, ax, ay, b);
+                        } else if (p.a_merged) {
+                            tma_load_4d_pair(a_dst, &tmA, fb, 0, k0, m0 / 64, b);
                         } else {
 #pragma unroll
                             for (int c = 0; c < BM / 64; ++c)
@@ -328,6 +332,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         }
                         if (p.b_major == 0) {
                             tma_load_3d_pair(b_dst, &tmB, fb, k0, n0, b);
+                        } else if (p.b_merged) {
+                            int cx, cy;
+                            b_chunk(n0, cx, cy);
+                            tma_load_4d_pair(b_dst, &tmB, fb, 0, cy, cx / 64, b);
                         } else {
 #pragma unroll
                             for (int c = 0; c < Cfg<PAIR, BN>::B_ROWS / 64; ++c) {
@@ -340,6 +348,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         mbar_arrive_expect_tx(&full[stage], STAGE_BYTES);
                         if (p.a_major == 0) {
                             tma_load_3d(a_dst, &tmA, &full[stage], ax, ay, b);
+                        } else if (p.a_merged) {
+                            tma_load_4d(a_dst, &tmA, &full[stage], 0, k0, m0 / 64, b);
                         } else {
 #pragma unroll
                             for (int c = 0; c < BM / 64; ++c)
@@ -348,6 +358,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         }
                         if (p.b_major == 0) {
                             tma_load_3d(b_dst, &tmB, &full[stage], k0, n0, b);
+                        } else if (p.b_merged) {
+                            int cx, cy;
+                            b_chunk(n0, cx, cy);
+                            tma_load_4d(b_dst, &tmB, &full[stage], 0, cy, cx / 64, b);
                         } else {
 #pragma unroll
                             for (int c = 0; c < BN / 64; ++c) {
@@ -896,6 +910,26 @@ int make_tmap_4d_f32(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d
     return r == CUDA_SUCCESS ? 0 : -static_cast<int>(r) - 1000;
 }
 
+// An MN-major operand [rows, 64 * chunks] as [chunk][row][64]: box of `n` chunks x 64 rows, 128-byte swizzle
+static int make_tmap_chunks(CUtensorMap* out, const void* base, int fmt, uint64_t rows, uint64_t chunks, uint64_t batch,
+                            uint64_t row_bytes, uint64_t batch_bytes, uint32_t n) {
+    EncodeTiledFn fn = get_encode_fn();
+    if (!fn) return -100;
+    cuuint64_t dims[4] = {64, rows, chunks, batch};
+    cuuint64_t strides[3] = {row_bytes, 128, batch_bytes};
+    cuuint32_t box[4] = {64, BK, n, 1};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = CUDA_SUCCESS;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        r = fn(out, fmt == 1 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
+               const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_ERROR_INVALID_CONTEXT) break;
+        cudaFree(nullptr);   // a thread without a context yet: see make_tmap_3d
+    }
+    return r == CUDA_SUCCESS ? 0 : -static_cast<int>(r) - 1000;
+}
+
 // A matrix the GEMM's epilogue writes (or reads) in 32 x 32 blocks: 16-bit elements with 64-byte swizzled block
 // rows, fp32 with 128-byte ones.  Blocks are clipped to d0 x d1 by the copy engine.
 static int make_tmap_block32(CUtensorMap* out, const void* base, bool fp32, int fmt, uint64_t d0, uint64_t d1,
@@ -1171,23 +1205,39 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     int rc;
     const uint64_t sA = a->batch > 1 ? a->strideA * 2 : (a->a_major == 0 ? a->M : a->K) * a->lda * 2;
     const uint64_t sB = a->batch > 1 ? a->strideB * 2 : (a->b_major == 0 ? a->N : a->K) * a->ldb * 2;
+    // An MN-major operand of whole 64-column chunks is seen as [chunk][row][64], so that one copy brings all chunks of a
+    // stage.  The copies are issued one by one, and with two or four per operand and stage it was their number, not
+    // the bytes, that kept the tensor core waiting (57 % active): 8192 x 4096 x 8192, both operands MN-major, 438 ->
+    // 386 us, with fp32 accumulation 498 -> 397 us; 30720 x 1024 x 8192 457 -> 397 us.  A last chunk that the matrix
+    // fills only in part would read past its rows, and column blocks that straddle filter taps need a shift each:
+    // those keep a copy per chunk.
+    const int b_cols = pair ? 128 : tn;   // columns of B one CTA loads
+    p.a_merged = a->a_major == 1 && a->M % 64 == 0;
+    p.b_merged = a->b_major == 1 && (a->conv_taps > 0    ? a->conv_b_tap_cols % 64 == 0
+                                     : a->wgrad_taps > 0 ? a->conv_c % b_cols == 0
+                                                         : a->N % 64 == 0);
     if (a->conv_taps > 0)
         rc = make_tmap_3d(&tmA, a->A, a->in_dtype, a->conv_c, a->M, 1, a->lda * 2, a->M * a->lda * 2, BK, BM, 1);
     else if (a->a_major == 0)
         rc = make_tmap_3d(&tmA, a->A, a->in_dtype, a->K, a->M, a->batch, a->lda * 2, sA, BK, BM, 1);
+    else if (p.a_merged)
+        rc = make_tmap_chunks(&tmA, a->A, a->in_dtype, a->K, a->M / 64, a->batch, a->lda * 2, sA, BM / 64);
     else
         rc = make_tmap_3d(&tmA, a->A, a->in_dtype, a->M, a->K, a->batch, a->lda * 2, sA, 64, BK, 1);
     if (rc) return rc;
+    // stored columns of an MN-major B: with filter taps [conv_c rows, conv_taps * conv_b_tap_cols] (tap t's block starts
+    // at column t * conv_b_tap_cols), for a weight gradient the activation's conv_c
+    const uint64_t stored = a->conv_taps > 0    ? static_cast<uint64_t>(a->conv_taps) * a->conv_b_tap_cols
+                            : a->wgrad_taps > 0 ? a->conv_c
+                                                : a->N;
+    const uint64_t b_rows = a->conv_taps > 0 ? a->conv_c : a->K;
+    const uint64_t sB1 = a->conv_taps > 0 ? static_cast<uint64_t>(a->conv_c) * a->ldb * 2 : sB;
     if (a->b_major == 0)
-        rc = make_tmap_3d(&tmB, a->B, a->in_dtype, a->K, a->N, a->batch, a->ldb * 2, sB, BK, pair ? 128 : tn, 1);
-    else if (a->conv_taps > 0)
-        // the stored matrix is [conv_c rows, conv_taps * conv_b_tap_cols columns]: tap t's [conv_c, N] block
-        // starts at column t * conv_b_tap_cols
-        rc = make_tmap_3d(&tmB, a->B, a->in_dtype, static_cast<uint64_t>(a->conv_taps) * a->conv_b_tap_cols,
-                          a->conv_c, 1, a->ldb * 2, static_cast<uint64_t>(a->conv_c) * a->ldb * 2, 64, BK, 1);
+        rc = make_tmap_3d(&tmB, a->B, a->in_dtype, a->K, a->N, a->batch, a->ldb * 2, sB, BK, b_cols, 1);
+    else if (p.b_merged)
+        rc = make_tmap_chunks(&tmB, a->B, a->in_dtype, b_rows, stored / 64, a->batch, a->ldb * 2, sB1, b_cols / 64);
     else
-        rc = make_tmap_3d(&tmB, a->B, a->in_dtype, a->wgrad_taps > 0 ? a->conv_c : a->N, a->K, a->batch, a->ldb * 2, sB,
-                          64, BK, 1);
+        rc = make_tmap_3d(&tmB, a->B, a->in_dtype, stored, b_rows, a->batch, a->ldb * 2, sB1, 64, BK, 1);
     if (rc) return rc;
 
     // The staged epilogue wants outputs the copy engine can address: plain rows in this GPU's memory, 16-byte
