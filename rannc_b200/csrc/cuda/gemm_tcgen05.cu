@@ -563,6 +563,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             uint8_t* stage_buf = sEpi + (warp - 2) * EPI_STAGE_BYTES;
             uint64_t* abar = &aux_full[warp - 2];
             uint32_t aux_phase = 0;
+            uint32_t turn = 0;   // which half the next 16-bit block takes: counted over tiles, whose blocks may be odd in number
             const uint32_t sw64 = (lane >> 1) & 3, sw128 = lane & 7;
             constexpr bool OUT16 = sizeof(OutT) == 2;
             const bool add_out = !OUT16 && (accum || p.split_k > 1);
@@ -665,7 +666,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     __syncwarp();
                     uint8_t* dst = stage_buf;
                     if constexpr (OUT16) {
-                        if (!two_slots || (c & 1)) dst += 2048;
+                        if (!two_slots || (turn & 1)) dst += 2048;
+                        ++turn;
 #pragma unroll
                         for (int g = 0; g < 4; ++g)
                             *reinterpret_cast<uint4*>(dst + lane * 64 + ((g ^ sw64) << 4)) =
