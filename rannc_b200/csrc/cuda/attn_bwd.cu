@@ -241,6 +241,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
             key_ok ? (p.key_bias ? p.key_bias[static_cast<long long>(b) * p.S + key] * 1.4426950408889634f : 0.f)
                    : -INFINITY;
         const uint32_t key_hash = drop_key_hash(p.seed, key);
+        const uint64_t kbias2 = f2_pack(kbias, kbias), scale2 = f2_pack(p.scale_log2, p.scale_log2),
+                       keep2 = f2_pack(p.inv_keep, p.inv_keep);
         const long long bh = static_cast<long long>(b) * p.H + h;
         const uint32_t sw = r & 7;
         const uint32_t row_off = half * (SQ_BYTES / 2) + (r >> 3) * 1024 + sw * 128;
@@ -261,8 +263,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
             bar_sync_named(1, BWD_MATH);
             if (half == 0) {
                 // +inf for rows past the end of the sequence: their probabilities come out as exp2(-inf) = 0
-                s_lse[r] = n_lse_raw ? n_lse * 1.4426950408889634f : n_lse;
-                s_delta[r] = n_delta;
+                // both negated: the element-wise chain adds them
+                s_lse[r] = n_lse_raw ? n_lse * -1.4426950408889634f : -n_lse;
+                s_delta[r] = -n_delta;
                 s_rhash[r] = drop_row_hash(p.seed, b, h, q0 + r, p.H, p.S);
                 // issued here (volatile: not sunk to the use), consumed at the top of the next step
                 const int qn = q0 + BQ + r;
@@ -302,32 +305,39 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
                 }
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {
+                    // Bound by issue slots (twelve per element with dropout): what has a two-wide form uses it --
+                    // P = 2^(S scale + (bias - lse)), dS = P (mask dP / (1 - p) - delta).  32 x 512 x 16 heads with
+                    // bias and dropout: 240 -> 226 us.
                     float pd[8], ds[8];
 #pragma unroll
                     for (int hq = 0; hq < 2; ++hq) {
                         const int qb = half * 64 + c * 32 + g * 8 + hq * 4;
-                        const float4 ls4 = *reinterpret_cast<const float4*>(s_lse + qb);
-                        const float4 dl4 = *reinterpret_cast<const float4*>(s_delta + qb);
-                        const float lsv[4] = {ls4.x, ls4.y, ls4.z, ls4.w};
-                        const float dlv[4] = {dl4.x, dl4.y, dl4.z, dl4.w};
+                        const ulonglong2 ls4 = *reinterpret_cast<const ulonglong2*>(s_lse + qb);
+                        const ulonglong2 dl4 = *reinterpret_cast<const ulonglong2*>(s_delta + qb);
                         uint32_t rhv[4] = {0, 0, 0, 0};
                         if (p.thr32) {
                             const uint4 rh4 = *reinterpret_cast<const uint4*>(s_rhash + qb);
                             rhv[0] = rh4.x, rhv[1] = rh4.y, rhv[2] = rh4.z, rhv[3] = rh4.w;
                         }
 #pragma unroll
-                        for (int x = 0; x < 4; ++x) {
+                        for (int x = 0; x < 4; x += 2) {
                             const int e = g * 8 + hq * 4 + x;
-                            const float pr = exp2f(fmaf(__uint_as_float(sv[e]), p.scale_log2, kbias) - lsv[x]);
-                            const float dp = __uint_as_float(dv[e]);
+                            const uint64_t nlse = x == 0 ? ls4.x : ls4.y, ndelta = x == 0 ? dl4.x : dl4.y;
+                            float e0, e1;
+                            f2_unpack(f2_fma(f2_pack_bits(sv[e], sv[e + 1]), scale2, f2_add(kbias2, nlse)), e0, e1);
+                            const float p0 = ex2_approx(e0), p1 = ex2_approx(e1);
+                            uint64_t t;
                             if (p.thr32) {
-                                const bool keep = drop_keep(rhv[x], key_hash, p.thr32);
-                                pd[hq * 4 + x] = keep ? pr : 0.f;
-                                ds[hq * 4 + x] = pr * fmaf(keep ? dp : 0.f, p.inv_keep, -dlv[x]);
+                                const bool k0 = drop_keep(rhv[x], key_hash, p.thr32), k1 = drop_keep(rhv[x + 1], key_hash, p.thr32);
+                                pd[hq * 4 + x] = k0 ? p0 : 0.f;
+                                pd[hq * 4 + x + 1] = k1 ? p1 : 0.f;
+                                t = f2_fma(f2_pack_bits(k0 ? dv[e] : 0u, k1 ? dv[e + 1] : 0u), keep2, ndelta);
                             } else {
-                                pd[hq * 4 + x] = pr;
-                                ds[hq * 4 + x] = pr * (dp - dlv[x]);
+                                pd[hq * 4 + x] = p0;
+                                pd[hq * 4 + x + 1] = p1;
+                                t = f2_add(f2_pack_bits(dv[e], dv[e + 1]), ndelta);
                             }
+                            f2_unpack(f2_mul(f2_pack(p0, p1), t), ds[hq * 4 + x], ds[hq * 4 + x + 1]);
                         }
                     }
                     pk[c][g] = make_uint4(pack2<T>(pd[0], pd[1]), pack2<T>(pd[2], pd[3]), pack2<T>(pd[4], pd[5]),
