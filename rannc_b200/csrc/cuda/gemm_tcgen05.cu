@@ -13,7 +13,7 @@
 // Structure: persistent CTAs (one per SM), 128 x 256 output tile, K step 64,
 // 4-stage TMA->smem ring, fp32 accumulators double-buffered in TMEM (2 x 256
 // columns) so the epilogue of tile i overlaps the main loop of tile i+1.
-// Warp 0 = TMA producer, warp 1 = MMA issuer, warps 2..9 = epilogue (with K = 1024 a tile's main loop is
+// Warp 0 = TMA producer, warp 1 = MMA issuer, warps 2..9 = epilogue, warps 10 and 11 = column sums of A where asked for (with K = 1024 a tile's main loop is
 // only 16 k steps, and four warps could not drain a 128 x 256 accumulator in that time); the epilogue writes through shared memory and
 // the copy engine.
 //
@@ -558,8 +558,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             // lines, 32 cycles each -- for two 16-bit outputs alone as long as the main loop.  Rows therefore go
             // to the staging block (conflict-free by the swizzle) and the copy engine moves 32 x 32 blocks; it
             // also clips them to M x N, adds fp32 blocks to D (accumulation, split K) and fetches the auxiliary
-            // block one step ahead.  16384 x 4096 x 1024 with bias, GELU and the value before it: 155 -> 142 us;
-            // 8192 x 30528 x 1024: 426 -> 386 us; weight gradient 4096 x 1024 x 16384: 122 -> 116 us.
+            // block one step ahead.  16384 x 4096 x 1024 with bias, GELU and the value before it: 155 -> 142 us (137 with
+            // the packed arithmetic below); 8192 x 30528 x 1024: 426 -> 386 us; weight gradient 4096 x 1024 x 16384:
+            // 122 -> 116 us.  A block of 128 rows per four warps (a quarter of the copies, two barriers a block) was
+            // slower: 137 -> 142 us.
             uint8_t* stage_buf = sEpi + (warp - 2) * EPI_STAGE_BYTES;
             uint64_t* abar = &aux_full[warp - 2];
             uint32_t aux_phase = 0;
@@ -1209,8 +1211,8 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     const uint64_t sB = a->batch > 1 ? a->strideB * 2 : (a->b_major == 0 ? a->N : a->K) * a->ldb * 2;
     // An MN-major operand of whole 64-column chunks is seen as [chunk][row][64], so that one copy brings all chunks of a
     // stage.  The copies are issued one by one, and with two or four per operand and stage it was their number, not
-    // the bytes, that kept the tensor core waiting (57 % active): 8192 x 4096 x 8192, both operands MN-major, 438 ->
-    // 386 us, with fp32 accumulation 498 -> 397 us; 30720 x 1024 x 8192 457 -> 397 us.  A last chunk that the matrix
+    // the bytes, that kept the tensor core waiting (57 % active): 8192 x 4096 x 8192, both operands MN-major, 421 ->
+    // 391 us, with fp32 accumulation 434 -> 402 us; 1024 x 9216 x 26912 445 -> 366 us.  A last chunk that the matrix
     // fills only in part would read past its rows, and column blocks that straddle filter taps need a shift each:
     // those keep a copy per chunk.
     const int b_cols = pair ? 128 : tn;   // columns of B one CTA loads

@@ -349,7 +349,7 @@ class _Conv2d(torch.autograd.Function):
         the GEMM reads the zero-padded activation tap by tap (a row shift per tap), so neither the k*k-fold
         ``im2col`` matrix nor its adjoint is ever written.  The product is taken over the PADDED grid (border
         positions are computed and dropped), so small feature maps pay more in extra arithmetic than the gather
-        costs in traffic: ``conv_implicit_max_overhead`` bounds (Hp * Wp) / (H * W)."""
+        costs in traffic: ``conv_implicit_max_overhead`` bounds (H + 2 pad)(W + 2 pad) / (H W)."""
         if not (k > 1 and k % 2 == 1 and stride == 1 and padding == (k - 1) // 2 and Ci % 64 == 0 and Co % 64 == 0
                 and k * k <= 49 and bool(conf("conv_implicit_gemm"))):
             return False
