@@ -10,12 +10,12 @@
 //   dgrad    dX = dY W   : A = dY (K-major),  B = W  (MN-major)
 //   wgrad    dW = dY^T X : A = dY (MN-major), B = X  (MN-major)
 //
-// Structure: persistent CTAs (one per SM), 128 x 256 output tile, K step 64,
-// 4-stage TMA->smem ring, fp32 accumulators double-buffered in TMEM (2 x 256
+// Structure: persistent CTAs (one per SM), 128 x 256 output tile (128 or 64 columns for small problems), K step 64,
+// 4-stage TMA->smem ring (6 or 8 with narrower tiles), fp32 accumulators double-buffered in TMEM (2 x 256
 // columns) so the epilogue of tile i overlaps the main loop of tile i+1.
-// Warp 0 = TMA producer, warp 1 = MMA issuer, warps 2..9 = epilogue, warps 10 and 11 = column sums of A where asked for (with K = 1024 a tile's main loop is
-// only 16 k steps, and four warps could not drain a 128 x 256 accumulator in that time); the epilogue writes through shared memory and
-// the copy engine.
+// Warp 0 = TMA producer, warp 1 = MMA issuer, warps 2..9 = epilogue, warps 10 and 11 = column sums of A where
+// asked for (with K = 1024 a tile's main loop is only 16 k steps, and four warps could not drain a 128 x 256
+// accumulator in that time); the epilogue writes through shared memory and the copy engine.
 //
 // PAIR variant (cta_group::2): two CTAs of a cluster -- the two SMs of a TPC -- share a 256 x 256 tile.
 // Each CTA loads its own 128 rows of A and HALF of the B tile (so a k step moves 32 KiB per SM instead

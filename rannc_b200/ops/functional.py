@@ -330,16 +330,15 @@ def _conv_weight(w):
 
 
 class _Conv2d(torch.autograd.Function):
-    """Convolution as a tcgen05 GEMM over channels-last activations: the [N*H*W, C] view itself for 1x1
-    kernels, the ``im2col`` matrix otherwise; input gradient through the adjoint gather, weight gradient as
+    """Convolution as a tcgen05 GEMM over channels-last activations: the picked pixels for strided 1x1 kernels
+    (unstrided ones are linear layers, see ``conv2d``), the padded image or the ``im2col`` matrix otherwise; input
+    gradient through the adjoint gather, weight gradient as
     one GEMM accumulated into the fp32 gradient buffer."""
 
     @staticmethod
     def _operand(x4, k, s, pad):
         N, H, W, C = x4.shape
         if k == 1 and pad == 0:
-            if s == 1:
-                return x4.reshape(N * H * W, C)
             return x4[:, ::s, ::s, :].contiguous().reshape(-1, C)
         return K.im2col(x4, k, s, pad)
 
@@ -463,11 +462,8 @@ class _Conv2d(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             da = gemm(dy2, _conv_weight(w), trans_b=False)
             if k == 1 and padding == 0:
-                if stride == 1:
-                    dx4 = da.view(N, H, W, C)
-                else:
-                    dx4 = torch.zeros(N, H, W, C, dtype=da.dtype, device=da.device)
-                    dx4[:, ::stride, ::stride, :] = da.view(N, -1, dx4[:, ::stride, ::stride, :].shape[2], C)
+                dx4 = torch.zeros(N, H, W, C, dtype=da.dtype, device=da.device)
+                dx4[:, ::stride, ::stride, :] = da.view(N, -1, dx4[:, ::stride, ::stride, :].shape[2], C)
             else:
                 dx4 = K.col2im(da, N, H, W, C, k, stride, padding)
             dx = dx4.permute(0, 3, 1, 2)
