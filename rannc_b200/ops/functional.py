@@ -332,14 +332,12 @@ def _conv_weight(w):
 class _Conv2d(torch.autograd.Function):
     """Convolution as a tcgen05 GEMM over channels-last activations: the picked pixels for strided 1x1 kernels
     (unstrided ones are linear layers, see ``conv2d``), the padded image or the ``im2col`` matrix otherwise; input
-    gradient through the adjoint gather, weight gradient as
-    one GEMM accumulated into the fp32 gradient buffer."""
+    gradient by the same kernel or through the adjoint gather, weight gradient as one GEMM."""
 
     @staticmethod
     def _operand(x4, k, s, pad):
-        N, H, W, C = x4.shape
         if k == 1 and pad == 0:
-            return x4[:, ::s, ::s, :].contiguous().reshape(-1, C)
+            return x4[:, ::s, ::s, :].contiguous().reshape(-1, x4.shape[-1])
         return K.im2col(x4, k, s, pad)
 
     @staticmethod
