@@ -581,18 +581,19 @@ const void* adjacent(const Tensor* t) {
     }
     return p;
 }
-Mat stacked(const Tensor* w, const Tensor& cat) {   // the three projection weights as one [3 Ho, hid] matrix
-    if (const void* p = adjacent(w)) {
-        if (aligned16(p) && w[0].size(1) % 8 == 0) {
-            Mat m;
-            m.keep = w[0];
-            m.p = p;
-            m.rows = 3 * w[0].size(0);
-            m.cols = m.ld = w[0].size(1);
-            return m;
-        }
-    }
-    return mat(cat.defined() ? cat : at::cat({w[0].detach(), w[1].detach(), w[2].detach()}, 0));
+// The three projection weights as one [3 Ho, hid] matrix: in place where they lie back to back, else a stack made for
+// this use (`copied`).  A stack is never kept from one call for another: nothing tells when the values it was made of
+// change (an update through .data or by a kernel leaves no trace on the parameter).
+Mat stacked(const Tensor* w, bool& copied) {
+    const void* p = adjacent(w);
+    copied = !(p && aligned16(p) && w[0].size(1) % 8 == 0);
+    if (copied) return mat(at::cat({w[0].detach(), w[1].detach(), w[2].detach()}, 0));
+    Mat m;
+    m.keep = w[0];
+    m.p = p;
+    m.rows = 3 * w[0].size(0);
+    m.cols = m.ld = w[0].size(1);
+    return m;
 }
 void attn_args(RbAttnArgs& a, const Tensor& qkv, const Tensor& o, const Tensor& lse, const Tensor& bias, int64_t B, int64_t S,
                int64_t H, double scale, double p, uint64_t seed, uint64_t offset) {
@@ -622,14 +623,14 @@ void attn_args(RbAttnArgs& a, const Tensor& qkv, const Tensor& o, const Tensor& 
     a.offset = offset;
 }
 struct QkvNode : Node {
-    SavedVariable x, qkv, o, lse, bias;
-    Tensor w[3], b[3], w_mg[3], b_mg[3], cat;
+    SavedVariable x, qkv, o, lse, bias, stack;   // stack: the weights, where the forward had to copy them together
+    Tensor w[3], b[3], w_mg[3], b_mg[3];
     int64_t B = 0, S = 0, H = 0;
     double p = 0, scale = 1;
     uint64_t seed = 0, offset = 0;
     RB_NODE("RbQkvAttentionBackward")
     void release_variables() override {
-        for (SavedVariable* s : {&x, &qkv, &o, &lse, &bias}) s->reset_data();
+        for (SavedVariable* s : {&x, &qkv, &o, &lse, &bias, &stack}) s->reset_data();
     }
     variable_list run(variable_list&& grads) {
         const Tensor X = x.unpack(), Q = qkv.unpack(), O = o.unpack(shared_from_this()), L = lse.unpack(), kb = bias.unpack();
@@ -664,7 +665,9 @@ struct QkvNode : Node {
         Tensor dx, dw[3], db[3];
         if (task_should_compute_output(0)) {
             dx = at::empty(X.sizes(), X.options());
-            gemm(dm, stacked(w, cat), false, false, dx.data_ptr(), false, dt, Epi());
+            const Tensor st = stack.unpack();
+            bool copied;
+            gemm(dm, st.defined() ? mat(st) : stacked(w, copied), false, false, dx.data_ptr(), false, dt, Epi());
         }
         // adjacent fp32 gradient buffers: one weight-gradient GEMM (with the column sums of the biases) serves all three
         // projections
@@ -697,15 +700,17 @@ struct QkvNode : Node {
     }
 };
 
-// cat_w / cat_b: the stacked projections when they are not adjacent in memory and the caller keeps such a stack (of
-// parameters that come and go it keeps none: they are stacked anew for every use)
+// streamed: parameters that come and go; when they have to be stacked, the backward does it again instead of keeping the
+// forward's copy on the device in between
 Tensor qkv_attention(const Tensor& x, const std::vector<Tensor>& ws, const std::vector<OptTensor>& bs, const OptTensor& key_bias,
                      double p, double scale, int64_t H, uint64_t seed, uint64_t offset, const std::vector<OptTensor>& w_mgs,
-                     const std::vector<OptTensor>& b_mgs, const OptTensor& cat_w, const OptTensor& cat_b) {
+                     const std::vector<OptTensor>& b_mgs, bool streamed) {
     const Tensor w[3] = {ws[0], ws[1], ws[2]}, b[3] = {opt(bs[0]), opt(bs[1]), opt(bs[2])};
     const bool req = wants_grad({&x, &w[0], &b[0], &w[1], &b[1], &w[2], &b[2]});
     const int64_t B = x.size(0), S = x.size(1), Ho = w[0].size(0);
-    Tensor xc, qkv, o, lse, bias_cat, kb = opt(key_bias), cat = opt(cat_w);
+    Tensor xc, qkv, o, lse, bias_cat, kb = opt(key_bias);
+    Mat wm;
+    bool copied;
     {
         at::NoGradGuard off;
         xc = dense(x);
@@ -716,11 +721,12 @@ Tensor qkv_attention(const Tensor& x, const std::vector<Tensor>& ws, const std::
         if (b[0].defined()) {
             e.bias = adjacent(b);
             if (!e.bias) {
-                bias_cat = cat_b.has_value() ? *cat_b : at::cat({b[0].detach(), b[1].detach(), b[2].detach()}, 0);
+                bias_cat = at::cat({b[0].detach(), b[1].detach(), b[2].detach()}, 0);
                 e.bias = bias_cat.data_ptr();
             }
         }
-        gemm(rows_of(xc), stacked(w, cat), false, true, qkv.data_ptr(), false, dt_code(x), e);
+        wm = stacked(w, copied);
+        gemm(rows_of(xc), wm, false, true, qkv.data_ptr(), false, dt_code(x), e);
         RbAttnArgs a;
         attn_args(a, qkv, o, lse, kb, B, S, H, scale, p, seed, offset);
         check(api.attn_fwd(&a, cur_stream()), "rb_attn_fwd");
@@ -740,7 +746,7 @@ Tensor qkv_attention(const Tensor& x, const std::vector<Tensor>& ws, const std::
             n->w_mg[i] = opt(w_mgs[i]);
             n->b_mg[i] = opt(b_mgs[i]);
         }
-        n->cat = cat;
+        if (copied && !streamed) n->stack = SavedVariable(wm.keep, false);
         n->B = B;
         n->S = S;
         n->H = H;
@@ -751,8 +757,6 @@ Tensor qkv_attention(const Tensor& x, const std::vector<Tensor>& ws, const std::
     }
     return o;
 }
-// whether the three lie back to back in one storage
-bool are_adjacent(const std::vector<Tensor>& t) { return t.size() == 3 && adjacent(t.data()) != nullptr; }
 
 // ------------------------------------------------------------------------------------------------ batch norm
 Tensor nhwc(const Tensor& t) { return t.contiguous(at::MemoryFormat::ChannelsLast); }
@@ -944,6 +948,5 @@ PYBIND11_MODULE(_host, m) {
     RB_DEF(embedding);
     RB_DEF(cross_entropy);
     RB_DEF(qkv_attention);
-    RB_DEF(are_adjacent);
     RB_DEF(batch_norm_act);
 }

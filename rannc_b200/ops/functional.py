@@ -247,29 +247,6 @@ def cross_entropy(logits, labels, num_classes=None, ignore_index: int = -100, we
 
 
 # ----------------------------------------------------------------------------- fused QKV projection + attention
-param_epoch = 0  # bumped whenever parameter values change in place (optimizer step, parameter sync)
-_cat_cache = {}
-
-
-def bump_param_epoch() -> None:
-    global param_epoch
-    param_epoch += 1
-
-
-def _cat_params(tensors):
-    """Concatenation of a few parameters along dim 0, cached until the parameters next change."""
-    key = tuple(id(t) for t in tensors)
-    volatile = any(getattr(t, "_rannc_host", None) is not None for t in tensors)
-    hit = None if volatile else _cat_cache.get(key)
-    if hit is not None and hit[0] == param_epoch and hit[2] == tuple(t.data_ptr() for t in tensors):
-        return hit[1]
-    with torch.no_grad():
-        cat = torch.cat([t.detach() for t in tensors], 0)
-    if not volatile:
-        _cat_cache[key] = (param_epoch, cat, tuple(t.data_ptr() for t in tensors))
-    return cat
-
-
 def qkv_attention(x, wq, bq, wk, bk, wv, bv, attn_mask=None, dropout_p: float = 0.0, is_causal: bool = False,
                   scale=None, num_heads: int = 1):
     """Self-attention block input side: the three projections of ``x`` [B, S, hid] and the attention itself.
@@ -292,13 +269,10 @@ def qkv_attention(x, wq, bq, wk, bk, wv, bv, attn_mask=None, dropout_p: float = 
         # [B, S, 3, H, D] output and write dq / dk / dv into one buffer that the single dgrad GEMM consumes
         h = _host()
         ws, bs = [wq, wk, wv], [bq, bk, bv]
-        # parameters that are streamed in and out are stacked anew by every use, without a copy that outlives it
-        volatile = any(getattr(t, "_rannc_host", None) is not None or getattr(t, "_rannc_window", False) for t in ws)
-        cat_w = None if volatile or h.are_adjacent(ws) else _cat_params(ws)
-        cat_b = None if volatile or bq is None or h.are_adjacent(bs) else _cat_params(bs)
+        streamed = any(getattr(t, "_rannc_host", None) is not None or getattr(t, "_rannc_window", False) for t in ws)
         seed, offset = rng.next() if dropout_p > 0.0 else (0, 0)
         return h.qkv_attention(x, ws, bs, key_bias, float(dropout_p), sc, num_heads, seed, offset,
-                               [_main_grad(t) for t in ws], [_main_grad(t) for t in bs], cat_w, cat_b)
+                               [_main_grad(t) for t in ws], [_main_grad(t) for t in bs], streamed)
     q = linear(x, wq, bq).view(B, S, num_heads, D).transpose(1, 2)
     k = linear(x, wk, bk).view(B, S, num_heads, D).transpose(1, 2)
     v = linear(x, wv, bv).view(B, S, num_heads, D).transpose(1, 2)
@@ -313,20 +287,15 @@ def _nhwc(x):
 
 
 def _conv_weight(w):
-    """[Co, kh * kw * Ci] with the taps outermost (the order ``im2col`` produces), cached until the
-    parameters next change.  A 1x1 kernel is a free view."""
+    """[Co, kh * kw * Ci] with the taps outermost (the order ``im2col`` produces): a view for 1x1 and channels-last
+    filters, otherwise a copy made for this use.  It is not kept: nothing tells when the filter's values change (an
+    update through ``.data`` or by a kernel leaves no trace on the parameter), and every micro-batch in flight
+    would hold one as large as the filter."""
     Co, Ci, kh, kw = w.shape
-    if kh == 1 and kw == 1:
-        return w.detach().reshape(Co, Ci)
-    key = ("conv", id(w))
-    hit = _cat_cache.get(key)
-    if hit is not None and hit[0] == param_epoch and hit[2] == (w.data_ptr(), tuple(w.shape)):
-        return hit[1]
-    with torch.no_grad():
-        w2 = w.detach().permute(0, 2, 3, 1).reshape(Co, kh * kw * Ci).contiguous()
-    # (an id and an address can both recur once the earlier tensor is gone: the shape is part of the check)
-    _cat_cache[key] = (param_epoch, w2, (w.data_ptr(), tuple(w.shape)))
-    return w2
+    taps_last = w.detach().permute(0, 2, 3, 1)
+    if not taps_last.is_contiguous() and K.pack_taps_ok(w):
+        return K.pack_taps(w.detach())
+    return taps_last.reshape(Co, kh * kw * Ci)
 
 
 class _Conv2d(torch.autograd.Function):

@@ -289,6 +289,24 @@ def pad_nhwc(x_nhwc, pad: int):
     return out
 
 
+PACK_MAX_TAPS = 1024   # 16 channels of a filter of that many taps still fit the kernel's shared memory
+
+
+def pack_taps_ok(w) -> bool:
+    """Whether ``pack_taps`` takes this [Co, Ci, k, k] filter."""
+    return (w.is_cuda and w.dtype in (torch.bfloat16, torch.float16) and w.is_contiguous() and w.shape[1] % 8 == 0 and
+            w.data_ptr() % 16 == 0 and w.shape[2] * w.shape[3] <= PACK_MAX_TAPS and w.numel() > 0)
+
+
+def pack_taps(w):
+    """[Co, Ci, k, k] (contiguous, 16-bit) -> [Co, k * k * Ci], taps outermost."""
+    Co, Ci, kh, kw = w.shape
+    out = torch.empty(Co, kh * kw * Ci, dtype=w.dtype, device=w.device)
+    _lib.check(_lib.lib().rb_pack_taps(_lib.vp(w), _lib.vp(out), c_int(Co), c_int(Ci), c_int(kh * kw),
+                                       _lib.stream_ptr()), "rb_pack_taps")
+    return out
+
+
 def wgrad_fold(dw2d, dst, taps: int):
     """fp32 [Co, taps * Ci] into the contiguous [Co, Ci, k, k] tensor ``dst``: added when it is fp32, written
     (rounded) when it is 16-bit."""

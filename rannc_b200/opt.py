@@ -27,7 +27,6 @@ from typing import Dict, List, Optional
 
 import torch
 
-from .ops import functional as RF
 from .parallel import comm
 from .utils.config import conf
 from .utils.log import get_logger
@@ -347,7 +346,6 @@ def patch_optimizer(module, optimizer):
                 fused_step(ctrl if isinstance(ctrl, torch.Tensor) else None, only=plain)
                 if storage.zero:
                     storage.allgather_params_zero(only=plain)
-            RF.bump_param_epoch()
             mod._after_step()
             return None
         use_fused = optimizer._rannc_kind is not None and all(
@@ -370,7 +368,6 @@ def patch_optimizer(module, optimizer):
                         g.scatter_local(g.flat_param, g.flat_master)
         if storage.zero:
             storage.allgather_params_zero()
-        RF.bump_param_epoch()
         if mod is not None:
             mod._after_step()
         return loss

@@ -499,7 +499,6 @@ def compare_with_collectives(module, optimizer, run_step) -> float:
                     fs.v.copy_(mom[1])
                 fs.step = mom[2]
         RF.rng.set_state(rng)
-        RF.bump_param_epoch()
 
     torch.cuda.synchronize()
     comm.barrier()

@@ -1,0 +1,89 @@
+"""What the operators promise beside their numbers: current weights, any batch and filter size, operand types, storage of
+gradients, reproducibility on request, other threads' progress."""
+import gc
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+from rannc_b200.ops import functional as RF
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+def _rel(got, want):
+    want = want.double()
+    return float((got.double() - want).norm() / want.norm().clamp_min(1e-30))
+
+
+def _randn(*shape, std=1.0, dtype=BF):
+    return (torch.randn(*shape, device="cuda") * std).to(dtype)
+
+
+# ------------------------------------------------------------------------------------------ current weights
+def _attention_ref(x, ws, bs, heads):
+    B, S, _ = x.shape
+    q, k, v = (F.linear(x.double(), w.double(), b.double()).view(B, S, heads, 64).transpose(1, 2) for w, b in zip(ws, bs))
+    return (torch.softmax(q @ k.transpose(2, 3) / 8, -1) @ v).transpose(1, 2).reshape(B, S, heads * 64)
+
+
+def _attention(x, ws, bs, heads):
+    return RF.qkv_attention(x, ws[0], bs[0], ws[1], bs[1], ws[2], bs[2], num_heads=heads)
+
+
+@pytest.mark.parametrize("through_data", [False, True])
+def test_projections_changed_in_place_are_seen(through_data):
+    """16-bit rounding of the projections, probabilities and outputs: 2^-8 each, three of them."""
+    torch.manual_seed(0)
+    x = _randn(2, 33, 128)
+    ws, bs = [_randn(128, 128, std=128 ** -0.5) for _ in range(3)], [_randn(128, std=0.1) for _ in range(3)]
+    for _ in range(3):
+        assert _rel(_attention(x, ws, bs, 2), _attention_ref(x, ws, bs, 2)) < 3 * 2.0 ** -8
+        for t in ws + bs:
+            (t.data if through_data else t).add_(torch.randn_like(t) * 0.1)
+
+
+@pytest.mark.parametrize("through_data", [False, True])
+def test_filters_changed_in_place_are_seen(through_data):
+    torch.manual_seed(1)
+    x, w = _randn(2, 64, 12, 12), _randn(72, 64, 3, 3, std=0.05)
+    for stride in (1, 2):
+        for _ in range(3):
+            xg = x.clone().requires_grad_(True)
+            y = RF.conv2d(xg, w, None, stride, 1)
+            xr = x.double().requires_grad_(True)
+            ref = F.conv2d(xr, w.double(), None, stride, 1)
+            assert _rel(y, ref) < 2.0 ** -8
+            y.backward(torch.ones_like(y))
+            ref.backward(torch.ones_like(ref))
+            # the gathered path rounds each of the nine taps' shares before it sums them
+            assert _rel(xg.grad, xr.grad) < 9 * 2.0 ** -9
+            (w.data if through_data else w).add_(torch.randn_like(w) * 0.05)
+
+
+def test_weights_at_a_freed_tensors_address_are_their_own():
+    torch.manual_seed(2)
+    x, xi = _randn(1, 16, 128), _randn(1, 64, 8, 8)
+    for _ in range(12):
+        ws, bs = [_randn(128, 128, std=128 ** -0.5) for _ in range(3)], [_randn(128, std=0.1) for _ in range(3)]
+        assert _rel(_attention(x, ws, bs, 2), _attention_ref(x, ws, bs, 2)) < 3 * 2.0 ** -8
+        w = _randn(64, 64, 3, 3, std=0.05)
+        assert _rel(RF.conv2d(xi, w, None, 1, 1), F.conv2d(xi.double(), w.double(), None, 1, 1)) < 2.0 ** -8
+        del ws, bs, w
+        gc.collect()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("Co,Ci", [(1, 8), (3, 264), (130, 256), (5, 72)])
+@pytest.mark.parametrize("k", [2, 3, 9, 10, 18, 19, 32])
+def test_filters_packed_tap_by_tap(dtype, Co, Ci, k):
+    """Each channel-block width of the kernel, last blocks of a few channels; a channels-last filter is read in place."""
+    torch.manual_seed(6)
+    w = _randn(Co, Ci, k, k, dtype=dtype)
+    want = w.permute(0, 2, 3, 1).reshape(Co, -1)
+    got = RF._conv_weight(w)
+    assert RF.K.pack_taps_ok(w) and torch.equal(got, want)
+    cl = w.to(memory_format=torch.channels_last)
+    assert RF._conv_weight(cl).data_ptr() == cl.data_ptr() and torch.equal(RF._conv_weight(cl), want)
+    assert torch.equal(RF._conv_weight(w[:, :, 1:, 1:]), w[:, :, 1:, 1:].permute(0, 2, 3, 1).reshape(Co, -1))
