@@ -307,6 +307,13 @@ def pack_taps(w):
     return out
 
 
+def wgrad_fold_ok(dst) -> bool:
+    """Whether ``wgrad_fold`` takes this [Co, Ci, k, k] destination: one grid row per filter, and a row of 132 floats
+    per tap within 48 KiB of shared memory (filters up to 9 x 9)."""
+    return (dst.is_cuda and dst.is_contiguous() and dst.shape[0] <= 65535 and dst.shape[2] * dst.shape[3] <= 93 and
+            dst.dtype in (torch.bfloat16, torch.float16, torch.float32))
+
+
 def wgrad_fold(dw2d, dst, taps: int):
     """fp32 [Co, taps * Ci] into the contiguous [Co, Ci, k, k] tensor ``dst``: added when it is fp32, written
     (rounded) when it is 16-bit."""

@@ -13,7 +13,7 @@ BF = torch.bfloat16
 
 
 def _rel(got, want):
-    want = want.double()
+    got, want = got.detach(), want.detach().double()
     return float((got.double() - want).norm() / want.norm().clamp_min(1e-30))
 
 
@@ -87,3 +87,23 @@ def test_filters_packed_tap_by_tap(dtype, Co, Ci, k):
     cl = w.to(memory_format=torch.channels_last)
     assert RF._conv_weight(cl).data_ptr() == cl.data_ptr() and torch.equal(RF._conv_weight(cl), want)
     assert torch.equal(RF._conv_weight(w[:, :, 1:, 1:]), w[:, :, 1:, 1:].permute(0, 2, 3, 1).reshape(Co, -1))
+
+
+# ------------------------------------------------------------------------------------------ filter sizes
+@pytest.mark.parametrize("flat", [False, True])
+@pytest.mark.parametrize("k,stride,pad", [(9, 1, 4), (10, 1, 0), (11, 4, 2), (16, 16, 0)])
+def test_large_filters(k, stride, pad, flat):
+    torch.manual_seed(3)
+    x = _randn(2, 16, 35, 34).requires_grad_(True)
+    w = _randn(24, 16, k, k, std=(16 * k * k) ** -0.5).requires_grad_(True)
+    if flat:
+        w.main_grad = torch.full(w.shape, 2.0, device="cuda")
+    y = RF.conv2d(x, w, None, stride, pad)
+    xr, wr = (t.detach().double().requires_grad_(True) for t in (x, w))
+    ref = F.conv2d(xr, wr, None, stride, pad)
+    dy = _randn(*y.shape)
+    y.backward(dy)
+    ref.backward(dy.double())
+    assert _rel(y, ref) < 2.0 ** -8
+    assert _rel(w.main_grad - 2.0 if flat else w.grad, wr.grad) < (1e-5 if flat else 2.0 ** -8)
+    assert _rel(x.grad, xr.grad) < k * 2.0 ** -8       # k * k roundings of parts that add up like a random walk
