@@ -1065,7 +1065,18 @@ static bool pair_enabled() {
 extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     using namespace rb;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-    if (a->M <= 0 || a->N <= 0 || a->K <= 0 || a->batch <= 0) return 0;
+    if (a->M <= 0 || a->N <= 0 || a->batch <= 0) return 0;
+    if (a->K <= 0) {
+        // a sum of nothing (the weight gradient of an empty batch) is zero; no caller has an epilogue for it
+        if (a->flags == RB_GEMM_ACCUM) return 0;
+        if (a->flags || a->map_hp > 0) return -9;
+        const size_t es = a->out_dtype == 1 ? 4 : 2;
+        for (int64_t b = 0; b < a->batch; ++b)
+            if (cudaMemset2DAsync(static_cast<char*>(a->D) + b * a->strideD * es, a->ldd * es, 0, a->N * es, a->M,
+                                  stream) != cudaSuccess)
+                return -4;
+        return 0;
+    }
     // TMA needs 16-byte aligned bases and row strides
     if ((reinterpret_cast<uintptr_t>(a->A) & 15) || (reinterpret_cast<uintptr_t>(a->B) & 15) ||
         (a->lda % 8) || (a->ldb % 8) || (a->batch > 1 && ((a->strideA % 8) || (a->strideB % 8))))

@@ -436,6 +436,11 @@ static int ln_bwd_sums(const float* partial, void* dgamma, void* dbeta, int grid
                                                                     static_cast<OutT*>(dbeta), grid, H, accumulate);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
+// An empty batch contributes nothing: the parameters' gradients are zero, or stay what they were.
+static int ln_bwd_empty(void* dgamma, void* dbeta, size_t bytes, int accumulate, cudaStream_t st) {
+    if (accumulate) return 0;
+    return cudaMemsetAsync(dgamma, 0, bytes, st) == cudaSuccess && cudaMemsetAsync(dbeta, 0, bytes, st) == cudaSuccess ? 0 : -1;
+}
 }  // namespace rb
 
 // `partial` is scratch of rb_ln_bwd_grid(rows) * 2 * H floats.  dgamma / dbeta are
@@ -445,7 +450,7 @@ extern "C" int rb_ln_bwd(const void* dy, const void* z, const void* gamma, const
                          float* partial, int rows, int H, float p, uint64_t seed, uint64_t offset,
                          int accumulate, int dtype, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (rows <= 0) return 0;
+    if (rows <= 0) return rb::ln_bwd_empty(dgamma, dbeta, H * sizeof(float), accumulate, st);
     const int grid = rb_ln_bwd_grid(rows);
     const int rc = rb::ln_bwd_rows(dy, z, gamma, mean, rstd, dz, dx, partial, grid, rows, H, p, seed, offset, dtype, st);
     return rc ? rc : rb::ln_bwd_sums<float>(partial, dgamma, dbeta, grid, H, accumulate, st);
@@ -456,7 +461,7 @@ extern "C" int rb_ln_bwd16(const void* dy, const void* z, const void* gamma, con
                            void* dz, void* dx, void* dgamma, void* dbeta, float* partial, int rows, int H, float p,
                            uint64_t seed, uint64_t offset, int dtype, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (rows <= 0) return 0;
+    if (rows <= 0) return rb::ln_bwd_empty(dgamma, dbeta, H * 2, 0, st);
     const int grid = rb_ln_bwd_grid(rows);
     const int rc = rb::ln_bwd_rows(dy, z, gamma, mean, rstd, dz, dx, partial, grid, rows, H, p, seed, offset, dtype, st);
     if (rc) return rc;
@@ -504,7 +509,11 @@ extern "C" int rb_ln_bwd_noalloc(const void* dy, const void* z, const void* gamm
                                  const float* rstd, void* dz, void* dx, float* dgamma, float* dbeta, int rows,
                                  int H, float p, uint64_t seed, uint64_t offset, int accumulate, int dtype,
                                  void* stream) {
-    if (rows <= 0) return RB_LN_NOALLOC_OK;
+    if (rows <= 0) {   // writes zero gradients unless it accumulates; needs no scratch
+        const int rc = rb_ln_bwd(dy, z, gamma, mean, rstd, dz, dx, dgamma, dbeta, nullptr, rows, H, p, seed, offset,
+                                 accumulate, dtype, stream);
+        return rc == 0 ? RB_LN_NOALLOC_OK : RB_LN_NOALLOC_LAUNCH_FAILED;
+    }
     if (!rb_ln_supported(H)) return RB_LN_NOALLOC_BAD_WIDTH;
     const long long need = static_cast<long long>(rb_ln_bwd_grid(rows)) * 2 * H;
     if (need > RB_LN_NOALLOC_MAX_FLOATS) return RB_LN_NOALLOC_TOO_LARGE;

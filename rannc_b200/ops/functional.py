@@ -83,7 +83,7 @@ def _kernel_ok(x) -> bool:
 
 
 def _aligned(t) -> bool:
-    return t.data_ptr() % 16 == 0 and t.shape[-1] % 8 == 0
+    return t.data_ptr() % 16 == 0 and t.shape[-1] % 8 == 0 and t.shape[-1] > 0
 
 
 def _bgrad(dy2, bias, mg):

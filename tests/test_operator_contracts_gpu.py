@@ -107,3 +107,46 @@ def test_large_filters(k, stride, pad, flat):
     assert _rel(y, ref) < 2.0 ** -8
     assert _rel(w.main_grad - 2.0 if flat else w.grad, wr.grad) < (1e-5 if flat else 2.0 ** -8)
     assert _rel(x.grad, xr.grad) < k * 2.0 ** -8       # k * k roundings of parts that add up like a random walk
+
+
+# ------------------------------------------------------------------------------------------ empty batches
+@pytest.mark.parametrize("op", ["linear", "mlp", "layer_norm", "conv1x1", "attention"])
+def test_an_empty_batch_has_zero_parameter_gradients(op):
+    mk = lambda *s: _randn(*s).requires_grad_(True)  # noqa: E731
+    poison = [torch.full((512, 512), float("nan"), device="cuda", dtype=BF) for _ in range(8)]   # noqa: F841
+    del poison
+    if op == "linear":
+        ps = [mk(64, 128), mk(64)]
+        y = RF.linear(torch.empty(0, 128, device="cuda", dtype=BF), *ps)
+    elif op == "mlp":
+        ps = [mk(256, 128), mk(256), mk(128, 256), mk(128)]
+        y = RF.mlp(torch.empty(0, 128, device="cuda", dtype=BF), *ps)
+    elif op == "layer_norm":
+        ps = [mk(256), mk(256)]
+        y = RF.dropout_add_layer_norm(torch.empty(0, 256, device="cuda", dtype=BF), None, *ps)
+    elif op == "attention":
+        ps = [mk(128, 128) for _ in range(3)] + [mk(128) for _ in range(3)]
+        y = _attention(torch.empty(0, 16, 128, device="cuda", dtype=BF), ps[:3], ps[3:], 2)
+    else:
+        ps = [mk(64, 128, 1, 1), mk(64)]
+        y = RF.conv2d(torch.empty(0, 128, 4, 4, device="cuda", dtype=BF), *ps)
+    y.sum().backward()
+    for p in ps:
+        assert p.grad is not None and bool((p.grad == 0).all())
+
+
+@pytest.mark.parametrize("out", [BF, torch.float32])
+def test_a_product_over_nothing_is_zero(out):
+    from rannc_b200.ops.gemm import gemm
+
+    buf = torch.full((40, 32), 3.0, device="cuda", dtype=out)
+    gemm(torch.empty(0, 40, device="cuda", dtype=BF), torch.empty(0, 24, device="cuda", dtype=BF), trans_a=True,
+         trans_b=False, out=buf[:, :24])
+    assert bool((buf[:, :24] == 0).all()) and bool((buf[:, 24:] == 3).all())
+    if out == torch.float32:
+        buf.fill_(3.0)
+        gemm(torch.empty(0, 40, device="cuda", dtype=BF), torch.empty(0, 32, device="cuda", dtype=BF), trans_a=True,
+             trans_b=False, out=buf, accumulate=True)
+        assert bool((buf == 3).all())
+    x, w, b = torch.empty(3, 0, device="cuda", dtype=BF), torch.empty(8, 0, device="cuda", dtype=BF), _randn(8)
+    assert torch.equal(RF.linear(x, w, b), b.expand(3, 8))
