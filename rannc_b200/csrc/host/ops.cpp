@@ -402,21 +402,19 @@ struct LnNode : Node {
         for (SavedVariable* s : {&z, &gamma, &mean, &rstd}) s->reset_data();
     }
     variable_list run(variable_list&& grads) {
-        const Tensor Z = z.unpack(), G = gamma.unpack(), M = mean.unpack(), R = rstd.unpack();
+        const Tensor Z = z.unpack(), G = dense(gamma.unpack()), M = mean.unpack(), R = rstd.unpack();
         const Tensor dy = dense(grads[0]);
         const int H = static_cast<int>(Z.size(-1)), rows = static_cast<int>(Z.numel() / H);
-        const bool flat = g_mg.defined() && b_mg.defined(), same = G.scalar_type() == Z.scalar_type();
+        const bool flat = g_mg.defined() && b_mg.defined();
         Tensor dz = at::empty(Z.sizes(), Z.options()), dx = dz;
         if (p > 0) dx = at::empty(Z.sizes(), Z.options());
         Tensor partial = f32({static_cast<int64_t>(api.ln_bwd_grid(rows)) * 2 * H}, Z);
         void* dx_drop = p > 0 ? dx.data_ptr() : nullptr;
-        if (flat || !same) {
-            Tensor dg = flat ? g_mg : f32({H}, Z), db = flat ? b_mg : f32({H}, Z);
+        if (flat) {
             check(api.ln_bwd(dy.data_ptr(), Z.data_ptr(), G.data_ptr(), mptr<float>(M), mptr<float>(R), dz.data_ptr(), dx_drop,
-                             mptr<float>(dg), mptr<float>(db), mptr<float>(partial), rows, H, static_cast<float>(p), seed,
-                             offset, flat ? 1 : 0, dt_code(Z), cur_stream()),
+                             mptr<float>(g_mg), mptr<float>(b_mg), mptr<float>(partial), rows, H, static_cast<float>(p),
+                             seed, offset, 1, dt_code(Z), cur_stream()),
                   "rb_ln_bwd", 2);
-            if (!flat) return {dx, dz, dg.to(G.scalar_type()), db.to(G.scalar_type())};
             notify({{&g_ref, &g_mg}, {&b_ref, &b_mg}});
             return {dx, dz, Tensor(), Tensor()};
         }
@@ -433,17 +431,25 @@ struct LnNode : Node {
 Tensor layer_norm(const Tensor& x, const OptTensor& res_, const Tensor& gamma, const Tensor& beta, double p, double eps,
                   uint64_t seed, uint64_t offset, const OptTensor& g_mg, const OptTensor& b_mg) {
     const Tensor res = opt(res_);
+    // the kernels read every operand in x's type and as many elements of it as x's sizes say
+    TORCH_CHECK_TYPE(gamma.scalar_type() == x.scalar_type() && beta.scalar_type() == x.scalar_type() &&
+                         (!res.defined() || res.scalar_type() == x.scalar_type()),
+                     "layer_norm: the operands' types differ");
+    TORCH_CHECK_VALUE(gamma.numel() == x.size(-1) && beta.numel() == x.size(-1) &&
+                          (!res.defined() || res.sizes() == x.sizes()),
+                      "layer_norm: the operands' sizes differ");
     const bool req = wants_grad({&x, &res, &gamma, &beta});
-    Tensor y, z, mean, rstd;
+    Tensor xc, y, z, mean, rstd;
     {
         at::NoGradGuard off;
-        const Tensor xc = dense(x), rc = res.defined() ? dense(res) : Tensor();
+        xc = dense(x);
+        const Tensor rc = res.defined() ? dense(res) : Tensor(), gc = dense(gamma), bc = dense(beta);
         const int H = static_cast<int>(x.size(-1)), rows = static_cast<int>(x.numel() / H);
         y = at::empty(xc.sizes(), xc.options());
         if (res.defined() || p > 0) z = at::empty(xc.sizes(), xc.options());
         mean = f32({rows}, x);
         rstd = f32({rows}, x);
-        check(api.ln_fwd(xc.data_ptr(), cptr(rc), gamma.data_ptr(), beta.data_ptr(), y.data_ptr(), mptr(z),
+        check(api.ln_fwd(xc.data_ptr(), cptr(rc), gc.data_ptr(), bc.data_ptr(), y.data_ptr(), mptr(z),
                          mptr<float>(mean), mptr<float>(rstd), rows, H, static_cast<float>(eps), static_cast<float>(p), seed,
                          offset, dt_code(x), cur_stream()),
               "rb_ln_fwd");

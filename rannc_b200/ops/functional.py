@@ -120,13 +120,20 @@ def mlp(x, w1, b1, w2, b2):
 
 # ----------------------------------------------------------------------------- layer norm
 def dropout_add_layer_norm(x, residual, gamma, beta, p: float = 0.0, eps: float = 1e-5, training: bool = True):
-    """``LayerNorm(dropout(x, p) + residual)`` over the last dimension."""
+    """``LayerNorm(dropout(x, p) + residual)`` over the last dimension; the result has x's type.  The kernels want
+    operands of one type and a residual of x's shape; parameters of another type are applied in fp32."""
     p = p if training else 0.0
-    if not (_kernel_ok(x) and K.ln_supported(x.shape[-1]) and gamma is not None and beta is not None):
+    H, dt = x.shape[-1], x.dtype
+    if not (_kernel_ok(x) and K.ln_supported(H) and gamma is not None and beta is not None and
+            gamma.dtype == dt and beta.dtype == dt and gamma.numel() == H and beta.numel() == H and
+            (residual is None or (residual.dtype == dt and residual.shape == x.shape))):
         h = torch.nn.functional.dropout(x, p, True) if p > 0 else x
         if residual is not None:
             h = h + residual
-        return torch.nn.functional.layer_norm(h, (x.shape[-1],), gamma, beta, eps)
+        if any(t is not None and t.dtype != h.dtype for t in (gamma, beta)):
+            gamma, beta = (None if t is None else t.float() for t in (gamma, beta))
+            return torch.nn.functional.layer_norm(h.float(), (H,), gamma, beta, eps).to(dt)
+        return torch.nn.functional.layer_norm(h, (H,), gamma, beta, eps)
     h = _host()
     seed, offset = rng.next() if p > 0.0 else (0, 0)
     return h.layer_norm(x, residual, gamma, beta, float(p), float(eps), seed, offset, _main_grad(gamma),

@@ -150,3 +150,46 @@ def test_a_product_over_nothing_is_zero(out):
         assert bool((buf == 3).all())
     x, w, b = torch.empty(3, 0, device="cuda", dtype=BF), torch.empty(8, 0, device="cuda", dtype=BF), _randn(8)
     assert torch.equal(RF.linear(x, w, b), b.expand(3, 8))
+
+
+# ------------------------------------------------------------------------------------------ operand types
+@pytest.mark.parametrize("res", [False, True])
+def test_layer_norm_with_parameters_of_another_type(res):
+    torch.manual_seed(4)
+    x = _randn(37, 512).requires_grad_(True)
+    r = _randn(37, 512).requires_grad_(True) if res else None
+    g, b = (torch.rand(512, device="cuda") + 0.5).requires_grad_(True), torch.randn(512, device="cuda").requires_grad_(True)
+    y = RF.dropout_add_layer_norm(x, r, g, b, 0.0, 1e-5)
+    dy = _randn(37, 512)
+    y.backward(dy.to(y.dtype))
+    xr, gr, br = (t.detach().double().requires_grad_(True) for t in (x, g, b))
+    ref = F.layer_norm(xr + (r.detach().double() if res else 0.0), (512,), gr, br, 1e-5)
+    ref.backward(dy.double())
+    assert y.dtype == BF and _rel(y, ref) < 2 * 2.0 ** -8
+    # the residual sum and the result are each rounded once
+    assert _rel(x.grad, xr.grad) < 3 * 2.0 ** -8
+    assert g.grad.dtype == torch.float32 and _rel(g.grad, gr.grad) < 2.0 ** -7 and _rel(b.grad, br.grad) < 2.0 ** -7
+
+
+@pytest.mark.parametrize("shape", [(1, 5, 256), (256,), (3, 1, 1)])
+def test_layer_norm_with_a_residual_that_broadcasts(shape):
+    torch.manual_seed(7)
+    x, r = _randn(3, 5, 256), _randn(*shape)
+    g, b = _randn(256) + 1, _randn(256)
+    y = RF.dropout_add_layer_norm(x, r, g, b, 0.0, 1e-5)
+    want = F.layer_norm(x.double() + r.double(), (256,), g.double(), b.double(), 1e-5)
+    assert y.shape == x.shape and _rel(y, want) < 2 * 2.0 ** -8     # the sum and the result are each rounded
+
+
+def test_layer_norm_refuses_operands_its_kernels_would_misread():
+    from rannc_b200.ops import _lib
+
+    h, x, g = _lib.host(), _randn(4, 256), _randn(256)
+    ln = lambda **k: h.layer_norm(k.get("x", x), k.get("r"), k.get("g", g), k.get("b", g), 0.0, 1e-5, 0, 0, None, None)  # noqa: E731
+    ln()
+    two = torch.stack((g, _randn(256)), 1)
+    assert torch.equal(ln(g=two[:, 0], b=two[:, 0].reshape(1, 256)), ln())      # a strided parameter is read as what it is
+    for bad, err in (({"g": g.float()}, TypeError), ({"b": g.half()}, TypeError), ({"r": x.float()}, TypeError),
+                     ({"g": g[:128]}, ValueError), ({"r": x[:2]}, ValueError)):
+        with pytest.raises(err):
+            ln(**bad)
