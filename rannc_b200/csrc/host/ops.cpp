@@ -87,6 +87,40 @@ T* mptr(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : 
 Tensor opt(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
 Tensor f32(at::IntArrayRef sizes, const Tensor& like) { return at::empty(sizes, like.options().dtype(at::kFloat)); }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+Tensor dense(const Tensor& t) { return !t.defined() || t.is_contiguous() ? t : t.contiguous(); }
+
+// ------------------------------------------------------------------------------------------------ operand checks
+// Kernels get bare addresses: they read an operand in the type, and as many elements of it, as the call's other operands
+// say.  What would be misread is refused here, before anything is launched.
+void same_type(const char* op, const Tensor& x, std::initializer_list<const Tensor*> others) {
+    for (const Tensor* t : others)
+        if (t->defined())
+            TORCH_CHECK_TYPE(t->scalar_type() == x.scalar_type() && t->device() == x.device(), op,
+                             ": the operands' types or devices differ (", x.scalar_type(), " on ", x.device(), " and ",
+                             t->scalar_type(), " on ", t->device(), ")");
+}
+void length(const char* op, const Tensor& t, int64_t n) {
+    TORCH_CHECK_VALUE(!t.defined() || t.numel() == n, op, ": ", n, " elements expected, not ", t.numel());
+}
+// a parameter's gradient buffer: fp32 and dense, as many elements as the parameter
+Tensor grad_buffer(const char* op, const OptTensor& buffer, const Tensor& param) {
+    if (!buffer.has_value() || !buffer->defined()) return Tensor();
+    length(op, *buffer, param.numel());
+    TORCH_CHECK_TYPE(buffer->scalar_type() == at::kFloat && buffer->device() == param.device(), op,
+                     ": gradient buffers are fp32, on the parameter's device");
+    TORCH_CHECK_VALUE(buffer->is_contiguous(), op, ": gradient buffers are contiguous");
+    return *buffer;
+}
+// a matrix that a GEMM adds to: rows of any stride, in fp32 or in the parameter's own type
+Tensor weight_grad_buffer(const char* op, const OptTensor& buffer, const Tensor& w) {
+    if (!buffer.has_value() || !buffer->defined()) return Tensor();
+    TORCH_CHECK_TYPE((buffer->scalar_type() == at::kFloat || buffer->scalar_type() == w.scalar_type()) &&
+                         buffer->device() == w.device(),
+                     op, ": a weight's gradient buffer is fp32 or of the weight's type, on its device");
+    TORCH_CHECK_VALUE(buffer->sizes() == w.sizes() && buffer->stride(1) == 1, op,
+                      ": a weight's gradient buffer has the weight's sizes and dense rows");
+    return *buffer;
+}
 
 // ------------------------------------------------------------------------------------------------ GEMM
 // A matrix as the copy engine wants it: 16-byte aligned base, unit column stride, row stride a multiple of 8.  One
@@ -181,7 +215,7 @@ Grads param_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& w_
         e.a_colsum = mptr<float>(db);
         if (w_mg.defined()) {
             e.accumulate = true;
-            gemm(dy, x, true, false, w_mg.data_ptr(), true, dtype, e, w_mg.stride(0));
+            gemm(dy, x, true, false, w_mg.data_ptr(), w_mg.scalar_type() == at::kFloat, dtype, e, w_mg.stride(0));
         } else if (dy.rows >= std::max<int64_t>(2048, 256 * ((dy.cols + 255) / 256) * ((x.cols + 255) / 256))) {
             // A long product with few 256 x 256 tiles leaves most of the GPU idle unless K is split, which takes an
             // fp32 result to add to: clearing it and rounding it are two more passes over the weight.  Measured, one
@@ -236,8 +270,6 @@ void notify(std::initializer_list<std::pair<const Tensor*, const Tensor*>> param
     }
     Py_DECREF(r);
 }
-Tensor dense(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
-
 #define RB_NODE(NAME)                                       \
     std::string name() const override { return NAME; }      \
     variable_list apply(variable_list&& grads) override {   \
@@ -282,8 +314,11 @@ struct LinearNode : Node {
 Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& bias_, bool gelu, const OptTensor& w_mg,
               const OptTensor& b_mg, const OptTensor& owner) {
     const Tensor bias = opt(bias_);
+    same_type("linear", x, {&w, &bias});
+    TORCH_CHECK_VALUE(w.dim() == 2, "linear: the weight is a matrix");
+    length("linear bias", bias, w.size(0));
     const bool req = wants_grad({&x, &w, &bias});
-    Tensor y, pre, xc;
+    Tensor y, pre, xc, bc;
     {
         at::NoGradGuard off;
         xc = dense(x);
@@ -291,7 +326,8 @@ Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& bias_, bool gel
         sizes.back() = w.size(0);
         y = at::empty(sizes, x.options());
         Epi e;
-        e.bias = cptr(bias);
+        bc = dense(bias);
+        e.bias = cptr(bc);
         if (gelu) {
             e.gelu = true;
             pre = at::empty(sizes, x.options());
@@ -307,8 +343,8 @@ Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& bias_, bool gel
         n->pre = SavedVariable(pre, false);
         n->w_ref = owner.has_value() ? *owner : w;
         n->bias = bias;
-        n->w_mg = opt(w_mg);
-        n->b_mg = opt(b_mg);
+        n->w_mg = weight_grad_buffer("linear", w_mg, w);
+        n->b_mg = grad_buffer("linear", b_mg, bias);
         torch::autograd::set_history(y, n);
     }
     return y;
@@ -349,8 +385,12 @@ struct MlpNode : Node {
 Tensor mlp(const Tensor& x, const Tensor& w1, const OptTensor& b1_, const Tensor& w2, const OptTensor& b2_,
            const OptTensor& w1_mg, const OptTensor& b1_mg, const OptTensor& w2_mg, const OptTensor& b2_mg) {
     const Tensor b1 = opt(b1_), b2 = opt(b2_);
+    same_type("mlp", x, {&w1, &b1, &w2, &b2});
+    TORCH_CHECK_VALUE(w1.dim() == 2 && w2.dim() == 2, "mlp: the weights are matrices");
+    length("mlp bias", b1, w1.size(0));
+    length("mlp bias", b2, w2.size(0));
     const bool req = wants_grad({&x, &w1, &b1, &w2, &b2});
-    Tensor xc, pre, h, y;
+    Tensor xc, pre, h, y, b1c, b2c;
     {
         at::NoGradGuard off;
         xc = dense(x);
@@ -361,13 +401,15 @@ Tensor mlp(const Tensor& x, const Tensor& w1, const OptTensor& b1_, const Tensor
         sizes.back() = w2.size(0);
         y = at::empty(sizes, x.options());
         const int dt = dt_code(x);
+        b1c = dense(b1);
+        b2c = dense(b2);
         Epi e;
-        e.bias = cptr(b1);
+        e.bias = cptr(b1c);
         e.gelu = true;
         e.aux_out = pre.data_ptr();
         gemm(rows_of(xc), mat(w1), false, true, h.data_ptr(), false, dt, e);
         Epi e2;
-        e2.bias = cptr(b2);
+        e2.bias = cptr(b2c);
         gemm(rows_of(h), mat(w2), false, true, y.data_ptr(), false, dt, e2);
     }
     if (req) {
@@ -382,10 +424,10 @@ Tensor mlp(const Tensor& x, const Tensor& w1, const OptTensor& b1_, const Tensor
         n->w2_ref = w2;
         n->b1 = b1;
         n->b2 = b2;
-        n->w1_mg = opt(w1_mg);
-        n->b1_mg = opt(b1_mg);
-        n->w2_mg = opt(w2_mg);
-        n->b2_mg = opt(b2_mg);
+        n->w1_mg = weight_grad_buffer("mlp", w1_mg, w1);
+        n->b1_mg = grad_buffer("mlp", b1_mg, b1);
+        n->w2_mg = weight_grad_buffer("mlp", w2_mg, w2);
+        n->b2_mg = grad_buffer("mlp", b2_mg, b2);
         torch::autograd::set_history(y, n);
     }
     return y;
@@ -431,19 +473,16 @@ struct LnNode : Node {
 Tensor layer_norm(const Tensor& x, const OptTensor& res_, const Tensor& gamma, const Tensor& beta, double p, double eps,
                   uint64_t seed, uint64_t offset, const OptTensor& g_mg, const OptTensor& b_mg) {
     const Tensor res = opt(res_);
-    // the kernels read every operand in x's type and as many elements of it as x's sizes say
-    TORCH_CHECK_TYPE(gamma.scalar_type() == x.scalar_type() && beta.scalar_type() == x.scalar_type() &&
-                         (!res.defined() || res.scalar_type() == x.scalar_type()),
-                     "layer_norm: the operands' types differ");
-    TORCH_CHECK_VALUE(gamma.numel() == x.size(-1) && beta.numel() == x.size(-1) &&
-                          (!res.defined() || res.sizes() == x.sizes()),
-                      "layer_norm: the operands' sizes differ");
+    same_type("layer_norm", x, {&res, &gamma, &beta});
+    length("layer_norm weight", gamma, x.size(-1));
+    length("layer_norm bias", beta, x.size(-1));
+    TORCH_CHECK_VALUE(!res.defined() || res.sizes() == x.sizes(), "layer_norm: the residual's sizes differ from x's");
     const bool req = wants_grad({&x, &res, &gamma, &beta});
     Tensor xc, y, z, mean, rstd;
     {
         at::NoGradGuard off;
         xc = dense(x);
-        const Tensor rc = res.defined() ? dense(res) : Tensor(), gc = dense(gamma), bc = dense(beta);
+        const Tensor rc = dense(res), gc = dense(gamma), bc = dense(beta);
         const int H = static_cast<int>(x.size(-1)), rows = static_cast<int>(x.numel() / H);
         y = at::empty(xc.sizes(), xc.options());
         if (res.defined() || p > 0) z = at::empty(xc.sizes(), xc.options());
@@ -464,8 +503,8 @@ Tensor layer_norm(const Tensor& x, const OptTensor& res_, const Tensor& gamma, c
         n->rstd = SavedVariable(rstd, false);
         n->g_ref = gamma;
         n->b_ref = beta;
-        n->g_mg = opt(g_mg);
-        n->b_mg = opt(b_mg);
+        n->g_mg = grad_buffer("layer_norm", g_mg, gamma);
+        n->b_mg = grad_buffer("layer_norm", b_mg, beta);
         n->p = p;
         n->seed = seed;
         n->offset = offset;
@@ -498,6 +537,9 @@ struct EmbeddingNode : Node {
 };
 
 Tensor embedding(const Tensor& w, const Tensor& ids, int64_t padding, const OptTensor& w_mg) {
+    TORCH_CHECK_TYPE(ids.scalar_type() == at::kLong && ids.device() == w.device(),
+                     "embedding: the ids are 64-bit integers on the table's device");
+    TORCH_CHECK_VALUE(w.dim() == 2 && w.is_contiguous(), "embedding: the table is a contiguous matrix");
     const bool req = wants_grad({&w});
     Tensor out, idc;
     {
@@ -515,7 +557,7 @@ Tensor embedding(const Tensor& w, const Tensor& ids, int64_t padding, const OptT
         n->set_next_edges(torch::autograd::collect_next_edges(w));
         n->ids = SavedVariable(idc, false);
         n->weight = w;
-        n->w_mg = opt(w_mg);
+        n->w_mg = grad_buffer("embedding", w_mg, w);
         n->padding = padding;
         torch::autograd::set_history(out, n);
     }
@@ -545,6 +587,11 @@ struct XentNode : Node {
 };
 
 Tensor cross_entropy(const Tensor& logits, const Tensor& labels, int64_t V, int64_t ignore, double weight) {
+    TORCH_CHECK_TYPE(labels.scalar_type() == at::kLong && labels.device() == logits.device(),
+                     "cross_entropy: the labels are 64-bit integers on the logits' device");
+    TORCH_CHECK_VALUE(logits.dim() == 2 && logits.stride(1) == 1 && labels.is_contiguous() &&
+                          labels.numel() == logits.size(0) && V > 0 && V <= logits.size(1),
+                      "cross_entropy: one label per row of logits, and no more classes than columns");
     const bool req = wants_grad({&logits});
     Tensor lse, acc, loss;
     {
@@ -678,7 +725,7 @@ struct QkvNode : Node {
         // adjacent fp32 gradient buffers: one weight-gradient GEMM (with the column sums of the biases) serves all three
         // projections
         auto all = [](const Tensor* t) { return t[0].defined() && t[1].defined() && t[2].defined(); };
-        const void* wm = all(w_mg) ? adjacent(w_mg) : nullptr;
+        const void* wm = all(w_mg) && w_mg[0].scalar_type() == at::kFloat ? adjacent(w_mg) : nullptr;
         const void* bm = b[0].defined() && all(b_mg) ? adjacent(b_mg) : nullptr;
         if (wm && (bm || !b[0].defined())) {
             Epi e;
@@ -711,10 +758,24 @@ struct QkvNode : Node {
 Tensor qkv_attention(const Tensor& x, const std::vector<Tensor>& ws, const std::vector<OptTensor>& bs, const OptTensor& key_bias,
                      double p, double scale, int64_t H, uint64_t seed, uint64_t offset, const std::vector<OptTensor>& w_mgs,
                      const std::vector<OptTensor>& b_mgs, bool streamed) {
+    TORCH_CHECK_VALUE(x.dim() == 3 && ws.size() == 3 && bs.size() == 3 && w_mgs.size() == 3 && b_mgs.size() == 3,
+                      "qkv_attention: three-dimensional input, three projections");
     const Tensor w[3] = {ws[0], ws[1], ws[2]}, b[3] = {opt(bs[0]), opt(bs[1]), opt(bs[2])};
+    same_type("qkv_attention", x, {&w[0], &w[1], &w[2], &b[0], &b[1], &b[2]});
+    for (int i = 0; i < 3; ++i) {
+        TORCH_CHECK_VALUE(w[i].dim() == 2 && w[i].sizes() == w[0].sizes() && w[0].size(0) == 64 * H &&
+                              b[i].defined() == b[0].defined(),
+                          "qkv_attention: three projections of one shape, 64 rows a head");
+        length("qkv_attention bias", b[i], w[0].size(0));
+    }
     const bool req = wants_grad({&x, &w[0], &b[0], &w[1], &b[1], &w[2], &b[2]});
     const int64_t B = x.size(0), S = x.size(1), Ho = w[0].size(0);
     Tensor xc, qkv, o, lse, bias_cat, kb = opt(key_bias);
+    if (kb.defined()) {
+        TORCH_CHECK_TYPE(kb.scalar_type() == at::kFloat && kb.device() == x.device(), "qkv_attention: the key bias is fp32");
+        TORCH_CHECK_VALUE(kb.is_contiguous(), "qkv_attention: the key bias is contiguous");
+        length("qkv_attention key bias", kb, B * S);
+    }
     Mat wm;
     bool copied;
     {
@@ -749,8 +810,8 @@ Tensor qkv_attention(const Tensor& x, const std::vector<Tensor>& ws, const std::
         for (int i = 0; i < 3; ++i) {
             n->w[i] = w[i];
             n->b[i] = b[i];
-            n->w_mg[i] = opt(w_mgs[i]);
-            n->b_mg[i] = opt(b_mgs[i]);
+            n->w_mg[i] = weight_grad_buffer("qkv_attention", w_mgs[i], w[i]);
+            n->b_mg[i] = grad_buffer("qkv_attention", b_mgs[i], b[i]);
         }
         if (copied && !streamed) n->stack = SavedVariable(wm.keep, false);
         n->B = B;
@@ -809,6 +870,10 @@ Tensor batch_norm_act(const Tensor& x, const OptTensor& res_, const Tensor& gamm
                       const OptTensor& run_mean_, const OptTensor& run_var_, double momentum, double eps, bool relu,
                       const OptTensor& g_mg, const OptTensor& b_mg) {
     const Tensor res = opt(res_), run_mean = opt(run_mean_), run_var = opt(run_var_);
+    same_type("batch_norm", x, {&res});
+    TORCH_CHECK_VALUE(x.dim() == 4 && (!res.defined() || res.sizes() == x.sizes()),
+                      "batch_norm: the residual's sizes differ from x's");
+    for (const Tensor* t : {&gamma, &beta, &run_mean, &run_var}) length("batch_norm parameter", *t, x.size(1));
     const bool req = wants_grad({&x, &res, &gamma, &beta});
     Tensor xc, y, mean, rstd, g32;
     {
@@ -816,9 +881,10 @@ Tensor batch_norm_act(const Tensor& x, const OptTensor& res_, const Tensor& gamm
         const int64_t C = x.size(1), R = x.numel() / C;
         xc = nhwc(x);
         const Tensor rc = res.defined() ? nhwc(res) : Tensor();
-        g32 = gamma.detach().to(at::kFloat);
-        const Tensor b32 = beta.detach().to(at::kFloat);
-        const bool in_kernel = run_mean.defined() && run_mean.scalar_type() == at::kFloat;
+        g32 = dense(gamma.detach().to(at::kFloat));
+        const Tensor b32 = dense(beta.detach().to(at::kFloat));
+        auto fp32 = [](const Tensor& t) { return t.defined() && t.scalar_type() == at::kFloat && t.is_contiguous(); };
+        const bool in_kernel = fp32(run_mean) && fp32(run_var);
         y = at::empty_like(xc);
         Tensor part = f32({2, C}, x);
         mean = f32({C}, x);
@@ -829,7 +895,7 @@ Tensor batch_norm_act(const Tensor& x, const OptTensor& res_, const Tensor& gamm
                          static_cast<float>(momentum), relu ? 1 : 0, dt_code(x), cur_stream()),
               "rb_bn_fwd", 2);
         if (run_mean.defined() && !in_kernel) {
-            // statistics kept in a 16-bit buffer: update them with a few tiny element-wise operations
+            // statistics kept in 16 bits, or strided: update them with a few tiny element-wise operations
             const Tensor var = (1.0 / (rstd * rstd) - eps) * (static_cast<double>(R) / std::max<int64_t>(R - 1, 1));
             run_mean.mul_(1 - momentum).add_((momentum * mean).to(run_mean.scalar_type()));
             run_var.mul_(1 - momentum).add_((momentum * var).to(run_var.scalar_type()));
@@ -869,13 +935,23 @@ Tensor product(const Tensor& a, const Tensor& b, bool trans_a, bool trans_b, con
     const int64_t kb = trans_b ? B.cols : B.rows;
     TORCH_CHECK_VALUE(kb == g.K, "gemm: inner dimensions differ (", g.K, " vs ", kb, ")");
     Tensor out = out_.has_value() ? *out_ : at::empty({g.M, g.N}, fp32_out ? a.options().dtype(at::kFloat) : a.options());
+    const Tensor bv = dense(opt(bias)), rv = opt(residual), ai = opt(aux_in), ao = opt(aux_out);
+    same_type("gemm", a, {&b, &bv, &rv, &ai, &ao});
+    length("gemm bias", bv, g.N);
+    TORCH_CHECK_TYPE(out.scalar_type() == (fp32_out ? at::kFloat : a.scalar_type()) && out.device() == a.device(),
+                     "gemm: the output is of the operands' type or fp32, on their device");
+    // the matrices beside the output share its row stride
+    for (const Tensor* t : {static_cast<const Tensor*>(&out), &rv, &ai, &ao})
+        TORCH_CHECK_VALUE(!t->defined() || (t->dim() == 2 && t->size(0) == g.M && t->size(1) == g.N &&
+                                            (g.N <= 1 || t->stride(1) == 1) && (g.M <= 1 || t->stride(0) == out.stride(0))),
+                          "gemm: the output and the matrices beside it are [", g.M, ", ", g.N, "] with one row stride");
     g.A = A.p;
     g.B = B.p;
     g.D = out.data_ptr();
-    g.bias = cptr(opt(bias));
-    g.residual = cptr(opt(residual));
-    g.aux_in = cptr(opt(aux_in));
-    g.aux_out = mptr(opt(aux_out));
+    g.bias = cptr(bv);
+    g.residual = cptr(rv);
+    g.aux_in = cptr(ai);
+    g.aux_out = mptr(ao);
     g.batch = 1;
     g.lda = A.ld;
     g.ldb = B.ld;

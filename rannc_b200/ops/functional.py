@@ -86,6 +86,11 @@ def _aligned(t) -> bool:
     return t.data_ptr() % 16 == 0 and t.shape[-1] % 8 == 0 and t.shape[-1] > 0
 
 
+def _bias_ok(bias, n, dtype) -> bool:
+    """None, or ``n`` values of the type the kernels read beside the operands."""
+    return bias is None or (bias.dtype == dtype and bias.numel() == n)
+
+
 def _bgrad(dy2, bias, mg):
     if bias is None:
         return None
@@ -105,7 +110,8 @@ def _host():
 # ----------------------------------------------------------------------------- linear
 def linear(x, weight, bias=None, act=None):
     """``act(x @ weight.T + bias)`` with ``act`` in (None, "gelu")."""
-    if not (_kernel_ok(x) and weight.dtype == x.dtype and _aligned(x) and _aligned(weight)):
+    if not (_kernel_ok(x) and weight.dtype == x.dtype and _aligned(x) and _aligned(weight) and weight.dim() == 2 and
+            _bias_ok(bias, weight.shape[0], x.dtype)):
         y = torch.nn.functional.linear(x, weight, bias)
         return torch.nn.functional.gelu(y) if act == "gelu" else y
     return _host().linear(x, weight, bias, act == "gelu", _main_grad(weight), _main_grad(bias), None)
@@ -113,7 +119,9 @@ def linear(x, weight, bias=None, act=None):
 
 def mlp(x, w1, b1, w2, b2):
     """y = gelu(x W1^T + b1) W2^T + b2; the GELU derivative rides in the epilogue of a backward GEMM."""
-    if not (_kernel_ok(x) and _aligned(x) and _aligned(w1) and _aligned(w2)):
+    dt = x.dtype
+    if not (_kernel_ok(x) and _aligned(x) and _aligned(w1) and _aligned(w2) and w1.dtype == dt and w2.dtype == dt and
+            _bias_ok(b1, w1.shape[0], dt) and _bias_ok(b2, w2.shape[0], dt)):
         return torch.nn.functional.linear(torch.nn.functional.gelu(torch.nn.functional.linear(x, w1, b1)), w2, b2)
     return _host().mlp(x, w1, b1, w2, b2, _main_grad(w1), _main_grad(b1), _main_grad(w2), _main_grad(b2))
 
@@ -181,7 +189,8 @@ def gelu(x):
 
 
 def embedding(weight, ids, padding_idx: int = -1):
-    if not (_kernel_ok(weight) and weight.shape[1] % 8 == 0 and ids.dtype == torch.int64):
+    if not (_kernel_ok(weight) and weight.shape[1] % 8 == 0 and weight.is_contiguous() and ids.dtype == torch.int64 and
+            ids.is_cuda):
         return torch.nn.functional.embedding(ids, weight, None if padding_idx < 0 else padding_idx)
     return _host().embedding(weight, ids, padding_idx, _main_grad(weight))
 
@@ -219,7 +228,7 @@ def sdpa(q, k, v, attn_mask=None, dropout_p: float = 0.0, is_causal: bool = Fals
     only depends on (batch, key) -- shape [B, 1, 1, S].  Anything else falls back to
     the ATen implementation."""
     ok = (_kernel_ok(q) and q.dim() == 4 and q.shape[-1] == 64 and not is_causal and k.shape == q.shape
-          and v.shape == q.shape)
+          and v.shape == q.shape and k.dtype == q.dtype and v.dtype == q.dtype)
     key_bias = None
     if ok and attn_mask is not None:
         B, H, S, D = q.shape
@@ -247,7 +256,8 @@ def cross_entropy(logits, labels, num_classes=None, ignore_index: int = -100, we
     ld = logits.shape[-1]
     V = int(num_classes) if num_classes is not None else ld
     l2 = logits.reshape(-1, ld)
-    if not (_kernel_ok(l2) and l2.stride(1) == 1):
+    if not (_kernel_ok(l2) and l2.stride(1) == 1 and 0 < V <= ld and labels.dtype == torch.int64 and labels.is_cuda and
+            labels.numel() == l2.shape[0]):
         return torch.nn.functional.cross_entropy(l2[:, :V].float(), labels.reshape(-1), ignore_index=ignore_index) * weight
     # the logits are dead after the loss: backward writes the gradient over them
     return _host().cross_entropy(l2, labels.reshape(-1).contiguous(), V, ignore_index, float(weight))
@@ -263,7 +273,8 @@ def qkv_attention(x, wq, bq, wk, bk, wv, bv, attn_mask=None, dropout_p: float = 
     D = Ho // num_heads
     same = wk.shape == wq.shape and wv.shape == wq.shape and (bq is None) == (bk is None) == (bv is None)
     ok = (_kernel_ok(x) and same and D == 64 and not is_causal and _aligned(x) and _aligned(wq)
-          and wq.dtype == x.dtype)
+          and wq.dtype == x.dtype and wk.dtype == x.dtype and wv.dtype == x.dtype
+          and all(_bias_ok(b, Ho, x.dtype) for b in (bq, bk, bv)))
     key_bias = None
     if ok and attn_mask is not None:
         if attn_mask.dtype != torch.bool and tuple(attn_mask.shape) == (B, 1, 1, S):
@@ -465,7 +476,8 @@ def conv2d(x, weight, bias=None, stride=1, padding=0, dilation=1, groups=1):
     s, p, d = _pair(stride), _pair(padding), _pair(dilation)
     Co, Ci, kh, kw = weight.shape
     ok = (_kernel_ok(x) and weight.dtype == x.dtype and groups == 1 and d == (1, 1) and kh == kw and s[0] == s[1] and
-          p[0] == p[1] and Ci % 8 == 0 and Co % 8 == 0 and x.dim() == 4 and isinstance(p[0], int))
+          p[0] == p[1] and Ci % 8 == 0 and Co % 8 == 0 and x.dim() == 4 and isinstance(p[0], int) and
+          _bias_ok(bias, Co, x.dtype))
     if not ok:
         return torch.nn.functional.conv2d(x, weight, bias, stride, padding, dilation, groups)
     if kh == 1 and s[0] == 1 and p[0] == 0:
@@ -482,7 +494,7 @@ def batch_norm_act(x, gamma, beta, running_mean, running_var, training: bool = T
     """``relu(batch_norm(x) + residual)`` with ``relu`` and ``residual`` optional.  Training mode with affine
     parameters on the kernels; evaluation mode (running statistics) and other cases on ATen."""
     ok = (_kernel_ok(x) and training and x.dim() == 4 and x.shape[1] % 8 == 0 and gamma is not None and
-          beta is not None and (residual is None or residual.shape == x.shape))
+          beta is not None and (residual is None or (residual.shape == x.shape and residual.dtype == x.dtype)))
     if not ok:
         y = torch.nn.functional.batch_norm(x, running_mean, running_var, gamma, beta, training, momentum, eps)
         if residual is not None:

@@ -193,3 +193,77 @@ def test_layer_norm_refuses_operands_its_kernels_would_misread():
                      ({"g": g[:128]}, ValueError), ({"r": x[:2]}, ValueError)):
         with pytest.raises(err):
             ln(**bad)
+
+
+def test_operands_the_kernels_would_misread_are_refused():
+    """Too short, of another type or elsewhere: ATen's own errors where a call falls back to it, the native entries' else."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops.gemm import gemm
+
+    h, x, w, b = _lib.host(), _randn(8, 128), _randn(64, 128), _randn(64)
+    w2 = _randn(128, 64)
+    ids, table = torch.arange(8, device="cuda"), _randn(16, 64)
+    logits, labels = _randn(8, 64), torch.arange(8, device="cuda")
+    for bad in (b[:32], b.float(), b.half()):
+        for call in (lambda: RF.linear(x, w, bad), lambda: RF.mlp(x, w, bad, w2, None),
+                     lambda: RF.conv2d(_randn(1, 128, 4, 4), w.view(64, 128, 1, 1), bad),
+                     lambda: RF.conv2d(_randn(1, 128, 4, 4), _randn(64, 128, 3, 3), bad)):
+            with pytest.raises(RuntimeError):
+                call()
+        for call in (lambda: h.linear(x, w, bad, False, None, None, None), lambda: gemm(x, w, bias=bad)):
+            with pytest.raises((TypeError, ValueError)):
+                call()
+    with pytest.raises(RuntimeError):
+        RF.mlp(x, w, b, w2.float(), None)
+    with pytest.raises(RuntimeError):
+        RF.cross_entropy(logits, labels.int())
+    with pytest.raises((RuntimeError, ValueError)):
+        RF.cross_entropy(logits, labels[:4])
+    qkv = lambda **k: RF.qkv_attention(_randn(1, 16, 128), *(k.get(n, d) for n, d in (  # noqa: E731
+        ("wq", w2.new_zeros(128, 128)), ("bq", w2.new_zeros(128)), ("wk", w2.new_zeros(128, 128)), ("bk", w2.new_zeros(128)),
+        ("wv", w2.new_zeros(128, 128)), ("bv", w2.new_zeros(128)))), num_heads=2)
+    qkv()
+    for bad in (dict(wk=torch.zeros(128, 128, device="cuda")), dict(bv=w2.new_zeros(64)), dict(bq=torch.zeros(128, device="cuda"))):
+        with pytest.raises(RuntimeError):
+            qkv(**bad)
+    for call in (lambda: h.embedding(table, ids.int(), -1, None), lambda: h.embedding(table.t(), ids, -1, None),
+                 lambda: h.cross_entropy(logits, labels, 65, -100, 1.0), lambda: h.cross_entropy(logits, labels[:4], 64, -100, 1.0),
+                 lambda: gemm(x, w, out=torch.empty(8, 32, device="cuda", dtype=BF)), lambda: gemm(x, w.half()),
+                 lambda: gemm(x, w, residual=_randn(8, 128)[:, :64]), lambda: gemm(x, w, gelu=True, aux_out=_randn(8, 32))):
+        with pytest.raises((TypeError, ValueError)):
+            call()
+    wg = w.clone().requires_grad_(True)
+    for mg in (torch.zeros(64, 64, device="cuda"), torch.zeros(64, 128, device="cuda", dtype=torch.float64),
+               torch.zeros(64, 128)):
+        wg.main_grad = mg
+        with pytest.raises((TypeError, ValueError)):
+            RF.linear(x, wg, b)
+
+
+def test_operands_laid_out_another_way_are_read_as_they_are():
+    torch.manual_seed(8)
+    x, w = _randn(8, 128), _randn(64, 128)
+    strided = _randn(64, 2)[:, 0]
+    assert torch.equal(RF.linear(x, w, strided), RF.linear(x, w, strided.contiguous()))
+    ids, table = torch.randint(0, 64, (9,), device="cuda"), _randn(64, 64).t()
+    assert torch.equal(RF.embedding(table, ids), table[ids])
+    logits, labels = _randn(8, 64), torch.arange(8, device="cuda")
+    assert torch.allclose(RF.cross_entropy(logits.clone(), labels, num_classes=99), F.cross_entropy(logits.float(), labels))
+    # running statistics that no kernel writes in place
+    img = _randn(4, 16, 5, 5).to(memory_format=torch.channels_last)
+    g, bt = torch.rand(16, 2, device="cuda")[:, 0], torch.rand(16, 2, device="cuda")[:, 1]
+    rm, rv = torch.zeros(16, 2, device="cuda")[:, 0], torch.ones(16, 2, device="cuda")[:, 0]
+    y = RF.batch_norm_act(img, g, bt, rm, rv)
+    rmr, rvr = torch.zeros(16, device="cuda"), torch.ones(16, device="cuda")
+    want = F.batch_norm(img.float(), rmr, rvr, g, bt, True)
+    assert _rel(y, want) < 2.0 ** -8 and torch.allclose(rm, rmr, atol=1e-5) and torch.allclose(rv, rvr, atol=1e-4)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+def test_a_weights_gradient_buffer_in_fp32_or_its_own_type(dtype):
+    torch.manual_seed(9)
+    x, dy = _randn(512, 128), _randn(512, 64)
+    w = _randn(64, 128).requires_grad_(True)
+    w.main_grad = torch.ones(64, 128, device="cuda", dtype=dtype)
+    RF.linear(x, w).backward(dy)
+    assert w.grad is None and _rel(w.main_grad, 1.0 + dy.double().t() @ x.double()) < (1e-5 if dtype == torch.float32 else 2.0 ** -8)
