@@ -95,6 +95,8 @@ struct GemmKernelParams {
     int staged;
     // MN-major operands: 1: all 64-column chunks of a stage in one copy (tensor map [chunk][row][64]); 0: one copy each
     int a_merged, b_merged;
+    // 1: the bias / the matrices beside the output / the output start their rows on 16-byte boundaries
+    int bias_al, in_al, out_al;
     float* a_colsum;   // not null: column sums of the stored A (MN-major) are added here
 };
 
@@ -539,8 +541,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         const bool act_dgelu = p.flags & RB_GEMM_DGELU;
         const bool aux_out = p.flags & RB_GEMM_AUX_OUT;
         const bool accum = p.flags & RB_GEMM_ACCUM;
-        const bool in_al = (p.ldd % 8 == 0);
-        const bool out_al = (sizeof(OutT) == 2) ? (p.ldd % 8 == 0) : (p.ldd % 4 == 0);
+        const bool bias_al = p.bias_al, in_al = p.in_al, out_al = p.out_al;
         auto release_acc = [&](int acc) {
             tc_fence_before();
             if constexpr (PAIR) {
@@ -603,7 +604,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     const uint64_t alpha2 = f2_pack(p.alpha, p.alpha);
                     if (has_bias) {
                         float t[32];
-                        load32(reinterpret_cast<const InT*>(p.bias) + col, full_chunk, valid, t);
+                        load32(reinterpret_cast<const InT*>(p.bias) + col, full_chunk && bias_al, valid, t);
 #pragma unroll
                         for (int j = 0; j < 32; j += 2)
                             f2_unpack(f2_fma(f2_pack_bits(r[j], r[j + 1]), alpha2, f2_pack(t[j], t[j + 1])), v[j], v[j + 1]);
@@ -763,7 +764,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                 }
                 if (has_bias) {
                     float t[32];
-                    load32(reinterpret_cast<const InT*>(p.bias) + col, full_chunk, valid, t);
+                    load32(reinterpret_cast<const InT*>(p.bias) + col, full_chunk && bias_al, valid, t);
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] += t[j];
                 }
@@ -1215,6 +1216,14 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
         for (int t = 0; t < a->wgrad_taps; ++t) p.conv_shift[t] = a->conv_shift[t];
     }
     if (a->map_hp > 0 && (a->batch != 1 || a->rs_nranks > 1 || a->map_wp <= 0)) return -7;
+
+    auto off16 = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) != 0; };
+    p.bias_al = !off16(a->bias);
+    p.in_al = !off16(a->residual) && !off16(a->aux_in) && !off16(a->aux_out) && a->ldd % 8 == 0 &&
+              (a->batch == 1 || a->strideD % 8 == 0);
+    const int64_t per16 = a->out_dtype == 1 ? 4 : 8;
+    p.out_al = !off16(a->D) && a->ldd % per16 == 0 && (a->batch == 1 || a->strideD % per16 == 0);
+    for (int r = 0; r < p.rs_nranks; ++r) p.out_al = p.out_al && !off16(a->rs_peer[r]);
 
     CUtensorMap tmA, tmB;
     int rc;

@@ -88,6 +88,10 @@ Tensor opt(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
 Tensor f32(at::IntArrayRef sizes, const Tensor& like) { return at::empty(sizes, like.options().dtype(at::kFloat)); }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 Tensor dense(const Tensor& t) { return !t.defined() || t.is_contiguous() ? t : t.contiguous(); }
+// contiguous and on a 16-byte boundary, for kernels that read whole vectors (a view may start at any element)
+Tensor dense16(const Tensor& t) {
+    return !t.defined() || (t.is_contiguous() && aligned16(t.data_ptr())) ? t : t.clone(at::MemoryFormat::Contiguous);
+}
 
 // ------------------------------------------------------------------------------------------------ operand checks
 // Kernels get bare addresses: they read an operand in the type, and as many elements of it, as the call's other operands
@@ -290,7 +294,7 @@ struct LinearNode : Node {
     }
     variable_list run(variable_list&& grads) {
         const Tensor X = x.unpack(), W = w.unpack(), P = pre.unpack();
-        Tensor dy = dense(grads[0]);
+        Tensor dy = P.defined() ? dense16(grads[0]) : dense(grads[0]);
         const int dt = dt_code(X);
         if (P.defined()) {
             Tensor d = at::empty(dy.sizes(), dy.options());
@@ -444,8 +448,8 @@ struct LnNode : Node {
         for (SavedVariable* s : {&z, &gamma, &mean, &rstd}) s->reset_data();
     }
     variable_list run(variable_list&& grads) {
-        const Tensor Z = z.unpack(), G = dense(gamma.unpack()), M = mean.unpack(), R = rstd.unpack();
-        const Tensor dy = dense(grads[0]);
+        const Tensor Z = z.unpack(), G = dense16(gamma.unpack()), M = mean.unpack(), R = rstd.unpack();
+        const Tensor dy = dense16(grads[0]);
         const int H = static_cast<int>(Z.size(-1)), rows = static_cast<int>(Z.numel() / H);
         const bool flat = g_mg.defined() && b_mg.defined();
         Tensor dz = at::empty(Z.sizes(), Z.options()), dx = dz;
@@ -481,8 +485,8 @@ Tensor layer_norm(const Tensor& x, const OptTensor& res_, const Tensor& gamma, c
     Tensor xc, y, z, mean, rstd;
     {
         at::NoGradGuard off;
-        xc = dense(x);
-        const Tensor rc = dense(res), gc = dense(gamma), bc = dense(beta);
+        xc = dense16(x);
+        const Tensor rc = dense16(res), gc = dense16(gamma), bc = dense16(beta);
         const int H = static_cast<int>(x.size(-1)), rows = static_cast<int>(x.numel() / H);
         y = at::empty(xc.sizes(), xc.options());
         if (res.defined() || p > 0) z = at::empty(xc.sizes(), xc.options());
@@ -548,7 +552,8 @@ Tensor embedding(const Tensor& w, const Tensor& ids, int64_t padding, const OptT
         auto sizes = ids.sizes().vec();
         sizes.push_back(w.size(1));
         out = at::empty(sizes, w.options().requires_grad(false));
-        check(api.embed_fwd(static_cast<const long long*>(idc.data_ptr()), w.data_ptr(), out.data_ptr(),
+        const Tensor table = dense16(w);
+        check(api.embed_fwd(static_cast<const long long*>(idc.data_ptr()), table.data_ptr(), out.data_ptr(),
                             static_cast<int>(ids.numel()), static_cast<int>(w.size(1)), w.size(0), dt_code(w), cur_stream()),
               "rb_embed_fwd");
     }
@@ -687,15 +692,14 @@ struct QkvNode : Node {
     }
     variable_list run(variable_list&& grads) {
         const Tensor X = x.unpack(), Q = qkv.unpack(), O = o.unpack(shared_from_this()), L = lse.unpack(), kb = bias.unpack();
-        const Tensor dO = dense(grads[0]);
+        const Tensor dO = dense16(grads[0]);
         const int dt = dt_code(X);
         const int64_t Ho = H * 64;
         Tensor dqkv = at::empty(Q.sizes(), Q.options());
         Tensor delta = f32({B, H, S}, Q), dq_acc = f32({B, S, H, 64}, Q);
         RbAttnArgs a;
         attn_args(a, Q, O, L, kb, B, S, H, scale, p, seed, offset);
-        Tensor dOa = aligned16(dO.data_ptr()) ? dO : dO.clone();
-        a.dO = dOa.data_ptr();
+        a.dO = dO.data_ptr();
         a.do_sb = S * Ho;
         a.do_ss = Ho;
         a.do_sh = 64;
@@ -826,7 +830,9 @@ Tensor qkv_attention(const Tensor& x, const std::vector<Tensor>& ws, const std::
 }
 
 // ------------------------------------------------------------------------------------------------ batch norm
-Tensor nhwc(const Tensor& t) { return t.contiguous(at::MemoryFormat::ChannelsLast); }
+Tensor nhwc(const Tensor& t) {   // channels-last on a 16-byte boundary
+    return t.is_contiguous(at::MemoryFormat::ChannelsLast) && aligned16(t.data_ptr()) ? t : t.clone(at::MemoryFormat::ChannelsLast);
+}
 struct BnNode : Node {
     SavedVariable x, y, mean, rstd, g32;
     Tensor gamma, beta, g_mg, b_mg;

@@ -86,6 +86,11 @@ def _aligned(t) -> bool:
     return t.data_ptr() % 16 == 0 and t.shape[-1] % 8 == 0 and t.shape[-1] > 0
 
 
+def _dense16(t):
+    """``t`` contiguous and on a 16-byte boundary, for kernels that read whole vectors."""
+    return t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
 def _bias_ok(bias, n, dtype) -> bool:
     """None, or ``n`` values of the type the kernels read beside the operands."""
     return bias is None or (bias.dtype == dtype and bias.numel() == n)
@@ -154,11 +159,11 @@ class _Dropout(torch.autograd.Function):
     def forward(ctx, x, p):
         ctx.p = p
         ctx.seed, ctx.offset = rng.next()
-        return K.dropout(x if x.is_contiguous() else x.contiguous(), p, ctx.seed, ctx.offset)
+        return K.dropout(_dense16(x), p, ctx.seed, ctx.offset)
 
     @staticmethod
     def backward(ctx, dy):
-        return K.dropout(dy if dy.is_contiguous() else dy.contiguous(), ctx.p, ctx.seed, ctx.offset), None
+        return K.dropout(_dense16(dy), ctx.p, ctx.seed, ctx.offset), None
 
 
 def dropout(x, p: float, training: bool = True):
@@ -172,14 +177,14 @@ def dropout(x, p: float, training: bool = True):
 class _Gelu(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x):
-        xc = x if x.is_contiguous() else x.contiguous()
+        xc = _dense16(x)
         ctx.save_for_backward(xc)
         return K.gelu(xc)
 
     @staticmethod
     def backward(ctx, dy):
         (x,) = ctx.saved_tensors
-        return K.gelu_bwd(x, dy if dy.is_contiguous() else dy.contiguous())
+        return K.gelu_bwd(x, _dense16(dy))
 
 
 def gelu(x):
@@ -239,7 +244,7 @@ def sdpa(q, k, v, attn_mask=None, dropout_p: float = 0.0, is_causal: bool = Fals
     if ok:
         qs, ks, vs = (t.transpose(1, 2) for t in (q, k, v))  # [B, S, H, D] views
         if not all(_attn_operand_ok(t) for t in (qs, ks, vs)):
-            qs, ks, vs = (t.contiguous() for t in (qs, ks, vs))
+            qs, ks, vs = (t.clone(memory_format=torch.contiguous_format) for t in (qs, ks, vs))
         sc = float(scale) if scale is not None else q.shape[-1] ** -0.5
         o = _Attention.apply(qs, ks, vs, key_bias, float(dropout_p), sc)
         return o.transpose(1, 2)
@@ -300,8 +305,10 @@ def qkv_attention(x, wq, bq, wk, bk, wv, bv, attn_mask=None, dropout_p: float = 
 
 # ----------------------------------------------------------------------------- convolution / batch norm
 def _nhwc(x):
-    """[N, H, W, C] contiguous view of a logically NCHW tensor (a copy only if it is not channels-last yet)."""
-    return x.contiguous(memory_format=torch.channels_last).permute(0, 2, 3, 1)
+    """[N, H, W, C] contiguous view of a logically NCHW tensor on a 16-byte boundary (a copy only if it is not
+    channels-last yet, or starts elsewhere)."""
+    cl = x.contiguous(memory_format=torch.channels_last)
+    return (cl if cl.data_ptr() % 16 == 0 else cl.clone()).permute(0, 2, 3, 1)
 
 
 def _conv_weight(w):

@@ -232,7 +232,7 @@ def attn_bwd(q, k, v, o, lse, do, key_bias=None, scale=None, p_drop=0.0, seed=0,
     B, S, H, D = q.shape
     scale = float(scale if scale is not None else D ** -0.5)
     if do.stride(3) != 1 or not _attn_ok(do):
-        do = do.contiguous()
+        do = do.clone(memory_format=torch.contiguous_format)
     dq = torch.empty(B, S, H, D, dtype=q.dtype, device=q.device) if dq is None else dq
     dk = torch.empty(B, S, H, D, dtype=q.dtype, device=q.device) if dk is None else dk
     dv = torch.empty(B, S, H, D, dtype=q.dtype, device=q.device) if dv is None else dv

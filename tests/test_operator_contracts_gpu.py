@@ -267,3 +267,72 @@ def test_a_weights_gradient_buffer_in_fp32_or_its_own_type(dtype):
     w.main_grad = torch.ones(64, 128, device="cuda", dtype=dtype)
     RF.linear(x, w).backward(dy)
     assert w.grad is None and _rel(w.main_grad, 1.0 + dy.double().t() @ x.double()) < (1e-5 if dtype == torch.float32 else 2.0 ** -8)
+
+
+def _off(t):
+    """The same values and strides, starting one element past a 16-byte boundary."""
+    buf = torch.empty(t.numel() + 1, device=t.device, dtype=t.dtype)
+    v = buf[1:].as_strided(t.shape, t.stride())
+    with torch.no_grad():
+        v.copy_(t)
+    assert v.data_ptr() % 16
+    return v
+
+
+def test_operands_that_start_at_any_element():
+    """The results are those of aligned copies, bit for bit, gradients included."""
+    torch.manual_seed(10)
+    cl = lambda *s: _randn(*s).to(memory_format=torch.channels_last)  # noqa: E731
+    ids = torch.randint(0, 33, (17,), device="cuda")
+    cases = {
+        "layer_norm": (lambda x, r, g, b: RF.dropout_add_layer_norm(x, r, g, b, 0.0, 1e-5),
+                       [_randn(9, 512), _randn(9, 512), _randn(512), _randn(512)]),
+        "gelu": (RF.gelu, [_randn(5, 24)]),
+        "embedding": (lambda w: RF.embedding(w, ids), [_randn(33, 64)]),
+        "linear bias": (lambda b, x=_randn(40, 64), w=_randn(96, 64): RF.linear(x, w, b, act="gelu"), [_randn(96)]),
+        "conv": (lambda x: RF.conv2d(x, w3, None, 1, 1), [cl(2, 64, 12, 12)]),
+        "strided conv": (lambda x: RF.conv2d(x, w3, None, 2, 1), [cl(2, 64, 12, 12)]),
+        "batch_norm": (lambda x, r, g, b: RF.batch_norm_act(x, g, b, None, None, relu=True, residual=r),
+                       [cl(2, 64, 5, 5), cl(2, 64, 5, 5), torch.rand(64, device="cuda"), torch.rand(64, device="cuda")]),
+        "sdpa": (lambda q, k, v: RF.sdpa(q, k, v), [_randn(2, 3, 20, 64) for _ in range(3)]),
+        "qkv": (lambda x, *p: RF.qkv_attention(x, *p, num_heads=2),
+                [_randn(2, 20, 128), _randn(128, 128), _randn(128), _randn(128, 128), _randn(128), _randn(128, 128), _randn(128)]),
+    }
+    w3 = _randn(64, 64, 3, 3, std=0.05)
+    for name, (fn, args) in cases.items():
+        got = []
+        for shift in (False, True):
+            # (the first projection weight and the attention input off a boundary select another path: left aligned)
+            leaves = [(_off(a) if shift and not (name == "qkv" and i in (0, 1)) else a.clone()).requires_grad_(True)
+                      for i, a in enumerate(args)]
+            y = fn(*leaves)
+            torch.manual_seed(11)
+            dy = torch.randn_like(y)
+            y.backward(_off(dy) if shift else dy)
+            got.append([y] + [t.grad for t in leaves])
+        tol = 2.0 ** -8 if name in ("batch_norm", "embedding") else 0.0      # sums whose order is not fixed
+        for a, b in zip(*got):
+            assert torch.equal(a, b) if tol == 0.0 else _rel(a, b) < tol, name
+    x = _randn(5, 24)
+    RF.manual_seed(3)
+    d0 = RF.dropout(x, 0.5)
+    RF.manual_seed(3)
+    assert torch.equal(RF.dropout(_off(x), 0.5), d0)
+
+
+@pytest.mark.parametrize("out_dtype", [BF, torch.float32])
+@pytest.mark.parametrize("M,N", [(3, 64), (150, 264)])
+def test_product_outputs_that_start_at_any_element(M, N, out_dtype):
+    from rannc_b200.ops.gemm import gemm
+
+    torch.manual_seed(12)
+    a, b, r = _randn(M, 72), _randn(N, 72, std=0.1), _randn(M, N)
+    bias, base = _randn(N), _randn(M, N, dtype=out_dtype)
+    want = gemm(a, b, bias=bias, residual=r, out=base.clone(), accumulate=True)
+    assert torch.equal(gemm(a, b, bias=_off(bias), residual=_off(r), out=_off(base), accumulate=True), want)
+    aux, pre = torch.empty(M, N, device="cuda", dtype=BF), _off(torch.zeros(M, N, device="cuda", dtype=BF))
+    y0, y1 = gemm(a, b, bias=bias, gelu=True, aux_out=aux), gemm(a, b, bias=bias, gelu=True, aux_out=pre)
+    # the two ways a result leaves the kernel evaluate GELU scalar by scalar and in pairs: a last fp32 bit apart, which 16-bit
+    # rounding may turn into one of its own
+    assert torch.equal(aux, pre) and _rel(y1, y0) < 2.0 ** -8
+    assert _rel(gemm(a, b, dgelu=True, aux_in=pre), gemm(a, b, dgelu=True, aux_in=aux)) < 2.0 ** -8
