@@ -975,7 +975,7 @@ int num_sms() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return 148;
-    if (!n[dev]) cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev);
+    if (!n[dev] && cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
     return n[dev];
 }
 
@@ -1061,6 +1061,72 @@ static bool pair_enabled() {
     return v == 1;
 }
 
+// How a product is cut up: the kernel variant, its output tiles, and the parts K is split into.
+struct Tiling {
+    bool pair;
+    int tn, m_blocks, n_blocks, split;
+};
+static Tiling choose_tiling(const RbGemmArgs& a) {
+    // The pair kernel (256 x 256 tile over two SMs) serves every GEMM with enough work to fill the GPU:
+    // enough tiles, or few tiles and a long K that is split (weight gradients); the gather prologue and the
+    // scatter epilogue are the same code in both variants.  Small problems stay on the single-CTA kernel.
+    const bool accum32 = a.out_dtype == 1 && a.flags == RB_GEMM_ACCUM;
+    Tiling t;
+    t.pair = pair_enabled() && (a.ag_nranks <= 1 || pair_gather_enabled());
+    if (t.pair) {
+        const long long pt = ((a.M + 2 * BM - 1) / (2 * BM)) * ((a.N + 255) / 256) * a.batch;
+        const long long kbs = (a.K + BK - 1) / BK;
+        if (pt < num_sms() / 2 && !(accum32 && a.M > BM && pt * (kbs / 4) >= num_sms() / 2)) t.pair = false;
+    }
+    t.m_blocks = static_cast<int>(t.pair ? (a.M + 2 * BM - 1) / (2 * BM) : (a.M + BM - 1) / BM);
+    const int num_kb = static_cast<int>((a.K + BK - 1) / BK);
+    const int units = t.pair ? num_sms() / 2 : num_sms();   // CTAs (or CTA pairs) that run at once
+    // Few output tiles and a long K (weight gradients): split K over CTAs and accumulate with
+    // reductions.  Only for fp32 outputs that accumulate and have no other epilogue work.
+    auto split_for = [&](int tiles) {
+        int split = 1;
+        if (accum32 && tiles < units && num_kb >= 8) {
+            double best = 0.0;
+            for (int s = 1; s <= 32 && s * 4 <= num_kb; ++s) {
+                const int work = tiles * s;
+                const int waves = (work + units - 1) / units;
+                const double eff = static_cast<double>(work) / (waves * units) - 0.005 * s;
+                if (eff > best + 1e-9) {
+                    best = eff;
+                    split = s;
+                }
+            }
+        }
+        return split;
+    };
+    t.tn = 256;
+    if (!t.pair && a.ag_nranks <= 1 && a.rs_nranks <= 1) {
+        if (a.tile_n == 64 || a.tile_n == 128 || a.tile_n == 256) {
+            t.tn = a.tile_n;
+        } else {
+            // Narrow tiles move more bytes per product but keep more SMs busy.  Estimated cycles: k steps one CTA
+            // does, each bound by its loads (48 / 32 / 24 KiB), plus the last tile's epilogue.  Measured with 256 /
+            // 128 / 64 columns (us): 32 x 1024 x 1024 10.1 / 9.0 / 8.5; 351 x 3072 x 768 9.5 / 8.7 / 8.0;
+            // 1182 x 768 x 2304 22.0 / 17.1 / 15.4; 2000 x 1024 x 1024 11.0 / 10.1 / 14.4;
+            // 1182 x 2304 x 768 9.9 / 13.0 / 16.2.  The rule took the best or one within 2 % in 21 of 22 shapes.
+            double best = 1e30;
+            for (int w : {256, 128, 64}) {
+                const int tiles = t.m_blocks * static_cast<int>((a.N + w - 1) / w * a.batch);
+                const int s = split_for(tiles);
+                const double steps = static_cast<double>((tiles * s + units - 1) / units) * ((num_kb + s - 1) / s);
+                const double cost = steps * (w == 256 ? 768 : (w == 128 ? 512 : 384)) + 12.0 * w;
+                if (cost < 0.98 * best) {
+                    best = cost;
+                    t.tn = w;
+                }
+            }
+        }
+    }
+    t.n_blocks = static_cast<int>((a.N + t.tn - 1) / t.tn);
+    t.split = split_for(t.m_blocks * t.n_blocks * static_cast<int>(a.batch));
+    return t;
+}
+
 }  // namespace rb
 
 extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
@@ -1089,61 +1155,12 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     p.batch = static_cast<int>(a->batch);
     p.a_major = a->a_major;
     p.b_major = a->b_major;
-    // The pair kernel (256 x 256 tile over two SMs) serves every GEMM with enough work to fill the GPU:
-    // enough tiles, or few tiles and a long K that is split (weight gradients); the gather prologue and the
-    // scatter epilogue are the same code in both variants.  Small problems stay on the single-CTA kernel.
-    const bool accum32 = a->out_dtype == 1 && a->flags == RB_GEMM_ACCUM;
-    bool pair = pair_enabled() && (a->ag_nranks <= 1 || pair_gather_enabled());
-    if (pair) {
-        const long long pt = ((a->M + 2 * BM - 1) / (2 * BM)) * ((a->N + 255) / 256) * a->batch;
-        const long long kbs = (a->K + BK - 1) / BK;
-        if (pt < num_sms() / 2 && !(accum32 && a->M > BM && pt * (kbs / 4) >= num_sms() / 2)) pair = false;
-    }
-    p.num_m_blocks = pair ? (p.M + 2 * BM - 1) / (2 * BM) : (p.M + BM - 1) / BM;
+    const Tiling tiling = choose_tiling(*a);
+    const bool pair = tiling.pair;
+    const int tn = tiling.tn;
+    p.num_m_blocks = tiling.m_blocks;
     p.num_kb = (p.K + BK - 1) / BK;
-    const int units = pair ? num_sms() / 2 : num_sms();   // CTAs (or CTA pairs) that run at once
-    // Few output tiles and a long K (weight gradients): split K over CTAs and accumulate with
-    // reductions.  Only for fp32 outputs that accumulate and have no other epilogue work.
-    auto split_for = [&](int tiles) {
-        int split = 1;
-        if (accum32 && tiles < units && p.num_kb >= 8) {
-            double best = 0.0;
-            for (int s = 1; s <= 32 && s * 4 <= p.num_kb; ++s) {
-                const int work = tiles * s;
-                const int waves = (work + units - 1) / units;
-                const double eff = static_cast<double>(work) / (waves * units) - 0.005 * s;
-                if (eff > best + 1e-9) {
-                    best = eff;
-                    split = s;
-                }
-            }
-        }
-        return split;
-    };
-    int tn = 256;
-    if (!pair && a->ag_nranks <= 1 && a->rs_nranks <= 1) {
-        if (a->tile_n == 64 || a->tile_n == 128 || a->tile_n == 256) {
-            tn = a->tile_n;
-        } else {
-            // Narrow tiles move more bytes per product but keep more SMs busy.  Estimated cycles: k steps one CTA
-            // does, each bound by its loads (48 / 32 / 24 KiB), plus the last tile's epilogue.  Measured with 256 /
-            // 128 / 64 columns (us): 32 x 1024 x 1024 10.1 / 9.0 / 8.5; 351 x 3072 x 768 9.5 / 8.7 / 8.0;
-            // 1182 x 768 x 2304 22.0 / 17.1 / 15.4; 2000 x 1024 x 1024 11.0 / 10.1 / 14.4;
-            // 1182 x 2304 x 768 9.9 / 13.0 / 16.2.  The rule took the best or one within 2 % in 21 of 22 shapes.
-            double best = 1e30;
-            for (int t : {256, 128, 64}) {
-                const int tiles = p.num_m_blocks * ((p.N + t - 1) / t) * p.batch;
-                const int s = split_for(tiles);
-                const double steps = static_cast<double>((tiles * s + units - 1) / units) * ((p.num_kb + s - 1) / s);
-                const double cost = steps * (t == 256 ? 768 : (t == 128 ? 512 : 384)) + 12.0 * t;
-                if (cost < 0.98 * best) {
-                    best = cost;
-                    tn = t;
-                }
-            }
-        }
-    }
-    p.num_n_blocks = (p.N + tn - 1) / tn;
+    p.num_n_blocks = tiling.n_blocks;
     p.base_tiles = p.num_m_blocks * p.num_n_blocks * p.batch;
     p.ag_nranks = a->ag_nranks > 1 ? a->ag_nranks : 0;
     p.ag_my_idx = a->ag_my_idx;
@@ -1167,7 +1184,7 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     if (p.rs_nranks > 1 && (a->out_dtype != 1 || a->flags != RB_GEMM_ACCUM || a->N % a->rs_nranks || p.rs_cols % 32 ||
                             a->rs_nranks > 8 || a->batch != 1))
         return -5;
-    p.split_k = split_for(p.base_tiles);
+    p.split_k = tiling.split;
     p.kb_per_split = (p.num_kb + p.split_k - 1) / p.split_k;
     p.split_k = (p.num_kb + p.kb_per_split - 1) / p.kb_per_split;
     p.num_tiles = p.base_tiles * p.split_k;
@@ -1289,6 +1306,15 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
 
     return a->in_dtype == 1 ? dispatch<__nv_bfloat16>(*a, pair, tn, tmA, tmB, tmD, tmAux, p, stream)
                             : dispatch<__half>(*a, pair, tn, tmA, tmB, tmD, tmAux, p, stream);
+}
+
+// Parts that the K dimension of an fp32 [M, N] += product is split into: 1 when its tiles fill the GPU by themselves
+extern "C" int rb_gemm_splits(long long M, long long N, long long K) {
+    RbGemmArgs a = {};
+    a.M = M, a.N = N, a.K = K, a.batch = 1;
+    a.out_dtype = 1;
+    a.flags = RB_GEMM_ACCUM;
+    return M > 0 && N > 0 && K > 0 ? rb::choose_tiling(a).split : 1;
 }
 
 // Copies the device error word into `host_dst` (pinned host memory) on `stream` without waiting: the caller

@@ -35,6 +35,7 @@ using OptTensor = std::optional<Tensor>;
 // ------------------------------------------------------------------------------------------------ C ABI
 struct Api {
     int (*gemm)(const RbGemmArgs*, void*);
+    int (*gemm_splits)(long long, long long, long long);
     int (*gelu)(const void*, const void*, void*, long long, int, int, void*);
     int (*colsum)(const void*, float*, int, int, long long, int, void*);
     int (*ln_fwd)(const void*, const void*, const void*, const void*, void*, void*, float*, float*, int, int, float,
@@ -220,13 +221,14 @@ Grads param_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& w_
         if (w_mg.defined()) {
             e.accumulate = true;
             gemm(dy, x, true, false, w_mg.data_ptr(), w_mg.scalar_type() == at::kFloat, dtype, e, w_mg.stride(0));
-        } else if (dy.rows >= std::max<int64_t>(2048, 256 * ((dy.cols + 255) / 256) * ((x.cols + 255) / 256))) {
+        } else if (dy.rows >= std::max<int64_t>(2048, 256 * ((dy.cols + 255) / 256) * ((x.cols + 255) / 256)) &&
+                   api.gemm_splits(dy.cols, x.cols, dy.rows) > 1) {
             // A long product with few 256 x 256 tiles leaves most of the GPU idle unless K is split, which takes an
             // fp32 result to add to: clearing it and rounding it are two more passes over the weight.  Measured, one
             // 16-bit product against clear + split + round (us, weight at rows): 256 x 256 at 2048 14.9 / 9.0;
             // 768 x 768 at 1024 10.0 / 10.9, at 8192 46.7 / 19.6; 1024 x 1024 at 2048 15.8 / 16.5, at 4096
             // 26.7 / 21.5; 3072 x 768 at 16384 104.5 / 66.6; 4096 x 1024 at 8192 71.9 / 73.3, at 16384 134 / 121:
-            // the line lies at 256 rows per tile.
+            // the line lies at 256 rows per tile.  Where the tiles fill the GPU the fp32 result would gain nothing.
             Tensor w32 = at::zeros({dy.cols, x.cols}, w.options().dtype(at::kFloat));
             e.accumulate = true;
             gemm(dy, x, true, false, w32.data_ptr(), true, dtype, e);
@@ -980,6 +982,7 @@ void init(const std::unordered_map<std::string, uintptr_t>& fns, py::object erro
         slot = reinterpret_cast<std::remove_reference_t<decltype(slot)>>(fns.at(name));
     };
     set(api.gemm, "rb_gemm");
+    set(api.gemm_splits, "rb_gemm_splits");
     set(api.gelu, "rb_gelu");
     set(api.colsum, "rb_colsum");
     set(api.ln_fwd, "rb_ln_fwd");

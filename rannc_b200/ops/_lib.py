@@ -19,7 +19,7 @@ _lib = None
 
 # device kernels launched per C entry point (the optimizer / element-wise entries launch one)
 _KERNELS_PER_CALL = {"rb_bn_fwd": 2, "rb_bn_bwd": 2, "rb_ln_bwd": 2, "rb_xent_fwd": 2, "rb_attn_bwd": 3, "rb_read_error": 0, "rb_ln_supported": 0,
-                     "rb_ln_bwd_grid": 0, "rb_error_peek_async": 0}
+                     "rb_ln_bwd_grid": 0, "rb_gemm_splits": 0, "rb_error_peek_async": 0}
 _launches = 0
 
 
@@ -84,7 +84,7 @@ def lib() -> ctypes.CDLL:
 
 
 _host = None
-_HOST_ENTRIES = ("rb_gemm", "rb_gelu", "rb_colsum", "rb_ln_fwd", "rb_ln_bwd", "rb_ln_bwd16", "rb_ln_bwd_grid", "rb_embed_fwd",
+_HOST_ENTRIES = ("rb_gemm", "rb_gemm_splits", "rb_gelu", "rb_colsum", "rb_ln_fwd", "rb_ln_bwd", "rb_ln_bwd16", "rb_ln_bwd_grid", "rb_embed_fwd",
                  "rb_embed_bwd", "rb_xent_fwd", "rb_xent_bwd", "rb_attn_fwd", "rb_attn_bwd", "rb_bn_fwd", "rb_bn_bwd")
 
 

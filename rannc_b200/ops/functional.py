@@ -18,7 +18,7 @@ import torch
 from . import _lib
 from . import kernels as K
 from ..utils.config import conf
-from .gemm import gemm
+from .gemm import gemm, splits
 
 
 # ----------------------------------------------------------------------------- RNG
@@ -364,8 +364,7 @@ class _Conv2d(torch.autograd.Function):
     @staticmethod
     def _wgrad32(dy2, act, shifts=None):
         """fp32 dy^T act (with ``shifts``: one block of columns per filter tap).  The GEMM splits a long K over the GPU
-        only when it accumulates: a product with fewer 256 x 256 tiles than the GPU has SM pairs is added to zeros, a
-        larger one is stored."""
+        only when it accumulates: a product it would split is added to zeros, any other is stored."""
         cols = act.shape[1] * (len(shifts) if shifts is not None else 1)
         Co = dy2.shape[1]
         if shifts is not None and not dy2.is_cuda:
@@ -376,10 +375,10 @@ class _Conv2d(torch.autograd.Function):
                 gemm(dy2, act, trans_a=True, trans_b=False, out=dw2[:, t * C:(t + 1) * C], accumulate=True,
                      b_row_shift=sh)
             return dw2
-        few = ((Co + 255) // 256) * ((cols + 255) // 256) < 74
-        dw2 = (torch.zeros if few else torch.empty)(Co, cols, dtype=torch.float32, device=dy2.device)
+        split = splits(Co, cols, dy2.shape[0]) > 1
+        dw2 = (torch.zeros if split else torch.empty)(Co, cols, dtype=torch.float32, device=dy2.device)
         more = {} if shifts is None else {"wgrad_shifts": shifts}
-        return gemm(dy2, act, trans_a=True, trans_b=False, out=dw2, accumulate=few, **more)
+        return gemm(dy2, act, trans_a=True, trans_b=False, out=dw2, accumulate=split, **more)
 
     @staticmethod
     def _fold(dw2, w, w_mg, k):

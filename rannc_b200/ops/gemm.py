@@ -68,6 +68,11 @@ def _mat(t: torch.Tensor):
     raise ValueError("gemm operands must be 2-D or 3-D")
 
 
+def splits(M: int, N: int, K: int) -> int:
+    """Parts that K is split into when an [M, N] product is added to an fp32 matrix (1: its tiles fill the GPU)."""
+    return int(_lib.lib().rb_gemm_splits(ctypes.c_longlong(M), ctypes.c_longlong(N), ctypes.c_longlong(K)))
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bool = True,
          bias=None, residual=None, aux_in=None, aux_out=None, gelu: bool = False,
          dgelu: bool = False, out: torch.Tensor | None = None, accumulate: bool = False,

@@ -336,3 +336,17 @@ def test_product_outputs_that_start_at_any_element(M, N, out_dtype):
     # rounding may turn into one of its own
     assert torch.equal(aux, pre) and _rel(y1, y0) < 2.0 ** -8
     assert _rel(gemm(a, b, dgelu=True, aux_in=pre), gemm(a, b, dgelu=True, aux_in=aux)) < 2.0 ** -8
+
+
+# ------------------------------------------------------------------------------------------ weight gradients
+def test_a_product_that_cannot_be_split_makes_no_fp32_copy():
+    rows, K, N = 24576, 2048, 3072          # 12 x 8 tiles of 256 x 256: more than the SM pairs that run at once
+    x, dy = _randn(rows, K), _randn(rows, N)
+    w = _randn(N, K).requires_grad_(True)
+    y = RF.linear(x, w)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    y.backward(dy)
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - before < 1.5 * w.numel() * 2
