@@ -9,6 +9,7 @@
 // Kernels are called through the C ABI of _kernels.so; their addresses are handed over once by ops/_lib.py, so that
 // the regular and the checked build of the library serve the same code.
 // Reference counterpart: the interpreter loop of src/torch/TorchDriver.cpp:566.
+#include <ATen/Context.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/forward_grad.h>
@@ -222,13 +223,15 @@ Grads param_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& w_
             e.accumulate = true;
             gemm(dy, x, true, false, w_mg.data_ptr(), w_mg.scalar_type() == at::kFloat, dtype, e, w_mg.stride(0));
         } else if (dy.rows >= std::max<int64_t>(2048, 256 * ((dy.cols + 255) / 256) * ((x.cols + 255) / 256)) &&
-                   api.gemm_splits(dy.cols, x.cols, dy.rows) > 1) {
+                   !at::globalContext().deterministicAlgorithms() && api.gemm_splits(dy.cols, x.cols, dy.rows) > 1) {
             // A long product with few 256 x 256 tiles leaves most of the GPU idle unless K is split, which takes an
             // fp32 result to add to: clearing it and rounding it are two more passes over the weight.  Measured, one
             // 16-bit product against clear + split + round (us, weight at rows): 256 x 256 at 2048 14.9 / 9.0;
             // 768 x 768 at 1024 10.0 / 10.9, at 8192 46.7 / 19.6; 1024 x 1024 at 2048 15.8 / 16.5, at 4096
             // 26.7 / 21.5; 3072 x 768 at 16384 104.5 / 66.6; 4096 x 1024 at 8192 71.9 / 73.3, at 16384 134 / 121:
             // the line lies at 256 rows per tile.  Where the tiles fill the GPU the fp32 result would gain nothing.
+            // The parts are added in the order they arrive, so the last bits differ from run to run: not when
+            // torch.use_deterministic_algorithms asks otherwise.
             Tensor w32 = at::zeros({dy.cols, x.cols}, w.options().dtype(at::kFloat));
             e.accumulate = true;
             gemm(dy, x, true, false, w32.data_ptr(), true, dtype, e);

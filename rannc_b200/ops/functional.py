@@ -364,7 +364,8 @@ class _Conv2d(torch.autograd.Function):
     @staticmethod
     def _wgrad32(dy2, act, shifts=None):
         """fp32 dy^T act (with ``shifts``: one block of columns per filter tap).  The GEMM splits a long K over the GPU
-        only when it accumulates: a product it would split is added to zeros, any other is stored."""
+        only when it accumulates: a product it would split is added to zeros, any other is stored.  The parts are added
+        in the order they arrive; ``torch.use_deterministic_algorithms`` keeps the product in one piece."""
         cols = act.shape[1] * (len(shifts) if shifts is not None else 1)
         Co = dy2.shape[1]
         if shifts is not None and not dy2.is_cuda:
@@ -375,7 +376,7 @@ class _Conv2d(torch.autograd.Function):
                 gemm(dy2, act, trans_a=True, trans_b=False, out=dw2[:, t * C:(t + 1) * C], accumulate=True,
                      b_row_shift=sh)
             return dw2
-        split = splits(Co, cols, dy2.shape[0]) > 1
+        split = not torch.are_deterministic_algorithms_enabled() and splits(Co, cols, dy2.shape[0]) > 1
         dw2 = (torch.zeros if split else torch.empty)(Co, cols, dtype=torch.float32, device=dy2.device)
         more = {} if shifts is None else {"wgrad_shifts": shifts}
         return gemm(dy2, act, trans_a=True, trans_b=False, out=dw2, accumulate=split, **more)

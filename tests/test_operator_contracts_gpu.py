@@ -350,3 +350,25 @@ def test_a_product_that_cannot_be_split_makes_no_fp32_copy():
     y.backward(dy)
     torch.cuda.synchronize()
     assert torch.cuda.max_memory_allocated() - before < 1.5 * w.numel() * 2
+
+
+@pytest.mark.parametrize("op", ["linear", "conv"])
+def test_weight_gradients_repeat_when_asked(op):
+    """Products that add up partial sums in the order they arrive give way to one that does not."""
+    torch.manual_seed(5)
+    if op == "linear":
+        x, w, dy = _randn(16384, 256), _randn(256, 256).requires_grad_(True), _randn(16384, 256)
+        run = lambda: RF.linear(x, w)  # noqa: E731
+    else:
+        x, w, dy = _randn(16, 64, 28, 28), _randn(64, 64, 3, 3).requires_grad_(True), _randn(16, 64, 14, 14)
+        run = lambda: RF.conv2d(x, w, None, 2, 1)  # noqa: E731
+    torch.use_deterministic_algorithms(True)
+    try:
+        grads = []
+        for _ in range(8):
+            w.grad = None
+            run().backward(dy)
+            grads.append(w.grad)
+        assert all(torch.equal(g, grads[0]) for g in grads)
+    finally:
+        torch.use_deterministic_algorithms(False)
