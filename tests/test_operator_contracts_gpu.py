@@ -372,3 +372,39 @@ def test_weight_gradients_repeat_when_asked(op):
         assert all(torch.equal(g, grads[0]) for g in grads)
     finally:
         torch.use_deterministic_algorithms(False)
+
+
+@pytest.mark.parametrize("rows", [64, 4096])
+def test_projection_gradients_have_their_own_storage(rows):
+    x = _randn(rows // 64, 64, 128).requires_grad_(True)
+    ws = [_randn(128, 128).requires_grad_(True) for _ in range(3)]
+    bs = [_randn(128).requires_grad_(True) for _ in range(3)]
+    _attention(x, ws, bs, 2).sum().backward()
+    grads = [t.grad for t in ws + bs]
+    assert len({g.untyped_storage().data_ptr() for g in grads}) == len(grads)
+    assert all(g.untyped_storage().nbytes() == g.numel() * g.element_size() for g in grads)
+    version = grads[1]._version
+    grads[0].mul_(2)
+    assert grads[1]._version == version
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,heads,hid,bias", [(37, 1, 8, True), (300, 2, 264, False), (4100, 1, 128, True), (197, 3, 72, True)])
+def test_projection_gradients_leave_one_product(dtype, rows, heads, hid, bias):
+    """Stored and split products, one vector per part up to many; with and without biases."""
+    torch.manual_seed(13)
+    n = 64 * heads
+    x = _randn(1, rows, hid, dtype=dtype)
+    ws = [_randn(n, hid, std=hid ** -0.5, dtype=dtype).requires_grad_(True) for _ in range(3)]
+    bs = [_randn(n, dtype=dtype).requires_grad_(True) if bias else None for _ in range(3)]
+    y = RF.qkv_attention(x, ws[0], bs[0], ws[1], bs[1], ws[2], bs[2], num_heads=heads)
+    dy = _randn(*y.shape, dtype=dtype)
+    y.backward(dy)
+    wr = [w.detach().double().requires_grad_(True) for w in ws]
+    br = [(b if bias else x.new_zeros(n)).detach().double().requires_grad_(True) for b in bs]
+    _attention_ref(x, wr, br, heads).backward(dy.double())
+    # dQ, dK and dV are rounded to 16 bits on their way, and the probabilities before them
+    tol = 6 * (2.0 ** -8 if dtype == BF else 2.0 ** -11)
+    for i, (got, want) in enumerate(zip(ws + (bs if bias else []), wr + br)):
+        # (the key bias shifts all scores of a row: its gradient is zero but for rounding)
+        assert i == 4 or _rel(got.grad, want.grad) < tol, i
