@@ -309,12 +309,14 @@ void notify(std::initializer_list<std::pair<const Tensor*, const Tensor*>> param
     }
     Py_DECREF(r);
 }
-#define RB_NODE(NAME)                                       \
-    std::string name() const override { return NAME; }      \
-    variable_list apply(variable_list&& grads) override {   \
-        std::lock_guard<std::mutex> lock(mutex_);            \
-        if (!grads[0].defined()) return variable_list(num_outputs()); \
-        return run(std::move(grads));                        \
+// A gradient that never arrived counts as zero: the parameters' buffers are complete and reported all the same, which is
+// what a gradient reducer waits for.
+#define RB_NODE(NAME)                                                              \
+    std::string name() const override { return NAME; }                             \
+    variable_list apply(variable_list&& grads) override {                          \
+        std::lock_guard<std::mutex> lock(mutex_);                                   \
+        if (!grads[0].defined()) grads[0] = input_metadata(0).zeros_like();        \
+        return run(std::move(grads));                                               \
     }
 
 // ------------------------------------------------------------------------------------------------ linear

@@ -408,3 +408,36 @@ def test_projection_gradients_leave_one_product(dtype, rows, heads, hid, bias):
     for i, (got, want) in enumerate(zip(ws + (bs if bias else []), wr + br)):
         # (the key bias shifts all scores of a row: its gradient is zero but for rounding)
         assert i == 4 or _rel(got.grad, want.grad) < tol, i
+
+
+# ------------------------------------------------------------------------------------------ autograd, threads
+class _NoGradient(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, y):
+        return y.clone()
+
+    @staticmethod
+    def backward(ctx, dy):
+        return None
+
+
+@pytest.mark.parametrize("op", ["linear", "layer_norm", "embedding"])
+def test_a_missing_gradient_counts_as_zero_and_is_reported(op):
+    """A parameter with a gradient buffer is reported although nothing flows back: a reducer counts on it."""
+    w = _randn(256, 256).requires_grad_(True)
+    g, b = _randn(256).requires_grad_(True), _randn(256).requires_grad_(True)
+    for p in (w, g, b):
+        p.main_grad = torch.zeros(p.shape, device="cuda")
+    x = _randn(8, 256).requires_grad_(True)
+    y = {"linear": lambda: RF.linear(x, w), "layer_norm": lambda: RF.dropout_add_layer_norm(x, None, g, b),
+         "embedding": lambda: RF.embedding(w, torch.arange(8, device="cuda"))}[op]()
+    seen = []
+    RF.set_grad_listener(lambda ps: seen.extend(ps))
+    try:
+        _NoGradient.apply(y).sum().backward()
+    finally:
+        RF.set_grad_listener(None)
+    want = [g, b] if op == "layer_norm" else [w]
+    assert len(seen) == len(want) and all(any(s is p for s in seen) for p in want)
+    assert all(float(p.main_grad.abs().max()) == 0.0 for p in want)
+    assert op == "embedding" or (x.grad is not None and float(x.grad.abs().max()) == 0.0)
