@@ -1037,7 +1037,10 @@ void set_listener(py::object fn) {
     has_listener.store(listener != nullptr, std::memory_order_release);
 }
 
-// Errors cross the boundary as the exceptions they are (the library's own error class, ValueError, TypeError, ...).
+// Errors cross the boundary as the exceptions they are (the library's own error class, ValueError, TypeError, ...).  The
+// interpreter lock is released meanwhile, as PyTorch's own operators do it: an allocation that has to wait, or a launch
+// into a full queue, must not stop the other Python threads.  (What needs the interpreter takes the lock itself: errors,
+// gradient listeners, saved-tensor hooks.)
 template <typename F>
 struct Guarded;
 template <typename R, typename... A>
@@ -1047,6 +1050,7 @@ struct Guarded<R (*)(A...)> {
         R result{};
         auto body = [&]() -> bool {
             HANDLE_TH_ERRORS
+            py::gil_scoped_release unlocked;
             result = F(std::forward<A>(a)...);
             return true;
             END_HANDLE_TH_ERRORS_RET(false)

@@ -441,3 +441,39 @@ def test_a_missing_gradient_counts_as_zero_and_is_reported(op):
     assert len(seen) == len(want) and all(any(s is p for s in seen) for p in want)
     assert all(float(p.main_grad.abs().max()) == 0.0 for p in want)
     assert op == "embedding" or (x.grad is not None and float(x.grad.abs().max()) == 0.0)
+
+
+def test_other_threads_run_while_a_launch_waits():
+    """The launch queue is filled behind a kernel that runs for 0.6 s; a thread that does nothing but look at the clock must
+    not stand still for the time the launches wait."""
+    import threading
+    import time
+
+    x, w = _randn(32, 256), _randn(256, 256)
+    with torch.no_grad():
+        RF.linear(x, w)
+        torch.cuda.synchronize()
+        stop, gap = threading.Event(), [0.0]
+
+        def watch():
+            last = time.perf_counter()
+            while not stop.is_set():
+                time.sleep(0.001)
+                now = time.perf_counter()
+                gap[0] = max(gap[0], now - last)
+                last = now
+
+        th = threading.Thread(target=watch)
+        th.start()
+        time.sleep(0.05)
+        torch.cuda._sleep(int(0.6 * 1.9e9))
+        t0 = time.perf_counter()
+        for _ in range(4096):
+            RF.linear(x, w)
+        waited = time.perf_counter() - t0
+        stop.set()
+        th.join()
+        torch.cuda.synchronize()
+    if waited < 0.4:
+        pytest.skip("the launch queue took all launches")
+    assert gap[0] < 0.2, gap[0]
