@@ -325,6 +325,7 @@ struct LinearNode : Node {
     Tensor w_ref, bias, w_mg, b_mg;
     RB_NODE("RbLinearBackward")
     void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
         x.reset_data();
         w.reset_data();
         pre.reset_data();
@@ -398,6 +399,7 @@ struct MlpNode : Node {
     Tensor w1_ref, w2_ref, b1, b2, w1_mg, b1_mg, w2_mg, b2_mg;
     RB_NODE("RbMlpBackward")
     void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
         for (SavedVariable* s : {&x, &w1, &w2, &pre, &h}) s->reset_data();
     }
     variable_list run(variable_list&& grads) {
@@ -482,6 +484,7 @@ struct LnNode : Node {
     uint64_t seed = 0, offset = 0;
     RB_NODE("RbLayerNormBackward")
     void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
         for (SavedVariable* s : {&z, &gamma, &mean, &rstd}) s->reset_data();
     }
     variable_list run(variable_list&& grads) {
@@ -560,7 +563,10 @@ struct EmbeddingNode : Node {
     Tensor weight, w_mg;
     int64_t padding = -1;
     RB_NODE("RbEmbeddingBackward")
-    void release_variables() override { ids.reset_data(); }
+    void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        ids.reset_data();
+    }
     variable_list run(variable_list&& grads) {
         const Tensor I = ids.unpack();
         const Tensor dy = dense(grads[0]);
@@ -613,6 +619,7 @@ struct XentNode : Node {
     double weight = 1;
     RB_NODE("RbCrossEntropyBackward")
     void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
         for (SavedVariable* s : {&logits, &labels, &lse, &acc}) s->reset_data();
     }
     variable_list run(variable_list&& grads) {
@@ -725,6 +732,7 @@ struct QkvNode : Node {
     uint64_t seed = 0, offset = 0;
     RB_NODE("RbQkvAttentionBackward")
     void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
         for (SavedVariable* s : {&x, &qkv, &o, &lse, &bias, &stack}) s->reset_data();
     }
     variable_list run(variable_list&& grads) {
@@ -872,6 +880,7 @@ struct BnNode : Node {
     bool relu = false, has_res = false;
     RB_NODE("RbBatchNormBackward")
     void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
         for (SavedVariable* s : {&x, &y, &mean, &rstd, &g32}) s->reset_data();
     }
     variable_list run(variable_list&& grads) {

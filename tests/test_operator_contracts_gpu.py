@@ -477,3 +477,27 @@ def test_other_threads_run_while_a_launch_waits():
     if waited < 0.4:
         pytest.skip("the launch queue took all launches")
     assert gap[0] < 0.2, gap[0]
+
+
+def test_two_threads_differentiate_one_graph():
+    """One keeps the graph, one releases it: each gets the gradient, or autograd's error about a released graph."""
+    import threading
+
+    torch.manual_seed(14)
+    w, x = _randn(64, 64).requires_grad_(True), _randn(16, 64)
+    want = torch.autograd.grad(RF.linear(x, w, act="gelu").sum(), w)[0]
+    for _ in range(100):
+        y, out = RF.linear(x, w, act="gelu").sum(), []
+
+        def go(keep):
+            try:
+                out.append(torch.autograd.grad(y, w, retain_graph=keep)[0])
+            except RuntimeError as e:
+                out.append(e)
+
+        ts = [threading.Thread(target=go, args=(k,)) for k in (True, False)]
+        [t.start() for t in ts]
+        [t.join() for t in ts]
+        assert len(out) == 2
+        for o in out:
+            assert torch.equal(o, want) if torch.is_tensor(o) else "second time" in str(o) or "already been freed" in str(o)
