@@ -113,9 +113,10 @@ def build_core(verbose: bool = False) -> Path:
     return out
 
 
-def build_host(verbose: bool = False) -> Path:
+def build_host(verbose: bool = False, force: bool = False) -> Path:
     """The fused operators' host side (``csrc/host/*.cpp``: autograd nodes and launches) against PyTorch's C++ API.
-    It calls the kernels through addresses it is given at run time, so it links to no CUDA code."""
+    It calls the kernels through addresses it is given at run time, so it links to no CUDA code.  ``force``: also when
+    the library is newer than its sources (it may have been built against another PyTorch)."""
     import torch
     from torch.utils.cpp_extension import include_paths
 
@@ -123,15 +124,17 @@ def build_host(verbose: bool = False) -> Path:
     out = HERE / ("_host" + ext)
     srcs = sorted(HOST_SRC.glob("*.cpp"))
     hdrs = [CUDA_SRC / "attn.h", CUDA_SRC / "gemm_tcgen05.h"]
-    if _newer(out, srcs + hdrs):
+    if not force and _newer(out, srcs + hdrs):
         return out
     inc = [d for p in include_paths() + [sysconfig.get_paths()["include"]] for d in ("-isystem", p)]
     cuda = Path(_nvcc()).parent.parent / "include"
     lib = Path(torch.__file__).resolve().parent / "lib"
+    tmp = out.with_name(f"{out.name}.{os.getpid()}")
     log = _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall", "-pthread",
                 "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-                *inc, "-isystem", str(cuda), *map(str, srcs), "-o", str(out), "-L", str(lib), f"-Wl,-rpath,{lib}",
+                *inc, "-isystem", str(cuda), *map(str, srcs), "-o", str(tmp), "-L", str(lib), f"-Wl,-rpath,{lib}",
                 "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"])
+    os.replace(tmp, out)   # several ranks may build at once: nobody loads half a library
     if verbose:
         print(log)
     return out

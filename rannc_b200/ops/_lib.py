@@ -111,7 +111,9 @@ def host():
             from .. import build
 
             try:
-                build.build_host()
+                # missing, or built against another PyTorch: then it is newer than its sources and fails to load
+                build.build_host(force=True)
+                importlib.invalidate_caches()
                 mod = importlib.import_module("rannc_b200._host")
             except Exception as e:  # noqa: BLE001
                 raise KernelLibraryError(f"cannot build the operators' host side: {e}") from e
