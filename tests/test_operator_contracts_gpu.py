@@ -501,3 +501,21 @@ def test_two_threads_differentiate_one_graph():
         assert len(out) == 2
         for o in out:
             assert torch.equal(o, want) if torch.is_tensor(o) else "second time" in str(o) or "already been freed" in str(o)
+
+
+@pytest.mark.parametrize("bias", [-1e4, -1e6, -1e9, -1e15, -2e38])
+def test_attention_backward_of_fully_masked_rows(bias):
+    """A sequence that is all padding under a finite mask value: scores are rounded away beside it.  A single key has
+    probability one, so dV is dO; of many keys none may exceed it."""
+    torch.manual_seed(15)
+    q, k, v, do = (_randn(1, 1, 2, 64, std=2.0) for _ in range(4))
+    mask = torch.full((1, 1), bias, device="cuda")
+    o, lse = RF.K.attn_fwd(q, k, v, mask)
+    assert torch.equal(RF.K.attn_bwd(q, k, v, o, lse, do, mask)[2], do)
+    B, S, H = 2, 160, 2
+    q, k, v, do = (_randn(B, S, H, 64, std=2.0) for _ in range(4))
+    mask = torch.full((B, S), bias, device="cuda")
+    o, lse = RF.K.attn_fwd(q, k, v, mask)
+    dv = RF.K.attn_bwd(q, k, v, o, lse, do, mask)[2]
+    # each of S probabilities is at most one (a few roundings of 2^-8 above)
+    assert bool((dv.abs().double() <= do.double().abs().sum(1, keepdim=True) * 1.02).all())
