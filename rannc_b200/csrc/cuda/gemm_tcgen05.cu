@@ -86,7 +86,7 @@ struct GemmKernelParams {
     int flags;
     int* err;
     // implicit-GEMM convolution: see RbGemmArgs
-    int conv_kb_per_tap, conv_b_tap_cols, b_row_shift;
+    int conv_kb_per_tap, conv_b_tap_cols;
     int wgrad_taps, wgrad_cols;
     int map_hp, map_wp, map_h, map_w, map_pad;
     int conv_shift[49];
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     uint8_t* b_dst = sB + stage * B_STAGE_BYTES;
                     const int k0 = kb * BK;
                     // A (K-major) reads columns ax of rows ay..; B (MN-major) reads columns +bx of rows bk..
-                    int ax = k0, ay = m0, bx = 0, bk = k0 + p.b_row_shift;
+                    int ax = k0, ay = m0, bx = 0, bk = k0;
                     if (p.conv_kb_per_tap > 0) {
                         const int tap = kb / p.conv_kb_per_tap;
                         ax = (kb - tap * p.conv_kb_per_tap) * BK;
@@ -1201,7 +1201,6 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     if (!p.err) return -3;
     p.conv_kb_per_tap = 0;
     p.conv_b_tap_cols = 0;
-    p.b_row_shift = a->b_major != 0 ? a->b_row_shift : 0;
     p.map_hp = a->map_hp;
     p.map_wp = a->map_wp;
     p.map_h = a->map_h;
@@ -1225,7 +1224,7 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     if (a->wgrad_taps > 0) {
         // a 64-column block of B must lie within one tap
         if (a->wgrad_taps > 49 || a->conv_taps > 0 || a->b_major != 1 || a->conv_c % 64 || a->conv_c <= 0 ||
-            a->N != static_cast<int64_t>(a->wgrad_taps) * a->conv_c || a->batch != 1 || a->b_row_shift ||
+            a->N != static_cast<int64_t>(a->wgrad_taps) * a->conv_c || a->batch != 1 ||
             a->ag_nranks > 1 || a->rs_nranks > 1)
             return -7;
         p.wgrad_taps = a->wgrad_taps;

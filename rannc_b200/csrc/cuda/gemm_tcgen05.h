@@ -50,7 +50,6 @@ typedef struct RbGemmArgs {
     // read as zero.  With B stored [K, N] (b_major = 1) tap t's block starts conv_b_tap_cols * t columns further
     // right and its rows are the tap's own channel range.  No filter-sized copy of the activation exists.
     int32_t conv_taps, conv_c, conv_b_tap_cols;
-    int32_t b_row_shift;   // b_major = 1: the rows of B that k-block kb reads start at kb * 64 + b_row_shift
     int32_t conv_shift[49];
     // output rows are positions of the padded grid: only the interior (map_pad <= y < map_pad + map_h, same for
     // x) is stored, at row (n * map_h + y - map_pad) * map_w + (x - map_pad) of D.  map_hp = 0: rows are rows.
@@ -60,7 +59,6 @@ typedef struct RbGemmArgs {
     // shifted by conv_shift[t].  One launch for all taps: the gradient operand A is read once per column of
     // tiles instead of once per tap.
     int32_t wgrad_taps;
-    int32_t reserved_;
     float* a_colsum;  // a_major = 1 only: the column sums of the stored A ([K, M]) are added to these M floats
     int32_t tile_n;   // columns of the single-CTA kernel's tile: 0 (chosen by size), 64, 128 or 256
 } RbGemmArgs;

@@ -368,14 +368,6 @@ class _Conv2d(torch.autograd.Function):
         in the order they arrive; ``torch.use_deterministic_algorithms`` keeps the product in one piece."""
         cols = act.shape[1] * (len(shifts) if shifts is not None else 1)
         Co = dy2.shape[1]
-        if shifts is not None and not dy2.is_cuda:
-            # the same addressing tap by tap, as the host-side check of it spells it out
-            C = act.shape[1]
-            dw2 = torch.zeros(Co, cols, dtype=torch.float32)
-            for t, sh in enumerate(shifts):
-                gemm(dy2, act, trans_a=True, trans_b=False, out=dw2[:, t * C:(t + 1) * C], accumulate=True,
-                     b_row_shift=sh)
-            return dw2
         split = not torch.are_deterministic_algorithms_enabled() and splits(Co, cols, dy2.shape[0]) > 1
         dw2 = (torch.zeros if split else torch.empty)(Co, cols, dtype=torch.float32, device=dy2.device)
         more = {} if shifts is None else {"wgrad_shifts": shifts}

@@ -26,10 +26,10 @@ class _Args(ctypes.Structure):
         ("ag_nranks", ctypes.c_int32), ("ag_my_idx", ctypes.c_int32), ("ag_rows", ctypes.c_int32),
         ("ag_cols", ctypes.c_int32), ("ag_flags", ctypes.c_void_p), ("ag_src", ctypes.c_void_p * 8),
         ("conv_taps", ctypes.c_int32), ("conv_c", ctypes.c_int32), ("conv_b_tap_cols", ctypes.c_int32),
-        ("b_row_shift", ctypes.c_int32), ("conv_shift", ctypes.c_int32 * 49),
+        ("conv_shift", ctypes.c_int32 * 49),
         ("map_hp", ctypes.c_int32), ("map_wp", ctypes.c_int32), ("map_h", ctypes.c_int32),
         ("map_w", ctypes.c_int32), ("map_pad", ctypes.c_int32), ("wgrad_taps", ctypes.c_int32),
-        ("reserved_", ctypes.c_int32), ("a_colsum", ctypes.c_void_p), ("tile_n", ctypes.c_int32),
+        ("a_colsum", ctypes.c_void_p), ("tile_n", ctypes.c_int32),
     ]
 
 
@@ -77,7 +77,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
          bias=None, residual=None, aux_in=None, aux_out=None, gelu: bool = False,
          dgelu: bool = False, out: torch.Tensor | None = None, accumulate: bool = False,
          out_dtype: torch.dtype | None = None, alpha: float = 1.0, max_ctas: int = 0,
-         rs_peers=None, rs_ld: int = 0, gather=None, conv=None, b_row_shift: int = 0,
+         rs_peers=None, rs_ld: int = 0, gather=None, conv=None,
          row_map=None, wgrad_shifts=None, tile_n: int = 0,
          a_colsum=None) -> torch.Tensor:
     """``out = epilogue(alpha * op(a) @ op(b))``.
@@ -90,7 +90,6 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
     channels-last activation as ``[rows, C]``; the product runs over K = T x C, k-block by k-block reading the
     rows shifted by ``shifts[tap]`` (rows outside ``a`` read as zero).  ``b`` is ``[N, T*C]`` (``trans_b=True``) or
     ``[C, T*b_tap_cols]`` with tap t's ``[C, N]`` block at column ``t * b_tap_cols`` (``trans_b=False``).
-    ``b_row_shift`` (``trans_b=False`` only): the rows of ``b`` a k-block reads are shifted by this many.
     ``wgrad_shifts`` (``trans_b=False`` only): ``b`` is the padded activation ``[rows, C]`` and the result has one
     block of C columns per shift, ``a``'s product with the rows of ``b`` shifted by it (weight gradient of a
     convolution, all taps in one launch).
@@ -100,7 +99,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
     stored, at the un-padded row index (``out`` has N_img * H * W rows).
     """
     if a.dim() == 2 and b.dim() == 2 and (out is None or out.dim() == 2) and rs_peers is None and gather is None and \
-            conv is None and row_map is None and wgrad_shifts is None and not b_row_shift and not tile_n and \
+            conv is None and row_map is None and wgrad_shifts is None and not tile_n and \
             a_colsum is None:
         odt = out_dtype or (out.dtype if out is not None else a.dtype)
         return _lib.host().product(a, b, trans_a, trans_b, bias, residual, aux_in, aux_out, gelu, dgelu, out, accumulate,
@@ -122,7 +121,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
                 raise ValueError("gemm: weight matrix does not hold the taps' blocks")
         K = Kb = T * ac
     if wgrad_shifts is not None:
-        if trans_b or b.dim() != 2 or a.dim() != 2 or conv is not None or b_row_shift or bc % 64:
+        if trans_b or b.dim() != 2 or a.dim() != 2 or conv is not None or bc % 64:
             raise ValueError("gemm: wgrad_shifts needs a 2-D b stored [rows, C], C a multiple of 64")
         N = bc * len(wgrad_shifts)
     if K != Kb:
@@ -188,10 +187,6 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         args.conv_c = bc
         for i, sh in enumerate(wgrad_shifts):
             args.conv_shift[i] = int(sh)
-    if b_row_shift:
-        if trans_b:
-            raise ValueError("gemm: b_row_shift needs b stored [K, N]")
-        args.b_row_shift = int(b_row_shift)
     if row_map is not None:
         args.map_hp, args.map_wp, args.map_h, args.map_w, args.map_pad = (int(v) for v in row_map)
     rc = _lib.lib().rb_gemm(ctypes.byref(args), _lib.stream_ptr())

@@ -4,8 +4,9 @@
 over the zero-padded channels-last activation, a padded-grid-to-output row map, and tap blocks of the weight matrix.
 Here the GEMM is replaced by a plain PyTorch function that follows the kernel's documented addressing rules (rows
 outside the matrix read as zero, tap t's block of a [K, N] operand starts ``b_tap_cols * t`` columns further right,
-``b_row_shift`` shifts the rows of the [K, N] operand, only interior rows of the padded grid are stored), and the
-Function's forward, input gradient and weight gradient are compared with ``torch.nn.functional.conv2d``."""
+with ``wgrad_shifts`` column block t is the product with the [K, C] operand's rows shifted by shifts[t], only interior
+rows of the padded grid are stored), and the Function's forward, input gradient and weight gradient are compared
+with ``torch.nn.functional.conv2d``.  A keyword the rules do not know is an error, not ignored."""
 import pytest
 import torch
 
@@ -24,7 +25,7 @@ def _shifted_rows(m: torch.Tensor, shift: int) -> torch.Tensor:
 
 
 def _gemm_by_the_rules(a, b, *, trans_a=False, trans_b=True, bias=None, out=None, accumulate=False, out_dtype=None,
-                       conv=None, b_row_shift=0, row_map=None, **_):
+                       conv=None, row_map=None, wgrad_shifts=None):
     a32, b32 = a.float(), b.float()
     if conv is not None:
         taps, chans = conv["taps"], a.shape[1]
@@ -38,7 +39,10 @@ def _gemm_by_the_rules(a, b, *, trans_a=False, trans_b=True, bias=None, out=None
         res = lhs @ rhs
     else:
         lhs = a32.t() if trans_a else a32
-        rhs = b32.t() if trans_b else (_shifted_rows(b32, b_row_shift) if b_row_shift else b32)
+        rhs = b32.t() if trans_b else b32
+        if wgrad_shifts is not None:
+            assert trans_a and not trans_b and b.shape[1] % 64 == 0
+            rhs = torch.cat([_shifted_rows(b32, sh) for sh in wgrad_shifts], 1)               # [rows, taps * C]
         res = lhs @ rhs
     if bias is not None:
         res = res + bias.float()
