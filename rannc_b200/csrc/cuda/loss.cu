@@ -98,7 +98,7 @@ template <typename T>
 __global__ void __launch_bounds__(XT)
     xent_bwd_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
                     const float* __restrict__ lse_in, const float* __restrict__ acc,
-                    const float* __restrict__ gout, T* __restrict__ dlogits, int V, long long ld,
+                    const float* __restrict__ gout, T* __restrict__ dlogits, int V, int cols, long long ld,
                     long long ignore_index, float weight) {
     const int row = blockIdx.x;
     const long long label = labels[row];
@@ -109,9 +109,11 @@ __global__ void __launch_bounds__(XT)
     const float lse = lse_in[row];
     const bool vec = (ld % 8 == 0) && ((reinterpret_cast<uintptr_t>(logits) & 15) == 0) &&
                      ((reinterpret_cast<uintptr_t>(dlogits) & 15) == 0);
-    const int width = static_cast<int>(ld);  // also clears padding columns [V, ld)
+    // the row's own columns, padding [V, cols) included, which is cleared; what lies between cols and ld belongs to
+    // another tensor (the logits may be a slice of a wider matrix)
+    const int nv = vec ? cols / 8 : 0;
     if (vec) {
-        for (int i = threadIdx.x; i < width / 8; i += XT) {
+        for (int i = threadIdx.x; i < nv; i += XT) {
             uint4 q = make_uint4(0, 0, 0, 0);
             if (live) {
                 q = *reinterpret_cast<const uint4*>(x + i * 8);
@@ -126,15 +128,14 @@ __global__ void __launch_bounds__(XT)
             }
             *reinterpret_cast<uint4*>(d + i * 8) = q;
         }
-    } else {
-        for (int c = threadIdx.x; c < width; c += XT) {
-            float v = 0.f;
-            if (live && c < V) {
-                v = __expf(to_f32<T>(x[c]) - lse);
-                if (c == label) v -= 1.f;
-            }
-            d[c] = from_f32<T>(v * g);
+    }
+    for (int c = nv * 8 + threadIdx.x; c < cols; c += XT) {
+        float v = 0.f;
+        if (live && c < V) {
+            v = __expf(to_f32<T>(x[c]) - lse);
+            if (c == label) v -= 1.f;
         }
+        d[c] = from_f32<T>(v * g);
     }
 }
 
@@ -160,19 +161,20 @@ extern "C" int rb_xent_fwd(const void* logits, const long long* labels, float* l
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
+// cols: columns of the logits (V and padding), rows ld apart
 extern "C" int rb_xent_bwd(const void* logits, const long long* labels, const float* lse,
                            const float* acc, const float* gout, void* dlogits, int rows, int V,
-                           long long ld, long long ignore_index, float weight, int dtype,
+                           int cols, long long ld, long long ignore_index, float weight, int dtype,
                            void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (rows <= 0) return 0;
     if (dtype == 1)
         xent_bwd_kernel<__nv_bfloat16><<<rows, XT, 0, st>>>(
             static_cast<const __nv_bfloat16*>(logits), labels, lse, acc, gout,
-            static_cast<__nv_bfloat16*>(dlogits), V, ld, ignore_index, weight);
+            static_cast<__nv_bfloat16*>(dlogits), V, cols, ld, ignore_index, weight);
     else
         xent_bwd_kernel<__half><<<rows, XT, 0, st>>>(static_cast<const __half*>(logits), labels,
                                                      lse, acc, gout, static_cast<__half*>(dlogits),
-                                                     V, ld, ignore_index, weight);
+                                                     V, cols, ld, ignore_index, weight);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

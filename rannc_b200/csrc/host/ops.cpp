@@ -52,7 +52,7 @@ struct Api {
     int (*embed_bwd)(const long long*, const void*, float*, int, int, long long, long long, int, void*);
     int (*xent_fwd)(const void*, const long long*, float*, float*, float*, int, int, long long, long long, float, int,
                     void*);
-    int (*xent_bwd)(const void*, const long long*, const float*, const float*, const float*, void*, int, int, long long,
+    int (*xent_bwd)(const void*, const long long*, const float*, const float*, const float*, void*, int, int, int, long long,
                     long long, float, int, void*);
     int (*attn_fwd)(const RbAttnArgs*, void*);
     int (*attn_bwd)(const RbAttnArgs*, void*);
@@ -628,8 +628,8 @@ struct XentNode : Node {
         // the logits are dead after the loss: their buffer receives the gradient
         Tensor d = L.detach();
         check(api.xent_bwd(L.data_ptr(), static_cast<const long long*>(lab.data_ptr()), mptr<float>(ls), mptr<float>(ac),
-                           mptr<float>(g), d.data_ptr(), static_cast<int>(L.size(0)), static_cast<int>(V), L.stride(0),
-                           ignore, static_cast<float>(weight), dt_code(L), cur_stream()),
+                           mptr<float>(g), d.data_ptr(), static_cast<int>(L.size(0)), static_cast<int>(V),
+                           static_cast<int>(L.size(1)), L.stride(0), ignore, static_cast<float>(weight), dt_code(L), cur_stream()),
               "rb_xent_bwd");
         return {d};
     }
@@ -639,7 +639,7 @@ Tensor cross_entropy(const Tensor& logits, const Tensor& labels, int64_t V, int6
     TORCH_CHECK_TYPE(labels.scalar_type() == at::kLong && labels.device() == logits.device(),
                      "cross_entropy: the labels are 64-bit integers on the logits' device");
     TORCH_CHECK_VALUE(logits.dim() == 2 && logits.stride(1) == 1 && labels.is_contiguous() &&
-                          labels.numel() == logits.size(0) && V > 0 && V <= logits.size(1),
+                          (logits.size(0) <= 1 || logits.stride(0) >= logits.size(1)) && labels.numel() == logits.size(0) && V > 0 && V <= logits.size(1),
                       "cross_entropy: one label per row of logits, and no more classes than columns");
     const bool req = wants_grad({&logits});
     Tensor lse, acc, loss;

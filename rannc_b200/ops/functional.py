@@ -261,8 +261,8 @@ def cross_entropy(logits, labels, num_classes=None, ignore_index: int = -100, we
     ld = logits.shape[-1]
     V = int(num_classes) if num_classes is not None else ld
     l2 = logits.reshape(-1, ld)
-    if not (_kernel_ok(l2) and l2.stride(1) == 1 and 0 < V <= ld and labels.dtype == torch.int64 and labels.is_cuda and
-            labels.numel() == l2.shape[0]):
+    if not (_kernel_ok(l2) and l2.stride(1) == 1 and (l2.shape[0] <= 1 or l2.stride(0) >= ld) and 0 < V <= ld and
+            labels.dtype == torch.int64 and labels.is_cuda and labels.numel() == l2.shape[0]):
         return torch.nn.functional.cross_entropy(l2[:, :V].float(), labels.reshape(-1), ignore_index=ignore_index) * weight
     # the logits are dead after the loss: backward writes the gradient over them
     return _host().cross_entropy(l2, labels.reshape(-1).contiguous(), V, ignore_index, float(weight))

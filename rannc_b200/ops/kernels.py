@@ -142,10 +142,12 @@ def xent_fwd(logits2d, labels, V, ignore_index=-100, weight=1.0):
 
 
 def xent_bwd(logits2d, labels, lse, acc, gout, V, ignore_index=-100, weight=1.0, inplace=True):
-    d = logits2d if inplace else torch.empty_like(logits2d)
+    d = logits2d if inplace else torch.empty_strided(logits2d.shape, logits2d.stride(), dtype=logits2d.dtype,
+                                                     device=logits2d.device)
     _lib.check(_lib.lib().rb_xent_bwd(_lib.vp(logits2d), _lib.vp(labels), _lib.vp(lse), _lib.vp(acc), _lib.vp(gout),
                                       _lib.vp(d), c_int(logits2d.shape[0]), c_int(V),
-                                      c_longlong(logits2d.stride(0)), c_longlong(ignore_index), c_float(weight),
+                                      c_int(logits2d.shape[1]), c_longlong(logits2d.stride(0)),
+                                      c_longlong(ignore_index), c_float(weight),
                                       c_int(dt_code(logits2d)), _lib.stream_ptr()), "rb_xent_bwd")
     return d
 

@@ -519,3 +519,36 @@ def test_attention_backward_of_fully_masked_rows(bias):
     dv = RF.K.attn_bwd(q, k, v, o, lse, do, mask)[2]
     # each of S probabilities is at most one (a few roundings of 2^-8 above)
     assert bool((dv.abs().double() <= do.double().abs().sum(1, keepdim=True) * 1.02).all())
+
+
+@pytest.mark.parametrize("first,last", [(0, 72), (8, 72), (8, 68), (3, 70), (0, 61)])
+@pytest.mark.parametrize("classes", [None, 50])
+def test_loss_of_a_slice_writes_only_the_slice(first, last, classes):
+    """The gradient is written over the logits: not over what lies beside them in a wider matrix."""
+    torch.manual_seed(16)
+    whole = torch.zeros(9, 80, device="cuda", dtype=BF)
+    whole[:8, :72] = _randn(8, 72)
+    kept = whole.clone()
+    logits = whole[:8, first:last].detach().requires_grad_(True)
+    labels = torch.randint(0, 50, (8,), device="cuda")
+    labels[3] = -100
+    ref = kept[:8, first:last].double().requires_grad_(True)
+    want = F.cross_entropy(ref[:, :classes], labels)
+    want.backward()
+    loss = RF.cross_entropy(logits, labels, num_classes=classes)
+    loss.backward()
+    assert abs(float(loss) - float(want)) < 1e-5 * abs(float(want))
+    assert logits.grad.shape == ref.shape and _rel(logits.grad, ref.grad) < 2.0 ** -8
+    beside = torch.ones_like(whole, dtype=torch.bool)
+    beside[:8, first:last] = False
+    assert torch.equal(whole[beside], kept[beside])
+
+
+def test_loss_of_rows_that_share_memory():
+    torch.manual_seed(17)
+    row, labels = _randn(1, 40).requires_grad_(True), torch.arange(8, device="cuda")
+    loss = RF.cross_entropy(row.expand(8, 40), labels)
+    loss.backward()
+    ref = row.detach().double().requires_grad_(True)
+    F.cross_entropy(ref.expand(8, 40), labels).backward()
+    assert _rel(row.grad, ref.grad) < 8 * 2.0 ** -8       # eight rows' gradients, each rounded
