@@ -293,3 +293,24 @@ def test_linear_weight_gradient_both_sides_of_the_split(dtype, rows, K, N):
     steps = rows / 16 * 2.0 ** -23
     _near(w.grad, dy.double().t() @ x.double(), dtype, 1, steps)
     _near(b.grad, dy.double().sum(0), dtype, 1, steps)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N,tile_n,max_ctas", [(160, 256, 2), (160, 0, 2), (416, 256, 3), (96, 128, 2), (32, 64, 1), (160, 0, 0)])
+def test_staged_blocks_of_many_tiles(dtype, N, tile_n, max_ctas):
+    """Tiles with an odd number of 32-column blocks per warp, many to a CTA and with short main loops: the two halves of the
+    staging memory must keep taking turns across tiles, or a block is overwritten while the copy engine reads it.  Every
+    value is a small whole number, so a block of another tile is seen exactly."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops.gemm import gemm
+
+    M, K = 128 * 300 + 5, 64
+    torch.manual_seed(9)
+    a = torch.zeros(M, K, device="cuda", dtype=dtype)
+    a[:, :8] = torch.randint(-3, 4, (M, 8), device="cuda").to(dtype)
+    b = torch.randint(-3, 4, (N, K), device="cuda").to(dtype)
+    want = (a.float() @ b.float().t()).to(dtype)
+    for _ in range(5):
+        assert torch.equal(gemm(a, b, tile_n=tile_n, max_ctas=max_ctas), want)
+    torch.cuda.synchronize()
+    assert _lib.read_error() == 0
