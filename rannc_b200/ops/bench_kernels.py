@@ -67,7 +67,9 @@ def main():
     ap.add_argument("--k", type=int, default=1024)
     ap.add_argument("--layout", default="nt", help="nt: forward, nn: dgrad, tn: wgrad")
     ap.add_argument("--acc", action="store_true", help="fp32 output with accumulation (wgrad epilogue)")
-    ap.add_argument("--gelu", action="store_true")
+    ap.add_argument("--gelu", action="store_true", help="bias and GELU in the epilogue")
+    ap.add_argument("--aux", action="store_true", help="... and the value before the activation as a second output")
+    ap.add_argument("--bias-grad", action="store_true", help="tn: column sums of the first operand beside the product")
     ap.add_argument("--batch", type=int, default=8)
     ap.add_argument("--heads", type=int, default=16)
     ap.add_argument("--seq", type=int, default=512)
@@ -95,7 +97,10 @@ def main():
         B = torch.randn((N, Kd) if tb else (Kd, N), device="cuda", dtype=dt)
         D = torch.zeros(M, N, device="cuda", dtype=torch.float32 if a.acc else dt)
         bias = torch.randn(N, device="cuda", dtype=dt) if a.gelu else None
-        fn = lambda: gemm(A, B, trans_a=ta, trans_b=tb, out=D, accumulate=a.acc, bias=bias, gelu=a.gelu)  # noqa: E731
+        pre = torch.empty(M, N, device="cuda", dtype=dt) if a.aux else None
+        sums = torch.zeros(M, device="cuda") if a.bias_grad else None
+        fn = lambda: gemm(A, B, trans_a=ta, trans_b=tb, out=D, accumulate=a.acc, bias=bias, gelu=a.gelu,  # noqa: E731
+                          aux_out=pre, a_colsum=sums)
         t = _time(fn, a.iters, a.warmup, not a.no_flush)
         fl = 2.0 * M * N * Kd
         out.update(M=M, N=N, K=Kd, layout=a.layout, acc=a.acc, ms=t * 1e3, tflops=fl / t / 1e12,

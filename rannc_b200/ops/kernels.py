@@ -310,9 +310,12 @@ def pack_taps(w):
 
 
 def wgrad_fold_ok(dst) -> bool:
-    """Whether ``wgrad_fold`` takes this [Co, Ci, k, k] destination: one grid row per filter, and a row of 132 floats
-    per tap within 48 KiB of shared memory (filters up to 9 x 9)."""
-    return (dst.is_cuda and dst.is_contiguous() and dst.shape[0] <= 65535 and dst.shape[2] * dst.shape[3] <= 93 and
+    """Whether ``wgrad_fold`` should serve this [Co, Ci, k, k] destination.  It can up to 9 x 9 (a row of 132 floats per tap
+    within 48 KiB of shared memory) and 65535 filters (one grid row each).  Up to 3 x 3 a strided copy or addition is
+    faster (us, kernel / strided: 1024 x 1024 x 3 x 3 added to fp32 43 / 37, rounded to 16 bits 35 / 27; 2048 x 2048 139 /
+    125 and 113 / 86), from 5 x 5 on the kernel (1024 x 1024 x 5 x 5 72 / 107 and 57 / 80; 7 x 7 125 / 229 and 92 / 182):
+    the strided side reads 4 bytes of every k * k * 4."""
+    return (dst.is_cuda and dst.is_contiguous() and dst.shape[0] <= 65535 and 9 < dst.shape[2] * dst.shape[3] <= 93 and
             dst.dtype in (torch.bfloat16, torch.float16, torch.float32))
 
 

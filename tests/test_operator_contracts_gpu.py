@@ -552,3 +552,21 @@ def test_loss_of_rows_that_share_memory():
     ref = row.detach().double().requires_grad_(True)
     F.cross_entropy(ref.expand(8, 40), labels).backward()
     assert _rel(row.grad, ref.grad) < 8 * 2.0 ** -8       # eight rows' gradients, each rounded
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("k,kernel", [(1, False), (3, False), (4, True), (5, True), (9, True), (10, False)])
+@pytest.mark.parametrize("Co,Ci", [(3, 8), (5, 264)])
+def test_weight_gradient_folds_on_both_sides_of_the_rule(dtype, k, kernel, Co, Ci):
+    """Added to an fp32 buffer or written in the filter's type, by the kernel or the strided operation."""
+    dw2 = torch.randn(Co, k * k * Ci, device="cuda")
+    w = torch.zeros(Co, Ci, k, k, device="cuda", dtype=BF if dtype == torch.float32 else dtype)
+    want = dw2.view(Co, k, k, Ci).permute(0, 3, 1, 2)
+    if dtype == torch.float32:
+        mg = torch.ones(Co, Ci, k, k, device="cuda")
+        assert RF.K.wgrad_fold_ok(mg) == kernel and RF._Conv2d._fold(dw2, w, mg, k) is None
+        assert torch.equal(mg, 1.0 + want)
+    else:
+        assert RF.K.wgrad_fold_ok(w) == kernel
+        got = RF._Conv2d._fold(dw2, w, None, k)
+        assert got.is_contiguous() and torch.equal(got, want.to(dtype))
