@@ -174,8 +174,10 @@ static int pack_taps_launch(const void* src, void* dst, int Co, int Ci, int taps
 
 // The weight gradient comes out of its GEMM as src [Co, taps, Ci] fp32 and belongs into a [Co, Ci, taps] tensor:
 // added to an fp32 gradient buffer (ADD) or rounded to a 16-bit gradient.  A block takes 128 channels of one
-// filter through shared memory so that both sides are touched in whole lines; the row stride (4 banks) keeps the
-// transposed reads of a 3 x 3 filter nearly conflict-free.
+// filter through shared memory so that both sides are touched in whole lines; the row stride shifts the banks by four
+// from tap to tap.  For filters from 4 x 4 to 9 x 9: a strided copy reads 4 bytes of every 4 * taps, which costs it
+// 107 us for 1024 x 1024 x 5 x 5 (added to fp32) where this takes 72, but only 37 us for 3 x 3 where this takes 43 --
+// a block's loads, its barrier and its stores follow one another with little in flight.
 constexpr int FOLD_C = 128, FOLD_LD = FOLD_C + 4;
 template <typename OutT, bool ADD>
 __global__ void __launch_bounds__(256)

@@ -1247,10 +1247,10 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     const uint64_t sB = a->batch > 1 ? a->strideB * 2 : (a->b_major == 0 ? a->N : a->K) * a->ldb * 2;
     // An MN-major operand of whole 64-column chunks is seen as [chunk][row][64], so that one copy brings all chunks of a
     // stage.  The copies are issued one by one, and with two or four per operand and stage it was their number, not
-    // the bytes, that kept the tensor core waiting (57 % active): 8192 x 4096 x 8192, both operands MN-major, 421 ->
-    // 391 us, with fp32 accumulation 434 -> 402 us; 1024 x 9216 x 26912 445 -> 366 us.  A last chunk that the matrix
-    // fills only in part would read past its rows, and column blocks that straddle filter taps need a shift each:
-    // those keep a copy per chunk.
+    // the bytes, that kept the tensor core waiting (4096 x 1024 x 32768: its pipe 69 % active that way and 73 % now,
+    // 210 -> 190 us): 8192 x 4096 x 8192, both operands MN-major, 421 -> 391 us, with fp32 accumulation 434 -> 402 us;
+    // 1024 x 9216 x 26912 445 -> 366 us.  A last chunk that the matrix fills only in part would read past its rows, and
+    // column blocks that straddle filter taps need a shift each: those keep a copy per chunk.
     const int b_cols = pair ? 128 : tn;   // columns of B one CTA loads
     p.a_merged = a->a_major == 1 && a->M % 64 == 0;
     p.b_merged = a->b_major == 1 && (a->conv_taps > 0    ? a->conv_b_tap_cols % 64 == 0

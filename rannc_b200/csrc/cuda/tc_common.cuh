@@ -441,7 +441,8 @@ __device__ __forceinline__ float ex2_approx(float x) {
     return r;
 }
 // GELU with the exact (erf) form.  Phi(x) = 0.5 (1 + erf(x / sqrt 2)) comes from the rational-exponential
-// approximation erf(z) = 1 - (a1 t + ... + a5 t^5) exp(-z^2), t = 1 / (1 + p z), z >= 0 (absolute error
+// approximation 7.1.26 of Abramowitz and Stegun, Handbook of Mathematical Functions (after Hastings):
+// erf(z) = 1 - (a1 t + ... + a5 t^5) exp(-z^2), t = 1 / (1 + p z), z >= 0 (absolute error
 // below 2e-7, far under 16-bit output precision): one reciprocal, one exponential and seven FMAs instead
 // of the library erff's branches.  The lower tail is formed without cancellation (Phi(x) = q for x < 0),
 // and exp(-z^2) = exp(-x^2 / 2) is shared with the density in the gradient.

@@ -639,7 +639,8 @@ Tensor cross_entropy(const Tensor& logits, const Tensor& labels, int64_t V, int6
     TORCH_CHECK_TYPE(labels.scalar_type() == at::kLong && labels.device() == logits.device(),
                      "cross_entropy: the labels are 64-bit integers on the logits' device");
     TORCH_CHECK_VALUE(logits.dim() == 2 && logits.stride(1) == 1 && labels.is_contiguous() &&
-                          (logits.size(0) <= 1 || logits.stride(0) >= logits.size(1)) && labels.numel() == logits.size(0) && V > 0 && V <= logits.size(1),
+                          (logits.size(0) <= 1 || logits.stride(0) >= logits.size(1)) &&
+                          labels.numel() == logits.size(0) && V > 0 && V <= logits.size(1),
                       "cross_entropy: one label per row of logits, and no more classes than columns");
     const bool req = wants_grad({&logits});
     Tensor lse, acc, loss;
