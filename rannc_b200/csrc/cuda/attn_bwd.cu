@@ -536,6 +536,10 @@ static int launch_bwd(const RbAttnArgs& a, cudaStream_t st) {
 extern "C" int rb_attn_bwd(const RbAttnArgs* a, void* stream) {
     if (a->D != 64) return -2;
     if (a->B <= 0 || a->H <= 0 || a->S <= 0) return 0;
+    // (the tensor maps check the bases and strides of Q, K, V, dO and the dQ scratch)
+    if (rb::off16(a->O, a->dQ, a->dK, a->dV) || (a->o_sb | a->o_ss | a->o_sh | a->dq_sb | a->dq_ss | a->dq_sh) % 8 ||
+        (a->dk_sb | a->dk_ss | a->dk_sh | a->dv_sb | a->dv_ss | a->dv_sh) % 8)
+        return -5;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     return a->dtype == 1 ? rb::launch_bwd<__nv_bfloat16>(*a, st) : rb::launch_bwd<__half>(*a, st);
 }

@@ -866,6 +866,7 @@ static int launch_fwd(const RbAttnArgs& a, cudaStream_t st) {
 extern "C" int rb_attn_fwd(const RbAttnArgs* a, void* stream) {
     if (a->D != 64) return -2;
     if (a->B <= 0 || a->H <= 0 || a->S <= 0) return 0;
+    if (rb::off16(a->O) || (a->o_sb | a->o_ss | a->o_sh) % 8) return -5;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     return a->dtype == 1 ? rb::launch_fwd<__nv_bfloat16>(*a, st) : rb::launch_fwd<__half>(*a, st);
 }

@@ -444,6 +444,7 @@ extern "C" int rb_im2col(const void* x, void* cols, int N, int H, int W, int C, 
     if (C % 8 || k < 1 || s < 1) return -2;
     const int Ho = (H + 2 * pad - k) / s + 1, Wo = (W + 2 * pad - k) / s + 1;
     if (Ho <= 0 || Wo <= 0) return -2;
+    if (off16(x, cols)) return -5;
     const long long total = static_cast<long long>(N) * Ho * Wo * k * k * (C / 8);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (dtype == 1)
@@ -461,6 +462,7 @@ extern "C" int rb_col2im(const void* dcols, void* dx, int N, int H, int W, int C
     if (C % 8 || k < 1 || s < 1) return -2;
     const int Ho = (H + 2 * pad - k) / s + 1, Wo = (W + 2 * pad - k) / s + 1;
     if (Ho <= 0 || Wo <= 0) return -2;
+    if (off16(dcols, dx)) return -5;
     const long long total = static_cast<long long>(N) * H * W * (C / 8);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (dtype == 1)
@@ -521,6 +523,7 @@ extern "C" int rb_bn_fwd(const void* x, const void* res, const float* gamma, con
                          float momentum, int relu, int dtype, void* stream) {
     using namespace rb;
     if (C % 8 || R <= 0) return -2;
+    if (off16(x, res, y, part)) return -5;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     return RB_BN_DISPATCH(bn_fwd_launch, x, res, gamma, beta, y, part, mean, rstd, run_mean, run_var, R, C, eps, momentum,
                           relu, st);
@@ -533,6 +536,7 @@ extern "C" int rb_bn_bwd(const void* x, const void* dy, const void* y, const flo
                          long long R, int C, int relu, int dtype, void* stream) {
     using namespace rb;
     if (C % 8 || R <= 0) return -2;
+    if (off16(x, dy, y, dx, dres) || off16(mean, rstd, part)) return -5;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     return RB_BN_DISPATCH(bn_bwd_launch, x, dy, y, mean, rstd, gamma, part, dgamma_acc, dbeta_acc, dx, dres, R, C, relu, st);
 }

@@ -321,6 +321,7 @@ extern "C" int rb_gelu(const void* x, const void* dy, void* y, long long n, int 
                        void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (n <= 0) return 0;
+    if (off16(x, dy, y)) return -5;
     const int g = grid_for(n / 8 + 1, 256);
     if (dtype == 1)
         gelu_kernel<__nv_bfloat16><<<g, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x),
@@ -337,6 +338,7 @@ extern "C" int rb_dropout(const void* x, void* y, long long n, float p, uint64_t
                           uint64_t offset, int dtype, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (n <= 0) return 0;
+    if (off16(x, y)) return -5;
     const uint32_t thr = drop_threshold(p);
     const float scale = 1.f / (1.f - p);
     const int g = grid_for(n / 8 + 1, 256);
@@ -412,13 +414,9 @@ extern "C" int rb_unstack3(const void* w, int w_fp32, const float* b, void* cons
                            long long bn, int dtype, void* stream) {
     if (wn % 8 || (b && bn % 8)) return -2;
     Unstack3 u = {w, b, {wd[0], wd[1], wd[2]}, {nullptr, nullptr, nullptr}, wn, bn};
-    uintptr_t bits = reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(b);
-    for (int i = 0; i < 3; ++i) {
-        if (b) u.bd[i] = bd[i];
-        bits |= reinterpret_cast<uintptr_t>(u.wd[i]) | reinterpret_cast<uintptr_t>(u.bd[i]);
-    }
-    if (bits & 15) return -2;
+    for (int i = 0; i < 3 && b; ++i) u.bd[i] = bd[i];
     if (wn <= 0) return 0;
+    if (off16(w, b) || off16(u.wd[0], u.wd[1], u.wd[2], u.bd[0], u.bd[1], u.bd[2])) return -5;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int g = grid_for(3 * (wn + (b ? bn : 0)) / 8, 256);
     if (dtype == 1)
@@ -434,6 +432,7 @@ extern "C" int rb_embed_fwd(const long long* ids, const void* table, void* out, 
     if (rows <= 0) return 0;
     RB_DEBUG_ARG(H % 8 == 0, "rb_embed_fwd: H must be a multiple of 8");
     if (H % 8) return -2;
+    if (off16(table, out)) return -5;
     RB_DEBUG_RANGE(ids, rows, 0, vocab, -1 - vocab, st);
     const int g = (rows * 32 + 255) / 256;
     if (dtype == 1)

@@ -1233,10 +1233,8 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     }
     if (a->map_hp > 0 && (a->batch != 1 || a->rs_nranks > 1 || a->map_wp <= 0)) return -7;
 
-    auto off16 = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) != 0; };
     p.bias_al = !off16(a->bias);
-    p.in_al = !off16(a->residual) && !off16(a->aux_in) && !off16(a->aux_out) && a->ldd % 8 == 0 &&
-              (a->batch == 1 || a->strideD % 8 == 0);
+    p.in_al = !off16(a->residual, a->aux_in, a->aux_out) && a->ldd % 8 == 0 && (a->batch == 1 || a->strideD % 8 == 0);
     const int64_t per16 = a->out_dtype == 1 ? 4 : 8;
     p.out_al = !off16(a->D) && a->ldd % per16 == 0 && (a->batch == 1 || a->strideD % per16 == 0);
     for (int r = 0; r < p.rs_nranks; ++r) p.out_al = p.out_al && !off16(a->rs_peer[r]);

@@ -411,6 +411,7 @@ extern "C" int rb_ln_fwd(const void* x, const void* residual, const void* gamma,
                          float p, uint64_t seed, uint64_t offset, int dtype, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (rows <= 0) return 0;
+    if (rb::off16(x, residual, gamma, beta, y, z)) return -5;
     if (dtype == 1) {
         RB_LN_DISPATCH(__nv_bfloat16, launch_fwd, x, residual, gamma, beta, y, z, mean, rstd, rows,
                        eps, p, seed, offset, st)
@@ -451,6 +452,7 @@ extern "C" int rb_ln_bwd(const void* dy, const void* z, const void* gamma, const
                          int accumulate, int dtype, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (rows <= 0) return rb::ln_bwd_empty(dgamma, dbeta, H * sizeof(float), accumulate, st);
+    if (rb::off16(dy, z, gamma, dz, dx)) return -5;
     const int grid = rb_ln_bwd_grid(rows);
     const int rc = rb::ln_bwd_rows(dy, z, gamma, mean, rstd, dz, dx, partial, grid, rows, H, p, seed, offset, dtype, st);
     return rc ? rc : rb::ln_bwd_sums<float>(partial, dgamma, dbeta, grid, H, accumulate, st);
@@ -462,6 +464,7 @@ extern "C" int rb_ln_bwd16(const void* dy, const void* z, const void* gamma, con
                            uint64_t seed, uint64_t offset, int dtype, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (rows <= 0) return rb::ln_bwd_empty(dgamma, dbeta, H * 2, 0, st);
+    if (rb::off16(dy, z, gamma, dz, dx)) return -5;
     const int grid = rb_ln_bwd_grid(rows);
     const int rc = rb::ln_bwd_rows(dy, z, gamma, mean, rstd, dz, dx, partial, grid, rows, H, p, seed, offset, dtype, st);
     if (rc) return rc;

@@ -12,6 +12,14 @@
 
 namespace rb {
 
+// Whether any of the addresses (null: absent) is off a 16-byte boundary.  Entries whose kernels move whole vectors ask
+// before they launch: on the device such an address is an error that takes the context with it.
+template <typename... P>
+inline bool off16(const P*... p) {
+    return ((reinterpret_cast<uintptr_t>(p) | ...) & 15) != 0;
+}
+
+
 // ---------------------------------------------------------------------------
 // error status word (one per library, device global); 0 = ok
 // ---------------------------------------------------------------------------

@@ -476,7 +476,7 @@ def test_other_threads_run_while_a_launch_waits():
         torch.cuda.synchronize()
     if waited < 0.4:
         pytest.skip("the launch queue took all launches")
-    assert gap[0] < 0.2, gap[0]
+    assert gap[0] < 0.6 * waited, (gap[0], waited)
 
 
 def test_two_threads_differentiate_one_graph():
@@ -570,3 +570,29 @@ def test_weight_gradient_folds_on_both_sides_of_the_rule(dtype, k, kernel, Co, C
         assert RF.K.wgrad_fold_ok(w) == kernel
         got = RF._Conv2d._fold(dw2, w, None, k)
         assert got.is_contiguous() and torch.equal(got, want.to(dtype))
+
+
+def test_kernel_entries_refuse_addresses_off_a_boundary():
+    """An error code from the host, nothing launched: on the device it would be a fault."""
+    from rannc_b200.ops import _lib
+
+    K = RF.K
+    x, v, f = _randn(8, 256), _randn(256), torch.zeros(8, device="cuda")
+    img, c32 = _randn(50, 64), torch.zeros(64, device="cuda")
+    q = _randn(1, 16, 2, 64)
+    o, lse = K.attn_fwd(q, q, q)
+    calls = [lambda: K.ln_fwd(_off(x), None, v, v, 1e-5), lambda: K.ln_fwd(x, _off(x), v, v, 1e-5),
+             lambda: K.ln_fwd(x, None, _off(v), v, 1e-5), lambda: K.ln_bwd(_off(x), x, v, f, f),
+             lambda: K.ln_bwd(x, x, _off(v), f, f), lambda: K.gelu(_off(x)), lambda: K.gelu_bwd(x, _off(x)),
+             lambda: K.dropout(_off(x), 0.5, 1, 1), lambda: K.embed_fwd(torch.zeros(3, dtype=torch.int64, device="cuda"), _off(x)),
+             lambda: K.im2col(_off(_randn(1, 5, 5, 8)), 3, 1, 1), lambda: K.col2im(_off(_randn(25, 72)), 1, 5, 5, 8, 3, 1, 1),
+             lambda: K.bn_fwd(_off(img), None, c32, c32, None, None, 1e-5, 0.1, False),
+             lambda: K.bn_bwd(img, img, img, _off(c32), c32, c32, False, False),
+             lambda: K.bn_bwd(img, _off(img), img, c32, c32, c32, False, False),
+             lambda: K.attn_bwd(q, q, q, _off(o), lse, q), lambda: K.attn_bwd(q, q, q, o, lse, q, dv=_off(q)),
+             lambda: K.attn_fwd(_off(q), q, q)]
+    for call in calls:
+        with pytest.raises(_lib.KernelLibraryError):
+            call()
+    torch.cuda.synchronize()
+    assert _lib.read_error() == 0
