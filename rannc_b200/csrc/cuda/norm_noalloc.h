@@ -41,7 +41,7 @@ extern "C" {
 
 enum {
     RB_LN_NOALLOC_OK = 0,
-    RB_LN_NOALLOC_LAUNCH_FAILED = -1,
+    RB_LN_NOALLOC_LAUNCH_FAILED = -1,   // also: a matrix or gamma off a 16-byte boundary
     RB_LN_NOALLOC_BAD_WIDTH = -2,   // H is not one of 256, 512, 768, 1024, 1536, 2048, 3072, 4096
     RB_LN_NOALLOC_NO_SYMBOL = -6,   // cudaGetSymbolAddress failed on this device
     RB_LN_NOALLOC_TOO_LARGE = -7,   // rows x H needs more scratch than the library holds
