@@ -4,18 +4,24 @@
 // query block i it recomputes, with the keys on the TMEM lanes,
 //     St  = K_j Q_i^T          dPt = V_j dO_i^T                (TMEM, 2 x 128 cols)
 //     Pt  = exp(St*scale + bias - lse_i)      dSt = Pt * (dPt - delta_i)
-// writes Pt / dSt as 16-bit tiles into swizzled shared memory (one thread per
-// key row) and feeds them back to the tensor core:
-//     dV_j += Pt  dO_i        dK_j += dSt Q_i                  (TMEM accumulators)
+// rounds both to 16 bits (four threads per key row) and feeds them back to the tensor core:
+//     dK_j += dSt Q_i         dV_j += Pt  dO_i                 (TMEM accumulators)
 //     dQ_i  = dSt^T K_j  -- the same dSt tile read as an MN-major A operand --
-// dQ_i is drained from TMEM into a swizzled fp32 staging tile and added to an
-// fp32 scratch buffer by ONE bulk tensor reduction per half tile (the copy
+// dSt goes through swizzled shared memory (dQ wants it transposed); Pt returns to tensor memory, from where the
+// tensor core takes it as its A operand: 64 KiB a step less on shared memory, which products, tiles and staging
+// kept busy for two thirds of the time.  dQ_i is drained from TMEM into a swizzled fp32 staging tile and added to
+// an fp32 scratch buffer by ONE bulk tensor reduction per half tile (the copy
 // engine does the read-modify-write; the math threads do not wait for it); a
 // last kernel converts the scratch to the 16-bit dQ.  Q_i / dO_i stream
-// through a 2-stage TMA ring; lse / delta of the next query block are fetched
-// while the current one is processed.  Warps 0..7 = element math, warp 8 = TMA + MMA issue, warps
-// 9..12 = dQ drain: the math warps' chain per query block is then only "S / dP -> P / dS", and the
-// drain of block i runs beside the math of block i + 1.
+// through a 3-stage TMA ring.  Warps 0..15 = element math, warp 16 = TMA + MMA issue, warps
+// 17..20 = dQ drain, and the row statistics (lse, delta, dropout hash) of the blocks to come: the math warps' chain
+// per query block is only "S / dP -> P / dS", without a barrier among them, and the drain of block i runs
+// beside the math of block i + 1.  Of a block's products those that read dSt come first, so that its tile is free
+// again before the next block's is ready.
+//
+// 32 x 512 x 16 heads with bias and dropout, with the delta and conversion passes: 278 -> 227 us; 2 x 2048 without:
+// 197 -> 136 us.  What bounded it was neither element math (without dropout it took as long) nor the tensor core but
+// one thread's issuing of 32 products a step.
 //
 // Takes the place of the autograd graph the reference runs for the traced
 // attention chain (src/torch/TorchDriver.cpp:642-847).
@@ -28,15 +34,17 @@ namespace rb {
 constexpr int BQ = 128, BKEYS = 128;
 constexpr int TILE = 128 * 64 * 2;       // 16 KiB
 constexpr int SQ_BYTES = 128 * 128 * 2;  // 32 KiB
-constexpr int BWD_MATH = 256;
-constexpr int BWD_DRAIN = 128;                 // warps 9..12: move dQ out of tensor memory
-constexpr int BWD_THREADS = BWD_MATH + 32 + BWD_DRAIN;
+constexpr int BWD_MATH = 512;                  // warps 0..15: four threads per key row
+constexpr int BWD_DRAIN = 128;                 // warps 17..20: move dQ out of tensor memory
+constexpr int LOAD_WARP = BWD_MATH / 32, GRAD_WARP = LOAD_WARP + 1;
+constexpr int BWD_THREADS = BWD_MATH + 64 + BWD_DRAIN;
 constexpr int BWD_TMEM_COLS = 512;
-constexpr int C_ST = 0, C_DPT = 128, C_DV = 256, C_DK = 320, C_DQ = 384;
+constexpr int C_ST = 0, C_DPT = 128, C_DV = 256, C_DK = 320, C_DQ = 384, C_P = 448;   // P: 128 16-bit columns
 constexpr int DQ_STAGE = 128 * 64 * 4;   // 32 KiB: [2 column halves][128 rows x 128 B]
 constexpr int QD_STAGES = 3;             // Q / dO ring: block i + 2 is loaded while blocks i and i + 1 are in use
-// K, V + (Q, dO) x 3 stages + Pt, dSt + dQ staging + per-step (lse, delta, row hash) + barriers
-constexpr int BWD_SMEM = 2 * TILE + 2 * QD_STAGES * TILE + 2 * SQ_BYTES + DQ_STAGE + 3 * 128 * 4 + 128;
+constexpr int STATS = 3 * 128;           // (lse, delta, row hash) of a query block
+// K, V + (Q, dO) x 3 stages + dSt + dQ staging + row statistics of two blocks + barriers
+constexpr int BWD_SMEM = 2 * TILE + 2 * QD_STAGES * TILE + SQ_BYTES + DQ_STAGE + 2 * STATS * 4 + 128;
 
 struct AttnBwdParams {
     int B, H, S;
@@ -64,26 +72,26 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
     uint8_t* sV = smem + TILE;
     uint8_t* sQ = smem + 2 * TILE;                     // [QD_STAGES]
     uint8_t* sdO = smem + (2 + QD_STAGES) * TILE;      // [QD_STAGES]
-    uint8_t* sPt = smem + (2 + 2 * QD_STAGES) * TILE;
-    uint8_t* sdSt = sPt + SQ_BYTES;
+    uint8_t* sdSt = smem + (2 + 2 * QD_STAGES) * TILE;
     uint8_t* sDQ = sdSt + SQ_BYTES;
-    float* s_lse = reinterpret_cast<float*>(sDQ + DQ_STAGE);        // [128], rewritten every step
-    float* s_delta = s_lse + 128;                                   // [128]
-    uint32_t* s_rhash = reinterpret_cast<uint32_t*>(s_delta + 128);  // [128]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(s_rhash + 128);
+    float* s_stats = reinterpret_cast<float*>(sDQ + DQ_STAGE);   // [2][-lse, -delta, row hash][128]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(s_stats + 2 * STATS);
     uint64_t* kv_full = bars;
-    uint64_t* qd_full = bars + 1;  // [QD_STAGES]
+    uint64_t* qd_full = bars + 1;     // [QD_STAGES]
     uint64_t* s_full = bars + 4;
     uint64_t* s_free = bars + 5;
     uint64_t* pds_ready = bars + 6;
-    uint64_t* mma_done = bars + 7;
-    uint64_t* dq_free = bars + 8;    // the previous bulk reduction has read the staging tile
-    uint64_t* dq_ready = bars + 9;   // every drain thread has written its part of the staging tile
-    uint64_t* dq_taken = bars + 10;  // dQ of the last step is out of tensor memory: the next may overwrite it
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+    uint64_t* ds_done = bars + 7;     // dK and dQ of the step are done: dSt may be overwritten, dQ drained
+    uint64_t* p_done = bars + 8;      // ... and dV: Pt, Q and dO may be
+    uint64_t* dq_free = bars + 9;     // the previous bulk reduction has read the staging tile
+    uint64_t* dq_ready = bars + 10;   // every drain thread has written its part of the staging tile
+    uint64_t* dq_taken = bars + 11;   // dQ of the last step is out of tensor memory: the next may overwrite it
+    uint64_t* stats_full = bars + 12;   // [2]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (the same for all lanes, for the compiler too: what the issuing warps compute from it stays in uniform registers)
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int key0 = blockIdx.x * BKEYS, h = blockIdx.y, b = blockIdx.z;
     const int nq = (p.S + BQ - 1) / BQ;
 
@@ -93,14 +101,16 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
         mbar_init(s_full, 1);
         mbar_init(s_free, BWD_MATH);
         mbar_init(pds_ready, BWD_MATH);
-        mbar_init(mma_done, 1);
+        mbar_init(ds_done, 1);
+        mbar_init(p_done, 1);
         mbar_init(dq_free, 1);
         mbar_init(dq_ready, BWD_DRAIN);
         mbar_init(dq_taken, BWD_DRAIN);
+        for (int u = 0; u < 2; ++u) mbar_init(&stats_full[u], BWD_DRAIN);
         *abort_flag = 0;
         fence_mbar_init();
     }
-    if (warp == 8) {
+    if (warp == LOAD_WARP) {
         tmem_alloc(tmem_slot, BWD_TMEM_COLS);
         tmem_relinquish();
     }
@@ -110,91 +120,127 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
     const uint32_t tmem = *tmem_slot;
     constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
 
-    if (warp == 8) {
-        if (lane == 0) {
-            const uint32_t id_s = make_idesc_f16(fmt, 0, 0, 128, 128);
-            const uint32_t id_kn = make_idesc_f16(fmt, 0, 1, 128, 64);  // A K-major, B MN-major
-            const uint32_t id_nn = make_idesc_f16(fmt, 1, 1, 128, 64);  // A MN-major, B MN-major
-            auto load_qd = [&](int i) {
-                const int st = i % QD_STAGES;
+    if (warp == LOAD_WARP) {
+        // ------------- loads, and the S / dP products -------------
+        // The whole warp goes through the loop and one lane's predicate lets the instructions through: a branch for that
+        // lane would keep descriptors out of the uniform registers, and eight products then take 600 cycles to issue, not
+        // 350 -- more with the math warps beside it.
+        const uint32_t el = elect_one();
+        const uint32_t id_s = make_idesc_f16(fmt, 0, 0, 128, 128);
+        const uint32_t k_desc = desc_lo_sw128(smem_u32(sK), 16), v_desc = desc_lo_sw128(smem_u32(sV), 16);
+        const uint32_t q_desc = desc_lo_sw128(smem_u32(sQ), 16), do_desc = desc_lo_sw128(smem_u32(sdO), 16);
+        auto load_qd = [&](int i, int st) {
+            if (el) {
                 mbar_arrive_expect_tx(&qd_full[st], 2 * TILE);
                 tma_load_4d(sQ + st * TILE, &tmQ, &qd_full[st], 0, i * BQ, h, b);
                 tma_load_4d(sdO + st * TILE, &tmdO, &qd_full[st], 0, i * BQ, h, b);
-            };
-            auto issue_s = [&](int i) {
-                const uint32_t ka = smem_u32(sK), va = smem_u32(sV);
-                const uint32_t qa = smem_u32(sQ + (i % QD_STAGES) * TILE), da = smem_u32(sdO + (i % QD_STAGES) * TILE);
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    umma_f16(tmem + C_ST, make_smem_desc_sw128(ka + k * 32, 16, 1024),
-                             make_smem_desc_sw128(qa + k * 32, 16, 1024), id_s, k != 0);
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    umma_f16(tmem + C_DPT, make_smem_desc_sw128(va + k * 32, 16, 1024),
-                             make_smem_desc_sw128(da + k * 32, 16, 1024), id_s, k != 0);
-                umma_commit(s_full);
-            };
+            }
+        };
+        if (el) {
             mbar_arrive_expect_tx(kv_full, 2 * TILE);
             tma_load_4d(sK, &tmK, kv_full, 0, key0, h, b);
             tma_load_4d(sV, &tmV, kv_full, 0, key0, h, b);
-            for (int i = 0; i < QD_STAGES && i < nq; ++i) load_qd(i);
-            bool ok = mbar_wait(kv_full, 0, abort_flag) && mbar_wait(&qd_full[0], 0, abort_flag);
-            if (ok) {
-                tc_fence_after();
-                issue_s(0);
+        }
+        for (int i = 0; i < QD_STAGES && i < nq; ++i) load_qd(i, i);
+        bool ok = mbar_wait_warp(kv_full, 0, abort_flag);
+        int st = 0, next = 2;   // stage of block i, and of block i + 2
+        uint32_t phase = 0;
+        for (int i = 0; i < nq && ok; ++i) {
+            // S / dP of a block go to the tensor core as soon as the math warps have read the last block's: they run
+            // behind that block's products, while its math is busy
+            ok = mbar_wait_warp(&qd_full[st], phase, abort_flag) && (i == 0 || mbar_wait_warp(s_free, (i - 1) & 1, abort_flag));
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t qa = q_desc + st * (TILE / 16), da = do_desc + st * (TILE / 16);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                umma_f16_lo(tmem + C_ST, k_desc + k * 2, qa + k * 2, id_s, k != 0, el);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                umma_f16_lo(tmem + C_DPT, v_desc + k * 2, da + k * 2, id_s, k != 0, el);
+            if (el) umma_commit(s_full);
+            // the stage block i - 1 used is free once its products are done: block i + 2 goes there
+            if (i >= 1 && i + 2 < nq) {
+                if (!mbar_wait_warp(p_done, (i - 1) & 1, abort_flag)) break;
+                load_qd(i + 2, next);
             }
-            for (int i = 0; i < nq && ok; ++i) {
-                // S / dP of the next block go to the tensor core as soon as the math warps have read this
-                // block's: they run behind the previous block's products, while this block's math is busy
-                if (i + 1 < nq) {
-                    ok = mbar_wait(&qd_full[(i + 1) % QD_STAGES], ((i + 1) / QD_STAGES) & 1, abort_flag) &&
-                         mbar_wait(s_free, i & 1, abort_flag);
-                    if (!ok) break;
-                    tc_fence_after();
-                    issue_s(i + 1);
-                }
-                // the stage block i - 1 used is free once its products are done: fetch block i + 2 into it,
-                // a whole step before its S / dP products are issued
-                if (i >= 1 && i + 2 < nq) {
-                    if (!mbar_wait(mma_done, (i - 1) & 1, abort_flag)) break;
-                    load_qd(i + 2);
-                }
-                if (!mbar_wait(pds_ready, i & 1, abort_flag)) break;
-                tc_fence_after();
-                const uint32_t pa = smem_u32(sPt), sa = smem_u32(sdSt), ka = smem_u32(sK);
-                const uint32_t qa = smem_u32(sQ + (i % QD_STAGES) * TILE), da = smem_u32(sdO + (i % QD_STAGES) * TILE);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const uint32_t koff = (k >> 2) * (SQ_BYTES / 2) + (k & 3) * 32;
-                    umma_f16(tmem + C_DV, make_smem_desc_sw128(pa + koff, 16, 1024),
-                             make_smem_desc_sw128(da + k * 2048, 8192, 1024), id_kn, (i | k) != 0);
-                }
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const uint32_t koff = (k >> 2) * (SQ_BYTES / 2) + (k & 3) * 32;
-                    umma_f16(tmem + C_DK, make_smem_desc_sw128(sa + koff, 16, 1024),
-                             make_smem_desc_sw128(qa + k * 2048, 8192, 1024), id_kn, (i | k) != 0);
-                }
-                // dQ of the previous step must have left tensor memory before this step's product replaces it
-                if (i > 0) {
-                    if (!mbar_wait(dq_taken, (i - 1) & 1, abort_flag)) break;
-                    tc_fence_after();
-                }
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    umma_f16(tmem + C_DQ, make_smem_desc_sw128(sa + k * 2048, SQ_BYTES / 2, 1024),
-                             make_smem_desc_sw128(ka + k * 2048, 8192, 1024), id_nn, k != 0);
-                umma_commit(mma_done);
+            if (++next == QD_STAGES) next = 0;
+            if (++st == QD_STAGES) {
+                st = 0;
+                phase ^= 1;
             }
         }
-    } else if (warp > 8) {
+    } else if (warp == GRAD_WARP) {
+        // ------------- the products with dSt and Pt.  A warp of its own: one that issued all products took 4400 cycles
+        // a step, between the math warps that share its scheduler, and S / dP queued behind them -------------
+        const uint32_t el = elect_one();
+        const uint32_t id_kn = make_idesc_f16(fmt, 0, 1, 128, 64);  // A K-major, B MN-major
+        const uint32_t id_nn = make_idesc_f16(fmt, 1, 1, 128, 64);  // A MN-major, B MN-major
+        const uint32_t ds_k = desc_lo_sw128(smem_u32(sdSt), 16), ds_n = desc_lo_sw128(smem_u32(sdSt), SQ_BYTES / 2);
+        const uint32_t k_desc = desc_lo_sw128(smem_u32(sK), 8192);
+        const uint32_t q_desc = desc_lo_sw128(smem_u32(sQ), 8192), do_desc = desc_lo_sw128(smem_u32(sdO), 8192);
+        int st = 0;
+        uint32_t phase = 0;
+        for (int i = 0; i < nq; ++i) {
+            if (!mbar_wait_warp(&qd_full[st], phase, abort_flag) || !mbar_wait_warp(pds_ready, i & 1, abort_flag)) break;
+            tc_fence_after();
+            const uint32_t qa = q_desc + st * (TILE / 16), da = do_desc + st * (TILE / 16);
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                umma_f16_lo(tmem + C_DK, ds_k + (k >> 2) * (SQ_BYTES / 32) + (k & 3) * 2, qa + k * 128, id_kn, (i | k) != 0, el);
+            // dQ of the previous step must have left tensor memory before this step's product replaces it
+            if (i > 0) {
+                if (!mbar_wait_warp(dq_taken, (i - 1) & 1, abort_flag)) break;
+                tc_fence_after();
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                umma_f16_lo(tmem + C_DQ, ds_n + k * 128, k_desc + k * 128, id_nn, k != 0, el);
+            if (el) umma_commit(ds_done);
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                umma_f16_ts_lo(tmem + C_DV, tmem + C_P + k * 8, da + k * 128, id_kn, (i | k) != 0, el);
+            if (el) umma_commit(p_done);
+            if (++st == QD_STAGES) {
+                st = 0;
+                phase ^= 1;
+            }
+        }
+    } else if (warp > GRAD_WARP) {
         // ------------- dQ drain: thread r owns query row r of the block (TMEM lane r), all 64 columns -------------
         const int r = (warp & 3) * 32 + lane;
         const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const uint32_t sw = r & 7;
-        const bool issuer = threadIdx.x == BWD_MATH + 32;
+        const bool issuer = threadIdx.x == BWD_MATH + 64;
+        // row statistics: thread t looks after row t of every query block, two buffers.  Both sums are negated (the
+        // element-wise chain adds them); past the end of the sequence lse is +inf, and probabilities come out as
+        // exp2(-inf) = 0.
+        const int t = threadIdx.x - (BWD_MATH + 64);
+        const long long bh_row = (static_cast<long long>(b) * p.H + h) * p.S;
+        float lse = 0.f, delta = 0.f;
+        auto fetch_stats = [&](int i) {   // (volatile: the loads are not sunk to their use)
+            const int q = i * BQ + t;
+            lse = INFINITY;
+            delta = 0.f;
+            if (q < p.S) {
+                asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(lse) : "l"(p.lse + bh_row + q));
+                asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(delta) : "l"(p.delta + bh_row + q));
+            }
+        };
+        auto put_stats = [&](int i) {
+            float* s = s_stats + (i & 1) * STATS;
+            s[t] = lse * -1.4426950408889634f;
+            s[128 + t] = -delta;
+            reinterpret_cast<uint32_t*>(s)[256 + t] = drop_row_hash(p.seed, b, h, i * BQ + t, p.H, p.S);
+            mbar_arrive(&stats_full[i & 1]);
+        };
+        for (int i = 0; i < 2 && i < nq; ++i) {
+            fetch_stats(i);
+            put_stats(i);
+        }
         for (int i = 0; i < nq; ++i) {
-            if (!mbar_wait(mma_done, i & 1, abort_flag)) break;
+            if (i + 2 < nq) fetch_stats(i + 2);
+            if (!mbar_wait(ds_done, i & 1, abort_flag)) break;
             tc_fence_after();
             uint32_t v0[32], v1[32];
             tmem_ld32(tmem + lane_addr + C_DQ, v0);
@@ -202,6 +248,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
             tmem_ld_wait();
             tc_fence_before();
             mbar_arrive(dq_taken);
+            // dSt of this step has been read, so it had been written: the math threads are past this step's statistics
+            if (i + 2 < nq) put_stats(i + 2);
             if (issuer) {
                 tma_store_wait_read<0>();   // the previous reduction no longer reads the staging tile
                 mbar_arrive(dq_free);
@@ -227,12 +275,13 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
                 tma_store_commit();
             }
         }
-        if (issuer) tma_store_wait<0>();   // the last reduction has landed
+        // the staging tile must outlive the copies that read it; their sums are complete when the kernel is
+        if (issuer) tma_store_wait_read<0>();
     } else {
-        // thread pair (r, r + 128): TMEM lane r = key row for St/dPt/dV/dK;
-        // `half` selects 64 of the 128 query columns of St/dPt and 32 of the 64 columns of dQ/dK/dV
+        // threads r, r + 128, r + 256, r + 384: TMEM lane r = key row for St/dPt/dV/dK;
+        // `part` selects 32 of the 128 query columns of St/dPt, and half the columns of dV or of dK
         const int r = threadIdx.x & 127;
-        const int half = threadIdx.x >> 7;
+        const int part = threadIdx.x >> 7;
         const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const int key = key0 + r;
         const bool key_ok = key < p.S;
@@ -243,60 +292,30 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
         const uint32_t key_hash = drop_key_hash(p.seed, key);
         const uint64_t kbias2 = f2_pack(kbias, kbias), scale2 = f2_pack(p.scale_log2, p.scale_log2),
                        keep2 = f2_pack(p.inv_keep, p.inv_keep);
-        const long long bh = static_cast<long long>(b) * p.H + h;
         const uint32_t sw = r & 7;
-        const uint32_t row_off = half * (SQ_BYTES / 2) + (r >> 3) * 1024 + sw * 128;
-        uint8_t* prow = sPt + row_off;
-        uint8_t* drow = sdSt + row_off;
+        uint8_t* drow = sdSt + (part >> 1) * (SQ_BYTES / 2) + (r >> 3) * 1024 + sw * 128;
         bool ok = true;
 
-        // lse / delta of the first query block; later blocks are fetched one step ahead
-        float n_lse = 0.f, n_delta = 0.f;
-        bool n_lse_raw = false;   // n_lse still in natural-log units (as loaded)
-        if (half == 0) {
-            n_lse = r < p.S ? p.lse[bh * p.S + r] * 1.4426950408889634f : INFINITY;
-            n_delta = r < p.S ? p.delta[bh * p.S + r] : 0.f;
-        }
         for (int i = 0; i < nq; ++i) {
-            const int q0 = i * BQ;
-            // every thread is done reading the previous step's row statistics before they are replaced
-            bar_sync_named(1, BWD_MATH);
-            if (half == 0) {
-                // +inf for rows past the end of the sequence: their probabilities come out as exp2(-inf) = 0
-                // both negated: the element-wise chain adds them
-                s_lse[r] = n_lse_raw ? n_lse * -1.4426950408889634f : -n_lse;
-                s_delta[r] = -n_delta;
-                s_rhash[r] = drop_row_hash(p.seed, b, h, q0 + r, p.H, p.S);
-                // issued here (volatile: not sunk to the use), consumed at the top of the next step
-                const int qn = q0 + BQ + r;
-                if (i + 1 < nq && qn < p.S) {
-                    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(n_lse) : "l"(p.lse + bh * p.S + qn));
-                    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(n_delta) : "l"(p.delta + bh * p.S + qn));
-                    n_lse_raw = true;
-                } else {
-                    n_lse = INFINITY;
-                    n_delta = 0.f;
-                    n_lse_raw = false;
-                }
-            }
-            bar_sync_named(1, BWD_MATH);
-            // after a failed wait the loop keeps running (every later wait fails at once) so that all threads
-            // still meet at the named barriers
-            if (!mbar_wait(s_full, i & 1, abort_flag)) {
+            if (!mbar_wait(&stats_full[i & 1], (i >> 1) & 1, abort_flag) || !mbar_wait(s_full, i & 1, abort_flag)) {
                 ok = false;
-                continue;
+                break;
             }
             tc_fence_after();
-            // Pt / dSt of this thread's 64 columns, packed to 16 bits, held in registers: the whole
+            const float* st_lse = s_stats + (i & 1) * STATS + part * 32;
+            const float* st_delta = st_lse + 128;
+            const uint32_t* st_hash = reinterpret_cast<const uint32_t*>(st_lse + 256);
+            // Pt / dSt of this thread's 32 columns, packed to 16 bits, held in registers: the whole
             // computation overlaps the tensor-core work of the previous step, whose operands still
-            // occupy the shared-memory tiles.  Pt carries the dropout mask without its 1 / (1 - p)
+            // occupy their places.  Pt carries the dropout mask without its 1 / (1 - p)
             // factor (dV is scaled once at the end); dSt = P (mask dP / (1 - p) - delta).
-            uint4 pk[2][4], dk4[2][4];
+            uint32_t pk[16], dk[16];
+            const uint32_t t_s = tmem + lane_addr + C_ST + part * 32, t_dp = tmem + lane_addr + C_DPT + part * 32;
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                uint32_t sv[32], dv[32];
-                tmem_ld32(tmem + lane_addr + C_ST + half * 64 + c * 32, sv);
-                tmem_ld32(tmem + lane_addr + C_DPT + half * 64 + c * 32, dv);
+                uint32_t s_[16], d_[16];
+                tmem_ld16(t_s + c * 16, s_);
+                tmem_ld16(t_dp + c * 16, d_);
                 tmem_ld_wait();
                 if (c == 1) {
                     // both TMEM tiles are in registers: the next step's MMAs may overwrite them
@@ -305,95 +324,94 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
                 }
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {
-                    // The longest link of the chain that bounds this kernel: a CTA holds all of tensor memory, so per SM the
-                    // MMAs of a query block wait for the P / dS of the one before and these threads for its S / dP (issue
-                    // slots 30 % busy, tensor pipe 19 %).  Some ten instructions per element; what has a two-wide form uses
-                    // it -- P = 2^((S scale + bias) - lse), dS = P (mask dP / (1 - p) - delta): 32 x 512 x 16 heads with bias
-                    // and dropout 240 -> 226 us.  The bias goes to the score first, as in the forward: where every key of a
+                    // A CTA holds all of tensor memory, so per SM the MMAs of a query block wait for the P / dS of the one
+                    // before and these threads for its S / dP.  Sixteen warps, four to a scheduler, hide each other's
+                    // latency: with eight, of 64 columns a thread, the passes above took 246 and 175 us.  Some ten instructions per element; what has a two-wide form uses
+                    // it -- P = 2^((S scale + bias) - lse), dS = P (mask dP / (1 - p) - delta).  The bias goes to the score first, as in the forward: where every key of a
                     // row carries a huge negative bias the score is rounded away in both, and P stays at most 1; bias - lse
                     // first would leave 2^(S scale).
-                    float pd[8], ds[8];
-#pragma unroll
-                    for (int hq = 0; hq < 2; ++hq) {
-                        const int qb = half * 64 + c * 32 + g * 8 + hq * 4;
-                        const ulonglong2 ls4 = *reinterpret_cast<const ulonglong2*>(s_lse + qb);
-                        const ulonglong2 dl4 = *reinterpret_cast<const ulonglong2*>(s_delta + qb);
-                        uint32_t rhv[4] = {0, 0, 0, 0};
-                        if (p.thr32) {
-                            const uint4 rh4 = *reinterpret_cast<const uint4*>(s_rhash + qb);
-                            rhv[0] = rh4.x, rhv[1] = rh4.y, rhv[2] = rh4.z, rhv[3] = rh4.w;
-                        }
-#pragma unroll
-                        for (int x = 0; x < 4; x += 2) {
-                            const int e = g * 8 + hq * 4 + x;
-                            const uint64_t nlse = x == 0 ? ls4.x : ls4.y, ndelta = x == 0 ? dl4.x : dl4.y;
-                            float e0, e1;
-                            f2_unpack(f2_add(f2_fma(f2_pack_bits(sv[e], sv[e + 1]), scale2, kbias2), nlse), e0, e1);
-                            const float p0 = ex2_approx(e0), p1 = ex2_approx(e1);
-                            uint64_t t;
-                            if (p.thr32) {
-                                const bool k0 = drop_keep(rhv[x], key_hash, p.thr32), k1 = drop_keep(rhv[x + 1], key_hash, p.thr32);
-                                pd[hq * 4 + x] = k0 ? p0 : 0.f;
-                                pd[hq * 4 + x + 1] = k1 ? p1 : 0.f;
-                                t = f2_fma(f2_pack_bits(k0 ? dv[e] : 0u, k1 ? dv[e + 1] : 0u), keep2, ndelta);
-                            } else {
-                                pd[hq * 4 + x] = p0;
-                                pd[hq * 4 + x + 1] = p1;
-                                t = f2_add(f2_pack_bits(dv[e], dv[e + 1]), ndelta);
-                            }
-                            f2_unpack(f2_mul(f2_pack(p0, p1), t), ds[hq * 4 + x], ds[hq * 4 + x + 1]);
-                        }
+                    const int qb = c * 16 + g * 4;
+                    const ulonglong2 ls4 = *reinterpret_cast<const ulonglong2*>(st_lse + qb);
+                    const ulonglong2 dl4 = *reinterpret_cast<const ulonglong2*>(st_delta + qb);
+                    uint32_t rhv[4] = {0, 0, 0, 0};
+                    if (p.thr32) {
+                        const uint4 rh4 = *reinterpret_cast<const uint4*>(st_hash + qb);
+                        rhv[0] = rh4.x, rhv[1] = rh4.y, rhv[2] = rh4.z, rhv[3] = rh4.w;
                     }
-                    pk[c][g] = make_uint4(pack2<T>(pd[0], pd[1]), pack2<T>(pd[2], pd[3]), pack2<T>(pd[4], pd[5]),
-                                          pack2<T>(pd[6], pd[7]));
-                    dk4[c][g] = make_uint4(pack2<T>(ds[0], ds[1]), pack2<T>(ds[2], ds[3]), pack2<T>(ds[4], ds[5]),
-                                           pack2<T>(ds[6], ds[7]));
+#pragma unroll
+                    for (int x = 0; x < 4; x += 2) {
+                        const int e = g * 4 + x;
+                        const uint64_t nlse = x == 0 ? ls4.x : ls4.y, ndelta = x == 0 ? dl4.x : dl4.y;
+                        float e0, e1;
+                        f2_unpack(f2_add(f2_fma(f2_pack_bits(s_[e], s_[e + 1]), scale2, kbias2), nlse), e0, e1);
+                        const float p0 = ex2_approx(e0), p1 = ex2_approx(e1);
+                        uint64_t t;
+                        float d0, d1;
+                        if (p.thr32) {
+                            const bool k0 = drop_keep(rhv[x], key_hash, p.thr32), k1 = drop_keep(rhv[x + 1], key_hash, p.thr32);
+                            pk[(qb + x) / 2] = pack2<T>(k0 ? p0 : 0.f, k1 ? p1 : 0.f);
+                            t = f2_fma(f2_pack_bits(k0 ? d_[e] : 0u, k1 ? d_[e + 1] : 0u), keep2, ndelta);
+                        } else {
+                            pk[(qb + x) / 2] = pack2<T>(p0, p1);
+                            t = f2_add(f2_pack_bits(d_[e], d_[e + 1]), ndelta);
+                        }
+                        f2_unpack(f2_mul(f2_pack(p0, p1), t), d0, d1);
+                        dk[(qb + x) / 2] = pack2<T>(d0, d1);
+                    }
                 }
             }
-            if (i > 0) {
-                // the previous step's dV / dK / dQ products read Pt / dSt: wait, then overwrite
-                if (!mbar_wait(mma_done, (i - 1) & 1, abort_flag)) {
-                    ok = false;
-                    continue;
-                }
-                tc_fence_after();
+            // the previous step's products read dSt and Pt: wait, then overwrite
+            if (i > 0 && !mbar_wait(ds_done, (i - 1) & 1, abort_flag)) {
+                ok = false;
+                break;
             }
 #pragma unroll
-            for (int c = 0; c < 2; ++c)
-#pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    const uint32_t off = (static_cast<uint32_t>(c * 4 + g) ^ sw) << 4;
-                    *reinterpret_cast<uint4*>(prow + off) = pk[c][g];
-                    *reinterpret_cast<uint4*>(drow + off) = dk4[c][g];
-                }
-            tc_fence_before();
+            for (int g = 0; g < 4; ++g)
+                *reinterpret_cast<uint4*>(drow + ((static_cast<uint32_t>((part & 1) * 4 + g) ^ sw) << 4)) =
+                    make_uint4(dk[g * 4], dk[g * 4 + 1], dk[g * 4 + 2], dk[g * 4 + 3]);
             fence_proxy_async();
+            if (i > 0 && !mbar_wait(p_done, (i - 1) & 1, abort_flag)) {
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            tmem_st16(tmem + lane_addr + C_P + part * 16, pk);
+            tmem_st_wait();
+            tc_fence_before();
             mbar_arrive(pds_ready);
         }
-        if (ok && mbar_wait(mma_done, (nq - 1) & 1, abort_flag)) {
+        // dK and dV: rows leave by way of the Q ring, which every product is done with, in pieces of 64 bytes that four
+        // lanes write together (a thread that stored its own row touched a line with every 16 bytes: 2800 cycles of a
+        // CTA's 24500 at S = 512)
+        if (ok && mbar_wait(p_done, (nq - 1) & 1, abort_flag)) {
             tc_fence_after();
-            T* dk = reinterpret_cast<T*>(p.dK) + b * p.dk_sb + static_cast<long long>(key) * p.dk_ss + h * p.dk_sh +
-                    half * 32;
-            T* dvp = reinterpret_cast<T*>(p.dV) + b * p.dv_sb + static_cast<long long>(key) * p.dv_ss + h * p.dv_sh +
-                     half * 32;
-            uint32_t a[32], d[32];
-            tmem_ld32(tmem + lane_addr + C_DV + half * 32, a);
-            tmem_ld32(tmem + lane_addr + C_DK + half * 32, d);
+            const int half = part & 1;
+            const bool is_k = part >> 1;
+            uint32_t a[32];
+            tmem_ld32(tmem + lane_addr + (is_k ? C_DK : C_DV) + half * 32, a);
             tmem_ld_wait();
-            if (key_ok) {
+            const float f = is_k ? p.scale : p.inv_keep;
+            uint8_t* stage = sQ + warp * 2048;   // [32 rows x 64 B]
+            const uint32_t sw64 = (lane >> 1) & 3;
 #pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    uint4 qa, qd;
-                    T* ea = reinterpret_cast<T*>(&qa);
-                    T* ed = reinterpret_cast<T*>(&qd);
+            for (int g = 0; g < 4; ++g) {
+                uint32_t e[4];
 #pragma unroll
-                    for (int x = 0; x < 8; ++x) {
-                        ea[x] = from_f32<T>(__uint_as_float(a[g * 8 + x]) * p.inv_keep);
-                        ed[x] = from_f32<T>(__uint_as_float(d[g * 8 + x]) * p.scale);
-                    }
-                    *reinterpret_cast<uint4*>(dvp + g * 8) = qa;
-                    *reinterpret_cast<uint4*>(dk + g * 8) = qd;
-                }
+                for (int x = 0; x < 4; ++x)
+                    e[x] = pack2<T>(__uint_as_float(a[g * 8 + x * 2]) * f, __uint_as_float(a[g * 8 + x * 2 + 1]) * f);
+                *reinterpret_cast<uint4*>(stage + lane * 64 + ((g ^ sw64) << 4)) = make_uint4(e[0], e[1], e[2], e[3]);
+            }
+            __syncwarp();
+            const long long ld = is_k ? p.dk_ss : p.dv_ss;
+            T* out = reinterpret_cast<T*>(is_k ? p.dK : p.dV) + b * (is_k ? p.dk_sb : p.dv_sb) + h * (is_k ? p.dk_sh : p.dv_sh) +
+                     half * 32 + (lane & 3) * 8;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int row = u * 8 + (lane >> 2);
+                const long long k = key0 + (warp & 3) * 32 + row;
+                if (k < p.S)
+                    *reinterpret_cast<uint4*>(out + k * ld) =
+                        *reinterpret_cast<const uint4*>(stage + row * 64 + (((lane & 3) ^ ((row >> 1) & 3)) << 4));
             }
         }
     }
@@ -409,7 +427,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
         }
         __syncthreads();
     }
-    if (warp == 8) {
+    if (warp == LOAD_WARP) {
         tc_fence_after();
         tmem_dealloc(tmem, BWD_TMEM_COLS);
     }

@@ -111,6 +111,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
     return false;
 }
 
+// The same for a whole converged warp: one answer for all lanes
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
 // ---------------------------------------------------------------------------
 // TMA
 // ---------------------------------------------------------------------------
@@ -377,6 +382,16 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
           "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        :
+        : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+          "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
+          "r"(r[14]), "r"(r[15])
+        : "memory");
+}
 
 // ---------------------------------------------------------------------------
 // descriptors
@@ -394,6 +409,41 @@ __device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr, uin
     d |= static_cast<uint64_t>(1) << 46;  // descriptor version (Blackwell)
     d |= static_cast<uint64_t>(2) << 61;  // SWIZZLE_128B
     return d;
+}
+// The same in parts, for issuing warps that have few cycles per product: the upper half is the same for every operand
+// with 1 KiB between its row groups, and the lower half moves on by bytes / 16.  `el`: nonzero in the lane that issues
+// (elect_one); the others pass by, so that the warp stays converged.
+constexpr uint32_t DESC_HI_SW128 = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t desc_lo_sw128(uint32_t smem_addr, uint32_t lbo) {
+    return ((smem_addr >> 4) & 0x3fff) | ((lbo >> 4) << 16);
+}
+__device__ __forceinline__ void umma_f16_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate,
+                                            uint32_t el) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "}\n"
+        :
+        : "r"(tmem_d), "l"(static_cast<uint64_t>(DESC_HI_SW128) << 32 | a_lo),
+          "l"(static_cast<uint64_t>(DESC_HI_SW128) << 32 | b_lo), "r"(idesc), "r"(accumulate), "r"(el)
+        : "memory");
+}
+__device__ __forceinline__ void umma_f16_ts_lo(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc,
+                                               uint32_t accumulate, uint32_t el) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "}\n"
+        :
+        : "r"(tmem_d), "r"(tmem_a), "l"(static_cast<uint64_t>(DESC_HI_SW128) << 32 | b_lo), "r"(idesc), "r"(accumulate),
+          "r"(el)
+        : "memory");
 }
 // Instruction descriptor for kind::f16, fp32 accumulate.
 //   fmt: 0 = fp16, 1 = bf16; major: 0 = K-major, 1 = MN-major.
