@@ -200,7 +200,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(used + STAGES);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5;
+    // (the same for all lanes, for the compiler too: what the issuing warps compute from it stays in uniform registers)
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int lane = threadIdx.x & 31;
     // PAIR: rank of this CTA in its pair; the first CTA issues the MMAs and owns the `full` / `tempty` counts
     const uint32_t crank = PAIR ? cluster_ctarank() : 0u;
@@ -243,155 +244,159 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
-            // ---------------- TMA producer ----------------
-            // One thread issues every copy, and a step must not take it longer than the 512 cycles its bytes need on the
-            // way from L2 (62 bytes a cycle): what does not change from step to step is worked out per tile, and the
-            // filter tap is counted on.  A division per step (and, MN-major, one per column block) for the tap held back
-            // the convolution's products: 3x3, 32 x 28 x 28, 1024 to 1024 channels with batch norm, forward and backward,
-            // 1550 -> 1354 us.
-            int stage = 0;
-            uint32_t phase = 0;
-            uint32_t ag_ready = 0;
-            bool ok = true;
-            const bool a_k = p.a_major == 0, b_k = p.b_major == 0, a_merged = p.a_merged, b_merged = p.b_merged;
-            const bool gather = p.ag_nranks > 1, conv = p.conv_kb_per_tap > 0;
-            // PAIR: both CTAs' bytes are counted on the first CTA's barrier
-            const uint32_t full0 = PAIR ? mapa_shared(smem_u32(full), 0) : smem_u32(full);
-            for (int tile = tile0; tile < p.num_tiles && ok; tile += tile_step) {
-                int mb, nb, b, kb_begin, kb_end;
-                tile_coords(p, tile, mb, nb, b, kb_begin, kb_end);
-                const int m0 = mb * TILE_M + static_cast<int>(crank) * BM;
-                const int n0 = nb * BN + (PAIR ? static_cast<int>(crank) * (BN / 2) : 0);
-                // position along K in A and in B, and the rows (columns) of each: A's (K-major) shift with the filter tap,
-                // B's (MN-major) move on by a block of columns per tap
-                int ak = kb_begin * BK, am = m0, bk = ak, bn = n0;
-                int tap = 0, left = 0x7fffffff;   // steps until the next tap, or until a gathered K wraps around
-                if (conv) {
-                    tap = kb_begin / p.conv_kb_per_tap;
-                    ak -= tap * p.conv_kb_per_tap * BK;
-                    am = m0 + p.conv_shift[tap];
-                    left = p.conv_kb_per_tap - ak / BK;
-                    if (!b_k) {
-                        bk = ak;
-                        bn = n0 + tap * p.conv_b_tap_cols;
-                    }
-                } else if (p.wgrad_taps > 0 && b_merged) {
-                    // column block -> filter tap: the tap's rows are shifted; past the last tap the columns lie outside
-                    // the matrix and read as zero
-                    const int t = min(n0 / p.wgrad_cols, p.wgrad_taps - 1);
-                    bn = n0 - t * p.wgrad_cols;
-                    bk += p.conv_shift[t];
-                } else if (gather && b_k) {
-                    // start with the k-range this rank holds itself
-                    const int own = p.ag_my_idx * (p.ag_cols / BK);
-                    ak = bk = (kb_begin + own < p.num_kb ? kb_begin + own : kb_begin + own - p.num_kb) * BK;
-                    left = p.num_kb - ak / BK;
+        // ---------------- TMA producer ----------------
+        // One lane issues every copy and the warp goes along: behind a branch for that lane, coordinates and addresses
+        // would have to be moved to the uniform registers for each instruction (16384 x 4096 x 1024, B MN-major: 128.4 ->
+        // 126.1 us; 4096 x 1024 x 6144 into fp32, both MN-major: 61.3 -> 58.4).  A step must not take longer than the 512
+        // cycles its bytes need on the way from L2 (62 bytes a cycle): what does not change from step to step is worked out
+        // per tile, and the filter tap is counted on.  A division per step (and, MN-major, one per column block) for the tap
+        // held back the convolution's products: 3x3, 32 x 28 x 28, 1024 to 1024 channels with batch norm, forward and
+        // backward, 1550 -> 1354 us.
+        const uint32_t el = elect_one();
+        int stage = 0;
+        uint32_t phase = 0;
+        uint32_t ag_ready = 0;
+        bool ok = true;
+        const bool a_k = p.a_major == 0, b_k = p.b_major == 0, a_merged = p.a_merged, b_merged = p.b_merged;
+        const bool gather = p.ag_nranks > 1, conv = p.conv_kb_per_tap > 0;
+        // PAIR: both CTAs' bytes are counted on the first CTA's barrier
+        const uint32_t full0 = PAIR ? mapa_shared(smem_u32(full), 0) : smem_u32(full);
+        for (int tile = tile0; tile < p.num_tiles && ok; tile += tile_step) {
+            int mb, nb, b, kb_begin, kb_end;
+            tile_coords(p, tile, mb, nb, b, kb_begin, kb_end);
+            const int m0 = mb * TILE_M + static_cast<int>(crank) * BM;
+            const int n0 = nb * BN + (PAIR ? static_cast<int>(crank) * (BN / 2) : 0);
+            // position along K in A and in B, and the rows (columns) of each: A's (K-major) shift with the filter tap,
+            // B's (MN-major) move on by a block of columns per tap
+            int ak = kb_begin * BK, am = m0, bk = ak, bn = n0;
+            int tap = 0, left = 0x7fffffff;   // steps until the next tap, or until a gathered K wraps around
+            if (conv) {
+                tap = kb_begin / p.conv_kb_per_tap;
+                ak -= tap * p.conv_kb_per_tap * BK;
+                am = m0 + p.conv_shift[tap];
+                left = p.conv_kb_per_tap - ak / BK;
+                if (!b_k) {
+                    bk = ak;
+                    bn = n0 + tap * p.conv_b_tap_cols;
                 }
-                for (int kbi = kb_begin; kbi < kb_end; ++kbi) {
-                    if (gather) {
-                        // wait until every CTA has copied the shard this step reads into the local B buffer
-                        const int shard = (b_k ? bk : n0) / p.ag_cols;
-                        if (!(ag_ready & (1u << shard))) {
-                            bool got = false;
-                            const uint64_t t0 = globaltimer_ns();
-                            for (uint32_t it = 0; it < RB_MBAR_SPIN_LIMIT && !*abort_flag; ++it) {
-                                unsigned int v;
-                                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.ag_flags + shard) : "memory");
-                                if (v >= gridDim.x) {
-                                    got = true;
-                                    break;
-                                }
-                                if ((it & 0xff) == 0xff && globaltimer_ns() - t0 > RB_WAIT_LIMIT_NS) break;
-                                __nanosleep(64);
-                            }
-                            if (!got) {
-                                *abort_flag = 1;
-                                ok = false;
+            } else if (p.wgrad_taps > 0 && b_merged) {
+                // column block -> filter tap: the tap's rows are shifted; past the last tap the columns lie outside
+                // the matrix and read as zero
+                const int t = min(n0 / p.wgrad_cols, p.wgrad_taps - 1);
+                bn = n0 - t * p.wgrad_cols;
+                bk += p.conv_shift[t];
+            } else if (gather && b_k) {
+                // start with the k-range this rank holds itself
+                const int own = p.ag_my_idx * (p.ag_cols / BK);
+                ak = bk = (kb_begin + own < p.num_kb ? kb_begin + own : kb_begin + own - p.num_kb) * BK;
+                left = p.num_kb - ak / BK;
+            }
+            for (int kbi = kb_begin; kbi < kb_end; ++kbi) {
+                if (gather) {
+                    // wait until every CTA has copied the shard this step reads into the local B buffer
+                    const int shard = (b_k ? bk : n0) / p.ag_cols;
+                    if (!(ag_ready & (1u << shard))) {
+                        bool got = false;
+                        const uint64_t t0 = globaltimer_ns();
+                        for (uint32_t it = 0; it < RB_MBAR_SPIN_LIMIT; ++it) {
+                            if (__any_sync(0xffffffffu, *abort_flag)) break;
+                            unsigned int v;
+                            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.ag_flags + shard) : "memory");
+                            if (__all_sync(0xffffffffu, v >= gridDim.x)) {
+                                got = true;
                                 break;
                             }
-                            asm volatile("fence.proxy.async.global;" ::: "memory");
-                            ag_ready |= 1u << shard;
+                            if ((it & 0xff) == 0xff && __any_sync(0xffffffffu, globaltimer_ns() - t0 > RB_WAIT_LIMIT_NS)) break;
+                            __nanosleep(64);
                         }
-                    }
-                    if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    uint8_t* a_dst = sA + stage * A_STAGE_BYTES;
-                    uint8_t* b_dst = sB + stage * B_STAGE_BYTES;
-                    const uint32_t fb = full0 + stage * 8;
-                    if (!PAIR || crank == 0) mbar_arrive_expect_tx(&full[stage], (PAIR ? 2 : 1) * STAGE_BYTES);
-                    auto load_3d = [&](uint8_t* dst, const CUtensorMap* m, int c0, int c1) {
-                        if constexpr (PAIR)
-                            tma_load_3d_pair(dst, m, fb, c0, c1, b);
-                        else
-                            tma_load_3d(dst, m, &full[stage], c0, c1, b);
-                    };
-                    auto load_chunks = [&](uint8_t* dst, const CUtensorMap* m, int k, int chunk) {
-                        if constexpr (PAIR)
-                            tma_load_4d_pair(dst, m, fb, 0, k, chunk, b);
-                        else
-                            tma_load_4d(dst, m, &full[stage], 0, k, chunk, b);
-                    };
-                    if (a_k) {
-                        load_3d(a_dst, &tmA, ak, am);
-                    } else if (a_merged) {
-                        load_chunks(a_dst, &tmA, ak, am >> 6);
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < BM / 64; ++c) load_3d(a_dst + c * (BK * 128), &tmA, am + c * 64, ak);
-                    }
-                    if (b_k) {
-                        load_3d(b_dst, &tmB, bk, bn);
-                    } else if (b_merged) {
-                        load_chunks(b_dst, &tmB, bk, bn >> 6);
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < Cfg<PAIR, BN>::B_ROWS / 64; ++c) {
-                            int cx = bn + c * 64, cy = bk;
-                            if (p.wgrad_taps > 0) {
-                                const int t = min(cx / p.wgrad_cols, p.wgrad_taps - 1);
-                                cx -= t * p.wgrad_cols;
-                                cy += p.conv_shift[t];
-                            }
-                            load_3d(b_dst + c * (BK * 128), &tmB, cx, cy);
+                        if (!got) {
+                            *abort_flag = 1;
+                            ok = false;
+                            break;
                         }
+                        asm volatile("fence.proxy.async.global;" ::: "memory");
+                        ag_ready |= 1u << shard;
                     }
-                    ak += BK;
-                    bk += BK;
-                    if (--left == 0) {
-                        ak = 0;
-                        if (conv) {
-                            left = p.conv_kb_per_tap;
-                            // (behind the last tap there is no further step)
-                            if (kbi + 1 < kb_end) am = m0 + p.conv_shift[++tap];
-                            if (!b_k) {
-                                bk = 0;
-                                bn += p.conv_b_tap_cols;
-                            }
-                        } else {
+                }
+                if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag)) {
+                    ok = false;
+                    break;
+                }
+                uint8_t* a_dst = sA + stage * A_STAGE_BYTES;
+                uint8_t* b_dst = sB + stage * B_STAGE_BYTES;
+                const uint32_t fb = full0 + stage * 8;
+                if (!PAIR || crank == 0) mbar_arrive_expect_tx_el(&full[stage], (PAIR ? 2 : 1) * STAGE_BYTES, el);
+                auto load_3d = [&](uint8_t* dst, const CUtensorMap* m, int c0, int c1) {
+                    if constexpr (PAIR)
+                        tma_load_3d_pair(dst, m, fb, c0, c1, b, el);
+                    else
+                        tma_load_3d_el(dst, m, &full[stage], c0, c1, b, el);
+                };
+                auto load_chunks = [&](uint8_t* dst, const CUtensorMap* m, int k, int chunk) {
+                    if constexpr (PAIR)
+                        tma_load_4d_pair(dst, m, fb, 0, k, chunk, b, el);
+                    else
+                        tma_load_4d_el(dst, m, &full[stage], 0, k, chunk, b, el);
+                };
+                if (a_k) {
+                    load_3d(a_dst, &tmA, ak, am);
+                } else if (a_merged) {
+                    load_chunks(a_dst, &tmA, ak, am >> 6);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < BM / 64; ++c) load_3d(a_dst + c * (BK * 128), &tmA, am + c * 64, ak);
+                }
+                if (b_k) {
+                    load_3d(b_dst, &tmB, bk, bn);
+                } else if (b_merged) {
+                    load_chunks(b_dst, &tmB, bk, bn >> 6);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < Cfg<PAIR, BN>::B_ROWS / 64; ++c) {
+                        int cx = bn + c * 64, cy = bk;
+                        if (p.wgrad_taps > 0) {
+                            const int t = min(cx / p.wgrad_cols, p.wgrad_taps - 1);
+                            cx -= t * p.wgrad_cols;
+                            cy += p.conv_shift[t];
+                        }
+                        load_3d(b_dst + c * (BK * 128), &tmB, cx, cy);
+                    }
+                }
+                ak += BK;
+                bk += BK;
+                if (--left == 0) {
+                    ak = 0;
+                    if (conv) {
+                        left = p.conv_kb_per_tap;
+                        // (behind the last tap there is no further step)
+                        if (kbi + 1 < kb_end) am = m0 + p.conv_shift[++tap];
+                        if (!b_k) {
                             bk = 0;
+                            bn += p.conv_b_tap_cols;
                         }
+                    } else {
+                        bk = 0;
                     }
-                    if (++stage == STAGES) {
-                        stage = 0;
-                        phase ^= 1;
-                    }
+                }
+                if (++stage == STAGES) {
+                    stage = 0;
+                    phase ^= 1;
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && crank == 0) {
+        if (crank == 0) {
             // ---------------- MMA issuer (PAIR: the first CTA issues for both) ----------------
+            // (one lane issues, the warp goes along: as above)
+            const uint32_t el = elect_one();
             constexpr int fmt = (sizeof(InT) == 2 && std::is_same<InT, __nv_bfloat16>::value) ? 1 : 0;
             const uint32_t idesc = make_idesc_f16(fmt, p.a_major, p.b_major, TILE_M, BN);
             // per-UMMA_K (16 elements) advance of the smem start address, in the descriptors' units of 16 bytes
             const uint32_t a_kstep = (p.a_major == 0) ? 32u / 16 : 2048u / 16;
             const uint32_t b_kstep = (p.b_major == 0) ? 32u / 16 : 2048u / 16;
-            // descriptors of the first stage: the address of any other is added to their low bits
-            const uint64_t a_desc = make_smem_desc_sw128(smem_u32(sA), (p.a_major == 0) ? 16u : BK * 128u, 1024);
-            const uint64_t b_desc = make_smem_desc_sw128(smem_u32(sB), (p.b_major == 0) ? 16u : BK * 128u, 1024);
+            // descriptors of the first stage (their low halves): the address of any other is added
+            const uint32_t a_desc = desc_lo_sw128(smem_u32(sA), (p.a_major == 0) ? 16u : BK * 128u);
+            const uint32_t b_desc = desc_lo_sw128(smem_u32(sB), (p.b_major == 0) ? 16u : BK * 128u);
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -399,42 +404,44 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             for (int tile = tile0; tile < p.num_tiles && ok; tile += tile_step, ++it) {
                 const int acc = it & 1;
                 const uint32_t acc_phase = (it >> 1) & 1;
-                if (!(PAIR ? mbar_wait_cluster(&tempty[acc], acc_phase ^ 1, abort_flag)
-                           : mbar_wait(&tempty[acc], acc_phase ^ 1, abort_flag)))
+                if (!(PAIR ? mbar_wait_cluster_warp(&tempty[acc], acc_phase ^ 1, abort_flag)
+                           : mbar_wait_warp(&tempty[acc], acc_phase ^ 1, abort_flag)))
                     break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
                 int mb_, nb_, b_, kb_begin, kb_end;
                 tile_coords(p, tile, mb_, nb_, b_, kb_begin, kb_end);
                 for (int kb = kb_begin; kb < kb_end; ++kb) {
-                    if (!(PAIR ? mbar_wait_cluster(&full[stage], phase, abort_flag)
-                               : mbar_wait(&full[stage], phase, abort_flag))) {
+                    if (!(PAIR ? mbar_wait_cluster_warp(&full[stage], phase, abort_flag)
+                               : mbar_wait_warp(&full[stage], phase, abort_flag))) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint64_t da0 = a_desc + static_cast<uint32_t>(stage) * (A_STAGE_BYTES / 16);
-                    const uint64_t db0 = b_desc + static_cast<uint32_t>(stage) * (B_STAGE_BYTES / 16);
+                    const uint32_t da0 = a_desc + static_cast<uint32_t>(stage) * (A_STAGE_BYTES / 16);
+                    const uint32_t db0 = b_desc + static_cast<uint32_t>(stage) * (B_STAGE_BYTES / 16);
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k) {
-                        const uint64_t da = da0 + k * a_kstep, db = db0 + k * b_kstep;
+                        const uint32_t da = da0 + k * a_kstep, db = db0 + k * b_kstep;
                         if constexpr (PAIR)
-                            umma_f16_pair(d_tmem, da, db, idesc, (kb > kb_begin || k > 0) ? 1u : 0u);
+                            umma_f16_pair_lo(d_tmem, da, db, idesc, (kb > kb_begin || k > 0) ? 1u : 0u, el);
                         else
-                            umma_f16(d_tmem, da, db, idesc, (kb > kb_begin || k > 0) ? 1u : 0u);
+                            umma_f16_lo(d_tmem, da, db, idesc, (kb > kb_begin || k > 0) ? 1u : 0u, el);
                     }
                     // frees the stage (PAIR: in both CTAs), or hands it on to the warps that sum its columns
                     uint64_t* done = p.a_colsum ? &used[stage] : &empty[stage];
-                    if constexpr (PAIR)
-                        umma_commit_pair(done, 3);
-                    else
-                        umma_commit(done);
+                    if (el) {
+                        if constexpr (PAIR)
+                            umma_commit_pair(done, 3);
+                        else
+                            umma_commit(done);
+                    }
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
-                if (ok) {
+                if (ok && el) {
                     if constexpr (PAIR)
                         umma_commit_pair(&tfull[acc], 3);
                     else

@@ -66,6 +66,17 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// (`el`: nonzero in the lane that does it; the rest of a converged warp passes by)
+__device__ __forceinline__ void mbar_arrive_expect_tx_el(uint64_t* bar, uint32_t bytes, uint32_t el) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "setp.ne.b32 q, %2, 0;\n\t"
+        "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t"
+        "}\n" ::"r"(smem_u32(bar)),
+        "r"(bytes), "r"(el)
+        : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -140,6 +151,35 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m
         :
         : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)),
           "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+        : "memory");
+}
+// (`el`: nonzero in the lane that issues; the rest of a converged warp passes by)
+__device__ __forceinline__ void tma_load_3d_el(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2,
+                                               uint32_t el) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "setp.ne.b32 q, %6, 0;\n\t"
+        "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5}], [%2];\n\t"
+        "}\n"
+        :
+        : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)),
+          "r"(c0), "r"(c1), "r"(c2), "r"(el)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_4d_el(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2,
+                                               int c3, uint32_t el) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "setp.ne.b32 q, %7, 0;\n\t"
+        "@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t"
+        "}\n"
+        :
+        : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)),
+          "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(el)
         : "memory");
 }
 
@@ -281,6 +321,9 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
     *abort_flag = 1;
     return false;
 }
+__device__ __forceinline__ bool mbar_wait_cluster_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag));
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(smem_result)),
@@ -294,20 +337,6 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
                  : "memory");
 }
-// One thread of the pair's first CTA issues; each CTA supplies its 128 rows of A and its half of B from
-// the same shared-memory offsets, and receives its 128 rows of D in its own tensor memory.
-__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                              uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-        "}\n"
-        :
-        : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 // arrives on the barrier at this offset in every CTA of `cta_mask` once the pair's MMAs so far are done
 __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t cta_mask) {
     asm volatile(
@@ -319,23 +348,31 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t cta_mas
 // tiled load into this CTA's shared memory whose completion is counted on a barrier of the pair's first
 // CTA (`bar_cluster_addr` from mapa_shared); no multicast: every CTA fetches its own tile
 __device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr,
-                                                 int c0, int c1, int c2) {
+                                                 int c0, int c1, int c2, uint32_t el) {
     asm volatile(
-        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5}], [%2];"
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "setp.ne.b32 q, %6, 0;\n\t"
+        "@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5}], [%2];\n\t"
+        "}\n"
         :
         : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr),
-          "r"(c0), "r"(c1), "r"(c2)
+          "r"(c0), "r"(c1), "r"(c2), "r"(el)
         : "memory");
 }
 __device__ __forceinline__ void tma_load_4d_pair(void* smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr,
-                                                 int c0, int c1, int c2, int c3) {
+                                                 int c0, int c1, int c2, int c3, uint32_t el) {
     asm volatile(
-        "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5, %6}], [%2];"
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "setp.ne.b32 q, %7, 0;\n\t"
+        "@q cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t"
+        "}\n"
         :
         : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr),
-          "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+          "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(el)
         : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() {
@@ -443,6 +480,22 @@ __device__ __forceinline__ void umma_f16_ts_lo(uint32_t tmem_d, uint32_t tmem_a,
         :
         : "r"(tmem_d), "r"(tmem_a), "l"(static_cast<uint64_t>(DESC_HI_SW128) << 32 | b_lo), "r"(idesc), "r"(accumulate),
           "r"(el)
+        : "memory");
+}
+// One thread of the pair's first CTA issues; each CTA supplies its 128 rows of A and its half of B from
+// the same shared-memory offsets, and receives its 128 rows of D in its own tensor memory.
+__device__ __forceinline__ void umma_f16_pair_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                                 uint32_t accumulate, uint32_t el) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "}\n"
+        :
+        : "r"(tmem_d), "l"(static_cast<uint64_t>(DESC_HI_SW128) << 32 | a_lo),
+          "l"(static_cast<uint64_t>(DESC_HI_SW128) << 32 | b_lo), "r"(idesc), "r"(accumulate), "r"(el)
         : "memory");
 }
 // Instruction descriptor for kind::f16, fp32 accumulate.
