@@ -29,6 +29,7 @@
 // (src/torch/TorchDriver.cpp:566) and in src/distop/DistMatmul.cpp:97-214.
 #include "gemm_tcgen05.h"
 
+#include <algorithm>
 #include <cstdlib>
 #include <mutex>
 
@@ -69,6 +70,9 @@ struct GemmKernelParams {
     int a_major, b_major;
     int num_m_blocks, num_n_blocks, num_tiles, num_kb;
     int base_tiles, split_k, kb_per_split;  // split-K: num_tiles = base_tiles * split_k
+    // the last, partly filled wave of tiles [tail_first, base_tiles) in an arrangement of its own (see Tail): 0 tiles: none
+    int tail_first, tail_tiles, tail_split, tail_kb, tail_units;
+    int partial;                            // a work item may hold part of a tile's K: results are added
     int rs_nranks, rs_cols;                 // reduce-scatter epilogue: column block j -> rs_peer[j]
     void* rs_peer[8];
     // all-gather prologue: B is assembled in local memory from column shards held by the ranks of a group
@@ -102,10 +106,29 @@ struct GemmKernelParams {
 
 __device__ __forceinline__ void tile_coords(const GemmKernelParams& p, int tile, int& mb, int& nb,
                                             int& b, int& kb_begin, int& kb_end) {
-    const int ks = tile / p.base_tiles;
-    tile -= ks * p.base_tiles;
-    kb_begin = ks * p.kb_per_split;
-    kb_end = min(p.num_kb, kb_begin + p.kb_per_split);
+    if (p.tail_tiles > 0 && tile >= p.tail_first) {
+        const int r = tile - p.tail_first;
+        int t = r % p.tail_tiles;
+        if (p.tail_split > 1) {   // equal parts of K, one wave of them
+            kb_begin = r / p.tail_tiles * p.tail_kb;
+            kb_end = min(p.num_kb, kb_begin + p.tail_kb);
+        } else if (r < p.tail_tiles) {   // owners: the first tail_kb steps of a tile each
+            kb_begin = 0;
+            kb_end = p.tail_kb;
+        } else {   // helpers: the rest of one tile after another
+            const int round = r / p.tail_units, x = r - round * p.tail_units - p.tail_tiles;
+            t = round * (p.tail_units - p.tail_tiles) + x;
+            kb_begin = p.tail_kb;
+            kb_end = p.num_kb;
+            if (x < 0 || t >= p.tail_tiles) t = kb_end = 0;   // (an owner's place in a later round: nothing to do)
+        }
+        tile = p.tail_first + t;
+    } else {
+        const int ks = tile / p.base_tiles;
+        tile -= ks * p.base_tiles;
+        kb_begin = ks * p.kb_per_split;
+        kb_end = min(p.num_kb, kb_begin + p.kb_per_split);
+    }
     const int per_batch = p.num_m_blocks * p.num_n_blocks;
     b = tile / per_batch;
     int t = tile - b * per_batch;
@@ -401,16 +424,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             uint32_t phase = 0;
             bool ok = true;
             int it = 0;
-            for (int tile = tile0; tile < p.num_tiles && ok; tile += tile_step, ++it) {
+            for (int tile = tile0; tile < p.num_tiles && ok; tile += tile_step) {
+                int mb_, nb_, b_, kb_begin, kb_end;
+                tile_coords(p, tile, mb_, nb_, b_, kb_begin, kb_end);
+                if (kb_begin >= kb_end) continue;
                 const int acc = it & 1;
                 const uint32_t acc_phase = (it >> 1) & 1;
+                ++it;
                 if (!(PAIR ? mbar_wait_cluster_warp(&tempty[acc], acc_phase ^ 1, abort_flag)
                            : mbar_wait_warp(&tempty[acc], acc_phase ^ 1, abort_flag)))
                     break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
-                int mb_, nb_, b_, kb_begin, kb_end;
-                tile_coords(p, tile, mb_, nb_, b_, kb_begin, kb_end);
                 for (int kb = kb_begin; kb < kb_end; ++kb) {
                     if (!(PAIR ? mbar_wait_cluster_warp(&full[stage], phase, abort_flag)
                                : mbar_wait_warp(&full[stage], phase, abort_flag))) {
@@ -577,12 +602,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             uint32_t turn = 0;   // which half the next 16-bit block takes: counted over tiles, whose blocks may be odd in number
             const uint32_t sw64 = (lane >> 1) & 3, sw128 = lane & 7;
             constexpr bool OUT16 = sizeof(OutT) == 2;
-            const bool add_out = !OUT16 && (accum || p.split_k > 1);
+            const bool add_out = !OUT16 && (accum || p.partial);
             bool ok = true;
-            for (int tile = tile0; tile < p.num_tiles && ok; tile += tile_step, ++it) {
+            for (int tile = tile0; tile < p.num_tiles && ok; tile += tile_step) {
                 int mb, nb, b, kb_begin, kb_end;
                 tile_coords(p, tile, mb, nb, b, kb_begin, kb_end);
+                if (kb_begin >= kb_end) continue;
                 const int acc = it & 1;
+                const uint32_t acc_phase = (it >> 1) & 1;
+                ++it;
                 const int row0 = mb * TILE_M + static_cast<int>(crank) * BM + q * 32;
                 const int col0 = nb * BN + chalf * (BN / 2);
                 const bool row_ok = row0 + lane < p.M;
@@ -593,7 +621,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     tma_load_3d(stage_buf, &tmAux, abar, col0 + c * 32, row0, b);
                 };
                 if (act_dgelu && nblk > 0 && lane == 0) fetch_aux(0);
-                if (!mbar_wait(&tfull[acc], (it >> 1) & 1, abort_flag)) break;
+                if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) break;
                 tc_fence_after();
                 if (nblk == 0) release_acc(acc);
                 const long long row_off = static_cast<long long>(b) * p.strideD +
@@ -711,11 +739,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             // the staging memory must outlive the copies that read it; their writes are complete when the kernel is
             if (lane == 0) tma_store_wait_read<0>();
         }
-        for (int tile = p.staged ? p.num_tiles : tile0; tile < p.num_tiles; tile += tile_step, ++it) {
+        for (int tile = p.staged ? p.num_tiles : tile0; tile < p.num_tiles; tile += tile_step) {
             int mb, nb, b, kb_begin, kb_end;
             tile_coords(p, tile, mb, nb, b, kb_begin, kb_end);
+            if (kb_begin >= kb_end) continue;
             const int acc = it & 1;
             const uint32_t acc_phase = (it >> 1) & 1;
+            ++it;
             if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) break;
             tc_fence_after();
             int row = mb * TILE_M + static_cast<int>(crank) * BM + row_in_tile;
@@ -746,7 +776,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 #pragma unroll
                 for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
                 if constexpr (std::is_same<OutT, float>::value) {
-                    if (p.split_k > 1 || p.rs_nranks > 1) {
+                    if (p.partial || p.rs_nranks > 1) {
                         // partial sums (a K slice, and/or one replica's share of a reduce-scatter):
                         // accumulate with vector reductions.  With rs_nranks > 1 the output columns
                         // are split in equal blocks and block j lives in rank j's buffer, so the
@@ -1073,7 +1103,38 @@ static bool pair_enabled() {
 struct Tiling {
     bool pair;
     int tn, m_blocks, n_blocks, split;
+    int tail_tiles, tail_split, tail_kb;   // see Tail
 };
+// The tiles that do not fill the last wave of the CTA pairs, of a product that is added to an fp32 matrix: K is shared out
+// so that every pair has something to do.
+//  - Fewer tiles than half the pairs (36 of 74): K in `split` equal parts, one wave of them.
+//  - More: each tile's pair takes the first `kb` steps, all in step, so that operands are shared through L2; the pairs left
+//    over take the remaining steps of one tile after another.
+// 30528 x 1024 (480 tiles: 6.5 waves, not 7) by 8192 rows 452 -> 443 us, by 6144 346 -> 340 us.  Only behind full waves:
+// with fewer tiles than pairs this is faster still (4096 x 1024 by 16384, 64 tiles: 129 -> 121 us), but its parts are
+// longer than those of the even split below, and the tensor core's sums lose with length (relative error 2.6e-6 ->
+// 1.6e-5).  Behind full waves parts are shorter than the whole tiles they replace.
+struct Tail {
+    int split, kb;       // split > 1: equal parts of kb steps; 1: owners and helpers; 0: whole tiles
+    double cost;         // in k steps of the longest chain of a pair
+};
+constexpr double DRAIN_STEPS = 6.0;   // what a part costs besides its own steps
+static Tail choose_tail(int tiles, int units, int num_kb) {
+    Tail t = {0, num_kb, num_kb + DRAIN_STEPS};
+    if (tiles <= 0 || tiles >= units) return t;
+    if (2 * tiles <= units) {
+        const int s = std::min(units / tiles, num_kb / 4);
+        if (s > 1) {
+            const int kb = (num_kb + s - 1) / s;
+            t = {(num_kb + kb - 1) / kb, kb, kb + DRAIN_STEPS};
+        }
+        return t;
+    }
+    const int rounds = (tiles + units - tiles - 1) / (units - tiles);
+    const int kb = static_cast<int>((rounds * (num_kb + DRAIN_STEPS) - DRAIN_STEPS) / (rounds + 1) + 0.999);
+    if (kb < num_kb && num_kb - kb >= 4) t = {1, kb, std::max(kb + DRAIN_STEPS, rounds * (num_kb - kb + DRAIN_STEPS))};
+    return t;
+}
 static Tiling choose_tiling(const RbGemmArgs& a) {
     // The pair kernel (256 x 256 tile over two SMs) serves every GEMM with enough work to fill the GPU:
     // enough tiles, or few tiles and a long K that is split (weight gradients); the gather prologue and the
@@ -1131,7 +1192,18 @@ static Tiling choose_tiling(const RbGemmArgs& a) {
         }
     }
     t.n_blocks = static_cast<int>((a.N + t.tn - 1) / t.tn);
-    t.split = split_for(t.m_blocks * t.n_blocks * static_cast<int>(a.batch));
+    const int tiles = t.m_blocks * t.n_blocks * static_cast<int>(a.batch);
+    t.split = split_for(tiles);
+    t.tail_tiles = t.tail_split = t.tail_kb = 0;
+    if (accum32 && t.pair && tiles > units && a.rs_nranks <= 1 && a.ag_nranks <= 1 && !a.in_order && num_kb >= 8) {
+        const Tail tail = choose_tail(tiles % units, units, num_kb);
+        // what the last wave takes less has to be worth it over all of them
+        if (tail.split > 0 && num_kb + DRAIN_STEPS - tail.cost > 0.01 * (tiles / units + 1) * num_kb) {
+            t.tail_tiles = tiles % units;
+            t.tail_split = tail.split;
+            t.tail_kb = tail.kb;
+        }
+    }
     return t;
 }
 
@@ -1196,6 +1268,17 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     p.kb_per_split = (p.num_kb + p.split_k - 1) / p.split_k;
     p.split_k = (p.num_kb + p.kb_per_split - 1) / p.kb_per_split;
     p.num_tiles = p.base_tiles * p.split_k;
+    p.tail_tiles = tiling.tail_tiles;
+    p.tail_first = p.base_tiles - tiling.tail_tiles;
+    p.tail_split = tiling.tail_split;
+    p.tail_kb = tiling.tail_kb;
+    p.tail_units = num_sms() / 2;
+    p.partial = p.split_k > 1 || p.tail_tiles > 0;
+    if (p.tail_tiles > 0) {
+        const int helpers = p.tail_units - p.tail_tiles;
+        p.num_tiles = p.tail_first + (p.tail_split > 1 ? p.tail_tiles * p.tail_split
+                                                       : p.tail_units * ((p.tail_tiles + helpers - 1) / helpers));
+    }
     p.D = a->D;
     p.bias = a->bias;
     p.residual = a->residual;

@@ -61,6 +61,9 @@ typedef struct RbGemmArgs {
     int32_t wgrad_taps;
     float* a_colsum;  // a_major = 1 only: the column sums of the stored A ([K, M]) are added to these M floats
     int32_t tile_n;   // columns of the single-CTA kernel's tile: 0 (chosen by size), 64, 128 or 256
+    // 1: tiles that could be summed whole are (torch.use_deterministic_algorithms): parts of one are added in the order
+    // they arrive
+    int32_t in_order;
 } RbGemmArgs;
 
 // returns 0 on success, <0 on a host-side error (-2: operand not 16 B aligned)

@@ -206,6 +206,7 @@ void gemm(const Mat& a, const Mat& b, bool trans_a, bool trans_b, void* out, boo
               (e.accumulate ? RB_GEMM_ACCUM : 0) | (e.aux_out ? RB_GEMM_AUX_OUT : 0);
     g.alpha = 1.f;
     g.a_colsum = e.a_colsum;
+    g.in_order = at::globalContext().deterministicAlgorithms() ? 1 : 0;
     check(api.gemm(&g, cur_stream()), "rb_gemm");
 }
 // Gradients of one weight and its bias: dW = dy^T x and, from the same pass over dy, db = its column sums.  Each is added
@@ -1013,6 +1014,7 @@ Tensor product(const Tensor& a, const Tensor& b, bool trans_a, bool trans_b, con
               (g.residual ? RB_GEMM_RESIDUAL : 0) | (accumulate ? RB_GEMM_ACCUM : 0) | (g.aux_out ? RB_GEMM_AUX_OUT : 0);
     g.alpha = static_cast<float>(alpha);
     g.max_ctas = static_cast<int32_t>(max_ctas);
+    g.in_order = at::globalContext().deterministicAlgorithms() ? 1 : 0;
     check(api.gemm(&g, cur_stream()), "rb_gemm");
     return out;
 }

@@ -30,6 +30,7 @@ class _Args(ctypes.Structure):
         ("map_hp", ctypes.c_int32), ("map_wp", ctypes.c_int32), ("map_h", ctypes.c_int32),
         ("map_w", ctypes.c_int32), ("map_pad", ctypes.c_int32), ("wgrad_taps", ctypes.c_int32),
         ("a_colsum", ctypes.c_void_p), ("tile_n", ctypes.c_int32),
+        ("in_order", ctypes.c_int32),
     ]
 
 
@@ -181,6 +182,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         for i, sh in enumerate(conv["shifts"]):
             args.conv_shift[i] = int(sh)
     args.tile_n = int(tile_n)
+    args.in_order = int(torch.are_deterministic_algorithms_enabled())
     args.a_colsum = _lib.ptr(a_colsum)
     if wgrad_shifts is not None:
         args.wgrad_taps = len(wgrad_shifts)

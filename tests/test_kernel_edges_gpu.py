@@ -314,3 +314,37 @@ def test_staged_blocks_of_many_tiles(dtype, N, tile_n, max_ctas):
         assert torch.equal(gemm(a, b, tile_n=tile_n, max_ctas=max_ctas), want)
     torch.cuda.synchronize()
     assert _lib.read_error() == 0
+
+
+# 74 pairs of SMs: 76 (2 left over), 111 (37: two parts each), 112 (38: 36 helpers, 2 rounds), 147 (73: one helper, too
+# little to share out) and 150 tiles
+@pytest.mark.parametrize("M,N", [(4864, 1024), (9472, 768), (3500, 2048), (5376, 1792), (3833, 2552)])
+@pytest.mark.parametrize("K", [448, 600, 1560])
+def test_gemm_last_wave_is_shared_out(M, N, K):
+    """Tiles of the last wave in parts, beside whole ones: small integers, so that every order of adding is exact."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops.gemm import gemm
+
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    dt = torch.bfloat16
+    a, b = (torch.randint(-3, 4, (K, n), generator=g, device="cuda").to(dt) for n in ((M + 7) // 8 * 8, (N + 7) // 8 * 8))
+    a, b = a[:, :M], b[:, :N]
+    want = a.double().t() @ b.double()
+    buf = torch.full((M + 1, N + 4), 5.0, device="cuda")
+    sums = torch.full((M,), 2.0, device="cuda")
+    gemm(a, b, trans_a=True, trans_b=False, out=buf[:M, :N], accumulate=True, a_colsum=sums)
+    assert torch.equal(buf[:M, :N].double(), want + 5.0) and (buf[M:] == 5.0).all() and (buf[:, N:] == 5.0).all()
+    assert torch.equal(sums.double(), a.double().sum(0) + 2.0)
+    # added whole when asked: the same bits every time
+    x, y = torch.randn(K, M, device="cuda").to(dt), torch.randn(K, N, device="cuda").to(dt)
+    torch.use_deterministic_algorithms(True)
+    try:
+        outs = []
+        for _ in range(4):
+            out = torch.full((M, N), 1e3, device="cuda")
+            gemm(x, y, trans_a=True, trans_b=False, out=out, accumulate=True)
+            outs.append(out)
+        assert all(torch.equal(o, outs[0]) for o in outs)
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert _lib.read_error() == 0
