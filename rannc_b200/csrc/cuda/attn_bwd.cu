@@ -27,6 +27,7 @@
 // attention chain (src/torch/TorchDriver.cpp:642-847).
 #include "attn.h"
 #include "attn_common.cuh"
+#include "launch.cuh"
 #include "tc_common.cuh"
 
 namespace rb {
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
     const int key0 = blockIdx.x * BKEYS, h = blockIdx.y, b = blockIdx.z;
     const int nq = (p.S + BQ - 1) / BQ;
 
+    grid_trigger();
     if (threadIdx.x == 0) {
         mbar_init(kv_full, 1);
         for (int st = 0; st < QD_STAGES; ++st) mbar_init(&qd_full[st], 1);
@@ -118,6 +120,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    grid_wait();   // all of the above runs beside the end of the kernel before
     constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
 
     if (warp == LOAD_WARP) {
@@ -438,10 +441,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
 // a [B, S, H, D] tensor), 8 lanes x 16 bytes per row, two rows of a thread in flight: bound by memory.
 template <typename T>
 __global__ void __launch_bounds__(256)
-    attn_delta_kernel(const T* __restrict__ O, const T* __restrict__ dO,
-                      float* __restrict__ delta, float* __restrict__ dq_accum, int B, int H, int S,
+    attn_delta_kernel(const T* O, const T* dO, float* __restrict__ delta, float* __restrict__ dq_accum, int B, int H, int S,
                       long long o_sb, long long o_ss, long long o_sh, long long d_sb, long long d_ss,
                       long long d_sh) {
+    grid_trigger();
+    grid_wait();
     const unsigned rows = static_cast<unsigned>(B) * S * H;   // < 2^31: checked by the caller
     const int sub = threadIdx.x & 7;
     // a block takes 64 consecutive rows: 32 and the 32 behind them
@@ -481,8 +485,10 @@ __global__ void __launch_bounds__(256)
 
 // dQ[b,q,h,:] = (T) acc[b,q,h,:]
 template <typename T>
-__global__ void attn_dq_convert_kernel(const float* __restrict__ acc, T* __restrict__ dQ, int B,
+__global__ void attn_dq_convert_kernel(const float* acc, T* __restrict__ dQ, int B,
                                        int H, int S, long long sb, long long ss, long long sh) {
+    grid_trigger();
+    grid_wait();
     const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;  // 8-element group
     const long long total = static_cast<long long>(B) * S * H * 8;
     if (i >= total) return;
@@ -511,7 +517,7 @@ static int launch_bwd(const RbAttnArgs& a, cudaStream_t st) {
     if ((rc = make_tmap_4d(&tdo, a.dO, a.dtype, D, S, H, B, a.do_ss * 2, a.do_sh * 2, a.do_sb * 2, 64, 128))) return rc;
     const long long rows = static_cast<long long>(a.B) * a.H * a.S;
     if (rows >= (1LL << 31) - 64) return -2;
-    attn_delta_kernel<T><<<static_cast<unsigned>((rows + 63) / 64), 256, 0, st>>>(
+    launch_after(attn_delta_kernel<T>, static_cast<unsigned>((rows + 63) / 64), 256, 0, st,
         static_cast<const T*>(a.O), static_cast<const T*>(a.dO), a.delta, a.dq_accum, a.B, a.H, a.S, a.o_sb,
         a.o_ss, a.o_sh, a.do_sb, a.do_ss, a.do_sh);
     AttnBwdParams p;
@@ -542,10 +548,10 @@ static int launch_bwd(const RbAttnArgs& a, cudaStream_t st) {
     dim3 grid((a.S + BKEYS - 1) / BKEYS, a.H, a.B);
     CUtensorMap tdq;
     if ((rc = make_tmap_4d_f32(&tdq, a.dq_accum, 64, S, H, B, H * 64 * 4, 64 * 4, S * H * 64 * 4, 32, 128))) return rc;
-    kern<<<grid, BWD_THREADS, BWD_SMEM, st>>>(tq, tk, tv, tdo, tdq, p);
+    launch_after(kern, grid, BWD_THREADS, BWD_SMEM, st, tq, tk, tv, tdo, tdq, p);
     const long long groups = rows * 8;
-    attn_dq_convert_kernel<T><<<static_cast<unsigned>((groups + 255) / 256), 256, 0, st>>>(
-        a.dq_accum, static_cast<T*>(a.dQ), a.B, a.H, a.S, a.dq_sb, a.dq_ss, a.dq_sh);
+    launch_after(attn_dq_convert_kernel<T>, static_cast<unsigned>((groups + 255) / 256), 256, 0, st,
+        static_cast<const float*>(a.dq_accum), static_cast<T*>(a.dQ), a.B, a.H, a.S, a.dq_sb, a.dq_ss, a.dq_sh);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

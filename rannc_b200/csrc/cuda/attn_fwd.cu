@@ -24,6 +24,7 @@
 
 #include "attn.h"
 #include "attn_common.cuh"
+#include "launch.cuh"
 #include "tc_common.cuh"
 
 namespace rb {
@@ -84,6 +85,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
     const int nchunks = (p.S + AK - 1) / AK;
     const int ntiles = (q_base + AQ < p.S) ? 2 : 1;
 
+    grid_trigger();
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
         for (int i = 0; i < 2; ++i) {
@@ -98,6 +100,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
         *abort_flag = 0;
         fence_mbar_init();
     }
+    grid_wait();   // (tensor memory is taken behind it here: the key bias decides the path, and is read first)
     int any_bias = FAST ? 0 : 1;
     if (FAST) {
         // per-key tables for the whole (padded) sequence: -inf bias masks the keys past its end
@@ -472,6 +475,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
     const int my_items = blockIdx.x < nitems ? (nitems - 1 - blockIdx.x) / gridDim.x + 1 : 0;
     const int total_chunks = my_items * nchunks;
 
+    grid_trigger();
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) {
             mbar_init(&q_full[i], 1);
@@ -497,6 +501,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    grid_wait();   // all of the above runs beside the end of the kernel before
     constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
     auto decode = [&](int item, int& b, int& h, int& q_base) {
         const int qp = item % nqp;
@@ -843,7 +848,7 @@ static int launch_fwd(const RbAttnArgs& a, cudaStream_t st) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pdev);
         if (sms <= 0) sms = 148;
         const int grid = nitems < sms ? static_cast<int>(nitems) : sms;
-        pk<<<grid, ATT_THREADS, ATTP_SMEM, st>>>(tq, tk, tv, p, static_cast<int>(nitems));
+        launch_after(pk, grid, ATT_THREADS, ATTP_SMEM, st, tq, tk, tv, p, static_cast<int>(nitems));
         return cudaGetLastError() == cudaSuccess ? 0 : -1;
     }
     const bool fast = (a.S + AK - 1) / AK * AK <= KB_MAX;
@@ -857,7 +862,7 @@ static int launch_fwd(const RbAttnArgs& a, cudaStream_t st) {
         attr_set[dev & 63][fast] = true;
     }
     dim3 grid((a.S + 2 * AQ - 1) / (2 * AQ), a.H, a.B);
-    kern<<<grid, ATT_THREADS, ATT_SMEM, st>>>(tq, tk, tv, p);
+    launch_after(kern, grid, ATT_THREADS, ATT_SMEM, st, tq, tk, tv, p);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

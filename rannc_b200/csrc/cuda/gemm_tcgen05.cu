@@ -33,6 +33,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "launch.cuh"
 #include "tc_common.cuh"
 
 namespace rb {
@@ -239,6 +240,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     const int tile0 = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
     const int tile_step = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
+    grid_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full[s], 1);
@@ -273,6 +275,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     if (PAIR) cluster_sync_all();   // the peer's barriers exist before anything signals them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    grid_wait();   // all of the above runs beside the end of the kernel before
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
@@ -1040,13 +1043,12 @@ static int launch(const RbGemmArgs& a, const CUtensorMap& tmA, const CUtensorMap
     if (!PAIR) {
         int grid = p.num_tiles < num_sms() ? p.num_tiles : num_sms();
         if (a.max_ctas > 0 && grid > a.max_ctas) grid = a.max_ctas;
-        kern<<<grid, GEMM_THREADS, smem, stream>>>(tmA, tmB, tmD, tmAux, p);
-        cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launch_after(kern, grid, GEMM_THREADS, smem, stream, tmA, tmB, tmD, tmAux, p);
         return e == cudaSuccess ? 0 : -static_cast<int>(e);
     }
     // one cluster of two CTAs per TPC; persistent over the pair tiles
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
@@ -1065,6 +1067,9 @@ static int launch(const RbGemmArgs& a, const CUtensorMap& tmA, const CUtensorMap
     int clusters = p.num_tiles < max_clusters[dev & 63] ? p.num_tiles : max_clusters[dev & 63];
     if (a.max_ctas > 1 && clusters > a.max_ctas / 2) clusters = a.max_ctas / 2;
     cfg.gridDim = dim3(2 * clusters, 1, 1);
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // (see launch_after)
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmD, tmAux, p);
     return e == cudaSuccess ? 0 : -static_cast<int>(e);
 }

@@ -1,0 +1,40 @@
+// Launches that overlap with the end of the kernel before them in the stream (programmatic dependent launch).
+//
+// Between two kernels a stream leaves the GPU idle for some microseconds: the last blocks of the first end one by one, the
+// second is launched, and its blocks set up barriers and tensor memory before their first load.  A kernel started by
+// launch_after begins while the one before it still runs: its blocks take the places that become free, do what depends
+// on no other kernel, and wait in grid_wait() until that kernel is complete and its writes are visible.
+//
+// Rules for a kernel that is launched this way:
+//  - every thread passes grid_wait() before its first access to global memory and before it ends.  (A kernel that ended
+//    without it could be complete before its predecessor, and the next one in the stream would wait for too little.)
+//  - what it reads is not declared const __restrict__: the compiler may move loads of memory that it takes to be constant
+//    for the kernel's lifetime across the wait.
+// grid_trigger() allows the next kernel's blocks to start as soon as all blocks of this one have called it or ended; it has
+// no effect on what that kernel may read.  Behind any other kernel, copy or event the launch is an ordinary one.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <utility>
+
+namespace rb {
+
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_after(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
+
+}  // namespace rb

@@ -17,6 +17,7 @@
 #include <cstdlib>
 #include <stdint.h>
 
+#include "launch.cuh"
 #include "philox.cuh"
 #include "tc_common.cuh"
 
@@ -98,13 +99,13 @@ struct LnRing {
 // A row of H = 256 * NCHUNK * WPR elements is shared by WPR warps.
 template <typename T, int NCHUNK, int WPR>
 __global__ void __launch_bounds__(LN_THREADS, LnRing<NCHUNK>::FWD_CTAS)
-    ln_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual,
-                  const T* __restrict__ gamma, const T* __restrict__ beta, T* __restrict__ y,
-                  T* __restrict__ z_out, float* __restrict__ mean_out, float* __restrict__ rstd_out,
+    ln_fwd_kernel(const T* x, const T* residual, const T* gamma, const T* beta, T* __restrict__ y, T* __restrict__ z_out, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                   int rows, float eps, uint32_t thr, float scale, uint64_t seed, uint64_t offset) {
     constexpr int H = NCHUNK * 256 * WPR;
     constexpr int RPB = LN_WARPS / WPR;  // rows per CTA per iteration
     constexpr int STAGES = LnRing<NCHUNK>::STAGES;
+    grid_trigger();
+    grid_wait();
     extern __shared__ uint4 ring[];  // [STAGES][x, residual][NCHUNK][LN_THREADS]
     __shared__ float2 sm[2][LN_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -189,13 +190,14 @@ __global__ void __launch_bounds__(LN_THREADS, LnRing<NCHUNK>::FWD_CTAS)
 // scratch layout: partial[blockIdx][0][H] = dgamma, partial[blockIdx][1][H] = dbeta
 template <typename T, int NCHUNK, int WPR>
 __global__ void __launch_bounds__(LN_THREADS, 2)
-    ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ z, const T* __restrict__ gamma,
-                  const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
+    ln_bwd_kernel(const T* dy, const T* z, const T* gamma, const float* mean_in, const float* rstd_in,
                   T* __restrict__ dz_out, T* __restrict__ dx_out, float* __restrict__ partial,
                   int rows, uint32_t thr, float scale, uint64_t seed, uint64_t offset) {
     constexpr int H = NCHUNK * 256 * WPR;
     constexpr int RPB = LN_WARPS / WPR;
     constexpr int STAGES = LnRing<NCHUNK>::STAGES;
+    grid_trigger();
+    grid_wait();
     extern __shared__ uint4 ring[];  // [STAGES][dy, z][NCHUNK][LN_THREADS]
     __shared__ float red[LN_WARPS][256 + 8];
     __shared__ float2 sm[2][LN_WARPS];
@@ -311,8 +313,9 @@ __global__ void __launch_bounds__(LN_THREADS, 2)
 // latency of its loads, so a thread has ten of them at most, four in flight (296 x 2048 floats: 5.2 -> 3.7 us).
 template <typename OutT>
 __global__ void __launch_bounds__(1024)
-    ln_bwd_reduce_kernel(const float* __restrict__ partial, OutT* __restrict__ dgamma,
-                         OutT* __restrict__ dbeta, int nblocks, int H, int accumulate) {
+    ln_bwd_reduce_kernel(const float* partial, OutT* dgamma, OutT* dbeta, int nblocks, int H, int accumulate) {
+    grid_trigger();
+    grid_wait();
     __shared__ float red[32][33];
     const int col2 = blockIdx.x * 32 + threadIdx.x;  // in [0, 2H)
     float s = 0.f;
@@ -352,11 +355,11 @@ static int launch_fwd(const void* x, const void* res, const void* g, const void*
     if (grid > cap) grid = cap;
     static bool allowed[64] = {false};
     if (!ln_allow_smem(ln_fwd_kernel<T, NCHUNK, WPR>, LnRing<NCHUNK>::BYTES, allowed)) return -1;
-    ln_fwd_kernel<T, NCHUNK, WPR><<<grid, LN_THREADS, LnRing<NCHUNK>::BYTES, st>>>(
-        static_cast<const T*>(x), static_cast<const T*>(res), static_cast<const T*>(g),
+    const cudaError_t e = launch_after(
+        ln_fwd_kernel<T, NCHUNK, WPR>, grid, LN_THREADS, LnRing<NCHUNK>::BYTES, st, static_cast<const T*>(x), static_cast<const T*>(res), static_cast<const T*>(g),
         static_cast<const T*>(b), static_cast<T*>(y), static_cast<T*>(z), mean, rstd, rows, eps,
         thr, scale, seed, offset);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return e == cudaSuccess ? 0 : -1;
 }
 
 template <typename T, int NCHUNK, int WPR>
@@ -367,11 +370,11 @@ static int launch_bwd(const void* dy, const void* z, const void* g, const float*
     const float scale = p > 0.f ? 1.f / (1.f - p) : 1.f;
     static bool allowed[64] = {false};
     if (!ln_allow_smem(ln_bwd_kernel<T, NCHUNK, WPR>, LnRing<NCHUNK>::BYTES, allowed)) return -1;
-    ln_bwd_kernel<T, NCHUNK, WPR><<<grid, LN_THREADS, LnRing<NCHUNK>::BYTES, st>>>(
-        static_cast<const T*>(dy), static_cast<const T*>(z), static_cast<const T*>(g), mean, rstd,
+    const cudaError_t e = launch_after(
+        ln_bwd_kernel<T, NCHUNK, WPR>, grid, LN_THREADS, LnRing<NCHUNK>::BYTES, st, static_cast<const T*>(dy), static_cast<const T*>(z), static_cast<const T*>(g), mean, rstd,
         static_cast<T*>(dz), static_cast<T*>(p > 0.f ? dx : nullptr), partial, rows, thr, scale,
         seed, offset);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return e == cudaSuccess ? 0 : -1;
 }
 
 }  // namespace rb
@@ -433,9 +436,10 @@ static int ln_bwd_rows(const void* dy, const void* z, const void* gamma, const f
 }
 template <typename OutT>
 static int ln_bwd_sums(const float* partial, void* dgamma, void* dbeta, int grid, int H, int accumulate, cudaStream_t st) {
-    ln_bwd_reduce_kernel<OutT><<<2 * H / 32, dim3(32, 32), 0, st>>>(partial, static_cast<OutT*>(dgamma),
-                                                                    static_cast<OutT*>(dbeta), grid, H, accumulate);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_after(ln_bwd_reduce_kernel<OutT>, 2 * H / 32, dim3(32, 32), 0, st, partial, static_cast<OutT*>(dgamma),
+                        static_cast<OutT*>(dbeta), grid, H, accumulate) == cudaSuccess
+               ? 0
+               : -1;
 }
 // An empty batch contributes nothing: the parameters' gradients are zero, or stay what they were.
 static int ln_bwd_empty(void* dgamma, void* dbeta, size_t bytes, int accumulate, cudaStream_t st) {

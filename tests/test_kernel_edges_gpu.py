@@ -348,3 +348,46 @@ def test_gemm_last_wave_is_shared_out(M, N, K):
     finally:
         torch.use_deterministic_algorithms(False)
     assert _lib.read_error() == 0
+
+
+@pytest.mark.parametrize("rows,S", [(96, 48), (384, 192), (6144, 512)])
+def test_kernels_in_a_row_wait_for_each_other(rows, S):
+    """Kernels that begin beside the end of the one before them, over buffers that are written again and again, with a
+    PyTorch kernel in between: the same bits as with the device idle before every launch."""
+    from rannc_b200.ops import kernels as K
+    from rannc_b200.ops.gemm import gemm
+
+    torch.manual_seed(3)
+    dt, H = torch.bfloat16, 256
+    w = [(torch.randn(3 * H, H, device="cuda") * H ** -0.5).to(dt), (torch.randn(H, H, device="cuda") * H ** -0.5).to(dt)]
+    g, b = torch.ones(H, device="cuda", dtype=dt), torch.zeros(H, device="cuda", dtype=dt)
+    x0 = torch.randn(rows, H, device="cuda").to(dt)
+
+    def run(idle):
+        sync = torch.cuda.synchronize if idle else (lambda: None)
+        x, qkv, y = x0.clone(), torch.empty(rows, 3 * H, device="cuda", dtype=dt), torch.empty_like(x0)
+        out = []
+        for step in range(12):
+            gemm(x, w[0], out=qkv)
+            sync()
+            q, k, v = (qkv.view(rows // S, S, 3, 4, 64)[:, :, i] for i in range(3))
+            o, lse = K.attn_fwd(q, k, v)
+            sync()
+            gemm(o.view(rows, H), w[1], out=y)
+            sync()
+            z, zin, mean, rstd = K.ln_fwd(y, x, g, b, 1e-5)
+            sync()
+            if step % 3 == 2:
+                z = z * 0.5
+                sync()
+            dx, dz, dg, db = K.ln_bwd(z, zin, g, mean, rstd)
+            sync()
+            dq, dk, dv = K.attn_bwd(q, k, v, o, lse, dx.view(rows // S, S, 4, 64))
+            sync()
+            x.copy_(z) if step % 2 else gemm(z, w[1], out=x)
+            sync()
+            out += [x.clone(), dk.clone(), dv.clone(), dz.clone()]   # (dQ and the parameters' sums: added as they arrive)
+        return out
+
+    for a, c in zip(run(True), run(False)):
+        assert torch.equal(a, c)
