@@ -20,7 +20,7 @@
 // PAIR variant (cta_group::2): two CTAs of a cluster -- the two SMs of a TPC -- share a 256 x 256 tile.
 // Each CTA loads its own 128 rows of A and HALF of the B tile (so a k step moves 32 KiB per SM instead
 // of 48 KiB: the single-CTA tile is limited by the L2 -> shared-memory path, not by the tensor core),
-// one thread of the first CTA issues the MMAs for both, and each CTA keeps and drains the accumulator of
+// one lane of the first CTA issues the MMAs for both, and each CTA keeps and drains the accumulator of
 // its own 128 rows.  Completion of both CTAs' loads is counted on the first CTA's barrier; stage-free
 // and accumulator-full signals go to both CTAs with one multicast commit.  No load is multicast.
 //
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             // block one step ahead.  16384 x 4096 x 1024 with bias, GELU and the value before it: 155 -> 142 us (137 with
             // the packed arithmetic below); 8192 x 30528 x 1024: 426 -> 386 us; weight gradient 4096 x 1024 x 16384:
             // 122 -> 116 us.  A block of 128 rows per four warps (a quarter of the copies, two barriers a block) was
-            // slower: 137 -> 142 us.
+            // slower: 137 -> 142 us; so were coalesced 16-byte stores from the staging block: 139 -> 159 us.
             uint8_t* stage_buf = sEpi + (warp - 2) * EPI_STAGE_BYTES;
             uint64_t* abar = &aux_full[warp - 2];
             uint32_t aux_phase = 0;

@@ -183,16 +183,6 @@ __device__ __forceinline__ void tma_load_4d_el(void* smem_dst, const CUtensorMap
         : "memory");
 }
 
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m, uint64_t* bar,
-                                            int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4}], [%2];"
-        :
-        : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)),
-          "r"(c0), "r"(c1)
-        : "memory");
-}
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, const void* smem_src, int c0,
                                              int c1, int c2) {
     asm volatile(
@@ -217,10 +207,6 @@ template <int N>
 __device__ __forceinline__ void tma_store_wait_read() {
     asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
-template <int N>
-__device__ __forceinline__ void tma_store_wait() {
-    asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
-}
 
 // ---------------------------------------------------------------------------
 // tcgen05 / TMEM
@@ -243,32 +229,6 @@ __device__ __forceinline__ void tc_fence_before() {
 }
 __device__ __forceinline__ void tc_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-// D[tmem] (+)= A[smem desc] * B[smem desc]; one thread issues.
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
-                                         uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-        "}\n"
-        :
-        : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem desc]
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b,
-                                            uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-        "}\n"
-        :
-        : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
 }
 // mbarrier arrives once all MMAs issued so far by this thread have completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -408,27 +368,18 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 // ---------------------------------------------------------------------------
 // descriptors
 // ---------------------------------------------------------------------------
-// Shared-memory matrix descriptor, 128-byte swizzle.  `lbo`/`sbo` in bytes.
-//   K-major  : rows of 128 B (64 x 16-bit along K); 8-row groups `sbo` apart.
+// Shared-memory matrix descriptor, 128-byte swizzle.  `lbo` in bytes.
+//   K-major  : rows of 128 B (64 x 16-bit along K); 8-row groups 1 KiB apart.
 //   MN-major : rows of 128 B (64 x 16-bit along M/N); 8 k-rows form a 1 KiB
-//              atom, atoms along K `sbo` apart, 64-wide M/N chunks `lbo` apart.
-__device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr, uint32_t lbo,
-                                                         uint32_t sbo) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((smem_addr >> 4) & 0x3fff);
-    d |= static_cast<uint64_t>((lbo >> 4) & 0x3fff) << 16;
-    d |= static_cast<uint64_t>((sbo >> 4) & 0x3fff) << 32;
-    d |= static_cast<uint64_t>(1) << 46;  // descriptor version (Blackwell)
-    d |= static_cast<uint64_t>(2) << 61;  // SWIZZLE_128B
-    return d;
-}
-// The same in parts, for issuing warps that have few cycles per product: the upper half is the same for every operand
-// with 1 KiB between its row groups, and the lower half moves on by bytes / 16.  `el`: nonzero in the lane that issues
-// (elect_one); the others pass by, so that the warp stays converged.
+//              atom, atoms along K 1 KiB apart, 64-wide M/N chunks `lbo` apart.
+// Its upper half is the same for every operand (groups 1 KiB apart, Blackwell's version, 128-byte swizzle), and its lower
+// half moves on by bytes / 16: an issuing warp has few cycles per product.
 constexpr uint32_t DESC_HI_SW128 = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t desc_lo_sw128(uint32_t smem_addr, uint32_t lbo) {
     return ((smem_addr >> 4) & 0x3fff) | ((lbo >> 4) << 16);
 }
+// D[tmem] (+)= A[smem desc] * B[smem desc], descriptors given by their lower halves.  `el`: nonzero in the lane that issues
+// (elect_one); the others pass by, so that the warp stays converged and operands in uniform registers.
 __device__ __forceinline__ void umma_f16_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate,
                                             uint32_t el) {
     asm volatile(
@@ -443,6 +394,7 @@ __device__ __forceinline__ void umma_f16_lo(uint32_t tmem_d, uint32_t a_lo, uint
           "l"(static_cast<uint64_t>(DESC_HI_SW128) << 32 | b_lo), "r"(idesc), "r"(accumulate), "r"(el)
         : "memory");
 }
+// D[tmem] (+)= A[tmem] * B[smem desc]
 __device__ __forceinline__ void umma_f16_ts_lo(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc,
                                                uint32_t accumulate, uint32_t el) {
     asm volatile(
@@ -457,7 +409,7 @@ __device__ __forceinline__ void umma_f16_ts_lo(uint32_t tmem_d, uint32_t tmem_a,
           "r"(el)
         : "memory");
 }
-// One thread of the pair's first CTA issues; each CTA supplies its 128 rows of A and its half of B from
+// One lane of the pair's first CTA issues; each CTA supplies its 128 rows of A and its half of B from
 // the same shared-memory offsets, and receives its 128 rows of D in its own tensor memory.
 __device__ __forceinline__ void umma_f16_pair_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
                                                  uint32_t accumulate, uint32_t el) {
