@@ -391,3 +391,55 @@ def test_kernels_in_a_row_wait_for_each_other(rows, S):
 
     for a, c in zip(run(True), run(False)):
         assert torch.equal(a, c)
+
+
+@pytest.mark.parametrize("how", ["captured", "two_streams"])
+def test_kernels_in_a_row_under_capture_and_across_streams(how):
+    """The order that a captured graph, or an event between two streams, asks for holds for kernels that begin early."""
+    from rannc_b200.ops import kernels as K
+    from rannc_b200.ops.gemm import gemm
+
+    torch.manual_seed(4)
+    dt, H, rows = torch.bfloat16, 512, 2048
+    w = (torch.randn(H, H, device="cuda") * H ** -0.5).to(dt)
+    g, b = torch.ones(H, device="cuda", dtype=dt), torch.zeros(H, device="cuda", dtype=dt)
+    x0 = torch.randn(rows, H, device="cuda").to(dt)
+    x, y = x0.clone(), torch.empty_like(x0)
+    other = torch.cuda.Stream()
+
+    def step(two):
+        """x = layer_norm(x w^T): the product on this stream, the norm on the other one when there are two."""
+        gemm(x, w, out=y)
+        here = torch.cuda.current_stream()
+        if two:
+            other.wait_stream(here)
+        with torch.cuda.stream(other if two else here):
+            z = K.ln_fwd(y, None, g, b, 1e-5)[0]
+            gemm(z, w, out=x)
+            z.record_stream(other)
+        if two:
+            here.wait_stream(other)
+
+    for _ in range(6):
+        step(False)
+        torch.cuda.synchronize()
+    want = x.clone()
+    x.copy_(x0)
+    torch.cuda.synchronize()
+    if how == "captured":
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            step(False)
+        torch.cuda.synchronize()
+        x.copy_(x0)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(3):
+                step(False)
+        for _ in range(2):
+            graph.replay()
+    else:
+        for _ in range(6):
+            step(True)
+    torch.cuda.synchronize()
+    assert torch.equal(x, want)
