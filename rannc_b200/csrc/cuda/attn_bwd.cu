@@ -221,13 +221,14 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
         const int t = threadIdx.x - (BWD_MATH + 64);
         const long long bh_row = (static_cast<long long>(b) * p.H + h) * p.S;
         float lse = 0.f, delta = 0.f;
-        auto fetch_stats = [&](int i) {   // (volatile: the loads are not sunk to their use)
+        auto fetch_stats = [&](int i) {   // (volatile: the loads are not sunk to their use.  Not the read-only path: the
+                                          // kernel before this one writes delta, and may still run when this one is resident)
             const int q = i * BQ + t;
             lse = INFINITY;
             delta = 0.f;
             if (q < p.S) {
-                asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(lse) : "l"(p.lse + bh_row + q));
-                asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(delta) : "l"(p.delta + bh_row + q));
+                asm volatile("ld.global.f32 %0, [%1];" : "=f"(lse) : "l"(p.lse + bh_row + q));
+                asm volatile("ld.global.f32 %0, [%1];" : "=f"(delta) : "l"(p.delta + bh_row + q));
             }
         };
         auto put_stats = [&](int i) {

@@ -8,8 +8,9 @@
 // Rules for a kernel that is launched this way:
 //  - every thread passes grid_wait() before its first access to global memory and before it ends.  (A kernel that ended
 //    without it could be complete before its predecessor, and the next one in the stream would wait for too little.)
-//  - what it reads is not declared const __restrict__: the compiler may move loads of memory that it takes to be constant
-//    for the kernel's lifetime across the wait.
+//  - what it reads is memory that changes while the kernel is resident, behind the wait too: it is not declared
+//    const __restrict__ (the compiler may move such loads across the wait) and not read by __ldg or ld.global.nc (the
+//    read-only path is not kept coherent during a kernel's life, whatever waits).
 // grid_trigger() allows the next kernel's blocks to start as soon as all blocks of this one have called it or ended; it has
 // no effect on what that kernel may read.  Behind any other kernel, copy or event the launch is an ordinary one.
 #pragma once
