@@ -45,7 +45,7 @@ constexpr int DQ_STAGE = 128 * 64 * 4;   // 32 KiB: [2 column halves][128 rows x
 constexpr int QD_STAGES = 3;             // Q / dO ring: block i + 2 is loaded while blocks i and i + 1 are in use
 constexpr int STATS = 3 * 128;           // (lse, delta, row hash) of a query block
 // K, V + (Q, dO) x 3 stages + dSt + dQ staging + row statistics of two blocks + barriers
-constexpr int BWD_SMEM = 2 * TILE + 2 * QD_STAGES * TILE + SQ_BYTES + DQ_STAGE + 2 * STATS * 4 + 128;
+constexpr int BWD_SMEM = 2 * TILE + 2 * QD_STAGES * TILE + SQ_BYTES + DQ_STAGE + 2 * STATS * 4 + 256;
 
 struct AttnBwdParams {
     int B, H, S;
@@ -83,12 +83,16 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
     uint64_t* s_free = bars + 5;
     uint64_t* pds_ready = bars + 6;
     uint64_t* ds_done = bars + 7;     // dK and dQ of the step are done: dSt may be overwritten, dQ drained
-    uint64_t* p_done = bars + 8;      // ... and dV: Pt, Q and dO may be
+    uint64_t* p_done = bars + 8;      // ... and dV: Pt may be
     uint64_t* dq_free = bars + 9;     // the previous bulk reduction has read the staging tile
     uint64_t* dq_ready = bars + 10;   // every drain thread has written its part of the staging tile
     uint64_t* dq_taken = bars + 11;   // dQ of the last step is out of tensor memory: the next may overwrite it
     uint64_t* stats_full = bars + 12;   // [2]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+    // [QD_STAGES] every product that reads the stage is done: it may be loaded again.  A barrier per stage, whose next phase
+    // cannot end before that load: p_done may be two blocks further by the time the loading warp looks, and a wait for a
+    // phase's parity would then wait for the block after, whose products wait for the loading warp.
+    uint64_t* qd_free = bars + 14;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14 + QD_STAGES);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     // (the same for all lanes, for the compiler too: what the issuing warps compute from it stays in uniform registers)
@@ -99,7 +103,10 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
     grid_trigger();
     if (threadIdx.x == 0) {
         mbar_init(kv_full, 1);
-        for (int st = 0; st < QD_STAGES; ++st) mbar_init(&qd_full[st], 1);
+        for (int st = 0; st < QD_STAGES; ++st) {
+            mbar_init(&qd_full[st], 1);
+            mbar_init(&qd_free[st], 1);
+        }
         mbar_init(s_full, 1);
         mbar_init(s_free, BWD_MATH);
         mbar_init(pds_ready, BWD_MATH);
@@ -146,8 +153,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
         }
         for (int i = 0; i < QD_STAGES && i < nq; ++i) load_qd(i, i);
         bool ok = mbar_wait_warp(kv_full, 0, abort_flag);
-        int st = 0, next = 2;   // stage of block i, and of block i + 2
-        uint32_t phase = 0;
+        int st = 0, next = 2;   // stage of block i, and of block i + 2 (which block i - 1 was in)
+        uint32_t phase = 0, free_phase = 1;   // (of block i - 1: it is 0 from block 1 on)
         for (int i = 0; i < nq && ok; ++i) {
             // S / dP of a block go to the tensor core as soon as the math warps have read the last block's: they run
             // behind that block's products, while its math is busy
@@ -164,10 +171,13 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
             if (el) umma_commit(s_full);
             // the stage block i - 1 used is free once its products are done: block i + 2 goes there
             if (i >= 1 && i + 2 < nq) {
-                if (!mbar_wait_warp(p_done, (i - 1) & 1, abort_flag)) break;
+                if (!mbar_wait_warp(&qd_free[next], free_phase, abort_flag)) break;
                 load_qd(i + 2, next);
             }
-            if (++next == QD_STAGES) next = 0;
+            if (++next == QD_STAGES) {
+                next = 0;
+                free_phase ^= 1;
+            }
             if (++st == QD_STAGES) {
                 st = 0;
                 phase ^= 1;
@@ -203,7 +213,10 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
 #pragma unroll
             for (int k = 0; k < 8; ++k)
                 umma_f16_ts_lo(tmem + C_DV, tmem + C_P + k * 8, da + k * 128, id_kn, (i | k) != 0, el);
-            if (el) umma_commit(p_done);
+            if (el) {
+                if (i + QD_STAGES < nq) umma_commit(&qd_free[st]);   // (someone waits for it, so it arrives while the block lives)
+                umma_commit(p_done);
+            }
             if (++st == QD_STAGES) {
                 st = 0;
                 phase ^= 1;

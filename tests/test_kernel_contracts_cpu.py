@@ -55,3 +55,134 @@ def test_what_a_kernel_that_begins_early_reads(file, kernel):
     assert not re.search(r"const\s+[\w:]+\s*\*\s*(?:const\s*)?__restrict__", params)
     for text in (body, _source(file), *(_source(h.name) for h in CUDA.glob("*.cuh"))):
         assert not re.search(r"ld\.global(\.\w+)*\.nc\b|\b__ldg\b", text)
+
+
+# ------------------------------------------------------------------------- barriers of the attention backward
+# The roles of one block run at any speed relative to each other.  Their loops over the query blocks are read from the
+# source as sequences of barrier operations, products and loads; the table says under which condition block i does one,
+# which barrier of an array it means and which phase of it.  A wait looks at a phase's parity alone: it is passed when the
+# number of phases that have ended is odd or even as it should be.
+STAGES = 3
+TOKEN = re.compile(r"mbar_(wait)(?:_warp)?\(&?(\w+)|mbar_(arrive)\(&?(\w+)|umma_(commit)\(&?(\w+)|"
+                   r"umma_f16\w*\(tmem \+ (C_)(\w+)|(load_qd|put_stats)\((i)")
+_always = lambda i, nq: True                       # noqa: E731
+_reload = lambda i, nq: i >= 1 and i + 2 < nq      # noqa: E731
+RULES = {   # (role, what, barrier): (condition, index in an array, phase that is waited for)
+    ("load", "wait", "qd_full"): (_always, lambda i: i % STAGES, lambda i: i // STAGES),
+    ("load", "wait", "s_free"): (lambda i, nq: i > 0, None, lambda i: i - 1),
+    ("load", "commit", "s_full"): (_always, None, None),
+    ("load", "wait", "p_done"): (_reload, None, lambda i: i - 1),
+    ("load", "wait", "qd_free"): (_reload, lambda i: (i + 2) % STAGES, lambda i: (i - 1) // STAGES),
+    ("load", "load_qd", "i"): (_reload, None, None),
+    ("grad", "wait", "qd_full"): (_always, lambda i: i % STAGES, lambda i: i // STAGES),
+    ("grad", "wait", "pds_ready"): (_always, None, lambda i: i),
+    ("grad", "wait", "dq_taken"): (lambda i, nq: i > 0, None, lambda i: i - 1),
+    ("grad", "commit", "ds_done"): (_always, None, None),
+    ("grad", "commit", "qd_free"): (lambda i, nq: i + STAGES < nq, lambda i: i % STAGES, None),
+    ("grad", "commit", "p_done"): (_always, None, None),
+    ("drain", "wait", "ds_done"): (_always, None, lambda i: i),
+    ("drain", "arrive", "dq_taken"): (_always, None, None),
+    ("drain", "put_stats", "i"): (lambda i, nq: i + 2 < nq, lambda i: i & 1, None),
+    ("drain", "arrive", "dq_free"): (_always, None, None),
+    ("drain", "wait", "dq_free"): (_always, None, lambda i: i),
+    ("drain", "arrive", "dq_ready"): (_always, None, None),
+    ("drain", "wait", "dq_ready"): (_always, None, lambda i: i),
+    ("math", "wait", "stats_full"): (_always, lambda i: i & 1, lambda i: i >> 1),
+    ("math", "wait", "s_full"): (_always, None, lambda i: i),
+    ("math", "arrive", "s_free"): (_always, None, None),
+    ("math", "wait", "ds_done"): (lambda i, nq: i > 0, None, lambda i: i - 1),
+    ("math", "wait", "p_done"): (lambda i, nq: i > 0, None, lambda i: i - 1),
+    ("math", "arrive", "pds_ready"): (_always, None, None),
+}
+
+
+def _bwd_roles():
+    """{role: [(what, barrier)]} of the loops over the query blocks."""
+    body = _kernels("attn_bwd.cu")["attn_bwd_kernel"][1]
+    start = body.index("if (warp == LOAD_WARP) {", body.index("grid_wait()"))
+    out = {}
+    for role in ("load", "grad", "drain", "math"):
+        open_ = body.index("{", start)
+        section = body[open_:_closing(body, open_)]
+        start = open_ + len(section)
+        loops = [m for m in re.finditer(r"for \(int i = 0; i < nq[^)]*\)\s*{", section)]
+        assert len(loops) == 1, role
+        loop = section[loops[0].start():_closing(section, loops[0].end() - 1)]
+        out[role] = [tuple(x for x in m.groups() if x) for m in TOKEN.finditer(loop)]
+    return out
+
+
+def _programs(nq):
+    """{actor: [step]}; products and the commits behind them are steps of a queue that the tensor core works off."""
+    progs = {a: [] for a in ("load", "grad", "drain", "math", "load queue", "grad queue")}
+    progs["load"] += [("put", i % STAGES, i) for i in range(min(STAGES, nq))]
+    progs["drain"] += [("arrive", ("stats_full", i & 1)) for i in range(min(2, nq))]
+    for role, tokens in _bwd_roles().items():
+        for i in range(nq):
+            for what, name in tokens:
+                if what == "C_":
+                    progs[role + " queue"].append(("read", None if name == "DQ" else (i % STAGES, i), len(progs[role])))
+                    continue
+                when, index, phase = RULES[role, what, name]
+                if not when(i, nq):
+                    continue
+                bar = (name, index(i) if index else 0)
+                if what == "wait":
+                    progs[role].append(("wait", bar, phase(i)))
+                elif what == "commit":
+                    progs[role + " queue"].append(("arrive", bar, len(progs[role])))
+                elif what == "load_qd":
+                    progs[role].append(("put", (i + 2) % STAGES, i + 2))
+                else:
+                    progs[role].append(("arrive", ("stats_full", i & 1) if what == "put_stats" else bar))
+    return progs
+
+
+@pytest.mark.parametrize("nq", [1, 2, 3, 4, 5, 7])
+def test_attention_backward_roles_at_any_speed(nq):
+    progs = _programs(nq)
+    actors = list(progs)
+    # how often each barrier has ended a phase, and what each stage holds, by the position of an actor
+    arrived = {a: [{}] for a in actors}
+    held = [{}]
+    for a in actors:
+        for step in progs[a]:
+            count = dict(arrived[a][-1])
+            if step[0] == "arrive":
+                count[step[1]] = count.get(step[1], 0) + 1
+            if step[0] == "put":
+                held.append({**held[-1], step[1]: step[2]})
+                count["qd_full", step[1]] = count.get(("qd_full", step[1]), 0) + 1
+            elif a == "load":
+                held.append(held[-1])
+            arrived[a].append(count)
+
+    def ended(bar, at):
+        return sum(arrived[a][pc].get(bar, 0) for a, pc in zip(actors, at))
+
+    seen, todo = set(), [(0,) * len(actors)]
+    while todo:
+        at = todo.pop()
+        if at in seen:
+            continue
+        seen.add(at)
+        moves = 0
+        for k, a in enumerate(actors):
+            if at[k] == len(progs[a]):
+                continue
+            step = progs[a][at[k]]
+            if step[0] == "wait":
+                n = ended(step[1], at)
+                if (n - step[2]) % 2 == 0:
+                    continue
+                assert n == step[2] + 1, f"{a} passes {step} with {n} phases ended"
+            elif a.endswith("queue"):
+                if at[actors.index(a.split()[0])] < step[2]:
+                    continue   # not issued yet
+                if step[0] == "read" and step[1]:
+                    assert held[at[actors.index("load")]].get(step[1][0]) == step[1][1], f"{step} reads another block"
+            moves += 1
+            todo.append(at[:k] + (at[k] + 1,) + at[k + 1:])
+        assert moves or all(pc == len(progs[a]) for a, pc in zip(actors, at)), \
+            "stuck before " + ", ".join(str(progs[a][pc]) for a, pc in zip(actors, at) if pc < len(progs[a]))
+    assert len(seen) > nq
