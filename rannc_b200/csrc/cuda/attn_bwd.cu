@@ -100,7 +100,6 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
     const int key0 = blockIdx.x * BKEYS, h = blockIdx.y, b = blockIdx.z;
     const int nq = (p.S + BQ - 1) / BQ;
 
-    grid_trigger();
     if (threadIdx.x == 0) {
         mbar_init(kv_full, 1);
         for (int st = 0; st < QD_STAGES; ++st) {
@@ -127,6 +126,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    grid_trigger();
     grid_wait();   // all of the above runs beside the end of the kernel before
     constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
 

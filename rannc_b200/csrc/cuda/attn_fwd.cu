@@ -114,7 +114,6 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
     const int nchunks = (p.S + AK - 1) / AK;
     const int ntiles = (q_base + AQ < p.S) ? 2 : 1;
 
-    grid_trigger();
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
         for (int i = 0; i < 2; ++i) {
@@ -151,6 +150,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
     const bool has_bias = __syncthreads_or(any_bias) != 0 || !(p.scale_log2 > 0.f);
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    grid_trigger();
     constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
 
     if (warp == 18) {
@@ -499,7 +499,6 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
     const int my_items = blockIdx.x < nitems ? (nitems - 1 - blockIdx.x) / gridDim.x + 1 : 0;
     const int total_chunks = my_items * nchunks;
 
-    grid_trigger();
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) {
             mbar_init(&q_full[i], 1);
@@ -525,6 +524,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    grid_trigger();
     grid_wait();   // all of the above runs beside the end of the kernel before
     constexpr int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
     auto decode = [&](int item, int& b, int& h, int& q_base) {

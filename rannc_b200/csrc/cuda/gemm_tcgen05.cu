@@ -240,7 +240,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     const int tile0 = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
     const int tile_step = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
-    grid_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full[s], 1);
@@ -275,6 +274,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     if (PAIR) cluster_sync_all();   // the peer's barriers exist before anything signals them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    grid_trigger();
     grid_wait();   // all of the above runs beside the end of the kernel before
 
     if (warp == 0) {

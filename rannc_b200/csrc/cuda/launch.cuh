@@ -11,6 +11,9 @@
 //  - what it reads is memory that changes while the kernel is resident, behind the wait too: it is not declared
 //    const __restrict__ (the compiler may move such loads across the wait) and not read by __ldg or ld.global.nc (the
 //    read-only path is not kept coherent during a kernel's life, whatever waits).
+//  - a kernel that takes tensor memory calls grid_trigger() behind the barrier that follows the allocation.  (Blocks of the
+//    next kernel take theirs before they wait: one that came to an SM first would wait there for this kernel's end, and
+//    this kernel's block for its columns, without a limit.  With all of this kernel's blocks served, none can.)
 // grid_trigger() allows the next kernel's blocks to start as soon as all blocks of this one have called it or ended; it has
 // no effect on what that kernel may read.  Behind any other kernel, copy or event the launch is an ordinary one.
 #pragma once

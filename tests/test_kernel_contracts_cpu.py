@@ -57,6 +57,15 @@ def test_what_a_kernel_that_begins_early_reads(file, kernel):
         assert not re.search(r"ld\.global(\.\w+)*\.nc\b|\b__ldg\b", text)
 
 
+@pytest.mark.parametrize("file,kernel", [(f, k) for f, k in EARLY if "tmem_alloc" in _kernels(f)[k][1]])
+def test_tensor_memory_is_taken_before_the_next_kernel_may_begin(file, kernel):
+    body = _kernels(file)[kernel][1]
+    taken = max(m.end() for m in re.finditer(r"tmem_alloc\w*\(", body))
+    trigger = [m.start() for m in re.finditer(r"grid_trigger\(\)", body)]
+    assert len(trigger) == 1 and trigger[0] > taken
+    assert "__syncthreads" in body[taken:trigger[0]]
+
+
 # ------------------------------------------------------------------------- barriers of the attention backward
 # The roles of one block run at any speed relative to each other.  Their loops over the query blocks are read from the
 # source as sequences of barrier operations, products and loads; the table says under which condition block i does one,
