@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
         }
         for (int i = 0; i < nq; ++i) {
             if (i + 2 < nq) fetch_stats(i + 2);
-            if (!mbar_wait(ds_done, i & 1, abort_flag)) break;
+            if (!mbar_wait_warp(ds_done, i & 1, abort_flag)) break;
             tc_fence_after();
             uint32_t v0[32], v1[32];
             tmem_ld32(tmem + lane_addr + C_DQ, v0);
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
                 tma_store_wait_read<0>();   // the previous reduction no longer reads the staging tile
                 mbar_arrive(dq_free);
             }
-            if (!mbar_wait(dq_free, i & 1, abort_flag)) break;
+            if (!mbar_wait_warp(dq_free, i & 1, abort_flag)) break;
             uint8_t* row = sDQ + (r >> 3) * 1024 + sw * 128;
 #pragma unroll
             for (int g = 0; g < 8; ++g) {
@@ -285,11 +285,13 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
             }
             fence_proxy_async();
             mbar_arrive(dq_ready);
-            if (issuer) {
-                if (!mbar_wait(dq_ready, i & 1, abort_flag)) break;
-                tma_reduce_add_4d(&tmDQ, sDQ, 0, i * BQ, h, b);
-                tma_reduce_add_4d(&tmDQ, sDQ + DQ_STAGE / 2, 32, i * BQ, h, b);
-                tma_store_commit();
+            if (warp == GRAD_WARP + 1) {
+                if (!mbar_wait_warp(dq_ready, i & 1, abort_flag)) break;
+                if (issuer) {
+                    tma_reduce_add_4d(&tmDQ, sDQ, 0, i * BQ, h, b);
+                    tma_reduce_add_4d(&tmDQ, sDQ + DQ_STAGE / 2, 32, i * BQ, h, b);
+                    tma_store_commit();
+                }
             }
         }
         // the staging tile must outlive the copies that read it; their sums are complete when the kernel is
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
         bool ok = true;
 
         for (int i = 0; i < nq; ++i) {
-            if (!mbar_wait(&stats_full[i & 1], (i >> 1) & 1, abort_flag) || !mbar_wait(s_full, i & 1, abort_flag)) {
+            if (!mbar_wait_warp(&stats_full[i & 1], (i >> 1) & 1, abort_flag) || !mbar_wait_warp(s_full, i & 1, abort_flag)) {
                 ok = false;
                 break;
             }
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
                 }
             }
             // the previous step's products read dSt and Pt: wait, then overwrite
-            if (i > 0 && !mbar_wait(ds_done, (i - 1) & 1, abort_flag)) {
+            if (i > 0 && !mbar_wait_warp(ds_done, (i - 1) & 1, abort_flag)) {
                 ok = false;
                 break;
             }
@@ -387,7 +389,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
                 *reinterpret_cast<uint4*>(drow + ((static_cast<uint32_t>((part & 1) * 4 + g) ^ sw) << 4)) =
                     make_uint4(dk[g * 4], dk[g * 4 + 1], dk[g * 4 + 2], dk[g * 4 + 3]);
             fence_proxy_async();
-            if (i > 0 && !mbar_wait(p_done, (i - 1) & 1, abort_flag)) {
+            if (i > 0 && !mbar_wait_warp(p_done, (i - 1) & 1, abort_flag)) {
                 ok = false;
                 break;
             }
@@ -400,7 +402,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
         // dK and dV: rows leave by way of the Q ring, which every product is done with, in pieces of 64 bytes that four
         // lanes write together (a thread that stored its own row touched a line with every 16 bytes: 2800 cycles of a
         // CTA's 24500 at S = 512)
-        if (ok && mbar_wait(p_done, (nq - 1) & 1, abort_flag)) {
+        if (ok && mbar_wait_warp(p_done, (nq - 1) & 1, abort_flag)) {
             tc_fence_after();
             const int half = part & 1;
             const bool is_k = part >> 1;

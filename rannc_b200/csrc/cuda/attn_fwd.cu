@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
         for (int j = 0; j < nchunks; ++j) {
             // after a failed wait the loop keeps running (every later wait fails at once) so that the pair of
             // threads sharing a row still meets at the named barrier below
-            if (!mbar_wait(&s_full[t], j & 1, abort_flag)) {
+            if (!mbar_wait_warp(&s_full[t], j & 1, abort_flag)) {
                 ok = false;
             }
             tc_fence_after();
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
             const float alpha = exp2f(m - m_use);
             // the previous P V product must be complete before P is overwritten and O rescaled
             if (j > 0) {
-                if (!mbar_wait(&o_done[t], (j - 1) & 1, abort_flag)) {
+                if (!mbar_wait_warp(&o_done[t], (j - 1) & 1, abort_flag)) {
                     ok = false;
                     break;
                 }
@@ -413,17 +413,18 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
             tc_fence_before();
             mbar_arrive(&p_ready[t]);
         }
-        if (ok && mbar_wait(&o_done[t], (nchunks - 1) & 1, abort_flag)) {
-            tc_fence_after();
-            // the pair's partial row sums
-            float* xch = xbase + (nchunks & 1) * 256;
-            xch[half * 128 + r] = l;
-            bar_sync_named(1 + t, GROUP);
-            l += xch[(half ^ 1) * 128 + r];
-            const float inv_l = l > 0.f ? p.inv_keep / l : 0.f;
-            uint32_t v[32];
-            tmem_ld32(col_o + lane_addr + half * 32, v);
-            tmem_ld_wait();
+        if (!mbar_wait_warp(&o_done[t], (nchunks - 1) & 1, abort_flag)) ok = false;
+        tc_fence_after();
+        // the pair's partial row sums
+        float* xch = xbase + (nchunks & 1) * 256;
+        xch[half * 128 + r] = l;
+        bar_sync_named(1 + t, GROUP);
+        l += xch[(half ^ 1) * 128 + r];
+        const float inv_l = l > 0.f ? p.inv_keep / l : 0.f;
+        uint32_t v[32];
+        tmem_ld32(col_o + lane_addr + half * 32, v);
+        tmem_ld_wait();
+        if (ok) {
             store_o_rows<T>(v, inv_l, sP + t * P_BYTES + half * (P_BYTES / 2) + (r >> 5) * 4096, lane,
                             reinterpret_cast<T*>(p.O) + b * p.o_sb + h * p.o_sh + half * 32, p.o_ss, q - lane, p.S);
             if (half == 0 && q < p.S)
@@ -544,7 +545,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
             int b, h, q_base;
             decode(item, b, h, q_base);
             // the buffer's previous item (k - 2) must be finished by every softmax thread
-            if (k >= 2 && !mbar_wait(&item_done[buf], ((k >> 1) - 1) & 1, abort_flag)) ok = false;
+            if (k >= 2 && !mbar_wait_warp(&item_done[buf], ((k >> 1) - 1) & 1, abort_flag)) ok = false;
             const float* kb = p.key_bias ? p.key_bias + static_cast<long long>(b) * p.S : nullptr;
             int any = 0;
             for (int i = lane; i < p.S; i += 32) {
@@ -562,7 +563,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
             }
             for (int j = 0; j < nchunks; ++j) {
                 const int c = k * nchunks + j, st = c & 1;
-                if (c >= 2 && !mbar_wait(&kv_free[st], ((c >> 1) - 1) & 1, abort_flag)) ok = false;
+                if (c >= 2 && !mbar_wait_warp(&kv_free[st], ((c >> 1) - 1) & 1, abort_flag)) ok = false;
                 if (lane == 0 && ok) {
                     mbar_arrive_expect_tx(&k_full[st], TILE_B);
                     tma_load_4d(sK + st * TILE_B, &tmK, &k_full[st], 0, j * AK, h, b);
@@ -648,13 +649,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
             const int q = q_base + t * AQ + r;
             const uint32_t row_hash = drop_row_hash(p.seed, b, h, q, p.H, p.S);
             // the item's key-bias table (and Q) have landed
-            if (!mbar_wait(&q_full[buf], (k >> 1) & 1, abort_flag)) ok = false;
+            if (!mbar_wait_warp(&q_full[buf], (k >> 1) & 1, abort_flag)) ok = false;
             const bool has_bias = s_flag[buf] != 0 || !(p.scale_log2 > 0.f);
             const float* kbt = s_kb + buf * KB_MAX;
             float m = -INFINITY, l = 0.f;
             for (int j = 0; j < nchunks; ++j) {
                 const int c = k * nchunks + j;
-                if (!mbar_wait(&s_full[t], c & 1, abort_flag)) ok = false;
+                if (!mbar_wait_warp(&s_full[t], c & 1, abort_flag)) ok = false;
                 tc_fence_after();
                 const int key0 = j * AK + half * 64;
                 float cm = -INFINITY;
@@ -705,7 +706,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
                     m_use = m_new == -INFINITY ? 0.f : m_new;
                 const float alpha = exp2f(m - m_use);
                 if (j > 0) {
-                    if (!mbar_wait(&o_done[t], (c - 1) & 1, abort_flag)) ok = false;
+                    if (!mbar_wait_warp(&o_done[t], (c - 1) & 1, abort_flag)) ok = false;
                     tc_fence_after();
                     if (__any_sync(0xffffffffu, alpha != 1.f)) {
                         uint32_t v[32];
@@ -787,7 +788,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
             }
             // ---- the item's output: wait for its last product, take O out of tensor memory, release it
             const int c_last = k * nchunks + nchunks - 1;
-            if (!mbar_wait(&o_done[t], c_last & 1, abort_flag)) ok = false;
+            if (!mbar_wait_warp(&o_done[t], c_last & 1, abort_flag)) ok = false;
             tc_fence_after();
             float* xch = xbase + 2 * 256;
             xch[half * 128 + r] = l;

@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                 for (int j = 0; j < 8; ++j) s[j] = 0.f;
                 bool any = false;
                 for (int kb = kb_begin; kb < kb_end; ++kb) {
-                    if (!mbar_wait(&used[stage], phase, abort_flag)) {
+                    if (!mbar_wait_warp(&used[stage], phase, abort_flag)) {
                         ok = false;
                         break;
                     }
@@ -630,7 +630,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     tma_load_3d(stage_buf, &tmAux, abar, col0 + c * 32, row0, b);
                 };
                 if (act_dgelu && nblk > 0 && lane == 0) fetch_aux(0);
-                if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) break;
+                if (!mbar_wait_warp(&tfull[acc], acc_phase, abort_flag)) break;
                 tc_fence_after();
                 if (nblk == 0) release_acc(acc);
                 const long long row_off = static_cast<long long>(b) * p.strideD +
@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         for (int j = 0; j < 32; j += 2) gelu_erf2(v[j], v[j + 1]);
                     }
                     if (act_dgelu) {
-                        if (!mbar_wait(abar, aux_phase, abort_flag)) {
+                        if (!mbar_wait_warp(abar, aux_phase, abort_flag)) {
                             ok = false;
                             break;
                         }
@@ -755,7 +755,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             const int acc = it & 1;
             const uint32_t acc_phase = (it >> 1) & 1;
             ++it;
-            if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) break;
+            if (!mbar_wait_warp(&tfull[acc], acc_phase, abort_flag)) break;
             tc_fence_after();
             int row = mb * TILE_M + static_cast<int>(crank) * BM + row_in_tile;
             bool row_ok = row < p.M;

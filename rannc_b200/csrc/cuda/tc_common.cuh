@@ -122,7 +122,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
     return false;
 }
 
-// The same for a whole converged warp: one answer for all lanes
+// The same for a whole converged warp: one answer for all lanes.  Every wait of a warp that goes on to collective instructions
+// (tensor-memory copies, __syncwarp, shuffles, named barriers) is of this kind: lanes that disagree about a wait whose limit
+// ran out would not meet again there, and the block would hang instead of reporting.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }

@@ -66,6 +66,25 @@ def test_tensor_memory_is_taken_before_the_next_kernel_may_begin(file, kernel):
     assert "__syncthreads" in body[taken:trigger[0]]
 
 
+@pytest.mark.parametrize("file,kernel", [(f, k) for f, k in EARLY if "abort_flag" in _kernels(f)[k][1]])
+def test_lanes_of_a_warp_agree_about_a_wait(file, kernel):
+    """A wait whose limit runs out ends the work of a whole warp: lanes that went different ways would not meet again at
+    the next collective instruction.  Only a role that one lane plays by itself waits by itself."""
+    body = _kernels(file)[kernel][1]
+    alone = [(m.end() - 1, _closing(body, m.end() - 1)) for m in re.finditer(r"if \(lane == 0\) {", body)]
+    for m in re.finditer(r"\bmbar_wait\(", body):
+        inside = [body[a:b] for a, b in alone if a < m.start() < b]
+        assert inside and not re.search(r"__sync|_sync\(|tmem_|bar_sync|mbar_wait_warp", inside[0])
+    # nor does one lane leave a loop that its warp goes through together
+    for m in re.finditer(r"if \(issuer\) {", body):
+        assert "break" not in body[m.start():_closing(body, m.end() - 1)]
+    # a barrier of several warps does not hang on what one of them found
+    for m in re.finditer(r"bar_sync_named\(|bar\.sync", body):
+        enclosing = [c for c in re.finditer(r"if \(([^{};]*)\) {", body[:m.start()])
+                     if _closing(body, c.end() - 1) > m.start()]
+        assert not any(re.search(r"\bok\b|mbar_wait", c.group(1)) for c in enclosing)
+
+
 # ------------------------------------------------------------------------- barriers of the attention backward
 # The roles of one block run at any speed relative to each other.  Their loops over the query blocks are read from the
 # source as sequences of barrier operations, products and loads; the table says under which condition block i does one,
