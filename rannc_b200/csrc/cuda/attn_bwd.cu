@@ -533,9 +533,10 @@ static int launch_bwd(const RbAttnArgs& a, cudaStream_t st) {
     if ((rc = make_tmap_4d(&tdo, a.dO, a.dtype, D, S, H, B, a.do_ss * 2, a.do_sh * 2, a.do_sb * 2, 64, 128))) return rc;
     const long long rows = static_cast<long long>(a.B) * a.H * a.S;
     if (rows >= (1LL << 31) - 64) return -2;
-    launch_after(attn_delta_kernel<T>, static_cast<unsigned>((rows + 63) / 64), 256, 0, st,
-        static_cast<const T*>(a.O), static_cast<const T*>(a.dO), a.delta, a.dq_accum, a.B, a.H, a.S, a.o_sb,
-        a.o_ss, a.o_sh, a.do_sb, a.do_ss, a.do_sh);
+    if (launch_after(attn_delta_kernel<T>, static_cast<unsigned>((rows + 63) / 64), 256, 0, st, static_cast<const T*>(a.O),
+                     static_cast<const T*>(a.dO), a.delta, a.dq_accum, a.B, a.H, a.S, a.o_sb, a.o_ss, a.o_sh, a.do_sb,
+                     a.do_ss, a.do_sh) != cudaSuccess)
+        return -1;
     AttnBwdParams p;
     p.B = a.B; p.H = a.H; p.S = a.S;
     p.scale = a.scale;
@@ -564,11 +565,13 @@ static int launch_bwd(const RbAttnArgs& a, cudaStream_t st) {
     dim3 grid((a.S + BKEYS - 1) / BKEYS, a.H, a.B);
     CUtensorMap tdq;
     if ((rc = make_tmap_4d_f32(&tdq, a.dq_accum, 64, S, H, B, H * 64 * 4, 64 * 4, S * H * 64 * 4, 32, 128))) return rc;
-    launch_after(kern, grid, BWD_THREADS, BWD_SMEM, st, tq, tk, tv, tdo, tdq, p);
+    if (launch_after(kern, grid, BWD_THREADS, BWD_SMEM, st, tq, tk, tv, tdo, tdq, p) != cudaSuccess) return -1;
     const long long groups = rows * 8;
-    launch_after(attn_dq_convert_kernel<T>, static_cast<unsigned>((groups + 255) / 256), 256, 0, st,
-        static_cast<const float*>(a.dq_accum), static_cast<T*>(a.dQ), a.B, a.H, a.S, a.dq_sb, a.dq_ss, a.dq_sh);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_after(attn_dq_convert_kernel<T>, static_cast<unsigned>((groups + 255) / 256), 256, 0, st,
+                        static_cast<const float*>(a.dq_accum), static_cast<T*>(a.dQ), a.B, a.H, a.S, a.dq_sb, a.dq_ss,
+                        a.dq_sh) == cudaSuccess
+               ? 0
+               : -1;
 }
 
 }  // namespace rb

@@ -873,8 +873,7 @@ static int launch_fwd(const RbAttnArgs& a, cudaStream_t st) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pdev);
         if (sms <= 0) sms = 148;
         const int grid = nitems < sms ? static_cast<int>(nitems) : sms;
-        launch_after(pk, grid, ATT_THREADS, ATTP_SMEM, st, tq, tk, tv, p, static_cast<int>(nitems));
-        return cudaGetLastError() == cudaSuccess ? 0 : -1;
+        return launch_after(pk, grid, ATT_THREADS, ATTP_SMEM, st, tq, tk, tv, p, static_cast<int>(nitems)) == cudaSuccess ? 0 : -1;
     }
     const bool fast = (a.S + AK - 1) / AK * AK <= KB_MAX;
     auto kern = fast ? attn_fwd_kernel<T, true> : attn_fwd_kernel<T, false>;
@@ -887,8 +886,7 @@ static int launch_fwd(const RbAttnArgs& a, cudaStream_t st) {
         attr_set[dev & 63][fast] = true;
     }
     dim3 grid((a.S + 2 * AQ - 1) / (2 * AQ), a.H, a.B);
-    launch_after(kern, grid, ATT_THREADS, ATT_SMEM, st, tq, tk, tv, p);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_after(kern, grid, ATT_THREADS, ATT_SMEM, st, tq, tk, tv, p) == cudaSuccess ? 0 : -1;
 }
 
 }  // namespace rb

@@ -1047,18 +1047,18 @@ static int launch(const RbGemmArgs& a, const CUtensorMap& tmA, const CUtensorMap
         return e == cudaSuccess ? 0 : -static_cast<int>(e);
     }
     // one cluster of two CTAs per TPC; persistent over the pair tiles
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     if (!max_clusters[dev & 63]) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
         cfg.gridDim = dim3(num_sms(), 1, 1);
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) n = num_sms() / 2;
@@ -1066,11 +1066,7 @@ static int launch(const RbGemmArgs& a, const CUtensorMap& tmA, const CUtensorMap
     }
     int clusters = p.num_tiles < max_clusters[dev & 63] ? p.num_tiles : max_clusters[dev & 63];
     if (a.max_ctas > 1 && clusters > a.max_ctas / 2) clusters = a.max_ctas / 2;
-    cfg.gridDim = dim3(2 * clusters, 1, 1);
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // (see launch_after)
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.numAttrs = 2;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmD, tmAux, p);
+    const cudaError_t e = launch_after_clusters(kern, 2, 2 * clusters, GEMM_THREADS, smem, stream, tmA, tmB, tmD, tmAux, p);
     return e == cudaSuccess ? 0 : -static_cast<int>(e);
 }
 

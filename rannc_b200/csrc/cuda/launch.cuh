@@ -26,19 +26,33 @@ namespace rb {
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// `cluster`: blocks of a cluster (0: none).  A failed launch is reported by the result alone: the runtime's last error is
+// taken back, or the next check of another launch would report it again.
 template <typename... P, typename... A>
-inline cudaError_t launch_after(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+[[nodiscard]] inline cudaError_t launch_after_clusters(void (*kern)(P...), unsigned cluster, dim3 grid, dim3 block, size_t smem,
+                                                       cudaStream_t stream, A&&... args) {
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+    cfg.numAttrs = cluster ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+template <typename... P, typename... A>
+[[nodiscard]] inline cudaError_t launch_after(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                              A&&... args) {
+    return launch_after_clusters(kern, 0, grid, block, smem, stream, std::forward<A>(args)...);
 }
 
 }  // namespace rb

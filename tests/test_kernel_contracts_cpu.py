@@ -1,6 +1,8 @@
 """What kernels that begin beside the end of the one before them (csrc/cuda/launch.cuh) have to keep to, checked in the
 sources: the faults it prevents come from rare timing, which no run on a GPU shows."""
 import re
+import shutil
+import subprocess
 from pathlib import Path
 
 import pytest
@@ -43,7 +45,7 @@ def test_every_kernel_that_begins_early_waits():
     names = {k for _, k in EARLY}
     assert {"gemm_tcgen05_kernel", "attn_fwd_kernel", "attn_fwd_persist_kernel", "attn_bwd_kernel", "ln_fwd_kernel"} <= names
     # a launch names the kernel, or a variable that was set to it
-    for m in re.finditer(r"launch_after\w*\(\s*(?:\w+,\s*)?(\w+)", text):
+    for m in re.finditer(r"launch_after\w*\(\s*(\w+)", text):
         arg = m.group(1)
         sets = set(re.findall(rf"auto {arg}\s*=\s*([^;]+);", text)) or {arg}
         assert all(set(re.findall(r"\w+_kernel", s)) <= names for s in sets), arg
@@ -83,6 +85,65 @@ def test_lanes_of_a_warp_agree_about_a_wait(file, kernel):
         enclosing = [c for c in re.finditer(r"if \(([^{};]*)\) {", body[:m.start()])
                      if _closing(body, c.end() - 1) > m.start()]
         assert not any(re.search(r"\bok\b|mbar_wait", c.group(1)) for c in enclosing)
+
+
+
+FAKE_RUNTIME = r"""
+#pragma once
+#include <cstddef>
+#define __device__
+#define __forceinline__ inline
+typedef int cudaError_t;
+typedef void* cudaStream_t;
+constexpr cudaError_t cudaSuccess = 0;
+struct dim3 { unsigned x, y, z; dim3(unsigned a = 1, unsigned b = 1, unsigned c = 1) : x(a), y(b), z(c) {} };
+enum { cudaLaunchAttributeProgrammaticStreamSerialization, cudaLaunchAttributeClusterDimension };
+struct cudaLaunchAttribute {
+    int id;
+    struct { int programmaticStreamSerializationAllowed; struct { unsigned x, y, z; } clusterDim; } val;
+};
+struct cudaLaunchConfig_t {
+    dim3 gridDim, blockDim; size_t dynamicSmemBytes; cudaStream_t stream; cudaLaunchAttribute* attrs; unsigned numAttrs;
+};
+inline cudaError_t last = 0, next = 0;
+inline unsigned clusters = 0;
+inline cudaError_t cudaGetLastError() { const cudaError_t e = last; last = 0; return e; }
+template <typename... P, typename... A>
+cudaError_t cudaLaunchKernelEx(const cudaLaunchConfig_t* c, void (*)(P...), A&&...) {
+    clusters = 0;
+    for (unsigned i = 0; i < c->numAttrs; ++i)
+        if (c->attrs[i].id == cudaLaunchAttributeClusterDimension) clusters = c->attrs[i].val.clusterDim.x;
+    if (next) last = next;
+    return next;
+}
+"""
+LAUNCHES = r"""
+#include "launch.cuh"
+void kernel(int) {}
+int main() {
+    next = 9;   // a launch that fails is reported once
+    if (rb::launch_after(kernel, 1, 32, 0, nullptr, 1) != 9 || clusters != 0 || last != 0) return 1;
+    if (rb::launch_after_clusters(kernel, 2, 2, 32, 0, nullptr, 1) != 9 || clusters != 2 || last != 0) return 2;
+    next = 0, last = 7;   // what somebody else left is theirs to find
+    if (rb::launch_after(kernel, 1, 32, 0, nullptr, 1) != 0 || last != 7) return 3;
+    return 0;
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="no C++ compiler")
+def test_a_failed_launch_is_reported_once(tmp_path):
+    (tmp_path / "cuda_runtime.h").write_text(FAKE_RUNTIME)
+    (tmp_path / "launches.cpp").write_text(LAUNCHES)
+    exe = str(tmp_path / "launches")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(tmp_path), "-I", str(CUDA), str(tmp_path / "launches.cpp"), "-o",
+                    exe], check=True)
+    assert subprocess.run([exe]).returncode == 0
+    # every result is looked at, and launches with these attributes go through these functions
+    for f in sorted(CUDA.glob("*.cu")):
+        text = _source(f.name)
+        assert all(text[:m.start()].rstrip()[-1] not in ";{}" for m in re.finditer(r"\blaunch_after\w*\(", text)), f.name
+        assert "cudaLaunchKernelEx" not in text, f.name
 
 
 # ------------------------------------------------------------------------- barriers of the attention backward
