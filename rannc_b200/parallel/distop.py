@@ -185,6 +185,7 @@ def _gemm_rs(dy2, x2, N, Kfull, grad_ptrs, Ks, alpha):
     M = ar
     args = _Args(_lib.ptr(a), _lib.ptr(b), grad_ptrs[0], None, None, None, None, N, Kfull, M, 1, lda, ldb, Ks, 0, 0,
                  0, 1, 1, _dt(a), 1, ACCUM, 0, float(alpha), 0)
+    args.in_order = int(torch.are_deterministic_algorithms_enabled())
     if len(grad_ptrs) > 1:
         args.rs_nranks = len(grad_ptrs)
         for i, p in enumerate(grad_ptrs):

@@ -275,3 +275,33 @@ def test_attention_backward_roles_at_any_speed(nq):
         assert moves or all(pc == len(progs[a]) for a, pc in zip(actors, at)), \
             "stuck before " + ", ".join(str(progs[a][pc]) for a, pc in zip(actors, at) if pc < len(progs[a]))
     assert len(seen) > nq
+
+
+# ------------------------------------------------------------------------- what a product is asked for
+@pytest.mark.parametrize("deterministic", [False, True])
+def test_partitioned_weight_gradient_passes_the_order_on(deterministic, monkeypatch):
+    """A tensor-partitioned linear's weight gradient asks for tiles that are summed whole under
+    torch.use_deterministic_algorithms, like every other product."""
+    import torch
+
+    from rannc_b200.ops import _lib
+    from rannc_b200.parallel import distop
+
+    seen = []
+
+    class Fake:
+        @staticmethod
+        def rb_gemm(args, stream):
+            seen.append(args._obj.in_order)
+            return 0
+
+    monkeypatch.setattr(_lib, "lib", lambda: Fake)
+    monkeypatch.setattr(_lib, "stream_ptr", lambda: None)
+    before = torch.are_deterministic_algorithms_enabled()
+    torch.use_deterministic_algorithms(deterministic)
+    try:
+        distop._gemm_rs(torch.zeros(16, 8, dtype=torch.bfloat16), torch.zeros(16, 8, dtype=torch.bfloat16), 8, 8, [4096], 8,
+                        1.0)
+    finally:
+        torch.use_deterministic_algorithms(before)
+    assert seen == [int(deterministic)]
