@@ -1114,18 +1114,33 @@ struct Tiling {
 };
 // The tiles that do not fill the last wave of the CTA pairs, of a product that is added to an fp32 matrix: K is shared out
 // so that every pair has something to do.
-//  - Fewer tiles than half the pairs (36 of 74): K in `split` equal parts, one wave of them.
+//  - No more tiles than half the pairs (37 of 74): K in `split` equal parts, one wave of them.
 //  - More: each tile's pair takes the first `kb` steps, all in step, so that operands are shared through L2; the pairs left
-//    over take the remaining steps of one tile after another.
-// 30528 x 1024 (480 tiles: 6.5 waves, not 7) by 8192 rows 452 -> 443 us, by 6144 346 -> 340 us.  Only behind full waves:
-// with fewer tiles than pairs this is faster still (4096 x 1024 by 16384, 64 tiles: 129 -> 121 us), but its parts are
-// longer than those of the even split below, and the tensor core's sums lose with length (relative error 2.6e-6 ->
-// 1.6e-5).  Behind full waves parts are shorter than the whole tiles they replace.
+//    over take the remaining steps of one tile after another, in at most six rounds.
+// What it is worth (us, whole tiles -> shared; the matrix comes from memory, as a gradient buffer does; w + t: full waves
+// and tiles left over):
+//     w + t     K = 512        1024           1536           2048           4096           8192
+//     1 + 14    25.6 -> 23.6   31.8 -> 28.7   35.9 -> 31.7   42.0 -> 35.9   64.4 -> 48.1   108 -> 75
+//     1 + 36    25.5 -> 25.6   30.7 -> 29.6   35.8 -> 33.8   41.9 -> 37.9   64.5 -> 55.6   107 -> 88
+//     3 + 34    42.0 -> 43.0   50.2 -> 52.1   61.5 -> 59.4   72.7 -> 68.6   117 -> 108     208 -> 187
+//     6 + 36    64.5 -> 67.5   77.8 -> 78.0   97.1 -> 93.2   115 -> 109     195 -> 185     373 -> 352
+//     1 + 46 (two rounds)                     35.9 -> 34.9   42.0 -> 39.9   65.6 -> 59.3   108 -> 95
+//     3 + 50 (three)                                                        118 -> 114     209 -> 200
+//     1 + 58 (four)                                                         61.1 -> 58.4   109 -> 103
+//     1 + 62 (six), 2 + 68 (twelve), 1 + 70 (eighteen) by 16384: 209 -> 202, 327 -> 328, 217 -> 222
+// With a short K the matrix bounds the product and a part's addition to it costs what the part saves: from 24 steps on, or
+// where one full wave is followed by a third of one at most.  Beyond six rounds the helpers' additions eat up the gain.
+// Only behind full waves: with fewer tiles than pairs this is faster still (4096 x 1024 by 16384, 64 tiles: 129 -> 121 us),
+// but its parts are longer than those of the even split below, and the tensor core's sums lose with length (relative error
+// 2.6e-6 -> 1.6e-5).  Behind full waves parts are shorter than the whole tiles they replace.
 struct Tail {
     int split, kb;       // split > 1: equal parts of kb steps; 1: owners and helpers; 0: whole tiles
     double cost;         // in k steps of the longest chain of a pair
 };
-constexpr double DRAIN_STEPS = 6.0;   // what a part costs besides its own steps
+// What a part costs besides its own steps.  (An estimate.  With anything from 4 to 10 the sizes above are cut up the same way
+// but for helpers' cases up to K = 4096, whose times differ by 4 % at most.)
+constexpr double DRAIN_STEPS = 6.0;
+constexpr int TAIL_ROUNDS = 6, TAIL_STEPS = 24;   // see above
 static Tail choose_tail(int tiles, int units, int num_kb) {
     Tail t = {0, num_kb, num_kb + DRAIN_STEPS};
     if (tiles <= 0 || tiles >= units) return t;
@@ -1138,6 +1153,7 @@ static Tail choose_tail(int tiles, int units, int num_kb) {
         return t;
     }
     const int rounds = (tiles + units - tiles - 1) / (units - tiles);
+    if (rounds > TAIL_ROUNDS) return t;
     const int kb = static_cast<int>((rounds * (num_kb + DRAIN_STEPS) - DRAIN_STEPS) / (rounds + 1) + 0.999);
     if (kb < num_kb && num_kb - kb >= 4) t = {1, kb, std::max(kb + DRAIN_STEPS, rounds * (num_kb - kb + DRAIN_STEPS))};
     return t;
@@ -1202,11 +1218,13 @@ static Tiling choose_tiling(const RbGemmArgs& a) {
     const int tiles = t.m_blocks * t.n_blocks * static_cast<int>(a.batch);
     t.split = split_for(tiles);
     t.tail_tiles = t.tail_split = t.tail_kb = 0;
-    if (accum32 && t.pair && tiles > units && a.rs_nranks <= 1 && a.ag_nranks <= 1 && !a.in_order && num_kb >= 8) {
-        const Tail tail = choose_tail(tiles % units, units, num_kb);
+    const int left = tiles % units;
+    if (accum32 && t.pair && tiles > units && a.rs_nranks <= 1 && a.ag_nranks <= 1 && !a.in_order &&
+        (num_kb >= TAIL_STEPS || (num_kb >= 8 && tiles < 2 * units && 3 * left <= units))) {
+        const Tail tail = choose_tail(left, units, num_kb);
         // what the last wave takes less has to be worth it over all of them
         if (tail.split > 0 && num_kb + DRAIN_STEPS - tail.cost > 0.01 * (tiles / units + 1) * num_kb) {
-            t.tail_tiles = tiles % units;
+            t.tail_tiles = left;
             t.tail_split = tail.split;
             t.tail_kb = tail.kb;
         }
@@ -1410,6 +1428,19 @@ extern "C" int rb_gemm_splits(long long M, long long N, long long K) {
     a.out_dtype = 1;
     a.flags = RB_GEMM_ACCUM;
     return M > 0 && N > 0 && K > 0 ? rb::choose_tiling(a).split : 1;
+}
+
+// How the last wave of tiles of an fp32 [M, N] += product is summed: 0 whole tiles, 1 the first part of K by the tiles' own pairs
+// of SMs and the rest by the pairs left over, n > 1: K in n parts
+extern "C" int rb_gemm_last_wave(long long M, long long N, long long K, int in_order) {
+    RbGemmArgs a = {};
+    a.M = M, a.N = N, a.K = K, a.batch = 1;
+    a.out_dtype = 1;
+    a.flags = RB_GEMM_ACCUM;
+    a.in_order = in_order;
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    const rb::Tiling t = rb::choose_tiling(a);
+    return t.tail_tiles > 0 ? t.tail_split : 0;
 }
 
 // Copies the device error word into `host_dst` (pinned host memory) on `stream` without waiting: the caller

@@ -61,8 +61,9 @@ typedef struct RbGemmArgs {
     int32_t wgrad_taps;
     float* a_colsum;  // a_major = 1 only: the column sums of the stored A ([K, M]) are added to these M floats
     int32_t tile_n;   // columns of the single-CTA kernel's tile: 0 (chosen by size), 64, 128 or 256
-    // 1: tiles that could be summed whole are (torch.use_deterministic_algorithms): parts of one are added in the order
-    // they arrive
+    // 1 (torch.use_deterministic_algorithms): with more tiles than pairs of SMs every tile is summed whole; otherwise the last
+    // wave of a product that is added to an fp32 matrix may be shared out, and its parts are added in the order they
+    // arrive.  Fewer tiles have K split either way (rb_gemm_splits).
     int32_t in_order;
 } RbGemmArgs;
 

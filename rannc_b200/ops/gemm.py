@@ -74,6 +74,12 @@ def splits(M: int, N: int, K: int) -> int:
     return int(_lib.lib().rb_gemm_splits(ctypes.c_longlong(M), ctypes.c_longlong(N), ctypes.c_longlong(K)))
 
 
+def last_wave(M: int, N: int, K: int, in_order: bool = False) -> int:
+    """How the last, partly filled wave of tiles of such a product is summed.  0: whole tiles; 1: the first part of K by the
+    SMs that have a tile, the rest by those that have none; n > 1: K in n parts."""
+    return int(_lib.lib().rb_gemm_last_wave(ctypes.c_longlong(M), ctypes.c_longlong(N), ctypes.c_longlong(K), int(in_order)))
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bool = True,
          bias=None, residual=None, aux_in=None, aux_out=None, gelu: bool = False,
          dgelu: bool = False, out: torch.Tensor | None = None, accumulate: bool = False,

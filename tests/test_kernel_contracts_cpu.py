@@ -305,3 +305,19 @@ def test_partitioned_weight_gradient_passes_the_order_on(deterministic, monkeypa
     finally:
         torch.use_deterministic_algorithms(before)
     assert seen == [int(deterministic)]
+
+
+# tiles of 256 x 256 on 74 pairs of SMs
+@pytest.mark.parametrize("m,n,K,how", [
+    (8, 9, 8192, 0), (2, 37, 8192, 0),                                         # no last wave
+    (8, 11, 448, 0), (8, 11, 512, 2), (8, 11, 1024, 4), (8, 11, 4096, 5),      # 1 + 14
+    (2, 49, 1024, 3), (11, 9, 1024, 0), (11, 9, 1536, 2),                      # 1 + 24, 1 + 25
+    (10, 11, 1024, 0), (10, 11, 1536, 2), (3, 37, 1536, 2),                    # 1 + 36, 1 + 37
+    (16, 16, 1024, 0), (16, 16, 1536, 2), (120, 4, 512, 0), (120, 4, 1024, 0), (120, 4, 2048, 2),   # 3 + 34, 6 + 36
+    (7, 16, 1024, 0), (7, 16, 1536, 1), (8, 17, 4096, 1), (8, 17, 2048, 0),    # 1 + 38, 1 + 62
+    (6, 23, 16384, 0), (12, 18, 16384, 0), (12, 12, 16384, 0), (3, 49, 16384, 0)])   # 1 + 64, 2 + 68, 1 + 70, 1 + 73
+def test_which_last_waves_are_shared_out(m, n, K, how):
+    from rannc_b200.ops.gemm import last_wave
+
+    assert last_wave(256 * m, 256 * n - 100, K) == how
+    assert last_wave(256 * m, 256 * n - 100, K, in_order=True) == 0

@@ -316,15 +316,18 @@ def test_staged_blocks_of_many_tiles(dtype, N, tile_n, max_ctas):
     assert _lib.read_error() == 0
 
 
-# 74 pairs of SMs: 76 (2 left over), 111 (37: two parts each), 112 (38: 36 helpers, 2 rounds), 147 (73: one helper, too
-# little to share out) and 150 tiles
-@pytest.mark.parametrize("M,N", [(4864, 1024), (9472, 768), (3500, 2048), (5376, 1792), (3833, 2552)])
-@pytest.mark.parametrize("K", [448, 600, 1560])
-def test_gemm_last_wave_is_shared_out(M, N, K):
+# 74 pairs of SMs and 76 (2 left over), 111 (37), 112 (38: two rounds of helpers), 124 (50: three), 136 (62: six), 147 (73)
+# and 150 (2) tiles; in `how` many parts the last wave is summed: see ops.gemm.last_wave
+@pytest.mark.parametrize("M,N,K,how", [
+    (4864, 1024, 448, 0), (4864, 1024, 600, 2), (4864, 1024, 1560, 5), (9472, 768, 1000, 0), (9472, 768, 1560, 2),
+    (3500, 2048, 1560, 1), (1000, 7930, 2560, 1), (2041, 4352, 4090, 1), (5376, 1792, 1560, 0), (3833, 2552, 600, 0),
+    (3833, 2552, 1560, 5)])
+def test_gemm_last_wave_is_shared_out(M, N, K, how):
     """Tiles of the last wave in parts, beside whole ones: small integers, so that every order of adding is exact."""
     from rannc_b200.ops import _lib
-    from rannc_b200.ops.gemm import gemm
+    from rannc_b200.ops.gemm import gemm, last_wave
 
+    assert last_wave(M, N, K) == how and last_wave(M, N, K, in_order=True) == 0
     g = torch.Generator(device="cuda").manual_seed(M + K)
     dt = torch.bfloat16
     a, b = (torch.randint(-3, 4, (K, n), generator=g, device="cuda").to(dt) for n in ((M + 7) // 8 * 8, (N + 7) // 8 * 8))
