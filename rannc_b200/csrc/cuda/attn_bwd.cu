@@ -13,11 +13,11 @@
 // an fp32 scratch buffer by ONE bulk tensor reduction per half tile (the copy
 // engine does the read-modify-write; the math threads do not wait for it); a
 // last kernel converts the scratch to the 16-bit dQ.  Q_i / dO_i stream
-// through a 3-stage TMA ring.  Warps 0..15 = element math, warp 16 = TMA + MMA issue, warps
-// 17..20 = dQ drain, and the row statistics (lse, delta, dropout hash) of the blocks to come: the math warps' chain
-// per query block is only "S / dP -> P / dS", without a barrier among them, and the drain of block i runs
-// beside the math of block i + 1.  Of a block's products those that read dSt come first, so that its tile is free
-// again before the next block's is ready.
+// through a 3-stage TMA ring.  Warps 0..15 = element math, warp 16 = loads and the S / dP products, warp 17 = the
+// products with dSt and Pt, warps 18..21 = dQ drain, and the row statistics (lse, delta, dropout hash) of the blocks to
+// come: the math warps' chain per query block is only "S / dP -> P / dS", without a barrier among them, and the drain
+// of block i runs beside the math of block i + 1.  Of a block's products those that read dSt come first, so that its
+// tile is free again before the next block's is ready.
 //
 // 32 x 512 x 16 heads with bias and dropout, with the delta and conversion passes: 278 -> 227 us; 2 x 2048 without:
 // 197 -> 136 us.  What bounded it was neither element math (without dropout it took as long) nor the tensor core but
@@ -200,7 +200,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
             const uint32_t qa = q_desc + st * (TILE / 16), da = do_desc + st * (TILE / 16);
 #pragma unroll
             for (int k = 0; k < 8; ++k)
-                umma_f16_lo(tmem + C_DK, ds_k + (k >> 2) * (SQ_BYTES / 32) + (k & 3) * 2, qa + k * 128, id_kn, (i | k) != 0, el);
+                umma_f16_lo(tmem + C_DK, ds_k + (k >> 2) * (SQ_BYTES / 32) + (k & 3) * 2, qa + k * 128, id_kn, (i | k) != 0,
+                            el);
             // dQ of the previous step must have left tensor memory before this step's product replaces it
             if (i > 0) {
                 if (!mbar_wait_warp(dq_taken, (i - 1) & 1, abort_flag)) break;
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
             for (int k = 0; k < 8; ++k)
                 umma_f16_ts_lo(tmem + C_DV, tmem + C_P + k * 8, da + k * 128, id_kn, (i | k) != 0, el);
             if (el) {
-                if (i + QD_STAGES < nq) umma_commit(&qd_free[st]);   // (someone waits for it, so it arrives while the block lives)
+                if (i + QD_STAGES < nq) umma_commit(&qd_free[st]);   // (waited for, so it arrives while the block lives)
                 umma_commit(p_done);
             }
             if (++st == QD_STAGES) {
@@ -345,10 +346,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
                 for (int g = 0; g < 4; ++g) {
                     // A CTA holds all of tensor memory, so per SM the MMAs of a query block wait for the P / dS of the one
                     // before and these threads for its S / dP.  Sixteen warps, four to a scheduler, hide each other's
-                    // latency: with eight, of 64 columns a thread, the passes above took 246 and 175 us.  Some ten instructions per element; what has a two-wide form uses
-                    // it -- P = 2^((S scale + bias) - lse), dS = P (mask dP / (1 - p) - delta).  The bias goes to the score first, as in the forward: where every key of a
-                    // row carries a huge negative bias the score is rounded away in both, and P stays at most 1; bias - lse
-                    // first would leave 2^(S scale).
+                    // latency: with eight, of 64 columns a thread, the passes above took 246 and 175 us.  Some ten
+                    // instructions per element; what has a two-wide form uses it -- P = 2^((S scale + bias) - lse), dS = P
+                    // (mask dP / (1 - p) - delta).  The bias goes to the score first, as in the forward: where every key
+                    // of a row carries a huge negative bias the score is rounded away in both, and P stays at most 1; bias
+                    // - lse first would leave 2^(S scale).
                     const int qb = c * 16 + g * 4;
                     const ulonglong2 ls4 = *reinterpret_cast<const ulonglong2*>(st_lse + qb);
                     const ulonglong2 dl4 = *reinterpret_cast<const ulonglong2*>(st_delta + qb);
@@ -422,8 +424,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
             }
             __syncwarp();
             const long long ld = is_k ? p.dk_ss : p.dv_ss;
-            T* out = reinterpret_cast<T*>(is_k ? p.dK : p.dV) + b * (is_k ? p.dk_sb : p.dv_sb) + h * (is_k ? p.dk_sh : p.dv_sh) +
-                     half * 32 + (lane & 3) * 8;
+            T* out = reinterpret_cast<T*>(is_k ? p.dK : p.dV) + b * (is_k ? p.dk_sb : p.dv_sb) +
+                     h * (is_k ? p.dk_sh : p.dv_sh) + half * 32 + (lane & 3) * 8;
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int row = u * 8 + (lane >> 2);

@@ -58,8 +58,9 @@ struct AttnFwdParams {
 // 32 rows x 32 columns of O, one row of fp32 sums per lane, times `f`: by way of the warp's own part of the P tile, which the
 // products are done with, so that four lanes write a row's 64 bytes together.  (A lane that stored its own row touched a
 // line with every 16 bytes: from one item's last chunk to the next item's first took 5400 cycles of an item's 26000, and 3600
-// this way.  With the issuing warps converged, 32 x 512 x 16 heads with bias and dropout 114.8 -> 105.9 us, without 94.3 ->
-// 82.5; 8 x 1024 x 16 with 114.6 -> 102.7.)
+// this way.  Together with converged issuing warps, which by themselves had made no difference outside the noise (119 and
+// 117.6 us): 32 x 512 x 16 heads with bias and dropout 114.8 -> 105.9 us, without 94.3 -> 82.5; 8 x 1024 x 16 with 114.6 ->
+// 102.7.)
 template <typename T>
 __device__ __forceinline__ void store_o_rows(const uint32_t (&v)[32], float f, uint8_t* stage, int lane, T* out, long long ld,
                                              int row0, int rows) {
@@ -873,7 +874,8 @@ static int launch_fwd(const RbAttnArgs& a, cudaStream_t st) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pdev);
         if (sms <= 0) sms = 148;
         const int grid = nitems < sms ? static_cast<int>(nitems) : sms;
-        return launch_after(pk, grid, ATT_THREADS, ATTP_SMEM, st, tq, tk, tv, p, static_cast<int>(nitems)) == cudaSuccess ? 0 : -1;
+        return launch_after(pk, grid, ATT_THREADS, ATTP_SMEM, st, tq, tk, tv, p, static_cast<int>(nitems)) == cudaSuccess ? 0
+                                                                                                                          : -1;
     }
     const bool fast = (a.S + AK - 1) / AK * AK <= KB_MAX;
     auto kern = fast ? attn_fwd_kernel<T, true> : attn_fwd_kernel<T, false>;

@@ -1430,8 +1430,8 @@ extern "C" int rb_gemm_splits(long long M, long long N, long long K) {
     return M > 0 && N > 0 && K > 0 ? rb::choose_tiling(a).split : 1;
 }
 
-// How the last wave of tiles of an fp32 [M, N] += product is summed: 0 whole tiles, 1 the first part of K by the tiles' own pairs
-// of SMs and the rest by the pairs left over, n > 1: K in n parts
+// How the last wave of tiles of an fp32 [M, N] += product is summed: 0 whole tiles, 1 the first part of K by the tiles' own
+// pairs of SMs and the rest by the pairs left over, n > 1: K in n parts
 extern "C" int rb_gemm_last_wave(long long M, long long N, long long K, int in_order) {
     RbGemmArgs a = {};
     a.M = M, a.N = N, a.K = K, a.batch = 1;

@@ -5,6 +5,10 @@
 // launch_after begins while the one before it still runs: its blocks take the places that become free, do what depends
 // on no other kernel, and wait in grid_wait() until that kernel is complete and its writes are visible.
 //
+// With and without the attribute, device time of a pass forward and backward on one B200: linear 32 x 1024 x 1024 26.8 and
+// 32.9 us, FFN 900 x 1536 x 4096 146 and 154, LayerNorm 387 x 4096 (which has nothing to set up: its launch overlaps)
+// 20.6 and 25.6.  The host takes no longer for a launch either way, so a pass that is bound by the host gains nothing.
+//
 // Rules for a kernel that is launched this way:
 //  - every thread passes grid_wait() before its first access to global memory and before it ends.  (A kernel that ended
 //    without it could be complete before its predecessor, and the next one in the stream would wait for too little.)

@@ -99,8 +99,9 @@ struct LnRing {
 // A row of H = 256 * NCHUNK * WPR elements is shared by WPR warps.
 template <typename T, int NCHUNK, int WPR>
 __global__ void __launch_bounds__(LN_THREADS, LnRing<NCHUNK>::FWD_CTAS)
-    ln_fwd_kernel(const T* x, const T* residual, const T* gamma, const T* beta, T* __restrict__ y, T* __restrict__ z_out, float* __restrict__ mean_out, float* __restrict__ rstd_out,
-                  int rows, float eps, uint32_t thr, float scale, uint64_t seed, uint64_t offset) {
+    ln_fwd_kernel(const T* x, const T* residual, const T* gamma, const T* beta, T* __restrict__ y, T* __restrict__ z_out,
+                  float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, float eps, uint32_t thr, float scale,
+                  uint64_t seed, uint64_t offset) {
     constexpr int H = NCHUNK * 256 * WPR;
     constexpr int RPB = LN_WARPS / WPR;  // rows per CTA per iteration
     constexpr int STAGES = LnRing<NCHUNK>::STAGES;
@@ -355,10 +356,10 @@ static int launch_fwd(const void* x, const void* res, const void* g, const void*
     if (grid > cap) grid = cap;
     static bool allowed[64] = {false};
     if (!ln_allow_smem(ln_fwd_kernel<T, NCHUNK, WPR>, LnRing<NCHUNK>::BYTES, allowed)) return -1;
-    const cudaError_t e = launch_after(
-        ln_fwd_kernel<T, NCHUNK, WPR>, grid, LN_THREADS, LnRing<NCHUNK>::BYTES, st, static_cast<const T*>(x), static_cast<const T*>(res), static_cast<const T*>(g),
-        static_cast<const T*>(b), static_cast<T*>(y), static_cast<T*>(z), mean, rstd, rows, eps,
-        thr, scale, seed, offset);
+    const cudaError_t e = launch_after(ln_fwd_kernel<T, NCHUNK, WPR>, grid, LN_THREADS, LnRing<NCHUNK>::BYTES, st,
+                                       static_cast<const T*>(x), static_cast<const T*>(res), static_cast<const T*>(g),
+                                       static_cast<const T*>(b), static_cast<T*>(y), static_cast<T*>(z), mean, rstd, rows,
+                                       eps, thr, scale, seed, offset);
     return e == cudaSuccess ? 0 : -1;
 }
 
@@ -370,10 +371,10 @@ static int launch_bwd(const void* dy, const void* z, const void* g, const float*
     const float scale = p > 0.f ? 1.f / (1.f - p) : 1.f;
     static bool allowed[64] = {false};
     if (!ln_allow_smem(ln_bwd_kernel<T, NCHUNK, WPR>, LnRing<NCHUNK>::BYTES, allowed)) return -1;
-    const cudaError_t e = launch_after(
-        ln_bwd_kernel<T, NCHUNK, WPR>, grid, LN_THREADS, LnRing<NCHUNK>::BYTES, st, static_cast<const T*>(dy), static_cast<const T*>(z), static_cast<const T*>(g), mean, rstd,
-        static_cast<T*>(dz), static_cast<T*>(p > 0.f ? dx : nullptr), partial, rows, thr, scale,
-        seed, offset);
+    const cudaError_t e = launch_after(ln_bwd_kernel<T, NCHUNK, WPR>, grid, LN_THREADS, LnRing<NCHUNK>::BYTES, st,
+                                       static_cast<const T*>(dy), static_cast<const T*>(z), static_cast<const T*>(g), mean,
+                                       rstd, static_cast<T*>(dz), static_cast<T*>(p > 0.f ? dx : nullptr), partial, rows,
+                                       thr, scale, seed, offset);
     return e == cudaSuccess ? 0 : -1;
 }
 
