@@ -446,3 +446,65 @@ def test_kernels_in_a_row_under_capture_and_across_streams(how):
             step(True)
     torch.cuda.synchronize()
     assert torch.equal(x, want)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_kernels_that_begin_early_on_streams_beside_each_other(captured):
+    """Chains of such kernels on two streams at once, each over its own buffers: blocks of one stream wait on the device in
+    places that kernels of the other want.  The same bits as one chain after the other; captured, the streams fork and
+    join inside the graph."""
+    from rannc_b200.ops import kernels as K
+    from rannc_b200.ops.gemm import gemm
+
+    torch.manual_seed(6)
+    dt, H, S = torch.bfloat16, 256, 192
+    w = [(torch.randn(3 * H, H, device="cuda") * H ** -0.5).to(dt), (torch.randn(H, H, device="cuda") * H ** -0.5).to(dt)]
+    g, b = torch.ones(H, device="cuda", dtype=dt), torch.zeros(H, device="cuda", dtype=dt)
+    start = [torch.randn(rows, H, device="cuda").to(dt) for rows in (5 * S, 24 * S)]
+    sums = [torch.zeros(3 * H, H, device="cuda") for _ in start]
+    xs = [x.clone() for x in start]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    kept = []
+
+    def chain(i, steps):
+        x, rows = xs[i], xs[i].shape[0]
+        for _ in range(steps):
+            qkv = gemm(x, w[0])
+            q, k, v = (qkv.view(rows // S, S, 3, 4, 64)[:, :, j] for j in range(3))
+            o, lse = K.attn_fwd(q, k, v)
+            z, zin, mean, rstd = K.ln_fwd(gemm(o.view(rows, H), w[1]), x, g, b, 1e-5)
+            dz = K.ln_bwd(z, zin, g, mean, rstd)[1]
+            dv = K.attn_bwd(q, k, v, o, lse, dz.view(rows // S, S, 4, 64))[2]
+            gemm(qkv, dv.reshape(rows, H), trans_a=True, trans_b=False, out=sums[i], accumulate=True)
+            x.copy_(z)
+            kept.extend((qkv, o, lse, z, zin, mean, rstd, dz, dv))
+
+    def both(steps):
+        here = torch.cuda.current_stream()
+        for i, s in enumerate(streams):
+            s.wait_stream(here)
+            with torch.cuda.stream(s):
+                chain(i, steps)
+        for s in streams:
+            here.wait_stream(s)
+
+    for i in range(2):
+        chain(i, 6)
+    torch.cuda.synchronize()
+    want, want_sums = [x.clone() for x in xs], [s.clone() for s in sums]
+    for x, x0, s in zip(xs, start, sums):
+        x.copy_(x0)
+        s.zero_()
+    torch.cuda.synchronize()
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            both(3)
+        for _ in range(2):
+            graph.replay()
+    else:
+        both(6)
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, y) for x, y in zip(xs, want))
+    for s, y in zip(sums, want_sums):   # (K is split: added as it arrives)
+        assert (s - y).norm() <= 1e-5 * y.norm()
