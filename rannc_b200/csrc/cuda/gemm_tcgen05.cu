@@ -19,7 +19,7 @@
 //
 // PAIR variant (cta_group::2): two CTAs of a cluster -- the two SMs of a TPC -- share a 256 x 256 tile.
 // Each CTA loads its own 128 rows of A and HALF of the B tile (so a k step moves 32 KiB per SM instead
-// of 48 KiB: the single-CTA tile is limited by the L2 -> shared-memory path, not by the tensor core),
+// of 48 KiB, and shared memory, which the products read too, takes that much less in),
 // one lane of the first CTA issues the MMAs for both, and each CTA keeps and drains the accumulator of
 // its own 128 rows.  Completion of both CTAs' loads is counted on the first CTA's barrier; stage-free
 // and accumulator-full signals go to both CTAs with one multicast commit.  No load is multicast.
@@ -281,11 +281,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         // ---------------- TMA producer ----------------
         // One lane issues every copy and the warp goes along: behind a branch for that lane, coordinates and addresses
         // would have to be moved to the uniform registers for each instruction (16384 x 4096 x 1024, B MN-major: 128.4 ->
-        // 126.1 us; 4096 x 1024 x 6144 into fp32, both MN-major: 61.3 -> 58.4).  A step must not take longer than the 512
-        // cycles its bytes need on the way from L2 (62 bytes a cycle): what does not change from step to step is worked out
-        // per tile, and the filter tap is counted on.  A division per step (and, MN-major, one per column block) for the tap
-        // held back the convolution's products: 3x3, 32 x 28 x 28, 1024 to 1024 channels with batch norm, forward and
-        // backward, 1550 -> 1354 us.
+        // 126.1 us; 4096 x 1024 x 6144 into fp32, both MN-major: 61.3 -> 58.4).
+        // What a step costs this one warp bounds the whole kernel: the products of a step take 512 cycles, the copy engine
+        // brings a step's bytes in some 300 (a loop that only copies: 100 to 115 bytes a cycle and SM, in either layout), but
+        // a step that chose its layout, its tap and its form of copy anew took 530 cycles (K-major) to 609 (MN-major) on an
+        // otherwise idle SM, and 790 beside a busy epilogue, which takes turns with it at the scheduler.  So a tile's steps
+        // are cut into runs without a decision in them -- one copy per operand, of one form, whose coordinates move on by
+        // constants -- and the next stage's barrier is asked before it is needed.  Cycles a step (one tile's products / its
+        // steps): 8192^3 K-major 530 -> 510, MN-major 609 -> 510; 16384 x 4096 x 1024 with bias 600 -> 485, with GELU and
+        // second output 790 -> 540 (now the accumulators are waited for); 4096 x 1024 x 16384 into fp32 690 -> 563.  Back to
+        // back under the power cap, where fewer cycles mean a lower clock (us): 117.6 -> 97.9 with bias, 129 -> 107 weight
+        // gradient, 428 -> 373 head (8192 x 30528 x 1024), 441 -> 365 its weight gradient; 32 x 1024 x 1024 9.7 -> 7.9.
         const uint32_t el = elect_one();
         int stage = 0;
         uint32_t phase = 0;
@@ -293,8 +299,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         bool ok = true;
         const bool a_k = p.a_major == 0, b_k = p.b_major == 0, a_merged = p.a_merged, b_merged = p.b_merged;
         const bool gather = p.ag_nranks > 1, conv = p.conv_kb_per_tap > 0;
+        // an MN-major operand whose columns are no whole number of 64-column chunks takes a copy per chunk
+        const bool chunked = !(a_k || a_merged) || !(b_k || b_merged);
         // PAIR: both CTAs' bytes are counted on the first CTA's barrier
         const uint32_t full0 = PAIR ? mapa_shared(smem_u32(full), 0) : smem_u32(full);
+        uint32_t empty_now = mbar_test_wait(&empty[0], 1);
         for (int tile = tile0; tile < p.num_tiles && ok; tile += tile_step) {
             int mb, nb, b, kb_begin, kb_end;
             tile_coords(p, tile, mb, nb, b, kb_begin, kb_end);
@@ -303,7 +312,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             // position along K in A and in B, and the rows (columns) of each: A's (K-major) shift with the filter tap,
             // B's (MN-major) move on by a block of columns per tap
             int ak = kb_begin * BK, am = m0, bk = ak, bn = n0;
-            int tap = 0, left = 0x7fffffff;   // steps until the next tap, or until a gathered K wraps around
+            int tap = 0, shift0 = 0, left = 0x7fffffff;   // steps until the next tap, or until a gathered K wraps around
             if (conv) {
                 tap = kb_begin / p.conv_kb_per_tap;
                 ak -= tap * p.conv_kb_per_tap * BK;
@@ -313,108 +322,117 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     bk = ak;
                     bn = n0 + tap * p.conv_b_tap_cols;
                 }
-            } else if (p.wgrad_taps > 0 && b_merged) {
+            } else if (p.wgrad_taps > 0) {
                 // column block -> filter tap: the tap's rows are shifted; past the last tap the columns lie outside
-                // the matrix and read as zero
+                // the matrix and read as zero.  (Of several chunks, this is the first.)
                 const int t = min(n0 / p.wgrad_cols, p.wgrad_taps - 1);
                 bn = n0 - t * p.wgrad_cols;
-                bk += p.conv_shift[t];
+                shift0 = p.conv_shift[t];
+                bk += shift0;
             } else if (gather && b_k) {
                 // start with the k-range this rank holds itself
                 const int own = p.ag_my_idx * (p.ag_cols / BK);
                 ak = bk = (kb_begin + own < p.num_kb ? kb_begin + own : kb_begin + own - p.num_kb) * BK;
                 left = p.num_kb - ak / BK;
             }
-            for (int kbi = kb_begin; kbi < kb_end; ++kbi) {
-                if (gather) {
-                    // wait until every CTA has copied the shard this step reads into the local B buffer
-                    const int shard = (b_k ? bk : n0) / p.ag_cols;
-                    if (!(ag_ready & (1u << shard))) {
-                        bool got = false;
-                        const uint64_t t0 = globaltimer_ns();
-                        for (uint32_t it = 0; it < RB_MBAR_SPIN_LIMIT; ++it) {
-                            if (__any_sync(0xffffffffu, *abort_flag)) break;
-                            unsigned int v;
-                            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.ag_flags + shard) : "memory");
-                            if (__all_sync(0xffffffffu, v >= gridDim.x)) {
-                                got = true;
+            int todo = kb_end - kb_begin;
+            while (todo > 0 && ok) {
+                // a run of steps that only move along K: coordinates of the operands' maps
+                // (four-dimensional, whatever the layout) and what they move on by
+                int run = min(todo, left);
+                todo -= run;
+                int a0 = a_k ? ak : (a_merged ? 0 : am), a1 = a_k ? am : ak;
+                int b0 = b_k ? bk : (b_merged ? 0 : bn), b1 = b_k ? bn : bk;
+                const int a2 = a_merged ? am >> 6 : 0, b2 = b_merged ? bn >> 6 : 0;
+                const int da0 = a_k ? BK : 0, da1 = BK - da0, db0 = b_k ? BK : 0, db1 = BK - db0;
+                for (; run > 0; --run) {
+                    if (gather) {
+                        // wait until every CTA has copied the shard this step reads into the local B buffer
+                        const int shard = (b_k ? b0 : n0) / p.ag_cols;
+                        if (!(ag_ready & (1u << shard))) {
+                            bool got = false;
+                            const uint64_t t0 = globaltimer_ns();
+                            for (uint32_t it = 0; it < RB_MBAR_SPIN_LIMIT; ++it) {
+                                if (__any_sync(0xffffffffu, *abort_flag)) break;
+                                unsigned int v;
+                                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.ag_flags + shard) : "memory");
+                                if (__all_sync(0xffffffffu, v >= gridDim.x)) {
+                                    got = true;
+                                    break;
+                                }
+                                if ((it & 0xff) == 0xff && __any_sync(0xffffffffu, globaltimer_ns() - t0 > RB_WAIT_LIMIT_NS)) break;
+                                __nanosleep(64);
+                            }
+                            if (!got) {
+                                *abort_flag = 1;
+                                ok = false;
                                 break;
                             }
-                            if ((it & 0xff) == 0xff && __any_sync(0xffffffffu, globaltimer_ns() - t0 > RB_WAIT_LIMIT_NS)) break;
-                            __nanosleep(64);
+                            asm volatile("fence.proxy.async.global;" ::: "memory");
+                            ag_ready |= 1u << shard;
                         }
-                        if (!got) {
-                            *abort_flag = 1;
-                            ok = false;
-                            break;
-                        }
-                        asm volatile("fence.proxy.async.global;" ::: "memory");
-                        ag_ready |= 1u << shard;
                     }
-                }
-                if (!mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag)) {
-                    ok = false;
-                    break;
-                }
-                uint8_t* a_dst = sA + stage * A_STAGE_BYTES;
-                uint8_t* b_dst = sB + stage * B_STAGE_BYTES;
-                const uint32_t fb = full0 + stage * 8;
-                if (!PAIR || crank == 0) mbar_arrive_expect_tx_el(&full[stage], (PAIR ? 2 : 1) * STAGE_BYTES, el);
-                auto load_3d = [&](uint8_t* dst, const CUtensorMap* m, int c0, int c1) {
-                    if constexpr (PAIR)
-                        tma_load_3d_pair(dst, m, fb, c0, c1, b, el);
-                    else
-                        tma_load_3d_el(dst, m, &full[stage], c0, c1, b, el);
-                };
-                auto load_chunks = [&](uint8_t* dst, const CUtensorMap* m, int k, int chunk) {
-                    if constexpr (PAIR)
-                        tma_load_4d_pair(dst, m, fb, 0, k, chunk, b, el);
-                    else
-                        tma_load_4d_el(dst, m, &full[stage], 0, k, chunk, b, el);
-                };
-                if (a_k) {
-                    load_3d(a_dst, &tmA, ak, am);
-                } else if (a_merged) {
-                    load_chunks(a_dst, &tmA, ak, am >> 6);
-                } else {
-#pragma unroll
-                    for (int c = 0; c < BM / 64; ++c) load_3d(a_dst + c * (BK * 128), &tmA, am + c * 64, ak);
-                }
-                if (b_k) {
-                    load_3d(b_dst, &tmB, bk, bn);
-                } else if (b_merged) {
-                    load_chunks(b_dst, &tmB, bk, bn >> 6);
-                } else {
-#pragma unroll
-                    for (int c = 0; c < Cfg<PAIR, BN>::B_ROWS / 64; ++c) {
-                        int cx = bn + c * 64, cy = bk;
-                        if (p.wgrad_taps > 0) {
-                            const int t = min(cx / p.wgrad_cols, p.wgrad_taps - 1);
-                            cx -= t * p.wgrad_cols;
-                            cy += p.conv_shift[t];
-                        }
-                        load_3d(b_dst + c * (BK * 128), &tmB, cx, cy);
+                    // (asked about at the end of the step before: the answer is there by now)
+                    if (!__all_sync(0xffffffffu, empty_now) && !mbar_wait_warp(&empty[stage], phase ^ 1, abort_flag)) {
+                        ok = false;
+                        break;
                     }
+                    uint8_t* a_dst = sA + stage * A_STAGE_BYTES;
+                    uint8_t* b_dst = sB + stage * B_STAGE_BYTES;
+                    const uint32_t fb = full0 + stage * 8;
+                    if (!PAIR || crank == 0) mbar_arrive_expect_tx_el(&full[stage], (PAIR ? 2 : 1) * STAGE_BYTES, el);
+                    auto load = [&](uint8_t* dst, const CUtensorMap* m, int c0, int c1, int c2) {
+                        if constexpr (PAIR)
+                            tma_load_4d_pair(dst, m, fb, c0, c1, c2, b, el);
+                        else
+                            tma_load_4d_el(dst, m, &full[stage], c0, c1, c2, b, el);
+                    };
+                    load(a_dst, &tmA, a0, a1, a2);
+                    load(b_dst, &tmB, b0, b1, b2);
+                    if (chunked) {
+                        if (!a_k && !a_merged) {
+#pragma unroll 1
+                            for (int c = 1; c < BM / 64; ++c) load(a_dst + c * (BK * 128), &tmA, a0 + c * 64, a1, 0);
+                        }
+                        if (!b_k && !b_merged) {
+#pragma unroll 1
+                            for (int c = 1; c < Cfg<PAIR, BN>::B_ROWS / 64; ++c) {
+                                int cx = b0 + c * 64, cy = b1;
+                                if (p.wgrad_taps > 0) {
+                                    cx = n0 + c * 64;
+                                    const int t = min(cx / p.wgrad_cols, p.wgrad_taps - 1);
+                                    cx -= t * p.wgrad_cols;
+                                    cy += p.conv_shift[t] - shift0;
+                                }
+                                load(b_dst + c * (BK * 128), &tmB, cx, cy, 0);
+                            }
+                        }
+                    }
+                    a0 += da0;
+                    a1 += da1;
+                    b0 += db0;
+                    b1 += db1;
+                    if (++stage == STAGES) {
+                        stage = 0;
+                        phase ^= 1;
+                    }
+                    empty_now = mbar_test_wait(&empty[stage], phase ^ 1);
                 }
-                ak += BK;
-                bk += BK;
-                if (--left == 0) {
+                if (todo > 0) {   // (behind the last tap there is no further step)
                     ak = 0;
                     if (conv) {
                         left = p.conv_kb_per_tap;
-                        // (behind the last tap there is no further step)
-                        if (kbi + 1 < kb_end) am = m0 + p.conv_shift[++tap];
-                        if (!b_k) {
+                        am = m0 + p.conv_shift[++tap];
+                        if (b_k) {
+                            bk = b0;
+                        } else {
                             bk = 0;
                             bn += p.conv_b_tap_cols;
                         }
                     } else {
+                        left = 0x7fffffff;
                         bk = 0;
                     }
-                }
-                if (++stage == STAGES) {
-                    stage = 0;
-                    phase ^= 1;
                 }
             }
         }
@@ -896,31 +914,6 @@ static EncodeTiledFn get_encode_fn() {
     return fn;
 }
 
-int make_tmap_3d(CUtensorMap* out, const void* base, int dtype_16bit_kind, uint64_t d0, uint64_t d1,
-                 uint64_t d2, uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0,
-                 uint32_t b1, int swizzle128) {
-    EncodeTiledFn fn = get_encode_fn();
-    if (!fn) return -100;
-    cuuint64_t dims[3] = {d0, d1, d2};
-    cuuint64_t strides[2] = {stride1_bytes, stride2_bytes};
-    cuuint32_t box[3] = {b0, b1, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUtensorMapDataType dt =
-        dtype_16bit_kind == 1 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-    CUresult r = CUDA_SUCCESS;
-    for (int attempt = 0; attempt < 2; ++attempt) {
-        r = fn(out, dt, 3, const_cast<void*>(base), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE,
-               swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_ERROR_INVALID_CONTEXT) break;
-        // a thread that has made no runtime call yet (an autograd worker whose first operator is ours) has
-        // no context bound for driver entry points: bind the device's primary context and try again
-        cudaFree(nullptr);
-    }
-    return r == CUDA_SUCCESS ? 0 : -static_cast<int>(r) - 1000;
-}
-
 int make_tmap_4d(CUtensorMap* out, const void* base, int fmt, uint64_t d0, uint64_t d1, uint64_t d2,
                  uint64_t d3, uint64_t s1, uint64_t s2, uint64_t s3, uint32_t b0, uint32_t b1) {
     EncodeTiledFn fn = get_encode_fn();
@@ -937,6 +930,8 @@ int make_tmap_4d(CUtensorMap* out, const void* base, int fmt, uint64_t d0, uint6
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_ERROR_INVALID_CONTEXT) break;
+        // a thread that has made no runtime call yet (an autograd worker whose first operator is ours) has
+        // no context bound for driver entry points: bind the device's primary context and try again
         cudaFree(nullptr);
     }
     return r == CUDA_SUCCESS ? 0 : -static_cast<int>(r) - 1000;
@@ -977,7 +972,7 @@ static int make_tmap_chunks(CUtensorMap* out, const void* base, int fmt, uint64_
                const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_ERROR_INVALID_CONTEXT) break;
-        cudaFree(nullptr);   // a thread without a context yet: see make_tmap_3d
+        cudaFree(nullptr);   // a thread without a context yet: see make_tmap_4d
     }
     return r == CUDA_SUCCESS ? 0 : -static_cast<int>(r) - 1000;
 }
@@ -1371,13 +1366,13 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
                                      : a->wgrad_taps > 0 ? a->conv_c % b_cols == 0
                                                          : a->N % 64 == 0);
     if (a->conv_taps > 0)
-        rc = make_tmap_3d(&tmA, a->A, a->in_dtype, a->conv_c, a->M, 1, a->lda * 2, a->M * a->lda * 2, BK, BM, 1);
+        rc = make_tmap_4d(&tmA, a->A, a->in_dtype, a->conv_c, a->M, 1, 1, a->lda * 2, sA, sA, BK, BM);
     else if (a->a_major == 0)
-        rc = make_tmap_3d(&tmA, a->A, a->in_dtype, a->K, a->M, a->batch, a->lda * 2, sA, BK, BM, 1);
+        rc = make_tmap_4d(&tmA, a->A, a->in_dtype, a->K, a->M, 1, a->batch, a->lda * 2, sA, sA, BK, BM);
     else if (p.a_merged)
         rc = make_tmap_chunks(&tmA, a->A, a->in_dtype, a->K, a->M / 64, a->batch, a->lda * 2, sA, BM / 64);
     else
-        rc = make_tmap_3d(&tmA, a->A, a->in_dtype, a->M, a->K, a->batch, a->lda * 2, sA, 64, BK, 1);
+        rc = make_tmap_4d(&tmA, a->A, a->in_dtype, a->M, a->K, 1, a->batch, a->lda * 2, sA, sA, 64, BK);
     if (rc) return rc;
     // stored columns of an MN-major B: with filter taps [conv_c rows, conv_taps * conv_b_tap_cols] (tap t's block starts
     // at column t * conv_b_tap_cols), for a weight gradient the activation's conv_c
@@ -1387,11 +1382,11 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     const uint64_t b_rows = a->conv_taps > 0 ? a->conv_c : a->K;
     const uint64_t sB1 = a->conv_taps > 0 ? static_cast<uint64_t>(a->conv_c) * a->ldb * 2 : sB;
     if (a->b_major == 0)
-        rc = make_tmap_3d(&tmB, a->B, a->in_dtype, a->K, a->N, a->batch, a->ldb * 2, sB, BK, b_cols, 1);
+        rc = make_tmap_4d(&tmB, a->B, a->in_dtype, a->K, a->N, 1, a->batch, a->ldb * 2, sB, sB, BK, b_cols);
     else if (p.b_merged)
         rc = make_tmap_chunks(&tmB, a->B, a->in_dtype, b_rows, stored / 64, a->batch, a->ldb * 2, sB1, b_cols / 64);
     else
-        rc = make_tmap_3d(&tmB, a->B, a->in_dtype, stored, b_rows, a->batch, a->ldb * 2, sB1, 64, BK, 1);
+        rc = make_tmap_4d(&tmB, a->B, a->in_dtype, stored, b_rows, 1, a->batch, a->ldb * 2, sB1, sB1, 64, BK);
     if (rc) return rc;
 
     // The staged epilogue wants outputs the copy engine can address: plain rows in this GPU's memory, 16-byte

@@ -78,9 +78,6 @@ int rb_error_peek_async(int* host_dst, void* stream);
 }
 #include <cuda.h>
 namespace rb {
-int make_tmap_3d(CUtensorMap* out, const void* base, int dtype_16bit_kind, uint64_t d0, uint64_t d1,
-                 uint64_t d2, uint64_t stride1_bytes, uint64_t stride2_bytes, uint32_t b0,
-                 uint32_t b1, int swizzle128);
 int* error_word_ptr();
 int num_sms();
 }  // namespace rb

@@ -90,6 +90,20 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// Whether the phase is over, without waiting for it.
+__device__ __forceinline__ uint32_t mbar_test_wait(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred P1;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, P1;\n\t"
+        "}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok;
+}
 // Bounded wait.  Returns false when the limit ran out (caller aborts).
 // `abort_flag` is a shared-memory word any role may set; every waiter polls it
 // so one timeout drains the whole CTA.
@@ -156,20 +170,6 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m
         : "memory");
 }
 // (`el`: nonzero in the lane that issues; the rest of a converged warp passes by)
-__device__ __forceinline__ void tma_load_3d_el(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2,
-                                               uint32_t el) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred q;\n\t"
-        "setp.ne.b32 q, %6, 0;\n\t"
-        "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5}], [%2];\n\t"
-        "}\n"
-        :
-        : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)),
-          "r"(c0), "r"(c1), "r"(c2), "r"(el)
-        : "memory");
-}
 __device__ __forceinline__ void tma_load_4d_el(void* smem_dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2,
                                                int c3, uint32_t el) {
     asm volatile(
@@ -284,20 +284,6 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t cta_mas
 }
 // tiled load into this CTA's shared memory whose completion is counted on a barrier of the pair's first
 // CTA (`bar_cluster_addr` from mapa_shared); no multicast: every CTA fetches its own tile
-__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr,
-                                                 int c0, int c1, int c2, uint32_t el) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred q;\n\t"
-        "setp.ne.b32 q, %6, 0;\n\t"
-        "@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5}], [%2];\n\t"
-        "}\n"
-        :
-        : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr),
-          "r"(c0), "r"(c1), "r"(c2), "r"(el)
-        : "memory");
-}
 __device__ __forceinline__ void tma_load_4d_pair(void* smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr,
                                                  int c0, int c1, int c2, int c3, uint32_t el) {
     asm volatile(
