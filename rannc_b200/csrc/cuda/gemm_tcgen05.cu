@@ -13,9 +13,9 @@
 // Structure: persistent CTAs (one per SM), 128 x 256 output tile (128 or 64 columns for small problems), K step 64,
 // 4-stage TMA->smem ring (6 or 8 with narrower tiles), fp32 accumulators double-buffered in TMEM (2 x 256
 // columns) so the epilogue of tile i overlaps the main loop of tile i+1.
-// Warp 0 = TMA producer, warp 1 = MMA issuer, warps 2..9 = epilogue, warps 10 and 11 = column sums of A where
-// asked for (with K = 1024 a tile's main loop is only 16 k steps, and four warps could not drain a 128 x 256
-// accumulator in that time); the epilogue writes through shared memory and the copy engine.
+// Warp 0 = TMA producer, warp 1 = MMA issuer, the next eight (sixteen with an activation) = epilogue, the last two =
+// column sums of A where asked for (with K = 1024 a tile's main loop is only 16 k steps, and four warps could not
+// drain a 128 x 256 accumulator in that time); the epilogue writes through shared memory and the copy engine.
 //
 // PAIR variant (cta_group::2): two CTAs of a cluster -- the two SMs of a TPC -- share a 256 x 256 tile.
 // Each CTA loads its own 128 rows of A and HALF of the B tile (so a k step moves 32 KiB per SM instead
@@ -41,19 +41,18 @@ namespace rb {
 constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int A_STAGE_BYTES = BM * BK * 2;  // 16 KiB
-constexpr int EPI_WARPS = 8;                         // two per TMEM lane quarter: each drains 128 of the 256 columns
-constexpr int EPI_THREADS = 32 * EPI_WARPS;
 constexpr int SUM_WARPS = 2;                         // column sums of A: one per 64-column chunk of its tile
-constexpr int GEMM_THREADS = 64 + EPI_THREADS + 32 * SUM_WARPS;
 constexpr int GROUP_M = 8;
-// Output staging: every epilogue warp owns 4 KiB of shared memory in which it lays out a 32 x 32 block of the
-// tile (16-bit: two blocks of 64-byte rows; fp32: one of 128-byte rows, both swizzled as the tensor map of D
-// says) that the copy engine then writes, or adds, to global memory.
-constexpr int EPI_STAGE_BYTES = 4096;
+constexpr int EPI_BYTES = 32 * 1024;                 // staging memory of the epilogue warps
 
 // TN: columns of the output tile.  A wide tile moves the fewest bytes per multiplication; a problem with too few
 // 256-wide tiles to give every SM one takes 128 or 64 columns instead (single-CTA kernel only).
-template <bool PAIR, int TN>
+// EW: epilogue warps, 8 or 16: two or four per TMEM lane quarter, each with 128 or 64 of the tile's 256 columns (and 32 at
+// least: with a 64-column tile half of sixteen have nothing to do).  Sixteen where an activation is part of the epilogue
+// (see there).  Each owns 4 or 2 KiB of shared memory in which it lays out 32 x 32 blocks of the tile (16-bit: 64-byte rows,
+// two blocks or one; fp32: 128-byte rows, eight warps only; both swizzled as the tensor map of D says) that the copy engine
+// then writes, or adds, to global memory.
+template <bool PAIR, int TN, int EW>
 struct Cfg {
     static_assert(TN == 256 || (!PAIR && (TN == 128 || TN == 64)), "unsupported tile");
     static constexpr int B_ROWS = PAIR ? TN / 2 : TN;       // extent of the B tile one CTA loads
@@ -61,9 +60,14 @@ struct Cfg {
     static constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
     static constexpr int STAGES = 192 * 1024 / STAGE_BYTES;  // 6 (pair) / 4 / 6 / 8
     static constexpr int SMEM_BYTES =
-        STAGES * STAGE_BYTES + EPI_WARPS * EPI_STAGE_BYTES + 1024 /*align slack*/ + 384 /*barriers*/;
+        STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align slack*/ + 384 /*barriers*/;
     static constexpr int TILE_M = PAIR ? 2 * BM : BM;       // rows of the output tile of a CTA (pair)
     static constexpr int TMEM_COLS = 2 * TN;                // two accumulators
+    static constexpr int EPI_THREADS = 32 * EW;
+    static constexpr int THREADS = 64 + EPI_THREADS + 32 * SUM_WARPS;
+    static constexpr int PARTS = TN / 32 < EW / 4 ? TN / 32 : EW / 4;   // column groups of the tile
+    static constexpr int PART_COLS = TN / PARTS;
+    static constexpr int DRAIN_WARPS = 4 * PARTS;
 };
 
 struct GemmKernelParams {
@@ -150,13 +154,13 @@ __device__ __forceinline__ void tile_coords(const GemmKernelParams& p, int tile,
     mb = first_m + (t - nb * gm);
 }
 
-template <typename T>
-__device__ __forceinline__ void load32(const T* ptr, bool vec_ok, int valid, float (&v)[32]) {
+template <int N, typename T>
+__device__ __forceinline__ void load_n(const T* ptr, bool vec_ok, int valid, float (&v)[N]) {
     if (vec_ok) {
         if constexpr (sizeof(T) == 2) {
             const uint4* p4 = reinterpret_cast<const uint4*>(ptr);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < N / 8; ++i) {
                 uint4 q = p4[i];
                 const T* e = reinterpret_cast<const T*>(&q);
 #pragma unroll
@@ -165,7 +169,7 @@ __device__ __forceinline__ void load32(const T* ptr, bool vec_ok, int valid, flo
         } else {
             const float4* p4 = reinterpret_cast<const float4*>(ptr);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < N / 4; ++i) {
                 float4 q = p4[i];
                 v[i * 4 + 0] = q.x;
                 v[i * 4 + 1] = q.y;
@@ -175,17 +179,17 @@ __device__ __forceinline__ void load32(const T* ptr, bool vec_ok, int valid, flo
         }
     } else {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = (j < valid) ? to_f32<T>(ptr[j]) : 0.f;
+        for (int j = 0; j < N; ++j) v[j] = (j < valid) ? to_f32<T>(ptr[j]) : 0.f;
     }
 }
 
-template <typename T>
-__device__ __forceinline__ void store32(T* ptr, bool vec_ok, int valid, const float (&v)[32]) {
+template <int N, typename T>
+__device__ __forceinline__ void store_n(T* ptr, bool vec_ok, int valid, const float (&v)[N]) {
     if (vec_ok) {
         if constexpr (sizeof(T) == 2) {
             uint4* p4 = reinterpret_cast<uint4*>(ptr);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < N / 8; ++i) {
                 uint4 q;
                 T* e = reinterpret_cast<T*>(&q);
 #pragma unroll
@@ -195,34 +199,36 @@ __device__ __forceinline__ void store32(T* ptr, bool vec_ok, int valid, const fl
         } else {
             float4* p4 = reinterpret_cast<float4*>(ptr);
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < N / 4; ++i)
                 p4[i] = make_float4(v[i * 4], v[i * 4 + 1], v[i * 4 + 2], v[i * 4 + 3]);
         }
     } else {
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
+        for (int j = 0; j < N; ++j)
             if (j < valid) ptr[j] = from_f32<T>(v[j]);
     }
 }
 
-template <typename InT, typename OutT, bool PAIR, int BN>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
+
+template <typename InT, typename OutT, bool PAIR, int BN, int EPI_WARPS>
+__global__ void __launch_bounds__(Cfg<PAIR, BN, EPI_WARPS>::THREADS, 1)
     gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
                         const __grid_constant__ CUtensorMap tmB,
                         const __grid_constant__ CUtensorMap tmD,
                         const __grid_constant__ CUtensorMap tmAux, const GemmKernelParams p) {
-    constexpr int STAGES = Cfg<PAIR, BN>::STAGES;
-    constexpr int B_STAGE_BYTES = Cfg<PAIR, BN>::B_STAGE_BYTES;
-    constexpr int STAGE_BYTES = Cfg<PAIR, BN>::STAGE_BYTES;
-    constexpr int TILE_M = Cfg<PAIR, BN>::TILE_M;
-    constexpr int TMEM_COLS = Cfg<PAIR, BN>::TMEM_COLS;
+    using C = Cfg<PAIR, BN, EPI_WARPS>;
+    constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES, B_STAGE_BYTES = C::B_STAGE_BYTES;
+    constexpr int TILE_M = C::TILE_M, TMEM_COLS = C::TMEM_COLS;
+    constexpr int EPI_THREADS = C::EPI_THREADS, EPI_STAGE_BYTES = EPI_BYTES / EPI_WARPS;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                ~static_cast<uintptr_t>(1023));
     uint8_t* sA = smem;
     uint8_t* sB = smem + STAGES * A_STAGE_BYTES;
     uint8_t* sEpi = smem + STAGES * STAGE_BYTES;   // [EPI_WARPS][EPI_STAGE_BYTES]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sEpi + EPI_WARPS * EPI_STAGE_BYTES);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sEpi + EPI_BYTES);
     uint64_t* full = bars;                  // [STAGES]
     uint64_t* empty = bars + STAGES;        // [STAGES]
     uint64_t* tfull = bars + 2 * STAGES;    // [2]
@@ -248,7 +254,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(&tfull[a], 1);
-            mbar_init(&tempty[a], PAIR ? 2 * EPI_WARPS : EPI_THREADS);   // PAIR: one arrival per epilogue warp of both CTAs
+            mbar_init(&tempty[a], (PAIR ? 2 : 32) * C::DRAIN_WARPS);   // PAIR: one arrival per epilogue warp of both CTAs
         }
         for (int w = 0; w < EPI_WARPS; ++w) mbar_init(&aux_full[w], 1);
         *abort_flag = 0;
@@ -396,7 +402,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         }
                         if (!b_k && !b_merged) {
 #pragma unroll 1
-                            for (int c = 1; c < Cfg<PAIR, BN>::B_ROWS / 64; ++c) {
+                            for (int c = 1; c < C::B_ROWS / 64; ++c) {
                                 int cx = b0 + c * 64, cy = b1;
                                 if (p.wgrad_taps > 0) {
                                     cx = n0 + c * 64;
@@ -554,7 +560,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             }
         }
     } else {
-        // ---------------- epilogue (warps 2..9) ----------------
+        // ---------------- epilogue (the EPI_WARPS warps from 2 on) ----------------
         if (p.ag_nranks > 1) {
             // all-gather prologue: the epilogue threads of every CTA copy their share of each peer's
             // shard into the local B buffer (plain 16-byte peer loads), in the order the k loop consumes
@@ -591,13 +597,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             }
         }
         const int q = warp & 3;  // TMEM lane quarter this warp may access
-        const int chalf = (warp - 2) >> 2;   // which 128 of the tile's 256 columns this warp drains
+        constexpr int PARTS = C::PARTS, PART_COLS = C::PART_COLS;
+        const int part = (warp - 2) >> 2;    // which columns of the tile this warp drains
         const int row_in_tile = q * 32 + lane;
+        const int first_tile = part < PARTS ? tile0 : p.num_tiles;
+        // activations and 16-bit matrices beside the output: not with eight warps and a 16-bit output (see dispatch)
+        constexpr bool OUT16 = sizeof(OutT) == 2, ACT = EPI_WARPS == 16 || !OUT16;
         const bool has_bias = p.flags & RB_GEMM_BIAS;
         const bool has_res = p.flags & RB_GEMM_RESIDUAL;
-        const bool act_gelu = p.flags & RB_GEMM_GELU;
-        const bool act_dgelu = p.flags & RB_GEMM_DGELU;
-        const bool aux_out = p.flags & RB_GEMM_AUX_OUT;
+        const bool act_gelu = ACT && (p.flags & RB_GEMM_GELU);
+        const bool act_dgelu = ACT && (p.flags & RB_GEMM_DGELU);
+        const bool aux_out = ACT && (p.flags & RB_GEMM_AUX_OUT);
         const bool accum = p.flags & RB_GEMM_ACCUM;
         const bool bias_al = p.bias_al, in_al = p.in_al, out_al = p.out_al;
         auto release_acc = [&](int acc) {
@@ -614,24 +624,39 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         };
         int it = 0;
         if (p.staged) {
-            // Bound by issue slots and the load / store unit: with K = 1024 a tile's main loop is some 8200 cycles,
-            // and a thread that stores (or loads) its own row makes every 16-byte access of its warp touch 32
-            // lines, 32 cycles each -- for two 16-bit outputs alone as long as the main loop.  Rows therefore go
-            // to the staging block (conflict-free by the swizzle) and the copy engine moves 32 x 32 blocks; it
-            // also clips them to M x N, adds fp32 blocks to D (accumulation, split K) and fetches the auxiliary
-            // block one step ahead.  16384 x 4096 x 1024 with bias, GELU and the value before it: 155 -> 142 us (137 with
-            // the packed arithmetic below); 8192 x 30528 x 1024: 426 -> 386 us; weight gradient 4096 x 1024 x 16384:
-            // 122 -> 116 us.  A block of 128 rows per four warps (a quarter of the copies, two barriers a block) was
-            // slower: 137 -> 142 us; so were coalesced 16-byte stores from the staging block: 139 -> 159 us.
+            // A thread that stores (or loads) its own row makes every 16-byte access of its warp touch 32 lines, 32 cycles
+            // each: for two 16-bit outputs alone as long as a main loop of K = 1024 (8200 cycles).  Rows therefore go to the
+            // staging block (conflict-free by the swizzle) and the copy engine moves 32 x 32 blocks; it also clips them to
+            // M x N, adds fp32 blocks to D (accumulation, split K) and fetches the auxiliary block one step ahead.
+            // 8192 x 30528 x 1024: 426 -> 386 us; weight gradient 4096 x 1024 x 16384: 122 -> 116 us.  Larger blocks (32 x
+            // 64, or 128 rows per four warps) hold up the loads for longer: GELU 131 -> 138 us, plain 108 -> 112.
+            //
+            // Sixteen warps for an activation: a block is a chain of tensor-memory load, bias, GELU (64 instructions of the
+            // special-function unit a thread), staging and copy, 2700 cycles long, and with two warps to a scheduler that
+            // is 11000 a tile, behind which the products of K = 1024 (8200) wait.  Four to a scheduler hide each other's
+            // latency: 16384 x 4096 x 1024 with GELU and second output 137 -> 121 us, GELU gradient 132 -> 123, 2000 x 3072
+            // x 768 with GELU and second output 21.7 -> 18.7.  Without an activation a block is short, and the extra warps
+            // only take turns with the one that issues the copies: 96.5 -> 100.4 with bias, fp32 sums 114 -> 122; those keep
+            // eight.  (GELU's value and the one before it share a block's place: the second is written once the first has
+            // left, which its arithmetic covers.)
             uint8_t* stage_buf = sEpi + (warp - 2) * EPI_STAGE_BYTES;
+            constexpr int SLOTS = EPI_STAGE_BYTES / (OUT16 ? 2048 : 4096);   // blocks the staging memory holds
             uint64_t* abar = &aux_full[warp - 2];
             uint32_t aux_phase = 0;
-            uint32_t turn = 0;   // which half the next 16-bit block takes: counted over tiles, whose blocks may be odd in number
+            uint32_t turn = 0;   // which slot the next block takes: counted over tiles, whose blocks may be odd in number
             const uint32_t sw64 = (lane >> 1) & 3, sw128 = lane & 7;
-            constexpr bool OUT16 = sizeof(OutT) == 2;
             const bool add_out = !OUT16 && (accum || p.partial);
+            // lays a row of 32 16-bit values out in a block
+            auto put_row = [&](uint8_t* block, const float (&v)[32], auto type) {
+                using T = decltype(type);
+#pragma unroll
+                for (int g = 0; g < 4; ++g)
+                    *reinterpret_cast<uint4*>(block + lane * 64 + ((g ^ sw64) << 4)) =
+                        make_uint4(pack2<T>(v[g * 8], v[g * 8 + 1]), pack2<T>(v[g * 8 + 2], v[g * 8 + 3]),
+                                   pack2<T>(v[g * 8 + 4], v[g * 8 + 5]), pack2<T>(v[g * 8 + 6], v[g * 8 + 7]));
+            };
             bool ok = true;
-            for (int tile = tile0; tile < p.num_tiles && ok; tile += tile_step) {
+            for (int tile = first_tile; tile < p.num_tiles && ok; tile += tile_step) {
                 int mb, nb, b, kb_begin, kb_end;
                 tile_coords(p, tile, mb, nb, b, kb_begin, kb_end);
                 if (kb_begin >= kb_end) continue;
@@ -639,26 +664,27 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                 const uint32_t acc_phase = (it >> 1) & 1;
                 ++it;
                 const int row0 = mb * TILE_M + static_cast<int>(crank) * BM + q * 32;
-                const int col0 = nb * BN + chalf * (BN / 2);
+                const int col0 = nb * BN + part * PART_COLS;
                 const bool row_ok = row0 + lane < p.M;
                 // blocks of this warp that hold part of the matrix
-                const int nblk = row0 < p.M ? max(0, min(BN / 64, (p.N - col0 + 31) / 32)) : 0;
-                auto fetch_aux = [&](int c) {
+                const int nblk = row0 < p.M ? max(0, min(PART_COLS / 32, (p.N - col0 + 31) / 32)) : 0;
+                auto fetch_aux = [&](int c) {   // (one lane; the block before has left its place)
+                    tma_store_wait_read<0>();
                     mbar_arrive_expect_tx(abar, 2048);
                     tma_load_3d(stage_buf, &tmAux, abar, col0 + c * 32, row0, b);
                 };
-                if (act_dgelu && nblk > 0 && lane == 0) fetch_aux(0);
+                if (OUT16 && act_dgelu && nblk > 0 && lane == 0) fetch_aux(0);
                 if (!mbar_wait_warp(&tfull[acc], acc_phase, abort_flag)) break;
                 tc_fence_after();
                 if (nblk == 0) release_acc(acc);
                 const long long row_off = static_cast<long long>(b) * p.strideD +
                                           static_cast<long long>(row_ok ? row0 + lane : 0) * p.ldd;
+                const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN + part * PART_COLS;
 #pragma unroll 1
                 for (int c = 0; c < nblk; ++c) {
                     const int col = col0 + c * 32;
                     uint32_t r[32];
-                    tmem_ld32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN + chalf * (BN / 2) + c * 32,
-                              r);
+                    tmem_ld32(t_acc + c * 32, r);
                     tmem_ld_wait();
                     if (c == nblk - 1) release_acc(acc);
                     const int valid = min(32, p.N - col);
@@ -667,7 +693,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     const uint64_t alpha2 = f2_pack(p.alpha, p.alpha);
                     if (has_bias) {
                         float t[32];
-                        load32(reinterpret_cast<const InT*>(p.bias) + col, full_chunk && bias_al, valid, t);
+                        load_n(reinterpret_cast<const InT*>(p.bias) + col, full_chunk && bias_al, valid, t);
 #pragma unroll
                         for (int j = 0; j < 32; j += 2)
                             f2_unpack(f2_fma(f2_pack_bits(r[j], r[j + 1]), alpha2, f2_pack(t[j], t[j + 1])), v[j], v[j + 1]);
@@ -676,75 +702,58 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         for (int j = 0; j < 32; j += 2)
                             f2_unpack(f2_mul(f2_pack_bits(r[j], r[j + 1]), alpha2), v[j], v[j + 1]);
                     }
-                    uint4 pre[4];   // the value before the activation, in storage precision
-                    if (aux_out) {
-#pragma unroll
-                        for (int g = 0; g < 4; ++g)
-                            pre[g] = make_uint4(pack2<InT>(v[g * 8], v[g * 8 + 1]), pack2<InT>(v[g * 8 + 2], v[g * 8 + 3]),
-                                                pack2<InT>(v[g * 8 + 4], v[g * 8 + 5]),
-                                                pack2<InT>(v[g * 8 + 6], v[g * 8 + 7]));
+                    // the block that is about to be overwritten has been read by the copy engine
+                    auto wait_slot = [&] {
+                        if (lane == 0) tma_store_wait_read<SLOTS - 1>();
+                        __syncwarp();
+                    };
+                    if (OUT16 && aux_out) {   // the value before the activation, in storage precision
+                        wait_slot();
+                        put_row(stage_buf, v, InT());
+                        fence_proxy_async();
+                        __syncwarp();
+                        if (lane == 0) {
+                            tma_store_3d(&tmAux, stage_buf, col, row0, b);
+                            tma_store_commit();
+                        }
                     }
                     if (act_gelu) {
 #pragma unroll
                         for (int j = 0; j < 32; j += 2) gelu_erf2(v[j], v[j + 1]);
                     }
-                    if (act_dgelu) {
+                    if (OUT16 && act_dgelu) {
                         if (!mbar_wait_warp(abar, aux_phase, abort_flag)) {
                             ok = false;
                             break;
                         }
                         aux_phase ^= 1;
-                        uint4 x[4];
-#pragma unroll
-                        for (int g = 0; g < 4; ++g)
-                            x[g] = *reinterpret_cast<const uint4*>(stage_buf + lane * 64 + ((g ^ sw64) << 4));
-                        __syncwarp();   // every lane has its row: the next block may land
-                        if (lane == 0 && c + 1 < nblk) fetch_aux(c + 1);
 #pragma unroll
                         for (int g = 0; g < 4; ++g) {
-                            const InT* e = reinterpret_cast<const InT*>(&x[g]);
+                            const uint4 x = *reinterpret_cast<const uint4*>(stage_buf + lane * 64 + ((g ^ sw64) << 4));
+                            const InT* e = reinterpret_cast<const InT*>(&x);
 #pragma unroll
                             for (int j = 0; j < 8; j += 2)
                                 gelu_erf_grad2(to_f32<InT>(e[j]), to_f32<InT>(e[j + 1]), v[g * 8 + j], v[g * 8 + j + 1]);
                         }
+                        __syncwarp();   // every lane has its row: the output takes its place
                     }
                     if (has_res && row_ok) {
                         float t[32];
-                        load32(reinterpret_cast<const InT*>(p.residual) + row_off + col, full_chunk && in_al, valid, t);
+                        load_n(reinterpret_cast<const InT*>(p.residual) + row_off + col, full_chunk && in_al, valid, t);
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[j] += t[j];
                     }
                     if (OUT16 && accum && row_ok) {
                         float t[32];
-                        load32(reinterpret_cast<const OutT*>(p.D) + row_off + col, full_chunk && out_al, valid, t);
+                        load_n(reinterpret_cast<const OutT*>(p.D) + row_off + col, full_chunk && out_al, valid, t);
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[j] += t[j];
                     }
-                    // the block that is about to be overwritten has been read by the copy engine: without an
-                    // auxiliary block the two halves of the staging memory take turns
-                    const bool two_slots = OUT16 && !aux_out && !act_dgelu;
-                    if (lane == 0) {
-                        if (two_slots)
-                            tma_store_wait_read<1>();
-                        else
-                            tma_store_wait_read<0>();
-                    }
-                    __syncwarp();
-                    uint8_t* dst = stage_buf;
+                    if (!(OUT16 && act_dgelu)) wait_slot();
+                    uint8_t* dst = stage_buf + (SLOTS > 1 && (turn & 1) ? 2048 : 0);
+                    ++turn;
                     if constexpr (OUT16) {
-                        if (!two_slots || (turn & 1)) dst += 2048;
-                        ++turn;
-#pragma unroll
-                        for (int g = 0; g < 4; ++g)
-                            *reinterpret_cast<uint4*>(dst + lane * 64 + ((g ^ sw64) << 4)) =
-                                make_uint4(pack2<OutT>(v[g * 8], v[g * 8 + 1]), pack2<OutT>(v[g * 8 + 2], v[g * 8 + 3]),
-                                           pack2<OutT>(v[g * 8 + 4], v[g * 8 + 5]),
-                                           pack2<OutT>(v[g * 8 + 6], v[g * 8 + 7]));
-                        if (aux_out) {
-#pragma unroll
-                            for (int g = 0; g < 4; ++g)
-                                *reinterpret_cast<uint4*>(stage_buf + lane * 64 + ((g ^ sw64) << 4)) = pre[g];
-                        }
+                        put_row(dst, v, OutT());
                     } else {
 #pragma unroll
                         for (int g = 0; g < 8; ++g)
@@ -754,19 +763,20 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     fence_proxy_async();
                     __syncwarp();
                     if (lane == 0) {
-                        if (aux_out) tma_store_3d(&tmAux, stage_buf, col, row0, b);
                         if (add_out)
                             tma_reduce_add_3d(&tmD, dst, col, row0, b);
                         else
                             tma_store_3d(&tmD, dst, col, row0, b);
                         tma_store_commit();
+                        if (OUT16 && act_dgelu && c + 1 < nblk) fetch_aux(c + 1);
                     }
                 }
             }
             // the staging memory must outlive the copies that read it; their writes are complete when the kernel is
             if (lane == 0) tma_store_wait_read<0>();
         }
-        for (int tile = p.staged ? p.num_tiles : tile0; tile < p.num_tiles; tile += tile_step) {
+        constexpr int DC = EPI_WARPS == 16 ? 16 : 32;   // columns at a time: sixteen warps leave a thread 96 registers
+        for (int tile = p.staged ? p.num_tiles : first_tile; tile < p.num_tiles; tile += tile_step) {
             int mb, nb, b, kb_begin, kb_end;
             tile_coords(p, tile, mb, nb, b, kb_begin, kb_end);
             if (kb_begin >= kb_end) continue;
@@ -790,18 +800,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             const long long row_off = static_cast<long long>(b) * p.strideD +
                                       static_cast<long long>(row_ok ? row : 0) * p.ldd;
 #pragma unroll 1
-            for (int c = chalf * (BN / 64); c < (chalf + 1) * (BN / 64); ++c) {
-                const int col = nb * BN + c * 32;
+            for (int c = part * (PART_COLS / DC); c < (part + 1) * (PART_COLS / DC); ++c) {
+                const int col = nb * BN + c * DC;
                 if (col >= p.N) break;
-                uint32_t r[32];
-                tmem_ld32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN + c * 32, r);
+                uint32_t r[DC];
+                tmem_ld(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN + c * DC, r);
                 tmem_ld_wait();
                 if (!row_ok) continue;
-                const int valid = min(32, p.N - col);
-                const bool full_chunk = valid == 32;
-                float v[32];
+                const int valid = min(DC, p.N - col);
+                const bool full_chunk = valid == DC;
+                float v[DC];
 #pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
+                for (int j = 0; j < DC; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
                 if constexpr (std::is_same<OutT, float>::value) {
                     if (p.partial || p.rs_nranks > 1) {
                         // partial sums (a K slice, and/or one replica's share of a reduce-scatter):
@@ -815,53 +825,53 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         }
                         if (full_chunk && out_al) {
 #pragma unroll
-                            for (int j = 0; j < 32; j += 4)
+                            for (int j = 0; j < DC; j += 4)
                                 asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dptr + j),
                                              "f"(v[j]), "f"(v[j + 1]), "f"(v[j + 2]), "f"(v[j + 3])
                                              : "memory");
                         } else {
 #pragma unroll
-                            for (int j = 0; j < 32; ++j)
+                            for (int j = 0; j < DC; ++j)
                                 if (j < valid) atomicAdd(dptr + j, v[j]);
                         }
                         continue;
                     }
                 }
                 if (has_bias) {
-                    float t[32];
-                    load32(reinterpret_cast<const InT*>(p.bias) + col, full_chunk && bias_al, valid, t);
+                    float t[DC];
+                    load_n(reinterpret_cast<const InT*>(p.bias) + col, full_chunk && bias_al, valid, t);
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] += t[j];
+                    for (int j = 0; j < DC; ++j) v[j] += t[j];
                 }
                 if (aux_out)
-                    store32(reinterpret_cast<InT*>(p.aux_out) + row_off + col, full_chunk && in_al,
+                    store_n(reinterpret_cast<InT*>(p.aux_out) + row_off + col, full_chunk && in_al,
                             valid, v);
                 if (act_gelu) {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
+                    for (int j = 0; j < DC; ++j) v[j] = gelu_erf(v[j]);
                 }
                 if (act_dgelu) {
-                    float t[32];
-                    load32(reinterpret_cast<const InT*>(p.aux_in) + row_off + col,
+                    float t[DC];
+                    load_n(reinterpret_cast<const InT*>(p.aux_in) + row_off + col,
                            full_chunk && in_al, valid, t);
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] *= gelu_erf_grad(t[j]);
+                    for (int j = 0; j < DC; ++j) v[j] *= gelu_erf_grad(t[j]);
                 }
                 if (has_res) {
-                    float t[32];
-                    load32(reinterpret_cast<const InT*>(p.residual) + row_off + col,
+                    float t[DC];
+                    load_n(reinterpret_cast<const InT*>(p.residual) + row_off + col,
                            full_chunk && in_al, valid, t);
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] += t[j];
+                    for (int j = 0; j < DC; ++j) v[j] += t[j];
                 }
                 OutT* dptr = reinterpret_cast<OutT*>(p.D) + row_off + col;
                 if (accum) {
-                    float t[32];
-                    load32(dptr, full_chunk && out_al, valid, t);
+                    float t[DC];
+                    load_n(dptr, full_chunk && out_al, valid, t);
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] += t[j];
+                    for (int j = 0; j < DC; ++j) v[j] += t[j];
                 }
-                store32(dptr, full_chunk && out_al, valid, v);
+                store_n(dptr, full_chunk && out_al, valid, v);
             }
             release_acc(acc);
         }
@@ -1021,11 +1031,11 @@ int num_sms() {
     return n[dev];
 }
 
-template <typename InT, typename OutT, bool PAIR, int TN>
+template <typename InT, typename OutT, bool PAIR, int TN, int EW>
 static int launch(const RbGemmArgs& a, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmD,
                   const CUtensorMap& tmAux, const GemmKernelParams& p, cudaStream_t stream) {
-    auto kern = gemm_tcgen05_kernel<InT, OutT, PAIR, TN>;
-    constexpr int smem = Cfg<PAIR, TN>::SMEM_BYTES;
+    auto kern = gemm_tcgen05_kernel<InT, OutT, PAIR, TN, EW>;
+    constexpr int smem = Cfg<PAIR, TN, EW>::SMEM_BYTES, GEMM_THREADS = Cfg<PAIR, TN, EW>::THREADS;
     static bool attr_set[64] = {false};
     static int max_clusters[64] = {0};
     int dev = 0;
@@ -1068,9 +1078,12 @@ static int launch(const RbGemmArgs& a, const CUtensorMap& tmA, const CUtensorMap
 template <typename InT>
 static int dispatch(const RbGemmArgs& a, bool pair, int tn, const CUtensorMap& tmA, const CUtensorMap& tmB,
                     const CUtensorMap& tmD, const CUtensorMap& tmAux, const GemmKernelParams& p, cudaStream_t st) {
-#define RB_GEMM_LAUNCH(PAIR, TN)                                                             \
-    return a.out_dtype == 0 ? launch<InT, InT, PAIR, TN>(a, tmA, tmB, tmD, tmAux, p, st) \
-                            : launch<InT, float, PAIR, TN>(a, tmA, tmB, tmD, tmAux, p, st)
+    // what the epilogue has to do decides on its warps; fp32 results with an activation are rare and stay on eight
+    const bool act = a.out_dtype == 0 && (a.flags & (RB_GEMM_GELU | RB_GEMM_DGELU | RB_GEMM_AUX_OUT));
+#define RB_GEMM_LAUNCH(PAIR, TN)                                                                \
+    return a.out_dtype == 1 ? launch<InT, float, PAIR, TN, 8>(a, tmA, tmB, tmD, tmAux, p, st) \
+           : act            ? launch<InT, InT, PAIR, TN, 16>(a, tmA, tmB, tmD, tmAux, p, st)  \
+                            : launch<InT, InT, PAIR, TN, 8>(a, tmA, tmB, tmD, tmAux, p, st)
     if (pair) RB_GEMM_LAUNCH(true, 256);
     if (tn == 64) RB_GEMM_LAUNCH(false, 64);
     if (tn == 128) RB_GEMM_LAUNCH(false, 128);
@@ -1390,9 +1403,8 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     if (rc) return rc;
 
     // The staged epilogue wants outputs the copy engine can address: plain rows in this GPU's memory, 16-byte
-    // aligned bases and row strides.  Its staging memory holds one fp32 block or two 16-bit ones, so an fp32
-    // output with an auxiliary matrix, or one that both reads and writes an auxiliary matrix, stays on the
-    // direct path, as do mapped rows (padded image grids) and peers' buffers (reduce-scatter).
+    // aligned bases and row strides.  Its staging blocks of an auxiliary matrix are 16-bit ones, so an fp32 output
+    // with one, or an output that both reads and writes an auxiliary matrix, stays on the direct path, as do mapped rows (padded image grids) and peers' buffers (reduce-scatter).
     CUtensorMap tmD = tmA, tmAux = tmA;
     const bool fp32_out = a->out_dtype == 1;
     const int64_t out_es = fp32_out ? 4 : 2;

@@ -316,6 +316,33 @@ def test_staged_blocks_of_many_tiles(dtype, N, tile_n, max_ctas):
     assert _lib.read_error() == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N,tile_n,max_ctas", [(160, 256, 2), (416, 0, 6), (96, 128, 2), (40, 64, 1), (200, 0, 0)])
+def test_activation_blocks_of_many_tiles(dtype, N, tile_n, max_ctas):
+    """Sixteen epilogue warps with one staging block each: the value before the activation, the one behind it and the
+    gradient's operand share the block's place, over many tiles.  The first is a small whole number and seen exactly; the
+    derivative of GELU at +-30 is exactly 1 or 0, so a foreign operand block is seen exactly too."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops.gemm import gemm
+
+    M, K = 128 * 300 + 5, 64
+    torch.manual_seed(9)
+    a = torch.zeros(M, K, device="cuda", dtype=dtype)
+    a[:, :8] = torch.randint(-3, 4, (M, 8), device="cuda").to(dtype)
+    b = torch.randint(-3, 4, (N, K), device="cuda").to(dtype)
+    z = a.float() @ b.float().t()
+    aux = torch.where(torch.rand(M, N, device="cuda") < 0.5, 30.0, -30.0).to(dtype)
+    for _ in range(3):
+        pre = torch.empty(M, N, device="cuda", dtype=dtype)
+        y = gemm(a, b, gelu=True, aux_out=pre, tile_n=tile_n, max_ctas=max_ctas)
+        assert torch.equal(pre, z.to(dtype))
+        _near(y, torch.nn.functional.gelu(z.double()), dtype, 1)
+        got = gemm(a, b, dgelu=True, aux_in=aux, tile_n=tile_n, max_ctas=max_ctas)
+        assert torch.equal(got, torch.where(aux > 0, z, torch.zeros_like(z)).to(dtype))
+    torch.cuda.synchronize()
+    assert _lib.read_error() == 0
+
+
 # 74 pairs of SMs and 76 (2 left over), 111 (37), 112 (38: two rounds of helpers), 124 (50: three), 136 (62: six), 147 (73)
 # and 150 (2) tiles; in `how` many parts the last wave is summed: see ops.gemm.last_wave
 @pytest.mark.parametrize("M,N,K,how", [
