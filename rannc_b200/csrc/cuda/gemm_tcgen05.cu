@@ -107,7 +107,40 @@ struct GemmKernelParams {
     // 1: the bias / the matrices beside the output / the output start their rows on 16-byte boundaries
     int bias_al, in_al, out_al;
     float* a_colsum;   // not null: column sums of the stored A (MN-major) are added here
+    const int* rows_ctl;   // see RbGemmArgs
+    int rows_mode;
 };
+
+// A product whose rows were gathered on the device (RbGemmArgs::rows_ctl): how many there are, and whether this form of the
+// product is the one in use, is read here.  (The host cannot choose: it does not wait for the device.)
+constexpr int ROWS_DRAIN_STEPS = 6;   // what a part costs besides its own steps (as DRAIN_STEPS below)
+__device__ __forceinline__ void apply_rows(GemmKernelParams& p, int units) {
+    const int count = p.rows_ctl[0], gathered = p.rows_ctl[1];
+    if ((p.rows_mode != RB_GEMM_ROWS_ALL) != (gathered != 0)) {
+        p.num_tiles = 0;   // the other form runs
+        return;
+    }
+    if (p.rows_mode == RB_GEMM_ROWS_K) {
+        // rows up to the next whole step are zero; whole tiles, as for any short K
+        p.num_kb = (count + BK - 1) / BK;
+        p.kb_per_split = p.num_kb;
+        p.tail_tiles = 0;
+        p.num_tiles = p.base_tiles;
+    } else if (p.rows_mode == RB_GEMM_ROWS_M) {
+        // one more row, of zeros: its product stands for every row that was left out
+        p.num_m_blocks = (count + 1 + 2 * BM - 1) / (2 * BM);
+        p.base_tiles = p.num_m_blocks * p.num_n_blocks;
+        // few tiles and a long K (the layer's outputs): parts whose waves take the fewest steps, each with its drain
+        int split = 1, best = 0x7fffffff;
+        for (int s = 1; s <= 16 && s * 4 <= p.num_kb; ++s) {
+            const int cost = (p.base_tiles * s + units - 1) / units * ((p.num_kb + s - 1) / s + ROWS_DRAIN_STEPS);
+            if (cost < best) best = cost, split = s;
+        }
+        p.kb_per_split = (p.num_kb + split - 1) / split;
+        p.split_k = (p.num_kb + p.kb_per_split - 1) / p.kb_per_split;
+        p.num_tiles = p.base_tiles * p.split_k;
+    }
+}
 
 __device__ __forceinline__ void tile_coords(const GemmKernelParams& p, int tile, int& mb, int& nb,
                                             int& b, int& kb_begin, int& kb_end) {
@@ -212,12 +245,13 @@ __device__ __forceinline__ void store_n(T* ptr, bool vec_ok, int valid, const fl
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
 
-template <typename InT, typename OutT, bool PAIR, int BN, int EPI_WARPS>
+// ROWS: the sizes are completed by apply_rows
+template <typename InT, typename OutT, bool PAIR, int BN, int EPI_WARPS, bool ROWS>
 __global__ void __launch_bounds__(Cfg<PAIR, BN, EPI_WARPS>::THREADS, 1)
     gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
                         const __grid_constant__ CUtensorMap tmB,
                         const __grid_constant__ CUtensorMap tmD,
-                        const __grid_constant__ CUtensorMap tmAux, const GemmKernelParams p) {
+                        const __grid_constant__ CUtensorMap tmAux, const GemmKernelParams params) {
     using C = Cfg<PAIR, BN, EPI_WARPS>;
     constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES, B_STAGE_BYTES = C::B_STAGE_BYTES;
     constexpr int TILE_M = C::TILE_M, TMEM_COLS = C::TMEM_COLS;
@@ -246,10 +280,11 @@ __global__ void __launch_bounds__(Cfg<PAIR, BN, EPI_WARPS>::THREADS, 1)
     const int tile0 = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
     const int tile_step = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
 
+    __shared__ std::conditional_t<ROWS, GemmKernelParams, char> s_params;
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], p.a_colsum ? SUM_WARPS : 1);
+            mbar_init(&empty[s], params.a_colsum ? SUM_WARPS : 1);
             mbar_init(&used[s], 1);
         }
         for (int a = 0; a < 2; ++a) {
@@ -261,9 +296,9 @@ __global__ void __launch_bounds__(Cfg<PAIR, BN, EPI_WARPS>::THREADS, 1)
         fence_mbar_init();
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
-        if (p.staged) {
+        if (params.staged) {
             tma_prefetch_desc(&tmD);
-            if (p.flags & (RB_GEMM_AUX_OUT | RB_GEMM_DGELU)) tma_prefetch_desc(&tmAux);
+            if (params.flags & (RB_GEMM_AUX_OUT | RB_GEMM_DGELU)) tma_prefetch_desc(&tmAux);
         }
     }
     if (warp == 2) {
@@ -282,6 +317,19 @@ __global__ void __launch_bounds__(Cfg<PAIR, BN, EPI_WARPS>::THREADS, 1)
     const uint32_t tmem_base = *tmem_slot;
     grid_trigger();
     grid_wait();   // all of the above runs beside the end of the kernel before
+    if constexpr (ROWS) {
+        if (threadIdx.x == 0) {
+            s_params = params;
+            apply_rows(s_params, tile_step);
+        }
+        __syncthreads();
+    }
+    const GemmKernelParams& p = [&]() -> const GemmKernelParams& {
+        if constexpr (ROWS)
+            return s_params;
+        else
+            return params;
+    }();
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
@@ -881,7 +929,7 @@ __global__ void __launch_bounds__(Cfg<PAIR, BN, EPI_WARPS>::THREADS, 1)
     __syncthreads();
     if (*abort_flag) {
         if (threadIdx.x == 0) {
-            atomicExch(p.err, ERR_MBAR_TIMEOUT);
+            atomicExch(params.err, ERR_MBAR_TIMEOUT);
             // let bulk copies that may still be in flight land before the CTA's
             // shared memory is released
             const long long t0 = clock64();
@@ -1031,10 +1079,10 @@ int num_sms() {
     return n[dev];
 }
 
-template <typename InT, typename OutT, bool PAIR, int TN, int EW>
+template <typename InT, typename OutT, bool PAIR, int TN, int EW, bool ROWS = false>
 static int launch(const RbGemmArgs& a, const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmD,
                   const CUtensorMap& tmAux, const GemmKernelParams& p, cudaStream_t stream) {
-    auto kern = gemm_tcgen05_kernel<InT, OutT, PAIR, TN, EW>;
+    auto kern = gemm_tcgen05_kernel<InT, OutT, PAIR, TN, EW, ROWS>;
     constexpr int smem = Cfg<PAIR, TN, EW>::SMEM_BYTES, GEMM_THREADS = Cfg<PAIR, TN, EW>::THREADS;
     static bool attr_set[64] = {false};
     static int max_clusters[64] = {0};
@@ -1069,7 +1117,7 @@ static int launch(const RbGemmArgs& a, const CUtensorMap& tmA, const CUtensorMap
         if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) n = num_sms() / 2;
         max_clusters[dev & 63] = n;
     }
-    int clusters = p.num_tiles < max_clusters[dev & 63] ? p.num_tiles : max_clusters[dev & 63];
+    int clusters = !ROWS && p.num_tiles < max_clusters[dev & 63] ? p.num_tiles : max_clusters[dev & 63];
     if (a.max_ctas > 1 && clusters > a.max_ctas / 2) clusters = a.max_ctas / 2;
     const cudaError_t e = launch_after_clusters(kern, 2, 2 * clusters, GEMM_THREADS, smem, stream, tmA, tmB, tmD, tmAux, p);
     return e == cudaSuccess ? 0 : -static_cast<int>(e);
@@ -1084,6 +1132,9 @@ static int dispatch(const RbGemmArgs& a, bool pair, int tn, const CUtensorMap& t
     return a.out_dtype == 1 ? launch<InT, float, PAIR, TN, 8>(a, tmA, tmB, tmD, tmAux, p, st) \
            : act            ? launch<InT, InT, PAIR, TN, 16>(a, tmA, tmB, tmD, tmAux, p, st)  \
                             : launch<InT, InT, PAIR, TN, 8>(a, tmA, tmB, tmD, tmAux, p, st)
+    if (a.rows_ctl)
+        return a.out_dtype == 1 ? launch<InT, float, true, 256, 8, true>(a, tmA, tmB, tmD, tmAux, p, st)
+                                : launch<InT, InT, true, 256, 8, true>(a, tmA, tmB, tmD, tmAux, p, st);
     if (pair) RB_GEMM_LAUNCH(true, 256);
     if (tn == 64) RB_GEMM_LAUNCH(false, 64);
     if (tn == 128) RB_GEMM_LAUNCH(false, 128);
@@ -1172,8 +1223,8 @@ static Tiling choose_tiling(const RbGemmArgs& a) {
     // scatter epilogue are the same code in both variants.  Small problems stay on the single-CTA kernel.
     const bool accum32 = a.out_dtype == 1 && a.flags == RB_GEMM_ACCUM;
     Tiling t;
-    t.pair = pair_enabled() && (a.ag_nranks <= 1 || pair_gather_enabled());
-    if (t.pair) {
+    t.pair = a.rows_ctl || (pair_enabled() && (a.ag_nranks <= 1 || pair_gather_enabled()));
+    if (t.pair && !a.rows_ctl) {
         const long long pt = ((a.M + 2 * BM - 1) / (2 * BM)) * ((a.N + 255) / 256) * a.batch;
         const long long kbs = (a.K + BK - 1) / BK;
         if (pt < num_sms() / 2 && !(accum32 && a.M > BM && pt * (kbs / 4) >= num_sms() / 2)) t.pair = false;
@@ -1342,6 +1393,17 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
         for (int t = 0; t < a->conv_taps; ++t) p.conv_shift[t] = a->conv_shift[t];
     }
     p.a_colsum = a->a_colsum;
+    p.rows_ctl = a->rows_ctl;
+    p.rows_mode = a->rows_mode;
+    if (a->rows_ctl) {
+        // plain products of one matrix; what is gathered along K or M is cut into whole tiles (ROWS_M: of sums)
+        if (a->batch != 1 || a->ag_nranks > 1 || a->rs_nranks > 1 || a->conv_taps > 0 || a->wgrad_taps > 0 || a->map_hp > 0 ||
+            (a->flags & ~RB_GEMM_ACCUM) || a->rows_mode < RB_GEMM_ROWS_ALL || a->rows_mode > RB_GEMM_ROWS_M ||
+            (a->rows_mode == RB_GEMM_ROWS_K && p.split_k > 1) ||
+            (a->rows_mode == RB_GEMM_ROWS_M && (a->a_major != 0 || a->out_dtype != 1 || a->flags != RB_GEMM_ACCUM)))
+            return -10;
+        if (a->rows_mode == RB_GEMM_ROWS_M) p.tail_tiles = 0, p.partial = 1;
+    }
     if (a->a_colsum && (a->a_major != 1 || a->batch != 1 || a->ag_nranks > 1)) return -8;
     p.wgrad_taps = 0;
     p.wgrad_cols = 1;

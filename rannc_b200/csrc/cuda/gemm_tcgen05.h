@@ -65,7 +65,17 @@ typedef struct RbGemmArgs {
     // wave of a product that is added to an fp32 matrix may be shared out, and its parts are added in the order they
     // arrive.  Fewer tiles have K split either way (rb_gemm_splits).
     int32_t in_order;
+    // products over rows that were gathered on the device (null: an ordinary product).  rows_ctl points to two integers in
+    // device memory: the number of gathered rows and whether they are to be used (sparse_rows.h).  rows_mode says which form
+    // of the product this is; the form that is not in use does nothing.
+    //  RB_GEMM_ROWS_ALL: the product over all rows
+    //  RB_GEMM_ROWS_K: K is the number of gathered rows (K here: room for them; those up to the next multiple of 64 are zero)
+    //  RB_GEMM_ROWS_M: M is that number plus one (M here: room for them); results are added to an fp32 matrix, in parts
+    const int32_t* rows_ctl;
+    int32_t rows_mode;
 } RbGemmArgs;
+
+enum { RB_GEMM_ROWS_ALL = 1, RB_GEMM_ROWS_K = 2, RB_GEMM_ROWS_M = 3 };
 
 // returns 0 on success, <0 on a host-side error (-2: operand not 16 B aligned)
 int rb_gemm(const RbGemmArgs* args, void* stream);

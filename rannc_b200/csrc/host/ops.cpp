@@ -25,6 +25,7 @@
 
 #include "../cuda/attn.h"
 #include "../cuda/gemm_tcgen05.h"
+#include "../cuda/sparse_rows.h"
 
 namespace {
 
@@ -60,6 +61,9 @@ struct Api {
                   long long, int, float, float, int, int, void*);
     int (*bn_bwd)(const void*, const void*, const void*, const float*, const float*, const float*, float*, float*, float*,
                   void*, void*, long long, int, int, int, void*);
+    decltype(&rb_rows_plan) rows_plan;
+    decltype(&rb_rows_gather) rows_gather;
+    decltype(&rb_rows_scatter) rows_scatter;
 } api;
 std::atomic<long long> launches{0};
 PyObject* error_class = nullptr;   // ops._lib.KernelLibraryError
@@ -177,6 +181,8 @@ struct Epi {
     void* aux_out = nullptr;
     bool gelu = false, dgelu = false, accumulate = false;
     float* a_colsum = nullptr;   // the column sums of a stored [K, M] are added here
+    const int32_t* rows_ctl = nullptr;   // see RbGemmArgs
+    int rows_mode = 0;
 };
 // out [M, N] = epilogue(op(a) op(b)), rows ldd apart (0: N)
 void gemm(const Mat& a, const Mat& b, bool trans_a, bool trans_b, void* out, bool out_fp32, int dtype, const Epi& e,
@@ -206,9 +212,61 @@ void gemm(const Mat& a, const Mat& b, bool trans_a, bool trans_b, void* out, boo
               (e.accumulate ? RB_GEMM_ACCUM : 0) | (e.aux_out ? RB_GEMM_AUX_OUT : 0);
     g.alpha = 1.f;
     g.a_colsum = e.a_colsum;
+    g.rows_ctl = e.rows_ctl;
+    g.rows_mode = e.rows_mode;
     g.in_order = at::globalContext().deterministicAlgorithms() ? 1 : 0;
     check(api.gemm(&g, cur_stream()), "rb_gemm");
 }
+// ---- rows of zeros in the gradient of a wide output layer (cuda/sparse_rows.cu) ----
+// The rows that count are gathered on the device, and each product is launched in two forms of which the device runs one.
+struct Rows {
+    Tensor idx, pos, ctl, dy, x, dx32;
+    Mat dym, xm;
+    int64_t room = 0;
+    const int32_t* ctl_ptr() const { return static_cast<const int32_t*>(ctl.data_ptr()); }
+};
+// Worth a look at the rows: a wide output layer (the rows of hidden layers' gradients are not zero), and products long enough
+// that the look costs next to nothing where every row counts.  Backward of the layer (us), one B200, over all rows ->
+// gathered, by the share of rows that count (up to three quarters are gathered):
+//     rows x inputs x outputs     2 %          15 %         30 %         45 %         60 %         80 %         100 %
+//     8192 x 1024 x 30528         633 -> 205   643 -> 281   660 -> 395   685 -> 520   701 -> 662   743 -> 748   735 -> 738
+//     6144 x 1024 x 30528         554 -> 180   556 -> 229   564 -> 311   615 -> 414   620 -> 509   603 -> 637   613 -> 618
+//     4096 x  768 x 30528         363 -> 149   320 -> 162   320 -> 200   321 -> 241   323 -> 291   326 -> 352   326 -> 328
+// Rows of zeros are read to find them (425 MB at 15 % of 8192 x 30528: 81 us), which is lost where a few rows more than
+// three quarters count: 8 % of the backward at worst.  Both products use the kernel of CTA pairs whichever form runs, so an
+// input gradient of fewer tiles than two thirds of the pairs stays out (2048 x 1024 x 30528, where all rows count: 235 ->
+// 281; 1024 x 1024 x 30528 gains at 15 %, 181 -> 132, and loses at 100 %, 189 -> 238).
+bool worth_gathering(const Mat& dy, const Mat& x) {
+    auto tiles = [](int64_t m, int64_t n) { return (m + 255) / 256 * ((n + 255) / 256); };
+    return dy.cols >= 4 * x.cols && dy.cols % 8 == 0 && x.cols % 8 == 0 && dy.cols <= (1 << 22) && dy.rows < (1 << 30) &&
+           tiles(dy.cols, x.cols) >= 74 && tiles(dy.rows, x.cols) >= 48 &&
+           static_cast<double>(dy.rows) * dy.cols * x.cols >= 9e10 && !at::globalContext().deterministicAlgorithms();
+}
+// (empty `ctl`: the call is not one for this)
+Rows gather_rows(const Mat& dy, const Mat& x, bool want_dx, int dtype, const at::TensorOptions& o) {
+    Rows r;
+    if (!worth_gathering(dy, x)) return r;
+    r.room = std::min<int64_t>(dy.rows / 4 * 3, (int64_t{1} << 30) / dy.cols) / 64 * 64;   // (2 GiB at most)
+    const auto ints = o.dtype(at::kInt);
+    r.ctl = at::empty({2}, ints);
+    r.idx = at::empty({r.room}, ints);
+    r.pos = at::empty({dy.rows}, ints);
+    const Tensor live = at::empty({dy.rows}, o.dtype(at::kByte));
+    r.dy = at::empty({r.room, dy.cols}, o);
+    r.x = at::empty({r.room, x.cols}, o);
+    if (want_dx) r.dx32 = at::empty({r.room, x.cols}, o.dtype(at::kFloat));
+    check(api.rows_plan(dy.p, dy.ld, x.p, x.ld, static_cast<int>(dy.rows), static_cast<int>(dy.cols), static_cast<int>(x.cols),
+                        static_cast<int>(r.room), mptr<uint8_t>(live), mptr<int32_t>(r.idx), mptr<int32_t>(r.pos),
+                        mptr<int32_t>(r.ctl), dtype, cur_stream()),
+          "rb_rows_plan", 2);
+    check(api.rows_gather(dy.p, dy.ld, x.p, x.ld, static_cast<int>(dy.cols), static_cast<int>(x.cols), mptr<int32_t>(r.idx),
+                          r.ctl_ptr(), r.dy.data_ptr(), r.x.data_ptr(), mptr<float>(r.dx32), cur_stream()),
+          "rb_rows_gather");
+    r.dym = rows_of(r.dy);
+    r.xm = rows_of(r.x);
+    return r;
+}
+
 // Gradients of one weight and its bias: dW = dy^T x and, from the same pass over dy, db = its column sums.  Each is added
 // to the fp32 buffer the parameter has, or returned in the parameter's own type.
 struct Grads {
@@ -227,8 +285,18 @@ bool in_parts(int64_t m, int64_t n, int64_t rows) {
            !at::globalContext().deterministicAlgorithms() && api.gemm_splits(m, n, rows) > 1;
 }
 Grads param_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& w_mg, bool want_w, const Tensor& bias,
-                  const Tensor& b_mg, bool want_b, int dtype) {
+                  const Tensor& b_mg, bool want_b, int dtype, const Rows* rows = nullptr) {
     Grads out;
+    // dW = dy^T x, over all rows or (whichever the device finds) over the gathered ones
+    auto product = [&](void* to, bool fp32, Epi e, int64_t ldd) {
+        if (rows) {
+            e.rows_ctl = rows->ctl_ptr();
+            e.rows_mode = RB_GEMM_ROWS_K;
+            gemm(rows->dym, rows->xm, true, false, to, fp32, dtype, e, ldd);
+            e.rows_mode = RB_GEMM_ROWS_ALL;
+        }
+        gemm(dy, x, true, false, to, fp32, dtype, e, ldd);
+    };
     Tensor db;
     if (bias.defined() && want_b) db = b_mg.defined() ? b_mg : at::zeros({dy.cols}, bias.options().dtype(at::kFloat));
     if (want_w) {
@@ -236,7 +304,7 @@ Grads param_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& w_
         e.a_colsum = mptr<float>(db);
         if (w_mg.defined()) {
             e.accumulate = true;
-            gemm(dy, x, true, false, w_mg.data_ptr(), w_mg.scalar_type() == at::kFloat, dtype, e, w_mg.stride(0));
+            product(w_mg.data_ptr(), w_mg.scalar_type() == at::kFloat, e, w_mg.stride(0));
         } else if (in_parts(dy.cols, x.cols, dy.rows)) {
             Tensor w32 = at::zeros({dy.cols, x.cols}, w.options().dtype(at::kFloat));
             e.accumulate = true;
@@ -244,7 +312,7 @@ Grads param_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& w_
             out.w = w32.to(w.scalar_type());
         } else {
             out.w = at::empty({dy.cols, x.cols}, w.options());
-            gemm(dy, x, true, false, out.w.data_ptr(), false, dtype, e);
+            product(out.w.data_ptr(), false, e, 0);
         }
     } else if (db.defined()) {
         check(api.colsum(dy.p, mptr<float>(db), static_cast<int>(dy.rows), static_cast<int>(dy.cols), dy.ld, dtype,
@@ -340,14 +408,31 @@ struct LinearNode : Node {
             check(api.gelu(P.data_ptr(), dy.data_ptr(), d.data_ptr(), d.numel(), 1, dt, cur_stream()), "rb_gelu");
             dy = d;
         }
-        const Mat d = rows_of(dy);
+        const Mat d = rows_of(dy), xm = rows_of(X);
+        const bool want_dx = task_should_compute_output(0), want_w = task_should_compute_output(1);
+        Rows rows;
+        if (!P.defined() && (want_dx || want_w)) rows = gather_rows(d, xm, want_dx, dt, X.options());
+        const bool look = rows.ctl.defined();
         Tensor dx;
-        if (task_should_compute_output(0)) {
+        if (want_dx) {
             dx = at::empty(X.sizes(), X.options());
-            gemm(d, mat(W), false, false, dx.data_ptr(), false, dt, Epi());
+            const Mat wm = mat(W);
+            Epi e;
+            if (look) {
+                e.rows_ctl = rows.ctl_ptr();
+                e.rows_mode = RB_GEMM_ROWS_M;
+                e.accumulate = true;
+                gemm(rows.dym, wm, false, false, rows.dx32.data_ptr(), true, dt, e);
+                check(api.rows_scatter(mptr<float>(rows.dx32), dx.data_ptr(), static_cast<int>(d.rows),
+                                       static_cast<int>(xm.cols), mptr<int32_t>(rows.pos), rows.ctl_ptr(), dt, cur_stream()),
+                      "rb_rows_scatter");
+                e.rows_mode = RB_GEMM_ROWS_ALL;
+                e.accumulate = false;
+            }
+            gemm(d, wm, false, false, dx.data_ptr(), false, dt, e);
         }
-        const Grads gr = param_grads(d, rows_of(X), W, w_mg, task_should_compute_output(1), bias, b_mg,
-                                     bias.defined() && task_should_compute_output(2), dt);
+        const Grads gr = param_grads(d, xm, W, w_mg, want_w, bias, b_mg, bias.defined() && task_should_compute_output(2), dt,
+                                     look ? &rows : nullptr);
         notify({{&w_ref, &w_mg}, {&bias, &b_mg}});
         return {dx, gr.w, gr.b};
     }
@@ -1041,6 +1126,9 @@ void init(const std::unordered_map<std::string, uintptr_t>& fns, py::object erro
     set(api.attn_bwd, "rb_attn_bwd");
     set(api.bn_fwd, "rb_bn_fwd");
     set(api.bn_bwd, "rb_bn_bwd");
+    set(api.rows_plan, "rb_rows_plan");
+    set(api.rows_gather, "rb_rows_gather");
+    set(api.rows_scatter, "rb_rows_scatter");
     error_class = error.release().ptr();
 }
 void set_listener(py::object fn) {

@@ -1,0 +1,134 @@
+"""Backward of a wide output layer whose gradient has rows of zeros: found, gathered and put back on the device."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _plan(dy, x, room):
+    from rannc_b200.ops import _lib
+
+    R = dy.shape[0]
+    i32 = dict(dtype=torch.int32, device="cuda")
+    live, idx, pos, ctl = torch.empty(R, dtype=torch.uint8, device="cuda"), torch.full((room,), -7, **i32), \
+        torch.full((R,), -7, **i32), torch.empty(2, **i32)
+    code = 1 if dy.dtype == torch.bfloat16 else 0
+    L = ctypes.c_longlong
+    rc = _lib.lib().rb_rows_plan(_lib.vp(dy), L(dy.stride(0)), _lib.vp(x), L(x.stride(0)), R, dy.shape[1], x.shape[1], room,
+                                 _lib.vp(live), _lib.vp(idx), _lib.vp(pos), _lib.vp(ctl), code, _lib.stream_ptr())
+    assert rc == 0
+    return idx, pos, ctl
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("R,V,H,room,count", [
+    (1, 8, 8, 64, 1), (7, 264, 8, 64, 0), (130, 1304, 72, 64, 63), (130, 1304, 72, 64, 64), (1500, 264, 40, 1024, 1023),
+    (3001, 1288, 264, 1024, 700), (5000, 520, 16, 4096, 5000)])
+def test_rows_are_found_gathered_and_put_back(dtype, R, V, H, room, count):
+    """Numbers of rows on both sides of a block, of the room and of a padded step; a row whose only value is its last; the
+    matrix a slice of a wider one; a row of zeros whose input is not finite."""
+    from rannc_b200.ops import _lib
+
+    torch.manual_seed(R + count)
+    wide = torch.randn(R, V + 16, device="cuda").to(dtype)
+    dy, x = wide[:, 8:8 + V], torch.randn(R, H, device="cuda").to(dtype)
+    on = torch.zeros(R, dtype=torch.bool, device="cuda")
+    on[torch.randperm(R, device="cuda")[:count]] = True
+    dy[~on] = 0
+    rows = on.nonzero().flatten()
+    if count > 2:
+        dy[rows[0], :-1] = 0
+        dy[rows[1]] = 0
+        x[rows[1], H - 1] = float("nan")
+        dy[rows[2]] = 0
+        x[rows[2], 0] = float("-inf")
+    idx, pos, ctl = _plan(dy, x, room)
+    use = 0 < count < room
+    assert ctl.tolist() == [count, int(use)]
+    L = ctypes.c_longlong
+    dyc, xc = torch.full((room, V), 3.0, device="cuda", dtype=dtype), torch.full((room, H), 3.0, device="cuda", dtype=dtype)
+    d32 = torch.full((room, H), 3.0, device="cuda")
+    assert _lib.lib().rb_rows_gather(_lib.vp(dy), L(dy.stride(0)), _lib.vp(x), L(H), V, H, _lib.vp(idx), _lib.vp(ctl),
+                                     _lib.vp(dyc), _lib.vp(xc), _lib.vp(d32), _lib.stream_ptr()) == 0
+    out = torch.full((R, H), 5.0, device="cuda", dtype=dtype)
+    if use:
+        assert torch.equal(idx[:count].long(), rows)
+        want = torch.full((R,), -1, device="cuda")
+        want[rows] = torch.arange(count, device="cuda")
+        assert torch.equal(pos.long(), want)
+        pad = (count + 64) // 64 * 64
+        assert torch.equal(dyc[:count], dy[rows]) and torch.equal(xc[:count].nan_to_num(9.0), x[rows].nan_to_num(9.0))
+        assert (dyc[count:pad] == 0).all() and (xc[count:pad] == 0).all() and (d32[:count + 1] == 0).all()
+        assert (dyc[pad:] == 3.0).all() and (xc[pad:] == 3.0).all() and (d32[count + 1:] == 3.0).all()
+        d32[:count + 1] = torch.randn(count + 1, H, device="cuda")
+    assert _lib.lib().rb_rows_scatter(_lib.vp(d32), _lib.vp(out), R, H, _lib.vp(pos), _lib.vp(ctl),
+                                      1 if dtype == torch.bfloat16 else 0, _lib.stream_ptr()) == 0
+    if use:
+        want = d32[count].to(dtype).expand(R, H).clone()
+        want[rows] = d32[:count].to(dtype)
+        assert torch.equal(out, want)
+    else:
+        assert (out == 5.0).all() and (dyc == 3.0).all() and (d32 == 3.0).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("share", [0.0, 0.0003, 0.15, 0.749, 0.9, 1.0])
+@pytest.mark.parametrize("flat", [True, False])
+def test_wide_layer_backward(dtype, share, flat):
+    """Gradients against fp64, whichever form runs, at the smallest size that looks at the rows; sums added to what is there."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops import functional as RF
+
+    R, H, V = 4099, 776, 28680
+    torch.manual_seed(7)
+    x = torch.randn(R, H, device="cuda").to(dtype).requires_grad_(True)
+    w = (torch.randn(V, H, device="cuda") * 0.05).to(dtype).requires_grad_(True)
+    b = torch.randn(V, device="cuda").to(dtype).requires_grad_(True)
+    if flat:
+        w.main_grad, b.main_grad = torch.full((V, H), 2.0, device="cuda"), torch.full((V,), -1.0, device="cuda")
+    dy = torch.randn(R, V, device="cuda").to(dtype)
+    on = torch.rand(R, device="cuda") < share
+    on[-1] = share > 0
+    dy[~on] = 0
+    RF.linear(x, w, b).backward(dy)
+    torch.cuda.synchronize()
+    assert _lib.read_error() == 0
+    gw, gb = (w.main_grad - 2.0, b.main_grad + 1.0) if flat else (w.grad, b.grad)
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    n = int(on.sum())
+    for got, want, terms, rounded in ((x.grad, dy.double() @ w.detach().double(), V, True),
+                                      (gw, dy.double().t() @ x.detach().double(), n, not flat), (gb, dy.double().sum(0), n, not flat)):
+        # one rounding of the result, a sum in steps of 16 terms that may lose 2^-23 of the running sum each, and (sums that
+        # start at 2) the rounding of the sum so far
+        bound = (u if rounded else 0.0) * want.abs() + (1e-5 + terms / 16 * 2.0 ** -23) * want.abs().max() + 1e-6
+        assert ((got.double() - want).abs() <= bound).all()
+    assert (x.grad[~on] == 0).all()
+
+
+def test_infinities_and_nan_reach_the_gradients_of_rows_of_zeros():
+    """0 * inf is NaN: a weight that is not finite shows in its column of every row's gradient, an input that is not finite in
+    its column of the weight's, as in the product over all rows."""
+    from rannc_b200.ops import functional as RF
+
+    R, H, V = 4096, 768, 30528
+    torch.manual_seed(8)
+    x, w, dy = (torch.randn(*s, device="cuda").bfloat16() for s in ((R, H), (V, H), (R, V)))
+    dy[100:] = 0
+    w[17, 5], w[400, 9] = float("inf"), float("nan")
+    x[4000, 11] = float("inf")
+    got = {}
+    for all_rows in (False, True):
+        xg, wg = x.clone().requires_grad_(True), w.clone().requires_grad_(True)
+        y = RF.linear(xg, wg)
+        torch.use_deterministic_algorithms(all_rows)     # (its products go over all rows)
+        try:
+            y.backward(dy)
+        finally:
+            torch.use_deterministic_algorithms(False)
+        got[all_rows] = (xg.grad, wg.grad)
+    for a, b in zip(got[False], got[True]):
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+    assert got[False][0][200].isnan().nonzero().flatten().tolist() == [5, 9]
+    assert got[False][1][:, 11].isnan().all() and not got[False][1][:, 12].isnan().any()
