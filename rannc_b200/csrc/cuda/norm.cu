@@ -276,10 +276,12 @@ __global__ void __launch_bounds__(LN_THREADS, 2)
             for (int j = 0; j < 8; ++j) o[j] = rstd * (d[j] * g[j] - s1 - (zz[j] - mean) * rstd * s2);
             *reinterpret_cast<uint4*>(dz_out + base + col) = pack8(o, static_cast<const T*>(nullptr));
             if (dx_out) {
-                bool k[8];
-                keep8(seed, offset, base + col, thr, k);
+                if (thr) {
+                    bool k[8];
+                    keep8(seed, offset, base + col, thr, k);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) o[j] = k[j] ? o[j] * scale : 0.f;
+                    for (int j = 0; j < 8; ++j) o[j] = k[j] ? o[j] * scale : 0.f;
+                }
                 *reinterpret_cast<uint4*>(dx_out + base + col) = pack8(o, static_cast<const T*>(nullptr));
             }
         }
@@ -373,7 +375,7 @@ static int launch_bwd(const void* dy, const void* z, const void* g, const float*
     if (!ln_allow_smem(ln_bwd_kernel<T, NCHUNK, WPR>, LnRing<NCHUNK>::BYTES, allowed)) return -1;
     const cudaError_t e = launch_after(ln_bwd_kernel<T, NCHUNK, WPR>, grid, LN_THREADS, LnRing<NCHUNK>::BYTES, st,
                                        static_cast<const T*>(dy), static_cast<const T*>(z), static_cast<const T*>(g), mean,
-                                       rstd, static_cast<T*>(dz), static_cast<T*>(p > 0.f ? dx : nullptr), partial, rows,
+                                       rstd, static_cast<T*>(dz), static_cast<T*>(dx), partial, rows,
                                        thr, scale, seed, offset);
     return e == cudaSuccess ? 0 : -1;
 }
@@ -450,7 +452,7 @@ static int ln_bwd_empty(void* dgamma, void* dbeta, size_t bytes, int accumulate,
 }  // namespace rb
 
 // `partial` is scratch of rb_ln_bwd_grid(rows) * 2 * H floats.  dgamma / dbeta are
-// fp32 [H]; accumulate != 0 adds to them.
+// fp32 [H]; accumulate != 0 adds to them.  dx (may be null): dz through the dropout mask, or dz once more without dropout.
 extern "C" int rb_ln_bwd(const void* dy, const void* z, const void* gamma, const float* mean,
                          const float* rstd, void* dz, void* dx, float* dgamma, float* dbeta,
                          float* partial, int rows, int H, float p, uint64_t seed, uint64_t offset,
@@ -527,7 +529,7 @@ extern "C" int rb_ln_bwd_noalloc(const void* dy, const void* z, const void* gamm
     if (need > RB_LN_NOALLOC_MAX_FLOATS) return RB_LN_NOALLOC_TOO_LARGE;
     float* scratch = ln_noalloc_scratch_ptr();
     if (!scratch) return RB_LN_NOALLOC_NO_SYMBOL;
-    const int rc = rb_ln_bwd(dy, z, gamma, mean, rstd, dz, dx, dgamma, dbeta, scratch, rows, H, p, seed, offset,
+    const int rc = rb_ln_bwd(dy, z, gamma, mean, rstd, dz, p > 0.f ? dx : nullptr, dgamma, dbeta, scratch, rows, H, p, seed, offset,
                              accumulate, dtype, stream);
     return rc == 0 ? RB_LN_NOALLOC_OK : (rc == -2 ? RB_LN_NOALLOC_BAD_WIDTH : RB_LN_NOALLOC_LAUNCH_FAILED);
 }

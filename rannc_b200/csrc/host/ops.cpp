@@ -14,6 +14,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/forward_grad.h>
 #include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/accumulate_grad.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
@@ -579,11 +580,17 @@ struct LnNode : Node {
         const int H = static_cast<int>(Z.size(-1)), rows = static_cast<int>(Z.numel() / H);
         const bool flat = g_mg.defined() && b_mg.defined();
         Tensor dz = at::empty(Z.sizes(), Z.options()), dx = dz;
-        if (p > 0) dx = at::empty(Z.sizes(), Z.options());
+        // One tensor for both inputs, unless one of them is a leaf: it would copy a gradient that it does not own alone, in
+        // a launch of its own, where the kernel writes a second one beside the first (387 x 4096, two leaves, forward and backward: 90.6 -> 82.6 us).
+        auto leaf = [&](size_t i) {
+            return dynamic_cast<torch::autograd::AccumulateGrad*>(next_edge(i).function.get()) != nullptr;
+        };
+        const bool both = task_should_compute_output(0) && task_should_compute_output(1);
+        if (p > 0 || (both && (leaf(0) || leaf(1)))) dx = at::empty(Z.sizes(), Z.options());
         Tensor partial = f32({static_cast<int64_t>(api.ln_bwd_grid(rows)) * 2 * H}, Z);
-        void* dx_drop = p > 0 ? dx.data_ptr() : nullptr;
+        void* dx_own = dx.is_same(dz) ? nullptr : dx.data_ptr();
         if (flat) {
-            check(api.ln_bwd(dy.data_ptr(), Z.data_ptr(), G.data_ptr(), mptr<float>(M), mptr<float>(R), dz.data_ptr(), dx_drop,
+            check(api.ln_bwd(dy.data_ptr(), Z.data_ptr(), G.data_ptr(), mptr<float>(M), mptr<float>(R), dz.data_ptr(), dx_own,
                              mptr<float>(g_mg), mptr<float>(b_mg), mptr<float>(partial), rows, H, static_cast<float>(p),
                              seed, offset, 1, dt_code(Z), cur_stream()),
                   "rb_ln_bwd", 2);
@@ -592,7 +599,7 @@ struct LnNode : Node {
         }
         // gradients in the parameters' own type, rounded once from the fp32 sums by the reducing kernel
         Tensor dg = at::empty({H}, G.options()), db = at::empty({H}, G.options());
-        check(api.ln_bwd16(dy.data_ptr(), Z.data_ptr(), G.data_ptr(), mptr<float>(M), mptr<float>(R), dz.data_ptr(), dx_drop,
+        check(api.ln_bwd16(dy.data_ptr(), Z.data_ptr(), G.data_ptr(), mptr<float>(M), mptr<float>(R), dz.data_ptr(), dx_own,
                            dg.data_ptr(), db.data_ptr(), mptr<float>(partial), rows, H, static_cast<float>(p), seed, offset,
                            dt_code(Z), cur_stream()),
               "rb_ln_bwd16", 2);

@@ -535,3 +535,24 @@ def test_kernels_that_begin_early_on_streams_beside_each_other(captured):
     assert all(torch.equal(x, y) for x, y in zip(xs, want))
     for s, y in zip(sums, want_sums):   # (K is split: added as it arrives)
         assert (s - y).norm() <= 1e-5 * y.norm()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H", [256, 768, 1024, 2048, 4096])
+@pytest.mark.parametrize("leaf", ["both", "x", "residual", "none"])
+def test_layernorm_gradients_of_two_inputs(dtype, H, leaf):
+    """Without dropout both inputs have the same gradient: written twice where one of them is a leaf, else one tensor."""
+    from rannc_b200.ops import functional as RF
+
+    torch.manual_seed(4)
+    x, r = (torch.randn(13, H, device="cuda").to(dtype).requires_grad_(True) for _ in range(2))
+    g, b = (torch.randn(H, device="cuda").to(dtype).requires_grad_(True) for _ in range(2))
+    dy = torch.randn(13, H, device="cuda").to(dtype)
+    RF.dropout_add_layer_norm(x if leaf in ("both", "x") else x * 1, r if leaf in ("both", "residual") else r * 1, g, b, 0.0,
+                              1e-5).backward(dy)
+    z = (x.detach() + r.detach()).double().requires_grad_(True)
+    torch.nn.functional.layer_norm(z, (H,), g.double(), b.double(), 1e-5).backward(dy.double())
+    assert torch.equal(x.grad, r.grad)
+    assert leaf != "both" or x.grad.data_ptr() != r.grad.data_ptr()
+    # z is rounded to 16 bits before it is normalised: one rounding more than the result's own
+    _near(x.grad, z.grad, dtype, 1, 4 * U[dtype])
