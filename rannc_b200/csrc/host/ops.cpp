@@ -457,8 +457,8 @@ Tensor linear(const Tensor& x, const Tensor& w, const OptTensor& bias_, bool gel
         Epi e;
         bc = dense(bias);
         e.bias = cptr(bc);
-        if (gelu) {
-            e.gelu = true;
+        e.gelu = gelu;
+        if (gelu && req) {   // (what the backward needs)
             pre = at::empty(sizes, x.options());
             e.aux_out = pre.data_ptr();
         }
@@ -526,7 +526,7 @@ Tensor mlp(const Tensor& x, const Tensor& w1, const OptTensor& b1_, const Tensor
         xc = dense(x);
         auto sizes = x.sizes().vec();
         sizes.back() = w1.size(0);
-        pre = at::empty(sizes, x.options());
+        if (req) pre = at::empty(sizes, x.options());   // (what the backward needs)
         h = at::empty(sizes, x.options());
         sizes.back() = w2.size(0);
         y = at::empty(sizes, x.options());
@@ -536,7 +536,7 @@ Tensor mlp(const Tensor& x, const Tensor& w1, const OptTensor& b1_, const Tensor
         Epi e;
         e.bias = cptr(b1c);
         e.gelu = true;
-        e.aux_out = pre.data_ptr();
+        e.aux_out = mptr(pre);
         gemm(rows_of(xc), mat(w1), false, true, h.data_ptr(), false, dt, e);
         Epi e2;
         e2.bias = cptr(b2c);

@@ -556,3 +556,18 @@ def test_layernorm_gradients_of_two_inputs(dtype, H, leaf):
     assert leaf != "both" or x.grad.data_ptr() != r.grad.data_ptr()
     # z is rounded to 16 bits before it is normalised: one rounding more than the result's own
     _near(x.grad, z.grad, dtype, 1, 4 * U[dtype])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows", [1, 351, 3000])
+def test_activation_without_a_graph(dtype, rows):
+    """Under no_grad the value before the activation is not written: the result is the same."""
+    from rannc_b200.ops import functional as RF
+
+    torch.manual_seed(5)
+    x = torch.randn(rows, 264, device="cuda").to(dtype)
+    w, v = (torch.randn(n, m, device="cuda").mul(0.1).to(dtype).requires_grad_(True) for n, m in ((520, 264), (264, 520)))
+    b, c = (torch.randn(n, device="cuda").to(dtype).requires_grad_(True) for n in (520, 264))
+    with torch.no_grad():
+        got = RF.linear(x, w, b, act="gelu"), RF.mlp(x, w, b, v, c)
+    assert torch.equal(got[0], RF.linear(x, w, b, act="gelu")) and torch.equal(got[1], RF.mlp(x, w, b, v, c))
