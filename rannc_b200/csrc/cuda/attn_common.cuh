@@ -18,6 +18,15 @@ __device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* m, const vo
         : "memory");
 }
 
+// Writes a tile of this CTA's shared memory to global memory; rows past the tensor's extent are dropped.
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* m, const void* smem_src, int c0, int c1, int c2, int c3) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+        :
+        : "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+        : "memory");
+}
+
 // barrier among `count` threads of the CTA (count % 32 == 0); id 0 is __syncthreads
 __device__ __forceinline__ void bar_sync_named(int id, int count) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");

@@ -571,3 +571,43 @@ def test_activation_without_a_graph(dtype, rows):
     with torch.no_grad():
         got = RF.linear(x, w, b, act="gelu"), RF.mlp(x, w, b, v, c)
     assert torch.equal(got[0], RF.linear(x, w, b, act="gelu")) and torch.equal(got[1], RF.mlp(x, w, b, v, c))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,S,H,p", [(20, 128, 16, 0.0), (23, 100, 16, 0.2), (11, 200, 16, 0.2), (5, 300, 16, 0.0),
+                                     (7, 512, 16, 0.2), (40, 33, 16, 0.0)])
+def test_attention_backward_over_many_items(dtype, B, S, H, p):
+    """Several blocks of 128 keys to a CTA, one after the other: of one to five query blocks, whole and ragged.  Each (batch,
+    head) by itself gives the same bits in dK and dV; dQ is added up in whichever order the key blocks come."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(11)
+    q, k, v, do = (torch.randn(B, S, H, 64, device="cuda").to(dtype) for _ in range(4))
+    bias = torch.where(torch.rand(B, S, device="cuda") < 0.2, -10000.0, 0.0)
+    bias[:, 0] = 0.0
+    o, lse = K.attn_fwd(q, k, v, bias, 0.125, p, 3, 4)
+    dq, dk, dv = K.attn_bwd(q, k, v, o, lse, do, bias, 0.125, p, 3, 4)
+    assert _lib.read_error() == 0
+    sc = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) / 8 + bias.double()[:, None, None]
+    if p == 0.0:
+        P = sc.softmax(-1)
+        dP = torch.einsum("bqhd,bkhd->bhqk", do.double(), v.double())
+        dS = P * (dP - (P * dP).sum(-1, keepdim=True))
+        want = (torch.einsum("bhqk,bkhd->bqhd", dS, k.double()) / 8, torch.einsum("bhqk,bqhd->bkhd", dS, q.double()) / 8,
+                torch.einsum("bhqk,bqhd->bkhd", P, do.double()))
+        scale = max(w.abs().max().item() for w in want)
+        for got, w in zip((dq, dk, dv), want):     # (as in test_attention_backward_blocks)
+            assert (got.double() - w).abs().max().item() / scale < 6 * U[dtype]
+    for b in (0, B // 2, B - 1):
+        # dropout depends on a row's place in the whole batch: without it a batch row by itself is the same problem
+        if p == 0.0:
+            r = slice(b, b + 1)
+            _, dk1, dv1 = K.attn_bwd(q[r], k[r], v[r], o[r], lse[r], do[r], bias[r].contiguous(), 0.125, p, 3, 4)
+            assert torch.equal(dk1, dk[r]) and torch.equal(dv1, dv[r])
+    # the same call again: no state is left behind
+    dq2, dk2, dv2 = K.attn_bwd(q, k, v, o, lse, do, bias, 0.125, p, 3, 4)
+    assert torch.equal(dk, dk2) and torch.equal(dv, dv2)
+    assert (dq.float() - dq2.float()).abs().max().item() <= 2 * U[dtype] * dq.float().abs().max().item()
+    torch.cuda.synchronize()
+    assert _lib.read_error() == 0
