@@ -611,3 +611,54 @@ def test_attention_backward_over_many_items(dtype, B, S, H, p):
     assert (dq.float() - dq2.float()).abs().max().item() <= 2 * U[dtype] * dq.float().abs().max().item()
     torch.cuda.synchronize()
     assert _lib.read_error() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("S", [64, 200, 256, 512, 1024, 1100])
+@pytest.mark.parametrize("p", [0.0, 0.25])
+def test_attention_forward_bias_by_64_keys(dtype, S, p):
+    """Blocks of 64 keys with, without and with nothing but padding, in every order: batch rows whose valid keys come first,
+    last or between, one without a valid key, one with a bias that is no mask, and a key past which NaN and infinity hide
+    behind the mask and must show."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(12)
+    H = 3
+    rows = torch.zeros(7, S, device="cuda")
+    rows[0, S // 2:] = -10000.0
+    rows[1, :S // 2] = -10000.0
+    rows[2, :S // 3], rows[2, -(S // 3):] = -10000.0, torch.finfo(torch.float32).min
+    rows[3] = -10000.0
+    rows[4] = torch.randn(S, device="cuda")
+    rows[5, -5:] = -10000.0
+    B = rows.shape[0]
+    q, k, v = (torch.randn(B, S, H, 64, device="cuda").to(dtype) for _ in range(3))
+    keep = torch.ones(B, H, S, S, device="cuda", dtype=torch.float64)
+    if p:
+        z = torch.zeros_like(q)
+        for w in range(0, S, 64):
+            n = min(64, S - w)
+            one = z.clone()
+            one[:, w:w + n, :, :n] = torch.eye(n, device="cuda", dtype=dtype)[None, :, None]
+            keep[:, :, :, w:w + n] = (K.attn_fwd(z, z, one, None, 0.125, p, 5, 9)[0][..., :n] > 0).permute(0, 2, 1, 3).double()
+        keep /= 1 - p
+    o, lse = K.attn_fwd(q, k, v, rows, 0.125, p, 5, 9)
+    sc = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) / 8 + rows.double()[:, None, None]
+    want = torch.einsum("bhqk,bkhd->bqhd", sc.softmax(-1) * keep, v.double())
+    # probabilities and the result are rounded once each; terms of the size of the largest value of v
+    assert (o.double() - want).abs().max().item() <= 2 * U[dtype] * v.double().abs().max().item() / (1 - p) + 1e-4
+    # (a row whose scores are all rounded away under the bias: 10000 log2(e) holds eleven binary places)
+    assert (lse.double() - torch.logsumexp(sc, -1)).abs().max().item() <= 2.0 ** -9
+    k2 = k.clone()
+    k2[0, S - 1, 0] = float("nan")
+    k2[1, 0, 1, 5] = float("inf")
+    o2, _ = K.attn_fwd(q, k2, v, rows, 0.125, 0.0, 5, 9)
+    o1, _ = K.attn_fwd(q, k, v, rows, 0.125, 0.0, 5, 9)
+    assert o2[0, :, 0].isnan().all()
+    assert o2[1, :, 1].isnan().any()     # (an infinite score beats the bias where it is positive)
+    same = torch.ones(B, S, H, dtype=torch.bool, device="cuda")
+    same[0, :, 0] = same[1, :, 1] = False
+    assert torch.equal(o1[same], o2[same])
+    torch.cuda.synchronize()
+    assert _lib.read_error() == 0
