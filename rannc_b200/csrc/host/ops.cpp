@@ -968,6 +968,89 @@ Tensor qkv_attention(const Tensor& x, const std::vector<Tensor>& ws, const std::
 Tensor nhwc(const Tensor& t) {   // channels-last on a 16-byte boundary
     return t.is_contiguous(at::MemoryFormat::ChannelsLast) && aligned16(t.data_ptr()) ? t : t.clone(at::MemoryFormat::ChannelsLast);
 }
+// A 1x1 convolution: the linear layer over the pixels of a channels-last activation.  As that layer between views (the pixels
+// of x, the filter as a matrix, the result as an image again) it was four autograd nodes, and 512 to 2048 channels at
+// 32 x 14 x 14 with batch norm, forward and backward, were bound by the host: 164 -> 135 us.
+Mat pixels(const Tensor& t) {
+    Mat m;
+    m.keep = t;
+    m.p = t.data_ptr();
+    m.cols = m.ld = t.size(1);
+    m.rows = t.numel() / m.cols;
+    return m;
+}
+Mat filter(const Tensor& w) {
+    if (!aligned16(w.data_ptr()) || w.stride(1) != 1 || w.stride(0) % 8)
+        return mat(w.detach().reshape({w.size(0), w.size(1)}));
+    Mat m;
+    m.keep = w;
+    m.p = w.data_ptr();
+    m.rows = w.size(0);
+    m.cols = w.size(1);
+    m.ld = w.stride(0);
+    return m;
+}
+struct Conv1x1Node : Node {
+    SavedVariable x, w;
+    Tensor bias, w_ref, w_mg, b_mg;
+    RB_NODE("RbConv1x1Backward")
+    void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        x.reset_data();
+        w.reset_data();
+    }
+    variable_list run(variable_list&& grads) {
+        const Tensor X = x.unpack(), W = w.unpack(), dy = nhwc(grads[0]);
+        const int dt = dt_code(X);
+        const Mat d = pixels(dy), wm = filter(W);
+        Tensor dx;
+        if (task_should_compute_output(0)) {
+            dx = at::empty_like(X);
+            gemm(d, wm, false, false, dx.data_ptr(), false, dt, Epi());
+        }
+        Grads gr = param_grads(d, pixels(X), W, w_mg, task_should_compute_output(1), bias, b_mg,
+                               bias.defined() && task_should_compute_output(2), dt);
+        if (gr.w.defined()) gr.w = gr.w.view(W.sizes());
+        notify({{&w_ref, &w_mg}, {&bias, &b_mg}});
+        return {dx, gr.w, gr.b};
+    }
+};
+Tensor conv1x1(const Tensor& x, const Tensor& w, const OptTensor& bias_, const OptTensor& w_mg, const OptTensor& b_mg) {
+    const Tensor bias = opt(bias_);
+    same_type("conv1x1", x, {&w, &bias});
+    TORCH_CHECK_VALUE(x.dim() == 4 && w.dim() == 4 && w.size(2) == 1 && w.size(3) == 1 && x.size(1) == w.size(1) &&
+                          x.size(1) % 8 == 0 && w.size(0) % 8 == 0 && x.size(1) > 0,
+                      "conv1x1: images and 1x1 filters of channels that are multiples of 8");
+    length("conv1x1 bias", bias, w.size(0));
+    const bool req = wants_grad({&x, &w, &bias});
+    Tensor xc, y;
+    {
+        at::NoGradGuard off;
+        xc = nhwc(x);
+        y = at::empty({x.size(0), w.size(0), x.size(2), x.size(3)}, x.options(), at::MemoryFormat::ChannelsLast);
+        const Tensor bc = dense(bias);
+        Epi e;
+        e.bias = cptr(bc);
+        gemm(pixels(xc), filter(w), false, true, y.data_ptr(), false, dt_code(x), e);
+    }
+    if (req) {
+        auto n = new_node<Conv1x1Node>();
+        n->set_next_edges(torch::autograd::collect_next_edges(x, w, bias));
+        n->x = SavedVariable(xc, false);
+        n->w = SavedVariable(w, false);
+        n->w_ref = w;
+        n->bias = bias;
+        const Tensor mg = opt(w_mg);
+        if (mg.defined()) {
+            TORCH_CHECK_VALUE(mg.numel() == w.numel(), "conv1x1: a filter's gradient buffer has the filter's size");
+            n->w_mg = weight_grad_buffer("conv1x1", mg.view({w.size(0), w.size(1)}), w.detach().reshape({w.size(0), w.size(1)}));
+        }
+        n->b_mg = grad_buffer("conv1x1", b_mg, bias);
+        torch::autograd::set_history(y, n);
+    }
+    return y;
+}
+
 struct BnNode : Node {
     SavedVariable x, y, mean, rstd, g32;
     Tensor gamma, beta, g_mg, b_mg;
@@ -1183,4 +1266,5 @@ PYBIND11_MODULE(_host, m) {
     RB_DEF(cross_entropy);
     RB_DEF(qkv_attention);
     RB_DEF(batch_norm_act);
+    RB_DEF(conv1x1);
 }

@@ -485,10 +485,7 @@ def conv2d(x, weight, bias=None, stride=1, padding=0, dilation=1, groups=1):
         return torch.nn.functional.conv2d(x, weight, bias, stride, padding, dilation, groups)
     if kh == 1 and s[0] == 1 and p[0] == 0:
         # a 1x1 convolution is the linear layer over the pixels of the channels-last activation
-        mg = _main_grad(weight)
-        y = _host().linear(_nhwc(x), weight.reshape(Co, Ci), bias, False, None if mg is None else mg.view(Co, Ci),
-                           _main_grad(bias), weight)
-        return y.permute(0, 3, 1, 2)
+        return _host().conv1x1(x, weight, bias, _main_grad(weight), _main_grad(bias))
     return _Conv2d.apply(x, weight, bias, s[0], p[0])
 
 

@@ -596,3 +596,40 @@ def test_kernel_entries_refuse_addresses_off_a_boundary():
             call()
     torch.cuda.synchronize()
     assert _lib.read_error() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("how", ["channels_last", "contiguous", "slice", "odd", "empty"])
+@pytest.mark.parametrize("flat,bias", [(True, False), (False, True)])
+def test_pointwise_convolution_takes_any_layout(dtype, how, flat, bias):
+    """A 1x1 convolution of images in any order, from any address, and of none: values, gradients and the layouts of both."""
+    from rannc_b200.ops import functional as RF
+
+    torch.manual_seed(3)
+    N, Ci, Co, H, W = (0 if how == "empty" else 3), 24, 40, 5, 7
+    x = torch.randn(N, Ci + 8, H, W, device="cuda").to(dtype)
+    if how == "odd":      # an address off a 16-byte boundary
+        x = torch.empty(x[:, :Ci].numel() + 1, device="cuda", dtype=dtype)[1:].view(N, H, W, Ci).normal_().permute(0, 3, 1, 2)
+    elif how == "slice":
+        x = x.to(memory_format=torch.channels_last)[:, 8:]
+    else:
+        x = x[:, :Ci].contiguous(memory_format=torch.contiguous_format if how == "contiguous" else torch.channels_last)
+    x = x.detach().requires_grad_(True)
+    w = torch.randn(Co, Ci, 1, 1, device="cuda").to(dtype).requires_grad_(True)
+    b = torch.randn(Co, device="cuda").to(dtype).requires_grad_(True) if bias else None
+    if flat:
+        w.main_grad = torch.full((Co, Ci, 1, 1), 2.0, device="cuda")
+    y = RF.conv2d(x, w, b)
+    assert y.shape == (N, Co, H, W) and (N == 0 or y.is_contiguous(memory_format=torch.channels_last))
+    dy = torch.randn(N, Co, H, W, device="cuda").to(dtype)
+    y.backward(dy)
+    assert x.grad.shape == x.shape and (w.grad is None) == flat
+    xr, wr = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    ref = torch.nn.functional.conv2d(xr, wr, None if b is None else b.detach().double())
+    ref.backward(dy.double())
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    pairs = [(y, ref, u), (x.grad, xr.grad, u), (w.main_grad - 2.0 if flat else w.grad, wr.grad, 0.0 if flat else u)]
+    if b is not None:
+        pairs.append((b.grad, dy.double().sum((0, 2, 3)), u))
+    for got, want, rounding in pairs:      # one rounding of the result; fp32 sums (that start at 2 where they are added)
+        assert ((got.double() - want).abs() <= rounding * want.abs() + 1e-5 * (want.abs().max() if N else 0) + 1e-6).all()
