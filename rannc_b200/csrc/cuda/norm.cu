@@ -17,6 +17,8 @@
 #include <cstdlib>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "launch.cuh"
 #include "philox.cuh"
 #include "tc_common.cuh"
@@ -26,26 +28,51 @@ namespace rb {
 constexpr int LN_WARPS = 8;
 constexpr int LN_THREADS = LN_WARPS * 32;
 
+// Eight 16-bit values as four pairs of fp32: both kernels are bound by issue slots as much as by memory (a row's bytes pass
+// an SM in some 175 cycles, and at 220 instructions a warp and row, dropout apart, that is what four schedulers take), so
+// what has a two-wide form uses it, and gamma and beta stay in registers where they suffice.
 template <typename T>
-__device__ __forceinline__ void ld8(const T* p, float (&v)[8]) {
-    uint4 q = *reinterpret_cast<const uint4*>(p);
-    const T* e = reinterpret_cast<const T*>(&q);
+__device__ __forceinline__ void unpack_pairs(const uint4& q, uint64_t (&v)[4]) {
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = to_f32<T>(e[j]);
-}
-__device__ __forceinline__ uint4 pack8(const float (&v)[8], const __nv_bfloat16*) {
-    return make_uint4(pack2<__nv_bfloat16>(v[0], v[1]), pack2<__nv_bfloat16>(v[2], v[3]),
-                      pack2<__nv_bfloat16>(v[4], v[5]), pack2<__nv_bfloat16>(v[6], v[7]));
-}
-__device__ __forceinline__ uint4 pack8(const float (&v)[8], const __half*) {
-    return make_uint4(pack2<__half>(v[0], v[1]), pack2<__half>(v[2], v[3]), pack2<__half>(v[4], v[5]),
-                      pack2<__half>(v[6], v[7]));
+    for (int j = 0; j < 4; ++j) {
+        if constexpr (std::is_same_v<T, __nv_bfloat16>) {
+            v[j] = f2_pack_bits(w[j] << 16, w[j] & 0xffff0000u);
+        } else {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+            v[j] = f2_pack(f.x, f.y);
+        }
+    }
 }
 template <typename T>
-__device__ __forceinline__ void unpack8(const uint4& q, float (&v)[8]) {
-    const T* e = reinterpret_cast<const T*>(&q);
+__device__ __forceinline__ uint4 pack_pairs(const uint64_t (&v)[4]) {
+    uint32_t w[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = to_f32<T>(e[j]);
+    for (int j = 0; j < 4; ++j) {
+        float a, b;
+        f2_unpack(v[j], a, b);
+        w[j] = pack2<T>(a, b);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+template <typename T>
+__device__ __forceinline__ void load_pairs(const T* p, uint64_t (&v)[4]) {
+    unpack_pairs<T>(*reinterpret_cast<const uint4*>(p), v);
+}
+__device__ __forceinline__ uint64_t f2_both(float x) { return f2_pack(x, x); }
+__device__ __forceinline__ float f2_sum(uint64_t v) {
+    float a, b;
+    f2_unpack(v, a, b);
+    return a + b;
+}
+// v * scale where the element is kept, else zero
+__device__ __forceinline__ void drop_pairs(uint64_t (&v)[4], const bool (&k)[8], uint64_t scale2) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        float a, b;
+        f2_unpack(f2_mul(v[j], scale2), a, b);
+        v[j] = f2_pack(k[2 * j] ? a : 0.f, k[2 * j + 1] ? b : 0.f);
+    }
 }
 // 16 bytes from global to this thread's own place in shared memory, asynchronously
 __device__ __forceinline__ void cp_async16(uint4* dst, const void* src) {
@@ -83,12 +110,13 @@ __device__ __forceinline__ float2 group_sum(float2 v, float2 (*sm)[LN_WARPS], in
     return v;
 }
 
-// Rows a thread has on their way while it works on one.  Both kernels are bound by memory, and what kept them
-// from it was latency: a row is one dependent chain load -> reduce -> store, so the bytes in flight were those
-// of the resident warps' current rows.  Each thread now fetches its own 16-byte pieces of the next rows into
-// its own places of a shared-memory ring (no barrier is needed to read them back), three deep or more.  16384 x 1024
-// bf16 with dropout and residual (134 MB each way, 20 us at the copy bandwidth): forward 32.3 -> 28.0 us, backward
-// 34.8 -> 29.9 us; 387 x 4096: 4.7 -> 4.0 and 7.2 -> 6.7 us.
+// Rows a thread has on their way while it works on one.  A row is one dependent chain load -> reduce -> store, and the bytes
+// in flight would be those of the resident warps' current rows.  Each thread fetches its own 16-byte pieces of the next rows
+// into its own places of a shared-memory ring (no barrier is needed to read them back), three deep or more.
+// Time, and at the copy bandwidth (us, bf16; backward with the sums' reduction): 16384 x 1024 with dropout and residual forward
+// 28.7 -> 27.1 (20.5), backward 33.6 -> 30.5 (20.5); without 15.1 -> 12.8 (10.3) and 23.3 -> 19.4 (15.4); 8192 x 2048 24.2
+// -> 20.8 and 25.4 -> 24.5; 4096 x 4096 25.4 -> 24.8 and 33.3 -> 29.8; before that, of one row at a time, 32.3 and 34.8 at
+// 16384 x 1024 with dropout.
 template <int NCHUNK>
 struct LnRing {
     static constexpr int STAGES = NCHUNK <= 2 ? 4 : 3;
@@ -124,6 +152,16 @@ __global__ void __launch_bounds__(LN_THREADS, LnRing<NCHUNK>::FWD_CTAS)
         }
         cp_async_commit();
     };
+    constexpr bool KEEP = NCHUNK <= 2;   // wider threads read gamma and beta again from L1 for every row
+    uint64_t kept_g[KEEP ? NCHUNK : 1][4], kept_b[KEEP ? NCHUNK : 1][4];
+    if constexpr (KEEP) {
+#pragma unroll
+        for (int c = 0; c < NCHUNK; ++c) {
+            load_pairs(gamma + col0 + c * 256, kept_g[c]);
+            load_pairs(beta + col0 + c * 256, kept_b[c]);
+        }
+    }
+    const uint64_t scale2 = f2_both(scale);
     long long row = static_cast<long long>(blockIdx.x) * RPB + slot;
 #pragma unroll
     for (int k = 0; k < STAGES - 1; ++k) fetch(k, row + k * step);
@@ -132,57 +170,62 @@ __global__ void __launch_bounds__(LN_THREADS, LnRing<NCHUNK>::FWD_CTAS)
         fetch(stage == 0 ? STAGES - 1 : stage - 1, row + (STAGES - 1) * step);
         cp_async_wait<STAGES - 1>();
         const size_t base = static_cast<size_t>(row) * H;
-        float v[NCHUNK][8];
-        float s = 0.f;
+        uint64_t v[NCHUNK][4];
+        uint64_t s2 = f2_both(0.f);
 #pragma unroll
         for (int c = 0; c < NCHUNK; ++c) {
             const int col = col0 + c * 256;
-            unpack8<T>(*place(stage, 0, c), v[c]);
+            unpack_pairs<T>(*place(stage, 0, c), v[c]);
             if (thr) {
                 bool k[8];
                 keep8(seed, offset, base + col, thr, k);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) v[c][j] = k[j] ? v[c][j] * scale : 0.f;
+                drop_pairs(v[c], k, scale2);
             }
             if (residual) {
-                float r[8];
-                unpack8<T>(*place(stage, 1, c), r);
+                uint64_t r[4];
+                unpack_pairs<T>(*place(stage, 1, c), r);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[c][j] += r[j];
+                for (int j = 0; j < 4; ++j) v[c][j] = f2_add(v[c][j], r[j]);
             }
             if (z_out) {
-                const uint4 q = pack8(v[c], static_cast<const T*>(nullptr));
+                const uint4 q = pack_pairs<T>(v[c]);
                 *reinterpret_cast<uint4*>(z_out + base + col) = q;
                 // the backward reads z in storage precision: normalise the same values
-                unpack8<T>(q, v[c]);
+                unpack_pairs<T>(q, v[c]);
             }
 #pragma unroll
-            for (int j = 0; j < 8; ++j) s += v[c][j];
+            for (int j = 0; j < 4; ++j) s2 = f2_add(s2, v[c][j]);
         }
-        const float mean = group_sum<WPR>(make_float2(s, 0.f), sm, turn, warp, lane).x * (1.f / H);
-        float sq = 0.f;
+        const float mean = group_sum<WPR>(make_float2(f2_sum(s2), 0.f), sm, turn, warp, lane).x * (1.f / H);
+        const uint64_t minus_mean = f2_both(-mean);
+        uint64_t sq2 = f2_both(0.f);
 #pragma unroll
         for (int c = 0; c < NCHUNK; ++c)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float d = v[c][j] - mean;
-                sq += d * d;
+            for (int j = 0; j < 4; ++j) {
+                v[c][j] = f2_add(v[c][j], minus_mean);
+                sq2 = f2_fma(v[c][j], v[c][j], sq2);
             }
-        const float rstd = rsqrtf(group_sum<WPR>(make_float2(sq, 0.f), sm, turn, warp, lane).x * (1.f / H) + eps);
+        const float rstd = rsqrtf(group_sum<WPR>(make_float2(f2_sum(sq2), 0.f), sm, turn, warp, lane).x * (1.f / H) + eps);
         if (lane == 0 && part == 0) {
             mean_out[row] = mean;
             rstd_out[row] = rstd;
         }
-        // gamma / beta are re-read per row (they stay in L1) instead of costing 16 * NCHUNK registers
+        const uint64_t rstd2 = f2_both(rstd);
 #pragma unroll
         for (int c = 0; c < NCHUNK; ++c) {
             const int col = col0 + c * 256;
-            float o[8], g[8], b[8];
-            ld8(gamma + col, g);
-            ld8(beta + col, b);
+            uint64_t g[4], b[4];
+            if constexpr (KEEP) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] = (v[c][j] - mean) * rstd * g[j] + b[j];
-            *reinterpret_cast<uint4*>(y + base + col) = pack8(o, static_cast<const T*>(nullptr));
+                for (int j = 0; j < 4; ++j) g[j] = kept_g[c][j], b[j] = kept_b[c][j];
+            } else {
+                load_pairs(gamma + col, g);
+                load_pairs(beta + col, b);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[c][j] = f2_fma(f2_mul(v[c][j], rstd2), g[j], b[j]);
+            *reinterpret_cast<uint4*>(y + base + col) = pack_pairs<T>(v[c]);
         }
         if (++stage == STAGES) stage = 0;
     }
@@ -219,70 +262,84 @@ __global__ void __launch_bounds__(LN_THREADS, 2)
     };
     // gamma stays in registers where they suffice; wider threads read it again from L1 (spills otherwise)
     constexpr bool KEEP_G = NCHUNK <= 2;
-    float kept[KEEP_G ? NCHUNK : 1][8], dg[NCHUNK][8], db[NCHUNK][8];
+    // a row's 16-bit values stay in registers across its sum where they suffice, else they are read again from the ring
+    // (16384 x 1024 24.0 -> 19.4 us; of 4096 elements a row, held: 49 us for 30)
+    constexpr bool HOLD = NCHUNK <= 2 && WPR <= 2;
+    uint64_t kept[KEEP_G ? NCHUNK : 1][4], dg[NCHUNK][4], db[NCHUNK][4];
 #pragma unroll
     for (int c = 0; c < NCHUNK; ++c) {
-        if constexpr (KEEP_G) ld8(gamma + col0 + c * 256, kept[c]);
+        if constexpr (KEEP_G) load_pairs(gamma + col0 + c * 256, kept[c]);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) dg[c][j] = db[c][j] = 0.f;
+        for (int j = 0; j < 4; ++j) dg[c][j] = db[c][j] = f2_both(0.f);
     }
-    auto get_gamma = [&](int c, float (&g)[8]) {
+    auto get_gamma = [&](int c, uint64_t (&g)[4]) {
         if constexpr (KEEP_G) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) g[j] = kept[c][j];
+            for (int j = 0; j < 4; ++j) g[j] = kept[c][j];
         } else {
-            ld8(gamma + col0 + c * 256, g);
+            load_pairs(gamma + col0 + c * 256, g);
         }
     };
+    const uint64_t scale2 = f2_both(scale);
     long long row = static_cast<long long>(blockIdx.x) * RPB + slot;
 #pragma unroll
     for (int k = 0; k < STAGES - 1; ++k) fetch(k, row + k * step);
     float mean = row < rows ? mean_in[row] : 0.f, rstd = row < rows ? rstd_in[row] : 0.f;
     int stage = 0, turn = 0;
     for (; row < rows; row += step) {
-        fetch(stage == 0 ? STAGES - 1 : stage - 1, row + (STAGES - 1) * step);
         // the next row's statistics, used one iteration later
         const bool more = row + step < rows;
         const float mean_next = more ? mean_in[row + step] : 0.f, rstd_next = more ? rstd_in[row + step] : 0.f;
-        cp_async_wait<STAGES - 1>();
+        cp_async_wait<STAGES - 2>();
         const size_t base = static_cast<size_t>(row) * H;
-        float2 s = make_float2(0.f, 0.f);
+        const uint64_t minus_mean = f2_both(-mean), rstd2 = f2_both(rstd);
+        uint64_t sx = f2_both(0.f), sy = sx;
+        uint4 hd[HOLD ? NCHUNK : 1], hz[HOLD ? NCHUNK : 1];
 #pragma unroll
         for (int c = 0; c < NCHUNK; ++c) {
-            float d[8], zz[8], g[8];
-            unpack8<T>(*place(stage, 0, c), d);
-            unpack8<T>(*place(stage, 1, c), zz);
+            uint64_t d[4], zz[4], g[4];
+            const uint4 qd = *place(stage, 0, c), qz = *place(stage, 1, c);
+            if constexpr (HOLD) hd[c] = qd, hz[c] = qz;
+            unpack_pairs<T>(qd, d);
+            unpack_pairs<T>(qz, zz);
             get_gamma(c, g);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float xh = (zz[j] - mean) * rstd, w = d[j] * g[j];
-                s.x += w;
-                s.y += w * xh;
-                dg[c][j] += d[j] * xh;
-                db[c][j] += d[j];
+            for (int j = 0; j < 4; ++j) {
+                const uint64_t xh = f2_mul(f2_add(zz[j], minus_mean), rstd2), w = f2_mul(d[j], g[j]);
+                sx = f2_add(sx, w);
+                sy = f2_fma(w, xh, sy);
+                dg[c][j] = f2_fma(d[j], xh, dg[c][j]);
+                db[c][j] = f2_add(db[c][j], d[j]);
             }
         }
-        s = group_sum<WPR>(s, sm, turn, warp, lane);
-        const float s1 = s.x * (1.f / H), s2 = s.y * (1.f / H);
+        // (here, behind the loads of this row and before the wait for the other warps: at the top of the loop 24.0 us, not 22)
+        fetch(stage == 0 ? STAGES - 1 : stage - 1, row + (STAGES - 1) * step);
+        const float2 s = group_sum<WPR>(make_float2(f2_sum(sx), f2_sum(sy)), sm, turn, warp, lane);
+        // o = rstd (d g - s1 - xh s2), with s1 and s2 the means of s.x and s.y
+        const uint64_t c1 = f2_both(-rstd * s.x * (1.f / H)), c2 = f2_both(-rstd * rstd * s.y * (1.f / H));
 #pragma unroll(NCHUNK <= 2 ? NCHUNK : 1)
         for (int c = 0; c < NCHUNK; ++c) {
             const int col = col0 + c * 256;
-            // read again from the ring: cheaper than 16 * NCHUNK registers held across the sum
-            float d[8], zz[8], g[8], o[8];
-            unpack8<T>(*place(stage, 0, c), d);
-            unpack8<T>(*place(stage, 1, c), zz);
+            uint64_t d[4], zz[4], g[4], o[4];
+            if constexpr (HOLD) {
+                unpack_pairs<T>(hd[c], d);
+                unpack_pairs<T>(hz[c], zz);
+            } else {
+                unpack_pairs<T>(*place(stage, 0, c), d);
+                unpack_pairs<T>(*place(stage, 1, c), zz);
+            }
             get_gamma(c, g);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] = rstd * (d[j] * g[j] - s1 - (zz[j] - mean) * rstd * s2);
-            *reinterpret_cast<uint4*>(dz_out + base + col) = pack8(o, static_cast<const T*>(nullptr));
+            for (int j = 0; j < 4; ++j)
+                o[j] = f2_fma(f2_mul(d[j], g[j]), rstd2, f2_fma(f2_add(zz[j], minus_mean), c2, c1));
+            *reinterpret_cast<uint4*>(dz_out + base + col) = pack_pairs<T>(o);
             if (dx_out) {
                 if (thr) {
                     bool k[8];
                     keep8(seed, offset, base + col, thr, k);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) o[j] = k[j] ? o[j] * scale : 0.f;
+                    drop_pairs(o, k, scale2);
                 }
-                *reinterpret_cast<uint4*>(dx_out + base + col) = pack8(o, static_cast<const T*>(nullptr));
+                *reinterpret_cast<uint4*>(dx_out + base + col) = pack_pairs<T>(o);
             }
         }
         mean = mean_next;
@@ -298,7 +355,8 @@ __global__ void __launch_bounds__(LN_THREADS, 2)
         for (int c = 0; c < NCHUNK; ++c) {
             __syncthreads();
 #pragma unroll
-            for (int j = 0; j < 8; ++j) red[warp][lane * 8 + j] = pass == 0 ? dg[c][j] : db[c][j];
+            for (int j = 0; j < 4; ++j)
+                f2_unpack(pass == 0 ? dg[c][j] : db[c][j], red[warp][lane * 8 + 2 * j], red[warp][lane * 8 + 2 * j + 1]);
             __syncthreads();
             const int t = threadIdx.x;  // 256 threads, 256 columns
 #pragma unroll

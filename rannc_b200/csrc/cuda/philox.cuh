@@ -19,8 +19,10 @@ __device__ __forceinline__ Philox4 philox4x32(uint64_t seed, uint64_t offset, ui
     uint32_t c2 = static_cast<uint32_t>(offset), c3 = static_cast<uint32_t>(offset >> 32);
 #pragma unroll
     for (int r = 0; r < 7; ++r) {
-        const uint32_t hi0 = __umulhi(0xD2511F53u, c0), lo0 = 0xD2511F53u * c0;
-        const uint32_t hi1 = __umulhi(0xCD9E8D57u, c2), lo1 = 0xCD9E8D57u * c2;
+        // (one wide multiplication for both halves)
+        const uint64_t m0 = static_cast<uint64_t>(0xD2511F53u) * c0, m1 = static_cast<uint64_t>(0xCD9E8D57u) * c2;
+        const uint32_t hi0 = static_cast<uint32_t>(m0 >> 32), lo0 = static_cast<uint32_t>(m0);
+        const uint32_t hi1 = static_cast<uint32_t>(m1 >> 32), lo1 = static_cast<uint32_t>(m1);
         const uint32_t n0 = hi1 ^ c1 ^ k0;
         const uint32_t n2 = hi0 ^ c3 ^ k1;
         c0 = n0;
