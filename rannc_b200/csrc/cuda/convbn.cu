@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
 #include "tc_common.cuh"
 
 namespace rb {
@@ -121,25 +122,35 @@ __global__ void col2im_kernel(const T* __restrict__ dcols, T* __restrict__ dx, i
 // out [N, H + pad, W + pad, C] = x [N, H, W, C] with zero columns behind every row and zero rows behind every image;
 // one block per padded image row.  Bound by memory: one pass that reads x once and writes every output vector once (a
 // generic pad clears the output and then copies the interior with a strided kernel: 32 x 28 x 28 x 1024 took 80 us
-// that way; this takes 17 us).
+// that way; this takes 16.4 us, of which a launch beside the end of the kernel before saves 1.6).
 __global__ void __launch_bounds__(256)
-    pad_nhwc_kernel(const uint4* __restrict__ x, uint4* __restrict__ out, int H, int W, int cv, int pad) {
+    pad_nhwc_kernel(const uint4* x, uint4* out, int H, int W, int cv, int pad) {
+    grid_trigger();
+    grid_wait();
     const int Wp = W + pad, Hp = H + pad;
     const int n = blockIdx.x / Hp, y = blockIdx.x - n * Hp;
     uint4* o = out + static_cast<long long>(blockIdx.x) * Wp * cv;
     const uint4* row = x + (static_cast<long long>(n) * H + y) * W * cv;
     const int live = y < H ? W * cv : 0;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < Wp * cv; i += 256) o[i] = i < live ? row[i] : make_uint4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < Wp * cv; i += 4 * 256) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = i + u * 256 < live ? row[i + u * 256] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i + u * 256 < Wp * cv) o[i + u * 256] = v[u];
+    }
 }
 
 // A filter [Co, Ci, taps] as the GEMM reads it, [Co, taps, Ci]; 16-bit elements, Ci a multiple of 8.  A block takes CH
 // channels of one filter through shared memory, so that both sides move in 16-byte pieces of consecutive addresses (a
-// generic strided copy reads 2 bytes of every 18: 1024 x 1024 x 3 x 3 took 258 us that way and takes 12.4 us here,
+// generic strided copy reads 2 bytes of every 18: 1024 x 1024 x 3 x 3 took 258 us that way and takes 10.3 us here,
 // 2048 x 2048 333 and 40 us, 3.7 TB/s).  The padded rows shift the banks by four from tap to tap.  CH shrinks as the taps grow, to stay below 48 KiB.
 template <int CH>
 __global__ void __launch_bounds__(256)
-    pack_taps_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, int Ci, int taps, int chunks) {
+    pack_taps_kernel(const uint16_t* src, uint16_t* dst, int Ci, int taps, int chunks) {
+    grid_trigger();
+    grid_wait();
     constexpr int LD = CH + 8;
     extern __shared__ uint4 pack_smem[];
     uint16_t* tile = reinterpret_cast<uint16_t*>(pack_smem);  // [taps][LD]
@@ -167,9 +178,10 @@ template <int CH>
 static int pack_taps_launch(const void* src, void* dst, int Co, int Ci, int taps, cudaStream_t st) {
     const int chunks = (Ci + CH - 1) / CH;
     if (static_cast<long long>(Co) * chunks > 0x7fffffffLL) return -2;
-    pack_taps_kernel<CH><<<static_cast<unsigned>(Co) * chunks, 256, taps * (CH + 8) * 2, st>>>(
-        static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), Ci, taps, chunks);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_after(pack_taps_kernel<CH>, static_cast<unsigned>(Co) * chunks, 256, taps * (CH + 8) * 2, st,
+                        static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), Ci, taps, chunks) == cudaSuccess
+               ? 0
+               : -1;
 }
 
 // The weight gradient comes out of its GEMM as src [Co, taps, Ci] fp32 and belongs into a [Co, Ci, taps] tensor:
@@ -226,16 +238,28 @@ __device__ __forceinline__ void ldf8_any(const float* p, float (&v)[8]) {
 // BX * 8 channels, rows are strided over threadIdx.y and blockIdx.y.  BX follows the channel count, so that a layer of
 // 64 channels does not leave three quarters of its threads without one.
 //
+// Clears the sums.  (A copy-engine or runtime memset between two kernels waits for the first's end and the second for
+// its own; this one is in place when the first ends.)
+__global__ void __launch_bounds__(256) bn_clear_kernel(float4* part, int n) {
+    grid_trigger();
+    grid_wait();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < n) part[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+static cudaError_t bn_clear(float* part, int C, cudaStream_t st) {  // 2 C floats, C a multiple of 8
+    return launch_after(bn_clear_kernel, (C / 2 + 255) / 256, 256, 0, st, reinterpret_cast<float4*>(part), C / 2);
+}
+
 // part[0][c] += sum_r a(r, c), part[1][c] += sum_r a(r, c) * b(r, c)
 //   MODE 0 (statistics):  a = x,                 b = x
 //   MODE 1 (backward):    a = dy masked by relu, b = xhat = (x - mean) * rstd
 template <typename T, int MODE, int BX>
 __global__ void __launch_bounds__(256)
-    bn_reduce_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ y,
-                     const float* __restrict__ mean, const float* __restrict__ rstd,
-                     float* __restrict__ part, long long R, int C, int relu) {
+    bn_reduce_kernel(const T* x, const T* dy, const T* y, const float* mean, const float* rstd, float* part, long long R,
+                     int C, int relu) {
     constexpr int TY = 256 / BX;
     __shared__ float red[2][TY][BX * 8 + 8];
+    grid_wait();
     const int col = (blockIdx.x * BX + threadIdx.x) * 8;
     float s0[8], s1[8], mu[8], rs[8];
 #pragma unroll
@@ -287,16 +311,31 @@ __global__ void __launch_bounds__(256)
 // its 8 channels' scale and shift from the two sums itself (a kernel of C threads in between cost 3 us and a launch for
 // a few hundred cycles of arithmetic: 32 x 14 x 14 x 2048 with residual 13.6 + 3.1 -> 12.6 us, its backward below 18.6 +
 // 2.2 -> 17.3 us); the first row of blocks also writes mean, rstd and the running statistics (momentum, unbiased
-// variance).  One wave of blocks, four per SM: twice as many left a thread five rows to pay for its coefficients with.
+// variance).  Bound by memory: four rows of a thread are on their way at a time, the first while the coefficients are
+// computed, and rows are taken from the last one on, because the reduction has just read those and they are still in
+// the L2 cache.
 template <typename T, int BX>
 __global__ void __launch_bounds__(256)
-    bn_apply_kernel(const T* __restrict__ x, const T* __restrict__ res, const float* __restrict__ part,
-                    const float* __restrict__ gamma, const float* __restrict__ beta, float* __restrict__ mean,
-                    float* __restrict__ rstd, float* __restrict__ run_mean, float* __restrict__ run_var,
-                    T* __restrict__ y, long long R, int C, float eps, float momentum, int relu) {
+    bn_apply_kernel(const T* x, const T* res, const float* part, const float* gamma, const float* beta, float* mean,
+                    float* rstd, float* run_mean, float* run_var, T* y, long long R, int C, float eps, float momentum,
+                    int relu) {
     constexpr int TY = 256 / BX;
     const int col = (blockIdx.x * BX + threadIdx.x) * 8;
+    grid_wait();
     if (col >= C) return;
+    const long long step = static_cast<long long>(gridDim.y) * TY;
+    long long r0 = blockIdx.y * TY + threadIdx.y;
+    uint4 qx[4], qr[4];   // (loads written out: the compiler may not move one before another row's store)
+    auto fetch = [&](long long r0) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const long long r = r0 + u * step;
+            if (r >= R) break;
+            qx[u] = *reinterpret_cast<const uint4*>(x + (R - 1 - r) * C + col);
+            if (res) qr[u] = *reinterpret_cast<const uint4*>(res + (R - 1 - r) * C + col);
+        }
+    };
+    fetch(r0);   // beside the coefficients' arithmetic
     float sc[8], sh[8], p0[8], p1[8];
     ldf8(part + col, p0);
     ldf8(part + C + col, p1);
@@ -322,24 +361,28 @@ __global__ void __launch_bounds__(256)
             }
         }
     }
-    const long long step = static_cast<long long>(gridDim.y) * TY;
-#pragma unroll 2
-    for (long long r = blockIdx.y * TY + threadIdx.y; r < R; r += step) {
-        float v[8], o[8];
-        ld8(x + r * C + col, v);
+    while (r0 < R) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = fmaf(v[j], sc[j], sh[j]);
-        if (res) {
-            float rr[8];
-            ld8(res + r * C + col, rr);
+        for (int u = 0; u < 4; ++u) {
+            const long long r = r0 + u * step;
+            if (r >= R) break;
+            float v[8], o[8];
+            ld8(reinterpret_cast<const T*>(&qx[u]), v);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] += rr[j];
+            for (int j = 0; j < 8; ++j) o[j] = fmaf(v[j], sc[j], sh[j]);
+            if (res) {
+                float rr[8];
+                ld8(reinterpret_cast<const T*>(&qr[u]), rr);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) o[j] += rr[j];
+            }
+            if (relu) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) o[j] = fmaxf(o[j], 0.f);
+            }
+            st8(y + (R - 1 - r) * C + col, o);
         }
-        if (relu) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] = fmaxf(o[j], 0.f);
-        }
-        st8(y + r * C + col, o);
+        fetch(r0 += 4 * step);
     }
 }
 
@@ -348,12 +391,11 @@ __global__ void __launch_bounds__(256)
 // the sums to the fp32 gradients of beta and gamma when it is given their buffers.
 template <typename T, int BX>
 __global__ void __launch_bounds__(256)
-    bn_bwd_apply_kernel(const T* __restrict__ x, const T* __restrict__ dy, const T* __restrict__ y,
-                        const float* __restrict__ part, const float* __restrict__ mean, const float* __restrict__ rstd,
-                        const float* __restrict__ gamma, float* __restrict__ dgamma, float* __restrict__ dbeta,
-                        T* __restrict__ dx, T* __restrict__ dres, long long R, int C, int relu) {
+    bn_bwd_apply_kernel(const T* x, const T* dy, const T* y, const float* part, const float* mean, const float* rstd,
+                        const float* gamma, float* dgamma, float* dbeta, T* dx, T* dres, long long R, int C, int relu) {
     constexpr int TY = 256 / BX;
     const int col = (blockIdx.x * BX + threadIdx.x) * 8;
+    grid_wait();
     if (col >= C) return;
     float A[8], B[8], Cc[8], p0[8], p1[8], rs[8], mu[8];
     ldf8(part + col, p0);
@@ -373,26 +415,47 @@ __global__ void __launch_bounds__(256)
         if (writer && dbeta) dbeta[c] += p0[j];
     }
     const long long step = static_cast<long long>(gridDim.y) * TY;
-#pragma unroll 2
-    for (long long r = blockIdx.y * TY + threadIdx.y; r < R; r += step) {
-        float v[8], g[8], o[8];
-        ld8(x + r * C + col, v);
-        ld8(dy + r * C + col, g);
-        if (relu) {
-            float yy[8];
-            ld8(y + r * C + col, yy);
+    for (long long r0 = blockIdx.y * TY + threadIdx.y; r0 < R; r0 += 2 * step) {  // (two rows' loads, as above)
+        uint4 qx[2], qd[2], qy[2];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) g[j] = yy[j] > 0.f ? g[j] : 0.f;
+        for (int u = 0; u < 2; ++u) {
+            const long long r = r0 + u * step;
+            if (r >= R) break;
+            qx[u] = *reinterpret_cast<const uint4*>(x + (R - 1 - r) * C + col);
+            qd[u] = *reinterpret_cast<const uint4*>(dy + (R - 1 - r) * C + col);
+            if (relu) qy[u] = *reinterpret_cast<const uint4*>(y + (R - 1 - r) * C + col);
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = fmaf(A[j], g[j], fmaf(B[j], v[j], Cc[j]));
-        st8(dx + r * C + col, o);
-        if (dres) st8(dres + r * C + col, g);
+        for (int u = 0; u < 2; ++u) {
+            const long long r = r0 + u * step;
+            if (r >= R) break;
+            float v[8], g[8], o[8];
+            ld8(reinterpret_cast<const T*>(&qx[u]), v);
+            ld8(reinterpret_cast<const T*>(&qd[u]), g);
+            if (relu) {
+                float yy[8];
+                ld8(reinterpret_cast<const T*>(&qy[u]), yy);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) g[j] = yy[j] > 0.f ? g[j] : 0.f;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] = fmaf(A[j], g[j], fmaf(B[j], v[j], Cc[j]));
+            st8(dx + (R - 1 - r) * C + col, o);
+            if (dres) st8(dres + (R - 1 - r) * C + col, g);
+        }
     }
 }
 
 // Grid of the batch-norm kernels: blocks of BX * 8 channels, and as many row groups as give the whole grid about
-// `per_sm` blocks per SM, each with four rows or more per thread.
+// `per_sm` blocks per SM, each with four rows or more per thread.  per_sm is what an SM holds at once of the kernel with
+// its registers (40 to 101 a thread), so that there is one wave: 6 and 4 for the reductions, 2 for the element-wise passes
+// (at four with half the rows in flight, or held to 64 registers, those take longer, as does the reduction of the forward
+// pass at 4 or 8).  Forward and backward of 32 x 14 x 14 x 2048 with residual and ReLU 22.7 and 39.4 -> 19.6 and 33.7 us, of
+// 32 x 28 x 28 x 1024 with ReLU 35.4 and 68.5 -> 30.1 and 58.5; the order of the rows gave 3 and 5 us of the backward
+// passes, the launches beside the end of the kernel before (which need a clearing kernel in the place of a memset) 1 to 3.
+// None of these kernels lets the next begin by grid_trigger(): a GEMM that does waits on the SMs with its shared memory, and
+// the first-level cache that this leaves to them costs more (a 1x1 convolution of 32 x 14 x 14 x 2048 with its norm, forward
+// and backward, 131.6 us of device time with the triggers, 120.3 without, 128.5 at ordinary launches).
 template <int BX>
 static dim3 bn_grid(long long R, int C, int per_sm) {
     const int cols = (C + BX * 8 - 1) / (BX * 8);
@@ -408,12 +471,16 @@ static int bn_fwd_launch(const void* x, const void* res, const float* gamma, con
                          float momentum, int relu, cudaStream_t st) {
     const dim3 block(BX, 256 / BX);
     const T* xt = static_cast<const T*>(x);
-    cudaMemsetAsync(part, 0, 2 * sizeof(float) * C, st);
-    bn_reduce_kernel<T, 0, BX><<<bn_grid<BX>(R, C, 4), block, 0, st>>>(xt, nullptr, nullptr, nullptr, nullptr, part, R, C, 0);
-    bn_apply_kernel<T, BX><<<bn_grid<BX>(R, C, 4), block, 0, st>>>(xt, static_cast<const T*>(res), part, gamma, beta, mean,
-                                                                   rstd, run_mean, run_var, static_cast<T*>(y), R, C, eps,
-                                                                   momentum, relu);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    const T* none = nullptr;
+    const float* nof = nullptr;
+    if (bn_clear(part, C, st) != cudaSuccess) return -1;
+    if (launch_after(bn_reduce_kernel<T, 0, BX>, bn_grid<BX>(R, C, 6), block, 0, st, xt, none, none, nof, nof, part, R, C, 0) !=
+        cudaSuccess)
+        return -1;
+    const cudaError_t e = launch_after(bn_apply_kernel<T, BX>, bn_grid<BX>(R, C, 2), block, 0, st, xt,
+                                       static_cast<const T*>(res), part, gamma, beta, mean, rstd, run_mean, run_var,
+                                       static_cast<T*>(y), R, C, eps, momentum, relu);
+    return e == cudaSuccess ? 0 : -1;
 }
 template <typename T, int BX>
 static int bn_bwd_launch(const void* x, const void* dy, const void* y, const float* mean, const float* rstd,
@@ -421,12 +488,13 @@ static int bn_bwd_launch(const void* x, const void* dy, const void* y, const flo
                          int C, int relu, cudaStream_t st) {
     const dim3 block(BX, 256 / BX);
     const T *xt = static_cast<const T*>(x), *dt = static_cast<const T*>(dy), *yt = static_cast<const T*>(y);
-    cudaMemsetAsync(part, 0, 2 * sizeof(float) * C, st);
-    bn_reduce_kernel<T, 1, BX><<<bn_grid<BX>(R, C, 4), block, 0, st>>>(xt, dt, yt, mean, rstd, part, R, C, relu);
-    bn_bwd_apply_kernel<T, BX><<<bn_grid<BX>(R, C, 4), block, 0, st>>>(xt, dt, yt, part, mean, rstd, gamma, dgamma, dbeta,
-                                                                       static_cast<T*>(dx), static_cast<T*>(dres), R, C,
-                                                                       relu);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    if (bn_clear(part, C, st) != cudaSuccess) return -1;
+    if (launch_after(bn_reduce_kernel<T, 1, BX>, bn_grid<BX>(R, C, 4), block, 0, st, xt, dt, yt, mean, rstd, part, R, C, relu) !=
+        cudaSuccess)
+        return -1;
+    const cudaError_t e = launch_after(bn_bwd_apply_kernel<T, BX>, bn_grid<BX>(R, C, 2), block, 0, st, xt, dt, yt, part, mean,
+                                       rstd, gamma, dgamma, dbeta, static_cast<T*>(dx), static_cast<T*>(dres), R, C, relu);
+    return e == cudaSuccess ? 0 : -1;
 }
 
 static inline int ew_grid(long long n) {
@@ -478,9 +546,10 @@ extern "C" int rb_col2im(const void* dcols, void* dx, int N, int H, int W, int C
 extern "C" int rb_pad_nhwc(const void* x, void* out, int N, int H, int W, int C, int pad, void* stream) {
     if (C % 8 || pad < 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15)) return -2;
     if (N <= 0 || H <= 0 || W <= 0) return 0;
-    rb::pad_nhwc_kernel<<<static_cast<unsigned>(N) * (H + pad), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint4*>(x), static_cast<uint4*>(out), H, W, C / 8, pad);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return rb::launch_after(rb::pad_nhwc_kernel, static_cast<unsigned>(N) * (H + pad), 256, 0, static_cast<cudaStream_t>(stream),
+                            static_cast<const uint4*>(x), static_cast<uint4*>(out), H, W, C / 8, pad) == cudaSuccess
+               ? 0
+               : -1;
 }
 
 // 16-bit filter src [Co, Ci, taps] -> dst [Co, taps, Ci]

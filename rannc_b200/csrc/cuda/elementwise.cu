@@ -14,6 +14,7 @@
 #include <type_traits>
 
 #include "debug_check.cuh"
+#include "launch.cuh"
 #include "philox.cuh"
 #include "tc_common.cuh"
 
@@ -171,6 +172,8 @@ struct Unstack3 {
 };
 template <typename T, typename SrcT>
 __global__ void __launch_bounds__(256) unstack3_kernel(const Unstack3 u) {
+    grid_trigger();
+    grid_wait();
     const long long wv = u.wn / 8, bv = u.b ? u.bn / 8 : 0, total = 3 * (wv + bv);
     for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
         const bool is_w = i < 3 * wv;
@@ -208,15 +211,23 @@ __global__ void cast_kernel(T* __restrict__ dst, const float* __restrict__ src, 
 
 // out[r, :] = table[ids[r], :]  (H % 8 == 0); one warp per row
 template <typename T>
-__global__ void embed_fwd_kernel(const long long* __restrict__ ids, const T* __restrict__ table,
-                                 T* __restrict__ out, int rows, int H, long long vocab) {
+__global__ void embed_fwd_kernel(const long long* ids, const T* table, T* out, int rows, int H, long long vocab) {
+    grid_trigger();
+    grid_wait();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= rows) return;
     long long id = ids[warp];
     const bool ok = id >= 0 && id < vocab;
     const uint4* src = reinterpret_cast<const uint4*>(table + (ok ? id : 0) * H);
     uint4* dst = reinterpret_cast<uint4*>(out + static_cast<long long>(warp) * H);
-    for (int i = lane; i < H / 8; i += 32) dst[i] = ok ? src[i] : make_uint4(0, 0, 0, 0);
+    for (int i = lane; i < H / 8; i += 4 * 32) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = ok && i + u * 32 < H / 8 ? src[i + u * 32] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i + u * 32 < H / 8) dst[i + u * 32] = v[u];
+    }
 }
 
 // dtable(fp32)[ids[r], :] += dout[r, :] ; rows with id == padding_idx are skipped
@@ -239,12 +250,14 @@ __global__ void embed_bwd_kernel(const long long* __restrict__ ids, const T* __r
 // column; equal neighbours (segments, padding) cost one reduction per strip here.  Ids that differ cost the same
 // 32-byte sectors as before in a quarter of the instructions.  (8 columns per thread, as two 16-byte reductions 32
 // bytes apart from lane to lane, touches every sector twice and was slower than the scalar kernel on such ids.)
-// Word, position and segment tables for 32 x 512 tokens x 1024: 107 -> 32.5 us.
+// Word, position and segment tables for 32 x 512 tokens x 1024: 107 -> 32.5 us; begun beside the end of the kernel before,
+// as are the lookups, 43.6 -> 39.7 us one behind the other.
 template <typename T, int STRIP>
 __global__ void __launch_bounds__(256)
-    embed_bwd_vec_kernel(const long long* __restrict__ ids, const T* __restrict__ dout,
-                         float* __restrict__ dtable, int rows, int nv, long long vocab,
+    embed_bwd_vec_kernel(const long long* ids, const T* dout, float* dtable, int rows, int nv, long long vocab,
                          long long padding_idx) {
+    grid_trigger();
+    grid_wait();
     constexpr int FLIGHT = STRIP < 8 ? STRIP : 8;   // rows on their way at a time
     const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
     const long long strip = t / nv;
@@ -419,11 +432,9 @@ extern "C" int rb_unstack3(const void* w, int w_fp32, const float* b, void* cons
     if (off16(w, b) || off16(u.wd[0], u.wd[1], u.wd[2], u.bd[0], u.bd[1], u.bd[2])) return -5;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int g = grid_for(3 * (wn + (b ? bn : 0)) / 8, 256);
-    if (dtype == 1)
-        (w_fp32 ? unstack3_kernel<__nv_bfloat16, float> : unstack3_kernel<__nv_bfloat16, uint16_t>)<<<g, 256, 0, st>>>(u);
-    else
-        (w_fp32 ? unstack3_kernel<__half, float> : unstack3_kernel<__half, uint16_t>)<<<g, 256, 0, st>>>(u);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    const auto kern = dtype == 1 ? (w_fp32 ? unstack3_kernel<__nv_bfloat16, float> : unstack3_kernel<__nv_bfloat16, uint16_t>)
+                                 : (w_fp32 ? unstack3_kernel<__half, float> : unstack3_kernel<__half, uint16_t>);
+    return launch_after(kern, g, 256, 0, st, u) == cudaSuccess ? 0 : -1;
 }
 
 extern "C" int rb_embed_fwd(const long long* ids, const void* table, void* out, int rows, int H,
@@ -435,14 +446,12 @@ extern "C" int rb_embed_fwd(const long long* ids, const void* table, void* out, 
     if (off16(table, out)) return -5;
     RB_DEBUG_RANGE(ids, rows, 0, vocab, -1 - vocab, st);
     const int g = (rows * 32 + 255) / 256;
-    if (dtype == 1)
-        embed_fwd_kernel<__nv_bfloat16><<<g, 256, 0, st>>>(
-            ids, static_cast<const __nv_bfloat16*>(table), static_cast<__nv_bfloat16*>(out), rows,
-            H, vocab);
-    else
-        embed_fwd_kernel<__half><<<g, 256, 0, st>>>(ids, static_cast<const __half*>(table),
-                                                   static_cast<__half*>(out), rows, H, vocab);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    const cudaError_t e =
+        dtype == 1 ? launch_after(embed_fwd_kernel<__nv_bfloat16>, g, 256, 0, st, ids, static_cast<const __nv_bfloat16*>(table),
+                                  static_cast<__nv_bfloat16*>(out), rows, H, vocab)
+                   : launch_after(embed_fwd_kernel<__half>, g, 256, 0, st, ids, static_cast<const __half*>(table),
+                                  static_cast<__half*>(out), rows, H, vocab);
+    return e == cudaSuccess ? 0 : -1;
 }
 
 extern "C" int rb_embed_bwd(const long long* ids, const void* dout, float* dtable, int rows, int H,
@@ -460,16 +469,12 @@ extern "C" int rb_embed_bwd(const long long* ids, const void* dout, float* dtabl
         const unsigned blocks = static_cast<unsigned>((threads + 255) / 256);
         auto go = [&](auto* d) {
             using T = std::remove_const_t<std::remove_pointer_t<decltype(d)>>;
-            if (longer)
-                embed_bwd_vec_kernel<T, 16><<<blocks, 256, 0, st>>>(ids, d, dtable, rows, nv, vocab, padding_idx);
-            else
-                embed_bwd_vec_kernel<T, 4><<<blocks, 256, 0, st>>>(ids, d, dtable, rows, nv, vocab, padding_idx);
+            return launch_after(longer ? embed_bwd_vec_kernel<T, 16> : embed_bwd_vec_kernel<T, 4>, blocks, 256, 0, st, ids, d,
+                                dtable, rows, nv, vocab, padding_idx);
         };
-        if (dtype == 1)
-            go(static_cast<const __nv_bfloat16*>(dout));
-        else
-            go(static_cast<const __half*>(dout));
-        return cudaGetLastError() == cudaSuccess ? 0 : -1;
+        const cudaError_t e =
+            dtype == 1 ? go(static_cast<const __nv_bfloat16*>(dout)) : go(static_cast<const __half*>(dout));
+        return e == cudaSuccess ? 0 : -1;
     }
     const int g = (rows * 32 + 255) / 256;
     if (dtype == 1)

@@ -15,6 +15,7 @@
 #include <stdint.h>
 
 #include "debug_check.cuh"
+#include "launch.cuh"
 #include "tc_common.cuh"
 
 namespace rb {
@@ -30,10 +31,11 @@ __device__ __forceinline__ void online_merge(float& m, float& s, float m2, float
 
 template <typename T>
 __global__ void __launch_bounds__(XT)
-    xent_fwd_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
-                    float* __restrict__ lse_out, float* __restrict__ acc, int V, long long ld,
+    xent_fwd_kernel(const T* logits, const long long* labels, float* lse_out, float* acc, int V, long long ld,
                     long long ignore_index) {
     __shared__ float sm_m[XT / 32], sm_s[XT / 32];
+    grid_trigger();
+    grid_wait();
     const int row = blockIdx.x;
     const long long label = labels[row];
     if (label == ignore_index || label < 0 || label >= V) {
@@ -89,17 +91,18 @@ __global__ void __launch_bounds__(XT)
 }
 
 // loss[0] = weight * acc[0] / max(acc[1], 1)
-__global__ void xent_finalize_kernel(const float* __restrict__ acc, float* __restrict__ loss,
-                                     float weight) {
+__global__ void xent_finalize_kernel(const float* acc, float* loss, float weight) {
+    grid_trigger();
+    grid_wait();
     loss[0] = weight * acc[0] / fmaxf(acc[1], 1.f);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(XT)
-    xent_bwd_kernel(const T* __restrict__ logits, const long long* __restrict__ labels,
-                    const float* __restrict__ lse_in, const float* __restrict__ acc,
-                    const float* __restrict__ gout, T* __restrict__ dlogits, int V, int cols, long long ld,
-                    long long ignore_index, float weight) {
+    xent_bwd_kernel(const T* logits, const long long* labels, const float* lse_in, const float* acc, const float* gout,
+                    T* dlogits, int V, int cols, long long ld, long long ignore_index, float weight) {
+    grid_trigger();
+    grid_wait();
     const int row = blockIdx.x;
     const long long label = labels[row];
     const bool live = !(label == ignore_index || label < 0 || label >= V);
@@ -112,12 +115,20 @@ __global__ void __launch_bounds__(XT)
     // the row's own columns, padding [V, cols) included, which is cleared; what lies between cols and ld belongs to
     // another tensor (the logits may be a slice of a wider matrix)
     const int nv = vec ? cols / 8 : 0;
-    if (vec) {
-        for (int i = threadIdx.x; i < nv; i += XT) {
-            uint4 q = make_uint4(0, 0, 0, 0);
-            if (live) {
-                q = *reinterpret_cast<const uint4*>(x + i * 8);
-                T* e = reinterpret_cast<T*>(&q);
+    if (!live) {
+#pragma unroll 4
+        for (int i = threadIdx.x; i < nv; i += XT) *reinterpret_cast<uint4*>(d + i * 8) = make_uint4(0, 0, 0, 0);
+    } else {
+        for (int i0 = threadIdx.x; i0 < nv; i0 += 4 * XT) {   // (the loads of four vectors, then their stores: d may be x)
+            uint4 q[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + u * XT < nv) q[u] = *reinterpret_cast<const uint4*>(x + (i0 + u * XT) * 8);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * XT;
+                if (i >= nv) break;
+                T* e = reinterpret_cast<T*>(&q[u]);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const int c = i * 8 + j;
@@ -125,8 +136,8 @@ __global__ void __launch_bounds__(XT)
                     if (c == label) v -= 1.f;
                     e[j] = from_f32<T>(v * g);
                 }
+                *reinterpret_cast<uint4*>(d + i * 8) = q[u];
             }
-            *reinterpret_cast<uint4*>(d + i * 8) = q;
         }
     }
     for (int c = nv * 8 + threadIdx.x; c < cols; c += XT) {
@@ -150,15 +161,14 @@ extern "C" int rb_xent_fwd(const void* logits, const long long* labels, float* l
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     RB_DEBUG_RANGE(labels, rows, 0, V, ignore_index, st);
     if (rows > 0) {
-        if (dtype == 1)
-            xent_fwd_kernel<__nv_bfloat16><<<rows, XT, 0, st>>>(
-                static_cast<const __nv_bfloat16*>(logits), labels, lse, acc, V, ld, ignore_index);
-        else
-            xent_fwd_kernel<__half><<<rows, XT, 0, st>>>(static_cast<const __half*>(logits), labels,
-                                                        lse, acc, V, ld, ignore_index);
+        const cudaError_t e =
+            dtype == 1 ? launch_after(xent_fwd_kernel<__nv_bfloat16>, rows, XT, 0, st, static_cast<const __nv_bfloat16*>(logits),
+                                      labels, lse, acc, V, ld, ignore_index)
+                       : launch_after(xent_fwd_kernel<__half>, rows, XT, 0, st, static_cast<const __half*>(logits), labels, lse,
+                                      acc, V, ld, ignore_index);
+        if (e != cudaSuccess) return -1;
     }
-    xent_finalize_kernel<<<1, 1, 0, st>>>(acc, loss, weight);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    return launch_after(xent_finalize_kernel, 1, 1, 0, st, acc, loss, weight) == cudaSuccess ? 0 : -1;
 }
 
 // cols: columns of the logits (V and padding), rows ld apart
@@ -168,13 +178,10 @@ extern "C" int rb_xent_bwd(const void* logits, const long long* labels, const fl
                            void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (rows <= 0) return 0;
-    if (dtype == 1)
-        xent_bwd_kernel<__nv_bfloat16><<<rows, XT, 0, st>>>(
-            static_cast<const __nv_bfloat16*>(logits), labels, lse, acc, gout,
-            static_cast<__nv_bfloat16*>(dlogits), V, cols, ld, ignore_index, weight);
-    else
-        xent_bwd_kernel<__half><<<rows, XT, 0, st>>>(static_cast<const __half*>(logits), labels,
-                                                     lse, acc, gout, static_cast<__half*>(dlogits),
-                                                     V, cols, ld, ignore_index, weight);
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    const cudaError_t e =
+        dtype == 1 ? launch_after(xent_bwd_kernel<__nv_bfloat16>, rows, XT, 0, st, static_cast<const __nv_bfloat16*>(logits),
+                                  labels, lse, acc, gout, static_cast<__nv_bfloat16*>(dlogits), V, cols, ld, ignore_index, weight)
+                   : launch_after(xent_bwd_kernel<__half>, rows, XT, 0, st, static_cast<const __half*>(logits), labels, lse, acc,
+                                  gout, static_cast<__half*>(dlogits), V, cols, ld, ignore_index, weight);
+    return e == cudaSuccess ? 0 : -1;
 }

@@ -662,3 +662,68 @@ def test_attention_forward_bias_by_64_keys(dtype, S, p):
     assert torch.equal(o1[same], o2[same])
     torch.cuda.synchronize()
     assert _lib.read_error() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 129, 1031])
+def test_vectors_moved_four_at_a_time(dtype, n):
+    """n vectors of 16 bytes a row in the kernels that fetch four per thread before they store one: an embedding row, a
+    padded row of an image, a row of the loss gradient (written over the logits and beside them)."""
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(13)
+    table = torch.randn(9, 8 * n, device="cuda").to(dtype)
+    ids = torch.tensor([0, 8, 3, 3, 7], device="cuda")
+    assert torch.equal(K.embed_fwd(ids, table), table[ids])
+
+    x = torch.randn(2, 3, n, 8, device="cuda").to(dtype)
+    for pad in (0, 1, 2):
+        assert torch.equal(K.pad_nhwc(x, pad), torch.nn.functional.pad(x, (0, 0, 0, pad, 0, pad)))
+
+    V = 8 * n - 3     # padding inside the last vector
+    logits = torch.randn(5, 8 * n, device="cuda").to(dtype)
+    labels = torch.tensor([0, V - 1, -100, V // 2, -100], device="cuda")
+    _, lse, acc = K.xent_fwd(logits, labels, V)
+    gout = torch.full((), 1.5, device="cuda")
+    apart = K.xent_bwd(logits, labels, lse, acc, gout, V, inplace=False)
+    p = logits[:, :V].double().softmax(-1)
+    p[torch.arange(5), labels.clamp(min=0)] -= 1
+    want = torch.nn.functional.pad(p * (labels >= 0).double()[:, None] * (1.5 / 3), (0, 3))
+    _near(apart, want, dtype, 1)
+    assert torch.equal(K.xent_bwd(logits, labels, lse, acc, gout, V), apart)
+
+
+@pytest.mark.parametrize("R,C", [(1, 8), (3, 24), (37, 72), (4 * 148 + 1, 2048), (5003, 264)])
+@pytest.mark.parametrize("relu,res", [(False, False), (True, True)])
+def test_batch_norm_rows_two_at_a_time(R, C, relu, res):
+    """Odd numbers of rows per thread, in a chain of launches whose sums start from memory that held NaN."""
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(14)
+    dtype = torch.bfloat16
+    x, dy = (torch.randn(R, C, device="cuda").to(dtype) for _ in range(2))
+    r = torch.randn(R, C, device="cuda").to(dtype) if res else None
+    g, b = torch.rand(C, device="cuda") + 0.5, torch.randn(C, device="cuda")
+    for _ in range(2):
+        junk = [torch.full((2, C), float("nan"), device="cuda") for _ in range(4)]
+        del junk   # (the next allocations of this size get that memory)
+        y, mean, rstd = K.bn_fwd(x, r, g, b, None, None, 1e-5, 0.1, relu)
+    xd = x.double()
+    var = xd.var(0, unbiased=False)
+    xhat = (xd - xd.mean(0)) / (var + 1e-5).sqrt()
+    want = xhat * g + b + (r.double() if res else 0)
+    want = want.relu() if relu else want
+    # sums of squares in fp32: the variance of rows that hardly differ (R = 1: exactly none) loses 2^-22 of the mean square
+    slack = 0.0 if R == 1 else 1e-4
+    if R > 1:
+        _near(y, want, dtype, 1, slack)
+    else:
+        _near(y, (b.double() + (r.double() if res else 0)).relu() if relu else b.double().expand(1, C), dtype, 1, 1e-4)
+    dx, dres, dgamma, dbeta = K.bn_bwd(x, dy, y, mean, rstd, g, relu, res)
+    gd = torch.where(y > 0, dy, torch.zeros_like(dy)).double() if relu else dy.double()
+    _near(dbeta, gd.sum(0), dtype, 0, 1e-5)
+    if res:
+        assert torch.equal(dres.double(), gd)
+    if R > 30:
+        _near(dgamma, (gd * xhat).sum(0), dtype, 0, 1e-4)
+        _near(dx, (gd - gd.mean(0) - xhat * (gd * xhat).mean(0)) * g / (var + 1e-5).sqrt(), dtype, 1, 1e-4)
