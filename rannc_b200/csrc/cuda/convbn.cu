@@ -187,9 +187,9 @@ static int pack_taps_launch(const void* src, void* dst, int Co, int Ci, int taps
 // The weight gradient comes out of its GEMM as src [Co, taps, Ci] fp32 and belongs into a [Co, Ci, taps] tensor:
 // added to an fp32 gradient buffer (ADD) or rounded to a 16-bit gradient.  A block takes 128 channels of one
 // filter through shared memory so that both sides are touched in whole lines; the row stride shifts the banks by four
-// from tap to tap.  For filters from 4 x 4 to 9 x 9: a strided copy reads 4 bytes of every 4 * taps, which costs it
-// 107 us for 1024 x 1024 x 5 x 5 (added to fp32) where this takes 72, but only 37 us for 3 x 3 where this takes 43 --
-// a block's loads, its barrier and its stores follow one another with little in flight.
+// from tap to tap.  For filters from 4 x 4 to 9 x 9 (and any number of channels): a strided copy reads 4 bytes of every
+// 4 * taps, which costs it 107 us for 1024 x 1024 x 5 x 5 (added to fp32) where this takes 72.  Smaller filters have the
+// kernel below: here a block's loads, its barrier and its stores follow one another with little in flight.
 constexpr int FOLD_C = 128, FOLD_LD = FOLD_C + 4;
 template <typename OutT, bool ADD>
 __global__ void __launch_bounds__(256)
@@ -214,6 +214,74 @@ __global__ void __launch_bounds__(256)
         else
             dst[i] = from_f32<OutT>(v);
     }
+}
+
+// The same for the filters of 2 x 2 and 3 x 3, whose taps are known to the compiler: what is added to, and the 256
+// channels of every tap (a warp has one), are on their way to a block before it waits for either, in 16-byte pieces, and
+// the results leave in such.  Bound by memory.  us, the strided operation and this, added to fp32 and rounded to 16 bits:
+// 512 x 512 x 3 x 3 8.4 -> 3.7 and 8.4 -> 2.9, 1024 x 1024 24.7 -> 10.7 and 20.6 -> 7.7, 2048 x 2048 (from memory) 121 -> 66
+// and 80 -> 36, 1024 x 1024 x 2 x 2 12.5 -> 5.9 and 10.6 -> 3.9; 128 channels a block: 11.5 where this takes 10.7.
+constexpr int FEW_C = 256;
+template <typename OutT, bool ADD, int TAPS>
+__global__ void __launch_bounds__(TAPS * 32)
+    wgrad_fold_few_kernel(const float* src, OutT* dst, int Ci, int chunks) {
+    constexpr int U = FEW_C / 128, LD = FEW_C + 4, V = 16 / sizeof(OutT);
+    constexpr int OUTS = FEW_C / V / 32;   // vectors of the result a thread writes
+    __shared__ __align__(16) float tile[TAPS * LD];
+    grid_wait();
+    const int co = blockIdx.x / chunks, c0 = (blockIdx.x - co * chunks) * FEW_C, nc = min(FEW_C, Ci - c0);
+    src += static_cast<long long>(co) * TAPS * Ci + c0;
+    dst += (static_cast<long long>(co) * Ci + c0) * TAPS;
+    const int nv = nc * TAPS / V;
+    uint4 old[OUTS];
+    if constexpr (ADD) {
+#pragma unroll
+        for (int u = 0; u < OUTS; ++u) {
+            const int i = threadIdx.x + u * TAPS * 32;
+            if (i < nv) old[u] = reinterpret_cast<const uint4*>(dst)[i];
+        }
+    }
+    float4 in[U];
+    const int t = threadIdx.x >> 5, lane = threadIdx.x & 31;   // a warp has a tap
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int c = (u * 32 + lane) * 4;
+        if (c < nc) in[u] = *reinterpret_cast<const float4*>(src + static_cast<long long>(t) * Ci + c);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) *reinterpret_cast<float4*>(tile + t * LD + (u * 32 + lane) * 4) = in[u];
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < OUTS; ++u) {
+        const int i = threadIdx.x + u * TAPS * 32;
+        if (i >= nv) break;
+        float v[V];
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+            const int e = i * V + j, c = e / TAPS;
+            v[j] = tile[(e - c * TAPS) * LD + c];
+        }
+        if constexpr (ADD) {
+            const float* o = reinterpret_cast<const float*>(&old[u]);
+            reinterpret_cast<float4*>(dst)[i] = make_float4(o[0] + v[0], o[1] + v[1], o[2] + v[2], o[3] + v[3]);
+        } else {
+            st8(dst + i * V, v);
+        }
+    }
+}
+template <int TAPS>
+static int wgrad_fold_few(const float* src, void* dst, int Co, int Ci, int dtype, cudaStream_t st) {
+    const int chunks = (Ci + FEW_C - 1) / FEW_C;
+    if (static_cast<long long>(Co) * chunks > 0x7fffffffLL) return -2;
+    const unsigned grid = static_cast<unsigned>(Co) * chunks;
+    const cudaError_t e =
+        dtype == 2   ? launch_after(wgrad_fold_few_kernel<float, true, TAPS>, grid, TAPS * 32, 0, st, src,
+                                    static_cast<float*>(dst), Ci, chunks)
+        : dtype == 1 ? launch_after(wgrad_fold_few_kernel<__nv_bfloat16, false, TAPS>, grid, TAPS * 32, 0, st, src,
+                                    static_cast<__nv_bfloat16*>(dst), Ci, chunks)
+                     : launch_after(wgrad_fold_few_kernel<__half, false, TAPS>, grid, TAPS * 32, 0, st, src,
+                                    static_cast<__half*>(dst), Ci, chunks);
+    return e == cudaSuccess ? 0 : -1;
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -561,6 +629,16 @@ extern "C" int rb_pack_taps(const void* src, void* dst, int Co, int Ci, int taps
     const auto fits = [&](int ch) { return taps * (ch + 8) * 2 <= 48 * 1024; };
     if (fits(256)) return pack_taps_launch<256>(src, dst, Co, Ci, taps, st);
     return fits(64) ? pack_taps_launch<64>(src, dst, Co, Ci, taps, st) : pack_taps_launch<16>(src, dst, Co, Ci, taps, st);
+}
+
+// rb_wgrad_fold for 4 or 9 taps, Ci a multiple of 8, both addresses on 16-byte boundaries
+extern "C" int rb_wgrad_fold_few(const float* src, void* dst, int Co, int Ci, int taps, int dtype, void* stream) {
+    using namespace rb;
+    if (Co <= 0 || Ci <= 0 || taps <= 0) return 0;
+    if (Ci % 8 || (taps != 4 && taps != 9)) return -2;
+    if (off16(src, dst)) return -5;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    return taps == 4 ? wgrad_fold_few<4>(src, dst, Co, Ci, dtype, st) : wgrad_fold_few<9>(src, dst, Co, Ci, dtype, st);
 }
 
 // src fp32 [Co, taps, Ci] into dst [Co, Ci, taps]; dtype 2: added to fp32, 1 / 0: written as bf16 / fp16

@@ -382,12 +382,17 @@ class _Conv2d(torch.autograd.Function):
         """The tap-major fp32 weight gradient into the fp32 gradient buffer, or as a gradient of w's own type."""
         Co, Ci = w.shape[:2]
         if w_mg is not None:
-            if w_mg.dtype == torch.float32 and K.wgrad_fold_ok(w_mg):
+            if w_mg.dtype == torch.float32 and K.wgrad_fold_few_ok(w_mg):
+                K.wgrad_fold_few(dw2, w_mg, k * k)
+            elif w_mg.dtype == torch.float32 and K.wgrad_fold_ok(w_mg):
                 K.wgrad_fold(dw2, w_mg, k * k)
             else:
                 w_mg.add_(dw2.view(Co, k, k, Ci).permute(0, 3, 1, 2))
             return None
         dw = torch.empty(w.shape, dtype=w.dtype, device=w.device)
+        if K.wgrad_fold_few_ok(dw) and dw.dtype != torch.float32:
+            K.wgrad_fold_few(dw2, dw, k * k)
+            return dw
         if K.wgrad_fold_ok(dw) and dw.dtype != torch.float32:
             K.wgrad_fold(dw2, dw, k * k)
             return dw

@@ -311,12 +311,26 @@ def pack_taps(w):
 
 def wgrad_fold_ok(dst) -> bool:
     """Whether ``wgrad_fold`` should serve this [Co, Ci, k, k] destination.  It can up to 9 x 9 (a row of 132 floats per tap
-    within 48 KiB of shared memory) and 65535 filters (one grid row each).  Up to 3 x 3 a strided copy or addition is
-    faster (us, kernel / strided: 1024 x 1024 x 3 x 3 added to fp32 43 / 37, rounded to 16 bits 35 / 27; 2048 x 2048 139 /
-    125 and 113 / 86), from 5 x 5 on the kernel (1024 x 1024 x 5 x 5 72 / 107 and 57 / 80; 7 x 7 125 / 229 and 92 / 182):
-    the strided side reads 4 bytes of every k * k * 4."""
+    within 48 KiB of shared memory) and 65535 filters (one grid row each).  From 5 x 5 on it is faster than a strided copy
+    or addition (us, kernel / strided: 1024 x 1024 x 5 x 5 added to fp32 72 / 107, rounded to 16 bits 57 / 80; 7 x 7 125 /
+    229 and 92 / 182): the strided side reads 4 bytes of every k * k * 4.  Up to 3 x 3 it is not (43 / 37, 35 / 27);
+    ``wgrad_fold_few`` is."""
     return (dst.is_cuda and dst.is_contiguous() and dst.shape[0] <= 65535 and 9 < dst.shape[2] * dst.shape[3] <= 93 and
             dst.dtype in (torch.bfloat16, torch.float16, torch.float32))
+
+
+def wgrad_fold_few_ok(dst) -> bool:
+    """Whether ``wgrad_fold_few`` takes this [Co, Ci, k, k] destination: 2 x 2 or 3 x 3, in 16-byte pieces on both sides.
+    Always faster than the strided operation (us, kernel / strided: 64 x 64 x 3 x 3 1.4 / 4.2, 1024 x 1024 10.7 / 24.7)."""
+    return (dst.is_cuda and dst.is_contiguous() and dst.shape[2] * dst.shape[3] in (4, 9) and dst.shape[1] % 8 == 0 and
+            dst.data_ptr() % 16 == 0 and dst.dtype in (torch.bfloat16, torch.float16, torch.float32))
+
+
+def wgrad_fold_few(dw2d, dst, taps: int):
+    """As ``wgrad_fold``, for the destinations of ``wgrad_fold_few_ok``."""
+    Co, Ci = dst.shape[0], dst.shape[1]
+    _lib.check(_lib.lib().rb_wgrad_fold_few(_lib.vp(dw2d), _lib.vp(dst), c_int(Co), c_int(Ci), c_int(taps),
+                                            c_int(dt_code(dst)), _lib.stream_ptr()), "rb_wgrad_fold_few")
 
 
 def wgrad_fold(dw2d, dst, taps: int):

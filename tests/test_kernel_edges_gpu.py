@@ -727,3 +727,31 @@ def test_batch_norm_rows_two_at_a_time(R, C, relu, res):
     if R > 30:
         _near(dgamma, (gd * xhat).sum(0), dtype, 0, 1e-4)
         _near(dx, (gd - gd.mean(0) - xhat * (gd * xhat).mean(0)) * g / (var + 1e-5).sqrt(), dtype, 1, 1e-4)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("k", [2, 3])
+@pytest.mark.parametrize("Co,Ci", [(1, 8), (5, 72), (3, 256), (2, 264), (7, 1032)])
+def test_weight_gradient_of_small_filters_folded(dtype, k, Co, Ci):
+    """Chunks of 256 channels and what is left of them, to the bit; a destination off a 16-byte boundary and a channel count
+    that is no multiple of 8 take the strided operation."""
+    from rannc_b200.ops import functional as RF
+
+    torch.manual_seed(15)
+    for ci, off in ((Ci, 0), (Ci, 1), (Ci + 4, 0)):
+        n = Co * ci * k * k
+        dw2 = torch.randn(Co, k * k * ci, device="cuda")
+        want = dw2.view(Co, k, k, ci).permute(0, 3, 1, 2)
+        mg = torch.full((n + 9,), 0.5, device="cuda", dtype=dtype)
+        dst = mg[off:off + n].view(Co, ci, k, k)
+        fast = off == 0 and ci % 8 == 0
+        assert RF.K.wgrad_fold_few_ok(dst) == fast
+        if dtype == torch.float32:
+            assert RF._Conv2d._fold(dw2, dst, dst, k) is None
+            assert torch.equal(dst, 0.5 + want)
+        else:
+            assert torch.equal(RF._Conv2d._fold(dw2, dst, None, k), want.to(dtype))
+            if fast:
+                RF.K.wgrad_fold_few(dw2, dst, k * k)
+                assert torch.equal(dst, want.to(dtype))
+        assert (mg[:off] == 0.5).all() and (mg[off + n:] == 0.5).all()
