@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(256)
 // A filter [Co, Ci, taps] as the GEMM reads it, [Co, taps, Ci]; 16-bit elements, Ci a multiple of 8.  A block takes CH
 // channels of one filter through shared memory, so that both sides move in 16-byte pieces of consecutive addresses (a
 // generic strided copy reads 2 bytes of every 18: 1024 x 1024 x 3 x 3 took 258 us that way and takes 10.3 us here,
-// 2048 x 2048 333 and 40 us, 3.7 TB/s).  The padded rows shift the banks by four from tap to tap.  CH shrinks as the taps grow, to stay below 48 KiB.
+// 2048 x 2048 333 and 39 us).  The padded rows shift the banks by four from tap to tap.  CH shrinks as the taps grow, to stay below 48 KiB.
 template <int CH>
 __global__ void __launch_bounds__(256)
     pack_taps_kernel(const uint16_t* src, uint16_t* dst, int Ci, int taps, int chunks) {
@@ -173,6 +173,38 @@ __global__ void __launch_bounds__(256)
         const int t = v / row, c = (v - t * row) * 8;
         *reinterpret_cast<uint4*>(to + static_cast<long long>(t) * Ci + c) = *reinterpret_cast<const uint4*>(tile + t * LD + c);
     }
+}
+// The same for 2 x 2 and 3 x 3 filters, 256 channels a block: the 8 * TAPS values of eight channels lie in shared memory as
+// they came, one word more apart, so that a thread's eight gathered values and its neighbours' are in different banks.
+// us, the kernel above and this: 64 x 64 x 3 x 3 1.7 -> 1.4, 1024 x 1024 10.3 -> 6.0, 2048 x 2048 39 -> 28 (5.3 TB/s),
+// 1024 x 1024 x 2 x 2 6.6 -> 3.8.  (There a thread's values go to shared memory one by one, four to a bank.)
+template <int TAPS>
+__global__ void __launch_bounds__(TAPS * 32)
+    pack_few_kernel(const uint4* src, uint4* dst, int Ci, int chunks) {
+    constexpr int LD = 8 * TAPS / 2 + 1;   // words of eight channels
+    __shared__ uint32_t tile[32 * LD];
+    grid_wait();
+    const int co = blockIdx.x / chunks, g0 = (blockIdx.x - co * chunks) * 32, ng = min(32, Ci / 8 - g0);   // groups of 8
+    const int i = threadIdx.x, t = i >> 5, lane = i & 31;
+    if (i < ng * TAPS) {
+        const uint4 q = src[(static_cast<long long>(co) * (Ci / 8) + g0) * TAPS + i];
+        uint32_t* to = tile + i / TAPS * LD + i % TAPS * 4;
+        to[0] = q.x, to[1] = q.y, to[2] = q.z, to[3] = q.w;
+    }
+    __syncthreads();
+    if (lane >= ng) return;
+    const uint16_t* e = reinterpret_cast<const uint16_t*>(tile + lane * LD) + t;
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = e[2 * j * TAPS] | static_cast<uint32_t>(e[(2 * j + 1) * TAPS]) << 16;
+    dst[(static_cast<long long>(co) * TAPS + t) * (Ci / 8) + g0 + lane] = make_uint4(w[0], w[1], w[2], w[3]);
+}
+template <int TAPS>
+static int pack_few_launch(const void* src, void* dst, int Co, int Ci, cudaStream_t st) {
+    const int chunks = (Ci + 255) / 256;
+    if (static_cast<long long>(Co) * chunks > 0x7fffffffLL) return -2;
+    return launch_after(pack_few_kernel<TAPS>, static_cast<unsigned>(Co) * chunks, TAPS * 32, 0, st,
+                        static_cast<const uint4*>(src), static_cast<uint4*>(dst), Ci, chunks) == cudaSuccess ? 0 : -1;
 }
 template <int CH>
 static int pack_taps_launch(const void* src, void* dst, int Co, int Ci, int taps, cudaStream_t st) {
@@ -626,6 +658,8 @@ extern "C" int rb_pack_taps(const void* src, void* dst, int Co, int Ci, int taps
     if (Co <= 0 || Ci <= 0 || taps <= 0) return 0;
     if (Ci % 8 || taps > 1024 || ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15)) return -2;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (taps == 9) return pack_few_launch<9>(src, dst, Co, Ci, st);
+    if (taps == 4) return pack_few_launch<4>(src, dst, Co, Ci, st);
     const auto fits = [&](int ch) { return taps * (ch + 8) * 2 <= 48 * 1024; };
     if (fits(256)) return pack_taps_launch<256>(src, dst, Co, Ci, taps, st);
     return fits(64) ? pack_taps_launch<64>(src, dst, Co, Ci, taps, st) : pack_taps_launch<16>(src, dst, Co, Ci, taps, st);

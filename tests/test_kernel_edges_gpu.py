@@ -755,3 +755,15 @@ def test_weight_gradient_of_small_filters_folded(dtype, k, Co, Ci):
                 RF.K.wgrad_fold_few(dw2, dst, k * k)
                 assert torch.equal(dst, want.to(dtype))
         assert (mg[:off] == 0.5).all() and (mg[off + n:] == 0.5).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("k", [2, 3, 5])
+@pytest.mark.parametrize("Co,Ci", [(1, 8), (5, 72), (3, 256), (2, 264), (7, 1032)])
+def test_filters_packed_by_tap(dtype, k, Co, Ci):
+    """Chunks of 256 channels and what is left of them, to the bit."""
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(16)
+    w = torch.randn(Co, Ci, k, k, device="cuda").to(dtype)
+    assert torch.equal(K.pack_taps(w), w.permute(0, 2, 3, 1).reshape(Co, -1))
