@@ -1178,20 +1178,22 @@ struct Tiling {
 //    over take the remaining steps of one tile after another, in at most six rounds.
 // What it is worth (us, whole tiles -> shared; the matrix comes from memory, as a gradient buffer does; w + t: full waves
 // and tiles left over):
-//     w + t     K = 512        1024           1536           2048           4096           8192
-//     1 + 14    25.6 -> 23.6   31.8 -> 28.7   35.9 -> 31.7   42.0 -> 35.9   64.4 -> 48.1   108 -> 75
-//     1 + 36    25.5 -> 25.6   30.7 -> 29.6   35.8 -> 33.8   41.9 -> 37.9   64.5 -> 55.6   107 -> 88
-//     3 + 34    42.0 -> 43.0   50.2 -> 52.1   61.5 -> 59.4   72.7 -> 68.6   117 -> 108     208 -> 187
-//     6 + 36    64.5 -> 67.5   77.8 -> 78.0   97.1 -> 93.2   115 -> 109     195 -> 185     373 -> 352
-//     1 + 46 (two rounds)                     35.9 -> 34.9   42.0 -> 39.9   65.6 -> 59.3   108 -> 95
-//     3 + 50 (three)                                                        118 -> 114     209 -> 200
-//     1 + 58 (four)                                                         61.1 -> 58.4   109 -> 103
-//     1 + 62 (six), 2 + 68 (twelve), 1 + 70 (eighteen) by 16384: 209 -> 202, 327 -> 328, 217 -> 222
+//     w + t          K = 1024       1536           2048           4096           8192
+//     1 + 14         27.5 -> 26.7   32.8 -> 28.7   36.9 -> 32.8   57.3 -> 43.1   94.2 -> 65.6
+//     1 + 36                        32.8 -> 30.8   36.9 -> 34.8   57.4 -> 51.1   96.3 -> 79.9
+//     3 + 34                        57.3 -> 55.3   65.6 -> 62.5   102 -> 94.2    184 -> 167
+//     6 + 36                        88.1 -> 86.1   102 -> 98.3    176 -> 166     347 -> 328
+//     1 + 46 (two rounds)           37.9 -> 37.9   42.0 -> 39.9   62.5 -> 56.4   104 -> 91.2
+//     3 + 50 (three)                                              104 -> 100     187 -> 178
+//     1 + 58 (four)                                               61.4 -> 57.5   100 -> 95.2
+//     1 + 62 (six) by 16384: 185 -> 178
+// and with copies that took longer to issue, where it is not used: 1 + 36 and 3 + 34 by 512 25.5 -> 25.6 and 42.0 -> 43.0, by
+// 1024 30.7 -> 29.6 and 50.2 -> 52.1; 2 + 68 (twelve rounds) and 1 + 70 (eighteen) by 16384 327 -> 328 and 217 -> 222.
 // With a short K the matrix bounds the product and a part's addition to it costs what the part saves: from 24 steps on, or
 // where one full wave is followed by a third of one at most.  Beyond six rounds the helpers' additions eat up the gain.
-// Only behind full waves: with fewer tiles than pairs this is faster still (4096 x 1024 by 16384, 64 tiles: 129 -> 121 us),
-// but its parts are longer than those of the even split below, and the tensor core's sums lose with length (relative error
-// 2.6e-6 -> 1.6e-5).  Behind full waves parts are shorter than the whole tiles they replace.
+// Only behind full waves: with fewer tiles than pairs its parts are longer than those of the even split below, and the tensor
+// core's sums lose with length (4096 x 1024 by 16384, 64 tiles: 101.0 -> 99.1 us, relative error 2.1e-6 -> 1.6e-5; with parts
+// as long as before, summed in registers, 100.9 us).  Behind full waves parts are shorter than the whole tiles they replace.
 struct Tail {
     int split, kb;       // split > 1: equal parts of kb steps; 1: owners and helpers; 0: whole tiles
     double cost;         // in k steps of the longest chain of a pair
@@ -1257,9 +1259,10 @@ static Tiling choose_tiling(const RbGemmArgs& a) {
         } else {
             // Narrow tiles move more bytes per product but keep more SMs busy.  Estimated cycles: k steps one CTA
             // does, each bound by its loads (48 / 32 / 24 KiB), plus the last tile's epilogue.  Measured with 256 /
-            // 128 / 64 columns (us): 32 x 1024 x 1024 10.1 / 9.0 / 8.5; 351 x 3072 x 768 9.5 / 8.7 / 8.0;
-            // 1182 x 768 x 2304 22.0 / 17.1 / 15.4; 2000 x 1024 x 1024 11.0 / 10.1 / 14.4;
-            // 1182 x 2304 x 768 9.9 / 13.0 / 16.2.  The rule took the best or one within 2 % in 21 of 22 shapes.
+            // 128 / 64 columns (us): 32 x 1024 x 1024 8.8 / 6.8 / 6.5; 351 x 3072 x 768 8.7 / 7.0 / 6.7;
+            // 1182 x 768 x 3072 18.9 / 14.9 / 14.1; 2000 x 1024 x 1024 10.2 / 8.1 / 11.1;
+            // 1182 x 2304 x 768 9.2 / 10.1 / 12.2.  The rule took the best or one within 3 % in 87 of 89 shapes (8 and 32 x
+            // 4096 x 1024: 128 columns are 0.2 to 1 us faster than the 64 it takes).
             double best = 1e30;
             for (int w : {256, 128, 64}) {
                 const int tiles = t.m_blocks * static_cast<int>((a.N + w - 1) / w * a.batch);
