@@ -767,3 +767,67 @@ def test_filters_packed_by_tap(dtype, k, Co, Ci):
     torch.manual_seed(16)
     w = torch.randn(Co, Ci, k, k, device="cuda").to(dtype)
     assert torch.equal(K.pack_taps(w), w.permute(0, 2, 3, 1).reshape(Co, -1))
+
+
+@pytest.mark.parametrize("how", ["captured", "two_streams"])
+def test_small_kernels_in_a_row_under_capture_and_across_streams(how):
+    """Lookup, batch norm, loss and their gradients, each of which begins beside the end of the one before, in a captured
+    graph and with every other kernel on a second stream: what came before is complete."""
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(17)
+    dt, C, rows = torch.bfloat16, 1024, 3001
+    table = torch.randn(64, C, device="cuda").to(dt)
+    ids, labels = (torch.randint(0, n, (rows,), device="cuda") for n in (64, C))
+    g, b, gout = torch.rand(C, device="cuda") + 0.5, torch.randn(C, device="cuda"), torch.ones((), device="cuda")
+    dtable = torch.zeros(64, C, device="cuda")
+    other = torch.cuda.Stream()
+
+    def step(two):
+        here = torch.cuda.current_stream()
+        kept = []
+
+        def on_other(f):
+            if two:
+                other.wait_stream(here)
+            with torch.cuda.stream(other if two else here):
+                out = f()
+            if two:
+                here.wait_stream(other)
+            kept.append(out)   # (alive until both streams are done)
+            return out
+
+        dtable.zero_()
+        e = K.embed_fwd(ids, table)
+        y, mean, rstd = on_other(lambda: K.bn_fwd(e, None, g, b, None, None, 1e-5, 0.1, False))
+        loss, lse, acc = K.xent_fwd(y, labels, C)
+        dy = on_other(lambda: K.xent_bwd(y, labels, lse, acc, gout, C, inplace=False))
+        dx = K.bn_bwd(e, dy, y, mean, rstd, g, False, False)[0]
+        on_other(lambda: K.embed_bwd(ids, dx, dtable))
+        kept.append((e, lse, acc, dx))
+        return loss, kept
+
+    t = table.double().requires_grad_(True)
+    e = t[ids]
+    y = torch.nn.functional.batch_norm(e, None, None, g.double(), b.double(), True, 0.1, 1e-5)
+    want = torch.nn.functional.cross_entropy(y, labels)
+    want.backward()
+    if how == "captured":
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            step(False)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            loss, kept = step(False)
+        for _ in range(3):
+            graph.replay()
+    else:
+        for _ in range(3):
+            loss, kept = step(True)
+    torch.cuda.synchronize()
+    # y, dy and dx are rounded once each, and alike for all tokens of one id: rounding y by U |y| changes its probability by
+    # that factor, dy and dx add U each, and one more covers the sums
+    assert abs(float(loss) - want.item()) <= U[dt] * want.item()
+    scale = t.grad.abs().max()
+    assert (dtable.double() - t.grad).abs().max() <= (y.abs().max() + 3) * U[dt] * scale
