@@ -86,7 +86,8 @@ __device__ __forceinline__ void store_o_rows(const uint32_t (&v)[32], float f, u
 }
 
 // FAST: the sequence fits the staged per-key tables (bias and dropout hash in shared memory)
-template <typename T, bool FAST>
+// HEADS (sequences of one query tile): the two tiles of a block are those of two heads, each with keys and values of its own
+template <typename T, bool FAST, bool HEADS>
 __global__ void __launch_bounds__(ATT_THREADS, 1)
     attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const AttnFwdParams p) {
@@ -113,9 +114,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
 
     // (the same for all lanes, for the compiler too: what the issuing warps compute from it stays in uniform registers)
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const int q_base = blockIdx.x * 2 * AQ, h = blockIdx.y, b = blockIdx.z;
-    const int nchunks = (p.S + AK - 1) / AK;
-    const int ntiles = (q_base + AQ < p.S) ? 2 : 1;
+    const int q_base = blockIdx.x * 2 * AQ, h0 = HEADS ? blockIdx.y * 2 : blockIdx.y, b = blockIdx.z;
+    const int nchunks = HEADS ? 1 : (p.S + AK - 1) / AK;
+    const int ntiles = (HEADS ? h0 + 1 < p.H : q_base + AQ < p.S) ? 2 : 1;
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
@@ -157,17 +158,18 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
     if (warp == 18) {
         // ------------- K / V loader: stage (j & 1) is refilled once every tile's P V of chunk j is done -------------
         if (lane == 0) {
-            auto load_kv = [&](int j) {
-                const int st = j & 1;
+            auto load_kv = [&](int j) {   // (HEADS: of head j, whose tile alone uses stage j)
+                const int st = j & 1, key = HEADS ? 0 : j * AK, h = HEADS ? h0 + j : h0;
                 mbar_arrive_expect_tx(&k_full[st], TILE_B);
-                tma_load_4d(sK + st * TILE_B, &tmK, &k_full[st], 0, j * AK, h, b);
+                tma_load_4d(sK + st * TILE_B, &tmK, &k_full[st], 0, key, h, b);
                 mbar_arrive_expect_tx(&v_full[st], TILE_B);
-                tma_load_4d(sV + st * TILE_B, &tmV, &v_full[st], 0, j * AK, h, b);
+                tma_load_4d(sV + st * TILE_B, &tmV, &v_full[st], 0, key, h, b);
             };
             mbar_arrive_expect_tx(q_full, ntiles * TILE_B);
-            for (int t = 0; t < ntiles; ++t) tma_load_4d(sQ + t * TILE_B, &tmQ, q_full, 0, q_base + t * AQ, h, b);
+            for (int t = 0; t < ntiles; ++t)
+                tma_load_4d(sQ + t * TILE_B, &tmQ, q_full, 0, HEADS ? 0 : q_base + t * AQ, HEADS ? h0 + t : h0, b);
             load_kv(0);
-            if (nchunks > 1) load_kv(1);
+            if (HEADS ? ntiles > 1 : nchunks > 1) load_kv(1);
             for (int j = 0; j + 2 < nchunks; ++j) {
                 if (!mbar_wait(&kv_free[j & 1], (j >> 1) & 1, abort_flag)) break;
                 load_kv(j + 2);
@@ -185,13 +187,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
             const uint32_t idesc_s = make_idesc_f16(fmt, 0, 0, AQ, AK);
             const uint32_t idesc_o = make_idesc_f16(fmt, 0, 1, AQ, AD);
             auto issue_s = [&](int j) {
-                const uint32_t ka = k_desc + (j & 1) * (TILE_B / 16);
+                const uint32_t ka = k_desc + (HEADS ? t : j & 1) * (TILE_B / 16);
 #pragma unroll
                 for (int k = 0; k < AD / 16; ++k)
                     umma_f16_lo(tmem + t * TILE_COLS, q_desc + k * 2, ka + k * 2, idesc_s, k != 0, el);
                 if (el) umma_commit(&s_full[t]);
             };
-            bool ok = mbar_wait_warp(q_full, 0, abort_flag) && mbar_wait_warp(&k_full[0], 0, abort_flag);
+            bool ok = mbar_wait_warp(q_full, 0, abort_flag) && mbar_wait_warp(&k_full[HEADS ? t : 0], 0, abort_flag);
             if (ok) {
                 tc_fence_after();
                 issue_s(0);
@@ -205,10 +207,10 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
                     tc_fence_after();
                     issue_s(j + 1);
                 }
-                ok = mbar_wait_warp(&p_ready[t], j & 1, abort_flag) && mbar_wait_warp(&v_full[j & 1], kv_phase, abort_flag);
+                ok = mbar_wait_warp(&p_ready[t], j & 1, abort_flag) && mbar_wait_warp(&v_full[HEADS ? t : j & 1], kv_phase, abort_flag);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t va = v_desc + (j & 1) * (TILE_B / 16);
+                const uint32_t va = v_desc + (HEADS ? t : j & 1) * (TILE_B / 16);
 #pragma unroll
                 for (int k = 0; k < AK / 16; ++k)
                     umma_f16_lo(tmem + t * TILE_COLS + 128, p_desc + (k >> 2) * (P_BYTES / 32) + (k & 3) * 2, va + k * 128,
@@ -227,7 +229,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
         const int half = idx >> 7;   // which 64 columns of a chunk / 32 columns of O
         const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
         const uint32_t col_s = tmem + t * TILE_COLS, col_o = col_s + 128;
-        const int q = q_base + t * AQ + r;
+        const int q = HEADS ? r : q_base + t * AQ + r, h = HEADS ? h0 + t : h0;
         const float* kbg = p.key_bias ? p.key_bias + static_cast<long long>(b) * p.S : nullptr;
         const uint32_t row_hash = drop_row_hash(p.seed, b, h, q, p.H, p.S);
         float m = -INFINITY, l = 0.f;
@@ -923,16 +925,23 @@ static int launch_fwd(const RbAttnArgs& a, cudaStream_t st) {
                                                                                                                           : -1;
     }
     const bool fast = (a.S + AK - 1) / AK * AK <= KB_MAX;
-    auto kern = fast ? attn_fwd_kernel<T, true> : attn_fwd_kernel<T, false>;
-    static bool attr_set[64][2] = {};
+    // Sequences of one query tile: two heads to a block where that takes fewer waves of blocks (an SM holds one, half of
+    // whose threads would have no tile).  us, one head to a block and two: 64 x 128 x 16 heads 31.9 -> 23.4, with mask and
+    // dropout 36.5 -> 24.3 (100 tokens), 32 x 64 x 16 19.2 -> 11.3, 10 x 128 x 16 (160 heads on 148 SMs) 9.2 -> 6.6; with no
+    // more heads than SMs the second tile only shares its SM: 9 x 128 x 16 6.6 -> 7.0, 4 x 128 x 16 5.1 -> 6.2.
+    const auto waves = [](long long blocks) { return (blocks + num_sms() - 1) / num_sms(); };
+    const bool heads = a.S <= AQ && waves(static_cast<long long>(a.B) * ((a.H + 1) / 2)) < waves(static_cast<long long>(a.B) * a.H);
+    auto kern = heads ? attn_fwd_kernel<T, true, true> : (fast ? attn_fwd_kernel<T, true, false> : attn_fwd_kernel<T, false, false>);
+    static bool attr_set[64][3] = {};
+    const int which = heads ? 2 : fast;
     int dev = 0;
     cudaGetDevice(&dev);
-    if (!attr_set[dev & 63][fast]) {
+    if (!attr_set[dev & 63][which]) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM) != cudaSuccess)
             return -4;
-        attr_set[dev & 63][fast] = true;
+        attr_set[dev & 63][which] = true;
     }
-    dim3 grid((a.S + 2 * AQ - 1) / (2 * AQ), a.H, a.B);
+    dim3 grid((a.S + 2 * AQ - 1) / (2 * AQ), heads ? (a.H + 1) / 2 : a.H, a.B);
     return launch_after(kern, grid, ATT_THREADS, ATT_SMEM, st, tq, tk, tv, p) == cudaSuccess ? 0 : -1;
 }
 

@@ -831,3 +831,31 @@ def test_small_kernels_in_a_row_under_capture_and_across_streams(how):
     assert abs(float(loss) - want.item()) <= U[dt] * want.item()
     scale = t.grad.abs().max()
     assert (dtable.double() - t.grad).abs().max() <= (y.abs().max() + 3) * U[dt] * scale
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("S", [1, 31, 64, 65, 100, 127, 128])
+@pytest.mark.parametrize("B,H", [(75, 2), (80, 3), (40, 7), (20, 16)])
+def test_attention_forward_two_heads_a_block(dtype, S, B, H):
+    """Short sequences with more heads than SMs: two heads to a block (an odd number leaves one alone), to the bit what each
+    batch row gives by itself, where a block has one head."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(18)
+    q, k, v = (t for t in torch.randn(B, S, 3, H, 64, device="cuda").to(dtype).unbind(2))
+    bias = torch.zeros(B, S, device="cuda")
+    bias[1::2, S // 2 + 1:] = -10000.0
+    for kb, p in ((None, 0.0), (bias, 0.0), (bias, 0.25)):
+        o, lse = K.attn_fwd(q, k, v, kb, 0.125, p, 3, 4)
+        for b in range(B) if p == 0 else (0,):   # (a row's dropout depends on its place in the batch)
+            one = slice(b, b + 1)
+            o1, lse1 = K.attn_fwd(q[one], k[one], v[one], None if kb is None else kb[one].contiguous(), 0.125, p, 3, 4)
+            assert torch.equal(o1, o[one]) and torch.equal(lse1, lse[one])
+    sc = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) / 8 + bias.double()[:, None, None]
+    o, _ = K.attn_fwd(q, k, v, bias, 0.125, 0.0, 3, 4)
+    want = torch.einsum("bhqk,bkhd->bqhd", sc.softmax(-1), v.double())
+    # probabilities and the result are rounded once each
+    assert (o.double() - want).abs().max().item() <= 2 * U[dtype] * v.double().abs().max().item() + 1e-4
+    torch.cuda.synchronize()
+    assert _lib.read_error() == 0
