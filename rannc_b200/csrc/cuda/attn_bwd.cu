@@ -12,8 +12,8 @@
 // kept busy for two thirds of the time.  dQ_i is drained from TMEM into a swizzled fp32 staging tile and added to
 // an fp32 scratch buffer by ONE bulk tensor reduction per half tile (the copy
 // engine does the read-modify-write; the math threads do not wait for it); a
-// last kernel converts the scratch to the 16-bit dQ.  dK and dV leave by way of the same staging tile.  Q_i / dO_i stream
-// through a 3-stage TMA ring.  Warps 0..15 = element math, warp 16 = loads and the S / dP products, warp 17 = the
+// last kernel converts the scratch to the 16-bit dQ.  (A sequence of one key block has nothing to add up: its dQ is rounded
+// and stored at once.)  dK and dV leave by way of the same staging tile.  Q_i / dO_i stream through a 3-stage TMA ring.  Warps 0..15 = element math, warp 16 = loads and the S / dP products, warp 17 = the
 // products with dSt and Pt, warps 18..21 = dQ, dK and dV drain, and the row statistics (lse, delta, dropout hash) of the
 // blocks to come: the math warps' chain per query block is only "S / dP -> P / dS", without a barrier among them, and the
 // drain of block i runs beside the math of block i + 1.  Of a block's products those that read dSt come first, so that its
@@ -70,7 +70,8 @@ struct AttnBwdParams {
     int* err;
 };
 
-template <typename T>
+// DQ16 (one key block): its product is all of dQ, which is rounded and stored at once
+template <typename T, bool DQ16>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
     attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -390,15 +391,29 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
                 ok = mbar_wait_warp(dq_free, c & 1, abort_flag);
                 if (!ok) break;
                 uint8_t* row = sDQ + (r >> 3) * 1024 + sw * 128;
+                if constexpr (DQ16) {
 #pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                    const uint32_t off = (static_cast<uint32_t>(g) ^ sw) << 4;
-                    *reinterpret_cast<float4*>(row + off) =
-                        make_float4(__uint_as_float(v0[g * 4]) * p.scale, __uint_as_float(v0[g * 4 + 1]) * p.scale,
-                                    __uint_as_float(v0[g * 4 + 2]) * p.scale, __uint_as_float(v0[g * 4 + 3]) * p.scale);
-                    *reinterpret_cast<float4*>(row + DQ_STAGE / 2 + off) =
-                        make_float4(__uint_as_float(v1[g * 4]) * p.scale, __uint_as_float(v1[g * 4 + 1]) * p.scale,
-                                    __uint_as_float(v1[g * 4 + 2]) * p.scale, __uint_as_float(v1[g * 4 + 3]) * p.scale);
+                    for (int g = 0; g < 8; ++g) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int x = 0; x < 4; ++x) {
+                            const int at = (g & 3) * 8 + 2 * x;
+                            w[x] = pack2<T>(__uint_as_float(g < 4 ? v0[at] : v1[at]) * p.scale,
+                                            __uint_as_float(g < 4 ? v0[at + 1] : v1[at + 1]) * p.scale);
+                        }
+                        *reinterpret_cast<uint4*>(row + ((static_cast<uint32_t>(g) ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                } else {
+#pragma unroll
+                    for (int g = 0; g < 8; ++g) {
+                        const uint32_t off = (static_cast<uint32_t>(g) ^ sw) << 4;
+                        *reinterpret_cast<float4*>(row + off) =
+                            make_float4(__uint_as_float(v0[g * 4]) * p.scale, __uint_as_float(v0[g * 4 + 1]) * p.scale,
+                                        __uint_as_float(v0[g * 4 + 2]) * p.scale, __uint_as_float(v0[g * 4 + 3]) * p.scale);
+                        *reinterpret_cast<float4*>(row + DQ_STAGE / 2 + off) =
+                            make_float4(__uint_as_float(v1[g * 4]) * p.scale, __uint_as_float(v1[g * 4 + 1]) * p.scale,
+                                        __uint_as_float(v1[g * 4 + 2]) * p.scale, __uint_as_float(v1[g * 4 + 3]) * p.scale);
+                    }
                 }
                 fence_proxy_async();
                 mbar_arrive(dq_ready);
@@ -406,8 +421,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
                     ok = mbar_wait_warp(dq_ready, c & 1, abort_flag);
                     if (!ok) break;
                     if (issuer) {
-                        tma_reduce_add_4d(&tmDQ, sDQ, 0, i * BQ, item.h, item.b);
-                        tma_reduce_add_4d(&tmDQ, sDQ + DQ_STAGE / 2, 32, i * BQ, item.h, item.b);
+                        if constexpr (DQ16) {
+                            tma_store_4d(&tmDQ, sDQ, 0, i * BQ, item.h, item.b);
+                        } else {
+                            tma_reduce_add_4d(&tmDQ, sDQ, 0, i * BQ, item.h, item.b);
+                            tma_reduce_add_4d(&tmDQ, sDQ + DQ_STAGE / 2, 32, i * BQ, item.h, item.b);
+                        }
                         tma_store_commit();
                     }
                 }
@@ -596,7 +615,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
     }
 }
 
-// delta[b,h,q] = sum_d dO[b,q,h,d] * O[b,q,h,d], D = 64, and the dQ scratch is cleared on the way (a memset of its
+// delta[b,h,q] = sum_d dO[b,q,h,d] * O[b,q,h,d], D = 64, and the dQ scratch, if it is used, is cleared (a memset of its
 // own cost as much as the rest of this pass).  Rows are taken in memory order ((b, q, h): h is the fastest index of
 // a [B, S, H, D] tensor), 8 lanes x 16 bytes per row, two rows of a thread in flight: bound by memory.
 template <typename T>
@@ -626,7 +645,7 @@ __global__ void __launch_bounds__(256)
     }
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-        if (at[u] >= 0) {
+        if (dq_accum && at[u] >= 0) {
             float4* z = reinterpret_cast<float4*>(dq_accum + static_cast<size_t>(row0 + u * 32u) * 64 + sub * 4);
             z[0] = make_float4(0.f, 0.f, 0.f, 0.f);   // 8 lanes cover the row in two runs of 128 bytes
             z[8] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -677,8 +696,15 @@ static int launch_bwd(const RbAttnArgs& a, cudaStream_t st) {
     if ((rc = make_tmap_4d(&tdo, a.dO, a.dtype, D, S, H, B, a.do_ss * 2, a.do_sh * 2, a.do_sb * 2, 64, 128))) return rc;
     const long long rows = static_cast<long long>(a.B) * a.H * a.S;
     if (rows >= (1LL << 31) - 64) return -2;
+    CUtensorMap tdq, tdk, tdv;
+    // A sequence of one key block has nothing to add up in dQ: without the clearing of the scratch, the additions and the
+    // conversion 64 x 128 x 16 heads take 38.4 us in place of 50.8, 32 x 64 x 16 18.6 (23.4), 8 x 128 x 16 11.2 (14.0),
+    // 1 x 32 x 4 7.7 (9.7).  A kernel of its own: asked in the drain loop, it cost the longer sequences 1 %.  (Strides of dQ
+    // that the copy engine does not take go the way of those.)
+    const bool dq16 =
+        a.S <= BKEYS && make_tmap_4d(&tdq, a.dQ, a.dtype, D, S, H, B, a.dq_ss * 2, a.dq_sh * 2, a.dq_sb * 2, 64, 128) == 0;
     if (launch_after(attn_delta_kernel<T>, static_cast<unsigned>((rows + 63) / 64), 256, 0, st, static_cast<const T*>(a.O),
-                     static_cast<const T*>(a.dO), a.delta, a.dq_accum, a.B, a.H, a.S, a.o_sb, a.o_ss, a.o_sh, a.do_sb,
+                     static_cast<const T*>(a.dO), a.delta, dq16 ? nullptr : a.dq_accum, a.B, a.H, a.S, a.o_sb, a.o_ss, a.o_sh, a.do_sb,
                      a.do_ss, a.do_sh) != cudaSuccess)
         return -1;
     AttnBwdParams p;
@@ -694,14 +720,14 @@ static int launch_bwd(const RbAttnArgs& a, cudaStream_t st) {
     p.seed = drop_seed(a.seed, a.offset);
     p.err = error_word_ptr();
     if (!p.err) return -3;
-    auto kern = attn_bwd_kernel<T>;
-    static bool attr_set[64] = {false};
+    auto kern = dq16 ? attn_bwd_kernel<T, true> : attn_bwd_kernel<T, false>;
+    static bool attr_set[64][2] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (!attr_set[dev & 63]) {
+    if (!attr_set[dev & 63][dq16]) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM) != cudaSuccess)
             return -4;
-        attr_set[dev & 63] = true;
+        attr_set[dev & 63][dq16] = true;
     }
     const long long nitems = static_cast<long long>((a.S + BKEYS - 1) / BKEYS) * a.H * a.B;   // (< 2^31, as the rows)
     const int sms = num_sms();
@@ -713,11 +739,11 @@ static int launch_bwd(const RbAttnArgs& a, cudaStream_t st) {
     auto inverse = [](unsigned d) { return d == 1 ? 0u : static_cast<uint32_t>(((1ull << 32) + d - 1) / d); };
     p.inv_nq = inverse(nq);
     p.inv_h = inverse(nh);
-    CUtensorMap tdq, tdk, tdv;
     if ((rc = make_tmap_4d(&tdk, a.dK, a.dtype, D, S, H, B, a.dk_ss * 2, a.dk_sh * 2, a.dk_sb * 2, 64, 128))) return rc;
     if ((rc = make_tmap_4d(&tdv, a.dV, a.dtype, D, S, H, B, a.dv_ss * 2, a.dv_sh * 2, a.dv_sb * 2, 64, 128))) return rc;
-    if ((rc = make_tmap_4d_f32(&tdq, a.dq_accum, 64, S, H, B, H * 64 * 4, 64 * 4, S * H * 64 * 4, 32, 128))) return rc;
+    if (!dq16 && (rc = make_tmap_4d_f32(&tdq, a.dq_accum, 64, S, H, B, H * 64 * 4, 64 * 4, S * H * 64 * 4, 32, 128))) return rc;
     if (launch_after(kern, grid, BWD_THREADS, BWD_SMEM, st, tq, tk, tv, tdo, tdq, tdk, tdv, p) != cudaSuccess) return -1;
+    if (dq16) return 0;
     const long long groups = rows * 8;
     return launch_after(attn_dq_convert_kernel<T>, static_cast<unsigned>((groups + 255) / 256), 256, 0, st,
                         static_cast<const float*>(a.dq_accum), static_cast<T*>(a.dQ), a.B, a.H, a.S, a.dq_sb, a.dq_ss,

@@ -859,3 +859,38 @@ def test_attention_forward_two_heads_a_block(dtype, S, B, H):
     assert (o.double() - want).abs().max().item() <= 2 * U[dtype] * v.double().abs().max().item() + 1e-4
     torch.cuda.synchronize()
     assert _lib.read_error() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("S", [1, 33, 64, 100, 127, 128, 129])
+@pytest.mark.parametrize("B,H", [(1, 1), (3, 4), (40, 7)])
+def test_attention_backward_of_one_key_block(dtype, S, B, H):
+    """dQ of a sequence of one key block is stored as it is made: into a part of a packed gradient whose other parts stay as
+    they are, and with strides of its own.  One key more goes by way of the sums."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(19)
+    q, k, v = (t for t in torch.randn(B, S, 3, H, 64, device="cuda").to(dtype).unbind(2))
+    do = torch.randn(B, S, H, 64, device="cuda").to(dtype)
+    bias = torch.zeros(B, S, device="cuda")
+    bias[::2, S // 2 + 1:] = -10000.0
+    o, lse = K.attn_fwd(q, k, v, bias, 0.125)
+    packed = torch.full((B, S, 4, H, 64), 3.0, device="cuda", dtype=dtype)
+    K.attn_bwd(q, k, v, o, lse, do, bias, 0.125, dq=packed[:, :, 0], dk=packed[:, :, 1], dv=packed[:, :, 2])
+    assert (packed[:, :, 3] == 3.0).all()
+    flipped = torch.full((H, B, S + 1, 72), 3.0, device="cuda", dtype=dtype)   # heads outermost, rows 72 apart
+    dq = flipped.permute(1, 2, 0, 3)[:, :S, :, :64]
+    K.attn_bwd(q, k, v, o, lse, do, bias, 0.125, dq=dq)
+    assert (flipped[:, :, S] == 3.0).all() and (flipped[..., 64:] == 3.0).all()
+    if S <= 128:
+        assert torch.equal(dq, packed[:, :, 0])
+    qd, kd, vd = (t.double().requires_grad_(True) for t in (q, k, v))
+    sc = torch.einsum("bqhd,bkhd->bhqk", qd, kd) / 8 + bias.double()[:, None, None]
+    torch.einsum("bhqk,bkhd->bqhd", sc.softmax(-1), vd).backward(do.double())
+    for got, want in zip(packed.unbind(2), (qd.grad, kd.grad, vd.grad)):
+        # o, the probabilities and the gradients of the scores are rounded, each sum's terms with errors of both signs
+        bound = 6 * U[dtype] * max(1.0, want.abs().max().item())
+        assert (got.double() - want).abs().max().item() <= bound
+    torch.cuda.synchronize()
+    assert _lib.read_error() == 0
