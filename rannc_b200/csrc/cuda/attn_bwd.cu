@@ -12,12 +12,13 @@
 // kept busy for two thirds of the time.  dQ_i is drained from TMEM into a swizzled fp32 staging tile and added to
 // an fp32 scratch buffer by ONE bulk tensor reduction per half tile (the copy
 // engine does the read-modify-write; the math threads do not wait for it); a
-// last kernel converts the scratch to the 16-bit dQ.  (A sequence of one key block has nothing to add up: its dQ is rounded
-// and stored at once.)  dK and dV leave by way of the same staging tile.  Q_i / dO_i stream through a 3-stage TMA ring.  Warps 0..15 = element math, warp 16 = loads and the S / dP products, warp 17 = the
-// products with dSt and Pt, warps 18..21 = dQ, dK and dV drain, and the row statistics (lse, delta, dropout hash) of the
-// blocks to come: the math warps' chain per query block is only "S / dP -> P / dS", without a barrier among them, and the
-// drain of block i runs beside the math of block i + 1.  Of a block's products those that read dSt come first, so that its
-// tile is free again before the next block's is ready.
+// last kernel converts the scratch to the 16-bit dQ.  (A sequence of one key block has nothing to add up: its dQ is
+// rounded and stored at once.)  dK and dV leave by way of the same staging tile.  Q_i / dO_i stream through a 3-stage TMA
+// ring.  Warps 0..15 = element math, warp 16 = loads and the S / dP products, warp 17 = the products with dSt and Pt,
+// warps 18..21 = dQ, dK and dV drain, and the row statistics (lse, delta, dropout hash) of the blocks to come: the math
+// warps' chain per query block is only "S / dP -> P / dS", without a barrier among them, and the drain of block i runs
+// beside the math of block i + 1.  Of a block's products those that read dSt come first, so that its tile is free again
+// before the next block's is ready.
 //
 // Every role runs on from item to item: blocks are counted over all items (barrier phases, ring stages, statistics), the
 // next item's K and V are loaded while the last block is in work, its first S / dP stand ready when the math warps come, and
