@@ -343,8 +343,9 @@ class _Conv2d(torch.autograd.Function):
         arithmetic, and in tiles that few rows leave empty, than the gather costs in traffic.
         ``conv_implicit_max_overhead`` bounds (H + 2 pad)(W + 2 pad) / (H W), the border on both sides: 1.15 at 28 x 28
         (the kernel's own grid 1.07), 1.31 at 14 x 14 (1.15).  Forward and backward of 32 fp16 images on the device,
-        implicit / gathered in us: 28 x 28 x 512 370 / 484, x 1024 1304 / 1475, x 2048 5608 / 5512; 14 x 14 x 512
-        147 / 167, x 1024 451 / 426, x 2048 1749 / 1435; 7 x 7 x 1024 240 / 201: the line lies at 14."""
+        implicit / gathered in us: 28 x 28 x 512 288 / 456, x 1024 1036 / 1356, x 2048 4702 / 5000; 14 x 14 x 512
+        115 / 158, x 1024 343 / 385, x 2048 1351 / 1265; 7 x 7 x 1024 153 / 168.  The line lies at 14 because of the host,
+        which takes 250 us for the one and 200 for the other, longer than the device for most of the smaller layers."""
         if not (k > 1 and k % 2 == 1 and stride == 1 and padding == (k - 1) // 2 and Ci % 64 == 0 and Co % 64 == 0
                 and k * k <= 49 and bool(conf("conv_implicit_gemm"))):
             return False
