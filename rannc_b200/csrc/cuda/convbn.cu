@@ -337,20 +337,7 @@ __device__ __forceinline__ void ldf8_any(const float* p, float (&v)[8]) {
 // A thread owns 8 adjacent channels (16 bytes a row) in every kernel here; a block of (BX, 256 / BX) threads covers
 // BX * 8 channels, rows are strided over threadIdx.y and blockIdx.y.  BX follows the channel count, so that a layer of
 // 64 channels does not leave three quarters of its threads without one.
-//
-// Clears the sums.  (A copy-engine or runtime memset between two kernels waits for the first's end and the second for
-// its own; this one is in place when the first ends.)
-__global__ void __launch_bounds__(256) bn_clear_kernel(float4* part, int n) {
-    grid_trigger();
-    grid_wait();
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i < n) part[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-}
-static cudaError_t bn_clear(float* part, int C, cudaStream_t st) {  // 2 C floats, C a multiple of 8
-    return launch_after(bn_clear_kernel, (C / 2 + 255) / 256, 256, 0, st, reinterpret_cast<float4*>(part), C / 2);
-}
-
-// part[0][c] += sum_r a(r, c), part[1][c] += sum_r a(r, c) * b(r, c)
+// Sums over a block's rows: part[blockIdx.y][0][c] = sum_r a(r, c), part[blockIdx.y][1][c] = sum_r a(r, c) * b(r, c)
 //   MODE 0 (statistics):  a = x,                 b = x
 //   MODE 1 (backward):    a = dy masked by relu, b = xhat = (x - mean) * rstd
 template <typename T, int MODE, int BX>
@@ -401,10 +388,39 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int w = 0; w < TY; ++w) a0 += red[0][w][t], a1 += red[1][w][t];
     const int c = blockIdx.x * BX * 8 + t;
+    part += blockIdx.y * 2LL * C;
     if (c < C) {
-        atomicAdd(part + c, a0);
-        atomicAdd(part + C + c, a1);
+        part[c] = a0;
+        part[C + c] = a1;
     }
+}
+
+// The blocks' sums added up, in fp64 and in a fixed order: total[0 .. 2 C).  (By atomics, in the order they arrived, the last
+// bits of a total changed from run to run, and a result of the norm that lies next to zero fell on either side of the ReLU,
+// with dy or 0 for its gradient.)  Bound by latency: a block has 16 columns only, and 128 rows on their way at a time.
+__global__ void __launch_bounds__(512) bn_total_kernel(const float* part, int parts, int C, float* total) {
+    __shared__ double red[16][16];
+    grid_trigger();
+    grid_wait();
+    const int t = threadIdx.x, col = blockIdx.x * 16 + (t & 3) * 4;   // (2 C is a multiple of 16)
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 5
+    for (int r = t >> 2; r < parts; r += 128) {
+        const float4 v = *reinterpret_cast<const float4*>(part + r * 2LL * C + col);
+        s[0] += v.x, s[1] += v.y, s[2] += v.z, s[3] += v.w;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+        if ((t & 31) < 4) red[t >> 5][t * 4 % 16 + j] = s[j];
+    }
+    __syncthreads();
+    if (t >= 16) return;
+    double sum = 0.0;
+#pragma unroll
+    for (int w = 0; w < 16; ++w) sum += red[w][t];
+    total[blockIdx.x * 16 + t] = static_cast<float>(sum);
 }
 
 // y = act(x * scale + shift (+ residual)) with scale = rstd gamma and shift = beta - mean scale.  Every thread derives
@@ -548,14 +564,17 @@ __global__ void __launch_bounds__(256)
 
 // Grid of the batch-norm kernels: blocks of BX * 8 channels, and as many row groups as give the whole grid about
 // `per_sm` blocks per SM, each with four rows or more per thread.  per_sm is what an SM holds at once of the kernel with
-// its registers (40 to 101 a thread), so that there is one wave: 6 and 4 for the reductions, 2 for the element-wise passes
-// (at four with half the rows in flight, or held to 64 registers, those take longer, as does the reduction of the forward
-// pass at 4 or 8).  Forward and backward of 32 x 14 x 14 x 2048 with residual and ReLU 22.7 and 39.4 -> 19.6 and 33.7 us, of
-// 32 x 28 x 28 x 1024 with ReLU 35.4 and 68.5 -> 30.1 and 58.5; the order of the rows gave 3 and 5 us of the backward
-// passes, the launches beside the end of the kernel before (which need a clearing kernel in the place of a memset) 1 to 3.
-// None of these kernels lets the next begin by grid_trigger(): a GEMM that does waits on the SMs with its shared memory, and
-// the first-level cache that this leaves to them costs more (a 1x1 convolution of 32 x 14 x 14 x 2048 with its norm, forward
-// and backward, 131.6 us of device time with the triggers, 120.3 without, 128.5 at ordinary launches).
+// its registers (40 to 101 a thread), so that there is one wave: 4 for the reductions, 2 for the element-wise passes (at four
+// with half the rows in flight, or held to 64 registers, those take longer).  The reductions' grid also decides which rows
+// make up a sum, and with it the last bits of the statistics: four blocks per SM, as it was when sums met by atomics.
+// Forward + backward in a captured graph, one B200 (us), at ordinary launches with atomics into memory that a memset had
+// cleared, and now: 6272 x 2048 with residual and ReLU 15.6 + 34.1 -> 16.1 + 33.5, 25088 x 1024 with ReLU 23.4 + 63.1 -> 26.3
+// + 57.5, 100352 x 256 with both 40.6 + 76.1 -> 36.1 + 67.8, 401408 x 64 with ReLU 26.0 + 65.0 -> 25.5 + 56.4.  With atomics,
+// and a kernel that clears in the place of the memset, these take 15.1 + 32.3, 25.5 + 56.0, 36.9 + 67.2 and 26.0 + 54.6: what a
+// fixed order costs.  (fp64 atomics, whose order hardly shows, take as long: 29.3 + 54 at 401408 x 64.)
+// Neither the reductions nor the passes let the next kernel begin by grid_trigger(): a GEMM that does waits on the SMs with its
+// shared memory, and the first-level cache that this leaves to them costs more (a 1x1 convolution of 32 x 14 x 14 x 2048 with
+// its norm, forward and backward, 131.6 us of device time with the triggers, 120.3 without, 128.5 at ordinary launches).
 template <int BX>
 static dim3 bn_grid(long long R, int C, int per_sm) {
     const int cols = (C + BX * 8 - 1) / (BX * 8);
@@ -565,18 +584,30 @@ static dim3 bn_grid(long long R, int C, int per_sm) {
     return dim3(cols, static_cast<unsigned>(split < 1 ? 1 : split));
 }
 
+// the reductions' blocks along the rows
+static long long bn_parts(long long R, int C) {
+    return (C >= 256 ? bn_grid<32>(R, C, 4) : C > 64 ? bn_grid<16>(R, C, 4) : bn_grid<8>(R, C, 4)).y;
+}
+
+// total: fp32 [2, C], and behind it the parts
+template <typename T, int MODE, int BX>
+static cudaError_t bn_reduce(const T* x, const T* dy, const T* y, const float* mean, const float* rstd, float* total, long long R,
+                             int C, int relu, cudaStream_t st) {
+    const dim3 grid = bn_grid<BX>(R, C, 4);
+    float* part = total + 2LL * C;
+    const cudaError_t e = launch_after(bn_reduce_kernel<T, MODE, BX>, grid, dim3(BX, 256 / BX), 0, st, x, dy, y, mean, rstd, part,
+                                       R, C, relu);
+    if (e != cudaSuccess) return e;
+    return launch_after(bn_total_kernel, C / 8, 512, 0, st, part, static_cast<int>(grid.y), C, total);
+}
+
 template <typename T, int BX>
 static int bn_fwd_launch(const void* x, const void* res, const float* gamma, const float* beta, void* y, float* part,
                          float* mean, float* rstd, float* run_mean, float* run_var, long long R, int C, float eps,
                          float momentum, int relu, cudaStream_t st) {
     const dim3 block(BX, 256 / BX);
     const T* xt = static_cast<const T*>(x);
-    const T* none = nullptr;
-    const float* nof = nullptr;
-    if (bn_clear(part, C, st) != cudaSuccess) return -1;
-    if (launch_after(bn_reduce_kernel<T, 0, BX>, bn_grid<BX>(R, C, 6), block, 0, st, xt, none, none, nof, nof, part, R, C, 0) !=
-        cudaSuccess)
-        return -1;
+    if (bn_reduce<T, 0, BX>(xt, nullptr, nullptr, nullptr, nullptr, part, R, C, 0, st) != cudaSuccess) return -1;
     const cudaError_t e = launch_after(bn_apply_kernel<T, BX>, bn_grid<BX>(R, C, 2), block, 0, st, xt,
                                        static_cast<const T*>(res), part, gamma, beta, mean, rstd, run_mean, run_var,
                                        static_cast<T*>(y), R, C, eps, momentum, relu);
@@ -588,10 +619,7 @@ static int bn_bwd_launch(const void* x, const void* dy, const void* y, const flo
                          int C, int relu, cudaStream_t st) {
     const dim3 block(BX, 256 / BX);
     const T *xt = static_cast<const T*>(x), *dt = static_cast<const T*>(dy), *yt = static_cast<const T*>(y);
-    if (bn_clear(part, C, st) != cudaSuccess) return -1;
-    if (launch_after(bn_reduce_kernel<T, 1, BX>, bn_grid<BX>(R, C, 4), block, 0, st, xt, dt, yt, mean, rstd, part, R, C, relu) !=
-        cudaSuccess)
-        return -1;
+    if (bn_reduce<T, 1, BX>(xt, dt, yt, mean, rstd, part, R, C, relu, st) != cudaSuccess) return -1;
     const cudaError_t e = launch_after(bn_bwd_apply_kernel<T, BX>, bn_grid<BX>(R, C, 2), block, 0, st, xt, dt, yt, part, mean,
                                        rstd, gamma, dgamma, dbeta, static_cast<T*>(dx), static_cast<T*>(dres), R, C, relu);
     return e == cudaSuccess ? 0 : -1;
@@ -697,7 +725,12 @@ extern "C" int rb_wgrad_fold(const float* src, void* dst, int Co, int Ci, int ta
      : C > 64 ? (dtype == 1 ? FN<__nv_bfloat16, 16>(__VA_ARGS__) : FN<__half, 16>(__VA_ARGS__))       \
               : (dtype == 1 ? FN<__nv_bfloat16, 8>(__VA_ARGS__) : FN<__half, 8>(__VA_ARGS__)))
 
-// Forward statistics + normalisation.  part: fp32 [2, C] scratch (zeroed here); mean / rstd: fp32 [C] outputs;
+// Floats that `part` of the two entries below has to hold.
+extern "C" long long rb_bn_part_floats(long long R, int C) {
+    return C % 8 || C <= 0 || R <= 0 ? 0 : (1 + rb::bn_parts(R, C)) * 2 * C;
+}
+
+// Forward statistics + normalisation.  part: fp32 scratch (rb_bn_part_floats); mean / rstd: fp32 [C] outputs;
 // run_mean / run_var may be null (evaluation of a frozen layer is not handled here: pass training only).
 extern "C" int rb_bn_fwd(const void* x, const void* res, const float* gamma, const float* beta, void* y, float* part,
                          float* mean, float* rstd, float* run_mean, float* run_var, long long R, int C, float eps,
@@ -710,8 +743,8 @@ extern "C" int rb_bn_fwd(const void* x, const void* res, const float* gamma, con
                           relu, st);
 }
 
-// Backward.  part: fp32 [2, C] scratch; on return part[0] = d beta, part[1] = d gamma, which are also added to
-// dbeta_acc / dgamma_acc when those are given.
+// Backward.  part: fp32 scratch (rb_bn_part_floats); on return its first C floats are d beta and the next C d gamma, which are
+// also added to dbeta_acc / dgamma_acc when those are given.
 extern "C" int rb_bn_bwd(const void* x, const void* dy, const void* y, const float* mean, const float* rstd,
                          const float* gamma, float* part, float* dgamma_acc, float* dbeta_acc, void* dx, void* dres,
                          long long R, int C, int relu, int dtype, void* stream) {

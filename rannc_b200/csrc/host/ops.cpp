@@ -62,6 +62,7 @@ struct Api {
                   long long, int, float, float, int, int, void*);
     int (*bn_bwd)(const void*, const void*, const void*, const float*, const float*, const float*, float*, float*, float*,
                   void*, void*, long long, int, int, int, void*);
+    long long (*bn_part_floats)(long long, int);
     decltype(&rb_rows_plan) rows_plan;
     decltype(&rb_rows_gather) rows_gather;
     decltype(&rb_rows_scatter) rows_scatter;
@@ -1065,7 +1066,7 @@ struct BnNode : Node {
         const Tensor dy = nhwc(grads[0]);
         const int64_t C = X.size(1);
         Tensor dx = at::empty_like(X), dres = has_res ? at::empty_like(X) : Tensor();
-        Tensor part = f32({2, C}, X);
+        Tensor part = f32({api.bn_part_floats(X.numel() / C, static_cast<int>(C))}, X);
         // fp32 gradient buffers take the sums inside the kernel
         auto acc = [](const Tensor& mg) {
             return mg.defined() && mg.scalar_type() == at::kFloat && mg.is_contiguous() ? mptr<float>(mg) : nullptr;
@@ -1074,17 +1075,17 @@ struct BnNode : Node {
         check(api.bn_bwd(X.data_ptr(), dy.data_ptr(), Y.data_ptr(), mptr<float>(M), mptr<float>(R), mptr<float>(G),
                          mptr<float>(part), ga, ba, dx.data_ptr(), mptr(dres), X.numel() / C, static_cast<int>(C), relu ? 1 : 0,
                          dt_code(X), cur_stream()),
-              "rb_bn_bwd", 2);
+              "rb_bn_bwd", 3);
         Tensor dg, db;
         if (g_mg.defined()) {
-            if (!ga) g_mg.add_(part[1]);
+            if (!ga) g_mg.add_(part.narrow(0, C, C));
         } else {
-            dg = part[1].to(gamma.scalar_type());
+            dg = part.narrow(0, C, C).to(gamma.scalar_type());
         }
         if (b_mg.defined()) {
-            if (!ba) b_mg.add_(part[0]);
+            if (!ba) b_mg.add_(part.narrow(0, 0, C));
         } else {
-            db = part[0].to(beta.scalar_type());
+            db = part.narrow(0, 0, C).to(beta.scalar_type());
         }
         notify({{&gamma, &g_mg}, {&beta, &b_mg}});
         return {dx, dres, dg, db};
@@ -1111,14 +1112,14 @@ Tensor batch_norm_act(const Tensor& x, const OptTensor& res_, const Tensor& gamm
         auto fp32 = [](const Tensor& t) { return t.defined() && t.scalar_type() == at::kFloat && t.is_contiguous(); };
         const bool in_kernel = fp32(run_mean) && fp32(run_var);
         y = at::empty_like(xc);
-        Tensor part = f32({2, C}, x);
+        Tensor part = f32({api.bn_part_floats(R, static_cast<int>(C))}, x);
         mean = f32({C}, x);
         rstd = f32({C}, x);
         check(api.bn_fwd(xc.data_ptr(), cptr(rc), mptr<float>(g32), mptr<float>(b32), y.data_ptr(), mptr<float>(part),
                          mptr<float>(mean), mptr<float>(rstd), in_kernel ? mptr<float>(run_mean) : nullptr,
                          in_kernel ? mptr<float>(run_var) : nullptr, R, static_cast<int>(C), static_cast<float>(eps),
                          static_cast<float>(momentum), relu ? 1 : 0, dt_code(x), cur_stream()),
-              "rb_bn_fwd", 2);
+              "rb_bn_fwd", 3);
         if (run_mean.defined() && !in_kernel) {
             // statistics kept in 16 bits, or strided: update them with a few tiny element-wise operations
             const Tensor var = (1.0 / (rstd * rstd) - eps) * (static_cast<double>(R) / std::max<int64_t>(R - 1, 1));
@@ -1216,6 +1217,7 @@ void init(const std::unordered_map<std::string, uintptr_t>& fns, py::object erro
     set(api.attn_bwd, "rb_attn_bwd");
     set(api.bn_fwd, "rb_bn_fwd");
     set(api.bn_bwd, "rb_bn_bwd");
+    set(api.bn_part_floats, "rb_bn_part_floats");
     set(api.rows_plan, "rb_rows_plan");
     set(api.rows_gather, "rb_rows_gather");
     set(api.rows_scatter, "rb_rows_scatter");

@@ -18,8 +18,8 @@ _lock = threading.Lock()
 _lib = None
 
 # device kernels launched per C entry point (the optimizer / element-wise entries launch one)
-_KERNELS_PER_CALL = {"rb_bn_fwd": 2, "rb_bn_bwd": 2, "rb_ln_bwd": 2, "rb_xent_fwd": 2, "rb_attn_bwd": 3, "rb_rows_plan": 2,
-                     "rb_read_error": 0, "rb_ln_supported": 0, "rb_ln_bwd_grid": 0, "rb_gemm_splits": 0,
+_KERNELS_PER_CALL = {"rb_bn_fwd": 3, "rb_bn_bwd": 3, "rb_ln_bwd": 2, "rb_xent_fwd": 2, "rb_attn_bwd": 3, "rb_rows_plan": 2,
+                     "rb_bn_part_floats": 0, "rb_read_error": 0, "rb_ln_supported": 0, "rb_ln_bwd_grid": 0, "rb_gemm_splits": 0,
                      "rb_gemm_last_wave": 0, "rb_error_peek_async": 0}
 _launches = 0
 
@@ -80,6 +80,7 @@ def lib() -> ctypes.CDLL:
         except OSError as e:
             raise KernelLibraryError(f"cannot load {path}: {e}") from e
         _lib.rb_read_error.restype = ctypes.c_int
+        _lib.rb_bn_part_floats.restype = ctypes.c_longlong
         _lib = _Counting(_lib)
         return _lib
 
@@ -87,7 +88,8 @@ def lib() -> ctypes.CDLL:
 _host = None
 _HOST_ENTRIES = ("rb_gemm", "rb_gemm_splits", "rb_unstack3", "rb_gelu", "rb_colsum", "rb_ln_fwd", "rb_ln_bwd",
                  "rb_ln_bwd16", "rb_ln_bwd_grid", "rb_embed_fwd", "rb_embed_bwd", "rb_xent_fwd", "rb_xent_bwd",
-                 "rb_attn_fwd", "rb_attn_bwd", "rb_bn_fwd", "rb_bn_bwd", "rb_rows_plan", "rb_rows_gather", "rb_rows_scatter")
+                 "rb_attn_fwd", "rb_attn_bwd", "rb_bn_fwd", "rb_bn_bwd", "rb_bn_part_floats", "rb_rows_plan", "rb_rows_gather",
+                 "rb_rows_scatter")
 
 
 def host_loaded() -> bool:

@@ -346,7 +346,7 @@ def bn_fwd(x2d, residual2d, gamma32, beta32, run_mean32, run_var32, eps: float, 
     the running statistics (fp32, may be None) are updated in place."""
     R, C = x2d.shape
     y = torch.empty_like(x2d)
-    part = torch.empty(2, C, dtype=torch.float32, device=x2d.device)
+    part = torch.empty(_lib.lib().rb_bn_part_floats(c_longlong(R), c_int(C)), dtype=torch.float32, device=x2d.device)
     mean = torch.empty(C, dtype=torch.float32, device=x2d.device)
     rstd = torch.empty(C, dtype=torch.float32, device=x2d.device)
     _lib.check(_lib.lib().rb_bn_fwd(_lib.vp(x2d), _lib.vp(residual2d), _lib.vp(gamma32), _lib.vp(beta32), _lib.vp(y),
@@ -361,9 +361,9 @@ def bn_bwd(x2d, dy2d, y2d, mean, rstd, gamma32, relu: bool, want_dres: bool):
     R, C = x2d.shape
     dx = torch.empty_like(x2d)
     dres = torch.empty_like(x2d) if want_dres else None
-    part = torch.empty(2, C, dtype=torch.float32, device=x2d.device)
+    part = torch.empty(_lib.lib().rb_bn_part_floats(c_longlong(R), c_int(C)), dtype=torch.float32, device=x2d.device)
     _lib.check(_lib.lib().rb_bn_bwd(_lib.vp(x2d), _lib.vp(dy2d), _lib.vp(y2d), _lib.vp(mean), _lib.vp(rstd),
                                     _lib.vp(gamma32), _lib.vp(part), c_void_p(0), c_void_p(0), _lib.vp(dx), _lib.vp(dres),
                                     c_longlong(R), c_int(C), c_int(1 if relu else 0), c_int(dt_code(x2d)),
                                     _lib.stream_ptr()), "rb_bn_bwd")
-    return dx, dres, part[1], part[0]
+    return dx, dres, part[C:2 * C], part[:C]

@@ -161,3 +161,27 @@ def test_conv2d_implicit_gemm_matches_fp32(N, Ci, Co, H, W, k, main_grad):
     finally:
         set_conf("conv_implicit_gemm", False)
         set_conf("conv_implicit_max_overhead", 1.2)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("R,C", [(6272, 2048), (25088, 64), (1000, 136)])
+def test_batch_norm_repeats_to_the_bit(R, C, dtype):
+    """The sums behind the statistics do not depend on the order in which the blocks arrive, and with them no bit of a result
+    (a result next to zero decides by its last bits whether the gradient passes the ReLU)."""
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(21)
+    x, r, dy = (torch.randn(R, C, device="cuda").to(dtype) for _ in range(3))
+    g, b = torch.rand(C, device="cuda") + 0.5, torch.randn(C, device="cuda")
+    first = None
+    for _ in range(100):
+        y, mean, rstd = K.bn_fwd(x, r, g, b, None, None, 1e-5, 0.1, True)
+        got = (y, mean, rstd, *K.bn_bwd(x, dy, y, mean, rstd, g, True, True))
+        first = first or [t.clone() for t in got]
+        for a, e in zip(got, first):
+            assert torch.equal(a, e)
+    # one rounding of the block sums (some ten rows a thread, sixteen or fewer threads: 2^-20 of the terms) and of the total
+    xd = x.double()
+    assert ((first[1] - xd.mean(0)).abs() <= 2.0 ** -20 * xd.abs().mean(0)).all()
+    var = 1.0 / first[2].double().square() - 1e-5
+    assert ((var - xd.var(0, unbiased=False)).abs() <= 2.0 ** -19 * xd.square().mean(0)).all()

@@ -705,7 +705,7 @@ def test_batch_norm_rows_two_at_a_time(R, C, relu, res):
     r = torch.randn(R, C, device="cuda").to(dtype) if res else None
     g, b = torch.rand(C, device="cuda") + 0.5, torch.randn(C, device="cuda")
     for _ in range(2):
-        junk = [torch.full((2, C), float("nan"), device="cuda") for _ in range(4)]
+        junk = [torch.full((n, C), float("nan"), device="cuda") for n in (2, 4, 6) for _ in range(3)]
         del junk   # (the next allocations of this size get that memory)
         y, mean, rstd = K.bn_fwd(x, r, g, b, None, None, 1e-5, 0.1, relu)
     xd = x.double()
