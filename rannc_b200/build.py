@@ -123,7 +123,7 @@ def build_host(verbose: bool = False, force: bool = False) -> Path:
     ext = sysconfig.get_config_var("EXT_SUFFIX") or ".so"
     out = HERE / ("_host" + ext)
     srcs = sorted(HOST_SRC.glob("*.cpp"))
-    hdrs = [CUDA_SRC / "attn.h", CUDA_SRC / "gemm_tcgen05.h"]
+    hdrs = [CUDA_SRC / h for h in ("attn.h", "gemm_tcgen05.h", "sparse_rows.h")]
     if not force and _newer(out, srcs + hdrs):
         return out
     inc = [d for p in include_paths() + [sysconfig.get_paths()["include"]] for d in ("-isystem", p)]
