@@ -13,7 +13,7 @@
 //
 // 8192 rows, 1024 to 30528, 15 % of the rows not zero: 636 -> 279 us for the backward, of which looking 81 (5.2 TB/s),
 // gathering 25, the two products 150; what it costs where every row counts, and the rule for when to look, stand in
-// host/ops.cpp (worth_gathering).
+// host/ops.cpp (gather_room).
 #include "sparse_rows.h"
 
 #include <cuda_bf16.h>

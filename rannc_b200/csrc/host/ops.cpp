@@ -238,17 +238,20 @@ struct Rows {
 // three quarters count: 8 % of the backward at worst.  Both products use the kernel of CTA pairs whichever form runs, so an
 // input gradient of fewer tiles than two thirds of the pairs stays out (2048 x 1024 x 30528, where all rows count: 235 ->
 // 281; 1024 x 1024 x 30528 gains at 15 %, 181 -> 132, and loses at 100 %, 189 -> 238).
-bool worth_gathering(const Mat& dy, const Mat& x) {
+// Returns how many rows there is room for, in steps of 64 (few rows leave none: 0, as where the look is not worth it).
+int64_t gather_room(int64_t rows, int64_t cols, int64_t inputs) {
     auto tiles = [](int64_t m, int64_t n) { return (m + 255) / 256 * ((n + 255) / 256); };
-    return dy.cols >= 4 * x.cols && dy.cols % 8 == 0 && x.cols % 8 == 0 && dy.cols <= (1 << 22) && dy.rows < (1 << 30) &&
-           tiles(dy.cols, x.cols) >= 74 && tiles(dy.rows, x.cols) >= 48 &&
-           static_cast<double>(dy.rows) * dy.cols * x.cols >= 9e10 && !at::globalContext().deterministicAlgorithms();
+    if (cols < 4 * inputs || cols % 8 || inputs % 8 || cols > (1 << 22) || rows >= (1 << 30) || tiles(cols, inputs) < 74 ||
+        tiles(rows, inputs) < 48 || static_cast<double>(rows) * cols * inputs < 9e10)
+        return 0;
+    return std::min<int64_t>(rows / 4 * 3, (int64_t{1} << 30) / cols) / 64 * 64;   // (2 GiB at most)
 }
 // (empty `ctl`: the call is not one for this)
 Rows gather_rows(const Mat& dy, const Mat& x, bool want_dx, int dtype, const at::TensorOptions& o) {
     Rows r;
-    if (!worth_gathering(dy, x)) return r;
-    r.room = std::min<int64_t>(dy.rows / 4 * 3, (int64_t{1} << 30) / dy.cols) / 64 * 64;   // (2 GiB at most)
+    if (at::globalContext().deterministicAlgorithms()) return r;
+    r.room = gather_room(dy.rows, dy.cols, x.cols);
+    if (r.room == 0) return r;
     const auto ints = o.dtype(at::kInt);
     r.ctl = at::empty({2}, ints);
     r.idx = at::empty({r.room}, ints);
@@ -1269,4 +1272,5 @@ PYBIND11_MODULE(_host, m) {
     RB_DEF(qkv_attention);
     RB_DEF(batch_norm_act);
     RB_DEF(conv1x1);
+    m.def("gather_room", &gather_room);
 }

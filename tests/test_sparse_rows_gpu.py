@@ -132,3 +132,25 @@ def test_infinities_and_nan_reach_the_gradients_of_rows_of_zeros():
         assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
     assert got[False][0][200].isnan().nonzero().flatten().tolist() == [5, 9]
     assert got[False][1][:, 11].isnan().all() and not got[False][1][:, 12].isnan().any()
+
+
+def test_few_rows_of_many_inputs():
+    """Less room than a step of 64 rows: the layer's backward goes over all of them."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops import functional as RF
+
+    R, H, V = 85, 16384, 65536
+    torch.manual_seed(9)
+    x = torch.randn(R, H, device="cuda", dtype=torch.bfloat16).requires_grad_(True)
+    w = torch.empty(V, H, device="cuda", dtype=torch.bfloat16).normal_(std=0.01).requires_grad_(True)
+    dy = torch.randn(R, V, device="cuda", dtype=torch.bfloat16)
+    dy[10:80] = 0
+    RF.linear(x, w).backward(dy)
+    torch.cuda.synchronize()
+    assert _lib.read_error() == 0
+    u = 2.0 ** -8
+    for got, a, b, terms in ((x.grad, dy, w.detach(), V), (w.grad[::97], dy.t()[::97], x.detach(), R)):
+        want = a.double() @ b.double()
+        bound = u * want.abs() + (1e-5 + terms / 16 * 2.0 ** -23) * want.abs().max() + 1e-6   # (as above)
+        assert ((got.double() - want).abs() <= bound).all()
+    assert (x.grad[10:80] == 0).all()
