@@ -1278,7 +1278,7 @@ static Tiling choose_tiling(const RbGemmArgs& a) {
     }
     t.n_blocks = static_cast<int>((a.N + t.tn - 1) / t.tn);
     const int tiles = t.m_blocks * t.n_blocks * static_cast<int>(a.batch);
-    t.split = split_for(tiles);
+    t.split = a.rows_ctl && a.rows_mode == RB_GEMM_ROWS_K ? 1 : split_for(tiles);   // (K is known on the device alone)
     t.tail_tiles = t.tail_split = t.tail_kb = 0;
     const int left = tiles % units;
     if (accum32 && t.pair && tiles > units && a.rs_nranks <= 1 && a.ag_nranks <= 1 && !a.in_order &&
@@ -1402,7 +1402,6 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
         // plain products of one matrix; what is gathered along K or M is cut into whole tiles (ROWS_M: of sums)
         if (a->batch != 1 || a->ag_nranks > 1 || a->rs_nranks > 1 || a->conv_taps > 0 || a->wgrad_taps > 0 || a->map_hp > 0 ||
             (a->flags & ~RB_GEMM_ACCUM) || a->rows_mode < RB_GEMM_ROWS_ALL || a->rows_mode > RB_GEMM_ROWS_M ||
-            (a->rows_mode == RB_GEMM_ROWS_K && p.split_k > 1) ||
             (a->rows_mode == RB_GEMM_ROWS_M && (a->a_major != 0 || a->out_dtype != 1 || a->flags != RB_GEMM_ACCUM)))
             return -10;
         if (a->rows_mode == RB_GEMM_ROWS_M) p.tail_tiles = 0, p.partial = 1;
@@ -1501,6 +1500,9 @@ extern "C" int rb_gemm_splits(long long M, long long N, long long K) {
     a.flags = RB_GEMM_ACCUM;
     return M > 0 && N > 0 && K > 0 ? rb::choose_tiling(a).split : 1;
 }
+
+// Pairs of SMs that work on 256 x 256 tiles at once (0: pairs are switched off)
+extern "C" int rb_gemm_pairs() { return rb::pair_enabled() ? rb::num_sms() / 2 : 0; }
 
 // How the last wave of tiles of an fp32 [M, N] += product is summed: 0 whole tiles, 1 the first part of K by the tiles' own
 // pairs of SMs and the rest by the pairs left over, n > 1: K in n parts

@@ -16,6 +16,8 @@
 // host/ops.cpp (gather_room).
 #include "sparse_rows.h"
 
+#include "gemm_tcgen05.h"
+
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -171,7 +173,7 @@ extern "C" int rb_rows_gather(const void* dy, long long ld, const void* x, long 
     if (cols % 8 || x_cols % 8 || ld % 8 || x_ld % 8) return -2;
     if (off16(dy, x, dy_out, x_out, dx32)) return -5;
     // (about four blocks of 256 threads to an SM: 64 KiB on their way there)
-    return launch_after(rows_gather_kernel, 148 * 4, 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(dy),
+    return launch_after(rows_gather_kernel, num_sms() * 4, 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(dy),
                         ld / 8, static_cast<const uint4*>(x), x_ld / 8, cols / 8, x_cols / 8, idx, ctl,
                         static_cast<uint4*>(dy_out), static_cast<uint4*>(x_out),
                         reinterpret_cast<float4*>(dx32)) == cudaSuccess

@@ -63,6 +63,7 @@ struct Api {
     int (*bn_bwd)(const void*, const void*, const void*, const float*, const float*, const float*, float*, float*, float*,
                   void*, void*, long long, int, int, int, void*);
     long long (*bn_part_floats)(long long, int);
+    int (*gemm_pairs)();
     decltype(&rb_rows_plan) rows_plan;
     decltype(&rb_rows_gather) rows_gather;
     decltype(&rb_rows_scatter) rows_scatter;
@@ -236,13 +237,14 @@ struct Rows {
 //     4096 x  768 x 30528         363 -> 149   320 -> 162   320 -> 200   321 -> 241   323 -> 291   326 -> 352   326 -> 328
 // Rows of zeros are read to find them (425 MB at 15 % of 8192 x 30528: 81 us), which is lost where a few rows more than
 // three quarters count: 8 % of the backward at worst.  Both products use the kernel of CTA pairs whichever form runs, so an
-// input gradient of fewer tiles than two thirds of the pairs stays out (2048 x 1024 x 30528, where all rows count: 235 ->
+// input gradient of fewer tiles than 0.64 of the pairs stays out (2048 x 1024 x 30528, where all rows count: 235 ->
 // 281; 1024 x 1024 x 30528 gains at 15 %, 181 -> 132, and loses at 100 %, 189 -> 238).
-// Returns how many rows there is room for, in steps of 64 (few rows leave none: 0, as where the look is not worth it).
-int64_t gather_room(int64_t rows, int64_t cols, int64_t inputs) {
+// `pairs`: of SMs that work on 256 x 256 tiles at once (rb_gemm_pairs).  Returns how many rows there is room for, in steps of 64 (few rows leave none: 0, as where the look is not worth it).
+int64_t gather_room(int64_t rows, int64_t cols, int64_t inputs, int64_t pairs) {
     auto tiles = [](int64_t m, int64_t n) { return (m + 255) / 256 * ((n + 255) / 256); };
-    if (cols < 4 * inputs || cols % 8 || inputs % 8 || cols > (1 << 22) || rows >= (1 << 30) || tiles(cols, inputs) < 74 ||
-        tiles(rows, inputs) < 48 || static_cast<double>(rows) * cols * inputs < 9e10)
+    if (pairs <= 0 || cols < 4 * inputs || cols % 8 || inputs % 8 || cols > (1 << 22) || rows >= (1 << 30) ||
+        tiles(cols, inputs) < pairs || 25 * tiles(rows, inputs) < 16 * pairs ||
+        static_cast<double>(rows) * cols * inputs < 9e10)
         return 0;
     return std::min<int64_t>(rows / 4 * 3, (int64_t{1} << 30) / cols) / 64 * 64;   // (2 GiB at most)
 }
@@ -250,7 +252,7 @@ int64_t gather_room(int64_t rows, int64_t cols, int64_t inputs) {
 Rows gather_rows(const Mat& dy, const Mat& x, bool want_dx, int dtype, const at::TensorOptions& o) {
     Rows r;
     if (at::globalContext().deterministicAlgorithms()) return r;
-    r.room = gather_room(dy.rows, dy.cols, x.cols);
+    r.room = gather_room(dy.rows, dy.cols, x.cols, api.gemm_pairs());
     if (r.room == 0) return r;
     const auto ints = o.dtype(at::kInt);
     r.ctl = at::empty({2}, ints);
@@ -1221,6 +1223,7 @@ void init(const std::unordered_map<std::string, uintptr_t>& fns, py::object erro
     set(api.bn_fwd, "rb_bn_fwd");
     set(api.bn_bwd, "rb_bn_bwd");
     set(api.bn_part_floats, "rb_bn_part_floats");
+    set(api.gemm_pairs, "rb_gemm_pairs");
     set(api.rows_plan, "rb_rows_plan");
     set(api.rows_gather, "rb_rows_gather");
     set(api.rows_scatter, "rb_rows_scatter");

@@ -20,7 +20,7 @@ _lib = None
 # device kernels launched per C entry point (the optimizer / element-wise entries launch one)
 _KERNELS_PER_CALL = {"rb_bn_fwd": 3, "rb_bn_bwd": 3, "rb_ln_bwd": 2, "rb_xent_fwd": 2, "rb_attn_bwd": 3, "rb_rows_plan": 2,
                      "rb_bn_part_floats": 0, "rb_read_error": 0, "rb_ln_supported": 0, "rb_ln_bwd_grid": 0, "rb_gemm_splits": 0,
-                     "rb_gemm_last_wave": 0, "rb_error_peek_async": 0}
+                     "rb_gemm_last_wave": 0, "rb_gemm_pairs": 0, "rb_error_peek_async": 0}
 _launches = 0
 
 
@@ -86,7 +86,7 @@ def lib() -> ctypes.CDLL:
 
 
 _host = None
-_HOST_ENTRIES = ("rb_gemm", "rb_gemm_splits", "rb_unstack3", "rb_gelu", "rb_colsum", "rb_ln_fwd", "rb_ln_bwd",
+_HOST_ENTRIES = ("rb_gemm", "rb_gemm_splits", "rb_gemm_pairs", "rb_unstack3", "rb_gelu", "rb_colsum", "rb_ln_fwd", "rb_ln_bwd",
                  "rb_ln_bwd16", "rb_ln_bwd_grid", "rb_embed_fwd", "rb_embed_bwd", "rb_xent_fwd", "rb_xent_bwd",
                  "rb_attn_fwd", "rb_attn_bwd", "rb_bn_fwd", "rb_bn_bwd", "rb_bn_part_floats", "rb_rows_plan", "rb_rows_gather",
                  "rb_rows_scatter")

@@ -48,16 +48,18 @@ def test_force_builds_a_library_newer_than_its_sources(monkeypatch, tmp_path, fo
     assert [p.name for p in tmp_path.iterdir()] == [path.name]      # written beside and moved into place
 
 
-@pytest.mark.parametrize("rows,cols,inputs,room", [
-    (85, 65536, 16384, 0), (42, 131072, 16384, 0), (87, 131072, 16384, 0), (88, 65536, 16384, 64),
-    (29, 256000, 12288, 0), (56, 131072, 12288, 0), (88, 131072, 12288, 64),
-    (8192, 30528, 1024, 6144), (6144, 30528, 1024, 4608), (4096, 30528, 768, 3072), (4099, 28680, 776, 3072),
-    (2048, 30528, 1024, 0), (8192, 30529, 1024, 0), (8192, 4095 * 8, 8192, 0), (1 << 20, 1 << 20, 1024, 1024)])
-def test_room_for_gathered_rows(rows, cols, inputs, room):
+@pytest.mark.parametrize("rows,cols,inputs,pairs,room", [
+    (85, 65536, 16384, 74, 0), (42, 131072, 16384, 74, 0), (87, 131072, 16384, 74, 0), (88, 65536, 16384, 74, 64),
+    (29, 256000, 12288, 74, 0), (56, 131072, 12288, 74, 0), (88, 131072, 12288, 74, 64),
+    (8192, 30528, 1024, 74, 6144), (6144, 30528, 1024, 74, 4608), (4096, 30528, 768, 74, 3072), (4099, 28680, 776, 74, 3072),
+    (2048, 30528, 1024, 74, 0), (8192, 30529, 1024, 74, 0), (8192, 4095 * 8, 8192, 74, 0), (1 << 20, 1 << 20, 1024, 74, 1024),
+    # the line for the tiles follows the SMs: an input gradient of 48 tiles on 74 pairs and on 76, a weight of 76
+    (4096, 30528, 768, 76, 0), (1 << 16, 76 * 256, 256, 76, 49152), (1 << 16, 76 * 256, 256, 77, 0), (8192, 30528, 1024, 0, 0)])
+def test_room_for_gathered_rows(rows, cols, inputs, pairs, room):
     """A wide layer's backward looks at its rows only where it has room for 64 of them or more: output layers of many inputs
     and few rows, for which nothing is left of three quarters in steps of 64, go over all rows."""
     import torch  # noqa: F401
 
     from rannc_b200 import _host
 
-    assert _host.gather_room(rows, cols, inputs) == room
+    assert _host.gather_room(rows, cols, inputs, pairs) == room

@@ -154,3 +154,55 @@ def test_few_rows_of_many_inputs():
         bound = u * want.abs() + (1e-5 + terms / 16 * 2.0 ** -23) * want.abs().max() + 1e-6   # (as above)
         assert ((got.double() - want).abs() <= bound).all()
     assert (x.grad[10:80] == 0).all()
+
+
+def _product(a, b, out, ctl, mode, flags, M, N, K, a_major, colsum=None, rows_out=0):
+    """rb_gemm over gathered rows; returns its code."""
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops.gemm import _Args
+
+    g = _Args()
+    g.A, g.B, g.D = a.data_ptr(), b.data_ptr(), out.data_ptr()
+    g.M, g.N, g.K, g.batch = M, N, K, 1
+    g.lda, g.ldb, g.ldd = a.stride(0), b.stride(0), out.stride(0)
+    g.a_major, g.b_major = a_major, 1
+    g.in_dtype = 1 if a.dtype == torch.bfloat16 else 0
+    g.out_dtype = 1 if out.dtype == torch.float32 else 0
+    g.flags, g.alpha = flags, 1.0
+    g.a_colsum = None if colsum is None else colsum.data_ptr()
+    g.rows_ctl, g.rows_mode = ctl.data_ptr(), mode
+    return _lib.lib().rb_gemm(ctypes.byref(g), _lib.stream_ptr())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("V,H,room,count", [(264, 72, 64, 1), (520, 264, 128, 63), (520, 264, 128, 64), (264, 72, 128, 65),
+                                            (1288, 520, 4096, 4095), (1288, 520, 4096, 2113)])
+def test_weight_gradient_over_gathered_rows(dtype, fp32, V, H, room, count):
+    """K counted on the device: the number of rows on both sides of a step, up to the room.  Few tiles, which an ordinary
+    product added to fp32 would share out; the form that is not in use leaves everything as it is."""
+    from rannc_b200.ops import _lib
+
+    torch.manual_seed(room + count)
+    dy, x = torch.randn(room, V, device="cuda").to(dtype), torch.randn(room, H, device="cuda").to(dtype)
+    pad = (count + 64) // 64 * 64
+    dy[count:pad] = 0
+    x[count:pad] = 0
+    dy[pad:] = float("nan")
+    x[pad:] = float("nan")
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for use in (1, 0):
+        ctl = torch.tensor([count, use], dtype=torch.int32, device="cuda")
+        out = torch.full((V, H), 3.0, dtype=torch.float32 if fp32 else dtype, device="cuda")
+        sums = torch.full((V,), 3.0, device="cuda")
+        assert _product(dy, x, out, ctl, 2, 16 if fp32 else 0, V, H, room, 1, sums) == 0
+        torch.cuda.synchronize()
+        assert _lib.read_error() == 0
+        if not use:
+            assert (out == 3.0).all() and (sums == 3.0).all()
+            continue
+        d, e = dy[:count].double(), x[:count].double()
+        for got, want in ((out.double() - (3.0 if fp32 else 0.0), d.t() @ e), (sums.double() - 3.0, d.sum(0))):
+            # (as above; a column sum has no rounding of its own)
+            bound = (0.0 if fp32 or got.dim() == 1 else u) * want.abs() + (1e-5 + count / 16 * 2.0 ** -23) * want.abs().max() + 1e-6
+            assert ((got - want).abs() <= bound).all()
