@@ -107,14 +107,14 @@ struct GemmKernelParams {
     // 1: the bias / the matrices beside the output / the output start their rows on 16-byte boundaries
     int bias_al, in_al, out_al;
     float* a_colsum;   // not null: column sums of the stored A (MN-major) are added here
-    const int* rows_ctl;   // see RbGemmArgs
-    int rows_mode;
+    int* rows_ctl;   // see RbGemmArgs
+    int rows_mode, rows_out;
 };
 
 // A product whose rows were gathered on the device (RbGemmArgs::rows_ctl): how many there are, and whether this form of the
 // product is the one in use, is read here.  (The host cannot choose: it does not wait for the device.)
 constexpr int ROWS_DRAIN_STEPS = 6;   // what a part costs besides its own steps (as DRAIN_STEPS below)
-__device__ __forceinline__ void apply_rows(GemmKernelParams& p, int units) {
+__device__ __forceinline__ void apply_rows(GemmKernelParams& p, int units, bool first) {
     const int count = p.rows_ctl[0], gathered = p.rows_ctl[1];
     if ((p.rows_mode != RB_GEMM_ROWS_ALL) != (gathered != 0)) {
         p.num_tiles = 0;   // the other form runs
@@ -130,15 +130,19 @@ __device__ __forceinline__ void apply_rows(GemmKernelParams& p, int units) {
         // one more row, of zeros: its product stands for every row that was left out
         p.num_m_blocks = (count + 1 + 2 * BM - 1) / (2 * BM);
         p.base_tiles = p.num_m_blocks * p.num_n_blocks;
-        // few tiles and a long K (the layer's outputs): parts whose waves take the fewest steps, each with its drain
+        // few tiles and a long K (the layer's outputs): parts whose waves take the fewest steps, each with its drain, and
+        // three eighths of a step for every tile of a part that is written and read once more (512 KiB from L2)
+        const int part_rows = p.num_m_blocks * 2 * BM;
         int split = 1, best = 0x7fffffff;
-        for (int s = 1; s <= 16 && s * 4 <= p.num_kb; ++s) {
-            const int cost = (p.base_tiles * s + units - 1) / units * ((p.num_kb + s - 1) / s + ROWS_DRAIN_STEPS);
+        for (int s = 1; s <= 16 && s * 4 <= p.num_kb && s * part_rows <= p.rows_out; ++s) {
+            const int cost = (p.base_tiles * s + units - 1) / units * ((p.num_kb + s - 1) / s + ROWS_DRAIN_STEPS) +
+                             p.base_tiles * s * 3 / 8;
             if (cost < best) best = cost, split = s;
         }
         p.kb_per_split = (p.num_kb + split - 1) / split;
         p.split_k = (p.num_kb + p.kb_per_split - 1) / p.kb_per_split;
         p.num_tiles = p.base_tiles * p.split_k;
+        if (first) p.rows_ctl[2] = p.split_k, p.rows_ctl[3] = part_rows;
     }
 }
 
@@ -320,7 +324,7 @@ __global__ void __launch_bounds__(Cfg<PAIR, BN, EPI_WARPS>::THREADS, 1)
     if constexpr (ROWS) {
         if (threadIdx.x == 0) {
             s_params = params;
-            apply_rows(s_params, tile_step);
+            apply_rows(s_params, tile_step, blockIdx.x == 0);
         }
         __syncthreads();
     }
@@ -714,6 +718,9 @@ __global__ void __launch_bounds__(Cfg<PAIR, BN, EPI_WARPS>::THREADS, 1)
                 const int row0 = mb * TILE_M + static_cast<int>(crank) * BM + q * 32;
                 const int col0 = nb * BN + part * PART_COLS;
                 const bool row_ok = row0 + lane < p.M;
+                int d_row = row0;
+                if constexpr (ROWS && !OUT16)   // (parts one below the other)
+                    if (p.rows_mode == RB_GEMM_ROWS_M) d_row += kb_begin / p.kb_per_split * p.num_m_blocks * TILE_M;
                 // blocks of this warp that hold part of the matrix
                 const int nblk = row0 < p.M ? max(0, min(PART_COLS / 32, (p.N - col0 + 31) / 32)) : 0;
                 auto fetch_aux = [&](int c) {   // (one lane; the block before has left its place)
@@ -812,9 +819,9 @@ __global__ void __launch_bounds__(Cfg<PAIR, BN, EPI_WARPS>::THREADS, 1)
                     __syncwarp();
                     if (lane == 0) {
                         if (add_out)
-                            tma_reduce_add_3d(&tmD, dst, col, row0, b);
+                            tma_reduce_add_3d(&tmD, dst, col, d_row, b);
                         else
-                            tma_store_3d(&tmD, dst, col, row0, b);
+                            tma_store_3d(&tmD, dst, col, d_row, b);
                         tma_store_commit();
                         if (OUT16 && act_dgelu && c + 1 < nblk) fetch_aux(c + 1);
                     }
@@ -1398,13 +1405,14 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
     p.a_colsum = a->a_colsum;
     p.rows_ctl = a->rows_ctl;
     p.rows_mode = a->rows_mode;
+    p.rows_out = a->rows_out;
+    const bool rows_m = a->rows_ctl && a->rows_mode == RB_GEMM_ROWS_M;
     if (a->rows_ctl) {
-        // plain products of one matrix; what is gathered along K or M is cut into whole tiles (ROWS_M: of sums)
+        // plain products of one matrix; what is gathered along K is cut into whole tiles
         if (a->batch != 1 || a->ag_nranks > 1 || a->rs_nranks > 1 || a->conv_taps > 0 || a->wgrad_taps > 0 || a->map_hp > 0 ||
             (a->flags & ~RB_GEMM_ACCUM) || a->rows_mode < RB_GEMM_ROWS_ALL || a->rows_mode > RB_GEMM_ROWS_M ||
-            (a->rows_mode == RB_GEMM_ROWS_M && (a->a_major != 0 || a->out_dtype != 1 || a->flags != RB_GEMM_ACCUM)))
+            (rows_m && (a->a_major != 0 || a->out_dtype != 1 || a->flags || a->rows_out % 256 || a->rows_out < a->M)))
             return -10;
-        if (a->rows_mode == RB_GEMM_ROWS_M) p.tail_tiles = 0, p.partial = 1;
     }
     if (a->a_colsum && (a->a_major != 1 || a->batch != 1 || a->ag_nranks > 1)) return -8;
     p.wgrad_taps = 0;
@@ -1482,11 +1490,13 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
                !(fp32_out && (aux_w || aux_r)) && (!(aux_w || aux_r) || addressable(aux, 2));
     if (p.staged) {
         const int64_t sd = a->batch > 1 ? a->strideD : a->M * a->ldd;
-        rc = make_tmap_block32(&tmD, a->D, fp32_out, a->in_dtype, a->N, a->M, a->batch, a->ldd * out_es, sd * out_es);
+        rc = make_tmap_block32(&tmD, a->D, fp32_out, a->in_dtype, a->N, rows_m ? a->rows_out : a->M, a->batch, a->ldd * out_es,
+                               (rows_m ? a->rows_out * a->ldd : sd) * out_es);
         if (!rc && (aux_w || aux_r))
             rc = make_tmap_block32(&tmAux, aux, false, a->in_dtype, a->N, a->M, a->batch, a->ldd * 2, sd * 2);
         if (rc) p.staged = 0;
     }
+    if (rows_m && !p.staged) return -10;   // (only the staged epilogue keeps the parts apart)
 
     return a->in_dtype == 1 ? dispatch<__nv_bfloat16>(*a, pair, tn, tmA, tmB, tmD, tmAux, p, stream)
                             : dispatch<__half>(*a, pair, tn, tmA, tmB, tmD, tmAux, p, stream);

@@ -70,9 +70,11 @@ typedef struct RbGemmArgs {
     // of the product this is; the form that is not in use does nothing.
     //  RB_GEMM_ROWS_ALL: the product over all rows
     //  RB_GEMM_ROWS_K: K is the number of gathered rows (K here: room for them; those up to the next multiple of 64 are zero)
-    //  RB_GEMM_ROWS_M: M is that number plus one (M here: room for them); results are added to an fp32 matrix, in parts
-    const int32_t* rows_ctl;
-    int32_t rows_mode;
+    //  RB_GEMM_ROWS_M: M is that number plus one (M here: room for them).  Its parts along K go to an fp32 matrix of rows_out
+    //    rows (room for one part at least: M up to the next multiple of 256) one below the other, and are added up by whoever
+    //    reads them: rows_ctl[2] says how many there are, rows_ctl[3] how many rows lie between two (rb_rows_scatter_parts)
+    int32_t* rows_ctl;
+    int32_t rows_mode, rows_out;
 } RbGemmArgs;
 
 enum { RB_GEMM_ROWS_ALL = 1, RB_GEMM_ROWS_K = 2, RB_GEMM_ROWS_M = 3 };

@@ -11,7 +11,7 @@
 // gradient is 0 * W, zero or NaN column by column and the same for every such row: a row of zeros behind the gathered ones
 // goes through the product, and its result is theirs.
 //
-// 8192 rows, 1024 to 30528, 15 % of the rows not zero: 636 -> 279 us for the backward, of which looking 81 (5.2 TB/s),
+// 8192 rows, 1024 to 30528, 15 % of the rows not zero: 649 -> 272 us for the backward, of which looking 81 (5.2 TB/s),
 // gathering 25, the two products 150; what it costs where every row counts, and the rule for when to look, stand in
 // host/ops.cpp (gather_room).
 #include "sparse_rows.h"
@@ -132,20 +132,39 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// A block has 256 columns of SCATTER_ROWS rows, a thread 8 columns of every eighth row.  The parts of the row of zeros, which
+// most rows get, are added up once for those.
+constexpr int SCATTER_ROWS = 32;
 template <typename T>
 __global__ void __launch_bounds__(256)
-    rows_scatter_kernel(const float4* dx32, uint4* dx, int rows, int nv, const int32_t* pos, const int32_t* ctl) {
+    rows_scatter_kernel(const float4* dx32, uint4* dx, int rows, int nv, const int32_t* pos, const int32_t* ctl, bool in_parts) {
     grid_trigger();
     grid_wait();
     if (!ctl[1]) return;
-    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (row >= rows) return;
-    const int k = pos[row];
-    const float4* src = dx32 + static_cast<long long>(k < 0 ? ctl[0] : k) * 2 * nv;
-    for (int i = lane; i < nv; i += 32) {
-        const float4 a = src[2 * i], b = src[2 * i + 1];
-        dx[static_cast<long long>(row) * nv + i] =
-            make_uint4(pack2<T>(a.x, a.y), pack2<T>(a.z, a.w), pack2<T>(b.x, b.y), pack2<T>(b.z, b.w));
+    const int col = blockIdx.y * 32 + (threadIdx.x & 31);
+    if (col >= nv) return;
+    const int parts = in_parts ? ctl[2] : 1;
+    const long long step = in_parts ? static_cast<long long>(ctl[3]) * 2 * nv : 0;
+    auto total = [&](int k) {
+        const float4* src = dx32 + static_cast<long long>(k) * 2 * nv + 2 * col;
+        float4 a = src[0], b = src[1];
+#pragma unroll 4
+        for (int s = 1; s < parts; ++s) {
+            const float4 c = src[s * step], d = src[s * step + 1];
+            a.x += c.x, a.y += c.y, a.z += c.z, a.w += c.w;
+            b.x += d.x, b.y += d.y, b.z += d.z, b.w += d.w;
+        }
+        return make_uint4(pack2<T>(a.x, a.y), pack2<T>(a.z, a.w), pack2<T>(b.x, b.y), pack2<T>(b.z, b.w));
+    };
+    const int first = blockIdx.x * SCATTER_ROWS + (threadIdx.x >> 5);
+    int k[SCATTER_ROWS / 8];
+#pragma unroll
+    for (int u = 0; u < SCATTER_ROWS / 8; ++u) k[u] = first + 8 * u < rows ? pos[first + 8 * u] : -1;
+    const uint4 left_out = total(ctl[0]);
+#pragma unroll
+    for (int u = 0; u < SCATTER_ROWS / 8; ++u) {
+        const int row = first + 8 * u;
+        if (row < rows) dx[static_cast<long long>(row) * nv + col] = k[u] < 0 ? left_out : total(k[u]);
     }
 }
 
@@ -181,15 +200,24 @@ extern "C" int rb_rows_gather(const void* dy, long long ld, const void* x, long 
                : -1;
 }
 
-extern "C" int rb_rows_scatter(const float* dx32, void* dx, int rows, int x_cols, const int32_t* pos, const int32_t* ctl,
-                               int dtype, void* stream) {
+static int rows_scatter(const float* dx32, void* dx, int rows, int x_cols, const int32_t* pos, const int32_t* ctl, int dtype,
+                        bool in_parts, void* stream) {
     if (rows <= 0) return 0;
     if (x_cols % 8) return -2;
     if (off16(dx32, dx)) return -5;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto kern = dtype == 1 ? rows_scatter_kernel<__nv_bfloat16> : rows_scatter_kernel<__half>;
-    return launch_after(kern, (rows + 7) / 8, 256, 0, st, reinterpret_cast<const float4*>(dx32), static_cast<uint4*>(dx), rows,
-                        x_cols / 8, pos, ctl) == cudaSuccess
+    const dim3 grid((rows + SCATTER_ROWS - 1) / SCATTER_ROWS, (x_cols / 8 + 31) / 32);
+    return launch_after(kern, grid, 256, 0, st, reinterpret_cast<const float4*>(dx32), static_cast<uint4*>(dx), rows,
+                        x_cols / 8, pos, ctl, in_parts) == cudaSuccess
                ? 0
                : -1;
+}
+extern "C" int rb_rows_scatter(const float* dx32, void* dx, int rows, int x_cols, const int32_t* pos, const int32_t* ctl,
+                               int dtype, void* stream) {
+    return rows_scatter(dx32, dx, rows, x_cols, pos, ctl, dtype, false, stream);
+}
+extern "C" int rb_rows_scatter_parts(const float* dx32, void* dx, int rows, int x_cols, const int32_t* pos, const int32_t* ctl,
+                                     int dtype, void* stream) {
+    return rows_scatter(dx32, dx, rows, x_cols, pos, ctl, dtype, true, stream);
 }

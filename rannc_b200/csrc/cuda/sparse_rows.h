@@ -16,7 +16,10 @@ int rb_rows_plan(const void* dy, long long ld, const void* x, long long x_ld, in
 // multiple of 64 (one at least); as many rows of dx32 [room, x_cols], and one more, are cleared (null: none)
 int rb_rows_gather(const void* dy, long long ld, const void* x, long long x_ld, int cols, int x_cols, const int32_t* idx,
                    const int32_t* ctl, void* dy_out, void* x_out, float* dx32, void* stream);
-// dx [rows, x_cols] (16-bit): each row's place in dx32, or the row behind the last for those that were left out
+// dx [rows, x_cols] (16-bit): each row's place in dx32, or the row behind the last for those that were left out.  _parts: the
+// sum of ctl[2] rows, ctl[3] rows apart, in that order (RB_GEMM_ROWS_M)
+int rb_rows_scatter_parts(const float* dx32, void* dx, int rows, int x_cols, const int32_t* pos, const int32_t* ctl, int dtype,
+                          void* stream);
 int rb_rows_scatter(const float* dx32, void* dx, int rows, int x_cols, const int32_t* pos, const int32_t* ctl, int dtype,
                     void* stream);
 

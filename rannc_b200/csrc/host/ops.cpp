@@ -66,7 +66,7 @@ struct Api {
     int (*gemm_pairs)();
     decltype(&rb_rows_plan) rows_plan;
     decltype(&rb_rows_gather) rows_gather;
-    decltype(&rb_rows_scatter) rows_scatter;
+    decltype(&rb_rows_scatter_parts) rows_scatter;
 } api;
 std::atomic<long long> launches{0};
 PyObject* error_class = nullptr;   // ops._lib.KernelLibraryError
@@ -184,8 +184,8 @@ struct Epi {
     void* aux_out = nullptr;
     bool gelu = false, dgelu = false, accumulate = false;
     float* a_colsum = nullptr;   // the column sums of a stored [K, M] are added here
-    const int32_t* rows_ctl = nullptr;   // see RbGemmArgs
-    int rows_mode = 0;
+    int32_t* rows_ctl = nullptr;   // see RbGemmArgs
+    int rows_mode = 0, rows_out = 0;
 };
 // out [M, N] = epilogue(op(a) op(b)), rows ldd apart (0: N)
 void gemm(const Mat& a, const Mat& b, bool trans_a, bool trans_b, void* out, bool out_fp32, int dtype, const Epi& e,
@@ -217,6 +217,7 @@ void gemm(const Mat& a, const Mat& b, bool trans_a, bool trans_b, void* out, boo
     g.a_colsum = e.a_colsum;
     g.rows_ctl = e.rows_ctl;
     g.rows_mode = e.rows_mode;
+    g.rows_out = e.rows_out;
     g.in_order = at::globalContext().deterministicAlgorithms() ? 1 : 0;
     check(api.gemm(&g, cur_stream()), "rb_gemm");
 }
@@ -226,17 +227,19 @@ struct Rows {
     Tensor idx, pos, ctl, dy, x, dx32;
     Mat dym, xm;
     int64_t room = 0;
-    const int32_t* ctl_ptr() const { return static_cast<const int32_t*>(ctl.data_ptr()); }
+    int32_t* ctl_ptr() const { return static_cast<int32_t*>(ctl.data_ptr()); }
 };
 // Worth a look at the rows: a wide output layer (the rows of hidden layers' gradients are not zero), and products long enough
 // that the look costs next to nothing where every row counts.  Backward of the layer (us), one B200, over all rows ->
 // gathered, by the share of rows that count (up to three quarters are gathered):
 //     rows x inputs x outputs     2 %          15 %         30 %         45 %         60 %         80 %         100 %
-//     8192 x 1024 x 30528         633 -> 205   643 -> 281   660 -> 395   685 -> 520   701 -> 662   743 -> 748   735 -> 738
-//     6144 x 1024 x 30528         554 -> 180   556 -> 229   564 -> 311   615 -> 414   620 -> 509   603 -> 637   613 -> 618
-//     4096 x  768 x 30528         363 -> 149   320 -> 162   320 -> 200   321 -> 241   323 -> 291   326 -> 352   326 -> 328
+//     8192 x 1024 x 30528         637 -> 217   649 -> 272   674 -> 381   708 -> 491   720 -> 620   747 -> 686   781 -> 690
+//     6144 x 1024 x 30528         560 -> 207   564 -> 247   570 -> 311   592 -> 385   617 -> 467   627 -> 587   637 -> 569
+//     4096 x  768 x 30528         308 -> 153   310 -> 170   312 -> 203   312 -> 237   314 -> 276   318 -> 321   320 -> 300
+//     4096 x 4096 x 32000        1377 -> 380  1444 -> 464  1479 -> 628  1561 -> 822  1580 ->1132  1668 ->1502  1723 ->1541
+// (all rows: before the look existed; what both sides do at 80 and 100 % differs by the clock under the power cap.)
 // Rows of zeros are read to find them (425 MB at 15 % of 8192 x 30528: 81 us), which is lost where a few rows more than
-// three quarters count: 8 % of the backward at worst.  Both products use the kernel of CTA pairs whichever form runs, so an
+// three quarters count: the look is 3 to 8 % of the backward there.  Both products use the kernel of CTA pairs whichever form runs, so an
 // input gradient of fewer tiles than 0.64 of the pairs stays out (2048 x 1024 x 30528, where all rows count: 235 ->
 // 281; 1024 x 1024 x 30528 gains at 15 %, 181 -> 132, and loses at 100 %, 189 -> 238).
 // `pairs`: of SMs that work on 256 x 256 tiles at once (rb_gemm_pairs).  Returns how many rows there is room for, in steps of 64 (few rows leave none: 0, as where the look is not worth it).
@@ -252,22 +255,28 @@ int64_t gather_room(int64_t rows, int64_t cols, int64_t inputs, int64_t pairs) {
 Rows gather_rows(const Mat& dy, const Mat& x, bool want_dx, int dtype, const at::TensorOptions& o) {
     Rows r;
     if (at::globalContext().deterministicAlgorithms()) return r;
-    r.room = gather_room(dy.rows, dy.cols, x.cols, api.gemm_pairs());
+    const int64_t pairs = api.gemm_pairs();
+    r.room = gather_room(dy.rows, dy.cols, x.cols, pairs);
     if (r.room == 0) return r;
     const auto ints = o.dtype(at::kInt);
-    r.ctl = at::empty({2}, ints);
+    r.ctl = at::empty({4}, ints);
     r.idx = at::empty({r.room}, ints);
     r.pos = at::empty({dy.rows}, ints);
     const Tensor live = at::empty({dy.rows}, o.dtype(at::kByte));
     r.dy = at::empty({r.room, dy.cols}, o);
     r.x = at::empty({r.room, x.cols}, o);
-    if (want_dx) r.dx32 = at::empty({r.room, x.cols}, o.dtype(at::kFloat));
+    if (want_dx) {
+        // the input gradient's product in parts along K, each in rows of its own and added up in their order (as reductions
+        // into one matrix they came in any, and dx did not repeat): room for as many as make four waves of tiles
+        const int64_t waves = 4 * pairs * 256 / ((x.cols + 255) / 256);
+        r.dx32 = at::empty({(std::max(r.room, waves) + 255) / 256 * 256, x.cols}, o.dtype(at::kFloat));
+    }
     check(api.rows_plan(dy.p, dy.ld, x.p, x.ld, static_cast<int>(dy.rows), static_cast<int>(dy.cols), static_cast<int>(x.cols),
                         static_cast<int>(r.room), mptr<uint8_t>(live), mptr<int32_t>(r.idx), mptr<int32_t>(r.pos),
                         mptr<int32_t>(r.ctl), dtype, cur_stream()),
           "rb_rows_plan", 2);
     check(api.rows_gather(dy.p, dy.ld, x.p, x.ld, static_cast<int>(dy.cols), static_cast<int>(x.cols), mptr<int32_t>(r.idx),
-                          r.ctl_ptr(), r.dy.data_ptr(), r.x.data_ptr(), mptr<float>(r.dx32), cur_stream()),
+                          r.ctl_ptr(), r.dy.data_ptr(), r.x.data_ptr(), nullptr, cur_stream()),
           "rb_rows_gather");
     r.dym = rows_of(r.dy);
     r.xm = rows_of(r.x);
@@ -428,13 +437,12 @@ struct LinearNode : Node {
             if (look) {
                 e.rows_ctl = rows.ctl_ptr();
                 e.rows_mode = RB_GEMM_ROWS_M;
-                e.accumulate = true;
+                e.rows_out = static_cast<int>(rows.dx32.size(0));
                 gemm(rows.dym, wm, false, false, rows.dx32.data_ptr(), true, dt, e);
                 check(api.rows_scatter(mptr<float>(rows.dx32), dx.data_ptr(), static_cast<int>(d.rows),
                                        static_cast<int>(xm.cols), mptr<int32_t>(rows.pos), rows.ctl_ptr(), dt, cur_stream()),
                       "rb_rows_scatter");
                 e.rows_mode = RB_GEMM_ROWS_ALL;
-                e.accumulate = false;
             }
             gemm(d, wm, false, false, dx.data_ptr(), false, dt, e);
         }
@@ -1226,7 +1234,7 @@ void init(const std::unordered_map<std::string, uintptr_t>& fns, py::object erro
     set(api.gemm_pairs, "rb_gemm_pairs");
     set(api.rows_plan, "rb_rows_plan");
     set(api.rows_gather, "rb_rows_gather");
-    set(api.rows_scatter, "rb_rows_scatter");
+    set(api.rows_scatter, "rb_rows_scatter_parts");
     error_class = error.release().ptr();
 }
 void set_listener(py::object fn) {

@@ -89,7 +89,7 @@ _host = None
 _HOST_ENTRIES = ("rb_gemm", "rb_gemm_splits", "rb_gemm_pairs", "rb_unstack3", "rb_gelu", "rb_colsum", "rb_ln_fwd", "rb_ln_bwd",
                  "rb_ln_bwd16", "rb_ln_bwd_grid", "rb_embed_fwd", "rb_embed_bwd", "rb_xent_fwd", "rb_xent_bwd",
                  "rb_attn_fwd", "rb_attn_bwd", "rb_bn_fwd", "rb_bn_bwd", "rb_bn_part_floats", "rb_rows_plan", "rb_rows_gather",
-                 "rb_rows_scatter")
+                 "rb_rows_scatter_parts")
 
 
 def host_loaded() -> bool:

@@ -31,7 +31,7 @@ class _Args(ctypes.Structure):
         ("map_w", ctypes.c_int32), ("map_pad", ctypes.c_int32), ("wgrad_taps", ctypes.c_int32),
         ("a_colsum", ctypes.c_void_p), ("tile_n", ctypes.c_int32),
         ("in_order", ctypes.c_int32),
-        ("rows_ctl", ctypes.c_void_p), ("rows_mode", ctypes.c_int32),
+        ("rows_ctl", ctypes.c_void_p), ("rows_mode", ctypes.c_int32), ("rows_out", ctypes.c_int32),
     ]
 
 

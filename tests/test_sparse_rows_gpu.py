@@ -170,7 +170,7 @@ def _product(a, b, out, ctl, mode, flags, M, N, K, a_major, colsum=None, rows_ou
     g.out_dtype = 1 if out.dtype == torch.float32 else 0
     g.flags, g.alpha = flags, 1.0
     g.a_colsum = None if colsum is None else colsum.data_ptr()
-    g.rows_ctl, g.rows_mode = ctl.data_ptr(), mode
+    g.rows_ctl, g.rows_mode, g.rows_out = ctl.data_ptr(), mode, rows_out
     return _lib.lib().rb_gemm(ctypes.byref(g), _lib.stream_ptr())
 
 
@@ -206,3 +206,61 @@ def test_weight_gradient_over_gathered_rows(dtype, fp32, V, H, room, count):
             # (as above; a column sum has no rounding of its own)
             bound = (0.0 if fp32 or got.dim() == 1 else u) * want.abs() + (1e-5 + count / 16 * 2.0 ** -23) * want.abs().max() + 1e-6
             assert ((got - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("V,H,room,count,rows_out", [(64, 8, 64, 1, 256), (1096, 264, 320, 255, 512), (1096, 264, 320, 256, 2048),
+                                                     (4104, 520, 320, 319, 4096), (30528, 136, 704, 511, 16 * 512)])
+def test_input_gradient_over_gathered_rows(dtype, V, H, room, count, rows_out):
+    """M counted on the device: rows on both sides of a tile, with room for one part of K and for many; the parts, added up,
+    are the gathered rows' gradients and that of a row of zeros, and the same to the bit every time."""
+    from rannc_b200.ops import _lib
+
+    torch.manual_seed(room + count)
+    dy, w = torch.randn(room, V, device="cuda").to(dtype), torch.randn(V, H, device="cuda").to(dtype)
+    dy[count:(count + 64) // 64 * 64] = 0
+    dy[(count + 64) // 64 * 64:] = float("nan")
+    rows = count + 5
+    pos = torch.arange(rows, dtype=torch.int32, device="cuda") - 5        # (five rows that were left out)
+    pos[:5] = -1
+    code = 1 if dtype == torch.bfloat16 else 0
+    first = None
+    for use in (1, 1, 1, 0):
+        ctl = torch.tensor([count, use, -9, -9], dtype=torch.int32, device="cuda")
+        parts = torch.full((rows_out, H), 3.0, device="cuda")
+        out = torch.full((rows, H), 5.0, dtype=dtype, device="cuda")
+        assert _product(dy, w, parts, ctl, 3, 0, room, H, V, 0, rows_out=rows_out) == 0
+        assert _lib.lib().rb_rows_scatter_parts(_lib.vp(parts), _lib.vp(out), rows, H, _lib.vp(pos), _lib.vp(ctl), code,
+                                                _lib.stream_ptr()) == 0
+        torch.cuda.synchronize()
+        assert _lib.read_error() == 0
+        if not use:
+            assert (parts == 3.0).all() and (out == 5.0).all() and ctl.tolist() == [count, 0, -9, -9]
+            continue
+        n, apart = ctl[2:].tolist()
+        assert apart == (count + 256) // 256 * 256 and 1 <= n * apart <= rows_out
+        assert n > 1 or rows_out < 2 * apart or V < 512
+        want = dy[:count].double() @ w.double()
+        u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+        bound = u * want.abs() + (1e-5 + V / 16 * 2.0 ** -23) * want.abs().max() + 1e-6   # (as above)
+        assert ((out[5:].double() - want).abs() <= bound).all() and (out[:5] == 0).all()
+        first = out.clone() if first is None else first
+        assert torch.equal(out, first)
+    assert _product(dy, w, parts, ctl, 3, 0, room, H, V, 0, rows_out=256 * ((room - 1) // 256)) == -10
+    assert _product(dy, w, parts, ctl, 3, 16, room, H, V, 0, rows_out=rows_out) == -10
+
+
+def test_wide_layer_backward_repeats_to_the_bit():
+    from rannc_b200.ops import functional as RF
+
+    R, H, V = 4099, 776, 28680
+    torch.manual_seed(10)
+    x = torch.randn(R, H, device="cuda", dtype=torch.bfloat16).requires_grad_(True)
+    w = torch.randn(V, H, device="cuda", dtype=torch.bfloat16).requires_grad_(True)
+    dy = torch.randn(R, V, device="cuda", dtype=torch.bfloat16)
+    dy[torch.rand(R, device="cuda") >= 0.15] = 0
+    first = None
+    for _ in range(30):
+        got = torch.autograd.grad(RF.linear(x, w), (x, w), dy)
+        first = got if first is None else first
+        assert torch.equal(got[0], first[0]) and torch.equal(got[1], first[1])
