@@ -239,10 +239,11 @@ struct Rows {
 //     4096 x 4096 x 32000        1377 -> 380  1444 -> 464  1479 -> 628  1561 -> 822  1580 ->1132  1668 ->1502  1723 ->1541
 // (all rows: before the look existed; what both sides do at 80 and 100 % differs by the clock under the power cap.)
 // Rows of zeros are read to find them (425 MB at 15 % of 8192 x 30528: 81 us), which is lost where a few rows more than
-// three quarters count: the look is 3 to 8 % of the backward there.  Both products use the kernel of CTA pairs whichever form runs, so an
-// input gradient of fewer tiles than 0.64 of the pairs stays out (2048 x 1024 x 30528, where all rows count: 235 ->
-// 281; 1024 x 1024 x 30528 gains at 15 %, 181 -> 132, and loses at 100 %, 189 -> 238).
-// `pairs`: of SMs that work on 256 x 256 tiles at once (rb_gemm_pairs).  Returns how many rows there is room for, in steps of 64 (few rows leave none: 0, as where the look is not worth it).
+// three quarters count: the look is 3 to 8 % of the backward there.  Both products use the kernel of CTA pairs whichever
+// form runs, so an input gradient of fewer tiles than 0.64 of the pairs stays out (2048 x 1024 x 30528, where all rows
+// count: 235 -> 281; 1024 x 1024 x 30528 gains at 15 %, 181 -> 132, and loses at 100 %, 189 -> 238).
+// `pairs`: of SMs that work on 256 x 256 tiles at once (rb_gemm_pairs).  Returns how many rows there is room for, in steps
+// of 64 (few rows leave none: 0, as where the look is not worth it).
 int64_t gather_room(int64_t rows, int64_t cols, int64_t inputs, int64_t pairs) {
     auto tiles = [](int64_t m, int64_t n) { return (m + 255) / 256 * ((n + 255) / 256); };
     if (pairs <= 0 || cols < 4 * inputs || cols % 8 || inputs % 8 || cols > (1 << 22) || rows >= (1 << 30) ||
@@ -251,25 +252,31 @@ int64_t gather_room(int64_t rows, int64_t cols, int64_t inputs, int64_t pairs) {
         return 0;
     return std::min<int64_t>(rows / 4 * 3, (int64_t{1} << 30) / cols) / 64 * 64;   // (2 GiB at most)
 }
-// (empty `ctl`: the call is not one for this)
-Rows gather_rows(const Mat& dy, const Mat& x, bool want_dx, int dtype, const at::TensorOptions& o) {
+int64_t gather_room(const Mat& dy, const Mat& x) {
+    return at::globalContext().deterministicAlgorithms() ? 0 : gather_room(dy.rows, dy.cols, x.cols, api.gemm_pairs());
+}
+// Scratch: three quarters of dy and of x, and 77 MB or three quarters of x in fp32, whatever the number of rows that count
+// (the host does not know it): 470 MB for 8192 x 1024 x 30528.  Where there is no memory for it, `ctl` stays empty.
+Rows gather_rows(const Mat& dy, const Mat& x, int64_t room, bool want_dx, int dtype, const at::TensorOptions& o) {
     Rows r;
-    if (at::globalContext().deterministicAlgorithms()) return r;
-    const int64_t pairs = api.gemm_pairs();
-    r.room = gather_room(dy.rows, dy.cols, x.cols, pairs);
-    if (r.room == 0) return r;
+    r.room = room;
     const auto ints = o.dtype(at::kInt);
-    r.ctl = at::empty({4}, ints);
-    r.idx = at::empty({r.room}, ints);
-    r.pos = at::empty({dy.rows}, ints);
-    const Tensor live = at::empty({dy.rows}, o.dtype(at::kByte));
-    r.dy = at::empty({r.room, dy.cols}, o);
-    r.x = at::empty({r.room, x.cols}, o);
-    if (want_dx) {
-        // the input gradient's product in parts along K, each in rows of its own and added up in their order (as reductions
-        // into one matrix they came in any, and dx did not repeat): room for as many as make four waves of tiles
-        const int64_t waves = 4 * pairs * 256 / ((x.cols + 255) / 256);
-        r.dx32 = at::empty({(std::max(r.room, waves) + 255) / 256 * 256, x.cols}, o.dtype(at::kFloat));
+    Tensor live;
+    try {
+        r.ctl = at::empty({4}, ints);
+        r.idx = at::empty({r.room}, ints);
+        r.pos = at::empty({dy.rows}, ints);
+        live = at::empty({dy.rows}, o.dtype(at::kByte));
+        r.dy = at::empty({r.room, dy.cols}, o);
+        r.x = at::empty({r.room, x.cols}, o);
+        if (want_dx) {
+            // the input gradient's product in parts along K, each in rows of its own and added up in their order (as
+            // reductions into one matrix they came in any, and dx did not repeat): room for four waves of tiles
+            const int64_t waves = 4 * api.gemm_pairs() * 256 / ((x.cols + 255) / 256);
+            r.dx32 = at::empty({(std::max(r.room, waves) + 255) / 256 * 256, x.cols}, o.dtype(at::kFloat));
+        }
+    } catch (const c10::OutOfMemoryError&) {
+        return Rows();   // the products over all rows need none of it
     }
     check(api.rows_plan(dy.p, dy.ld, x.p, x.ld, static_cast<int>(dy.rows), static_cast<int>(dy.cols), static_cast<int>(x.cols),
                         static_cast<int>(r.room), mptr<uint8_t>(live), mptr<int32_t>(r.idx), mptr<int32_t>(r.pos),
@@ -301,7 +308,7 @@ bool in_parts(int64_t m, int64_t n, int64_t rows) {
            !at::globalContext().deterministicAlgorithms() && api.gemm_splits(m, n, rows) > 1;
 }
 Grads param_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& w_mg, bool want_w, const Tensor& bias,
-                  const Tensor& b_mg, bool want_b, int dtype, const Rows* rows = nullptr) {
+                  const Tensor& b_mg, bool want_b, int dtype, const Rows* rows = nullptr, const Tensor& w_out = Tensor()) {
     Grads out;
     // dW = dy^T x, over all rows or (whichever the device finds) over the gathered ones
     auto product = [&](void* to, bool fp32, Epi e, int64_t ldd) {
@@ -327,7 +334,7 @@ Grads param_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& w_
             gemm(dy, x, true, false, w32.data_ptr(), true, dtype, e);
             out.w = w32.to(w.scalar_type());
         } else {
-            out.w = at::empty({dy.cols, x.cols}, w.options());
+            out.w = w_out.defined() ? w_out : at::empty({dy.cols, x.cols}, w.options());
             product(out.w.data_ptr(), false, e, 0);
         }
     } else if (db.defined()) {
@@ -426,12 +433,15 @@ struct LinearNode : Node {
         }
         const Mat d = rows_of(dy), xm = rows_of(X);
         const bool want_dx = task_should_compute_output(0), want_w = task_should_compute_output(1);
+        Tensor dx, dw;
+        if (want_dx) dx = at::empty(X.sizes(), X.options());
         Rows rows;
-        if (!P.defined() && (want_dx || want_w)) rows = gather_rows(d, xm, want_dx, dt, X.options());
+        if (const int64_t room = P.defined() || !(want_dx || want_w) ? 0 : gather_room(d, xm)) {
+            if (want_w && !w_mg.defined()) dw = at::empty({d.cols, xm.cols}, W.options());   // (before the look's scratch)
+            rows = gather_rows(d, xm, room, want_dx, dt, X.options());
+        }
         const bool look = rows.ctl.defined();
-        Tensor dx;
         if (want_dx) {
-            dx = at::empty(X.sizes(), X.options());
             const Mat wm = mat(W);
             Epi e;
             if (look) {
@@ -447,7 +457,7 @@ struct LinearNode : Node {
             gemm(d, wm, false, false, dx.data_ptr(), false, dt, e);
         }
         const Grads gr = param_grads(d, xm, W, w_mg, want_w, bias, b_mg, bias.defined() && task_should_compute_output(2), dt,
-                                     look ? &rows : nullptr);
+                                     look ? &rows : nullptr, dw);
         notify({{&w_ref, &w_mg}, {&bias, &b_mg}});
         return {dx, gr.w, gr.b};
     }
@@ -1283,5 +1293,5 @@ PYBIND11_MODULE(_host, m) {
     RB_DEF(qkv_attention);
     RB_DEF(batch_norm_act);
     RB_DEF(conv1x1);
-    m.def("gather_room", &gather_room);
+    m.def("gather_room", py::overload_cast<int64_t, int64_t, int64_t, int64_t>(&gather_room));
 }

@@ -264,3 +264,48 @@ def test_wide_layer_backward_repeats_to_the_bit():
         got = torch.autograd.grad(RF.linear(x, w), (x, w), dy)
         first = got if first is None else first
         assert torch.equal(got[0], first[0]) and torch.equal(got[1], first[1])
+
+
+@pytest.mark.parametrize("flat", [True, False])
+def test_backward_without_memory_for_the_gathered_rows(flat):
+    """An allocator with room for the gradients alone: the products go over all rows, as under deterministic algorithms."""
+    from rannc_b200.ops import functional as RF
+
+    R, H, V = 4099, 776, 28680
+    torch.manual_seed(11)
+    x = torch.randn(R, H, device="cuda", dtype=torch.bfloat16).requires_grad_(True)
+    w = torch.randn(V, H, device="cuda", dtype=torch.bfloat16).requires_grad_(True)
+    dy = torch.randn(R, V, device="cuda", dtype=torch.bfloat16)
+    dy[500:] = 0
+    want = None
+    for short in (False, True):
+        if flat:
+            w.main_grad = torch.zeros(V, H, device="cuda")
+        x.grad = w.grad = None
+        y = RF.linear(x, w)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        total = torch.cuda.get_device_properties(0).total_memory
+        try:
+            if short:
+                reserved = torch.cuda.memory_reserved()
+                torch.cuda.set_per_process_memory_fraction(reserved / total)
+                kept = []
+                try:                                        # (what other tests left free in blocks of theirs)
+                    while True:
+                        kept.append(torch.empty(32 << 20, dtype=torch.uint8, device="cuda"))
+                except torch.OutOfMemoryError:
+                    pass
+                torch.cuda.set_per_process_memory_fraction((reserved + (96 << 20)) / total)
+                failed = torch.cuda.memory_stats()["num_ooms"]
+            else:
+                torch.use_deterministic_algorithms(True)
+            y.backward(dy)
+        finally:
+            torch.use_deterministic_algorithms(False)
+            torch.cuda.set_per_process_memory_fraction(1.0)
+        assert not short or torch.cuda.memory_stats()["num_ooms"] > failed
+        got = (x.grad, w.main_grad if flat else w.grad)
+        want = want or got
+        for a, b in zip(got, want):
+            assert torch.equal(a, b) or (flat and (a - b).abs().max() <= 1e-4 * b.abs().max())   # (fp32: last wave in parts)
