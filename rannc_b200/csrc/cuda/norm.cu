@@ -315,8 +315,9 @@ __global__ void __launch_bounds__(LN_THREADS, 2)
         // (here, behind the loads of this row and before the wait for the other warps: at the top of the loop 24.0 us, not 22)
         fetch(stage == 0 ? STAGES - 1 : stage - 1, row + (STAGES - 1) * step);
         const float2 s = group_sum<WPR>(make_float2(f2_sum(sx), f2_sum(sy)), sm, turn, warp, lane);
-        // o = rstd (d g - s1 - xh s2), with s1 and s2 the means of s.x and s.y
-        const uint64_t c1 = f2_both(-rstd * s.x * (1.f / H)), c2 = f2_both(-rstd * rstd * s.y * (1.f / H));
+        // o = rstd (d g - s1 - xh s2), with s1 and s2 the means of s.x and s.y.  (Not with rstd^2 taken out of the loop: it is
+        // out of fp32's range where rstd itself and every term are not.)
+        const uint64_t c1 = f2_both(-s.x * (1.f / H)), c2 = f2_both(-s.y * (1.f / H));
 #pragma unroll(NCHUNK <= 2 ? NCHUNK : 1)
         for (int c = 0; c < NCHUNK; ++c) {
             const int col = col0 + c * 256;
@@ -331,7 +332,7 @@ __global__ void __launch_bounds__(LN_THREADS, 2)
             get_gamma(c, g);
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                o[j] = f2_fma(f2_mul(d[j], g[j]), rstd2, f2_fma(f2_add(zz[j], minus_mean), c2, c1));
+                o[j] = f2_mul(rstd2, f2_fma(d[j], g[j], f2_fma(f2_mul(f2_add(zz[j], minus_mean), rstd2), c2, c1)));
             *reinterpret_cast<uint4*>(dz_out + base + col) = pack_pairs<T>(o);
             if (dx_out) {
                 if (thr) {

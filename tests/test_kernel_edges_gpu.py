@@ -894,3 +894,27 @@ def test_attention_backward_of_one_key_block(dtype, S, B, H):
         assert (got.double() - want).abs().max().item() <= bound
     torch.cuda.synchronize()
     assert _lib.read_error() == 0
+
+
+@pytest.mark.parametrize("H", [256, 768, 2048])
+@pytest.mark.parametrize("std,scale,eps", [(1.0, 1.0, 1e-5), (2.0 ** 58, 1e-4, 1e-5), (2.0 ** -58, 2.0 ** 20, 0.0)])
+def test_layer_norm_backward_of_rows_far_from_one(H, std, scale, eps):
+    """Rows whose reciprocal deviation is in fp32's range and its square, times a gradient, is not."""
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(31)
+    z = (torch.randn(37, H, device="cuda") * std).bfloat16()
+    dy = (torch.randn(37, H, device="cuda") * scale).bfloat16()
+    g = (torch.rand(H, device="cuda") + 0.5).bfloat16()
+    b = torch.zeros_like(g)
+    y, _, mean, rstd = K.ln_fwd(z, None, g, b, eps)
+    dz, _, dgamma, dbeta = K.ln_bwd(dy, z, g, mean, rstd)
+    zd, w = z.double(), dy.double() * g.double()
+    r = 1.0 / (zd.var(1, unbiased=False, keepdim=True) + eps).sqrt()
+    xh = (zd - zd.mean(1, keepdim=True)) * r
+    want = r * (w - w.mean(1, keepdim=True) - xh * (w * xh).mean(1, keepdim=True))
+    # one rounding to 16 bits, and fp32 sums of H terms
+    bound = 2.0 ** -8 * want.abs() + 1e-5 * (r * w.abs().amax(1, keepdim=True))
+    assert ((dz.double() - want).abs() <= bound).all()
+    _near(dgamma, (dy.double() * xh).sum(0), torch.bfloat16, 0, 1e-4)
+    _near(dbeta, dy.double().sum(0), torch.bfloat16, 0, 1e-4)
