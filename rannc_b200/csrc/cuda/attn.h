@@ -21,7 +21,7 @@ typedef struct RbAttnArgs {
     void* dK;
     void* dV;
     float* delta;     // [B, H, S] scratch: rowsum(dO * O)
-    float* dq_accum;  // [B, S, H, D] fp32 scratch, zeroed by the callee
+    float* dq_accum;  // [B, S, H, D] fp32 scratch, zeroed by the callee; not used (null will do) where rb_attn_bwd_adds is 0
     int64_t q_sb, q_ss, q_sh;
     int64_t k_sb, k_ss, k_sh;
     int64_t v_sb, v_ss, v_sh;
@@ -40,6 +40,8 @@ typedef struct RbAttnArgs {
 
 int rb_attn_fwd(const RbAttnArgs* args, void* stream);
 int rb_attn_bwd(const RbAttnArgs* args, void* stream);
+// 1: the backward adds dQ up in dq_accum, in three kernels; 0: dQ leaves as it is made, in two
+int rb_attn_bwd_adds(const RbAttnArgs* args);
 
 #ifdef __cplusplus
 }

@@ -698,15 +698,22 @@ static int launch_bwd(const RbAttnArgs& a, cudaStream_t st) {
     const long long rows = static_cast<long long>(a.B) * a.H * a.S;
     if (rows >= (1LL << 31) - 64) return -2;
     CUtensorMap tdq, tdk, tdv;
-    // A sequence of one key block has nothing to add up in dQ: without the clearing of the scratch, the additions and the
-    // conversion 64 x 128 x 16 heads take 38.4 us in place of 50.8, 32 x 64 x 16 18.6 (23.4), 8 x 128 x 16 11.2 (14.0),
-    // 1 x 32 x 4 7.7 (9.7).  A kernel of its own: asked in the drain loop, it cost the longer sequences 1 %.  (Strides of dQ
-    // that the copy engine does not take go the way of those.)
-    const bool dq16 =
-        a.S <= BKEYS && make_tmap_4d(&tdq, a.dQ, a.dtype, D, S, H, B, a.dq_ss * 2, a.dq_sh * 2, a.dq_sb * 2, 64, 128) == 0;
+    const bool dq16 = !rb_attn_bwd_adds(&a);
+    if (!dq16 && !a.dq_accum) return -2;
+    // (a dimension of one has any stride; the copy engine wants one it can take)
+    auto stride = [](uint64_t n, int64_t s) { return static_cast<uint64_t>(n > 1 ? s * 2 : 128); };
+    if (dq16)
+        rc = make_tmap_4d(&tdq, a.dQ, a.dtype, D, S, H, B, stride(S, a.dq_ss), stride(H, a.dq_sh), stride(B, a.dq_sb), 64, 128);
+    else
+        rc = make_tmap_4d_f32(&tdq, a.dq_accum, 64, S, H, B, H * 64 * 4, 64 * 4, S * H * 64 * 4, 32, 128);
+    if (rc) return rc;
+    if ((rc = make_tmap_4d(&tdk, a.dK, a.dtype, D, S, H, B, stride(S, a.dk_ss), stride(H, a.dk_sh), stride(B, a.dk_sb), 64, 128)))
+        return rc;
+    if ((rc = make_tmap_4d(&tdv, a.dV, a.dtype, D, S, H, B, stride(S, a.dv_ss), stride(H, a.dv_sh), stride(B, a.dv_sb), 64, 128)))
+        return rc;
     if (launch_after(attn_delta_kernel<T>, static_cast<unsigned>((rows + 63) / 64), 256, 0, st, static_cast<const T*>(a.O),
-                     static_cast<const T*>(a.dO), a.delta, dq16 ? nullptr : a.dq_accum, a.B, a.H, a.S, a.o_sb, a.o_ss, a.o_sh, a.do_sb,
-                     a.do_ss, a.do_sh) != cudaSuccess)
+                     static_cast<const T*>(a.dO), a.delta, dq16 ? nullptr : a.dq_accum, a.B, a.H, a.S, a.o_sb, a.o_ss, a.o_sh,
+                     a.do_sb, a.do_ss, a.do_sh) != cudaSuccess)
         return -1;
     AttnBwdParams p;
     p.B = a.B; p.H = a.H; p.S = a.S;
@@ -740,9 +747,6 @@ static int launch_bwd(const RbAttnArgs& a, cudaStream_t st) {
     auto inverse = [](unsigned d) { return d == 1 ? 0u : static_cast<uint32_t>(((1ull << 32) + d - 1) / d); };
     p.inv_nq = inverse(nq);
     p.inv_h = inverse(nh);
-    if ((rc = make_tmap_4d(&tdk, a.dK, a.dtype, D, S, H, B, a.dk_ss * 2, a.dk_sh * 2, a.dk_sb * 2, 64, 128))) return rc;
-    if ((rc = make_tmap_4d(&tdv, a.dV, a.dtype, D, S, H, B, a.dv_ss * 2, a.dv_sh * 2, a.dv_sb * 2, 64, 128))) return rc;
-    if (!dq16 && (rc = make_tmap_4d_f32(&tdq, a.dq_accum, 64, S, H, B, H * 64 * 4, 64 * 4, S * H * 64 * 4, 32, 128))) return rc;
     if (launch_after(kern, grid, BWD_THREADS, BWD_SMEM, st, tq, tk, tv, tdo, tdq, tdk, tdv, p) != cudaSuccess) return -1;
     if (dq16) return 0;
     const long long groups = rows * 8;
@@ -754,6 +758,15 @@ static int launch_bwd(const RbAttnArgs& a, cudaStream_t st) {
 }
 
 }  // namespace rb
+
+// A sequence of one key block has nothing to add up in dQ: without the clearing of the scratch, the additions and the
+// conversion 64 x 128 x 16 heads take 38.4 us in place of 50.8, 32 x 64 x 16 18.6 (23.4), 8 x 128 x 16 11.2 (14.0),
+// 1 x 32 x 4 7.7 (9.7).  A kernel of its own: asked in the drain loop, it cost the longer sequences 1 %.  (Strides of dQ
+// that the copy engine does not take go the way of those.)
+extern "C" int rb_attn_bwd_adds(const RbAttnArgs* a) {
+    auto takes = [](int n, int64_t s) { return n <= 1 || (s > 0 && s < (int64_t{1} << 39)); };
+    return a->S > rb::BKEYS || !takes(a->S, a->dq_ss) || !takes(a->H, a->dq_sh) || !takes(a->B, a->dq_sb);
+}
 
 extern "C" int rb_attn_bwd(const RbAttnArgs* a, void* stream) {
     if (a->D != 64) return -2;

@@ -58,6 +58,7 @@ struct Api {
                     long long, float, int, void*);
     int (*attn_fwd)(const RbAttnArgs*, void*);
     int (*attn_bwd)(const RbAttnArgs*, void*);
+    int (*attn_bwd_adds)(const RbAttnArgs*);
     int (*bn_fwd)(const void*, const void*, const float*, const float*, void*, float*, float*, float*, float*, float*,
                   long long, int, float, float, int, int, void*);
     int (*bn_bwd)(const void*, const void*, const void*, const float*, const float*, const float*, float*, float*, float*,
@@ -859,7 +860,7 @@ struct QkvNode : Node {
         const int dt = dt_code(X);
         const int64_t Ho = H * 64;
         Tensor dqkv = at::empty(Q.sizes(), Q.options());
-        Tensor delta = f32({B, H, S}, Q), dq_acc = f32({B, S, H, 64}, Q);
+        Tensor delta = f32({B, H, S}, Q), dq_acc;
         RbAttnArgs a;
         attn_args(a, Q, O, L, kb, B, S, H, scale, p, seed, offset);
         a.dO = dO.data_ptr();
@@ -874,8 +875,10 @@ struct QkvNode : Node {
         a.dq_ss = a.dk_ss = a.dv_ss = 3 * Ho;
         a.dq_sh = a.dk_sh = a.dv_sh = 64;
         a.delta = mptr<float>(delta);
+        const bool adds = api.attn_bwd_adds(&a);
+        if (adds) dq_acc = f32({B, S, H, 64}, Q);
         a.dq_accum = mptr<float>(dq_acc);
-        check(api.attn_bwd(&a, cur_stream()), "rb_attn_bwd", 3);
+        check(api.attn_bwd(&a, cur_stream()), "rb_attn_bwd", adds ? 3 : 2);
         Mat dm;
         dm.keep = dqkv;
         dm.p = d;
@@ -1238,6 +1241,7 @@ void init(const std::unordered_map<std::string, uintptr_t>& fns, py::object erro
     set(api.xent_bwd, "rb_xent_bwd");
     set(api.attn_fwd, "rb_attn_fwd");
     set(api.attn_bwd, "rb_attn_bwd");
+    set(api.attn_bwd_adds, "rb_attn_bwd_adds");
     set(api.bn_fwd, "rb_bn_fwd");
     set(api.bn_bwd, "rb_bn_bwd");
     set(api.bn_part_floats, "rb_bn_part_floats");

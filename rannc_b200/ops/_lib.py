@@ -17,10 +17,12 @@ _HERE = Path(__file__).resolve().parent.parent
 _lock = threading.Lock()
 _lib = None
 
-# device kernels launched per C entry point (the optimizer / element-wise entries launch one)
-_KERNELS_PER_CALL = {"rb_bn_fwd": 3, "rb_bn_bwd": 3, "rb_ln_bwd": 2, "rb_xent_fwd": 2, "rb_attn_bwd": 3, "rb_rows_plan": 2,
-                     "rb_bn_part_floats": 0, "rb_read_error": 0, "rb_ln_supported": 0, "rb_ln_bwd_grid": 0, "rb_gemm_splits": 0,
-                     "rb_gemm_last_wave": 0, "rb_gemm_pairs": 0, "rb_error_peek_async": 0}
+# device kernels launched per C entry point (the optimizer / element-wise entries launch one; rb_attn_bwd two, and a third
+# where it adds dQ up, which its caller counts)
+_KERNELS_PER_CALL = {"rb_bn_fwd": 3, "rb_bn_bwd": 3, "rb_ln_bwd": 2, "rb_xent_fwd": 2, "rb_attn_bwd": 2, "rb_rows_plan": 2,
+                     "rb_attn_bwd_adds": 0, "rb_bn_part_floats": 0, "rb_read_error": 0, "rb_ln_supported": 0,
+                     "rb_ln_bwd_grid": 0, "rb_gemm_splits": 0, "rb_gemm_last_wave": 0, "rb_gemm_pairs": 0,
+                     "rb_error_peek_async": 0}
 _launches = 0
 
 
@@ -46,6 +48,12 @@ class _Counting:
             fn.raw = raw
             cache[name] = fn
         return fn
+
+
+def count_launches(n: int):
+    """Kernels of a call beyond those that are counted for its entry point."""
+    global _launches
+    _launches += n
 
 
 def launch_count() -> int:
@@ -88,7 +96,7 @@ def lib() -> ctypes.CDLL:
 _host = None
 _HOST_ENTRIES = ("rb_gemm", "rb_gemm_splits", "rb_gemm_pairs", "rb_unstack3", "rb_gelu", "rb_colsum", "rb_ln_fwd", "rb_ln_bwd",
                  "rb_ln_bwd16", "rb_ln_bwd_grid", "rb_embed_fwd", "rb_embed_bwd", "rb_xent_fwd", "rb_xent_bwd",
-                 "rb_attn_fwd", "rb_attn_bwd", "rb_bn_fwd", "rb_bn_bwd", "rb_bn_part_floats", "rb_rows_plan", "rb_rows_gather",
+                 "rb_attn_fwd", "rb_attn_bwd", "rb_attn_bwd_adds", "rb_bn_fwd", "rb_bn_bwd", "rb_bn_part_floats", "rb_rows_plan", "rb_rows_gather",
                  "rb_rows_scatter_parts")
 
 

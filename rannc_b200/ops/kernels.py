@@ -239,12 +239,11 @@ def attn_bwd(q, k, v, o, lse, do, key_bias=None, scale=None, p_drop=0.0, seed=0,
     dk = torch.empty(B, S, H, D, dtype=q.dtype, device=q.device) if dk is None else dk
     dv = torch.empty(B, S, H, D, dtype=q.dtype, device=q.device) if dv is None else dv
     delta = torch.empty(B, H, S, dtype=torch.float32, device=q.device)
-    dq_acc = torch.empty(B, S, H, D, dtype=torch.float32, device=q.device)
     a = _AttnArgs()
     a.Q, a.K, a.V, a.O, a.lse = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr()
     a.key_bias = None if key_bias is None else key_bias.data_ptr()
     a.dO, a.dQ, a.dK, a.dV = do.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
-    a.delta, a.dq_accum = delta.data_ptr(), dq_acc.data_ptr()
+    a.delta = delta.data_ptr()
     a.q_sb, a.q_ss, a.q_sh = _bshd_strides(q)
     a.k_sb, a.k_ss, a.k_sh = _bshd_strides(k)
     a.v_sb, a.v_ss, a.v_sh = _bshd_strides(v)
@@ -255,6 +254,10 @@ def attn_bwd(q, k, v, o, lse, do, key_bias=None, scale=None, p_drop=0.0, seed=0,
     a.dv_sb, a.dv_ss, a.dv_sh = _bshd_strides(dv)
     a.B, a.H, a.S, a.D, a.dtype = B, H, S, D, dt_code(q)
     a.scale, a.p_drop, a.seed, a.offset = scale, float(p_drop), int(seed), int(offset)
+    if _lib.lib().rb_attn_bwd_adds(ctypes.byref(a)):
+        dq_acc = torch.empty(B, S, H, D, dtype=torch.float32, device=q.device)
+        a.dq_accum = dq_acc.data_ptr()
+        _lib.count_launches(1)
     _lib.check(_lib.lib().rb_attn_bwd(ctypes.byref(a), _lib.stream_ptr()), "rb_attn_bwd")
     return dq, dk, dv
 

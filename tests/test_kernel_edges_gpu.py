@@ -918,3 +918,43 @@ def test_layer_norm_backward_of_rows_far_from_one(H, std, scale, eps):
     assert ((dz.double() - want).abs() <= bound).all()
     _near(dgamma, (dy.double() * xh).sum(0), torch.bfloat16, 0, 1e-4)
     _near(dbeta, dy.double().sum(0), torch.bfloat16, 0, 1e-4)
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_launches_are_counted_as_they_are(native):
+    """Batch norm and attention backward, of one key block and of two, through the operators' host side and past it: what
+    the library says it launched, and the kernels of its that the device ran."""
+    from torch.profiler import ProfilerActivity, profile
+
+    from rannc_b200.ops import _lib
+    from rannc_b200.ops import functional as RF
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(32)
+    img = torch.randn(2, 64, 8, 8, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
+    rows = torch.randn(128, 64, device="cuda").bfloat16()
+    g = torch.ones(64, device="cuda", requires_grad=True)
+    ws = [torch.randn(128, 128, device="cuda").bfloat16().requires_grad_(True) for _ in range(3)]
+    qkv = [torch.randn(2, s, 2, 64, device="cuda").bfloat16() for s in (100, 200)]
+
+    def work():
+        if native:
+            RF.batch_norm_act(img.clone().requires_grad_(True), g, torch.zeros_like(g), None, None).sum().backward()
+            for s in (100, 200):
+                x = torch.randn(2, s, 128, device="cuda").bfloat16()
+                RF.qkv_attention(x, ws[0], None, ws[1], None, ws[2], None, num_heads=2).sum().backward()
+        else:
+            y, mean, rstd = K.bn_fwd(rows, None, g.detach(), g.detach(), None, None, 1e-5, 0.1, True)
+            K.bn_bwd(rows, rows, y, mean, rstd, g.detach(), True, False)
+            for t in qkv:
+                o, lse = K.attn_fwd(t, t, t)
+                K.attn_bwd(t, t, t, o, lse, t)
+
+    work()
+    torch.cuda.synchronize()
+    before = _lib.launch_count()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        work()
+        torch.cuda.synchronize()
+    ran = sum(e.count for e in p.key_averages() if "rb::" in e.key)
+    assert ran > 0 and _lib.launch_count() - before == ran
