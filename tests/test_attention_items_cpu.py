@@ -1,16 +1,47 @@
 """The roles of the attention backward kernel over several items of one CTA (blocks of 128 keys, one after the other), at any
-speed relative to each other.  Steps of a block are read from the source; what lies between two items stands here."""
+speed relative to each other.  The programs stand here; the operations they are made of are compared with the source."""
 import pytest
 
-from tests.test_kernel_contracts_cpu import STAGES, _bwd_roles
+from tests.test_kernel_contracts_cpu import STAGES, TOKEN, _closing, _kernels
+
+# A role's barrier operations, products and loads in the order of the source, over a block and between items
+SOURCE = {
+    "load": "wait kv_full, wait qd_full, wait s_free, C_ ST, C_ DPT, commit s_full, wait qd_free, load_qd i, wait s_full, "
+            "wait k_free, wait qd_free",
+    "grad": "wait dkv_taken, wait qd_full, wait pds_ready, C_ DK, wait dq_taken, C_ DQ, commit ds_done, C_ DV, commit qd_free, "
+            "commit p_done, commit k_free",
+    "drain": "arrive stats_full, wait ds_done, arrive dq_taken, put_stats i, arrive dq_free, wait dq_free, arrive dq_ready, "
+             "wait dq_ready, wait p_done, arrive dkv_taken, arrive dkv_free, wait dkv_free, arrive dkv_ready, wait dkv_ready",
+    "math": "wait stats_full, wait s_full, arrive s_free, wait ds_done, wait p_done, arrive pds_ready",
+}
+# the drain's first warp issues the copies; the others are the second actor, and barriers count both
+BOTH = ("dq_taken", "dkv_taken", "stats_full", "dq_ready", "dkv_ready")
+
+
+def test_operations_of_the_roles_are_those_of_the_source():
+    body = _kernels("attn_bwd.cu")["attn_bwd_kernel"][1]
+    start = body.index("if (warp == LOAD_WARP) {", body.index("grid_wait()"))
+    for role, want in SOURCE.items():
+        open_ = body.index("{", start)
+        section = body[open_:_closing(body, open_)]
+        start = open_ + len(section)
+        assert ", ".join(" ".join(x for x in m.groups() if x) for m in TOKEN.finditer(section)) == want, role
+        if role == "drain":
+            # every write to the staging memory behind the copies that read it, every copy behind the writes
+            assert section.count("tma_store_wait_read<0>()") == 3
+            for bar in ("dq", "dkv"):
+                at = [section.index(f"mbar_arrive({bar}_free)"), section.index(f"mbar_wait_warp({bar}_free"),
+                      section.index(f"mbar_arrive({bar}_ready)"), section.index(f"mbar_wait_warp({bar}_ready")]
+                assert at == sorted(at)
+                assert section.rindex("tma_store_wait_read<0>()", 0, at[0]) > at[0] - 200
+                assert "fence_proxy_async()" in section[at[1]:at[2]]
 
 
 def _programs(nq, items):
-    """{actor: [step]}; products and the commits behind them are steps of a queue that the tensor core works off.  `data`:
-    what a place holds, (name, place) -> block or item."""
+    """{actor: [step]}; products and the commits behind them are steps of a queue that the tensor core works off, the copies
+    out of the staging memory of one that the copy engine does.  A place holds a block or an item."""
     total = nq * items
-    roles = _bwd_roles()
-    P = {a: [] for a in ("load", "grad", "drain", "math", "load queue", "grad queue")}
+    P = {a: [] for a in ("load", "grad", "drain", "drain 2", "math", "load queue", "grad queue", "drain queue")}
 
     def wait(role, name, index, phase):
         P[role].append(("wait", (name, index), phase))
@@ -33,7 +64,6 @@ def _programs(nq, items):
         wait("load", "kv_full", 0, k)
         for i in range(nq):
             c = k * nq + i
-            assert [n for w, n in roles["load"] if w != "C_"] == ["qd_full", "s_free", "s_full", "qd_free", "i"]
             wait("load", "qd_full", c % STAGES, c // STAGES)
             if c > 0:
                 wait("load", "s_free", 0, c - 1)
@@ -70,17 +100,40 @@ def _programs(nq, items):
         if k + 2 < items:
             queue("grad", ("arrive", ("k_free", k & 1)))
     # ---- drain
+    def staged(bar, c, places, what):
+        """Both halves of the drain write `what` to a place each, and the first warp has the copy engine read them."""
+        if bar:
+            P["drain"].append(("drained", len(P["drain queue"])))
+            arrive("drain", bar + "_free")
+        for h, role in enumerate(("drain", "drain 2")):
+            if bar:
+                wait(role, bar + "_free", 0, c)
+            P[role].append(("put", None, places[h], what))
+            arrive(role, ("dkv" if what[0] == "dkv" else "dq") + "_ready")
+        wait("drain", ("dkv" if what[0] == "dkv" else "dq") + "_ready", 0, what[1])
+        queue("drain", ("read", [(places[0], what), (places[1], what)]))
+
+    def both(name, index=0):
+        arrive("drain", name, index)
+        arrive("drain 2", name, index)
+
     for c in range(min(2, total)):
-        arrive("drain", "stats_full", c & 1)
+        both("stats_full", c & 1)
     for k in range(items):
         for i in range(nq):
             c = k * nq + i
-            wait("drain", "ds_done", 0, c)
-            arrive("drain", "dq_taken")
+            for role in ("drain", "drain 2"):
+                wait(role, "ds_done", 0, c)
+            both("dq_taken")
             if c + 2 < total:
-                arrive("drain", "stats_full", c & 1)
-        wait("drain", "p_done", 0, (k + 1) * nq - 1)
-        arrive("drain", "dkv_taken")
+                both("stats_full", c & 1)
+            staged("dq", c, (("T", 0), ("T", 1)), ("dq", c))
+        for role in ("drain", "drain 2"):
+            wait(role, "p_done", 0, (k + 1) * nq - 1)
+        both("dkv_taken")
+        # (the last item's go where nothing is loaded any more: each half of the drain writes to both, here to one)
+        last = k + 1 == items
+        staged(None if last else "dkv", k, (("K", (k + 1) & 1), ("V", 0)) if last else (("T", 0), ("T", 1)), ("dkv", k))
     # ---- math
     for c in range(total):
         wait("math", "stats_full", c & 1, c >> 1)
@@ -101,7 +154,7 @@ def test_roles_over_several_items_at_any_speed(nq, items):
     progs = _programs(nq, items)
     actors = list(progs)
     arrived = {a: [{}] for a in actors}
-    held = {a: [{}] for a in ("load", "math")}
+    held = {a: [{}] for a in ("load", "math", "drain", "drain 2")}
     for a in actors:
         for step in progs[a]:
             count = dict(arrived[a][-1])
@@ -114,7 +167,14 @@ def test_roles_over_several_items_at_any_speed(nq, items):
             arrived[a].append(count)
 
     def ended(bar, at):
+        if bar[0] in BOTH:
+            n = [arrived[a][at[actors.index(a)]].get(bar, 0) for a in ("drain", "drain 2")]
+            assert abs(n[0] - n[1]) <= 1, f"{bar} counts one actor twice"
+            return min(n)
         return sum(arrived[a][pc].get(bar, 0) for a, pc in zip(actors, at))
+
+    def holds(owner, place, at):
+        return held[owner][at[actors.index(owner)]].get(place)
 
     seen, todo = set(), [(0,) * len(actors)]
     while todo:
@@ -132,13 +192,19 @@ def test_roles_over_several_items_at_any_speed(nq, items):
                 if (n - step[2]) % 2 == 0:
                     continue
                 assert n == step[2] + 1, f"{a} passes {step} with {n} phases ended"
+            elif step[0] == "drained":
+                if at[actors.index("drain queue")] < step[1]:
+                    continue   # a copy still reads
             elif a.endswith("queue"):
                 if at[actors.index(a.split()[0])] < step[-1]:
                     continue   # not issued yet
                 if step[0] == "read":
-                    for place, what in step[1]:
-                        owner = "math" if place[0] in ("dS", "P") else "load"
-                        assert held[owner][at[actors.index(owner)]].get(place) == what, f"{a}: {place} holds another's"
+                    for h, (place, what) in enumerate(step[1]):
+                        drains = ("drain", "drain 2")
+                        owner = drains[h] if a == "drain queue" else "math" if place[0] in ("dS", "P") else "load"
+                        assert holds(owner, place, at) == what, f"{a}: {place} holds another's"
+                        # (K and V have two writers: what the products read has not been written over by the drain)
+                        assert owner != "load" or all(holds(d, place, at) is None for d in drains), f"{a}: {place} is gone"
             moves += 1
             todo.append(at[:k] + (at[k] + 1,) + at[k + 1:])
         assert moves or all(pc == len(progs[a]) for a, pc in zip(actors, at)), \

@@ -92,9 +92,13 @@ def test_wide_layer_backward(dtype, share, flat):
     on = torch.rand(R, device="cuda") < share
     on[-1] = share > 0
     dy[~on] = 0
-    RF.linear(x, w, b).backward(dy)
+    y = RF.linear(x, w, b)
+    before = _lib.launch_count()
+    y.backward(dy)
     torch.cuda.synchronize()
     assert _lib.read_error() == 0
+    # the look at the rows (three kernels), each product in two forms, and the one that puts rows back
+    assert _lib.launch_count() - before == 8
     gw, gb = (w.main_grad - 2.0, b.main_grad + 1.0) if flat else (w.grad, b.grad)
     u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     n = int(on.sum())
@@ -110,6 +114,7 @@ def test_wide_layer_backward(dtype, share, flat):
 def test_infinities_and_nan_reach_the_gradients_of_rows_of_zeros():
     """0 * inf is NaN: a weight that is not finite shows in its column of every row's gradient, an input that is not finite in
     its column of the weight's, as in the product over all rows."""
+    from rannc_b200.ops import _lib
     from rannc_b200.ops import functional as RF
 
     R, H, V = 4096, 768, 30528
@@ -122,11 +127,13 @@ def test_infinities_and_nan_reach_the_gradients_of_rows_of_zeros():
     for all_rows in (False, True):
         xg, wg = x.clone().requires_grad_(True), w.clone().requires_grad_(True)
         y = RF.linear(xg, wg)
+        before = _lib.launch_count()
         torch.use_deterministic_algorithms(all_rows)     # (its products go over all rows)
         try:
             y.backward(dy)
         finally:
             torch.use_deterministic_algorithms(False)
+        assert _lib.launch_count() - before == (2 if all_rows else 8)
         got[all_rows] = (xg.grad, wg.grad)
     for a, b in zip(got[False], got[True]):
         assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
@@ -251,6 +258,7 @@ def test_input_gradient_over_gathered_rows(dtype, V, H, room, count, rows_out):
 
 
 def test_wide_layer_backward_repeats_to_the_bit():
+    from rannc_b200.ops import _lib
     from rannc_b200.ops import functional as RF
 
     R, H, V = 4099, 776, 28680
@@ -261,7 +269,10 @@ def test_wide_layer_backward_repeats_to_the_bit():
     dy[torch.rand(R, device="cuda") >= 0.15] = 0
     first = None
     for _ in range(30):
-        got = torch.autograd.grad(RF.linear(x, w), (x, w), dy)
+        y = RF.linear(x, w)
+        before = _lib.launch_count()
+        got = torch.autograd.grad(y, (x, w), dy)
+        assert _lib.launch_count() - before == 8        # (over the gathered rows)
         first = got if first is None else first
         assert torch.equal(got[0], first[0]) and torch.equal(got[1], first[1])
 
