@@ -1476,7 +1476,8 @@ extern "C" int rb_gemm(const RbGemmArgs* a, void* stream_) {
 
     // The staged epilogue wants outputs the copy engine can address: plain rows in this GPU's memory, 16-byte
     // aligned bases and row strides.  Its staging blocks of an auxiliary matrix are 16-bit ones, so an fp32 output
-    // with one, or an output that both reads and writes an auxiliary matrix, stays on the direct path, as do mapped rows (padded image grids) and peers' buffers (reduce-scatter).
+    // with one, or an output that both reads and writes an auxiliary matrix, stays on the direct path, as do mapped
+    // rows (padded image grids) and peers' buffers (reduce-scatter).
     CUtensorMap tmD = tmA, tmAux = tmA;
     const bool fp32_out = a->out_dtype == 1;
     const int64_t out_es = fp32_out ? 4 : 2;

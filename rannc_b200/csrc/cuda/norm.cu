@@ -114,8 +114,8 @@ __device__ __forceinline__ float2 group_sum(float2 v, float2 (*sm)[LN_WARPS], in
 // in flight would be those of the resident warps' current rows.  Each thread fetches its own 16-byte pieces of the next rows
 // into its own places of a shared-memory ring (no barrier is needed to read them back), three deep or more.
 // Time, and at the copy bandwidth (us, bf16; backward with the sums' reduction): 16384 x 1024 with dropout and residual forward
-// 28.7 -> 27.1 (20.5), backward 33.6 -> 30.5 (20.5); without 15.1 -> 12.8 (10.3) and 23.3 -> 19.4 (15.4); 8192 x 2048 24.2
-// -> 20.8 and 25.4 -> 24.5; 4096 x 4096 25.4 -> 24.8 and 33.3 -> 29.8; before that, of one row at a time, 32.3 and 34.8 at
+// 28.7 -> 27.2 (20.5), backward 33.5 -> 31.3 (20.5); without 15.2 -> 12.9 (10.3) and 23.6 -> 19.9 (15.4); 8192 x 2048 24.5
+// -> 21.1 and 25.2 -> 24.7; 4096 x 4096 25.4 -> 24.8 and 33.4 -> 30.0; before that, of one row at a time, 32.3 and 34.8 at
 // 16384 x 1024 with dropout.
 template <int NCHUNK>
 struct LnRing {

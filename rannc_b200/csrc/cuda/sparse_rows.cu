@@ -60,8 +60,10 @@ __global__ void __launch_bounds__(256)
     if (lane == 0) live[row] = found;
 }
 
-// One block numbers the rows that count: each thread takes a run of rows, sixteen flags at a time.
-__global__ void __launch_bounds__(1024) rows_plan_kernel(const uint8_t* live, int rows, int room, int32_t* idx, int32_t* pos, int32_t* ctl) {
+// One block numbers the rows that count: each thread takes a run of rows, counts its flags and, behind the sums of all, goes
+// through them once more.
+__global__ void __launch_bounds__(1024)
+    rows_plan_kernel(const uint8_t* live, int rows, int room, int32_t* idx, int32_t* pos, int32_t* ctl) {
     grid_trigger();
     grid_wait();
     __shared__ int sums[32];
