@@ -254,7 +254,8 @@ int64_t gather_room(int64_t rows, int64_t cols, int64_t inputs, int64_t pairs) {
     return std::min<int64_t>(rows / 4 * 3, (int64_t{1} << 30) / cols) / 64 * 64;   // (2 GiB at most)
 }
 int64_t gather_room(const Mat& dy, const Mat& x) {
-    return at::globalContext().deterministicAlgorithms() ? 0 : gather_room(dy.rows, dy.cols, x.cols, api.gemm_pairs());
+    if (dy.cols < 4 * x.cols || at::globalContext().deterministicAlgorithms()) return 0;   // (most layers, before any call)
+    return gather_room(dy.rows, dy.cols, x.cols, api.gemm_pairs());
 }
 // Scratch: three quarters of dy and of x, and 77 MB or three quarters of x in fp32, whatever the number of rows that count
 // (the host does not know it): 470 MB for 8192 x 1024 x 30528.  Where there is no memory for it, `ctl` stays empty.
