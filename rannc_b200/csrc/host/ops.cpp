@@ -243,19 +243,21 @@ struct Rows {
 // three quarters count: the look is 3 to 8 % of the backward there.  Both products use the kernel of CTA pairs whichever
 // form runs, so an input gradient of fewer tiles than 0.64 of the pairs stays out (2048 x 1024 x 30528, where all rows
 // count: 235 -> 281; 1024 x 1024 x 30528 gains at 15 %, 181 -> 132, and loses at 100 %, 189 -> 238).
+// Where one of the two products is not wanted the other has to be as long as both (4249 x 736 x 30336, 80 % of the rows, the
+// weight's gradient alone: 158 -> 186 us).
 // `pairs`: of SMs that work on 256 x 256 tiles at once (rb_gemm_pairs).  Returns how many rows there is room for, in steps
 // of 64 (few rows leave none: 0, as where the look is not worth it).
-int64_t gather_room(int64_t rows, int64_t cols, int64_t inputs, int64_t pairs) {
+int64_t gather_room(int64_t rows, int64_t cols, int64_t inputs, int64_t pairs, int64_t products) {
     auto tiles = [](int64_t m, int64_t n) { return (m + 255) / 256 * ((n + 255) / 256); };
     if (pairs <= 0 || cols < 4 * inputs || cols % 8 || inputs % 8 || cols > (1 << 22) || rows >= (1 << 30) ||
         tiles(cols, inputs) < pairs || 25 * tiles(rows, inputs) < 16 * pairs ||
-        static_cast<double>(rows) * cols * inputs < 9e10)
+        static_cast<double>(products) * rows * cols * inputs < 1.8e11)
         return 0;
     return std::min<int64_t>(rows / 4 * 3, (int64_t{1} << 30) / cols) / 64 * 64;   // (2 GiB at most)
 }
-int64_t gather_room(const Mat& dy, const Mat& x) {
+int64_t gather_room(const Mat& dy, const Mat& x, int64_t products) {
     if (dy.cols < 4 * x.cols || at::globalContext().deterministicAlgorithms()) return 0;   // (most layers, before any call)
-    return gather_room(dy.rows, dy.cols, x.cols, api.gemm_pairs());
+    return gather_room(dy.rows, dy.cols, x.cols, api.gemm_pairs(), products);
 }
 // Scratch: three quarters of dy and of x, and 77 MB or three quarters of x in fp32, whatever the number of rows that count
 // (the host does not know it): 470 MB for 8192 x 1024 x 30528.  Where there is no memory for it, `ctl` stays empty.
@@ -438,7 +440,7 @@ struct LinearNode : Node {
         Tensor dx, dw;
         if (want_dx) dx = at::empty(X.sizes(), X.options());
         Rows rows;
-        if (const int64_t room = P.defined() || !(want_dx || want_w) ? 0 : gather_room(d, xm)) {
+        if (const int64_t room = P.defined() ? 0 : gather_room(d, xm, want_dx + want_w)) {
             if (want_w && !w_mg.defined()) dw = at::empty({d.cols, xm.cols}, W.options());   // (before the look's scratch)
             rows = gather_rows(d, xm, room, want_dx, dt, X.options());
         }
@@ -1299,5 +1301,5 @@ PYBIND11_MODULE(_host, m) {
     RB_DEF(qkv_attention);
     RB_DEF(batch_norm_act);
     RB_DEF(conv1x1);
-    m.def("gather_room", py::overload_cast<int64_t, int64_t, int64_t, int64_t>(&gather_room));
+    m.def("gather_room", py::overload_cast<int64_t, int64_t, int64_t, int64_t, int64_t>(&gather_room));
 }

@@ -62,4 +62,8 @@ def test_room_for_gathered_rows(rows, cols, inputs, pairs, room):
 
     from rannc_b200 import _host
 
-    assert _host.gather_room(rows, cols, inputs, pairs) == room
+    assert _host.gather_room(rows, cols, inputs, pairs, 2) == room
+    # one of the two products alone has to be as long as both; none is not worth a look
+    alone = rows * cols * inputs >= 1.8e11
+    assert _host.gather_room(rows, cols, inputs, pairs, 1) == (room if alone else 0)
+    assert _host.gather_room(rows, cols, inputs, pairs, 0) == 0
