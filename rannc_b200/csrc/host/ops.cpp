@@ -614,7 +614,8 @@ struct LnNode : Node {
         auto leaf = [&](size_t i) {
             return dynamic_cast<torch::autograd::AccumulateGrad*>(next_edge(i).function.get()) != nullptr;
         };
-        const bool both = task_should_compute_output(0) && task_should_compute_output(1);
+        // (not where both are the same one, whose gradients the engine adds up)
+        const bool both = task_should_compute_output(0) && task_should_compute_output(1) && !(next_edge(0) == next_edge(1));
         if (p > 0 || (both && (leaf(0) || leaf(1)))) dx = at::empty(Z.sizes(), Z.options());
         Tensor partial = f32({static_cast<int64_t>(api.ln_bwd_grid(rows)) * 2 * H}, Z);
         void* dx_own = dx.is_same(dz) ? nullptr : dx.data_ptr();
