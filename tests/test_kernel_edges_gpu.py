@@ -958,3 +958,19 @@ def test_launches_are_counted_as_they_are(native):
         torch.cuda.synchronize()
     ran = sum(e.count for e in p.key_averages() if "rb::" in e.key)
     assert ran > 0 and _lib.launch_count() - before == ran
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_layernorm_of_one_leaf_twice(dtype):
+    """Both inputs the same leaf: its gradient is twice that of either, whose one tensor the backward writes."""
+    from rannc_b200.ops import functional as RF
+    from rannc_b200.ops import kernels as K
+
+    torch.manual_seed(33)
+    x = torch.randn(37, 1024, device="cuda").to(dtype).requires_grad_(True)
+    g, b = torch.randn(1024, device="cuda").to(dtype), torch.randn(1024, device="cuda").to(dtype)
+    dy = torch.randn(37, 1024, device="cuda").to(dtype)
+    RF.dropout_add_layer_norm(x, x, g, b, 0.0, 1e-5).backward(dy)
+    y, z, mean, rstd = K.ln_fwd(x.detach(), x.detach(), g, b, 1e-5)
+    dz = K.ln_bwd(dy, z, g, mean, rstd)[0]
+    assert torch.equal(x.grad, dz + dz)
