@@ -225,10 +225,11 @@ void gemm(const Mat& a, const Mat& b, bool trans_a, bool trans_b, void* out, boo
 // ---- rows of zeros in the gradient of a wide output layer (cuda/sparse_rows.cu) ----
 // The rows that count are gathered on the device, and each product is launched in two forms of which the device runs one.
 struct Rows {
-    Tensor idx, pos, ctl, dy, x, dx32;
-    Mat dym, xm;
-    int64_t room = 0;
-    int32_t* ctl_ptr() const { return static_cast<int32_t*>(ctl.data_ptr()); }
+    Tensor keep;   // all of it: one allocation
+    int32_t *idx = nullptr, *pos = nullptr, *ctl = nullptr;
+    float* dx32 = nullptr;   // the input gradient's parts, rows_out rows
+    Mat dy, x;
+    int64_t rows_out = 0;
 };
 // Worth a look at the rows: a wide output layer (the rows of hidden layers' gradients are not zero), and products long enough
 // that the look costs next to nothing where every row counts.  Backward of the layer (us), one B200, over all rows ->
@@ -260,37 +261,46 @@ int64_t gather_room(const Mat& dy, const Mat& x, int64_t products) {
     return gather_room(dy.rows, dy.cols, x.cols, api.gemm_pairs(), products);
 }
 // Scratch: three quarters of dy and of x, and 77 MB or three quarters of x in fp32, whatever the number of rows that count
-// (the host does not know it): 470 MB for 8192 x 1024 x 30528.  Where there is no memory for it, `ctl` stays empty.
+// (the host does not know it): 470 MB for 8192 x 1024 x 30528.  Where there is no memory for it, `keep` stays empty.
 Rows gather_rows(const Mat& dy, const Mat& x, int64_t room, bool want_dx, int dtype, const at::TensorOptions& o) {
     Rows r;
-    r.room = room;
-    const auto ints = o.dtype(at::kInt);
-    Tensor live;
+    // The input gradient's product is cut into parts along K, each in rows of its own and added up in their order (as
+    // reductions into one matrix they came in any, and dx did not repeat): room for four waves of tiles.
+    if (want_dx) r.rows_out = (std::max(room, 4 * api.gemm_pairs() * 256 / ((x.cols + 255) / 256)) + 255) / 256 * 256;
+    int64_t bytes = 0;
+    auto take = [&](int64_t n) {
+        const int64_t at = bytes;
+        bytes += (n + 255) / 256 * 256;
+        return at;
+    };
+    const int64_t ctl = take(16), idx = take(room * 4), pos = take(dy.rows * 4), live = take(dy.rows),
+                  dy_at = take(room * dy.cols * 2), x_at = take(room * x.cols * 2), dx_at = take(r.rows_out * x.cols * 4);
     try {
-        r.ctl = at::empty({4}, ints);
-        r.idx = at::empty({r.room}, ints);
-        r.pos = at::empty({dy.rows}, ints);
-        live = at::empty({dy.rows}, o.dtype(at::kByte));
-        r.dy = at::empty({r.room, dy.cols}, o);
-        r.x = at::empty({r.room, x.cols}, o);
-        if (want_dx) {
-            // the input gradient's product in parts along K, each in rows of its own and added up in their order (as
-            // reductions into one matrix they came in any, and dx did not repeat): room for four waves of tiles
-            const int64_t waves = 4 * api.gemm_pairs() * 256 / ((x.cols + 255) / 256);
-            r.dx32 = at::empty({(std::max(r.room, waves) + 255) / 256 * 256, x.cols}, o.dtype(at::kFloat));
-        }
+        r.keep = at::empty({bytes}, o.dtype(at::kByte));
     } catch (const c10::OutOfMemoryError&) {
-        return Rows();   // the products over all rows need none of it
+        return r;   // the products over all rows need none of it
     }
+    char* base = static_cast<char*>(r.keep.data_ptr());
+    r.ctl = reinterpret_cast<int32_t*>(base + ctl);
+    r.idx = reinterpret_cast<int32_t*>(base + idx);
+    r.pos = reinterpret_cast<int32_t*>(base + pos);
+    if (want_dx) r.dx32 = reinterpret_cast<float*>(base + dx_at);
+    auto gathered = [&](int64_t at, const Mat& of) {
+        Mat m;
+        m.keep = r.keep;
+        m.p = base + at;
+        m.rows = room;
+        m.cols = m.ld = of.cols;
+        return m;
+    };
+    r.dy = gathered(dy_at, dy);
+    r.x = gathered(x_at, x);
     check(api.rows_plan(dy.p, dy.ld, x.p, x.ld, static_cast<int>(dy.rows), static_cast<int>(dy.cols), static_cast<int>(x.cols),
-                        static_cast<int>(r.room), mptr<uint8_t>(live), mptr<int32_t>(r.idx), mptr<int32_t>(r.pos),
-                        mptr<int32_t>(r.ctl), dtype, cur_stream()),
+                        static_cast<int>(room), reinterpret_cast<uint8_t*>(base + live), r.idx, r.pos, r.ctl, dtype, cur_stream()),
           "rb_rows_plan", 2);
-    check(api.rows_gather(dy.p, dy.ld, x.p, x.ld, static_cast<int>(dy.cols), static_cast<int>(x.cols), mptr<int32_t>(r.idx),
-                          r.ctl_ptr(), r.dy.data_ptr(), r.x.data_ptr(), nullptr, cur_stream()),
+    check(api.rows_gather(dy.p, dy.ld, x.p, x.ld, static_cast<int>(dy.cols), static_cast<int>(x.cols), r.idx, r.ctl, base + dy_at,
+                          base + x_at, nullptr, cur_stream()),
           "rb_rows_gather");
-    r.dym = rows_of(r.dy);
-    r.xm = rows_of(r.x);
     return r;
 }
 
@@ -317,9 +327,9 @@ Grads param_grads(const Mat& dy, const Mat& x, const Tensor& w, const Tensor& w_
     // dW = dy^T x, over all rows or (whichever the device finds) over the gathered ones
     auto product = [&](void* to, bool fp32, Epi e, int64_t ldd) {
         if (rows) {
-            e.rows_ctl = rows->ctl_ptr();
+            e.rows_ctl = rows->ctl;
             e.rows_mode = RB_GEMM_ROWS_K;
-            gemm(rows->dym, rows->xm, true, false, to, fp32, dtype, e, ldd);
+            gemm(rows->dy, rows->x, true, false, to, fp32, dtype, e, ldd);
             e.rows_mode = RB_GEMM_ROWS_ALL;
         }
         gemm(dy, x, true, false, to, fp32, dtype, e, ldd);
@@ -444,17 +454,17 @@ struct LinearNode : Node {
             if (want_w && !w_mg.defined()) dw = at::empty({d.cols, xm.cols}, W.options());   // (before the look's scratch)
             rows = gather_rows(d, xm, room, want_dx, dt, X.options());
         }
-        const bool look = rows.ctl.defined();
+        const bool look = rows.keep.defined();
         if (want_dx) {
             const Mat wm = mat(W);
             Epi e;
             if (look) {
-                e.rows_ctl = rows.ctl_ptr();
+                e.rows_ctl = rows.ctl;
                 e.rows_mode = RB_GEMM_ROWS_M;
-                e.rows_out = static_cast<int>(rows.dx32.size(0));
-                gemm(rows.dym, wm, false, false, rows.dx32.data_ptr(), true, dt, e);
-                check(api.rows_scatter(mptr<float>(rows.dx32), dx.data_ptr(), static_cast<int>(d.rows),
-                                       static_cast<int>(xm.cols), mptr<int32_t>(rows.pos), rows.ctl_ptr(), dt, cur_stream()),
+                e.rows_out = static_cast<int>(rows.rows_out);
+                gemm(rows.dy, wm, false, false, rows.dx32, true, dt, e);
+                check(api.rows_scatter(rows.dx32, dx.data_ptr(), static_cast<int>(d.rows), static_cast<int>(xm.cols), rows.pos,
+                                       rows.ctl, dt, cur_stream()),
                       "rb_rows_scatter");
                 e.rows_mode = RB_GEMM_ROWS_ALL;
             }
